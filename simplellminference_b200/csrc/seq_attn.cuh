@@ -1,5 +1,5 @@
 // csrc/seq_attn.cuh — what the attention kernels of the ragged token batch share (seq_attn.cu, seq_attn_talk.cu): tile sizes, which keys a
-// query sees and which key tiles a CTA visits, the bf16 tensor-core product and its operand packing, asynchronous copies.
+// query sees and which key tiles a CTA visits, the bf16 tensor-core product and its operand packing.
 #pragma once
 #include <climits>
 
@@ -48,15 +48,6 @@ __device__ __forceinline__ void split_bf16(float p0, float p1, uint32_t* hi, uin
     *hi = h;
     *lo = pack_bf16(p0 - __uint_as_float(h << 16), p1 - __uint_as_float(h & 0xffff0000u));
 }
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-// 16 bytes global -> shared without passing through registers; bytes = 0 writes zeros and reads nothing
-__device__ __forceinline__ void cp_async16(void* dst, const void* src, int bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 #endif
 

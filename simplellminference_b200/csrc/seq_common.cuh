@@ -54,6 +54,29 @@ __device__ __forceinline__ void seq_angle(int pos, double freq, float* sn, float
     *cs = (float)c;
 }
 
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// 16 bytes global -> shared without passing through registers; bytes = 0 writes zeros and reads nothing
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// two fp32 values in one 64-bit register, and the multiply-add that works on both at once (each half rounded as fmaf rounds)
+__device__ __forceinline__ uint64_t pair_f32(uint32_t lo, uint32_t hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+    return r;
+}
+__device__ __forceinline__ uint64_t pair_f32(float lo, float hi) { return pair_f32(__float_as_uint(lo), __float_as_uint(hi)); }
+__device__ __forceinline__ float pair_sum(uint64_t v) {
+    uint32_t lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v));
+    return __uint_as_float(lo) + __uint_as_float(hi);
+}
+__device__ __forceinline__ void fma_pair(uint64_t& acc, uint64_t a, uint64_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
+
 // element index of (page, kv head, row in page, 0) in a pool [pages][kv_heads][page_len][width]
 __device__ __forceinline__ size_t seq_pool_row(int page, int kv_heads, int g, int page_len, int in_page, int width) {
     return (((size_t)page * kv_heads + g) * page_len + in_page) * width;

@@ -1,7 +1,6 @@
 // csrc/seq_linear.cu — sllm_seq_linear: C = alpha * (A . W^T + bias) (+ C) for the ragged token batch. Three bodies:
-//   * rows_kernel  (T <= 8, decode-sized steps): 1 to 8 warps per output column stream that weight row once with 16-byte loads, two batches of two in
-//     flight per lane, one accumulator per activation row — the bandwidth-bound shape of the one-sequence path's GEMV, any size (scalar
-//     loads when unaligned);
+//   * rows_kernel  (T <= 8, decode-sized steps): every weight streamed once, the activations of a lane's columns in registers; a body without that
+//     set-up for small matrices, with scalar loads where 16-byte accesses do not fit;
 //   * tile_kernel  (any shape): 64 x 64 x 16 shared-memory tiles, 4 x 4 outputs per thread, fp32 FMAs with fp32 accumulation. This is
 //     the body of the all-fp32 mode, and of bf16 products whose shape the tensor-core tiles do not take;
 //   * the tcgen05 GEMM of the prefill path (prefill_gemm.cu) for bf16 weights when the caller passes a bf16 scratch for A and the shape
@@ -26,18 +25,200 @@ struct LinArgs {
 };
 
 constexpr int kRowsMax = 8;
-#ifndef SLLM_ROWS_INFLIGHT
-#define SLLM_ROWS_INFLIGHT 2
-#endif
-#ifndef SLLM_ROWS_MINB
-#define SLLM_ROWS_MINB 4   // resident CTAs per SM the register budget is cut for (measured: 4 streams 14 % faster than the unconstrained 3; 5 and more spill)
-#endif
-constexpr int kInFlight = SLLM_ROWS_INFLIGHT;   // 16-byte weight loads per batch and lane; two batches are in flight (measured: 2 x 2 at four resident CTAs beats 1 x 4 by 12 %)
+constexpr int kRowsBlock = 64;     // weight rows between two flushes of the partial sums
 
-// `wpr` warps (1, 2, 4 or 8) share one output column and cut K among them, so that a matrix with few rows and long rows still fills the
+// TT: activation rows the products are computed for (T rounded up to 1, 2, 4 or 8). A lane owns two 16-byte chunks of every weight row of a panel
+// of K and keeps the matching activations of all TT rows in registers (8 rows: half as many warps, so that they fit); kGroup weight rows are
+// reduced across the lanes together; kDeep rows are in flight per warp. The ring comes to 128 KB per SM, more than twice what the HBM rate asks
+// for at its latency.
+template <int TT>
+struct RowsShape {
+    static constexpr int kWarps = TT <= 4 ? 16 : 8, kChunks = 2, kGroup = TT <= 4 ? 4 : 2, kDeep = TT <= 4 ? 8 : 16;
+    static constexpr int kRing = kWarps * kDeep * kChunks * 512;
+};
+
+// Up to 8 activation rows against a stream of weight rows. Bound: HBM, every weight is read once. One CTA per SM takes a contiguous
+// share of the weight rows; WK = 2^wk_log2 of its warps cut K among themselves (so that every SM's share ends at the same time whatever N), the
+// others take other rows. What a weight costs beside its load was the bound of a body whose lanes read the activations from memory for every weight
+// row (2 T bytes of activations through L1 per byte of weights: 1.1 TB/s at 4 rows of 6144 x 4096 bf16, now 3.1; one row 2.6, now 4.2 and 5.3 at
+// 32000 x 2048): here the activations of a lane's columns stay in registers for all rows, the
+// weights arrive through cp.async in a ring that only their own lane reads back (no barrier in the stream), fma.rn.f32x2 does two products per
+// instruction, and TT x kGroup sums cross the lanes in one halving exchange.
+template <int WD, int TT>
+__global__ void __launch_bounds__(RowsShape<TT>::kWarps * 32, 1) seq_linear_rows_kernel(LinArgs p, int wk_log2) {
+    using Shape = RowsShape<TT>;
+    constexpr int E = WD == SLLM_BF16 ? 8 : 4;                 // weights per 16-byte chunk
+    constexpr int C = Shape::kChunks, RG = Shape::kGroup, D = Shape::kDeep, V = RG * TT;
+    extern __shared__ __align__(16) uint8_t rows_smem[];
+    const int b = blockIdx.y;
+    const int wb = p.w_index ? p.w_index[b] : b;               // which matrix of W; negative: none (the outputs are zeros)
+    const float* A = p.A + (size_t)(p.a_div > 1 ? b / p.a_div : b) * p.a_bs;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int WK = 1 << wk_log2, WR = Shape::kWarps >> wk_log2, wk = warp & (WK - 1), wr = warp >> wk_log2;
+    const int n_lo = (int)((long long)p.N * blockIdx.x / gridDim.x), rows = (int)((long long)p.N * (blockIdx.x + 1) / gridDim.x) - n_lo;
+    const int chunks = wb >= 0 ? p.K / E : 0, panel = WK * 32 * C, panels = max(1, (chunks + panel - 1) / panel);
+    const int blocks = (rows + kRowsBlock - 1) / kRowsBlock;
+    const size_t row_bytes = (size_t)p.ldw * (16 / E);
+    const uint8_t* w = reinterpret_cast<const uint8_t*>(p.W) + ((size_t)max(wb, 0) * p.w_bs) * (16 / E) + (size_t)(n_lo + wr) * row_bytes;
+    const uint32_t ring = smem_u32(rows_smem) + warp * (D * C * 512) + lane * 16;
+    float* table = reinterpret_cast<float*>(rows_smem + Shape::kRing);      // [2][WK][kRowsBlock][TT]
+
+    // Weight rows in the order in which they are consumed: per block of rows, per panel of K, the warp's rows in groups of RG. `run` counts the rows
+    // of the current (block, panel) that are still to be asked for; rows that only fill up a group are not fetched and their sums not used.
+    int i_blk = 0, i_pan = 0, run = 0, pad = 0;
+    const uint8_t* src = w;
+    uint32_t off[C], bytes[C], fill = ring;
+    const size_t step = row_bytes << (__ffs(WR) - 1);
+    auto begin_run = [&]() {
+        const int cur = min(kRowsBlock, rows - i_blk * kRowsBlock);
+        run = max(0, (cur - wr + WR - 1) / WR);
+        pad = ((cur + WR - 1) / WR + RG - 1) / RG * RG - run;
+        src = w + (size_t)i_blk * kRowsBlock * row_bytes;
+#pragma unroll
+        for (int j = 0; j < C; ++j) {
+            const int ch = i_pan * panel + (j * WK + wk) * 32 + lane;
+            off[j] = ch < chunks ? ch * 16 : 0;
+            bytes[j] = ch < chunks ? 16 : 0;
+        }
+    };
+    auto issue = [&]() {
+        if (run > 0) {
+#pragma unroll
+            for (int j = 0; j < C; ++j)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(fill + j * 512), "l"(src + off[j]), "r"(bytes[j]) : "memory");
+            src += step;
+            --run;
+        } else {
+            --pad;
+        }
+        fill = fill + C * 512 == ring + D * C * 512 ? ring : fill + C * 512;
+        cp_async_commit();
+        if (run + pad == 0 && i_blk < blocks) {
+            if (++i_pan == panels) {
+                i_pan = 0;
+                ++i_blk;
+            }
+            if (i_blk < blocks) begin_run();
+            else pad = 1 << 30;          // nothing left: empty groups from here on
+        }
+    };
+    // the activations of this lane's columns of a panel
+    uint64_t act[TT][C][E / 2];
+    auto load_act = [&](int pan) {
+#pragma unroll
+        for (int t = 0; t < TT; ++t)
+#pragma unroll
+            for (int j = 0; j < C; ++j) {
+                const int ch = pan * panel + (j * WK + wk) * 32 + lane;
+                const bool ok = t < p.T && ch < chunks;
+#pragma unroll
+                for (int e = 0; e < E; e += 4) {
+                    float4 a = ok ? *reinterpret_cast<const float4*>(A + (size_t)t * p.lda + (size_t)ch * E + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (p.round_a) a = make_float4(seq_round_bf16(a.x), seq_round_bf16(a.y), seq_round_bf16(a.z), seq_round_bf16(a.w));
+                    act[t][j][e / 2] = pair_f32(a.x, a.y);
+                    act[t][j][e / 2 + 1] = pair_f32(a.z, a.w);
+                }
+            }
+    };
+    if (blocks) begin_run(); else pad = 1 << 30;
+#pragma unroll
+    for (int i = 0; i < D / 2; ++i) issue();
+    load_act(0);
+#pragma unroll
+    for (int i = D / 2; i < D; ++i) issue();
+
+    // after the exchange a lane holds the sum of row `which / TT` of the group and activation row `which % TT`
+    int which = 0;
+#pragma unroll
+    for (int n = V / 2, bit = 16; n >= 1; n /= 2, bit /= 2) which = which * 2 + ((lane & bit) ? 1 : 0);
+    const bool writes = lane % (32 / V) == 0;
+    uint32_t slot = ring;
+    for (int blk = 0; blk < blocks; ++blk) {
+        const int cur = min(kRowsBlock, rows - blk * kRowsBlock), steps = (cur + WR - 1) / WR;
+        float* tab = table + (size_t)(blk & 1) * (WK * kRowsBlock * TT);
+        for (int pan = 0; pan < panels; ++pan) {
+            if (pan + blk > 0 && panels > 1) load_act(pan);
+            float* cell = tab + (size_t)(wk * kRowsBlock + (which / TT) * WR + wr) * TT + which % TT;
+            for (int g = 0; g < steps; g += RG, cell += RG * WR * TT) {
+                cp_async_wait<D - RG>();
+                uint64_t acc[RG][TT];
+                uint4 us[2][C];       // two rows' chunks on their way (D is a multiple of RG: a group's slots are adjacent)
+                auto fetch = [&](int r) {
+#pragma unroll
+                    for (int j = 0; j < C; ++j)
+                        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                                     : "=r"(us[r & 1][j].x), "=r"(us[r & 1][j].y), "=r"(us[r & 1][j].z), "=r"(us[r & 1][j].w)
+                                     : "r"(slot + (r * C + j) * 512)
+                                     : "memory");
+                };
+                fetch(0);
+#pragma unroll
+                for (int r = 0; r < RG; ++r) {
+                    if (r + 1 < RG) fetch(r + 1);
+#pragma unroll
+                    for (int t = 0; t < TT; ++t) acc[r][t] = 0ull;
+#pragma unroll
+                    for (int j = 0; j < C; ++j) {
+                        const uint4 u = us[r & 1][j];
+                        uint64_t wv[E / 2];
+                        if (WD == SLLM_BF16) {
+                            wv[0] = pair_f32(u.x << 16, u.x & 0xffff0000u);
+                            wv[1] = pair_f32(u.y << 16, u.y & 0xffff0000u);
+                            wv[E / 2 - 2] = pair_f32(u.z << 16, u.z & 0xffff0000u);
+                            wv[E / 2 - 1] = pair_f32(u.w << 16, u.w & 0xffff0000u);
+                        } else {
+                            wv[0] = pair_f32(u.x, u.y);
+                            wv[1] = pair_f32(u.z, u.w);
+                        }
+#pragma unroll
+                        for (int t = 0; t < TT; ++t)
+#pragma unroll
+                            for (int e = 0; e < E / 2; ++e) fma_pair(acc[r][t], wv[e], act[t][j][e]);
+                    }
+                }
+                slot = slot + RG * C * 512 == ring + D * C * 512 ? ring : slot + RG * C * 512;
+#pragma unroll
+                for (int r = 0; r < RG; ++r) issue();
+                // V sums over 32 lanes: in every step a lane keeps half of its values and gets the partner's part of them
+                float v[V];
+#pragma unroll
+                for (int r = 0; r < RG; ++r)
+#pragma unroll
+                    for (int t = 0; t < TT; ++t) v[r * TT + t] = pair_sum(acc[r][t]);
+#pragma unroll
+                for (int n = V / 2, bit = 16; n >= 1; n /= 2, bit /= 2) {
+                    const bool up = lane & bit;
+#pragma unroll
+                    for (int i = 0; i < n; ++i) {
+                        const float give = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+                        v[i] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+                    }
+                }
+#pragma unroll
+                for (int o = 16 / V; o >= 1; o /= 2) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+                if (writes && (g + which / TT) * WR + wr < kRowsBlock) *cell = pan ? *cell + v[0] : v[0];
+            }
+        }
+        __syncthreads();
+        const float* bias = p.bias ? p.bias + (size_t)b * p.bias_bs : nullptr;
+        float* out = p.C + (size_t)b * p.c_bs;
+        for (int o = threadIdx.x; o < cur * p.T; o += Shape::kWarps * 32) {
+            const int t = o / cur, r = o % cur, n = n_lo + blk * kRowsBlock + r;
+            float sum = 0.0f;
+            for (int k = 0; k < WK; ++k) sum += tab[(size_t)(k * kRowsBlock + r) * TT + t];
+            const float val = p.alpha * (sum + (bias ? bias[n] : 0.0f));
+            float* c = out + (size_t)t * p.ldc + n;
+            *c = p.accumulate ? *c + val : val;
+        }
+    }
+}
+
+constexpr int kInFlight = 2;   // 16-byte weight loads per batch and lane; two batches are in flight (measured: 2 x 2 at four resident CTAs beats 1 x 4 by 12 %)
+
+// Small matrices (launch_rows says which) and accesses that are not 16 bytes wide: `wpr` warps (1, 2, 4 or 8) share one output column and cut K among them, so that a matrix with few rows and long rows still fills the
 // machine; a lane keeps two batches of 16-byte weight loads in flight (the next batch travels while this one is multiplied). The partial sums of a column meet in shared memory in a fixed order.
 template <int WD>
-__global__ void __launch_bounds__(256, SLLM_ROWS_MINB) seq_linear_rows_kernel(LinArgs p, int vec, int wpr) {
+__global__ void __launch_bounds__(256, 4) seq_linear_rows_small_kernel(LinArgs p, int vec, int wpr) {
     __shared__ float part_sum[8][kRowsMax];
     const int b = blockIdx.y;
     const int wb = p.w_index ? p.w_index[b] : b;             // which matrix of W; negative: none (the outputs are zeros)
@@ -220,17 +401,49 @@ __global__ void seq_linear_epilogue_kernel(const float* __restrict__ P, const fl
 
 using namespace sllm;
 
+template <int WD, int TT>
+static int launch_rows_body(const sllm::LinArgs& p, int batch, cudaStream_t st) {
+    using namespace sllm;
+    using Shape = RowsShape<TT>;
+    constexpr int E = WD == SLLM_BF16 ? 8 : 4;
+    int wk_log2 = 0;      // as many warps along K as one panel of it needs
+    while ((1 << wk_log2) < Shape::kWarps && (32 * Shape::kChunks << wk_log2) < p.K / E) ++wk_log2;
+    const size_t smem = Shape::kRing + 2 * ((size_t)kRowsBlock * TT * sizeof(float) << wk_log2);
+    static bool sized = false;
+    if (!sized) {
+        SLLM_CUDA(cudaFuncSetAttribute(seq_linear_rows_kernel<WD, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       Shape::kRing + 2 * Shape::kWarps * kRowsBlock * TT * (int)sizeof(float)));
+        sized = true;
+    }
+    const dim3 grid(std::max(1, std::min(p.N, sm_count() / batch)), batch);      // one CTA per SM, however many products share the launch
+    seq_linear_rows_kernel<WD, TT><<<grid, Shape::kWarps * 32, smem, st>>>(p, wk_log2);
+    return SLLM_OK;
+}
+
 // the rows body: up to 8 activation rows per product, `batch` products
 static int launch_rows(const sllm::LinArgs& p, int batch, cudaStream_t st) {
     using namespace sllm;
-    const int e = p.w_dtype == SLLM_BF16 ? 8 : 4;   // elements per 16-byte weight load
+    const bool bf16 = p.w_dtype == SLLM_BF16;
+    const int e = bf16 ? 8 : 4;   // elements per 16-byte weight load
     const bool vec = p.K % e == 0 && p.ldw % e == 0 && (p.w_bs % e) == 0 && p.lda % 4 == 0 && (p.a_bs % 4) == 0 && ((uintptr_t)p.W % 16) == 0 &&
                      ((uintptr_t)p.A % 16) == 0;
-    int wpr = 1;   // warps per output column: enough CTAs for ~4 per SM, and no warp with less than 256 weights
-    while (wpr < 8 && (long long)p.N * batch * wpr / 8 < 4LL * sm_count() && p.K / (2 * wpr) >= 256) wpr *= 2;
-    dim3 grid(((long long)p.N * wpr + 7) / 8, batch);
-    if (p.w_dtype == SLLM_BF16) seq_linear_rows_kernel<SLLM_BF16><<<grid, 256, 0, st>>>(p, vec, wpr);
-    else seq_linear_rows_kernel<SLLM_F32><<<grid, 256, 0, st>>>(p, vec, wpr);
+    // The streaming body starts 1.4 to 2 us later than the small one (its ring, its activations, more code) and is faster from about 2 million
+    // weights on. Measured, bf16, old | new: 1024 x 1024 3.8 | 4.5 us (one row) and 4.7 | 6.9 (four), 2048 x 2048 6.4 | 5.2 and 9.4 | 7.9, 32 matrices of
+    // 512 x 128 13.4 | 8.7 (four), 6144 x 4096 19.4 | 12.0 (one), 46.9 | 16.3 (four) and 85.4 | 21.7 (eight), 32000 x 2048 40.1 | 24.8 (one row).
+    if (vec && (long long)p.N * batch * p.K >= 1500000LL) {
+        int rc;
+        if (p.T == 1) rc = bf16 ? launch_rows_body<SLLM_BF16, 1>(p, batch, st) : launch_rows_body<SLLM_F32, 1>(p, batch, st);
+        else if (p.T == 2) rc = bf16 ? launch_rows_body<SLLM_BF16, 2>(p, batch, st) : launch_rows_body<SLLM_F32, 2>(p, batch, st);
+        else if (p.T <= 4) rc = bf16 ? launch_rows_body<SLLM_BF16, 4>(p, batch, st) : launch_rows_body<SLLM_F32, 4>(p, batch, st);
+        else rc = bf16 ? launch_rows_body<SLLM_BF16, 8>(p, batch, st) : launch_rows_body<SLLM_F32, 8>(p, batch, st);
+        if (rc != SLLM_OK) return rc;
+    } else {
+        int wpr = 1;   // warps per output column: enough CTAs for ~4 per SM, and no warp with less than 256 weights
+        while (wpr < 8 && (long long)p.N * batch * wpr / 8 < 4LL * sm_count() && p.K / (2 * wpr) >= 256) wpr *= 2;
+        dim3 grid(((long long)p.N * wpr + 7) / 8, batch);
+        if (bf16) seq_linear_rows_small_kernel<SLLM_BF16><<<grid, 256, 0, st>>>(p, vec, wpr);
+        else seq_linear_rows_small_kernel<SLLM_F32><<<grid, 256, 0, st>>>(p, vec, wpr);
+    }
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;
