@@ -11,8 +11,9 @@
 // queries. A tile of 32 keys and values of the head's kv head is staged in shared memory (fp32); a lane owns one key for the scores
 // (16-byte shared loads, rows padded by 4 floats: conflict-free) and dv/32 output columns for the weighted sum; online softmax per query
 // with warp reductions. The key tiles are dealt to `nsplit` CTAs in turn (long contexts with few queries: decode), every CTA leaves
-// (max, sum, unnormalised output) and seq_attention_finish_kernel merges them.
-#include "seq_attn.cuh"
+// (max, sum, unnormalised output) and seq_attention_finish_kernel merges them. Steps of single tokens with the common head widths run in
+// seq_attn_decode.cuh instead.
+#include "seq_attn_decode.cuh"
 
 namespace sllm {
 
@@ -20,31 +21,6 @@ extern int g_tune_seq_attn_mma;   // runtime.cu: 1 (default) = tensor-core atten
 
 constexpr int kQW = 4;   // queries per warp of the fp32 body
 
-struct AttnArgs {
-    sllm_seq_batch b;
-    const float* q; int ldq, heads, kv_heads, dk, dv; float scale;
-    const void *k_pool, *v_pool;
-    int nsplit; float* ws;
-    int by_head;   // fp32 body, steps of single tokens: a CTA's "queries" are the query heads of ONE kv head at one token (they share its tiles)
-    int window, keep_first;   // query i sees key j <= i when i - j < window or j < keep_first (window INT_MAX = everything before it)
-    float softcap;            // > 0: score <- softcap * tanh(score / softcap)
-    const float* slopes;      // [heads] or NULL: score <- score - slopes[h] * (i - j)
-    int v_in_k;               // values = the first dv columns of the key rows (v_pool unused)
-    const float* logdist;     // [2][heads] or NULL: score <- score - r1[h] * ln(1 + r2[h] * (i - j)), r1 = row 0, r2 = row 1
-    // Every query head's weights on every key/value head's values: `heads` then counts kv_heads * q_heads results, result u = (value
-    // head u / q_heads, query head u % q_heads); the query head reads the KEYS of its own key/value head as always. Otherwise q_heads = heads.
-    int q_heads, cross;
-    int chunk;                // > 0: a query sees its own chunk of `chunk` positions only (then window / keep_first are not used)
-    float* out; int ldo; uint16_t* out16;   // tensor-core body, one share: the normalised result goes here (fp32 [T][ldo] and / or dense bf16) instead of ws
-};
-
-__device__ __forceinline__ float seq_score(float dot, float scale, float softcap, float slope, float r1, float r2, int qpos, int key) {
-    float sc = dot * scale;
-    if (softcap > 0.0f) sc = softcap * tanhf(sc / softcap);
-    sc -= slope * (float)(qpos - key);
-    if (r1 != 0.0f) sc -= r1 * log1pf(r2 * (float)(qpos - key));
-    return sc;
-}
 template <typename KV, int kMaxDvChunks>   // dv <= 32 * kMaxDvChunks
 __global__ void __launch_bounds__(256) seq_attention_kernel(AttnArgs p) {
     extern __shared__ __align__(16) float sm[];
@@ -577,6 +553,49 @@ int sllm_seq_rotary_kv(const sllm_seq_batch* b, float* q, int32_t ldq, int32_t h
 
 }  // extern "C"
 
+// One query per sequence, head widths the register body takes. Contexts live on the device, so the spread does not depend on them: a cluster of up to
+// 16 CTAs per (sequence, query heads of a kv head, share), at most four CTAs of 128 threads per SM in all.
+template <typename KV, int KL, int VL, int G, int kSteps>
+static int launch_attention_decode(const sllm::AttnArgs& p, cudaStream_t st) {
+    using namespace sllm;
+    auto* kernel = seq_attention_decode_kernel<KV, KL, VL, G, kSteps>;
+    static bool allowed = false;
+    if (!allowed) {
+        SLLM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        allowed = true;
+    }
+    const long long items = (long long)p.b.n_qtiles * (p.heads / G) * p.nsplit;
+    int cs = kDecodeCluster;
+    while (cs > 1 && items * cs > 4LL * sm_count()) cs /= 2;
+    while (cs > 1 && (long long)p.nsplit * cs > 65535) cs /= 2;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(p.b.n_qtiles, p.heads / G, p.nsplit * cs);
+    cfg.blockDim = dim3(kDecodeWarps * 32);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = cs;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    SLLM_CUDA(cudaLaunchKernelEx(&cfg, kernel, p));
+    ++g_launches;
+    return SLLM_OK;
+}
+
+template <typename KV, int L128, int S4, int S2, int S1>      // loads per lane of a 128-wide row, rows in flight per lane by query heads of a CTA
+static int attention_decode(const sllm::AttnArgs& p, cudaStream_t st) {
+    const int group = p.heads / p.kv_heads;
+    if (p.dk == 128) {
+        if (group % 4 == 0) return launch_attention_decode<KV, L128, L128, 4, S4>(p, st);
+        if (group % 2 == 0) return launch_attention_decode<KV, L128, L128, 2, S2>(p, st);
+        return launch_attention_decode<KV, L128, L128, 1, S1>(p, st);
+    }
+    if (group % 4 == 0) return launch_attention_decode<KV, L128 / 2, L128 / 2, 4, S4>(p, st);
+    if (group % 2 == 0) return launch_attention_decode<KV, L128 / 2, L128 / 2, 2, S2>(p, st);
+    return launch_attention_decode<KV, L128 / 2, L128 / 2, 1, S1>(p, st);
+}
+
 // out / out16 given: the merged result goes there; *merged says whether this launch has written it (else the shares wait in ws)
 static int attention_run(const sllm_seq_batch* b, const float* q, int32_t ldq, int32_t heads, int32_t kv_heads, int32_t dk, int32_t dv, float scale, const void* k_pool,
                          const void* v_pool, int32_t kv_dtype, int32_t nsplit, float* ws, const sllm_seq_attn_opts* opts, float* out, int32_t ldo, uint16_t* out16,
@@ -631,6 +650,18 @@ static int attention_run(const sllm_seq_batch* b, const float* q, int32_t ldq, i
         ++g_launches;
         SLLM_LAUNCH_CHECK();
         return SLLM_OK;
+    }
+    // Single tokens with heads of 64 or 128: rows straight from the pools into registers, a cluster per sequence and kv head. The staged body below waits for
+    // every tile of 32 keys (12 us each) and cuts a context into nsplit shares only. Measured, staged with its merge | this one: 8 requests of 77 to
+    // 8000 positions, 32 heads over 8 of 128 bf16 columns 751 | 57 us; one of 8000 106 | 25; 32 of 2048 770 | 84; one of 64 positions 17 | 7.
+    if (b->T == b->nseg && b->n_qtiles == b->nseg && !p.cross && !v_in_k && dk == dv && (dk == 64 || dk == 128) && ((uintptr_t)k_pool % 16) == 0 &&
+        ((uintptr_t)v_pool % 16) == 0) {
+        if (out || out16) {
+            p.out = out; p.ldo = ldo; p.out16 = out16;
+            p.nsplit = 1;
+            *merged = true;
+        }
+        return kv_dtype == SLLM_F32 ? attention_decode<float, 4, 2, 2, 4>(p, as_stream(stream)) : attention_decode<uint16_t, 2, 4, 4, 8>(p, as_stream(stream));
     }
     if (b->T == b->nseg && heads / kv_heads <= kBQ) {   // single tokens only: the query heads of a kv head share one CTA and its tiles
         p.by_head = 1;
