@@ -553,24 +553,20 @@ int sllm_seq_rotary_kv(const sllm_seq_batch* b, float* q, int32_t ldq, int32_t h
 
 }  // extern "C"
 
-// One query per sequence, head widths the register body takes. Contexts live on the device, so the spread does not depend on them: a cluster of up to
-// 16 CTAs per (sequence, query heads of a kv head, share), at most four CTAs of 128 threads per SM in all.
-template <typename KV, int KL, int VL, int G, int kSteps>
-static int launch_attention_decode(const sllm::AttnArgs& p, cudaStream_t st) {
+// One query per sequence, head widths the bodies of seq_attn_decode.cuh take. Contexts live on the device, so the spread does not depend on them: a
+// cluster of up to 16 CTAs per (sequence, G query heads of a kv head, share), two CTAs of 128 threads per SM in all. Clusters of 16 find few places at a
+// time, so they pay only when the step has no more of them than fit at once. Measured (us) at 16 | 8 | 4 CTAs: one request of 8000 positions, 8 kv
+// heads 17.9 | 23.4 | 35.0; four of 2048, 4 kv heads 17.6 | 11.2 | 13.1; with twice as many CTAs 32 requests of 2048 take 54 instead of 47.
+template <typename Kernel, typename... Args>
+static int launch_attention_decode(Kernel* kernel, int G, int smem, const sllm::AttnArgs& p, cudaStream_t st, Args... args) {
     using namespace sllm;
-    auto* kernel = seq_attention_decode_kernel<KV, KL, VL, G, kSteps>;
-    static bool allowed = false;
-    if (!allowed) {
-        SLLM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        allowed = true;
-    }
     const long long items = (long long)p.b.n_qtiles * (p.heads / G) * p.nsplit;
-    int cs = kDecodeCluster;
-    while (cs > 1 && items * cs > 4LL * sm_count()) cs /= 2;
-    while (cs > 1 && (long long)p.nsplit * cs > 65535) cs /= 2;
+    int cs = items * kDecodeCluster <= sm_count() ? kDecodeCluster : kDecodeCluster / 2;
+    while (cs > 1 && (items * cs > 2LL * sm_count() || (long long)p.nsplit * cs > 65535)) cs /= 2;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(p.b.n_qtiles, p.heads / G, p.nsplit * cs);
     cfg.blockDim = dim3(kDecodeWarps * 32);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -578,22 +574,48 @@ static int launch_attention_decode(const sllm::AttnArgs& p, cudaStream_t st) {
     attr[0].val.clusterDim.z = cs;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    SLLM_CUDA(cudaLaunchKernelEx(&cfg, kernel, p));
+    SLLM_CUDA(cudaLaunchKernelEx(&cfg, kernel, p, args...));
     ++g_launches;
     return SLLM_OK;
 }
 
-template <typename KV, int L128, int S4, int S2, int S1>      // loads per lane of a 128-wide row, rows in flight per lane by query heads of a CTA
-static int attention_decode(const sllm::AttnArgs& p, cudaStream_t st) {
-    const int group = p.heads / p.kv_heads;
-    if (p.dk == 128) {
-        if (group % 4 == 0) return launch_attention_decode<KV, L128, L128, 4, S4>(p, st);
-        if (group % 2 == 0) return launch_attention_decode<KV, L128, L128, 2, S2>(p, st);
-        return launch_attention_decode<KV, L128, L128, 1, S1>(p, st);
+template <int D, bool kOpts>
+static int attention_decode_bf16(const sllm::AttnArgs& p, cudaStream_t st) {
+    using namespace sllm;
+    auto* kernel = seq_attention_decode_mma_kernel<D, kOpts>;
+    static bool ready = false;
+    if (!ready) {
+        SLLM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        SLLM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DecodeTile<D>::kSmem));
+        ready = true;
     }
-    if (group % 4 == 0) return launch_attention_decode<KV, L128 / 2, L128 / 2, 4, S4>(p, st);
-    if (group % 2 == 0) return launch_attention_decode<KV, L128 / 2, L128 / 2, 2, S2>(p, st);
-    return launch_attention_decode<KV, L128 / 2, L128 / 2, 1, S1>(p, st);
+    const int group = p.heads / p.kv_heads;
+    const int G = group % 4 == 0 ? 4 : group % 3 == 0 ? 3 : group % 2 == 0 ? 2 : 1;
+    return launch_attention_decode(kernel, G, DecodeTile<D>::kSmem, p, st, G);
+}
+
+template <int L, int G, int S>      // loads per lane of a row, query heads of a CTA, rows in flight per lane
+static int attention_decode_f32(const sllm::AttnArgs& p, cudaStream_t st) {
+    using namespace sllm;
+    auto* kernel = seq_attention_decode_kernel<float, L, L, G, S>;
+    static bool ready = false;
+    if (!ready) {
+        SLLM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        ready = true;
+    }
+    return launch_attention_decode(kernel, G, 0, p, st);
+}
+
+static int attention_decode(const sllm::AttnArgs& p, int kv_dtype, cudaStream_t st) {
+    const int group = p.heads / p.kv_heads;
+    if (kv_dtype == SLLM_BF16) {
+        const bool opts = p.softcap > 0.0f || p.slopes || p.logdist;
+        if (p.dk == 128) return opts ? attention_decode_bf16<128, true>(p, st) : attention_decode_bf16<128, false>(p, st);
+        return opts ? attention_decode_bf16<64, true>(p, st) : attention_decode_bf16<64, false>(p, st);
+    }
+    if (p.dk == 128)
+        return group % 4 == 0 ? attention_decode_f32<4, 4, 2>(p, st) : group % 2 == 0 ? attention_decode_f32<4, 2, 2>(p, st) : attention_decode_f32<4, 1, 4>(p, st);
+    return group % 4 == 0 ? attention_decode_f32<2, 4, 2>(p, st) : group % 2 == 0 ? attention_decode_f32<2, 2, 2>(p, st) : attention_decode_f32<2, 1, 4>(p, st);
 }
 
 // out / out16 given: the merged result goes there; *merged says whether this launch has written it (else the shares wait in ws)
@@ -615,7 +637,7 @@ static int attention_run(const sllm_seq_batch* b, const float* q, int32_t ldq, i
     const int dkp = ((dk + 3) & ~3) + 4;
     const size_t smem = ((size_t)(kBQ + kBK) * dkp + (v_in_k ? 0 : (size_t)kBK * dv)) * sizeof(float);
     SLLM_REQUIRE(smem <= (size_t)smem_optin_bytes(), SLLM_ENOTSUP, "seq_attention: heads of %d + %d floats need %zu bytes of shared memory", dk, dv, smem);
-    AttnArgs p{*b, q, ldq, heads, kv_heads, dk, dv, scale, k_pool, v_pool, nsplit, ws, 0, INT_MAX, 0, 0.0f, nullptr, 0, nullptr, heads, 0, 0, nullptr, 0, nullptr};
+    AttnArgs p{*b, q, ldq, heads, kv_heads, dk, dv, scale, k_pool, v_pool, nsplit, ws, 0, INT_MAX, 0, 0.0f, nullptr, 0, nullptr, heads, 0, 0, nullptr, 0, nullptr, (uint32_t)(((1ull << 32) + b->page_len - 1) / b->page_len)};
     if (opts && opts->cross_values) {
         SLLM_REQUIRE(!v_in_k, SLLM_EINVAL, "seq_attention: values of every head need a value pool");
         p.cross = 1;
@@ -651,9 +673,9 @@ static int attention_run(const sllm_seq_batch* b, const float* q, int32_t ldq, i
         SLLM_LAUNCH_CHECK();
         return SLLM_OK;
     }
-    // Single tokens with heads of 64 or 128: rows straight from the pools into registers, a cluster per sequence and kv head. The staged body below waits for
-    // every tile of 32 keys (12 us each) and cuts a context into nsplit shares only. Measured, staged with its merge | this one: 8 requests of 77 to
-    // 8000 positions, 32 heads over 8 of 128 bf16 columns 751 | 57 us; one of 8000 106 | 25; 32 of 2048 770 | 84; one of 64 positions 17 | 7.
+    // Single tokens with heads of 64 or 128: the bodies of seq_attn_decode.cuh, a cluster per sequence and kv head. The staged body below waits for
+    // every tile of 32 keys (12 us each) and cuts a context into nsplit shares only. Measured, staged with its merge | cluster, bf16 pools: 8 requests
+    // of 77 to 8000 positions, 32 heads over 8 of 128 columns 751 | 40 us; one of 8000 106 | 18; 32 of 2048 770 | 47; one of 64 positions 17 | 6.5.
     if (b->T == b->nseg && b->n_qtiles == b->nseg && !p.cross && !v_in_k && dk == dv && (dk == 64 || dk == 128) && ((uintptr_t)k_pool % 16) == 0 &&
         ((uintptr_t)v_pool % 16) == 0) {
         if (out || out16) {
@@ -661,7 +683,7 @@ static int attention_run(const sllm_seq_batch* b, const float* q, int32_t ldq, i
             p.nsplit = 1;
             *merged = true;
         }
-        return kv_dtype == SLLM_F32 ? attention_decode<float, 4, 2, 2, 4>(p, as_stream(stream)) : attention_decode<uint16_t, 2, 4, 4, 8>(p, as_stream(stream));
+        return attention_decode(p, kv_dtype, as_stream(stream));
     }
     if (b->T == b->nseg && heads / kv_heads <= kBQ) {   // single tokens only: the query heads of a kv head share one CTA and its tiles
         p.by_head = 1;

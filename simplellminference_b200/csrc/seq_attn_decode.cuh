@@ -22,6 +22,7 @@ struct AttnArgs {
     int q_heads, cross;
     int chunk;                // > 0: a query sees its own chunk of `chunk` positions only (then window / keep_first are not used)
     float* out; int ldo; uint16_t* out16;   // one share: the normalised result goes here (fp32 [T][ldo] and / or dense bf16) instead of ws
+    uint32_t page_magic;      // ceil(2^32 / page_len): the page of a position without a division (page_of)
 };
 
 #ifdef __CUDACC__
@@ -32,6 +33,17 @@ __device__ __forceinline__ float seq_score(float dot, float scale, float softcap
     sc -= slope * (float)(qpos - key);
     if (r1 != 0.0f) sc -= r1 * log1pf(r2 * (float)(qpos - key));
     return sc;
+}
+
+// page of a position and its row there: the product with the rounded-up reciprocal is at most one too large
+__device__ __forceinline__ int page_of(int pos, int page_len, uint32_t magic, int& in_page) {
+    int page = (int)__umulhi((uint32_t)pos, magic);
+    in_page = pos - page * page_len;
+    if (in_page < 0) {
+        --page;
+        in_page += page_len;
+    }
+    return page;
 }
 
 // 16 bytes of a cache row as pairs of floats
@@ -48,7 +60,7 @@ __device__ __forceinline__ void cache_pairs(const uint4& u, uint64_t (&p)[2], co
 
 constexpr int kDecodeWarps = 4, kDecodeCluster = 16;     // warps of a CTA, CTAs of a cluster at most
 
-// One query per sequence: G query heads of one kv head against that head's cache rows. Bound: HBM (each row is read once and used G times), so
+// fp32 pools. One query per sequence: G query heads of one kv head against that head's cache rows. Bound: HBM (each row is read once and used G times), so
 // rows go from global memory to registers and nothing is staged: eight lanes share a row (16-byte loads, neighbours next to each other), the four
 // groups of lanes of a warp hold neighbouring rows, kSteps of them in flight per lane, values requested before the scores are worked on. Everything
 // is fp32 (queries as they are, two products per instruction); G x kSteps scores cross the eight lanes in one halving exchange, which leaves
@@ -284,6 +296,258 @@ __global__ void __launch_bounds__(kDecodeWarps * 32) seq_attention_decode_kernel
             if (c == 0) {
                 rec[0] = total[g][0];
                 rec[1] = total[g][1];
+            }
+        }
+    }
+}
+
+// The same step over bf16 pools, on the tensor cores without giving up fp32 working accuracy. The body above spends 1100 instructions per 16 bf16 rows
+// and four query heads (28 % of the issue slots busy with the two warps per scheduler its registers allow: 57 us on eight requests of 77 to
+// 8000 positions); mma.sync does the same in some 460 with the softmax and the loads (40 us; 32 requests of 2048 positions 84 -> 47 us, 5.7 TB/s). Operands: cache rows are bf16 as they are; every query value is the sum of three bf16 terms (24 bits), and
+// the three terms of up to four heads are the 16 rows of the A fragment (row 2h first term, 2h + 1 second, 8 + 2h third), so S costs no more
+// products than one bf16 query would; the softmax weights are split the same way and land in the A fragment of the second product without
+// leaving their lane. Sums: products of bf16 terms are exact, a chain is at most two instructions long (32 products) before it is added to an fp32
+// register with ordinary rounding, because the tensor core's own accumulation truncates. Rows come in runs of 16 through a ring of kRing stages per
+// warp (cp.async, chunks swizzled for ldmatrix), no barrier between warps until the merge, which is that of the register body.
+template <int D>
+struct DecodeTile {
+    static constexpr int kRun = 16, kRing = D == 128 ? 3 : 6;                    // keys of a stage, stages (two CTAs per SM)
+    static constexpr int kStage = 2 * kRun * D;                                 // key rows, then value rows; 16-byte chunk i of row r lies at i ^ (r % 8)
+    static constexpr int kSmem = kDecodeWarps * kRing * kStage * 2;
+};
+
+// v = a + b + c with three bf16 terms
+__device__ __forceinline__ void split3_bf16(float v0, float v1, uint32_t& a, uint32_t& b, uint32_t& c) {
+    a = pack_bf16(v0, v1);
+    const float r0 = v0 - __uint_as_float(a << 16), r1 = v1 - __uint_as_float(a & 0xffff0000u);
+    b = pack_bf16(r0, r1);
+    c = pack_bf16(r0 - __uint_as_float(b << 16), r1 - __uint_as_float(b & 0xffff0000u));
+}
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldmatrix4_trans(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+
+// one k-step of a product from zero
+__device__ __forceinline__ void mma_bf16_zero(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                 : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.0f));
+}
+
+template <int D, bool kOpts>     // kOpts: capped scores or charges on the distance (a window, kept positions and chunks are part of both)
+__global__ void __launch_bounds__(kDecodeWarps * 32, 2) seq_attention_decode_mma_kernel(AttnArgs p, int G) {
+    namespace cg = cooperative_groups;
+    using Tile = DecodeTile<D>;
+    constexpr int kRun = Tile::kRun, kRing = Tile::kRing, kSteps = D / 16, kTiles = D / 8;
+    extern __shared__ __align__(16) uint16_t dsm[];
+    __shared__ __align__(16) float got_o[kDecodeWarps * 4 * D];
+    __shared__ __align__(16) float2 got_ml[kDecodeCluster * kDecodeWarps * 4];
+    __shared__ float weight[kDecodeCluster * kDecodeWarps][4], total[4][2];
+    const sllm_seq_batch& b = p.b;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int CS = (int)cluster.num_blocks(), rank = (int)cluster.block_rank(), split = blockIdx.z / CS;
+    cluster.barrier_arrive();       // waited for before anything is sent: every CTA of the cluster runs by then
+    const int seg = b.qt_seg[blockIdx.x], t = b.seg_start[seg], pos = b.seg_pos0[seg], slot = b.seg_slot[seg];
+    const int group = p.heads / p.kv_heads, subsets = group / G, gkv = blockIdx.y / subsets, h0 = gkv * group + (blockIdx.y % subsets) * G;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3, h = g >> 1;
+    const bool live = h < G, second = g & 1;           // this lane's head exists; it holds the second terms (and no third ones)
+    const int wnd = seq_row_window(pos, p.window, p.chunk);
+    const TileList tiles(pos, pos, wnd, p.keep_first, kBK);
+    const int n_runs = tiles.n * (kBK / kRun), workers = p.nsplit * CS * kDecodeWarps;
+    const int32_t* table = b.block_table + (size_t)slot * b.max_pages;
+    const uint16_t* kp = reinterpret_cast<const uint16_t*>(p.k_pool);
+    const uint16_t* vp = reinterpret_cast<const uint16_t*>(p.v_pool);
+    auto first_key = [&](int run) { return tiles.tile_of(run / (kBK / kRun)) * kBK + run % (kBK / kRun) * kRun; };
+
+    // run -> stage of this warp's ring; rows the sequence does not have yet become zeros (their memory may hold anything)
+    const uint32_t ring = smem_u32(dsm) + warp * (kRing * Tile::kStage * 2);
+    constexpr int kChunks = D / 8, kPer = 32 / kChunks;          // 16-byte chunks of a row, rows one instruction of the warp brings
+    const int lr = lane / kChunks, lc = lane % kChunks;
+    const uint16_t* kl = kp + lc * 8;
+    const uint16_t* vl = vp + lc * 8;
+    auto issue = [&](int run, int stage) {
+        if (run < n_runs) {
+            const int j0 = first_key(run);
+            int in_page;
+            const int page = table[page_of(j0, b.page_len, p.page_magic, in_page)];
+            const size_t row = seq_pool_row(page, p.kv_heads, gkv, b.page_len, in_page + lr, D);
+            const uint16_t *ks = kl + row, *vs = vl + row;
+            const uint32_t dst = ring + (stage * Tile::kStage + lr * D) * 2;
+            const int have = pos - j0 - lr;           // row i * kPer of this lane exists when that is at least i * kPer
+#pragma unroll
+            for (int i = 0; i < kRun / kPer; ++i) {
+                const uint32_t at = dst + i * kPer * D * 2 + ((lc ^ ((lr + i * kPer) & 7)) << 4);
+                const int bytes = have >= i * kPer ? 16 : 0;         // (the rows of a run lie in one page: the address is good either way)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(at), "l"(ks + i * kPer * D), "r"(bytes) : "memory");
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(at + kRun * D * 2), "l"(vs + i * kPer * D), "r"(bytes) : "memory");
+            }
+        }
+        cp_async_commit();
+    };
+    int run = (split * CS + rank) * kDecodeWarps + warp;
+#pragma unroll
+    for (int i = 0; i < kRing - 1; ++i) issue(run + i * workers, i);
+
+    uint32_t qa[kSteps][4];
+    {
+        const float* src = p.q + (size_t)t * p.ldq + (size_t)(h0 + (live ? h : 0)) * D + 2 * c;
+#pragma unroll
+        for (int ks = 0; ks < kSteps; ++ks)
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                uint32_t t1, t2, t3;
+                split3_bf16(src[ks * 16 + half * 8], src[ks * 16 + half * 8 + 1], t1, t2, t3);
+                qa[ks][half * 2] = !live ? 0u : second ? t2 : t1;
+                qa[ks][half * 2 + 1] = !live || second ? 0u : t3;
+            }
+    }
+    const float slope = p.slopes && live ? p.slopes[h0 + h] : 0.0f;
+    const float r1 = p.logdist && live ? p.logdist[h0 + h] : 0.0f, r2 = p.logdist && live ? p.logdist[p.heads + h0 + h] : 0.0f;
+    float m = -INFINITY, l = 0.0f, o[kTiles][2];          // first and third terms' sums together, or the second ones'
+#pragma unroll
+    for (int i = 0; i < kTiles; ++i) o[i][0] = o[i][1] = 0.0f;
+    // ldmatrix rows: keys as they lie (two key tiles x two halves of a k-step), values transposed (two value tiles x two halves of the keys)
+    const uint32_t k_at = (((lane & 7) + (lane & 16 ? 8 : 0)) * D * 2) | (((lane & 8 ? 1 : 0) ^ (lane & 7)) << 4);
+    const uint32_t v_at = ((kRun + (lane & 15)) * D * 2) | (((lane & 16 ? 1 : 0) ^ (lane & 7)) << 4);
+    int stage = 0;
+    for (; run < n_runs; run += workers) {
+        cp_async_wait<kRing - 2>();
+        __syncwarp();
+        const int j0 = first_key(run);
+        const uint32_t base = ring + stage * Tile::kStage * 2;
+        float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+        for (int ks = 0; ks < kSteps; ks += 2) {
+            float part[2][4];
+            uint32_t ka[4], kb[4];
+            ldmatrix4(ka, base + (k_at ^ (ks * 32)));
+            ldmatrix4(kb, base + (k_at ^ ((ks + 1) * 32)));
+            mma_bf16_zero(part[0], qa[ks], ka[0], ka[1]);
+            mma_bf16_zero(part[1], qa[ks], ka[2], ka[3]);
+            mma_bf16_16816(part[0], qa[ks + 1], kb[0], kb[1]);
+            mma_bf16_16816(part[1], qa[ks + 1], kb[2], kb[3]);
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) s[i][e] += part[i][e];
+        }
+        // first + third term here, the second on the neighbouring lane: both then hold the head's scores of keys 2c, 2c + 1 (+ 8)
+        float w[4], mx = -INFINITY;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float mine = s[i >> 1][i & 1] + s[i >> 1][2 + (i & 1)];
+            w[i] = mine + __shfl_xor_sync(0xffffffffu, mine, 4);
+            w[i] = kOpts ? seq_score(w[i], p.scale, p.softcap, slope, r1, r2, pos, j0 + (i >> 1) * 8 + 2 * c + (i & 1)) : w[i] * p.scale;
+        }
+        if (j0 + kRun - 1 > pos || (pos - j0 >= wnd && j0 + kRun > p.keep_first)) {      // some key of the run is hidden
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (!seq_sees(pos, j0 + (i >> 1) * 8 + 2 * c + (i & 1), wnd, p.keep_first)) w[i] = -INFINITY;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) mx = fmaxf(mx, w[i]);
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        const float mn = fmaxf(m, mx);
+        if (__any_sync(0xffffffffu, mn != m)) {
+            const float corr = mn == -INFINITY ? 1.0f : expf(m - mn);
+            l *= corr;
+#pragma unroll
+            for (int i = 0; i < kTiles; ++i)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) o[i][e] *= corr;
+            m = mn;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            w[i] = w[i] == -INFINITY ? 0.0f : expf(w[i] - mn);
+            l += w[i];
+        }
+        uint32_t pa[4];
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            uint32_t t1, t2, t3;
+            split3_bf16(w[half * 2], w[half * 2 + 1], t1, t2, t3);
+            pa[half * 2] = second ? t2 : t1;
+            pa[half * 2 + 1] = second ? 0u : t3;
+        }
+#pragma unroll
+        for (int nt = 0; nt < kTiles; nt += 2) {
+            uint32_t vb[4];
+            ldmatrix4_trans(vb, base + (v_at ^ (nt * 16)));
+            float part[2][4];
+            mma_bf16_zero(part[0], pa, vb[0], vb[1]);
+            mma_bf16_zero(part[1], pa, vb[2], vb[3]);
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) o[nt + i][e] += part[i][e] + part[i][2 + e];
+        }
+        __syncwarp();                       // every lane has read the stage that is filled next
+        issue(run + (kRing - 1) * workers, stage == 0 ? kRing - 1 : stage - 1);
+        stage = stage + 1 == kRing ? 0 : stage + 1;
+    }
+    // The terms' results meet on neighbouring lanes: the lane of the first and third terms keeps the first half of the columns, the other the second.
+    float v[kTiles / 2][2];
+#pragma unroll
+    for (int i = 0; i < kTiles / 2; ++i)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const float lo = o[i][e], hi = o[i + kTiles / 2][e];
+            v[i][e] = (second ? hi : lo) + __shfl_xor_sync(0xffffffffu, second ? lo : hi, 4);
+        }
+    l += __shfl_xor_sync(0xffffffffu, l, 1);
+    l += __shfl_xor_sync(0xffffffffu, l, 2);
+    // every CTA of the cluster gets the sums of its own share of the results, and everybody's maxima
+    const int share = (G * D + 2 * CS - 1) / (2 * CS) * 2, worker = rank * kDecodeWarps + warp, columns = G * D;
+    cluster.barrier_wait();
+    if (live) {
+#pragma unroll
+        for (int i = 0; i < kTiles / 2; ++i) {
+            const int item = h * D + (second ? D / 2 : 0) + i * 8 + 2 * c, to = item / share;
+            *reinterpret_cast<float2*>(cluster.map_shared_rank(got_o, to) + worker * share + item % share) = make_float2(v[i][0], v[i][1]);
+        }
+        if (!second)
+            for (int r = c; r < CS; r += 4) cluster.map_shared_rank(got_ml, r)[worker * 4 + h] = make_float2(m, l);
+    }
+    cluster.sync();
+    if (warp < G) {
+        const int n = CS * kDecodeWarps;
+        float M = -INFINITY, L = 0.0f;
+        for (int i = lane; i < n; i += 32) M = fmaxf(M, got_ml[i * 4 + warp].x);
+        M = warp_max(M);
+        for (int i = lane; i < n; i += 32) {
+            const float2 ml = got_ml[i * 4 + warp];
+            const float f = ml.x == -INFINITY ? 0.0f : expf(ml.x - M);
+            weight[i][warp] = f;
+            L = fmaf(ml.y, f, L);
+        }
+        L = warp_sum(L);
+        if (lane == 0) {
+            total[warp][0] = M;
+            total[warp][1] = L;
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < share; i += kDecodeWarps * 32) {
+        const int item = rank * share + i, hh = item / D, col = item % D;
+        if (item >= columns) break;
+        float acc = 0.0f;
+#pragma unroll 4
+        for (int wkr = 0; wkr < CS * kDecodeWarps; ++wkr) acc = fmaf(got_o[wkr * share + i], weight[wkr][hh], acc);
+        if (p.out || p.out16) {
+            acc *= 1.0f / total[hh][1];
+            if (p.out) p.out[(size_t)t * p.ldo + (size_t)(h0 + hh) * D + col] = acc;
+            if (p.out16) p.out16[((size_t)t * p.heads + h0 + hh) * D + col] = f32_to_bf16_bits(acc);
+        } else {
+            float* rec = p.ws + (((size_t)t * p.heads + h0 + hh) * p.nsplit + split) * (D + 2);
+            rec[2 + col] = acc;
+            if (col == 0) {
+                rec[0] = total[hh][0];
+                rec[1] = total[hh][1];
             }
         }
     }
