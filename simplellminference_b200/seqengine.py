@@ -98,6 +98,13 @@ class Step:
         n = self.engine.ops.chunk_ws_floats(self.b.n_qtiles, heads, dk, dv)
         return self.scratch("chunk_blocks", n) if n else None
 
+    def ssd_block_scratch(self, heads: int, groups: int, n_state: int):
+        """Scratch with which state-space duality walks this step's portions in blocks of tokens on the tensor cores, or None (as ``chunk_scratch``)."""
+        if not self.engine.tensor_cores or self.T - self.nseg + 1 < self.chunk_min_tokens:
+            return None
+        n = self.engine.ops.ssd_block_ws_floats(self.b.n_qtiles, self.nseg, heads, groups, n_state)
+        return self.scratch("ssd_blocks", n) if n else None
+
     def gemm_scratch(self, K: int, N: int):
         """bf16 copy of the activations + the plain product, for products that go to the tensor cores (None: too few rows to pay)."""
         if not self.engine.tensor_cores or self.T < 64:

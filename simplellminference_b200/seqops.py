@@ -227,6 +227,16 @@ class Ops:
         self._ck(self.lib.sllm_seq_ssd_scan(C.byref(b), x_ptr, ldx, B_ptr, ldb, C_ptr, ldc, step_ptr, lda, _p(a_log), _p(dt_bias), _p(skip), heads, groups, n_state,
                                             dv, _p(state), _p(y), ldy, conv_x_ptr, ld_conv, channels, taps, _p(ring), _p(scratch), st))
 
+    def ssd_block_ws_floats(self, n_qtiles, nseg, heads, groups, n_state):
+        """Floats of scratch of ``ssd_blocks``, 0 when these sizes have no block form."""
+        return (self.lib.sllm_seq_ssd_block_ws_bytes(n_qtiles, nseg, heads, groups, n_state) + 3) // 4
+
+    def ssd_blocks(self, b, x_ptr, ldx, B_ptr, ldb, C_ptr, ldc, step_ptr, lda, a_log, dt_bias, skip, heads, groups, n_state, dv, state, y, ldy, conv_x_ptr, ld_conv,
+                   channels, taps, ring, st, block_ws):
+        """``ssd_scan`` in blocks of tokens on the tensor cores."""
+        self._ck(self.lib.sllm_seq_ssd_blocks(C.byref(b), x_ptr, ldx, B_ptr, ldb, C_ptr, ldc, step_ptr, lda, _p(a_log), _p(dt_bias), _p(skip), heads, groups, n_state,
+                                              dv, _p(state), _p(y), ldy, conv_x_ptr, ld_conv, channels, taps, _p(ring), _p(block_ws), st))
+
     def selective_scan(self, b, x_ptr, ldx, step_ptr, lddt, B_ptr, ldb, C_ptr, ldc, z_ptr, ldz, a_log, skip, inner, n_state, state, out, ldo, conv_x_ptr, ld_conv,
                        taps, ring, st, out16=None, scratch=None):
         self._ck(self.lib.sllm_seq_selective_scan(C.byref(b), x_ptr, ldx, step_ptr, lddt, B_ptr, ldb, C_ptr, ldc, z_ptr, ldz, _p(a_log), _p(skip), inner, n_state,
