@@ -53,6 +53,9 @@ int pf_gemm(PfCache* cache, const PfGemmArgs& a, cudaStream_t st);
 // causal attention of T queries at positions pos0.. over cache rows [0, pos0+T): q bf16 [T][q_loc] -> out bf16 [T][q_loc]
 int pf_attention(const uint16_t* q, const void* k_cache, const void* v_cache, int kv_dtype, uint16_t* out, int T, int pos0, int S, int hd,
                  int heads, int kv_heads, cudaStream_t st);
+// the same on tcgen05: bf16 cache, head_dim 64 or 128, 16-byte aligned pointers (prefill_attn_tc.cu)
+int pf_attention_tc(const uint16_t* q, const void* k_cache, const void* v_cache, uint16_t* out, int T, int pos0, int S, int hd, int heads, int kv_heads,
+                    cudaStream_t st);
 // x[t][:] = E[ids[t]][:] from the tiled embedding matrix (emb_kernel.cpp:9-16), fp32
 int pf_embed(const int32_t* ids_dev, const void* emb_tiled, int vocab, int d, float* x, int T, cudaStream_t st);
 // x[t] += add[t] (optional), y[t] = bf16(rmsnorm(x[t]) * w)   (rms_kernel.cpp:12-22)

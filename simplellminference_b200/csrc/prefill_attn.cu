@@ -2,11 +2,11 @@
 // path: embedding gather, RMSNorm with bf16 output).
 //
 // Attention replaces T calls of mha_kernel_cpu (reference source/kernel/cpu/mha_kernel.cpp:36-77): query t at
-// position pos0+t attends to cache rows 0..pos0+t of its KV head. It is ~1 % of the prefill flops (the GEMMs on
-// tcgen05 are the other 99 %), so it uses the warp-level mma.sync.m16n8k16 bf16 path with fp32 online softmax:
+// position pos0+t attends to cache rows 0..pos0+t of its KV head. Warp-level mma.sync.m16n8k16 bf16 with fp32 online softmax:
 // CTA = 64 queries of one head (4 warps x 16 rows), K/V tiles of 64 positions double-buffered in shared memory
 // with cp.async, XOR-swizzled 16-byte chunks (conflict-free ldmatrix), S = QK^T and O += PV with the P fragments
-// taken straight from the S accumulators. Heaviest query tiles are scheduled first (causal imbalance).
+// taken straight from the S accumulators. Heaviest query tiles are scheduled first (causal imbalance). bf16 caches go to the
+// tcgen05 kernel of prefill_attn_tc.cu.
 #include "mega_common.cuh"
 #include "prefill.cuh"
 
@@ -209,6 +209,11 @@ static int attn_launch(const uint16_t* q, const void* kc, const void* vc, uint16
 int pf_attention(const uint16_t* q, const void* kc, const void* vc, int kv_dtype, uint16_t* out, int T, int pos0, int S, int hd, int heads,
                  int kv_heads, cudaStream_t st) {
     SLLM_REQUIRE(q && kc && vc && out && T > 0 && pos0 >= 0 && pos0 + T <= S, SLLM_EINVAL, "pf_attention: bad argument");
+    // bf16 caches: tcgen05. Measured, mma.sync | tcgen05: 2048 queries behind 6144 positions, 32 heads over 8 of 128 1062 | 350 us (687 TFLOP/s); 2048 and 512
+    // queries from position 0, 32 heads 180 | 83 and 23 | 14 us; 64 and 128 queries of 32 and 8 heads 11.5 | 11.8 and 12.0 | 11.9 us. The kernel below keeps fp32
+    // caches, and results that do not start at a multiple of 16 bytes.
+    const bool aligned = (((uintptr_t)q | (uintptr_t)kc | (uintptr_t)vc | (uintptr_t)out) % 16) == 0;
+    if (kv_dtype == SLLM_BF16 && aligned && (hd == 64 || hd == 128)) return pf_attention_tc(q, kc, vc, out, T, pos0, S, hd, heads, kv_heads, st);
     if (hd == 128) return kv_dtype == SLLM_F32 ? attn_launch<128, SLLM_F32>(q, kc, vc, out, T, pos0, S, heads, kv_heads, st)
                                                : attn_launch<128, SLLM_BF16>(q, kc, vc, out, T, pos0, S, heads, kv_heads, st);
     if (hd == 64) return kv_dtype == SLLM_F32 ? attn_launch<64, SLLM_F32>(q, kc, vc, out, T, pos0, S, heads, kv_heads, st)

@@ -1,0 +1,372 @@
+// csrc/prefill_attn_tc.cu — causal attention for a block of T prompt positions on the 5th-generation tensor cores (bf16 cache).
+//
+// Same work as pf_attn_kernel (prefill_attn.cu; reference source/kernel/cpu/mha_kernel.cpp:36-77): query t at position pos0 + t attends to cache rows
+// 0 .. pos0 + t of its kv head; operands bf16, scores, softmax and sums fp32, weights rounded to bf16 for the second product. One CTA per SM, up to TWO
+// tiles of 128 queries that share every key and value tile (two query heads of one kv head at the same positions; without such pairs two
+// neighbouring query tiles of one head): while one tile's softmax runs, the other's products do. Roles:
+//   warp 0 (one lane)   TMA producer: query tiles once, then key and value tiles of 128 positions into rings (128B swizzle; positions beyond the
+//                       prompt lie outside the tensor map and read as zeros);
+//   warp 1 (one lane)   MMA issuer: S = Q K^T (both K-major) into TMEM; O += P V with P read from TMEM, V as the MN-major operand as it lies;
+//   warps 4-7, 8-11     softmax of tile 0 / 1, a thread per query row: tcgen05.ld the scores (once for the maximum, the second half once more for the
+//                       weights), exponentials in powers of two, weights packed as bf16 over the scores' own TMEM columns. O stays in TMEM and is
+//                       rescaled only when a row's maximum has grown by more than 2^8 since its last reference (the weights are relative to that
+//                       reference, so the result is the same), sums in fp32.
+// TMEM: S0 | S1 | O0 | O1, 128 columns each. Bound: the tensor pipe and the exponentials, 1024 clocks each per pair of 128 x 128 tiles at head_dim 128;
+// mma.sync, which it replaces for bf16 caches, spent them one after the other in the same warps. Measured, 2048 queries behind 6144 positions, 32 heads
+// over 8 of 128: 350 us, 687 TFLOP/s (mma.sync 1062 us, 227); 256 CTAs on 148 SMs leave a last wave of 108.
+#include "prefill.cuh"
+#include "tcgen05.cuh"
+
+namespace sllm {
+extern int g_tune_pf_pdl;
+
+constexpr int kTaThreads = 384, kTaTile = 128;      // queries of a tile = keys of a tile
+constexpr uint32_t kTaTmem = 512;
+constexpr unsigned kTaSpin = 1u << 24;              // polls after which a wait gives up (seconds; nothing legitimate waits that long)
+
+template <int HD>
+struct TaShape {
+    static constexpr int kBlocks = HD / 64;                                   // 64-column blocks (128-byte rows) of a tile
+    static constexpr int kBlockBytes = kTaTile * 128, kTileBytes = kBlocks * kBlockBytes;
+    static constexpr int kStages = HD == 128 ? 2 : 4;
+    static constexpr int kSmem = 1024 + (2 + 2 * kStages) * kTileBytes + 512;
+};
+
+struct TaArgs {
+    uint16_t* out;
+    int T, pos0, ldq, heads, group, pair_heads;     // pair_heads: a CTA's two tiles are two heads of a kv head; else two query tiles of one head
+    int tiles, items;                               // query tiles of the prompt; tiles of a CTA (1 or 2)
+    float scale_log2;
+};
+
+__device__ int g_ta_timeout;                        // set when a wait gave up: the results of that launch are not valid
+
+// value operand: [keys][64 columns] blocks of 128-byte rows in the 128B swizzle, read with the columns as the N dimension (MN-major): the next 64
+// columns one block away (leading offset), the next 8 keys 1024 bytes away (stride offset)
+__device__ __forceinline__ uint64_t ta_desc_values(const void* tile, int block_bytes) {
+    uint64_t d = (uint64_t)((s_addr(tile) & 0x3FFFFu) >> 4);
+    d |= (uint64_t)(block_bytes >> 4) << 16;
+    d |= (uint64_t)(1024 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)2 << 61;
+    return d;
+}
+// A from TMEM (bf16 pairs, one column per two elements of K), B from shared memory
+__device__ __forceinline__ void ta_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void ta_st16(uint32_t taddr, const uint32_t* r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};" ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]),
+        "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
+        : "memory");
+}
+__device__ __forceinline__ void ta_st32(uint32_t taddr, const uint32_t* r) {
+    ta_st16(taddr, r);
+    ta_st16(taddr + 16, r + 16);
+}
+__device__ __forceinline__ void ta_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// the loads issued so far have arrived; the registers pass through so that nothing that uses them can be moved in front
+__device__ __forceinline__ void ta_arrived(uint32_t* r) {
+    tc_wait_ld();
+#pragma unroll
+    for (int i = 0; i < 32; ++i) asm volatile("" : "+r"(r[i]));
+}
+__device__ __forceinline__ float ta_exp2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ uint32_t ta_pack(float lo, float hi) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+// bounded wait; false once this CTA has given up
+__device__ __forceinline__ bool ta_wait(uint64_t* bar, uint32_t parity, volatile int* gave_up) {
+    uint32_t done;
+    unsigned spins = 0;
+    while (true) {
+        asm volatile(
+            "{\n.reg .pred p;\n"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+            "selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(done) : "r"(s_addr(bar)), "r"(parity) : "memory");
+        if (done) return true;
+        if ((++spins & 1023) == 0 && *gave_up) return false;
+        if (spins > kTaSpin) {
+            *gave_up = 1;
+            g_ta_timeout = 1;
+            return false;
+        }
+    }
+}
+
+template <int HD>
+__global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                                                                   const __grid_constant__ CUtensorMap tmV, const TaArgs p) {
+    using Sh = TaShape<HD>;
+    constexpr int ST = Sh::kStages;
+    extern __shared__ uint8_t ta_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(ta_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t* sK = smem;
+    uint8_t* sV = sK + ST * Sh::kTileBytes;
+    uint8_t* sQ = sV + ST * Sh::kTileBytes;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sQ + 2 * Sh::kTileBytes);
+    uint64_t *kfull = bars, *kempty = kfull + ST, *vfull = kempty + ST, *vempty = vfull + ST, *qfull = vempty + ST;
+    uint64_t *sfull = qfull + 1, *pready = sfull + 2, *odone = pready + 2;      // per tile: scores written / weights written / product with the values done
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(odone + 2);
+    volatile int* gave_up = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    // this CTA's tiles: (head, first query) and the key tiles each has to see; the longest first
+    const int bx = (int)gridDim.x - 1 - (int)blockIdx.x;
+    int head[2], t0[2], nkt[2], items = p.items;
+    for (int j = 0; j < 2; ++j) {
+        head[j] = p.items == 2 && p.pair_heads ? 2 * (int)blockIdx.y + j : (int)blockIdx.y;
+        const int tile = p.items == 2 && !p.pair_heads ? 2 * bx + j : bx;
+        t0[j] = tile * kTaTile;
+        nkt[j] = (p.pos0 + min(p.T, t0[j] + kTaTile) + kTaTile - 1) / kTaTile;
+        if (j == 1 && (p.items < 2 || tile >= p.tiles)) items = 1;
+    }
+    if (items == 1) nkt[1] = 0;
+    const int kvh = head[0] / p.group, kts = max(nkt[0], nkt[1]);
+
+    if (warp == 0 && lane == 0) {
+        tma_prefetch_desc(&tmQ);
+        tma_prefetch_desc(&tmK);
+        tma_prefetch_desc(&tmV);
+        for (int i = 0; i < ST; ++i) { mb_init(kfull + i, 1); mb_init(kempty + i, 1); mb_init(vfull + i, 1); mb_init(vempty + i, 1); }
+        mb_init(qfull, 1);
+        for (int j = 0; j < 2; ++j) { mb_init(sfull + j, 1); mb_init(pready + j, 128); mb_init(odone + j, 1); }
+        *gave_up = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) tc_alloc(tmem_slot, kTaTmem);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    pdl_wait();
+    pdl_launch_dependents();
+
+    if (warp == 0) {
+        if (lane == 0) {   // ===== TMA producer =====
+            mb_expect(qfull, (uint32_t)(items * Sh::kTileBytes));
+            for (int j = 0; j < items; ++j)
+                for (int c = 0; c < Sh::kBlocks; ++c) tma_load_2d(sQ + j * Sh::kTileBytes + c * Sh::kBlockBytes, &tmQ, head[j] * HD + 64 * c, t0[j], qfull);
+            for (int kt = 0; kt < kts; ++kt) {
+                const int s = kt % ST;
+                const uint32_t ph = (uint32_t)(kt / ST) & 1;
+                if (!ta_wait(kempty + s, ph ^ 1, gave_up)) break;
+                mb_expect(kfull + s, Sh::kTileBytes);
+                for (int c = 0; c < Sh::kBlocks; ++c) tma_load_3d(sK + s * Sh::kTileBytes + c * Sh::kBlockBytes, &tmK, 64 * c, kt * kTaTile, kvh, kfull + s);
+                if (!ta_wait(vempty + s, ph ^ 1, gave_up)) break;
+                mb_expect(vfull + s, Sh::kTileBytes);
+                for (int c = 0; c < Sh::kBlocks; ++c) tma_load_3d(sV + s * Sh::kTileBytes + c * Sh::kBlockBytes, &tmV, 64 * c, kt * kTaTile, kvh, vfull + s);
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {   // ===== MMA issuer =====
+            constexpr uint32_t idesc_s = umma_idesc_bf16(kTaTile, kTaTile), idesc_o = umma_idesc_bf16(kTaTile, HD) | (1u << 16);      // B MN-major
+            auto scores = [&](int j, int kt) {
+                const uint8_t *q = sQ + j * Sh::kTileBytes, *k = sK + (kt % ST) * Sh::kTileBytes;
+#pragma unroll
+                for (int ks = 0; ks < HD / 16; ++ks)
+                    tc_mma_bf16(tmem + 128 * j, umma_desc_sw128(q + (ks / 4) * Sh::kBlockBytes) + (uint64_t)(2 * (ks % 4)),
+                                umma_desc_sw128(k + (ks / 4) * Sh::kBlockBytes) + (uint64_t)(2 * (ks % 4)), idesc_s, ks != 0);
+                tc_commit(sfull + j);
+            };
+            auto values = [&](int j, int kt) {
+                const uint8_t* v = sV + (kt % ST) * Sh::kTileBytes;
+#pragma unroll
+                for (int ks = 0; ks < kTaTile / 16; ++ks)
+                    ta_mma_ts(tmem + 256 + 128 * j, tmem + 128 * j + 8 * ks, ta_desc_values(v + ks * 16 * 128, Sh::kBlockBytes), idesc_o, (kt | ks) != 0);
+                tc_commit(odone + j);
+            };
+            bool ok = ta_wait(qfull, 0, gave_up) && ta_wait(kfull, 0, gave_up);
+            if (ok) {
+                tc_fence_after();
+                for (int j = 0; j < items; ++j) scores(j, 0);
+                tc_commit(kempty);
+            }
+            for (int kt = 0; ok && kt < kts; ++kt) {
+                ok = ta_wait(vfull + kt % ST, (uint32_t)(kt / ST) & 1, gave_up);
+                bool keys = false;
+                for (int j = 0; ok && j < items; ++j) {
+                    if (kt >= nkt[j]) continue;
+                    ok = ta_wait(pready + j, (uint32_t)kt & 1, gave_up);
+                    if (!ok) break;
+                    tc_fence_after();
+                    values(j, kt);
+                    if (kt + 1 >= nkt[j]) continue;
+                    if (!keys) {
+                        ok = ta_wait(kfull + (kt + 1) % ST, (uint32_t)((kt + 1) / ST) & 1, gave_up);
+                        keys = true;
+                    }
+                    // the next scores land where the weights lie that this product is still reading
+                    ok = ok && ta_wait(odone + j, (uint32_t)kt & 1, gave_up);
+                    if (!ok) break;
+                    tc_fence_after();
+                    scores(j, kt + 1);
+                }
+                if (!ok) break;
+                tc_commit(vempty + kt % ST);
+                if (kt + 1 < kts) tc_commit(kempty + (kt + 1) % ST);
+            }
+        }
+    } else if (warp >= 4) {   // ===== softmax: TMEM lane quadrant = warp % 4 =====
+        const int j = (warp - 4) >> 2, quad = warp & 3, row = quad * 32 + lane;
+        if (j < items) {
+            const uint32_t lanes = (uint32_t)(quad * 32) << 16, s_tmem = tmem + lanes + 128 * j, o_tmem = tmem + lanes + 256 + 128 * j;
+            const int t = t0[j] + row, qpos = p.pos0 + t, first_pos = p.pos0 + t0[j] + quad * 32;
+            float ref = -INFINITY, l = 0.0f;            // what the weights are relative to (log2 units); their sum
+            bool ok = true;
+            for (int kt = 0; kt < nkt[j]; ++kt) {
+                ok = ta_wait(sfull + j, (uint32_t)kt & 1, gave_up);
+                if (!ok) break;
+                tc_fence_after();
+                const bool masked = kt * kTaTile + kTaTile - 1 > first_pos;       // some row of this warp does not see every key of the tile
+                const int seen = qpos - kt * kTaTile;                             // columns 0 .. seen are visible to this row
+                uint32_t a[32], b[32];
+                tc_ld32_async(s_tmem + 64, a);
+                tc_ld32_async(s_tmem + 96, b);
+                ta_arrived(a);
+                ta_arrived(b);
+                float m0 = -INFINITY, m1 = -INFINITY;
+                auto top = [&](const uint32_t* v, int c0) {
+#pragma unroll
+                    for (int i = 0; i < 32; i += 2) {
+                        const float x = !masked || c0 + i <= seen ? __uint_as_float(v[i]) : -INFINITY, y = !masked || c0 + i + 1 <= seen ? __uint_as_float(v[i + 1]) : -INFINITY;
+                        m0 = fmaxf(m0, x);
+                        m1 = fmaxf(m1, y);
+                    }
+                };
+                top(a, 64);
+                top(b, 96);
+                tc_ld32_async(s_tmem, a);
+                tc_ld32_async(s_tmem + 32, b);
+                ta_arrived(a);
+                ta_arrived(b);
+                top(a, 0);
+                top(b, 32);
+                const float mx = fmaxf(m0, m1) * p.scale_log2;
+                if (kt == 0) {
+                    ref = mx;
+                } else if (__any_sync(0xffffffffu, mx > ref + 8.0f)) {            // the product before this one has completed: these scores follow it
+                    const float nr = fmaxf(ref, mx), f = ta_exp2(ref - nr);
+                    l *= f;
+                    ref = nr;
+#pragma unroll 1
+                    for (int c = 0; c < HD; c += 32) {
+                        uint32_t o[32];
+                        tc_ld32_async(o_tmem + c, o);
+                        ta_arrived(o);
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f);
+                        ta_st32(o_tmem + c, o);
+                    }
+                }
+                float l0 = 0.0f, l1 = 0.0f;
+                auto weigh = [&](const uint32_t* v, int c0) {                     // 32 scores -> 16 columns of weights
+                    uint32_t w[16];
+#pragma unroll
+                    for (int i = 0; i < 32; i += 2) {
+                        float x = ta_exp2(fmaf(__uint_as_float(v[i]), p.scale_log2, -ref)), y = ta_exp2(fmaf(__uint_as_float(v[i + 1]), p.scale_log2, -ref));
+                        if (masked) {
+                            x = c0 + i <= seen ? x : 0.0f;
+                            y = c0 + i + 1 <= seen ? y : 0.0f;
+                        }
+                        l0 += x;
+                        l1 += y;
+                        w[i / 2] = ta_pack(x, y);
+                    }
+                    ta_st16(s_tmem + c0 / 2, w);
+                };
+                weigh(a, 0);
+                weigh(b, 32);
+                tc_ld32_async(s_tmem + 64, a);
+                tc_ld32_async(s_tmem + 96, b);
+                ta_arrived(a);
+                ta_arrived(b);
+                weigh(a, 64);
+                weigh(b, 96);
+                l += l0 + l1;
+                ta_wait_st();
+                tc_fence_before();
+                mb_arrive(pready + j);
+            }
+            ok = ok && ta_wait(odone + j, (uint32_t)(nkt[j] - 1) & 1, gave_up);
+            tc_fence_after();
+            const float inv = 1.0f / l;
+#pragma unroll 1
+            for (int c = 0; ok && c < HD; c += 32) {
+                uint32_t o[32];
+                tc_ld32_async(o_tmem + c, o);
+                ta_arrived(o);
+                if (t < p.T) {
+                    uint4* dst = reinterpret_cast<uint4*>(p.out + (size_t)t * p.ldq + (size_t)head[j] * HD + c);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        auto two = [&](int e) { return ta_pack(__uint_as_float(o[8 * i + e]) * inv, __uint_as_float(o[8 * i + e + 1]) * inv); };
+                        dst[i] = make_uint4(two(0), two(2), two(4), two(6));
+                    }
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (*gave_up) {        // copies may still be on their way into this CTA's memory: give them time before it is handed on
+        const long long until = clock64() + 4000000;
+        while (clock64() < until) {}
+        __syncthreads();
+    }
+    if (warp == 1) {
+        tc_fence_after();
+        tc_dealloc(tmem, kTaTmem);
+    }
+}
+
+template <int HD>
+static int ta_launch(const uint16_t* q, const void* kc, const void* vc, uint16_t* out, int T, int pos0, int S, int heads, int kv_heads, cudaStream_t st) {
+    using Sh = TaShape<HD>;
+    static bool configured = false;
+    if (!configured) {
+        SLLM_CUDA(cudaFuncSetAttribute(pf_attn_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, Sh::kSmem));
+        configured = true;
+    }
+    CUtensorMap tmQ, tmK, tmV;
+    {
+        const cuuint64_t dims[2] = {(cuuint64_t)heads * HD, (cuuint64_t)T};
+        const cuuint64_t strides[1] = {(cuuint64_t)heads * HD * 2};
+        const cuuint32_t box[2] = {64, kTaTile};
+        if (int rc = tc_encode_bf16(&tmQ, q, 2, dims, strides, box)) return rc;
+    }
+    const cuuint64_t dims[3] = {HD, (cuuint64_t)(pos0 + T), (cuuint64_t)kv_heads};      // positions beyond the prompt read as zeros
+    const cuuint64_t strides[2] = {HD * 2, (cuuint64_t)S * HD * 2};
+    const cuuint32_t box[3] = {64, kTaTile, 1};
+    if (int rc = tc_encode_bf16(&tmK, kc, 3, dims, strides, box)) return rc;
+    if (int rc = tc_encode_bf16(&tmV, vc, 3, dims, strides, box)) return rc;
+    TaArgs a{};
+    a.out = out; a.T = T; a.pos0 = pos0; a.ldq = heads * HD; a.heads = heads; a.group = heads / kv_heads;
+    a.pair_heads = a.group % 2 == 0;
+    a.tiles = (T + kTaTile - 1) / kTaTile;
+    // two tiles per CTA hide each other's softmax and share their loads, unless single ones would still leave SMs idle
+    a.items = (long long)a.tiles * heads > sm_count() ? 2 : 1;
+    a.scale_log2 = (1.0f / sqrtf((float)HD)) * 1.4426950408889634f;
+    const dim3 grid(a.items == 2 && !a.pair_heads ? (a.tiles + 1) / 2 : a.tiles, a.items == 2 && a.pair_heads ? heads / 2 : heads);
+    LaunchCfg lc(grid, dim3(kTaThreads), Sh::kSmem, st, g_tune_pf_pdl != 0);
+    SLLM_CUDA(cudaLaunchKernelEx(&lc.cfg, pf_attn_tc_kernel<HD>, tmQ, tmK, tmV, a));
+    g_launches++;
+    return SLLM_OK;
+}
+
+int pf_attention_tc(const uint16_t* q, const void* kc, const void* vc, uint16_t* out, int T, int pos0, int S, int hd, int heads, int kv_heads, cudaStream_t st) {
+    return hd == 128 ? ta_launch<128>(q, kc, vc, out, T, pos0, S, heads, kv_heads, st) : ta_launch<64>(q, kc, vc, out, T, pos0, S, heads, kv_heads, st);
+}
+
+}  // namespace sllm
