@@ -413,6 +413,13 @@ typedef struct {
     const int32_t* seg_tile0;    /* [nseg] running count of tiles of the segments before this one (tile ids in segment order) */
 } sllm_seq_batch;
 
+/* The index arrays of a step as ONE run of int32 (host arithmetic only): for the nseg segments [slot, first position, tokens, the token before the
+ * first one or -1] and their tokens one behind the other, writes to out, in this order, ids, tok_slot, tok_pos, seg_start, seg_len, seg_slot, seg_pos0,
+ * qt_seg, qt_off (tiles of `tile` queries, the latest first), the n_rows rows (room for one when there are none), the block table of kp, seg_tile0 and
+ * the token before each token. offsets [13]: where each array starts. Returns the length of the run (nothing is written beyond offsets and n_qtiles
+ * when out is NULL or holds less than that), or SLLM_EINVAL. */
+int64_t sllm_seq_step_fill(int32_t* out, int64_t capacity, int32_t nseg, const int32_t* segments, const int32_t* tokens, const int32_t* rows, int32_t n_rows,
+                           const sllm_kvpages* kp, int32_t tile, int64_t* offsets, int32_t* n_qtiles);
 /* out[s][t][:] = table[ids[t]][:] * scale for every stream s (a model with one residual stream passes streams = 1) */
 int sllm_seq_embed(const int32_t* ids, const void* table, int32_t w_dtype, int32_t vocab, int32_t d, int32_t streams, float scale,
                    float* out, int32_t T, sllm_stream_t stream);

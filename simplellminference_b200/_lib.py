@@ -136,6 +136,7 @@ class SeqMoeOpts(C.Structure):
 
 _B = C.POINTER(SeqBatch)
 SIGNATURES.update({
+    "sllm_seq_step_fill": (_L, [_P, _L, _I, _P, _P, _P, _I, _P, _I, _P, _P]),
     "sllm_seq_embed": (C.c_int, [_P, _P, _I, _I, _I, _I, _F, _P, _I, _P]),
     "sllm_seq_hyper_read": (C.c_int, [_P, _I, _I, _I, _P, _P, _I, _F, _P, _P]),
     "sllm_seq_hyper_write": (C.c_int, [_P, _I, _I, _I, _P, _P, _P, _P]),

@@ -13,6 +13,7 @@ with prompts processed in chunks beside the decoding requests and the device sam
 Additive to the reference, which decodes one sequence token by token (source/model/model.cpp:148-185)."""
 from __future__ import annotations
 
+import ctypes as C
 import gc
 import weakref
 
@@ -149,6 +150,8 @@ class SequenceEngine:
         self._meta_dev = None
         self._meta_host = None
         self._meta_event = None
+        self._meta_used = False
+        self._meta_offsets = np.zeros(13, np.int64)
         self.step_obj = Step(self)
         self.steps_run = 0
         # Steps of single tokens (decoding) are launch-bound: their kernel sequence depends only on how many requests step and how many
@@ -202,29 +205,35 @@ class SequenceEngine:
             self._sides[i] = torch.cuda.Stream(self.device)
         return self._sides[i]
 
-    def _upload(self, arrays):
-        """The step's index arrays as ONE host-to-device copy; returns their device addresses."""
-        sizes = [a.size for a in arrays]
-        total = sum(sizes)
+    def _upload(self, segments, tokens, rows):
+        """The step's index arrays (sllm_seq_step_fill) as ONE host-to-device copy; returns their device addresses and the number of query tiles."""
+        fill, n_tiles = self.pages.lib.sllm_seq_step_fill, C.c_int32()
+
+        def run(host):
+            n = fill(host.data_ptr() if host is not None else None, host.numel() if host is not None else 0, len(segments), segments.ctypes.data, tokens.ctypes.data,
+                     rows.ctypes.data if rows.size else None, rows.size, self.pages.h, QUERY_TILE, self._meta_offsets.ctypes.data, C.byref(n_tiles))
+            if n < 0:
+                _lib.check_seq(int(n))
+            return int(n)
+
+        if self._meta_used:
+            self._meta_event.synchronize()          # the previous step's copy has left the pinned buffer
+        total = run(self._meta_host)
         if self._meta_host is None or self._meta_host.numel() < total:
             # sized once for the largest step the pool can hold, so that the addresses captured in graphs stay valid
             cap = max(total, 6 * self.max_len + 16 * self.max_seqs + self.max_seqs * self.max_pages + 64)
             self._graphs = {}
             self._meta_host = torch.empty(cap, dtype=torch.int32).pin_memory() if self.device.type == "cuda" else torch.empty(cap, dtype=torch.int32)
             self._meta_dev = torch.empty(cap, dtype=torch.int32, device=self.device)
-        if self._meta_event is not None:
-            self._meta_event.synchronize()          # the previous step's copy has left the pinned buffer
-        host = self._meta_host.numpy()
-        off, ptrs = 0, []
-        for a, n in zip(arrays, sizes):
-            host[off:off + n] = a.reshape(-1)
-            ptrs.append(self._meta_dev.data_ptr() + 4 * off)
-            off += n
+            run(self._meta_host)
         self._meta_dev[:total].copy_(self._meta_host[:total], non_blocking=True)
         if self.device.type == "cuda":
-            self._meta_event = torch.cuda.Event()
+            if self._meta_event is None:
+                self._meta_event = torch.cuda.Event()
             self._meta_event.record()
-        return ptrs
+            self._meta_used = True
+        base = self._meta_dev.data_ptr()
+        return [base + 4 * o for o in self._meta_offsets.tolist()], n_tiles.value
 
     # ---- the step ----
     def run(self, entries, tap=None):
@@ -244,33 +253,17 @@ class SequenceEngine:
             raise _lib.SllmError(_lib.ENOMEM, f"out of cache pages: this step needs {need} more, {self.pages.free} free")
         for slot, toks, _ in entries:
             self.pages.reserve(slot, self.pos[slot] + toks.size)
-        T = sum(t.size for _, t, _ in entries)
         nseg = len(entries)
-        ids = np.concatenate([t for _, t, _ in entries])
-        prev_ids = np.concatenate([np.concatenate([[self.last_token[s]], t[:-1]]) for s, t, _ in entries]).astype(np.int32)
-        tok_slot = np.concatenate([np.full(t.size, s, dtype=np.int32) for s, t, _ in entries])
-        tok_pos = np.concatenate([np.arange(self.pos[s], self.pos[s] + t.size, dtype=np.int32) for s, t, _ in entries])
-        seg_len = np.array([t.size for _, t, _ in entries], dtype=np.int32)
-        seg_start = np.concatenate([[0], np.cumsum(seg_len)[:-1]]).astype(np.int32)
-        seg_slot = np.array([s for s, _, _ in entries], dtype=np.int32)
-        seg_pos0 = np.array([self.pos[s] for s, _, _ in entries], dtype=np.int32)
-        seg_tile0 = np.concatenate([[0], np.cumsum(-(-seg_len // QUERY_TILE))[:-1]]).astype(np.int32)
-        qt_seg, qt_off = [], []
-        for i, n in enumerate(seg_len):
-            for off in range(0, int(n), QUERY_TILE):
-                qt_seg.append(i)
-                qt_off.append(off)
-        # long tiles first: a tile's work grows with its last position
-        order = sorted(range(len(qt_seg)), key=lambda j: -(int(seg_pos0[qt_seg[j]]) + qt_off[j]))
-        qt_seg = np.array([qt_seg[j] for j in order], dtype=np.int32)
-        qt_off = np.array([qt_off[j] for j in order], dtype=np.int32)
-        rows = np.array([int(seg_start[i]) + int(k) for i, (_, t, w) in enumerate(entries) for k in w], dtype=np.int32)
-        for i, (_, t, w) in enumerate(entries):
+        segments = np.array([(s, self.pos[s], t.size, self.last_token[s]) for s, t, _ in entries], dtype=np.int32)
+        tokens = entries[0][1] if nseg == 1 else np.concatenate([t for _, t, _ in entries])
+        T = tokens.size
+        wanted, start = [], 0
+        for _, t, w in entries:
             if any(k < 0 or k >= t.size for k in w):
                 raise ValueError("a wanted index lies outside the entry's tokens")
-        table = self.pages.table().astype(np.int32)
-        arrays = [ids, tok_slot, tok_pos, seg_start, seg_len, seg_slot, seg_pos0, qt_seg, qt_off, rows if rows.size else np.zeros(1, np.int32), table, seg_tile0, prev_ids]
-        p = self._upload(arrays)
+            wanted += [start + int(k) for k in w]
+            start += t.size
+        p, n_qtiles = self._upload(segments, tokens, np.array(wanted, dtype=np.int32))
         step = self.step_obj
         step.T, step.nseg = T, nseg
         step.turned.clear()
@@ -278,21 +271,21 @@ class SequenceEngine:
         b = step.b
         b.T, b.nseg = T, nseg
         b.tok_slot, b.tok_pos, b.seg_start, b.seg_len, b.seg_slot, b.seg_pos0 = p[1], p[2], p[3], p[4], p[5], p[6]
-        b.qt_seg, b.qt_off, b.n_qtiles = p[7], p[8], int(qt_seg.size)
+        b.qt_seg, b.qt_off, b.n_qtiles = p[7], p[8], n_qtiles
         b.block_table, b.max_pages, b.page_len = p[10], self.max_pages, self.page_len
         b.seg_tile0 = p[11]
         step.prev_ids = _PtrView(p[12])
         ids_t = _PtrView(p[0])
         rows_t = _PtrView(p[9])
-        n_rows = int(rows.size)
+        n_rows = len(wanted)
         decode_only = T == nseg
         if decode_only:
             # a fixed share count per batch size keeps the launch sequence of a decoding step independent of the context lengths
             step.nsplit = max(1, 32 // nseg)
         else:
             # share the key tiles of long contexts among CTAs when the step has few query tiles
-            key_tiles = max(1, -(-int((seg_pos0 + seg_len).max()) // KEY_TILE))
-            step.nsplit = int(min(key_tiles, max(1, 64 // max(1, int(qt_seg.size)))))
+            key_tiles = max(1, -(-max(self.pos[s] + t.size for s, t, _ in entries) // KEY_TILE))
+            step.nsplit = int(min(key_tiles, max(1, 64 // max(1, n_qtiles))))
         key = (nseg, n_rows)
         if decode_only and self.graphs and tap is None and key in self._graphs:
             entry = self._graphs[key]
