@@ -22,7 +22,6 @@ extern int g_tune_pf_pdl;
 
 constexpr int kTaThreads = 384, kTaTile = 128;      // queries of a tile = keys of a tile
 constexpr uint32_t kTaTmem = 512;
-constexpr unsigned kTaSpin = 1u << 24;              // polls after which a wait gives up (seconds; nothing legitimate waits that long)
 
 template <int HD>
 struct TaShape {
@@ -38,72 +37,6 @@ struct TaArgs {
     int tiles, items;                               // query tiles of the prompt; tiles of a CTA (1 or 2)
     float scale_log2;
 };
-
-__device__ int g_ta_timeout;                        // set when a wait gave up: the results of that launch are not valid
-
-// value operand: [keys][64 columns] blocks of 128-byte rows in the 128B swizzle, read with the columns as the N dimension (MN-major): the next 64
-// columns one block away (leading offset), the next 8 keys 1024 bytes away (stride offset)
-__device__ __forceinline__ uint64_t ta_desc_values(const void* tile, int block_bytes) {
-    uint64_t d = (uint64_t)((s_addr(tile) & 0x3FFFFu) >> 4);
-    d |= (uint64_t)(block_bytes >> 4) << 16;
-    d |= (uint64_t)(1024 >> 4) << 32;
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)2 << 61;
-    return d;
-}
-// A from TMEM (bf16 pairs, one column per two elements of K), B from shared memory
-__device__ __forceinline__ void ta_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-__device__ __forceinline__ void ta_st16(uint32_t taddr, const uint32_t* r) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};" ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]),
-        "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
-        : "memory");
-}
-__device__ __forceinline__ void ta_st32(uint32_t taddr, const uint32_t* r) {
-    ta_st16(taddr, r);
-    ta_st16(taddr + 16, r + 16);
-}
-__device__ __forceinline__ void ta_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// the loads issued so far have arrived; the registers pass through so that nothing that uses them can be moved in front
-__device__ __forceinline__ void ta_arrived(uint32_t* r) {
-    tc_wait_ld();
-#pragma unroll
-    for (int i = 0; i < 32; ++i) asm volatile("" : "+r"(r[i]));
-}
-__device__ __forceinline__ float ta_exp2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ uint32_t ta_pack(float lo, float hi) {
-    uint32_t r;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
-    return r;
-}
-// bounded wait; false once this CTA has given up
-__device__ __forceinline__ bool ta_wait(uint64_t* bar, uint32_t parity, volatile int* gave_up) {
-    uint32_t done;
-    unsigned spins = 0;
-    while (true) {
-        asm volatile(
-            "{\n.reg .pred p;\n"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-            "selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(done) : "r"(s_addr(bar)), "r"(parity) : "memory");
-        if (done) return true;
-        if ((++spins & 1023) == 0 && *gave_up) return false;
-        if (spins > kTaSpin) {
-            *gave_up = 1;
-            g_ta_timeout = 1;
-            return false;
-        }
-    }
-}
 
 template <int HD>
 __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -161,10 +94,10 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
             for (int kt = 0; kt < kts; ++kt) {
                 const int s = kt % ST;
                 const uint32_t ph = (uint32_t)(kt / ST) & 1;
-                if (!ta_wait(kempty + s, ph ^ 1, gave_up)) break;
+                if (!tc_wait(kempty + s, ph ^ 1, gave_up)) break;
                 mb_expect(kfull + s, Sh::kTileBytes);
                 for (int c = 0; c < Sh::kBlocks; ++c) tma_load_3d(sK + s * Sh::kTileBytes + c * Sh::kBlockBytes, &tmK, 64 * c, kt * kTaTile, kvh, kfull + s);
-                if (!ta_wait(vempty + s, ph ^ 1, gave_up)) break;
+                if (!tc_wait(vempty + s, ph ^ 1, gave_up)) break;
                 mb_expect(vfull + s, Sh::kTileBytes);
                 for (int c = 0; c < Sh::kBlocks; ++c) tma_load_3d(sV + s * Sh::kTileBytes + c * Sh::kBlockBytes, &tmV, 64 * c, kt * kTaTile, kvh, vfull + s);
             }
@@ -184,31 +117,31 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
                 const uint8_t* v = sV + (kt % ST) * Sh::kTileBytes;
 #pragma unroll
                 for (int ks = 0; ks < kTaTile / 16; ++ks)
-                    ta_mma_ts(tmem + 256 + 128 * j, tmem + 128 * j + 8 * ks, ta_desc_values(v + ks * 16 * 128, Sh::kBlockBytes), idesc_o, (kt | ks) != 0);
+                    tc_mma_bf16_ts(tmem + 256 + 128 * j, tmem + 128 * j + 8 * ks, umma_desc_mn_sw128(v + ks * 16 * 128, Sh::kBlockBytes), idesc_o, (kt | ks) != 0);
                 tc_commit(odone + j);
             };
-            bool ok = ta_wait(qfull, 0, gave_up) && ta_wait(kfull, 0, gave_up);
+            bool ok = tc_wait(qfull, 0, gave_up) && tc_wait(kfull, 0, gave_up);
             if (ok) {
                 tc_fence_after();
                 for (int j = 0; j < items; ++j) scores(j, 0);
                 tc_commit(kempty);
             }
             for (int kt = 0; ok && kt < kts; ++kt) {
-                ok = ta_wait(vfull + kt % ST, (uint32_t)(kt / ST) & 1, gave_up);
+                ok = tc_wait(vfull + kt % ST, (uint32_t)(kt / ST) & 1, gave_up);
                 bool keys = false;
                 for (int j = 0; ok && j < items; ++j) {
                     if (kt >= nkt[j]) continue;
-                    ok = ta_wait(pready + j, (uint32_t)kt & 1, gave_up);
+                    ok = tc_wait(pready + j, (uint32_t)kt & 1, gave_up);
                     if (!ok) break;
                     tc_fence_after();
                     values(j, kt);
                     if (kt + 1 >= nkt[j]) continue;
                     if (!keys) {
-                        ok = ta_wait(kfull + (kt + 1) % ST, (uint32_t)((kt + 1) / ST) & 1, gave_up);
+                        ok = tc_wait(kfull + (kt + 1) % ST, (uint32_t)((kt + 1) / ST) & 1, gave_up);
                         keys = true;
                     }
                     // the next scores land where the weights lie that this product is still reading
-                    ok = ok && ta_wait(odone + j, (uint32_t)kt & 1, gave_up);
+                    ok = ok && tc_wait(odone + j, (uint32_t)kt & 1, gave_up);
                     if (!ok) break;
                     tc_fence_after();
                     scores(j, kt + 1);
@@ -226,7 +159,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
             float ref = -INFINITY, l = 0.0f;            // what the weights are relative to (log2 units); their sum
             bool ok = true;
             for (int kt = 0; kt < nkt[j]; ++kt) {
-                ok = ta_wait(sfull + j, (uint32_t)kt & 1, gave_up);
+                ok = tc_wait(sfull + j, (uint32_t)kt & 1, gave_up);
                 if (!ok) break;
                 tc_fence_after();
                 const bool masked = kt * kTaTile + kTaTile - 1 > first_pos;       // some row of this warp does not see every key of the tile
@@ -234,8 +167,8 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
                 uint32_t a[32], b[32];
                 tc_ld32_async(s_tmem + 64, a);
                 tc_ld32_async(s_tmem + 96, b);
-                ta_arrived(a);
-                ta_arrived(b);
+                tc_arrived(a);
+                tc_arrived(b);
                 float m0 = -INFINITY, m1 = -INFINITY;
                 auto top = [&](const uint32_t* v, int c0) {
 #pragma unroll
@@ -249,25 +182,25 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
                 top(b, 96);
                 tc_ld32_async(s_tmem, a);
                 tc_ld32_async(s_tmem + 32, b);
-                ta_arrived(a);
-                ta_arrived(b);
+                tc_arrived(a);
+                tc_arrived(b);
                 top(a, 0);
                 top(b, 32);
                 const float mx = fmaxf(m0, m1) * p.scale_log2;
                 if (kt == 0) {
                     ref = mx;
                 } else if (__any_sync(0xffffffffu, mx > ref + 8.0f)) {            // the product before this one has completed: these scores follow it
-                    const float nr = fmaxf(ref, mx), f = ta_exp2(ref - nr);
+                    const float nr = fmaxf(ref, mx), f = tc_exp2(ref - nr);
                     l *= f;
                     ref = nr;
 #pragma unroll 1
                     for (int c = 0; c < HD; c += 32) {
                         uint32_t o[32];
                         tc_ld32_async(o_tmem + c, o);
-                        ta_arrived(o);
+                        tc_arrived(o);
 #pragma unroll
                         for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f);
-                        ta_st32(o_tmem + c, o);
+                        tc_st32(o_tmem + c, o);
                     }
                 }
                 float l0 = 0.0f, l1 = 0.0f;
@@ -275,46 +208,47 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
                     uint32_t w[16];
 #pragma unroll
                     for (int i = 0; i < 32; i += 2) {
-                        float x = ta_exp2(fmaf(__uint_as_float(v[i]), p.scale_log2, -ref)), y = ta_exp2(fmaf(__uint_as_float(v[i + 1]), p.scale_log2, -ref));
+                        float x = tc_exp2(fmaf(__uint_as_float(v[i]), p.scale_log2, -ref)), y = tc_exp2(fmaf(__uint_as_float(v[i + 1]), p.scale_log2, -ref));
                         if (masked) {
                             x = c0 + i <= seen ? x : 0.0f;
                             y = c0 + i + 1 <= seen ? y : 0.0f;
                         }
                         l0 += x;
                         l1 += y;
-                        w[i / 2] = ta_pack(x, y);
+                        w[i / 2] = tc_pack(x, y);
                     }
-                    ta_st16(s_tmem + c0 / 2, w);
+                    tc_st16(s_tmem + c0 / 2, w);
                 };
                 weigh(a, 0);
                 weigh(b, 32);
                 tc_ld32_async(s_tmem + 64, a);
                 tc_ld32_async(s_tmem + 96, b);
-                ta_arrived(a);
-                ta_arrived(b);
+                tc_arrived(a);
+                tc_arrived(b);
                 weigh(a, 64);
                 weigh(b, 96);
                 l += l0 + l1;
-                ta_wait_st();
+                tc_wait_st();
                 tc_fence_before();
                 mb_arrive(pready + j);
             }
-            ok = ok && ta_wait(odone + j, (uint32_t)(nkt[j] - 1) & 1, gave_up);
+            ok = ok && tc_wait(odone + j, (uint32_t)(nkt[j] - 1) & 1, gave_up);
             tc_fence_after();
             const float inv = 1.0f / l;
 #pragma unroll 1
             for (int c = 0; ok && c < HD; c += 32) {
                 uint32_t o[32];
                 tc_ld32_async(o_tmem + c, o);
-                ta_arrived(o);
+                tc_arrived(o);
                 if (t < p.T) {
                     uint4* dst = reinterpret_cast<uint4*>(p.out + (size_t)t * p.ldq + (size_t)head[j] * HD + c);
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
-                        auto two = [&](int e) { return ta_pack(__uint_as_float(o[8 * i + e]) * inv, __uint_as_float(o[8 * i + e + 1]) * inv); };
+                        auto two = [&](int e) { return tc_pack(__uint_as_float(o[8 * i + e]) * inv, __uint_as_float(o[8 * i + e + 1]) * inv); };
                         dst[i] = make_uint4(two(0), two(2), two(4), two(6));
                     }
                 }
+                __syncwarp();
             }
         }
     }

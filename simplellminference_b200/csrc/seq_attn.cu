@@ -660,10 +660,19 @@ static int attention_run(const sllm_seq_batch* b, const float* q, int32_t ldq, i
         grid.y = p.heads / hpc;
         const dim3 block(64 * hpc);
         cudaStream_t st = as_stream(stream);
-        if (nsplit == 1 && !p.cross && (out || out16)) {
+        // Heads of 64 or 128 and steps of some size: tcgen05 (seq_attn_tc.cu). Measured, this body | tcgen05 with the merge where there is one, us: prompts of
+        // 1000, 311, 700 and 37 tokens, 16 heads over 4 of 128 170 | 50, capped 218 | 74; one of 4096, 32 heads over 8 2050 | 377; one of 512 51 | 33 (heads of
+        // 64, 32 over 32: 54 | 49); 256 tokens from the start and behind 2000 34 | 31 and 96 | 39 (heads of 64: 32 | 40); 128 and 16 tokens from the
+        // start 15 | 21 and 7.7 | 16 (a fixed part of some 14 us: queries, TMEM, barriers, rows out): below that size this body stays.
+        const bool tc = dk == dv && (dk == 64 || dk == 128) && b->n_qtiles >= (dk == 128 ? 8 : 16) && !p.cross && !v_in_k &&
+                        (((uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)out16) % 16) == 0;
+        // shares are for steps whose query tiles leave SMs idle (the tcgen05 body takes 128 rows of query heads and queries at a time)
+        if (tc && (out || out16) && (long long)b->n_qtiles * kBQ * heads / 128 >= 2LL * sm_count()) p.nsplit = 1;
+        if (p.nsplit == 1 && !p.cross && (out || out16)) {
             p.out = out; p.ldo = ldo; p.out16 = out16;
             *merged = true;
         }
+        if (tc) return launch_attention_tc(p, st);
         if (dk == 128 && dv == 128) seq_attention_mma_kernel<8, 16, true><<<grid, block, smem_mma, st>>>(p);
         else if (dk == 192 && dv == 128) seq_attention_mma_kernel<12, 16, true><<<grid, block, smem_mma, st>>>(p);
         else if (dk == 64 && dv == 64) seq_attention_mma_kernel<4, 8, true><<<grid, block, smem_mma, st>>>(p);

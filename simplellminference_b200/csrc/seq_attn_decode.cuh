@@ -25,6 +25,9 @@ struct AttnArgs {
     uint32_t page_magic;      // ceil(2^32 / page_len): the page of a position without a division (page_of)
 };
 
+// prompt portions over bf16 pools on tcgen05: dk = dv = 64 or 128, pools 16-byte aligned, no values inside keys, no cross values (seq_attn_tc.cu)
+int launch_attention_tc(const AttnArgs& p, cudaStream_t st);
+
 #ifdef __CUDACC__
 
 __device__ __forceinline__ float seq_score(float dot, float scale, float softcap, float slope, float r1, float r2, int qpos, int key) {

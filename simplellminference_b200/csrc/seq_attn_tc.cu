@@ -1,0 +1,366 @@
+// csrc/seq_attn_tc.cu — attention of prompt portions over the paged cache on the 5th-generation tensor cores: bf16 pools, key and value heads of 64 or 128.
+//
+// The tensor-core body of seq_attn.cu keeps a warp's 16 queries in its registers and stages tiles of 32 keys for 64 rows; here 128 rows = the query heads
+// of a kv head (four, two or one) x 32, 64 or 128 neighbouring queries share tiles of 64 keys, and two CTAs per SM hide each other's softmax.
+//   warps 0-3  softmax, a thread per row: q to bf16 rows in shared memory once; per tile the scores from TMEM, capped / charged / masked as the
+//              launch asks, fp32 maximum and sum; the weights go back over the scores' TMEM columns as TWO bf16 terms (p = hi + lo), as in that
+//              body, so that the product with the values keeps them to 2^-17. O stays in TMEM and is rescaled only when a row's maximum has
+//              grown by more than ln 2^8 since its last reference.
+//   warp 4     (one lane) TMA producer: boxes of 32 positions, looked up in the block table; boxes behind the portion's last position lie
+//              outside the tensor map and read as zeros;
+//   warp 5     (one lane) tcgen05.mma issuer: S = Q K^T, O += hi V + lo V with the weights read from TMEM, V MN-major as it lies;
+//   warp 6     zeros the value rows between the last position and the end of its box (the pool may hold anything there).
+// Bound: the fp32 work per score; the tensor pipe needs 768 clocks per 128 x 64 scores at heads of 128. Caps and charges are applied in loops of
+// their own: with tanhf and log1pf inlined 64 times the code left the instruction cache (210 us where the loops take 74). Measured: attention_run.
+#include "seq_attn_decode.cuh"
+#include "tcgen05.cuh"
+
+namespace sllm {
+
+constexpr int kSaRows = 128, kSaKeys = 64, kSaThreads = 256, kSaBox = 32;
+constexpr uint32_t kSaTmem = 256;        // scores / weights at 0, O at 128; two CTAs share an SM's 512 columns
+constexpr float kSaLog2e = 1.4426950408889634f;
+
+// tanh to 5e-7 of its value without a branch: 1 - 2 / (1 + e^2|x|), and below 1/4, where that cancels, the Taylor series to x^9 (remainder 0.0089 x^11)
+__device__ __forceinline__ float sa_tanh(float x) {
+    const float a = fabsf(x), x2 = x * x;
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + tc_exp2(a * (2.0f * kSaLog2e))));
+    const float small = x * fmaf(x2, fmaf(x2, fmaf(x2, fmaf(x2, 62.0f / 2835.0f, -17.0f / 315.0f), 2.0f / 15.0f), -1.0f / 3.0f), 1.0f);
+    return a < 0.25f ? small : copysignf(fmaf(-2.0f, r, 1.0f), x);
+}
+__device__ __forceinline__ float sa_log2(float x) {
+    float y;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+template <int HD>
+struct SaShape {
+    static constexpr int kBlocks = HD / 64, kQBlock = kSaRows * 128, kQBytes = kBlocks * kQBlock, kKBlock = kSaKeys * 128, kTile = kBlocks * kKBlock;
+    static constexpr int kStages = HD == 128 ? 2 : 4;
+    static constexpr int kSmem = 1024 + kQBytes + 2 * kStages * kTile + 512;
+};
+
+struct SaArgs {
+    AttnArgs a;
+    int hpc, hpc_log2, queries;          // query heads and queries of a CTA: hpc * queries = 128
+    int vec_q;
+};
+
+template <int HD, bool kOpts>
+__global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const SaArgs sa) {
+    using Sh = SaShape<HD>;
+    constexpr int ST = Sh::kStages;
+    const AttnArgs& p = sa.a;
+    const sllm_seq_batch& b = p.b;
+    const int seg = b.qt_seg[blockIdx.x], off = b.qt_off[blockIdx.x], split = blockIdx.z;
+    if (off % sa.queries) return;        // the first 32-query tile of a run of `queries` stands for all of it
+    extern __shared__ uint8_t sa_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(sa_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t *sK = smem, *sV = sK + ST * Sh::kTile, *sQ = sV + ST * Sh::kTile;
+    uint64_t* kfull = reinterpret_cast<uint64_t*>(sQ + Sh::kQBytes);
+    uint64_t *kempty = kfull + ST, *vfull = kempty + ST, *vready = vfull + ST, *vempty = vready + ST, *qready = vempty + ST, *sfull = qready + 1, *pready = sfull + 1, *odone = pready + 1;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(odone + 1);
+    volatile int* gave_up = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nq = min(sa.queries, b.seg_len[seg] - off), tok0 = b.seg_start[seg] + off, pos0 = b.seg_pos0[seg] + off, slot = b.seg_slot[seg];
+    const int group = p.heads / p.kv_heads, sets = group / sa.hpc, gkv = blockIdx.y / sets, h0 = gkv * group + (blockIdx.y % sets) * sa.hpc;
+    const int last_pos = pos0 + nq - 1;
+    const TileList tiles(pos0, last_pos, seq_row_window(pos0, p.window, p.chunk), p.keep_first, kSaKeys);
+    const int n = tiles.n > split ? (tiles.n - split + p.nsplit - 1) / p.nsplit : 0;      // this share's tiles: split, split + nsplit, ...
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < ST; ++i) { mb_init(kfull + i, 1); mb_init(kempty + i, 1); mb_init(vfull + i, 1); mb_init(vready + i, 1); mb_init(vempty + i, 1); }
+        mb_init(qready, 128); mb_init(sfull, 1); mb_init(pready, 128); mb_init(odone, 1);
+        *gave_up = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 5) tc_alloc(tmem_slot, kSaTmem);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    const int32_t* table = b.block_table + (size_t)slot * b.max_pages;
+
+    if (warp == 4) {
+        if (lane == 0) {   // ===== TMA producer =====
+            for (int i = 0; i < n; ++i) {
+                const int s = i % ST, j0 = tiles.tile_of(split + i * p.nsplit) * kSaKeys;
+                const uint32_t ph = (uint32_t)(i / ST) & 1;
+                int at[2], row[2];
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    const int pos = j0 + x * kSaBox;
+                    int in_page;
+                    const int idx = page_of(pos, b.page_len, p.page_magic, in_page);
+                    at[x] = pos <= last_pos ? in_page : b.page_len;                           // behind the last position: outside the map, zeros
+                    row[x] = pos <= last_pos ? table[idx] * p.kv_heads + gkv : 0;
+                }
+                if (!tc_wait(kempty + s, ph ^ 1, gave_up)) break;
+                mb_expect(kfull + s, Sh::kTile);
+#pragma unroll
+                for (int x = 0; x < 2; ++x)
+                    for (int c = 0; c < Sh::kBlocks; ++c) tma_load_3d(sK + s * Sh::kTile + c * Sh::kKBlock + x * kSaBox * 128, &tmK, 64 * c, at[x], row[x], kfull + s);
+                if (!tc_wait(vempty + s, ph ^ 1, gave_up)) break;
+                mb_expect(vfull + s, Sh::kTile);
+#pragma unroll
+                for (int x = 0; x < 2; ++x)
+                    for (int c = 0; c < Sh::kBlocks; ++c) tma_load_3d(sV + s * Sh::kTile + c * Sh::kKBlock + x * kSaBox * 128, &tmV, 64 * c, at[x], row[x], vfull + s);
+            }
+        }
+    } else if (warp == 5) {
+        if (lane == 0) {   // ===== MMA issuer =====
+            constexpr uint32_t idesc_s = umma_idesc_bf16(kSaRows, kSaKeys), idesc_o = umma_idesc_bf16(kSaRows, HD) | (1u << 16);      // B MN-major
+            auto scores = [&](int i) {
+                const uint8_t* k = sK + (i % ST) * Sh::kTile;
+#pragma unroll
+                for (int ks = 0; ks < HD / 16; ++ks)
+                    tc_mma_bf16(tmem, umma_desc_sw128(sQ + (ks / 4) * Sh::kQBlock) + (uint64_t)(2 * (ks % 4)), umma_desc_sw128(k + (ks / 4) * Sh::kKBlock) + (uint64_t)(2 * (ks % 4)),
+                                idesc_s, ks != 0);
+                tc_commit(sfull);
+                tc_commit(kempty + i % ST);
+            };
+            bool ok = n > 0 && tc_wait(qready, 0, gave_up) && tc_wait(kfull, 0, gave_up);
+            if (ok) {
+                tc_fence_after();
+                scores(0);
+            }
+            for (int i = 0; ok && i < n; ++i) {
+                ok = tc_wait(vready + i % ST, (uint32_t)(i / ST) & 1, gave_up) && tc_wait(pready, (uint32_t)i & 1, gave_up);
+                if (!ok) break;
+                tc_fence_after();
+                const uint8_t* v = sV + (i % ST) * Sh::kTile;
+#pragma unroll
+                for (int ks = 0; ks < 2 * kSaKeys / 16; ++ks)                    // first terms, then second ones, against the same values
+                    tc_mma_bf16_ts(tmem + 128, tmem + 8 * ks, umma_desc_mn_sw128(v + (ks % (kSaKeys / 16)) * 16 * 128, Sh::kKBlock), idesc_o, (i | ks) != 0);
+                tc_commit(odone);
+                tc_commit(vempty + i % ST);
+                if (i + 1 < n) {        // the next scores land where the weights lie that this product is still reading
+                    ok = tc_wait(kfull + (i + 1) % ST, (uint32_t)((i + 1) / ST) & 1, gave_up) && tc_wait(odone, (uint32_t)i & 1, gave_up);
+                    if (!ok) break;
+                    tc_fence_after();
+                    scores(i + 1);
+                }
+            }
+        }
+    } else if (warp == 6) {   // ===== value rows that the sequence does not have yet =====
+        for (int i = 0; i < n; ++i) {
+            const int s = i % ST, have = last_pos + 1 - tiles.tile_of(split + i * p.nsplit) * kSaKeys;
+            if (!tc_wait(vfull + s, (uint32_t)(i / ST) & 1, gave_up)) break;
+            if (have < kSaKeys) {
+                for (int x = lane; x < (kSaKeys - have) * 8 * Sh::kBlocks; x += 32) {
+                    const int c = x / ((kSaKeys - have) * 8), y = x % ((kSaKeys - have) * 8);
+                    *reinterpret_cast<uint4*>(sV + s * Sh::kTile + c * Sh::kKBlock + (have + y / 8) * 128 + (y % 8) * 16) = make_uint4(0u, 0u, 0u, 0u);
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            }
+            __syncwarp();
+            if (lane == 0) mb_arrive(vready + s);
+        }
+    } else if (warp < 4) {   // ===== softmax: row = warp * 32 + lane = query * hpc + head =====
+        const int row = threadIdx.x, qi = row >> sa.hpc_log2, h = h0 + (row & (sa.hpc - 1));
+        const bool live = qi < nq;
+        const int qpos = pos0 + qi;
+        {   // the warp's 32 rows, one row (or two) per load so that neighbouring lanes read neighbouring columns
+            constexpr int kLanes = HD / 4, kPer = 32 / kLanes;                  // lanes of a row, rows of a load
+#pragma unroll 16
+            for (int r0 = 0; r0 < 32; r0 += kPer) {
+                const int r = warp * 32 + r0 + lane / kLanes, col = (lane % kLanes) * 4;
+                const float* src = p.q + (size_t)(tok0 + min(r >> sa.hpc_log2, nq - 1)) * p.ldq + (size_t)(h0 + (r & (sa.hpc - 1))) * HD + col;
+                const float4 x = sa.vec_q ? *reinterpret_cast<const float4*>(src) : make_float4(src[0], src[1], src[2], src[3]);
+                *reinterpret_cast<uint2*>(sQ + (col / 64) * Sh::kQBlock + r * 128 + ((((col % 64) / 8) ^ (r & 7)) << 4) + (col % 8) * 2) =
+                    make_uint2(tc_pack(x.x, x.y), tc_pack(x.z, x.w));
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            mb_arrive(qready);
+        }
+        const uint32_t s_tmem = tmem + ((uint32_t)(warp * 32) << 16), o_tmem = s_tmem + 128;
+        const int wnd = seq_row_window(qpos, p.window, p.chunk);
+        const float slope = kOpts && p.slopes ? p.slopes[h] : 0.0f, r1 = kOpts && p.logdist ? p.logdist[h] : 0.0f, r2 = kOpts && p.logdist ? p.logdist[p.heads + h] : 0.0f;
+        float ref = -INFINITY, l = 0.0f;            // what the weights are relative to; their sum
+        bool ok = true;
+        for (int i = 0; i < n; ++i) {
+            const int j0 = tiles.tile_of(split + i * p.nsplit) * kSaKeys;
+            ok = tc_wait(sfull, (uint32_t)i & 1, gave_up);
+            if (!ok) break;
+            tc_fence_after();
+            uint32_t s[64];
+            tc_ld32_async(s_tmem, s);
+            tc_ld32_async(s_tmem + 32, s + 32);
+            tc_arrived(s);
+            tc_arrived(s + 32);
+            // every key of the tile is visible to every row of the warp
+            const bool all = __all_sync(0xffffffffu, j0 + kSaKeys - 1 <= qpos && (qpos - j0 < wnd || j0 + kSaKeys <= p.keep_first));
+            if (kOpts && p.softcap > 0.0f) {
+                const float inv = p.scale / p.softcap;
+#pragma unroll
+                for (int e = 0; e < 64; ++e) s[e] = __float_as_uint(p.softcap * sa_tanh(__uint_as_float(s[e]) * inv));
+            } else {
+#pragma unroll
+                for (int e = 0; e < 64; ++e) s[e] = __float_as_uint(__uint_as_float(s[e]) * p.scale);
+            }
+            if (kOpts && p.slopes) {
+                const float d0 = (float)(qpos - j0);
+#pragma unroll
+                for (int e = 0; e < 64; ++e) s[e] = __float_as_uint(fmaf(-slope, d0 - (float)e, __uint_as_float(s[e])));
+            }
+            if (kOpts && p.logdist) {
+                const float d0 = (float)(qpos - j0), r1l = r1 * 0.6931471805599453f;
+#pragma unroll
+                for (int e = 0; e < 64; ++e) s[e] = __float_as_uint(fmaf(-r1l, sa_log2(fmaf(r2, fmaxf(d0 - (float)e, 0.0f), 1.0f)), __uint_as_float(s[e])));
+            }
+            if (!all) {
+#pragma unroll
+                for (int e = 0; e < 64; ++e)
+                    if (!seq_sees(qpos, j0 + e, wnd, p.keep_first)) s[e] = 0xff800000u;       // -inf
+            }
+            float m0 = -INFINITY, m1 = -INFINITY;
+#pragma unroll
+            for (int e = 0; e < 64; e += 2) {
+                m0 = fmaxf(m0, __uint_as_float(s[e]));
+                m1 = fmaxf(m1, __uint_as_float(s[e + 1]));
+            }
+            const float mx = fmaxf(m0, m1);
+            if (i == 0) {
+                ref = mx;
+            } else if (__any_sync(0xffffffffu, mx > ref + 5.5f)) {              // the product before this one has completed: these scores follow it
+                const float nr = fmaxf(ref, mx), f = nr == -INFINITY ? 1.0f : tc_exp2((ref - nr) * kSaLog2e);
+                l *= f;
+                ref = nr;
+#pragma unroll 1
+                for (int c = 0; c < HD; c += 16) {
+                    uint32_t o[16];
+                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                                 : "=r"(o[0]), "=r"(o[1]), "=r"(o[2]), "=r"(o[3]), "=r"(o[4]), "=r"(o[5]), "=r"(o[6]), "=r"(o[7]), "=r"(o[8]), "=r"(o[9]), "=r"(o[10]), "=r"(o[11]),
+                                   "=r"(o[12]), "=r"(o[13]), "=r"(o[14]), "=r"(o[15])
+                                 : "r"(o_tmem + c)
+                                 : "memory");
+                    tc_wait_ld();
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) asm volatile("" : "+r"(o[e]));
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * f);
+                    tc_st16(o_tmem + c, o);
+                }
+            }
+            float l0 = 0.0f, l1 = 0.0f;
+            const float from = ref == -INFINITY ? 0.0f : ref;                   // nothing seen yet: every weight is exp(-inf) = 0
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                uint32_t hi[16], lo[16];
+#pragma unroll
+                for (int e = 0; e < 16; ++e) {
+                    const float x = tc_exp2((__uint_as_float(s[half * 32 + 2 * e]) - from) * kSaLog2e), y = tc_exp2((__uint_as_float(s[half * 32 + 2 * e + 1]) - from) * kSaLog2e);
+                    l0 += x;
+                    l1 += y;
+                    hi[e] = tc_pack(x, y);
+                    lo[e] = tc_pack(x - __uint_as_float(hi[e] << 16), y - __uint_as_float(hi[e] & 0xffff0000u));
+                }
+                tc_st16(s_tmem + half * 16, hi);
+                tc_st16(s_tmem + 32 + half * 16, lo);
+            }
+            l += l0 + l1;
+            tc_wait_st();
+            tc_fence_before();
+            mb_arrive(pready);
+        }
+        if (ok && n > 0) ok = tc_wait(odone, (uint32_t)(n - 1) & 1, gave_up);
+        tc_fence_after();
+        const bool direct = p.out || p.out16;
+        const float inv = direct ? 1.0f / l : 1.0f;
+        const int t = tok0 + qi;
+        float* rec = direct ? nullptr : p.ws + (((size_t)t * p.heads + h) * p.nsplit + split) * (HD + 2);
+        if (ok && live && !direct) {
+            rec[0] = ref;
+            rec[1] = l;
+        }
+        // fp32 results: where this lane's column of the first row goes, and how far the next query and the next head are
+        float* to = lane + (p.out ? p.out + (size_t)tok0 * p.ldo + (size_t)h0 * HD : p.ws + (((size_t)tok0 * p.heads + h0) * p.nsplit + split) * (HD + 2) + 2);
+        const int step_h = p.out ? HD : p.nsplit * (HD + 2), step_q = p.out ? p.ldo : p.heads * step_h;
+#pragma unroll 1
+        for (int c = 0; ok && c < HD; c += 32) {
+            uint32_t o[32];
+            if (n > 0) {
+                tc_ld32_async(o_tmem + c, o);
+                tc_arrived(o);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 32; ++e) o[e] = 0u;
+            }
+#pragma unroll
+            for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * inv);
+            if (live && p.out16) {
+                uint4* dst = reinterpret_cast<uint4*>(p.out16 + ((size_t)t * p.heads + h) * HD + c);
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    auto two = [&](int e) { return tc_pack(__uint_as_float(o[8 * x + e]), __uint_as_float(o[8 * x + e + 1])); };
+                    dst[x] = make_uint4(two(0), two(2), two(4), two(6));
+                }
+            }
+            if (p.out || !direct) {     // fp32 rows: through shared memory (the rings' place, every tile has been read), so that a store covers neighbouring columns of one row
+                float* mine = reinterpret_cast<float*>(smem) + warp * (32 * 33);
+                __syncwarp();
+#pragma unroll
+                for (int e = 0; e < 32; ++e) mine[lane * 33 + e] = __uint_as_float(o[e]);
+                __syncwarp();
+                const int rows = min(32, (nq << sa.hpc_log2) - warp * 32);
+#pragma unroll 8
+                for (int r = 0; r < 32; ++r)
+                    if (r < rows) {
+                        const int rr = warp * 32 + r;
+                        to[(size_t)(uint32_t)((rr >> sa.hpc_log2) * step_q + (rr & (sa.hpc - 1)) * step_h + c)] = mine[r * 33 + lane];
+                    }
+            }
+            __syncwarp();
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (*gave_up) {        // copies may still be on their way into this CTA's memory: give them time before it is handed on
+        const long long until = clock64() + 4000000;
+        while (clock64() < until) {}
+        __syncthreads();
+    }
+    if (warp == 5) {
+        tc_fence_after();
+        tc_dealloc(tmem, kSaTmem);
+    }
+}
+
+template <int HD, bool kOpts>
+static int sa_launch(const AttnArgs& p, cudaStream_t st) {
+    using Sh = SaShape<HD>;
+    auto* kernel = seq_attention_tc_kernel<HD, kOpts>;
+    static bool configured = false;
+    if (!configured) {
+        SLLM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Sh::kSmem));
+        configured = true;
+    }
+    SaArgs a{};
+    a.a = p;
+    const int group = p.heads / p.kv_heads;
+    a.hpc = group % 4 == 0 ? 4 : group % 2 == 0 ? 2 : 1;
+    a.hpc_log2 = a.hpc / 2;
+    a.queries = kSaRows / a.hpc;
+    a.vec_q = p.ldq % 4 == 0 && ((uintptr_t)p.q % 16) == 0;
+    // a pool [pages][kv_heads][page_len][HD]: how many pages it has is the caller's knowledge, the block table names existing ones only
+    CUtensorMap tmK, tmV;
+    const cuuint64_t dims[3] = {HD, (cuuint64_t)p.b.page_len, (cuuint64_t)1 << 31};
+    const cuuint64_t strides[2] = {HD * 2, (cuuint64_t)p.b.page_len * HD * 2};
+    const cuuint32_t box[3] = {64, kSaBox, 1};
+    if (int rc = tc_encode_bf16(&tmK, p.k_pool, 3, dims, strides, box)) return rc;
+    if (int rc = tc_encode_bf16(&tmV, p.v_pool, 3, dims, strides, box)) return rc;
+    kernel<<<dim3(p.b.n_qtiles, p.heads / a.hpc, p.nsplit), kSaThreads, Sh::kSmem, st>>>(tmK, tmV, a);
+    ++g_launches;
+    SLLM_LAUNCH_CHECK();
+    return SLLM_OK;
+}
+
+int launch_attention_tc(const AttnArgs& p, cudaStream_t st) {
+    const bool opts = p.softcap > 0.0f || p.slopes || p.logdist;
+    if (p.dk == 128) return opts ? sa_launch<128, true>(p, st) : sa_launch<128, false>(p, st);
+    return opts ? sa_launch<64, true>(p, st) : sa_launch<64, false>(p, st);
+}
+
+}  // namespace sllm

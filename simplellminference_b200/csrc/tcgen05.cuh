@@ -75,6 +75,70 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
+// value operand: [keys][64 columns] blocks of 128-byte rows in the 128B swizzle, read with the columns as the N dimension (MN-major): the next 64
+// columns one block away (leading offset), the next 8 keys 1024 bytes away (stride offset)
+__device__ __forceinline__ uint64_t umma_desc_mn_sw128(const void* tile, int block_bytes) {
+    uint64_t d = (uint64_t)((s_addr(tile) & 0x3FFFFu) >> 4);
+    d |= (uint64_t)(block_bytes >> 4) << 16;
+    d |= (uint64_t)(1024 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)2 << 61;
+    return d;
+}
+// A from TMEM (bf16 pairs, one column per two elements of K), B from shared memory
+__device__ __forceinline__ void tc_mma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t* r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};" ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]),
+        "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
+        : "memory");
+}
+__device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t* r) {
+    tc_st16(taddr, r);
+    tc_st16(taddr + 16, r + 16);
+}
+__device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// the loads issued so far have arrived; the registers pass through so that nothing that uses them can be moved in front
+__device__ __forceinline__ void tc_arrived(uint32_t* r) {
+    tc_wait_ld();
+#pragma unroll
+    for (int i = 0; i < 32; ++i) asm volatile("" : "+r"(r[i]));
+}
+__device__ __forceinline__ float tc_exp2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ uint32_t tc_pack(float lo, float hi) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+// Bounded wait on a barrier; false once some thread of this CTA has given up (a flag in shared memory): the kernel then tears down without its result
+constexpr unsigned kTcSpin = 1u << 24;              // polls, seconds: nothing legitimate waits that long
+__device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile int* gave_up) {
+    uint32_t done;
+    unsigned spins = 0;
+    while (true) {
+        asm volatile(
+            "{\n.reg .pred p;\n"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+            "selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(done) : "r"(s_addr(bar)), "r"(parity) : "memory");
+        if (done) return true;
+        if ((++spins & 1023) == 0 && *gave_up) return false;
+        if (spins > kTcSpin) {
+            *gave_up = 1;
+            return false;
+        }
+    }
+}
+
 #endif
 
 }  // namespace sllm
