@@ -376,12 +376,24 @@ __global__ void __launch_bounds__(256) seq_linear_tile_kernel(LinArgs p) {
     }
 }
 
-// A (fp32, row stride lda) -> bf16 [T][K] dense
-__global__ void seq_to_bf16_kernel(const float* __restrict__ A, int lda, uint16_t* __restrict__ out, int T, int K) {
-    const size_t n = (size_t)T * K;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t t = i / K, k = i % K;
-        out[i] = f32_to_bf16_bits(A[t * lda + k]);
+// A (fp32, row stride lda) -> bf16 [T][K] dense, K a multiple of 8: eight values per thread, 16-byte accesses where A allows them. Bound: HBM. Element by
+// element, with a 64-bit division each, 2048 x 2048 took 13.1 us; 5 us like this.
+__global__ void __launch_bounds__(256) seq_to_bf16_kernel(const float* __restrict__ A, int lda, uint16_t* __restrict__ out, int T, int K, int vec) {
+    const int per_row = K / 8;
+    const long long n = (long long)T * per_row, stride = (long long)gridDim.x * blockDim.x;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+        const int t = (int)(i / per_row), c = (int)(i - (long long)t * per_row) * 8;
+        const float* src = A + (size_t)t * lda + c;
+        float4 x, y;
+        if (vec) {
+            x = *reinterpret_cast<const float4*>(src);
+            y = *reinterpret_cast<const float4*>(src + 4);
+        } else {
+            x = make_float4(src[0], src[1], src[2], src[3]);
+            y = make_float4(src[4], src[5], src[6], src[7]);
+        }
+        auto two = [](float lo, float hi) { return (uint32_t)f32_to_bf16_bits(lo) | ((uint32_t)f32_to_bf16_bits(hi) << 16); };
+        *reinterpret_cast<uint4*>(out + (size_t)i * 8) = make_uint4(two(x.x, x.y), two(x.z, x.w), two(y.x, y.y), two(y.z, y.w));
     }
 }
 
@@ -475,11 +487,12 @@ extern "C" int sllm_seq_linear(const float* A, int32_t lda, const void* W, int32
     LinArgs p{A, W, bias, C, lda, ldw, ldc, T, N, K, w_dtype, accumulate, round_a, alpha, a_bs, w_bs, bias_bs, c_bs, rows_dev, nullptr, 0, 0};
     if (T <= kRowsMax) return launch_rows(p, batch, st);
     // tensor cores: bf16 weights, a dense bf16 copy of A, rows that TMA can address (16-byte multiples) and enough work to fill tiles
-    if (a16 && sllm_seq_linear_on_tensor_cores(T, N, K, w_dtype, ldw, batch, round_a) && ((uintptr_t)W % 16) == 0) {
+    if (a16 && sllm_seq_linear_on_tensor_cores(T, N, K, w_dtype, ldw, batch, round_a) && (((uintptr_t)W | (uintptr_t)a16) % 16) == 0) {
         static PfCache* cache = pf_cache_create();
         if (!a16_ready) {   // else the kernel that produced A has left its bf16 rows in a16 already
-            const size_t n = (size_t)T * K;
-            seq_to_bf16_kernel<<<(int)std::min<size_t>((n + 255) / 256, (size_t)sm_count() * 8), 256, 0, st>>>(A, lda, reinterpret_cast<uint16_t*>(a16), T, K);
+            const size_t n = (size_t)T * K / 8;
+            const int vec = lda % 4 == 0 && ((uintptr_t)A % 16) == 0;
+            seq_to_bf16_kernel<<<(int)std::min<size_t>((n + 255) / 256, (size_t)sm_count() * 8), 256, 0, st>>>(A, lda, reinterpret_cast<uint16_t*>(a16), T, K, vec);
             ++g_launches;
             SLLM_LAUNCH_CHECK();
         }
