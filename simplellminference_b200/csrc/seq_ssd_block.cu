@@ -3,20 +3,21 @@
 //     y_i = e^G_i S0^T C_i + sum_{j<=i} (C_i . B_j) e^(G_i - G_j) dt_j x_j + D x_i,        S' = e^G_n S0 + sum_j e^(G_n - G_j) dt_j B_j x_j^T
 // (1) seq_ssd_prepare_kernel: what does not depend on the state, all blocks in parallel. B and C belong to a group of heads, so their tensor-core fragments
 // and the products C_i . B_j (fp32) are made once per (block, group); step sizes and G once per (block, head).
-// (2) seq_ssd_walk_kernel, CTA = (portion, head, 32 columns), 8 warps: S^T stays in the accumulators (fp32) from the portion's first token to its last,
-// a warp owning 16 columns x a quarter of the states; it is handed to the others as A fragments through shared memory once per block. Everything is
+// (2) seq_ssd_walk_kernel, CTA = (portion, head, 32 columns), 16 warps: S^T stays in the accumulators (fp32) from the portion's first token to its last,
+// a warp owning 16 columns x an eighth of the states (and of the tokens); it is handed to the others as A fragments through shared memory once per block. Everything is
 // computed transposed (columns are rows), so that accumulators become operands register for register. Every operand is two bf16 terms (x = hi + lo,
 // error <= 2^-17), three products with fp32 accumulation, as in the block form of the delta rule; decays are applied in fp32 to accumulators, to x
 // before it is split and to the C_i . B_j, never to the shared fragments. No factor exceeds 1.
 // Bound: 888 mma per block and CTA (1800 clocks of an SM's tensor pipe) beside 90 KB of fragments from L2; the token-by-token passes over
 // ranges it replaces for portions were bound by fp32 FMAs through shared memory. Measured, 2048 tokens, 64 heads of 64 columns, 128 states: ranges
-// 712 us (249 + 14 + 450), blocks 156 us (18 + 138: a block of the walk takes 4.3 us, two barriers and the latency of its products).
+// 712 us (249 + 14 + 450), blocks 143 us (18 + 125: a block of the walk takes 3.9 us, some 600 instructions per warp at four warps per scheduler and
+// two barriers; 8 warps of twice the work 137).
 #include "seq_attn.cuh"
 #include "seq_ssd_block.cuh"
 
 namespace sllm {
 
-constexpr int kSsdCols = 32, kSsdThreads = 256;
+constexpr int kSsdCols = 32, kSsdThreads = 256, kSsdWalk = 512;      // columns of a walk's CTA, threads of the preparation, of the walk
 constexpr float kSsdLog2e = 1.4426950408889634f;
 constexpr int kSsdLdx = kSsdCols + 4;                         // padded row of x in shared memory
 
@@ -141,9 +142,9 @@ __device__ __forceinline__ void ssd_load(uint32_t (&r)[4], const uint4* at) {
 }
 
 template <int NK>
-__global__ void __launch_bounds__(kSsdThreads, 1) seq_ssd_walk_kernel(SsdBlockArgs p, int vec) {
+__global__ void __launch_bounds__(kSsdWalk, 1) seq_ssd_walk_kernel(SsdBlockArgs p, int vec) {
     using Group = SsdGroup<NK>;
-    constexpr int kX = kSsdBlock * kSsdLdx * 4, kHead = 3 * kSsdBlock * 4, kStage = Group::kBytes + kX + kHead, kSteps = NK / 16, kQuarter = NK / 4, kTiles = kQuarter / 8;
+    constexpr int kX = kSsdBlock * kSsdLdx * 4, kHead = 3 * kSsdBlock * 4, kStage = Group::kBytes + kX + kHead, kSteps = NK / 16, kEighth = NK / 8, kTiles = kEighth / 8;
     extern __shared__ __align__(16) uint8_t sw_sm[];
     uint4* s_frag = reinterpret_cast<uint4*>(sw_sm + 2 * kStage);                      // S^T: [column tile][k-step][hi, lo][lane]
     uint4* x_frag = s_frag + 2 * kSteps * 64;                                         // x^T: [plain, scaled][column tile][k-step][hi, lo][lane]
@@ -156,18 +157,18 @@ __global__ void __launch_bounds__(kSsdThreads, 1) seq_ssd_walk_kernel(SsdBlockAr
     auto issue = [&](int blk) {
         uint8_t* dst = sw_sm + (blk & 1) * kStage;
         const uint8_t* src = p.group_ws + ((id0 + blk) * p.groups + grp) * Group::kBytes;
-        for (int i = threadIdx.x; i < Group::kBytes / 16; i += kSsdThreads) cp_async16(dst + 16 * i, src + 16 * i, 16);
+        for (int i = threadIdx.x; i < Group::kBytes / 16; i += kSsdWalk) cp_async16(dst + 16 * i, src + 16 * i, 16);
         const int n = min(kSsdBlock, len - blk * kSsdBlock);
         float* dx = reinterpret_cast<float*>(dst + Group::kBytes);
         const float* xb = xs + (size_t)blk * kSsdBlock * p.ldx;
         if (vec) {
-            for (int i = threadIdx.x; i < kSsdBlock * kSsdCols / 4; i += kSsdThreads) {
+            for (int i = threadIdx.x; i < kSsdBlock * kSsdCols / 4; i += kSsdWalk) {
                 const int tok = i / (kSsdCols / 4), j = (i % (kSsdCols / 4)) * 4;
                 const bool has = tok < n && col0 + j < p.dv;
                 cp_async16(dx + tok * kSsdLdx + j, has ? xb + (size_t)tok * p.ldx + j : p.x, has ? 16 : 0);
             }
         } else {
-            for (int i = threadIdx.x; i < kSsdBlock * kSsdCols; i += kSsdThreads) {
+            for (int i = threadIdx.x; i < kSsdBlock * kSsdCols; i += kSsdWalk) {
                 const int tok = i / kSsdCols, j = i % kSsdCols;
                 const bool has = tok < n && col0 + j < p.dv;
                 asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dx + tok * kSsdLdx + j)), "l"(has ? xb + (size_t)tok * p.ldx + j : p.x), "r"(has ? 4 : 0)
@@ -179,7 +180,7 @@ __global__ void __launch_bounds__(kSsdThreads, 1) seq_ssd_walk_kernel(SsdBlockAr
         cp_async_commit();
     };
     if (blocks > 0) issue(0);
-    // this warp's part of S^T: columns r0 / r1, states qu * kQuarter + nt * 8 + 2c, + 1
+    // this warp's part of S^T: columns r0 / r1, states qu * kEighth + nt * 8 + 2c, + 1
     const int cl = ct * 16 + g, r0 = col0 + cl, r1 = r0 + 8;
     const bool ok0 = r0 < p.dv, ok1 = r1 < p.dv;
     float* st = p.state + ((size_t)slot * p.heads + h) * p.n_state * p.dv;
@@ -188,7 +189,7 @@ __global__ void __launch_bounds__(kSsdThreads, 1) seq_ssd_walk_kernel(SsdBlockAr
     for (int nt = 0; nt < kTiles; ++nt)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            const int row = qu * kQuarter + nt * 8 + 2 * c + (e & 1);
+            const int row = qu * kEighth + nt * 8 + 2 * c + (e & 1);
             S[nt][e] = (e < 2 ? ok0 : ok1) && row < p.n_state ? st[(size_t)row * p.dv + (e < 2 ? r0 : r1)] : 0.0f;
         }
     const float skip = p.skip ? p.skip[h] : 0.0f;
@@ -206,27 +207,27 @@ __global__ void __launch_bounds__(kSsdThreads, 1) seq_ssd_walk_kernel(SsdBlockAr
         const float* sd = sL + kSsdBlock;
         const float Gn = sG[kSsdBlock - 1], Ln = sL[kSsdBlock - 1];
 #pragma unroll
-        for (int j = 0; j < kTiles / 2; ++j) {               // the state as A fragments for all warps
-            uint4 hi, lo;
-            split_bf16(S[2 * j][0], S[2 * j][1], &hi.x, &lo.x);
-            split_bf16(S[2 * j][2], S[2 * j][3], &hi.y, &lo.y);
-            split_bf16(S[2 * j + 1][0], S[2 * j + 1][1], &hi.z, &lo.z);
-            split_bf16(S[2 * j + 1][2], S[2 * j + 1][3], &hi.w, &lo.w);
-            uint4* at = s_frag + (ct * kSteps + qu * (kTiles / 2) + j) * 64 + lane;
+        for (int nt = 0; nt < kTiles; ++nt) {                // the state as halves of A fragments for all warps
+            uint2 hi, lo;
+            split_bf16(S[nt][0], S[nt][1], &hi.x, &lo.x);
+            split_bf16(S[nt][2], S[nt][3], &hi.y, &lo.y);
+            const int tile = qu * kTiles + nt;
+            uint2* at = reinterpret_cast<uint2*>(s_frag + (ct * kSteps + tile / 2) * 64 + lane) + tile % 2;
             at[0] = hi;
-            at[32] = lo;
+            at[64] = lo;
         }
-        {                                                    // x^T as A fragments, plain and decayed to the block's end: a fragment per thread
-            const float* at = sx + (qu * 16 + 2 * c) * kSsdLdx + cl;
-            float v[8], f[4];
+        {                                                    // x^T as A fragments: a plain one or one decayed to the block's end per thread
+            const int ks = qu & 3, scaled = qu >> 2;
+            const float* at = sx + (ks * 16 + 2 * c) * kSsdLdx + cl;
+            float v[8];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {                    // token 2c + (i & 1) + 8 (i >> 1): columns g and g + 8
-                const int tok = qu * 16 + 2 * c + (i & 1) + 8 * (i >> 1);
-                v[2 * i] = at[((i & 1) + 8 * (i >> 1)) * kSsdLdx];
-                v[2 * i + 1] = at[((i & 1) + 8 * (i >> 1)) * kSsdLdx + 8];
-                f[i] = exp2f((Gn - sG[tok]) + (Ln - sL[tok])) * sd[tok];
+                const int tok = ks * 16 + 2 * c + (i & 1) + 8 * (i >> 1);
+                const float f = scaled ? exp2f((Gn - sG[tok]) + (Ln - sL[tok])) * sd[tok] : 1.0f;
+                v[2 * i] = at[((i & 1) + 8 * (i >> 1)) * kSsdLdx] * f;
+                v[2 * i + 1] = at[((i & 1) + 8 * (i >> 1)) * kSsdLdx + 8] * f;
             }
-            uint4* to = x_frag + (ct * 4 + qu) * 64 + lane;
+            uint4* to = x_frag + (scaled * 8 + ct * 4 + ks) * 64 + lane;
             uint4 hi, lo;
             split_bf16(v[0], v[2], &hi.x, &lo.x);
             split_bf16(v[1], v[3], &hi.y, &lo.y);
@@ -234,38 +235,31 @@ __global__ void __launch_bounds__(kSsdThreads, 1) seq_ssd_walk_kernel(SsdBlockAr
             split_bf16(v[5], v[7], &hi.w, &lo.w);
             to[0] = hi;
             to[32] = lo;
-            split_bf16(v[0] * f[0], v[2] * f[1], &hi.x, &lo.x);
-            split_bf16(v[1] * f[0], v[3] * f[1], &hi.y, &lo.y);
-            split_bf16(v[4] * f[2], v[6] * f[3], &hi.z, &lo.z);
-            split_bf16(v[5] * f[2], v[7] * f[3], &hi.w, &lo.w);
-            to[2 * 4 * 64] = hi;
-            to[2 * 4 * 64 + 32] = lo;
         }
         __syncthreads();
-        // outputs: columns of tile ct, tokens qu * 16 + nt * 8 + 2c, + 1
-        float y[2][3][4] = {};
+        // outputs: columns of tile ct, tokens qu * 8 + 2c, + 1
+        float y[3][4] = {};
 #pragma unroll
         for (int ks = 0; ks < kSteps; ++ks) {
             uint32_t ah[4], al[4];
             ssd_load(ah, s_frag + (ct * kSteps + ks) * 64 + lane);
             ssd_load(al, s_frag + (ct * kSteps + ks) * 64 + 32 + lane);
-#pragma unroll
-            for (int nt = 0; nt < 2; ++nt) ssd_mma(y[nt], ah, al, Cf[((qu * 2 + nt) * kSteps + ks) * 32]);
+            ssd_mma(y, ah, al, Cf[(qu * kSteps + ks) * 32]);
         }
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-            const float2 G2 = *reinterpret_cast<const float2*>(sG + qu * 16 + nt * 8 + 2 * c);
-            const float2 L2 = *reinterpret_cast<const float2*>(sL + qu * 16 + nt * 8 + 2 * c);
+        {
+            const float2 G2 = *reinterpret_cast<const float2*>(sG + qu * 8 + 2 * c), L2 = *reinterpret_cast<const float2*>(sL + qu * 8 + 2 * c);
             const float e0 = exp2f(G2.x + L2.x), e1 = exp2f(G2.y + L2.y);
 #pragma unroll
             for (int q = 0; q < 3; ++q) {
-                y[nt][q][0] *= e0;
-                y[nt][q][1] *= e1;
-                y[nt][q][2] *= e0;
-                y[nt][q][3] *= e1;
+                y[q][0] *= e0;
+                y[q][1] *= e1;
+                y[q][2] *= e0;
+                y[q][3] *= e1;
             }
         }
-        for (int ks = 0; ks <= qu; ++ks) {                   // tokens j of the block's earlier quarters and of this one
+        const int i = qu * 8 + g;
+        const float Gi = sG[i], Li = sL[i];
+        for (int ks = 0; ks <= qu / 2; ++ks) {               // tokens j up to these
             uint32_t ah[4], al[4];
             ssd_load(ah, x_frag + (ct * 4 + ks) * 64 + lane);
             ssd_load(al, x_frag + (ct * 4 + ks) * 64 + 32 + lane);
@@ -273,26 +267,19 @@ __global__ void __launch_bounds__(kSsdThreads, 1) seq_ssd_walk_kernel(SsdBlockAr
             const float2 Ga = *reinterpret_cast<const float2*>(sG + j), Gb = *reinterpret_cast<const float2*>(sG + j + 8);
             const float2 La = *reinterpret_cast<const float2*>(sL + j), Lb = *reinterpret_cast<const float2*>(sL + j + 8);
             const float2 da = *reinterpret_cast<const float2*>(sd + j), db = *reinterpret_cast<const float2*>(sd + j + 8);
-#pragma unroll
-            for (int nt = 0; nt < 2; ++nt) {
-                const int i = qu * 16 + nt * 8 + g;
-                const float Gi = sG[i], Li = sL[i];
-                const float4 w = Wf[((qu * 2 + nt) * 4 + ks) * 32];
-                const float w0 = j <= i ? w.x * (exp2f((Gi - Ga.x) + (Li - La.x)) * da.x) : 0.0f, w1 = j + 1 <= i ? w.y * (exp2f((Gi - Ga.y) + (Li - La.y)) * da.y) : 0.0f;
-                const float w2 = j + 8 <= i ? w.z * (exp2f((Gi - Gb.x) + (Li - Lb.x)) * db.x) : 0.0f, w3 = j + 9 <= i ? w.w * (exp2f((Gi - Gb.y) + (Li - Lb.y)) * db.y) : 0.0f;
-                ssd_mma(y[nt], ah, al, ssd_frag(w0, w1, w2, w3));
-            }
+            const float4 w = Wf[(qu * 4 + ks) * 32];
+            const float w0 = j <= i ? w.x * (exp2f((Gi - Ga.x) + (Li - La.x)) * da.x) : 0.0f, w1 = j + 1 <= i ? w.y * (exp2f((Gi - Ga.y) + (Li - La.y)) * da.y) : 0.0f;
+            const float w2 = j + 8 <= i ? w.z * (exp2f((Gi - Gb.x) + (Li - Lb.x)) * db.x) : 0.0f, w3 = j + 9 <= i ? w.w * (exp2f((Gi - Gb.y) + (Li - Lb.y)) * db.y) : 0.0f;
+            ssd_mma(y, ah, al, ssd_frag(w0, w1, w2, w3));
         }
         const int n = min(kSsdBlock, len - blk * kSsdBlock);
 #pragma unroll
-        for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int tok = qu * 16 + nt * 8 + 2 * c + (e & 1);
-                if (tok < n && (e < 2 ? ok0 : ok1))
-                    p.y[(size_t)(start + blk * kSsdBlock + tok) * p.ldy + (size_t)h * p.dv + (e < 2 ? r0 : r1)] =
-                        fmaf(skip, sx[tok * kSsdLdx + cl + (e < 2 ? 0 : 8)], y[nt][0][e] + (y[nt][1][e] + y[nt][2][e]));
-            }
+        for (int e = 0; e < 4; ++e) {
+            const int tok = qu * 8 + 2 * c + (e & 1);
+            if (tok < n && (e < 2 ? ok0 : ok1))
+                p.y[(size_t)(start + blk * kSsdBlock + tok) * p.ldy + (size_t)h * p.dv + (e < 2 ? r0 : r1)] =
+                    fmaf(skip, sx[tok * kSsdLdx + cl + (e < 2 ? 0 : 8)], y[0][e] + (y[1][e] + y[2][e]));
+        }
         // the state
         const float dn = exp2f(Gn + Ln);
         float add[kTiles][3][4] = {};
@@ -313,7 +300,7 @@ __global__ void __launch_bounds__(kSsdThreads, 1) seq_ssd_walk_kernel(SsdBlockAr
     for (int nt = 0; nt < kTiles; ++nt)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            const int row = qu * kQuarter + nt * 8 + 2 * c + (e & 1);
+            const int row = qu * kEighth + nt * 8 + 2 * c + (e & 1);
             if ((e < 2 ? ok0 : ok1) && row < p.n_state) st[(size_t)row * p.dv + (e < 2 ? r0 : r1)] = S[nt][e];
         }
 }
@@ -336,7 +323,7 @@ static int launch_ssd(SsdBlockArgs p, cudaStream_t st) {
     seq_ssd_prepare_kernel<NK><<<dim3(p.b.n_qtiles, p.groups + (p.heads + per - 1) / per), kSsdThreads, smem_prep, st>>>(p, vec_prep);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
-    seq_ssd_walk_kernel<NK><<<dim3(p.b.nseg, p.heads, (p.dv + kSsdCols - 1) / kSsdCols), kSsdThreads, smem, st>>>(p, vec);
+    seq_ssd_walk_kernel<NK><<<dim3(p.b.nseg, p.heads, (p.dv + kSsdCols - 1) / kSsdCols), kSsdWalk, smem, st>>>(p, vec);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;
