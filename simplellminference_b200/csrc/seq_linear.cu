@@ -29,18 +29,19 @@ constexpr int kRowsBlock = 64;     // weight rows between two flushes of the par
 
 // TT: activation rows the products are computed for (T rounded up to 1, 2, 4 or 8). A lane owns two 16-byte chunks of every weight row of a panel
 // of K and keeps the matching activations of all TT rows in registers (8 rows: half as many warps, so that they fit); kGroup weight rows are
-// reduced across the lanes together; kDeep rows are in flight per warp. The ring comes to 128 KB per SM, more than twice what the HBM rate asks
-// for at its latency.
+// reduced across the lanes together; kDeep rows are in flight per warp: a ring of 64 KB per SM (8 rows: 128 KB), where the HBM rate asks for some 35 at
+// its latency. Groups of two, not four: less code to fetch at the start of every launch (2048 x 2048, one row 5.2 -> 4.7 us; 6144 x 4096, four
+// rows 16.5 -> 14.6 us).
 template <int TT>
 struct RowsShape {
-    static constexpr int kWarps = TT <= 4 ? 16 : 8, kChunks = 2, kGroup = TT <= 4 ? 4 : 2, kDeep = TT <= 4 ? 8 : 16;
+    static constexpr int kWarps = TT <= 4 ? 16 : 8, kChunks = 2, kGroup = 2, kDeep = TT <= 4 ? 4 : 16;
     static constexpr int kRing = kWarps * kDeep * kChunks * 512;
 };
 
 // Up to 8 activation rows against a stream of weight rows. Bound: HBM, every weight is read once. One CTA per SM takes a contiguous
 // share of the weight rows; WK = 2^wk_log2 of its warps cut K among themselves (so that every SM's share ends at the same time whatever N), the
 // others take other rows. What a weight costs beside its load was the bound of a body whose lanes read the activations from memory for every weight
-// row (2 T bytes of activations through L1 per byte of weights: 1.1 TB/s at 4 rows of 6144 x 4096 bf16, now 3.1; one row 2.6, now 4.2 and 5.3 at
+// row (2 T bytes of activations through L1 per byte of weights: 1.1 TB/s at 4 rows of 6144 x 4096 bf16, now 3.4; one row 2.6, now 4.4 and 5.3 at
 // 32000 x 2048): here the activations of a lane's columns stay in registers for all rows, the
 // weights arrive through cp.async in a ring that only their own lane reads back (no barrier in the stream), fma.rn.f32x2 does two products per
 // instruction, and TT x kGroup sums cross the lanes in one halving exchange.
@@ -440,8 +441,8 @@ static int launch_rows(const sllm::LinArgs& p, int batch, cudaStream_t st) {
     const bool vec = p.K % e == 0 && p.ldw % e == 0 && (p.w_bs % e) == 0 && p.lda % 4 == 0 && (p.a_bs % 4) == 0 && ((uintptr_t)p.W % 16) == 0 &&
                      ((uintptr_t)p.A % 16) == 0;
     // The streaming body starts 1.4 to 2 us later than the small one (its ring, its activations, more code) and is faster from about 2 million
-    // weights on. Measured, bf16, old | new: 1024 x 1024 3.8 | 4.5 us (one row) and 4.7 | 6.9 (four), 2048 x 2048 6.4 | 5.2 and 9.4 | 7.9, 32 matrices of
-    // 512 x 128 13.4 | 8.7 (four), 6144 x 4096 19.4 | 12.0 (one), 46.9 | 16.3 (four) and 85.4 | 21.7 (eight), 32000 x 2048 40.1 | 24.8 (one row).
+    // weights on. Measured, bf16, old | new: 1024 x 1024 3.8 | 4.1 us (one row) and 4.7 | 6.4 (four), 2048 x 2048 6.4 | 4.7 and 9.4 | 7.4, 32 matrices of
+    // 512 x 128 13.4 | 8.7 (four), 6144 x 4096 19.4 | 11.4 (one), 46.9 | 14.6 (four) and 85.4 | 21.7 (eight), 32000 x 2048 40.1 | 24.5 (one row).
     if (vec && (long long)p.N * batch * p.K >= 1500000LL) {
         int rc;
         if (p.T == 1) rc = bf16 ? launch_rows_body<SLLM_BF16, 1>(p, batch, st) : launch_rows_body<SLLM_F32, 1>(p, batch, st);
