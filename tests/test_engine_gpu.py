@@ -56,7 +56,7 @@ def test_golden_models(golden_models, name, mode):
     if name.endswith("_256"):
         # BASELINE.json configs[1] at its full 256 tokens. Over such a run the fp32 rounding noise of ANY re-ordered sum compounds through
         # the cache (every CUDA path alike: 3e-3 of max|logit| by position 120, 1e-2 by position 170 against the oracle on identical
-        # tokens, tools/v2_locate.py), while the reference's own stream has top-1/top-2 margins down to 0.02 (position 159): identity
+        # tokens), while the reference's own stream has top-1/top-2 margins down to 0.02 (position 159): identity
         # beyond ~140 tokens is luck. Held to: the first 128 tokens identical in free-running greedy decode, and — teacher-forced on
         # the reference's tokens — the echo of all 255 and the final logits within 5e-2 of max|logit|.
         toks = eng.greedy(prompt, n_total)
