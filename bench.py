@@ -1,11 +1,11 @@
 #!/usr/bin/env python
-"""bench.py — decode tokens/s (batch 1, greedy) and fraction of the HBM roofline (BASELINE.json metric).
+"""bench.py — decode tokens/s (batch 1, greedy) and fraction of the HBM roofline (the headline metric).
 
   python bench.py [--gpus N] [--steps K] [--warmup W]                 our arm (CUDA, sm_100a)
   python bench.py --impl reference [--gpus N] [--steps K] [--warmup W] the reference's CPU path, host cores
   torchrun ... bench.py --gpus N ...                                   tensor parallel over N GPUs (one rank each)
 
-Workload (config.workload): Llama-2-7B-shaped model (BASELINE.json configs[3], the configuration the metric
+Workload (config.workload): Llama-2-7B-shaped model (the configuration the metric
 and the >=70 % target are quoted on; it fits one GPU), random-init synthetic weights (counter-based hash, bf16
 storage), batch-1 greedy decode continuing a 512-token synthetic prompt. A "step" is ONE decoded token = one
 pass of the whole forward hot path (all weights + the KV cache read once). Per-step working set (13.5 GB) is
@@ -54,7 +54,7 @@ def parse():
     ap.add_argument("--no-mega", action="store_true", help="use the per-kernel fused CUDA-graph path instead of the persistent megakernel")
     ap.add_argument("--mega-ll", action="store_true", help="single GPU: the barrier-free {value,epoch}-word megakernel instead of the grid-barrier one")
     ap.add_argument("--mega-fuse-down", action="store_true", help="single GPU, experimental: the megakernel variant with the down projection fused into the gate_up phase (SLLM_ENGINE_MEGA_FUSE_DOWN)")
-    ap.add_argument("--mega-v1", action="store_true", help="single GPU: the round-1 grid-barrier megakernel (five grid-wide dependency points per layer, deterministic sums) instead of "
+    ap.add_argument("--mega-v1", action="store_true", help="single GPU: the first, grid-barrier megakernel (five grid-wide dependency points per layer, deterministic sums) instead of "
                                                            "the default: csrc/megakernel2.cu with the fused down projection and the calibrated partition")
     ap.add_argument("--no-calibrate", action="store_true", help="skip sllm_engine_calibrate (per-CTA shares of every phase sized by the measured streaming rate of each SM)")
     ap.add_argument("--extras", action="store_true", help="after the timed regions, also run the secondary measurements in child processes (batched multi-sequence decode, "
@@ -101,7 +101,7 @@ def tensor_peak():
 
 
 def prefill_flops(ms, T):
-    """SURVEY.md 8d: GEMM flops of T prompt rows + last-row classifier + causal attention."""
+    """GEMM flops of T prompt rows + last-row classifier + causal attention."""
     d, kv, I, L, V = ms.hidden, ms.kv_hidden, ms.inter, ms.layers, ms.vocab
     return 2.0 * T * L * (2 * d * d + 2 * kv * d + 3 * I * d) + 2.0 * V * d + 2.0 * L * d * T * T
 
@@ -347,7 +347,7 @@ def experiments_sample(args, main_checksum, K, W):
     """Secondary, N = 1 only, each in its own child process after every timed region of the main arm (nothing here can touch the headline):
     (1) the experimental megakernel with the down projection fused into the gate_up phase on the main arm's exact workload — tokens/s and
     whether its tokens equal the main arm's; (2) tools/microbench/fusion_probe — what combining 148 partial vectors with vector reductions
-    costs against the grid barrier, cluster co-residency, TMA ingest from L2-resident against HBM-resident tiles (DESIGN.md section 10);
+    costs against the grid barrier, cluster co-residency, TMA ingest from L2-resident against HBM-resident tiles;
     (3) the per-phase timelines of both kernels."""
     out = {}
     if args.wdtype in ("f32", "bf16"):
@@ -510,7 +510,7 @@ def run_ours(args):
         prefill = {"tokens": P, "ms": pf_ms, "tokens_per_sec": P / (pf_ms * 1e-3), "tflops": tf, "peak_tflops": tpeak * world,
                    "tensor_pipe_frac": tf / (tpeak * world), "peak_source": tsrc, "reps": R,
                    "what": "sllm_engine_prefill: all layers over the whole prompt (tcgen05/TMEM GEMMs + block attention) + last-row logits/arg-max; "
-                           "algorithmic flops per SURVEY.md 8d",
+                           "algorithmic flops: GEMMs of the prompt rows, last-row classifier, causal attention",
                    "ms_without_exchanges": pf_noex_ms, "exchange_trace": pf_trace,
                    "tp_exchange": None if world == 1 else ("peer memory (csrc/prefill_tp.cu: sum over ranks + residual + RMSNorm + row distribution in one kernel)"
                                                            if getattr(eng, "prefill_p2p", False) else "ncclAllReduce + RMSNorm kernel")}
@@ -584,7 +584,7 @@ def run_ours(args):
         roof = {"bound": "hbm", "kernel": kname,
                 "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak, "traffic": traffic, "bytes_per_launch": step_bytes,
                 "us_per_launch": 1e3 * ms_total / K, "peak_source": peak_src, "traffic_source": traffic_src,
-                "how": f"{K} launches = the timed region itself, CUDA events on the launching stream; B(p) per SURVEY.md 8d"}
+                "how": f"{K} launches = the timed region itself, CUDA events on the launching stream; B(p): the weights once, the cache rows read and the row written"}
     elif not args.unfused:
         eng.set_state(tok, min(pos, ms.max_len - 1))
         reps = max(2, 64 // ms.layers)
@@ -622,7 +622,7 @@ def run_ours(args):
     if world == 1 and args.extras:
         eng.close()
         try:   # secondary: never lose the line over any of it. Order = cost: the two short experiments, the batched decoder, the timelines
-            if mode == "megakernel":   # the round-1 kernel: measure its fused-down variant beside it
+            if mode == "megakernel":   # the grid-barrier kernel: measure its fused-down variant beside it
                 experiments = experiments_sample(args, int(np.sum(tokens.astype(np.int64)) % 1000003), K, W)
             batch = batch_decode_sample(args)
             # the parity cases of the batched decoder that no GPU has run yet (pytest reports them as xfail / xpass only): PASS / FAIL per

@@ -22,7 +22,7 @@
  *  - activations, RoPE tables and accumulators are fp32. Matrix weights are stored as fp32, bf16 or
  *    int8-with-group-scales (SLLM_F32 / SLLM_BF16 / SLLM_INT8); the KV cache as fp32 or bf16.
  *  - there is NO CPU fallback anywhere behind this header;
- *  - threading: the model of the reference (source/model/model.cpp drives one model from one host thread, SURVEY.md 8b) and of the
+ *  - threading: the model of the reference (source/model/model.cpp drives one model from one host thread) and of the
  *    tensor-parallel runtime here — ONE process per GPU, one host thread driving an engine / batch at a time. The library keeps
  *    per-process caches of device facts and of per-kernel shared-memory attributes for the device that was current at first use, and
  *    the development knobs of sllm_tune are process-wide: do not drive two devices, or one engine from two threads, in one process.
@@ -97,7 +97,7 @@ int sllm_rope_tables(int32_t head_dim, int32_t max_len, float theta, float* sin_
                      sllm_stream_t stream);
 
 /* replaces kernel::rope_kernel_cuda (rope_kernel.cuh:7-8): rotate-half RoPE in place on q[0..q_dim) and
- * k[0..k_dim). The reference rotates k over q_dim too (GQA over-run, SURVEY.md Appendix D); here k_dim is
+ * k[0..k_dim). The reference rotates k over q_dim too (GQA over-run); here k_dim is
  * explicit. k may be fp32 only (it is a row of an fp32 cache or a scratch vector). */
 int sllm_rope_f32(float* q, float* k, const int32_t* pos_dev, int32_t pos, const float* sin_tab,
                   const float* cos_tab, int32_t q_dim, int32_t k_dim, int32_t head_dim, sllm_stream_t stream);
@@ -216,7 +216,7 @@ int sllm_engine_p2p_import(sllm_engine* e, const void* all_handles /* tp_size * 
    SLLM_ENOTSUP: the engine has no such block (one rank, no SLLM_ENGINE_P2P_ALLREDUCE, shape not taken by the batched prefill) — prefill
    then needs the NCCL communicator. Every rank must issue the same sequence of sllm_engine_prefill calls (the exchange kernels wait for each
    other's epoch flags; a wait that is never answered traps after ~20 s instead of hanging the GPU): a prefill that failed on one rank only leaves
-   the ranks out of step — destroy the engines. Replaces nothing in the reference (it has neither prefill nor a working multi-GPU build, SURVEY 8e). */
+   the ranks out of step — destroy the engines. Replaces nothing in the reference (it has neither prefill nor a working multi-GPU build). */
 int sllm_engine_prefill_p2p_export(sllm_engine* e, void* handle_bytes_64);
 int sllm_engine_prefill_p2p_import(sllm_engine* e, const void* all_handles /* tp_size * 64 bytes */);
 
@@ -346,7 +346,7 @@ int sllm_batch_buffer(sllm_batch* b, int32_t buffer_id, void** dev_ptr, int64_t*
 int32_t sllm_batch_free_pages(const sllm_batch* b);
 int32_t sllm_batch_position(const sllm_batch* b, int32_t slot);   /* position of the slot's next step; -1 = free slot */
 /* algorithmic HBM bytes of the NEXT step: every weight once, plus per live sequence its embedding row, the K/V rows
- * 0..pos it reads and the row it writes (SURVEY.md 8d B(p) with the weight term shared) */
+ * 0..pos it reads and the row it writes (the weights counted once for all slots) */
 int64_t sllm_batch_step_bytes(const sllm_batch* b);
 int64_t sllm_batch_total_launches(const sllm_batch* b);
 /* Device bytes sllm_batch_create(max_seqs, page_len, n_pages, kv_dtype) takes on an engine of this shape (the two page pools
@@ -366,7 +366,7 @@ float sllm_engine_calibration(const sllm_engine* e, int32_t cta);
 /* Introspection for parity tests and the roofline: named buffers follow the reference's ModelBufferType
  * numbering (include/model/model.h:14-34); returns a device pointer and its element count/dtype. */
 int sllm_engine_buffer(sllm_engine* e, int32_t buffer_id, void** dev_ptr, int64_t* n_elems, int32_t* dtype);
-/* algorithmic HBM bytes one decode step at position pos must move on this rank (SURVEY.md §8d B(p)) */
+/* algorithmic HBM bytes one decode step at position pos must move on this rank */
 int64_t sllm_engine_step_bytes(const sllm_engine* e, int32_t pos);
 /* Enqueue ONE fused kernel of the decode step for `layer` at the current device-side position, for per-kernel
  * timing and profiling. kind: 0 embedding, 1 qkv (RMSNorm+QKV GEMV+RoPE+cache write), 2 mha (flash decoding),

@@ -5,12 +5,12 @@
  * and (kind "port") a CPU baseline. Only tests/, __graft_entry__.smoke() and bench.py's cpu_baseline /
  * --impl reference legs may load it. The product path never calls into this file.
  *
- * Pinning: the reference ships no golden vectors (SURVEY.md §4), so this restatement is pinned against the
+ * Pinning: the reference ships no golden vectors, so this restatement is pinned against the
  * reference ITSELF: oracle/_ref (the unmodified reference sources compiled by oracle/Makefile) is run on
  * seeded inputs, op by op and whole-model, and must agree BIT-FOR-BIT (tests/test_oracle_cpu.py), and against
  * the fixtures under tests/golden/ that tests/golden/make_golden.py generated from oracle/_ref.
  *
- * Deliberate differences from the reference (SURVEY.md Appendix D "do not mirror"): K is rotated over
+ * Deliberate differences from the reference: K is rotated over
  * kv_hidden elements only (the reference over-runs into the next cache rows for GQA, rope_kernel.cpp:27-38),
  * which leaves results unchanged for pos <= max_len - heads/kv_heads; 64-bit offsets.
  * One extension: orc_set_kv_bf16() rounds every K/V cache row to bfloat16 (after RoPE), which is the

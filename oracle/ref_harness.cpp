@@ -6,7 +6,7 @@
 // tests/, __graft_entry__.smoke() and bench.py's cpu_baseline / --impl reference legs as the CHECKER and
 // the CPU BASELINE, never as the product path.
 //
-// Driving technique (SURVEY.md §8c): model::LlamaModel keeps config_/raw_model_data_/Llama_layers_/buffers_
+// Driving technique: model::LlamaModel keeps config_/raw_model_data_/Llama_layers_/buffers_
 // and its init steps protected (include/model/model.h:69-88), so a subclass can set an arbitrary shape and
 // point the weight accessor at a caller-owned fp32 blob in the reference's own tensor order
 // (source/model/model.cpp:336-469) without touching a file and without editing the reference.

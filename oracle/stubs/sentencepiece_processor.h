@@ -1,5 +1,5 @@
 // Stub for the third-party sentencepiece header that op/encode.h includes.
-// TEST INFRASTRUCTURE ONLY (oracle build). The tokenizer is out of scope (SURVEY.md §2.1):
+// TEST INFRASTRUCTURE ONLY (oracle build). The tokenizer is out of scope:
 // op::SPELayer is constructed unconditionally by LlamaModel::create_nonparam_layers, so the
 // type must exist and Load() must succeed; nothing on the forward path calls it.
 #pragma once

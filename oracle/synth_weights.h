@@ -2,7 +2,7 @@
  *
  * Counter-based, integer-exact weight generator shared by the CPU oracle and the CUDA product path
  * (simplellminference_b200/csrc/synth.cuh restates the same arithmetic for the device), so both sides
- * materialise BIT-IDENTICAL weights without shipping multi-GiB files (SURVEY.md §8d "Weight values").
+ * materialise BIT-IDENTICAL weights without shipping multi-GiB files.
  *
  *   stream(t)   = sm64(seed * 0x100000001B3 + t)                  t = tensor id (blob segment, below)
  *   h(t, i)     = sm64(stream(t) + i)                             i = element index inside the segment

@@ -7,7 +7,7 @@ Layers (bottom-up):
   kernels.py   one Python wrapper per op launcher (torch tensors are only the carriers of device pointers)
   engine.py    the decode engine (arena + KV cache + CUDA-graph decode step, tensor parallel)
   batch.py     batched multi-sequence decode over a paged KV cache (sllm_batch_* / sllm_kvpages_*)
-  config.py    the model-shape presets named by BASELINE.json
+  config.py    the model-shape presets
 """
 from .config import ModelShape, PRESETS, F32, BF16, INT8  # noqa: F401
 

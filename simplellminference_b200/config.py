@@ -1,4 +1,4 @@
-"""Model-shape presets (reference: include/model/config.h:5-17 hard-codes ONE shape; BASELINE.json names five)."""
+"""Model-shape presets (reference: include/model/config.h:5-17 hard-codes ONE shape)."""
 from __future__ import annotations
 
 from dataclasses import dataclass, asdict, replace
@@ -34,7 +34,7 @@ class ModelShape:
         return V * d + (2 * L + 1) * d + L * (2 * d * d + 2 * kv * d + 3 * I * d)
 
     def step_bytes(self, pos: int, w_dtype: int = BF16, kv_dtype: int = BF16, group: int = 64) -> float:
-        """Algorithmic HBM bytes of one decode step at position `pos` (SURVEY.md §8d, B(p))."""
+        """Algorithmic HBM bytes of one decode step at position `pos`."""
         bw = {F32: 4.0, BF16: 2.0, INT8: 1.0 + 4.0 / group}[w_dtype]
         bkv = 4.0 if kv_dtype == F32 else 2.0
         d, kv, I, L, V = self.hidden, self.kv_hidden, self.inter, self.layers, self.vocab
@@ -45,7 +45,7 @@ class ModelShape:
         return asdict(self)
 
 
-# BASELINE.json configs (shapes only; weights are random-init)
+# shapes only; weights are random
 PRESETS = {
     "stories15M": ModelShape(32000, 48, 288, 288, 768, 256, 6, 6, 6),
     "stories110M": ModelShape(32000, 64, 768, 768, 2048, 1024, 12, 12, 12),

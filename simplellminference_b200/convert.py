@@ -1,4 +1,4 @@
-"""Checkpoint converters into the reference's weight file (SURVEY.md 8f rank 1).
+"""Checkpoint converters into the reference's weight file.
 
 The reference mmaps a HEADERLESS raw little-endian fp32 blob in its own tensor order (source/model/model.cpp:340-468):
     E[V][d] | (2L+1) norm vectors [d] (attention norm l, ffn norm l, ..., final) | wq[L][d][d] | wk[L][kv][d] | wv[L][kv][d] |

@@ -1,5 +1,5 @@
 // csrc/batch.cu — sllm_batch_* / sllm_kvpages_*: batched multi-sequence greedy decode over a paged KV cache
-// (SURVEY.md §8f rank 3). Additive: the reference decodes ONE sequence (include/model/model.h:15-18 input_token{1},
+// Additive: the reference decodes ONE sequence (include/model/model.h:15-18 input_token{1},
 // position{1}; source/model/model.cpp:148-185); here up to 64 sequences, each at its own position, advance one token
 // per step and share a single pass over the weights.
 //

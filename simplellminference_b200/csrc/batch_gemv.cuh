@@ -2,7 +2,7 @@
 //
 // Y[b][r] = sum_j X[b][j] * W[r][j] for up to NB activation vectors against ONE pass over the weight matrix: the
 // weights are the HBM traffic of a decode step, so B sequences stepping together read them once instead of B times
-// ("turns GEMV into skinny GEMM"). Same kernel shape as gemv_core.cuh, whose building blocks it
+// Same kernel shape as gemv_core.cuh, whose building blocks it
 // reuses unchanged (plane-staged activations, 128-bit streaming weight loads, two-row units, warp-shuffle
 // reductions): every sequence's dot product is accumulated in exactly the order of the one-sequence kernel, so a
 // GEMV result does not depend on which other sequences share the launch. Activations stay fp32 (the decode parity

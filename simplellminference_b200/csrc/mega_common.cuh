@@ -169,7 +169,7 @@ __device__ __forceinline__ void down_t_rows(int g0, int g1, int rg, int RG, int&
     b = g0 + (cnt * (rg + 1)) / RG;
 }
 
-// ---- L2 prefetch of the weight stream: built twice in round 2, measured, removed ------------------------------------------------------
+// ---- L2 prefetch of the weight stream: built twice, measured, removed ------------------------------------------------------
 // The rings hold 128 KB per SM; at a dependency point (grid barrier, attention, per-head counters) the consumers stall and HBM runs dry
 // (with the dot products removed the step takes exactly as long, with the barriers removed it is 20 % shorter: r02_mega_debug_v1.jsonl).
 // Asking the L2 for the tiles beyond the ring with cp.async.bulk.prefetch.L2 works IN ISOLATION (r02_prefetch_probe.jsonl: 39 MB asked

@@ -2,7 +2,7 @@
 // kernel::*_cuda entry point (include/sllm_b200.h names each). These are the drop-in kernels behind the C++
 // op layers; the fused decode step (decode_fused.cu) folds them into the GEMV kernels instead.
 //
-// Numerics follow the CPU reference's order of operations (SURVEY.md Appendix A) except for reduction order:
+// Numerics follow the CPU reference's order of operations except for reduction order:
 // IEEE sqrt/divide (no rsqrtf, no --use_fast_math), accurate expf, (x*inv)*w association in RMSNorm.
 #include <cmath>
 #include <vector>

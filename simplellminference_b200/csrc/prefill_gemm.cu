@@ -17,8 +17,9 @@
 // {k inside a K slice, row inside a tile, K slice, tile row}: prefill and decode share one copy of the weights.
 // Rows of the tiled layout are in unit order, so the two values an epilogue needs together (RoPE partners,
 // (up, gate)) sit in ADJACENT accumulator columns of the same thread.
-// What bounds it (profiles/r01_prefill_ncu_raw.md): the bytes an SM can ingest (~65 GB/s per SM through TMA),
-// not the tensor pipe — hence the two-SM tile; L2 prefetch, TMA multicast across pairs and stream-K were measured and dropped.
+// The one-SM tile took its operands in at ~65 GB/s per SM with the tensor pipe half busy (profiles/r01_prefill_ncu_raw.md) — hence the two-SM tile; L2
+// prefetch and stream-K were measured and dropped. What a two-SM tile waits for is not known: at 2048 x 12288 x 4096 its 440 tiles fill the waves and take
+// 188 us, two thirds of the rate that a library product reaches here, which asks for more bytes per SM than that.
 #include <map>
 #include <tuple>
 

@@ -1,4 +1,4 @@
-// csrc/sample.cu — temperature / top-k / top-p sampling of one logits vector on the device (SURVEY.md 8f rank 4).
+// csrc/sample.cu — temperature / top-k / top-p sampling of one logits vector on the device.
 //
 // The reference only has arg-max (source/op/argmax.cpp:7-17; LayerType::kLayerSoftmax is declared and unused, layer.h:17), so this op
 // is additive and NOT part of the parity contract with the reference; its contract is the numpy restatement in

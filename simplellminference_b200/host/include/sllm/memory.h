@@ -1,7 +1,7 @@
 // sllm/memory.h — mem::DeviceAllocator / Buffer / Tensor with the reference's contracts
 // (include/memory/alloc.h:32-137, buffer.h:18-55, tensor.h:10-127), re-implemented:
 //  * CUDADeviceAllocator is a slab pool with address-ordered coalescing (the reference's pool mixes remnants
-//    between its two size classes and never returns slabs, SURVEY.md Appendix D); allocate/release/memcpy/
+//    between its two size classes and never returns slabs); allocate/release/memcpy/
 //    memset_zero keep their signatures and error behaviour (std::bad_alloc on device OOM after a cache flush);
 //  * Tensor carries an element type (fp32 default) instead of the hard-wired 4 bytes; sizes are 64-bit;
 //  * Buffer/Tensor ownership rules are the reference's: a Tensor is a value sharing a shared_ptr<Buffer>;

@@ -78,7 +78,7 @@ void rope_cache_cal_cuda(int head_size, int max_seq_len, const mem::Tensor sin_c
 void rope_kernel_cuda(const mem::Tensor& q, const mem::Tensor& k, const mem::Tensor& pos_now, const mem::Tensor& sin_cache,
                       const mem::Tensor& cos_cache, int32_t hidden_dim_size, int32_t head_dim) {
     // k is rotated over ITS OWN length (a kv_hidden-sized cache row), not over hidden_dim_size like the reference
-    // does (GQA over-run, SURVEY.md Appendix D).
+    // does (GQA over-run).
     const int32_t k_dim = static_cast<int32_t>(k.size());
     if (pos_now.device_type() == base::DeviceType::kDeviceCUDA)
         SLLM_DO(sllm_rope_f32(out_ptr<float>(q), out_ptr<float>(k), pos_now.ptr<int32_t>(), 0, sin_cache.ptr<float>(), cos_cache.ptr<float>(),

@@ -2,7 +2,7 @@
 
 The reference tokenises with sentencepiece (op::SPELayer, include/op/encode.h:17-28, source/op/encode.cpp:5-27), feeds the prompt
 token by token, then feeds back the arg-max and prints each piece — and never stops before max_length (no EOS handling).
-Here (SURVEY.md 8f rank 2):
+Here:
   * `SPELayer` keeps the reference's three calls (encode / decode / GetVocabularySize) over the SAME third-party library
     (the `sentencepiece` Python package instead of the C++ one); nothing of the tokenizer is re-implemented;
   * `predict` feeds the prompt token by token through the decode step, exactly as the reference does (model.cpp:157-166: fp32
@@ -10,7 +10,7 @@ Here:
     STOPPING at an EOS id (additive: `eos_id=None` is the reference's behaviour) and streaming decoded text to a callback like the
     reference's std::cout. `batched_prefill=True` (opt-in) runs the prompt as ONE tensor-core pass instead (sllm_engine_prefill):
     ~200x faster on a 512-token prompt, but the operands of its GEMMs are rounded to bf16, so its KV rows and logits agree with the
-    reference within the prefill tolerance (DESIGN.md "Tolerances"), not bit for bit — token identity with the reference is only
+    reference within the prefill tolerance, not bit for bit — token identity with the reference is only
     contracted for the default.
 Token ids, not text, are what the parity tests compare; with the default arguments this module adds no arithmetic to the path.
 """

@@ -2,7 +2,7 @@
 
 Stored weights are [out][in] row-major (reference matmul_kernel.cpp:21). Column-parallel matrices (Wq, Wk, Wv, up,
 gate, classifier) are split by OUTPUT rows; row-parallel ones (Wo, Wdown) by INPUT columns; partial results of the
-row-parallel matmuls are summed over ranks (all-reduce). SURVEY.md §8e.
+row-parallel matmuls are summed over ranks (all-reduce).
 """
 from __future__ import annotations
 

@@ -3,7 +3,7 @@
     python tests/golden/make_bench_golden.py [n_generated=160]
 
 Llama-2-7B-shaped model at full depth (32 layers), synthetic weights seed 1234 rounded to bf16, bf16-rounded KV rows
-(orc_set_kv_bf16 — the definition of the bf16 cache, DESIGN.md "Tolerances"), the 512-token prompt of bench.prompt_ids fed
+(orc_set_kv_bf16 — the definition of the bf16 cache), the 512-token prompt of bench.prompt_ids fed
 token by token exactly as LlamaModel::predict does (model.cpp:157-166), then greedy arg-max feedback. Needs ~30 GiB of host
 RAM and ~10-15 minutes on 8 cores (the C restatement, pinned bit-for-bit to oracle/_ref by tests/test_oracle_cpu.py, with its
 row-parallel matmul threads; the sums inside a row are the reference's serial sums, so threading changes no bit).

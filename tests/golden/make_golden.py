@@ -3,7 +3,7 @@
 Run in the dev container (needs /root/reference):   python tests/golden/make_golden.py
 It builds oracle/_ref (oracle/Makefile: g++ -O2 -ffp-contract=off on the reference sources where they lie),
 feeds it seeded inputs and stores the reference's outputs. The reference itself ships no golden vectors
-(SURVEY.md §4), so these files ARE the pin: tests compare the C restatement (oracle/llama_oracle.c) and the
+so these files ARE the pin: tests compare the C restatement (oracle/llama_oracle.c) and the
 CUDA path against them on any box, including the GPU box where /root/reference does not exist.
 Inputs are not stored: they are regenerated from the seeds below (numpy PCG64 / the synthetic weight hash).
 """
@@ -18,7 +18,7 @@ from oracle import loader  # noqa: E402
 
 OUT = os.path.dirname(os.path.abspath(__file__))
 
-# shapes used by the fixtures (name -> loader.Shape); cfg1/cfg2 are BASELINE.json configs[0]/[1]
+# shapes used by the fixtures (name -> loader.Shape); cfg1/cfg2: stories15M and stories110M
 SHAPES = {
     "cfg1_stories15M": loader.Shape(32000, 48, 288, 288, 768, 256, 6, 6, 6),
     "cfg2_stories110M": loader.Shape(32000, 64, 768, 768, 2048, 1024, 12, 12, 12),
@@ -28,7 +28,7 @@ SHAPES = {
 MODEL_RUNS = {  # name -> (prompt, n_total, wdtype, positions whose full logits are stored)
     "cfg1_stories15M": ([1], 128, loader.F32),
     "cfg2_stories110M": ([1], 24, loader.F32),
-    "cfg2_stories110M_256": ([1], 256, loader.F32),          # BASELINE.json configs[1] at its full length: 256 greedy tokens
+    "cfg2_stories110M_256": ([1], 256, loader.F32),          # stories110M at its full length: 256 greedy tokens
     "tiny_gqa": ([1, 7, 300, 12, 44], 46, loader.F32),       # S=48, H/KVH=2 -> parity domain pos <= 46
     "tiny_gqa_bf16w": ([1, 7, 300, 12, 44], 46, loader.BF16),
     "tiny_gqa_int8w": ([1, 7, 300, 12, 44], 46, loader.INT8),

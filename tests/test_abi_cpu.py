@@ -57,7 +57,6 @@ def test_product_never_imports_oracle():
 
 
 def test_roofline_bytes_match_survey():
-    # SURVEY.md Appendix C / BASELINE.md §4
     assert abs(PRESETS["llama2-7b"].step_bytes(511, BF16, BF16) / 1e9 - 13.484) < 2e-3
     assert abs(PRESETS["stories110M"].step_bytes(255, F32, F32) / 1e9 - 0.457) < 2e-3
     assert abs(PRESETS["stories15M"].step_bytes(127, F32, F32) / 1e9 - 0.0626) < 2e-4

@@ -1,5 +1,5 @@
 """bench.py's reference arm runs on host cores only, so its JSON line — the contract the driver parses — can be checked here: one
-line on stdout, the keys of the base contract plus this tier's `cpu_baseline` and `e2e`, the metric and workload of BASELINE.json."""
+line on stdout, the keys of the base contract plus this tier's `cpu_baseline` and `e2e`, the metric and its workload."""
 import json
 import os
 import subprocess

@@ -3,11 +3,11 @@ token streams/logits produced by the unmodified reference, and against the CPU o
 
 Decode tolerance: token sequence IDENTICAL; max|dlogit| <= 3e-4 * max(1, max|logit|) at the end of a greedy run
 of up to 256 tokens, 1e-4 for a single forward from oracle-identical history; and the oracle's top1-top2 margin
-must dwarf the observed logit error so identity is meaningful. Why 3e-4 and not SURVEY.md's 1e-4: everything is
+must dwarf the observed logit error so identity is meaningful. Why 3e-4 and not 1e-4: everything is
 fp32 on both sides and only the summation order differs, but the synthetic projections have gain 4
 (std 4/sqrt(fan_in)), which amplifies rounding noise layer by layer. The yardstick is the reference against
 ITSELF: its -O2 -ffp-contract=off and -O3 -march=x86-64-v3 (FMA-contracted) builds differ by 8.1e-5 * max|logit|
-in the final logits of the cfg2 run below (measured in the dev container, see DESIGN.md "Tolerances").
+in the final logits of the cfg2 run below (measured in the dev container).
 Residual stream / KV rows are held to the same relative bound against their own max magnitude."""
 import importlib.util
 import os
@@ -54,7 +54,7 @@ def test_golden_models(golden_models, name, mode):
     want = golden_models[name + "/tokens"]
     want_l = golden_models[name + "/last_logits"]
     if name.endswith("_256"):
-        # BASELINE.json configs[1] at its full 256 tokens. Over such a run the fp32 rounding noise of ANY re-ordered sum compounds through
+        # stories110M at its full 256 tokens. Over such a run the fp32 rounding noise of ANY re-ordered sum compounds through
         # the cache (every CUDA path alike: 3e-3 of max|logit| by position 120, 1e-2 by position 170 against the oracle on identical
         # tokens), while the reference's own stream has top-1/top-2 margins down to 0.02 (position 159): identity
         # beyond ~140 tokens is luck. Held to: the first 128 tokens identical in free-running greedy decode, and — teacher-forced on
@@ -157,7 +157,7 @@ def test_medium_shape_tokens(port, mega):
     blob = port.fill_blob(oracle_shape(ms), 3, BF16)
     want, want_l = port.model(oracle_shape(ms), blob, threads=os.cpu_count() or 1).greedy(list(range(1, 33)), 150)
     eng = Engine(ms, w_dtype=BF16, kv_dtype=F32, mega=bool(mega), mega_v2=str(mega).startswith("v2"), mega_fuse_down=(mega == "v2fuse")).load_synthetic(3)
-    # fp32 cache rows of 128-wide heads (the parity-mode cache on the production shapes): in the megakernels since round 2 (K/V stages of 32 positions)
+    # fp32 cache rows of 128-wide heads (the parity-mode cache on the production shapes): in the megakernels (K/V stages of 32 positions)
     assert eng.mode == {True: "megakernel", False: "fused+graph", "v2": "megakernel(v2)", "v2fuse": "megakernel(v2,fused-down)"}[mega], eng.mode
     got = eng.greedy(list(range(1, 33)), 150)
     assert np.array_equal(got, want)
@@ -217,7 +217,7 @@ def test_full_width_llama2_7b_two_layers(port, wd, mega):
     do. bf16 KV cache (fp32 K/V tiles of 128-wide heads do not fit the megakernel), so the oracle rounds its cache rows too."""
     import dataclasses
     ms = dataclasses.replace(PRESETS["llama2-7b"], layers=2, max_len=64)
-    # seed 10: the oracle's top-1/top-2 margins along this stream are >= 5.8 (on logits of ~280). Seed 9, used until round 2, has a
+    # seed 10: the oracle's top-1/top-2 margins along this stream are >= 5.8 (on logits of ~280). Seed 9, used before, has a
     # 0.0018 margin at the first generated token: the grid-barrier kernel itself lands on either side of it depending on max_len
     # (the number of attention splits), so a token-identity assertion there tested luck, not parity
     blob = port.fill_blob(oracle_shape(ms), 10, wd, 64, threads=os.cpu_count() or 1)
@@ -290,7 +290,7 @@ def test_predict_driver(port):
     want2, _ = port.model(sh2, blob2, threads=os.cpu_count() or 1, kv_bf16=True).greedy(prompt, 121)
     eng2 = Engine(ms2, w_dtype=BF16, kv_dtype=BF16, mega=True).load_blob(blob2)
     assert eng2.prefill_supported
-    got2 = predict_ids(eng2, prompt, 120, batched_prefill=True)   # opt-in tensor-core prompt pass (bf16 operands): gain-1 model, see DESIGN.md
+    got2 = predict_ids(eng2, prompt, 120, batched_prefill=True)   # opt-in tensor-core prompt pass (bf16 operands): gain-1 model
     assert np.array_equal(got2[:99], prompt[1:])
     assert np.array_equal(got2, want2), int(np.flatnonzero(got2 != want2)[0])
     eng2.close()

@@ -1,4 +1,4 @@
-"""GPU parity at the BASELINE.json configurations THEMSELVES (full depth, full width, late positions).
+"""GPU parity at the benchmarked configurations THEMSELVES (full depth, full width, late positions).
 
 The small-shape tests cannot reach what decides correctness at depth: the 129-entry phase table, the barrier / counter epochs over
 hundreds of dependency points per step, ring run-ahead across 32 layers, split-KV attention past position 512 with 32 KV heads

@@ -42,7 +42,7 @@ def geometry(rows, cols, kind, wd):
     ("llama2-7b", BF16, BF16, 1), ("llama2-7b", INT8, BF16, 1), ("llama2-7b", BF16, BF16, 2), ("llama2-7b", BF16, BF16, 4),
     ("llama2-7b", BF16, BF16, 8), ("llama3-8b", BF16, BF16, 1), ("llama3-8b", BF16, BF16, 8)])
 def test_benchmark_configurations_run_as_one_launch_per_token(name, wd, kvd, tp):
-    """Every BASELINE.json configuration that is benchmarked through the megakernel gets a plan on a B200: one CTA per SM, within
+    """Every configuration that is benchmarked through the megakernel gets a plan on a B200: one CTA per SM, within
     the opt-in shared memory, and at most one 64-position tile per KV split at full context."""
     ms = PRESETS[name]
     ok, grid, nbytes, nsplit, why = plan(ms, wd, kvd, tp)
@@ -66,7 +66,7 @@ def test_shapes_the_megakernel_declines_say_why():
     ok, *_, why = plan(ms, INT8, BF16, group=32)
     assert not ok and "group" in why
     ok, grid, nbytes, *_ = plan(ms, BF16, F32)         # fp32 cache rows of 128-wide heads (the parity-mode cache on the 7B / 8B shapes): taken since
-    assert ok and nbytes <= B200_SMEM                  # round 2 — a K/V stage holds 32 positions instead of 64 when a row is wider than 256 bytes
+    assert ok and nbytes <= B200_SMEM                  # a K/V stage holds 32 positions instead of 64 when a row is wider than 256 bytes
     ok, *_, why = plan(ms, BF16, BF16, smem=48 * 1024)
     assert not ok and "shared memory" in why
     odd = dataclasses.replace(PRESETS["tiny_gqa"], hidden=132, heads=4, head_dim=33, kv_hidden=66)

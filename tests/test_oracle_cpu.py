@@ -111,7 +111,7 @@ def test_synthetic_weights_contract(port):
 def test_port_vs_reference_live_random_shapes(port, ref):
     """Property test (hypothesis): every op of the C restatement against the compiled reference on random shapes — head_dim not a
     power of two, grouped-query attention with 1..8 query heads per KV head, every position of the context, ties in the arg-max,
-    RoPE at theta 1e4 / 5e5 — bit for bit. The reference rotates k over q's length (Appendix D of SURVEY.md), so RoPE is compared
+    RoPE at theta 1e4 / 5e5 — bit for bit. The reference rotates k over q's length, so RoPE is compared
     with k.size == q.size, where both agree by construction."""
     from hypothesis import given, settings, strategies as st, HealthCheck
 
@@ -147,7 +147,7 @@ def test_port_vs_reference_live_random_shapes(port, ref):
 def test_port_model_vs_reference_live_random_shapes(port, ref):
     """The whole forward loop (LlamaModel::forward, model.cpp:40-140) on random small model shapes, weight types and prompts:
     token streams, final logits, residual stream and the cache rows inside the parity domain (positions <= S - H/KVH: beyond it
-    the reference's RoPE over-run corrupts rows, SURVEY.md Appendix D) — bit for bit."""
+    the reference's RoPE over-run corrupts rows) — bit for bit."""
     from hypothesis import given, settings, strategies as st, HealthCheck
 
     @settings(max_examples=12, deadline=None, suppress_health_check=list(HealthCheck), derandomize=True)

@@ -30,7 +30,7 @@ def test_plan_invariants(T, N, K, residual):
 
 
 def test_plan_llama2_7b_prompt_of_512():
-    """The shapes of the headline prefill (DESIGN.md section 7): 74 SM pairs."""
+    """The shapes of the headline prefill: 74 SM pairs."""
     assert plan(512, 12288, 4096, False)[1:3] == (192, 1)           # qkv: 2 x 64 tiles of 256 x 192 = 2 waves, 86 % full
     two_sm, bn, ksplit, units = plan(512, 4096, 4096, True)         # wo: one wave of 256 x 128 tiles left 10 pairs idle and 1.5 MB per CTA
     assert ksplit >= 2 and units <= 74

@@ -1,4 +1,4 @@
-"""Device sampling (sllm_sample_f32, SURVEY.md 8f rank 4) against a numpy restatement of its contract. Additive to the reference
+"""Device sampling (sllm_sample_f32) against a numpy restatement of its contract. Additive to the reference
 (which only has arg-max): temperature, top-k and top-p thresholds are defined on the float32 values z = logit * (1/T); the draw is
 a pure function of (logits, parameters, seed, step)."""
 import numpy as np

@@ -152,7 +152,7 @@ def test_requests_submitted_while_running_join_the_batch():
 
 def test_request_longer_than_max_len_is_refused_at_submit():
     """A request whose prompt + new tokens exceed the engine's max_len must be refused by submit(): admitted, it would fail inside
-    a chunk of steps and leave every other live request un-retired (ADVICE r1)."""
+    a chunk of steps and leave every other live request un-retired."""
     dec = FakeDecoder(max_seqs=2, page_len=4, n_pages=100, max_len=32)
     cb = ContinuousBatcher(dec)
     ok = cb.submit([1, 2, 3], 10)

@@ -1,4 +1,4 @@
-"""GPU parity tests of the batched multi-sequence decode over a paged KV cache (sllm_batch_*, SURVEY.md §8f rank 3).
+"""GPU parity tests of the batched multi-sequence decode over a paged KV cache (sllm_batch_*).
 
 The reference decodes one sequence at a time, so the oracle of a batch is the oracle run once per sequence: every
 sequence of a batch — whatever its neighbours, its slot, its pages and the moment it was admitted — must produce the
@@ -183,7 +183,7 @@ def test_step_bytes_share_the_weights(port):
     bd.close(); eng.close()
 
 
-# ---- the cases below first ran at the end of round 1 on the driver's B200 (all passed): plain tests since then, so a regression
+# ---- the cases below are plain tests, so a regression
 # of the batched decoder turns the suite red.
 
 

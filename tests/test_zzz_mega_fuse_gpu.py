@@ -6,8 +6,7 @@ contract of tests/test_engine_gpu.py: token stream IDENTICAL to the reference / 
 (fp32 cache) or 5e-3 (bf16 cache).
 
 (The file sorts after every other GPU test on purpose: a fault of this never-run kernel must not poison the CUDA context of verified tests.)
-
-First ran (and passed) at the end of round 1 on the driver's B200; plain tests since then."""
+"""
 import importlib.util
 import os
 

@@ -95,7 +95,7 @@ def main():
             if exch == "peer memory":   # the exchange blocks travel with init_p2p: no communicator is ever created
                 eng.init_p2p(dist)
                 assert eng.prefill_p2p
-            else:                        # the decode areas by hand, then NCCL for the prefill's all-reduce (the round-1 path)
+            else:                        # the decode areas by hand, then NCCL for the prefill's all-reduce (the first path)
                 buf = (C.c_uint8 * 64)()
                 _lib.check(eng.lib.sllm_engine_p2p_export(eng.h, buf))
                 mine = torch.frombuffer(bytearray(buf), dtype=torch.uint8).clone().cuda()

@@ -1,4 +1,4 @@
-// tools/microbench/fusion_probe.cu — three measurements that decide the next step of the decode megakernel (DESIGN.md section 10)
+// tools/microbench/fusion_probe.cu — three measurements that decide the next step of the decode megakernel
 // before any of it is written. Stand-alone (no library): nvcc -gencode arch=compute_100a,code=sm_100a, run on one B200.
 //
 //   1. What does it cost to combine K-split partial vectors with red.global.add.v4.f32 instead of a grid barrier?

@@ -2,7 +2,7 @@
 """tools/prefill_bench.py — time sllm_engine_prefill (tcgen05 GEMMs + block attention) on a shape preset.
 
   python tools/prefill_bench.py [--config llama2-7b] [--tokens 512] [--reps 5] [--bn 0|128|256]
-Prints one JSON line: ms per prefill, prompt tokens/s, algorithmic TFLOP/s (SURVEY.md 8d) and the fraction of the
+Prints one JSON line: ms per prefill, prompt tokens/s, algorithmic TFLOP/s and the fraction of the
 measured dense-bf16 peak (MEASURED_PEAKS.json). Run it under `ncu --metrics gpu__time_duration.sum` for the per-kernel list."""
 import argparse
 import json
