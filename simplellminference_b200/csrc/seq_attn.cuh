@@ -42,11 +42,24 @@ __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], const uint32_t (&a
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// one k-step of a product from zero
+__device__ __forceinline__ void mma_bf16_zero(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                 : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.0f));
+}
 // p = hi + lo with both terms bf16: hi = round(p), lo = round(p - hi)
 __device__ __forceinline__ void split_bf16(float p0, float p1, uint32_t* hi, uint32_t* lo) {
     const uint32_t h = pack_bf16(p0, p1);
     *hi = h;
     *lo = pack_bf16(p0 - __uint_as_float(h << 16), p1 - __uint_as_float(h & 0xffff0000u));
+}
+// v = a + b + c with three bf16 terms
+__device__ __forceinline__ void split3_bf16(float v0, float v1, uint32_t& a, uint32_t& b, uint32_t& c) {
+    a = pack_bf16(v0, v1);
+    const float r0 = v0 - __uint_as_float(a << 16), r1 = v1 - __uint_as_float(a & 0xffff0000u);
+    b = pack_bf16(r0, r1);
+    c = pack_bf16(r0 - __uint_as_float(b << 16), r1 - __uint_as_float(b & 0xffff0000u));
 }
 
 #endif

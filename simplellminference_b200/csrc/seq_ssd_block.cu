@@ -5,13 +5,13 @@
 // and the products C_i . B_j (fp32) are made once per (block, group); step sizes and G once per (block, head).
 // (2) seq_ssd_walk_kernel, CTA = (portion, head, 32 columns), 16 warps: S^T stays in the accumulators (fp32) from the portion's first token to its last,
 // a warp owning 16 columns x an eighth of the states (and of the tokens); it is handed to the others as A fragments through shared memory once per block. Everything is
-// computed transposed (columns are rows), so that accumulators become operands register for register. Every operand is two bf16 terms (x = hi + lo,
-// error <= 2^-17), three products with fp32 accumulation, as in the block form of the delta rule; decays are applied in fp32 to accumulators, to x
-// before it is split and to the C_i . B_j, never to the shared fragments. No factor exceeds 1.
-// Bound: 888 mma per block and CTA (1800 clocks of an SM's tensor pipe) beside 90 KB of fragments from L2; the token-by-token passes over
-// ranges it replaces for portions were bound by fp32 FMAs through shared memory. Measured, 2048 tokens, 64 heads of 64 columns, 128 states: ranges
-// 712 us (249 + 14 + 450), blocks 143 us (18 + 125: a block of the walk takes 3.9 us, some 600 instructions per warp at four warps per scheduler and
-// two barriers; 8 warps of twice the work 137).
+// computed transposed (columns are rows), so that accumulators become operands register for register. Every operand is three bf16 terms (24 bits), of whose
+// products the six largest are kept, with fp32 sums (ssd_mma): the passes over ranges that this replaces for portions work on fp32 products, and the error
+// must not grow. Decays are applied in fp32 to accumulators, to x before it is split and to the C_i . B_j, never to the shared fragments. No factor exceeds 1.
+// Bound: 1776 mma per block and CTA (3600 clocks of an SM's tensor pipe) beside 85 KB of fragments from L2, which are fp32 and split where they are used (three
+// terms would not fit twice). Error of the outputs alone against float64, ranges | blocks: 1.3e-7 | 1.3e-7 at usual decays, 1.7e-6 | 2.4e-7 at memories of
+// thousands of tokens; two terms left 4.5e-6 and 6.1e-6. Measured, 2048 tokens, 64 heads of 64 columns, 128 states: ranges 698 us, blocks 193 us (with two terms 146:
+// the walk 125, with 8 warps of twice the work 137). 2048 tokens of few heads are better off in ranges (8 heads 105 | 185 us).
 #include "seq_attn.cuh"
 #include "seq_ssd_block.cuh"
 
@@ -21,19 +21,13 @@ constexpr int kSsdCols = 32, kSsdThreads = 256, kSsdWalk = 512;      // columns 
 constexpr float kSsdLog2e = 1.4426950408889634f;
 constexpr int kSsdLdx = kSsdCols + 4;                         // padded row of x in shared memory
 
-// fragments of a (block, group): C as [token tile][k-step of states][lane], B as [state tile][k-step of tokens][lane], 16 bytes each: two registers of
-// first terms, two of second ones; the products as [tile of i][k-step of j][lane], four floats each
+// fp32 fragments of a (block, group), four floats per lane: C as [token tile][k-step of states][lane], B as [state tile][k-step of tokens][lane], the
+// products as [tile of i][k-step of j][lane] for the k-steps that hold a j <= i (ssd_w_tile)
 template <int NK> struct SsdGroup {
-    static constexpr int kC = 8 * (NK / 16) * 512, kB = (NK / 8) * 4 * 512, kW = 8 * 4 * 512, kBytes = kC + kB + kW;
+    static constexpr int kC = 8 * (NK / 16) * 512, kB = (NK / 8) * 4 * 512, kW = 20 * 512, kBytes = kC + kB + kW;
 };
+__device__ __forceinline__ int ssd_w_tile(int nt, int ks) { return ((nt + 1) / 2) * ((nt + 2) / 2) + ks; }
 static_assert(SsdGroup<128>::kBytes == ssd_block_group_bytes(128) && SsdGroup<64>::kBytes == ssd_block_group_bytes(64), "scratch sizes");
-
-__device__ __forceinline__ uint4 ssd_frag(float a0, float a1, float b0, float b1) {
-    uint4 r;
-    split_bf16(a0, a1, &r.x, &r.z);
-    split_bf16(b0, b1, &r.y, &r.w);
-    return r;
-}
 
 template <int NK>
 __global__ void __launch_bounds__(kSsdThreads) seq_ssd_prepare_kernel(SsdBlockArgs p, int vec) {
@@ -92,18 +86,26 @@ __global__ void __launch_bounds__(kSsdThreads) seq_ssd_prepare_kernel(SsdBlockAr
     {   // C . B^T, four by four per thread
         const int ti = threadIdx.x >> 4, tj = threadIdx.x & 15;
         float acc[4][4] = {};
-        for (int k = 0; k < NK; k += 4) {
-            float4 cv[4], bv[4];
+        for (int k0 = 0; k0 < NK; k0 += 16) {                // sums of 16 products, then the sum of those: fewer roundings in a row
+            float part[4][4] = {};
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                cv[r] = *reinterpret_cast<const float4*>(s_c + (ti + 16 * r) * ld + k);
-                bv[r] = *reinterpret_cast<const float4*>(s_b + (tj + 16 * r) * ld + k);
+            for (int k = k0; k < k0 + 16; k += 4) {
+                float4 cv[4], bv[4];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    cv[r] = *reinterpret_cast<const float4*>(s_c + (ti + 16 * r) * ld + k);
+                    bv[r] = *reinterpret_cast<const float4*>(s_b + (tj + 16 * r) * ld + k);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        part[i][j] = fmaf(cv[i].x, bv[j].x, fmaf(cv[i].y, bv[j].y, fmaf(cv[i].z, bv[j].z, fmaf(cv[i].w, bv[j].w, part[i][j]))));
             }
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    acc[i][j] = fmaf(cv[i].x, bv[j].x, fmaf(cv[i].y, bv[j].y, fmaf(cv[i].z, bv[j].z, fmaf(cv[i].w, bv[j].w, acc[i][j]))));
+                for (int j = 0; j < 4; ++j) acc[i][j] += part[i][j];
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -115,30 +117,50 @@ __global__ void __launch_bounds__(kSsdThreads) seq_ssd_prepare_kernel(SsdBlockAr
     for (int x = threadIdx.x; x < Group::kC / 16; x += kSsdThreads) {
         const int l = x & 31, g = l >> 2, c = l & 3, ks = (x >> 5) % (NK / 16), nt = (x >> 5) / (NK / 16);
         const float* row = s_c + (nt * 8 + g) * ld + ks * 16 + 2 * c;
-        reinterpret_cast<uint4*>(rec)[x] = ssd_frag(row[0], row[1], row[8], row[9]);
+        reinterpret_cast<float4*>(rec)[x] = make_float4(row[0], row[1], row[8], row[9]);
     }
     for (int x = threadIdx.x; x < Group::kB / 16; x += kSsdThreads) {
         const int l = x & 31, g = l >> 2, c = l & 3, ks = (x >> 5) & 3, nt = x >> 7;
         const float* at = s_b + (ks * 16 + 2 * c) * ld + nt * 8 + g;
-        reinterpret_cast<uint4*>(rec + Group::kC)[x] = ssd_frag(at[0], at[ld], at[8 * ld], at[9 * ld]);
+        reinterpret_cast<float4*>(rec + Group::kC)[x] = make_float4(at[0], at[ld], at[8 * ld], at[9 * ld]);
     }
     __syncthreads();
-    for (int x = threadIdx.x; x < Group::kW / 16; x += kSsdThreads) {
+    for (int x = threadIdx.x; x < 8 * 4 * 32; x += kSsdThreads) {
         const int l = x & 31, g = l >> 2, c = l & 3, ks = (x >> 5) & 3, nt = x >> 7;
+        if (ks > nt / 2) continue;
         const float* row = &s_w[nt * 8 + g][ks * 16 + 2 * c];
-        reinterpret_cast<float4*>(rec + Group::kC + Group::kB)[x] = make_float4(row[0], row[1], row[8], row[9]);
+        reinterpret_cast<float4*>(rec + Group::kC + Group::kB)[ssd_w_tile(nt, ks) * 32 + l] = make_float4(row[0], row[1], row[8], row[9]);
     }
 }
 
-// three products of two-term operands, each into an accumulator of its own
-__device__ __forceinline__ void ssd_mma(float (&d)[3][4], const uint32_t (&ah)[4], const uint32_t (&al)[4], const uint4& f) {
-    mma_bf16_16816(d[0], ah, f.x, f.y);
-    mma_bf16_16816(d[1], al, f.x, f.y);
-    mma_bf16_16816(d[2], ah, f.z, f.w);
+__device__ __forceinline__ bool ssd_finite(float v) { return fabsf(v) <= 3.402823466e38f; }
+
+// A k-step of a product at fp32 accuracy: both operands are three bf16 terms (24 bits), of whose products the six largest are kept (the rest is below 2^-24). The
+// product of the first terms starts from zero and is added to `sum` with ordinary rounding, because the tensor core's own accumulation truncates; the
+// others are 2^8 times smaller and share two accumulators.
+struct SsdTerms { uint32_t h[4], m[4], l[4]; };
+struct SsdSum { float s[4], d[2][4]; };
+__device__ __forceinline__ void ssd_mma(SsdSum& y, const SsdTerms& a, const float4& f) {
+    uint32_t h0, h1, m0, m1, l0, l1;
+    split3_bf16(f.x, f.y, h0, m0, l0);
+    split3_bf16(f.z, f.w, h1, m1, l1);
+    float p[4];
+    mma_bf16_zero(p, a.h, h0, h1);
+    mma_bf16_16816(y.d[0], a.h, m0, m1);
+    mma_bf16_16816(y.d[1], a.m, h0, h1);
+    mma_bf16_16816(y.d[0], a.h, l0, l1);
+    mma_bf16_16816(y.d[1], a.l, h0, h1);
+    mma_bf16_16816(y.d[0], a.m, m0, m1);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) y.s[e] += p[e];
 }
-__device__ __forceinline__ void ssd_load(uint32_t (&r)[4], const uint4* at) {
-    const uint4 v = *at;
-    r[0] = v.x; r[1] = v.y; r[2] = v.z; r[3] = v.w;
+__device__ __forceinline__ float ssd_total(const SsdSum& y, int e) { return y.s[e] + (y.d[0][e] + y.d[1][e]); }
+// the three terms of a fragment lie 32 lanes x 16 bytes apart
+__device__ __forceinline__ void ssd_load(SsdTerms& t, const uint4* at) {
+    const uint4 h = at[0], m = at[32], l = at[64];
+    t.h[0] = h.x; t.h[1] = h.y; t.h[2] = h.z; t.h[3] = h.w;
+    t.m[0] = m.x; t.m[1] = m.y; t.m[2] = m.z; t.m[3] = m.w;
+    t.l[0] = l.x; t.l[1] = l.y; t.l[2] = l.z; t.l[3] = l.w;
 }
 
 template <int NK>
@@ -146,8 +168,8 @@ __global__ void __launch_bounds__(kSsdWalk, 1) seq_ssd_walk_kernel(SsdBlockArgs 
     using Group = SsdGroup<NK>;
     constexpr int kX = kSsdBlock * kSsdLdx * 4, kHead = 3 * kSsdBlock * 4, kStage = Group::kBytes + kX + kHead, kSteps = NK / 16, kEighth = NK / 8, kTiles = kEighth / 8;
     extern __shared__ __align__(16) uint8_t sw_sm[];
-    uint4* s_frag = reinterpret_cast<uint4*>(sw_sm + 2 * kStage);                      // S^T: [column tile][k-step][hi, lo][lane]
-    uint4* x_frag = s_frag + 2 * kSteps * 64;                                         // x^T: [plain, scaled][column tile][k-step][hi, lo][lane]
+    uint4* s_frag = reinterpret_cast<uint4*>(sw_sm + 2 * kStage);                      // S^T: [column tile][k-step][term][lane]
+    uint4* x_frag = s_frag + 2 * kSteps * 96;                                         // x^T: [plain, scaled][column tile][k-step][term][lane]
     const sllm_seq_batch& b = p.b;
     const int seg = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * kSsdCols, grp = h / (p.heads / p.groups);
     const int start = b.seg_start[seg], len = b.seg_len[seg], slot = b.seg_slot[seg], blocks = (len + kSsdBlock - 1) / kSsdBlock;
@@ -198,8 +220,8 @@ __global__ void __launch_bounds__(kSsdWalk, 1) seq_ssd_walk_kernel(SsdBlockArgs 
         __syncthreads();                                     // the block has landed for everyone, and everyone has left the one before
         if (blk + 1 < blocks) issue(blk + 1);
         const uint8_t* rec = sw_sm + (blk & 1) * kStage;
-        const uint4* Cf = reinterpret_cast<const uint4*>(rec) + lane;
-        const uint4* Bf = reinterpret_cast<const uint4*>(rec + Group::kC) + lane;
+        const float4* Cf = reinterpret_cast<const float4*>(rec) + lane;
+        const float4* Bf = reinterpret_cast<const float4*>(rec + Group::kC) + lane;
         const float4* Wf = reinterpret_cast<const float4*>(rec + Group::kC + Group::kB) + lane;
         const float* sx = reinterpret_cast<const float*>(rec + Group::kBytes);
         const float* sG = reinterpret_cast<const float*>(rec + Group::kBytes + kX);
@@ -208,14 +230,15 @@ __global__ void __launch_bounds__(kSsdWalk, 1) seq_ssd_walk_kernel(SsdBlockArgs 
         const float Gn = sG[kSsdBlock - 1], Ln = sL[kSsdBlock - 1];
 #pragma unroll
         for (int nt = 0; nt < kTiles; ++nt) {                // the state as halves of A fragments for all warps
-            uint2 hi, lo;
-            split_bf16(S[nt][0], S[nt][1], &hi.x, &lo.x);
-            split_bf16(S[nt][2], S[nt][3], &hi.y, &lo.y);
+            uint2 t[3];
+            split3_bf16(S[nt][0], S[nt][1], t[0].x, t[1].x, t[2].x);
+            split3_bf16(S[nt][2], S[nt][3], t[0].y, t[1].y, t[2].y);
             const int tile = qu * kTiles + nt;
-            uint2* at = reinterpret_cast<uint2*>(s_frag + (ct * kSteps + tile / 2) * 64 + lane) + tile % 2;
-            at[0] = hi;
-            at[64] = lo;
+            uint2* at = reinterpret_cast<uint2*>(s_frag + (ct * kSteps + tile / 2) * 96 + lane) + tile % 2;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) at[64 * i] = t[i];
         }
+        bool wild = false;                                   // a value is infinite or no number
         {                                                    // x^T as A fragments: a plain one or one decayed to the block's end per thread
             const int ks = qu & 3, scaled = qu >> 2;
             const float* at = sx + (ks * 16 + 2 * c) * kSsdLdx + cl;
@@ -227,74 +250,100 @@ __global__ void __launch_bounds__(kSsdWalk, 1) seq_ssd_walk_kernel(SsdBlockArgs 
                 v[2 * i] = at[((i & 1) + 8 * (i >> 1)) * kSsdLdx] * f;
                 v[2 * i + 1] = at[((i & 1) + 8 * (i >> 1)) * kSsdLdx + 8] * f;
             }
-            uint4* to = x_frag + (scaled * 8 + ct * 4 + ks) * 64 + lane;
-            uint4 hi, lo;
-            split_bf16(v[0], v[2], &hi.x, &lo.x);
-            split_bf16(v[1], v[3], &hi.y, &lo.y);
-            split_bf16(v[4], v[6], &hi.z, &lo.z);
-            split_bf16(v[5], v[7], &hi.w, &lo.w);
-            to[0] = hi;
-            to[32] = lo;
+            // such a value would reach tokens before its own through the weights of zero that hide it from them: it is added by itself below
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (!ssd_finite(v[i])) {
+                    wild = true;
+                    v[i] = 0.0f;
+                }
+            uint4* to = x_frag + (scaled * 8 + ct * 4 + ks) * 96 + lane;
+            uint4 t[3];
+            split3_bf16(v[0], v[2], t[0].x, t[1].x, t[2].x);
+            split3_bf16(v[1], v[3], t[0].y, t[1].y, t[2].y);
+            split3_bf16(v[4], v[6], t[0].z, t[1].z, t[2].z);
+            split3_bf16(v[5], v[7], t[0].w, t[1].w, t[2].w);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) to[32 * i] = t[i];
         }
-        __syncthreads();
+        wild = __syncthreads_or(wild);
         // outputs: columns of tile ct, tokens qu * 8 + 2c, + 1
-        float y[3][4] = {};
+        SsdSum y = {};
 #pragma unroll
         for (int ks = 0; ks < kSteps; ++ks) {
-            uint32_t ah[4], al[4];
-            ssd_load(ah, s_frag + (ct * kSteps + ks) * 64 + lane);
-            ssd_load(al, s_frag + (ct * kSteps + ks) * 64 + 32 + lane);
-            ssd_mma(y, ah, al, Cf[(qu * kSteps + ks) * 32]);
+            SsdTerms a;
+            ssd_load(a, s_frag + (ct * kSteps + ks) * 96 + lane);
+            ssd_mma(y, a, Cf[(qu * kSteps + ks) * 32]);
         }
         {
             const float2 G2 = *reinterpret_cast<const float2*>(sG + qu * 8 + 2 * c), L2 = *reinterpret_cast<const float2*>(sL + qu * 8 + 2 * c);
-            const float e0 = exp2f(G2.x + L2.x), e1 = exp2f(G2.y + L2.y);
+            const float e[2] = {exp2f(G2.x + L2.x), exp2f(G2.y + L2.y)};
 #pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                y[q][0] *= e0;
-                y[q][1] *= e1;
-                y[q][2] *= e0;
-                y[q][3] *= e1;
+            for (int q = 0; q < 4; ++q) {
+                y.s[q] *= e[q & 1];
+                y.d[0][q] *= e[q & 1];
+                y.d[1][q] *= e[q & 1];
             }
         }
         const int i = qu * 8 + g;
         const float Gi = sG[i], Li = sL[i];
         for (int ks = 0; ks <= qu / 2; ++ks) {               // tokens j up to these
-            uint32_t ah[4], al[4];
-            ssd_load(ah, x_frag + (ct * 4 + ks) * 64 + lane);
-            ssd_load(al, x_frag + (ct * 4 + ks) * 64 + 32 + lane);
+            SsdTerms a;
+            ssd_load(a, x_frag + (ct * 4 + ks) * 96 + lane);
             const int j = ks * 16 + 2 * c;
             const float2 Ga = *reinterpret_cast<const float2*>(sG + j), Gb = *reinterpret_cast<const float2*>(sG + j + 8);
             const float2 La = *reinterpret_cast<const float2*>(sL + j), Lb = *reinterpret_cast<const float2*>(sL + j + 8);
             const float2 da = *reinterpret_cast<const float2*>(sd + j), db = *reinterpret_cast<const float2*>(sd + j + 8);
-            const float4 w = Wf[(qu * 4 + ks) * 32];
+            const float4 w = Wf[ssd_w_tile(qu, ks) * 32];
             const float w0 = j <= i ? w.x * (exp2f((Gi - Ga.x) + (Li - La.x)) * da.x) : 0.0f, w1 = j + 1 <= i ? w.y * (exp2f((Gi - Ga.y) + (Li - La.y)) * da.y) : 0.0f;
             const float w2 = j + 8 <= i ? w.z * (exp2f((Gi - Gb.x) + (Li - Lb.x)) * db.x) : 0.0f, w3 = j + 9 <= i ? w.w * (exp2f((Gi - Gb.y) + (Li - Lb.y)) * db.y) : 0.0f;
-            ssd_mma(y, ah, al, ssd_frag(w0, w1, w2, w3));
+            ssd_mma(y, a, make_float4(w0, w1, w2, w3));
+        }
+        if (wild) {
+            const float* W = reinterpret_cast<const float*>(rec + Group::kC + Group::kB);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int tok = qu * 8 + 2 * c + (e & 1);
+                for (int j = 0; j <= tok; ++j) {
+                    const float v = sx[j * kSsdLdx + cl + (e < 2 ? 0 : 8)];
+                    if (ssd_finite(v)) continue;
+                    const float w = W[(ssd_w_tile(qu, j / 16) * 32 + (tok & 7) * 4 + j % 8 / 2) * 4 + j % 16 / 8 * 2 + j % 2];
+                    y.s[e] = fmaf(w * (exp2f((sG[tok] - sG[j]) + (sL[tok] - sL[j])) * sd[j]), v, y.s[e]);
+                }
+            }
         }
         const int n = min(kSsdBlock, len - blk * kSsdBlock);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int tok = qu * 8 + 2 * c + (e & 1);
             if (tok < n && (e < 2 ? ok0 : ok1))
-                p.y[(size_t)(start + blk * kSsdBlock + tok) * p.ldy + (size_t)h * p.dv + (e < 2 ? r0 : r1)] =
-                    fmaf(skip, sx[tok * kSsdLdx + cl + (e < 2 ? 0 : 8)], y[0][e] + (y[1][e] + y[2][e]));
+                p.y[(size_t)(start + blk * kSsdBlock + tok) * p.ldy + (size_t)h * p.dv + (e < 2 ? r0 : r1)] = fmaf(skip, sx[tok * kSsdLdx + cl + (e < 2 ? 0 : 8)], ssd_total(y, e));
         }
         // the state
         const float dn = exp2f(Gn + Ln);
-        float add[kTiles][3][4] = {};
+        SsdSum add[kTiles] = {};
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) {
-            uint32_t ah[4], al[4];
-            ssd_load(ah, x_frag + (2 * 4 + ct * 4 + ks) * 64 + lane);
-            ssd_load(al, x_frag + (2 * 4 + ct * 4 + ks) * 64 + 32 + lane);
+            SsdTerms a;
+            ssd_load(a, x_frag + (2 * 4 + ct * 4 + ks) * 96 + lane);
 #pragma unroll
-            for (int nt = 0; nt < kTiles; ++nt) ssd_mma(add[nt], ah, al, Bf[((qu * kTiles + nt) * 4 + ks) * 32]);
+            for (int nt = 0; nt < kTiles; ++nt) ssd_mma(add[nt], a, Bf[((qu * kTiles + nt) * 4 + ks) * 32]);
+        }
+        if (wild) {
+            const float* B = reinterpret_cast<const float*>(rec + Group::kC);
+#pragma unroll
+            for (int nt = 0; nt < kTiles; ++nt)
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    for (int j = 0; j < n; ++j) {
+                        const float f = exp2f((Gn - sG[j]) + (Ln - sL[j])) * sd[j], v = sx[j * kSsdLdx + cl + (e < 2 ? 0 : 8)] * f;
+                        if (!ssd_finite(v)) add[nt].s[e] = fmaf(B[(((qu * kTiles + nt) * 4 + j / 16) * 32 + (2 * c + (e & 1)) * 4 + j % 8 / 2) * 4 + j % 16 / 8 * 2 + j % 2], v, add[nt].s[e]);
+                    }
         }
 #pragma unroll
         for (int nt = 0; nt < kTiles; ++nt)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) S[nt][e] = fmaf(dn, S[nt][e], add[nt][0][e] + (add[nt][1][e] + add[nt][2][e]));
+            for (int e = 0; e < 4; ++e) S[nt][e] = fmaf(dn, S[nt][e], ssd_total(add[nt], e));
     }
 #pragma unroll
     for (int nt = 0; nt < kTiles; ++nt)
@@ -312,7 +361,7 @@ static int launch_ssd(SsdBlockArgs p, cudaStream_t st) {
     const int vec_prep = p.n_state % 4 == 0 && p.ldb % 4 == 0 && p.ldc % 4 == 0 && aligned(p.B) && aligned(p.C);
     const int vec = p.dv % 4 == 0 && p.ldx % 4 == 0 && aligned(p.x);
     constexpr int smem_prep = (2 * kSsdBlock * (NK + 4) + kSsdBlock * (kSsdBlock + 1)) * 4;
-    constexpr int smem = 2 * (Group::kBytes + kSsdBlock * kSsdLdx * 4 + 3 * kSsdBlock * 4) + 2 * (NK / 16) * 64 * 16 + 2 * 2 * 4 * 64 * 16;
+    constexpr int smem = 2 * (Group::kBytes + kSsdBlock * kSsdLdx * 4 + 3 * kSsdBlock * 4) + 2 * (NK / 16) * 96 * 16 + 2 * 2 * 4 * 96 * 16;
     static bool sized = false;
     if (!sized) {
         SLLM_CUDA(cudaFuncSetAttribute(seq_ssd_prepare_kernel<NK>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_prep));

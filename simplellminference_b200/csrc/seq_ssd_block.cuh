@@ -20,6 +20,6 @@ struct SsdBlockArgs {
 // number of a portion's block in the scratch; portions follow each other with room for a last half block
 __host__ __device__ __forceinline__ size_t ssd_block_id(int seg_tile0, int seg, int blk) { return (size_t)(seg_tile0 / 2 + seg + blk); }
 inline size_t ssd_block_count(int n_qtiles, int nseg) { return (size_t)(n_qtiles / 2 + nseg + 1); }
-constexpr size_t ssd_block_group_bytes(int nk) { return (size_t)8 * (nk / 16) * 512 + (size_t)(nk / 8) * 4 * 512 + 8 * 4 * 512; }
+constexpr size_t ssd_block_group_bytes(int nk) { return (size_t)8 * (nk / 16) * 512 + (size_t)(nk / 8) * 4 * 512 + 20 * 512; }
 
 }  // namespace sllm
