@@ -9,11 +9,13 @@
 //   warp 1 (one lane)   MMA issuer: S = Q K^T (both K-major) into TMEM; O += P V with P read from TMEM, V as the MN-major operand as it lies;
 //   warps 4-7, 8-11     softmax of tile 0 / 1, a thread per query row: tcgen05.ld the scores (once for the maximum, the second half once more for the
 //                       weights), exponentials in powers of two, weights packed as bf16 over the scores' own TMEM columns. O stays in TMEM and is
-//                       rescaled only when a row's maximum has grown by more than 2^8 since its last reference (the weights are relative to that
-//                       reference, so the result is the same), sums in fp32.
+//                       rescaled whenever the maximum of one of the warp's rows has grown: a row's largest weights, which decide its error, are then
+//                       rounded to bf16 next to 1, where they lose least, and their sum is that of the rounded ones. (With a reference that lagged by up to
+//                       2^8 and the sum of the unrounded ones the result was off by 2.34e-3 instead of 2.29e-3 on the case below and by 2.12e-3 instead
+//                       of 1.72e-3 with scores four times as wide; mma.sync 2.29e-3 and 1.73e-3.)
 // TMEM: S0 | S1 | O0 | O1, 128 columns each. Bound: the tensor pipe and the exponentials, 1024 clocks each per pair of 128 x 128 tiles at head_dim 128;
 // mma.sync, which it replaces for bf16 caches, spent them one after the other in the same warps. Measured, 2048 queries behind 6144 positions, 32 heads
-// over 8 of 128: 350 us, 687 TFLOP/s (mma.sync 1062 us, 227); 256 CTAs on 148 SMs leave a last wave of 108.
+// over 8 of 128: 390 us, 617 TFLOP/s (mma.sync 1061 us, 227; with the lagging reference 348); 256 CTAs on 148 SMs leave a last wave of 108.
 #include "prefill.cuh"
 #include "tcgen05.cuh"
 
@@ -189,7 +191,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
                 const float mx = fmaxf(m0, m1) * p.scale_log2;
                 if (kt == 0) {
                     ref = mx;
-                } else if (__any_sync(0xffffffffu, mx > ref + 8.0f)) {            // the product before this one has completed: these scores follow it
+                } else if (__any_sync(0xffffffffu, mx > ref)) {                   // the product before this one has completed: these scores follow it
                     const float nr = fmaxf(ref, mx), f = tc_exp2(ref - nr);
                     l *= f;
                     ref = nr;
@@ -213,9 +215,9 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
                             x = c0 + i <= seen ? x : 0.0f;
                             y = c0 + i + 1 <= seen ? y : 0.0f;
                         }
-                        l0 += x;
-                        l1 += y;
                         w[i / 2] = tc_pack(x, y);
+                        l0 += __uint_as_float(w[i / 2] << 16);                    // the weights as they are used
+                        l1 += __uint_as_float(w[i / 2] & 0xffff0000u);
                     }
                     tc_st16(s_tmem + c0 / 2, w);
                 };
