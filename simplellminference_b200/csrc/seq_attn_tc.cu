@@ -3,25 +3,29 @@
 // The tensor-core body of seq_attn.cu keeps a warp's 16 queries in its registers and stages tiles of 32 keys for 64 rows; here 128 rows = the query heads
 // of a kv head (four, two or one) x 32, 64 or 128 neighbouring queries share tiles of 64 keys, and two CTAs per SM hide each other's softmax.
 //   warps 0-3  softmax, a thread per row: q to bf16 rows in shared memory once; per tile the scores from TMEM, capped / charged / masked as the
-//              launch asks, fp32 maximum and sum; the weights go back over the scores' TMEM columns as TWO bf16 terms (p = hi + lo), as in that
-//              body, so that the product with the values keeps them to 2^-17. O stays in TMEM and is rescaled only when a row's maximum has
-//              grown by more than ln 2^8 since its last reference.
+//              launch asks, fp32 maximum and sum; the weights go back to TMEM, over the scores and the columns behind them, as THREE bf16 terms
+//              (24 bits; that body's two leave 2^-18). O stays in TMEM and is rescaled only when a row's maximum has grown by more than 2^8 since its last
+//              reference. The tensor core truncates as it accumulates, so every kSaFlush tiles O is added, with ordinary rounding, to the row's place in
+//              the scratch. Error of the result, that body | this one: 1.7e-6 | 8e-7 on prompts of up to 1000 tokens, 3.1e-6 | 1.5e-6 on one of 4096,
+//              9.3e-6 | 2.7e-6 on 256 tokens behind 4000. (Two terms, nothing flushed: 1.84e-6, 3.3e-6, 9.4e-6 in 45, 372 and 258 us instead of 54, 468 and 339.)
 //   warp 4     (one lane) TMA producer: boxes of 32 positions, looked up in the block table; boxes behind the portion's last position lie
 //              outside the tensor map and read as zeros;
-//   warp 5     (one lane) tcgen05.mma issuer: S = Q K^T, O += hi V + lo V with the weights read from TMEM, V MN-major as it lies;
+//   warp 5     (one lane) tcgen05.mma issuer: S = Q K^T, O += (hi + mid + lo) V with the weights read from TMEM, V MN-major as it lies;
 //   warp 6     zeros the value rows between the last position and the end of its box (the pool may hold anything there).
-// Bound: the fp32 work per score; the tensor pipe needs 768 clocks per 128 x 64 scores at heads of 128. Caps and charges are applied in loops of
-// their own: with tanhf and log1pf inlined 64 times the code left the instruction cache (210 us where the loops take 74). Measured: attention_run.
+// Bound: the fp32 work per score; the tensor pipe needs 1024 clocks per 128 x 64 scores at heads of 128. Caps and charges are applied in loops of
+// their own: with tanhf and log1pf inlined 64 times the code left the instruction cache (210 us where the loops take 81). Measured: attention_run.
 #include "seq_attn_decode.cuh"
 #include "tcgen05.cuh"
 
 namespace sllm {
 
 constexpr int kSaRows = 128, kSaKeys = 64, kSaThreads = 256, kSaBox = 32;
-constexpr uint32_t kSaTmem = 256;        // scores / weights at 0, O at 128; two CTAs share an SM's 512 columns
+constexpr int kSaFlush = 12;             // tiles between two flushes of O: from there on three terms' products would be further off than that body's two
+constexpr uint32_t kSaTmem = 256;        // scores at 0 .. 63, then the weights' terms at 0 .. 95, O at 128; two CTAs share an SM's 512 columns
 constexpr float kSaLog2e = 1.4426950408889634f;
 
-// tanh to 5e-7 of its value without a branch: 1 - 2 / (1 + e^2|x|), and below 1/4, where that cancels, the Taylor series to x^9 (remainder 0.0089 x^11)
+// tanh to 1e-6 of its value without a branch: 1 - 2 / (1 + e^2|x|), and below 1/4, where that cancels, the Taylor series to x^9 (remainder 0.0089 x^11). The worst
+// place is just above 1/4: the documented errors of ex2.approx (2^-22) and rcp.approx (1 ulp) and the rounding of 1 + e leave 2.2e-7 of a result of 0.245.
 __device__ __forceinline__ float sa_tanh(float x) {
     const float a = fabsf(x), x2 = x * x;
     float r;
@@ -33,6 +37,17 @@ __device__ __forceinline__ float sa_log2(float x) {
     float y;
     asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
+}
+
+__device__ __forceinline__ void sa_ld16(uint32_t taddr, uint32_t* o) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(o[0]), "=r"(o[1]), "=r"(o[2]), "=r"(o[3]), "=r"(o[4]), "=r"(o[5]), "=r"(o[6]), "=r"(o[7]), "=r"(o[8]), "=r"(o[9]), "=r"(o[10]), "=r"(o[11]),
+                   "=r"(o[12]), "=r"(o[13]), "=r"(o[14]), "=r"(o[15])
+                 : "r"(taddr)
+                 : "memory");
+    tc_wait_ld();
+#pragma unroll
+    for (int e = 0; e < 16; ++e) asm volatile("" : "+r"(o[e]));
 }
 
 template <int HD>
@@ -132,8 +147,8 @@ __global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const _
                 tc_fence_after();
                 const uint8_t* v = sV + (i % ST) * Sh::kTile;
 #pragma unroll
-                for (int ks = 0; ks < 2 * kSaKeys / 16; ++ks)                    // first terms, then second ones, against the same values
-                    tc_mma_bf16_ts(tmem + 128, tmem + 8 * ks, umma_desc_mn_sw128(v + (ks % (kSaKeys / 16)) * 16 * 128, Sh::kKBlock), idesc_o, (i | ks) != 0);
+                for (int ks = 0; ks < 3 * kSaKeys / 16; ++ks)                    // first terms, then second ones, then third ones, against the same values
+                    tc_mma_bf16_ts(tmem + 128, tmem + 8 * ks, umma_desc_mn_sw128(v + (ks % (kSaKeys / 16)) * 16 * 128, Sh::kKBlock), idesc_o, (i % kSaFlush | ks) != 0);
                 tc_commit(odone);
                 tc_commit(vempty + i % ST);
                 if (i + 1 < n) {        // the next scores land where the weights lie that this product is still reading
@@ -178,7 +193,58 @@ __global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const _
         const uint32_t s_tmem = tmem + ((uint32_t)(warp * 32) << 16), o_tmem = s_tmem + 128;
         const int wnd = seq_row_window(qpos, p.window, p.chunk);
         const float slope = kOpts && p.slopes ? p.slopes[h] : 0.0f, r1 = kOpts && p.logdist ? p.logdist[h] : 0.0f, r2 = kOpts && p.logdist ? p.logdist[p.heads + h] : 0.0f;
-        float ref = -INFINITY, l = 0.0f;            // what the weights are relative to; their sum
+        // Weights are 2^(score * mul - ref): one rounding between a score and its exponential. Without caps or charges mul holds the scale, too.
+        const bool plain = !kOpts && p.scale > 0.0f;
+        const float mul = plain ? p.scale * kSaLog2e : kSaLog2e;
+        float ref = -INFINITY, l = 0.0f, flushed = -INFINITY;      // what the weights are relative to; their sum; the reference of what has been flushed
+        const int rows = min(32, (nq << sa.hpc_log2) - warp * 32);
+        // the records of this warp's rows, and how far the next head's and the next query's are
+        float* recs = p.ws + (((size_t)tok0 * p.heads + h0) * p.nsplit + split) * (HD + 2);
+        const int rec_h = p.nsplit * (HD + 2), rec_q = p.heads * rec_h;
+        auto rec_of = [&](int r) { return recs + (size_t)(uint32_t)(((warp * 32 + r) >> sa.hpc_log2) * rec_q + ((warp * 32 + r) & (sa.hpc - 1)) * rec_h); };
+        // Where this row's sums are flushed to, 16 columns at a time. Rows of its own when a record follows; when the result does, all the records of the query's heads are
+        // free, and the heads' lanes take turns of 16 bytes there so that a store covers whole sectors.
+        const bool direct = p.out || p.out16;
+        const int turn = direct ? sa.hpc : 1, hh = row & (sa.hpc - 1);
+        float* place = direct ? reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(rec_of(lane) - hh * rec_h) + 15) & ~(uintptr_t)15) + 4 * hh : rec_of(lane) + 2;
+        auto prefetch_flushed = [&]() {
+            const float* line = direct ? place - 4 * hh + hh * HD : place;
+#pragma unroll
+            for (int c = 0; c < HD; c += 32) asm volatile("prefetch.global.L1 [%0];" ::"l"(line + c));
+        };
+        auto store_flushed = [&](const uint32_t* o, int c) {
+#pragma unroll
+            for (int e = 0; e < 16; e += 4) {
+                float* at = place + (c + e) * turn;
+                if (direct) {
+                    *reinterpret_cast<uint4*>(at) = make_uint4(o[e], o[e + 1], o[e + 2], o[e + 3]);
+                } else {
+                    *reinterpret_cast<uint2*>(at) = make_uint2(o[e], o[e + 1]);
+                    *reinterpret_cast<uint2*>(at + 2) = make_uint2(o[e + 2], o[e + 3]);
+                }
+            }
+        };
+        auto add_flushed = [&](uint32_t* o, int c) {        // carried over to the present reference
+            const float f = flushed == ref ? 1.0f : tc_exp2(flushed - ref);
+            float4 w[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float* at = place + (c + 4 * e) * turn;
+                if (direct) {
+                    w[e] = *reinterpret_cast<const float4*>(at);
+                } else {
+                    const float2 a = *reinterpret_cast<const float2*>(at), b2 = *reinterpret_cast<const float2*>(at + 2);
+                    w[e] = make_float4(a.x, a.y, b2.x, b2.y);
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                o[4 * e] = __float_as_uint(fmaf(w[e].x, f, __uint_as_float(o[4 * e])));
+                o[4 * e + 1] = __float_as_uint(fmaf(w[e].y, f, __uint_as_float(o[4 * e + 1])));
+                o[4 * e + 2] = __float_as_uint(fmaf(w[e].z, f, __uint_as_float(o[4 * e + 2])));
+                o[4 * e + 3] = __float_as_uint(fmaf(w[e].w, f, __uint_as_float(o[4 * e + 3])));
+            }
+        };
         bool ok = true;
         for (int i = 0; i < n; ++i) {
             const int j0 = tiles.tile_of(split + i * p.nsplit) * kSaKeys;
@@ -196,7 +262,7 @@ __global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const _
                 const float inv = p.scale / p.softcap;
 #pragma unroll
                 for (int e = 0; e < 64; ++e) s[e] = __float_as_uint(p.softcap * sa_tanh(__uint_as_float(s[e]) * inv));
-            } else {
+            } else if (!plain) {
 #pragma unroll
                 for (int e = 0; e < 64; ++e) s[e] = __float_as_uint(__uint_as_float(s[e]) * p.scale);
             }
@@ -221,24 +287,31 @@ __global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const _
                 m0 = fmaxf(m0, __uint_as_float(s[e]));
                 m1 = fmaxf(m1, __uint_as_float(s[e + 1]));
             }
-            const float mx = fmaxf(m0, m1);
+            const float mx = fmaxf(m0, m1) * mul;
+            if (i % kSaFlush == 0 && i > 0) {           // the product before this tile has completed: these scores follow it
+                if (live && i > kSaFlush) prefetch_flushed();
+#pragma unroll 1
+                for (int c = 0; c < HD; c += 16) {
+                    uint32_t o[16];
+                    sa_ld16(o_tmem + c, o);
+                    if (live) {
+                        if (i > kSaFlush) add_flushed(o, c);
+                        store_flushed(o, c);
+                    }
+                    __syncwarp();
+                }
+                flushed = ref;
+            }
             if (i == 0) {
                 ref = mx;
-            } else if (__any_sync(0xffffffffu, mx > ref + 5.5f)) {              // the product before this one has completed: these scores follow it
-                const float nr = fmaxf(ref, mx), f = nr == -INFINITY ? 1.0f : tc_exp2((ref - nr) * kSaLog2e);
+            } else if (__any_sync(0xffffffffu, mx > ref + 8.0f)) {
+                const float nr = fmaxf(ref, mx), f = nr == ref ? 1.0f : tc_exp2(ref - nr);
                 l *= f;
                 ref = nr;
 #pragma unroll 1
                 for (int c = 0; c < HD; c += 16) {
                     uint32_t o[16];
-                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                                 : "=r"(o[0]), "=r"(o[1]), "=r"(o[2]), "=r"(o[3]), "=r"(o[4]), "=r"(o[5]), "=r"(o[6]), "=r"(o[7]), "=r"(o[8]), "=r"(o[9]), "=r"(o[10]), "=r"(o[11]),
-                                   "=r"(o[12]), "=r"(o[13]), "=r"(o[14]), "=r"(o[15])
-                                 : "r"(o_tmem + c)
-                                 : "memory");
-                    tc_wait_ld();
-#pragma unroll
-                    for (int e = 0; e < 16; ++e) asm volatile("" : "+r"(o[e]));
+                    sa_ld16(o_tmem + c, o);
 #pragma unroll
                     for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * f);
                     tc_st16(o_tmem + c, o);
@@ -248,36 +321,43 @@ __global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const _
             const float from = ref == -INFINITY ? 0.0f : ref;                   // nothing seen yet: every weight is exp(-inf) = 0
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
-                uint32_t hi[16], lo[16];
+                uint32_t hi[16], mid[16], lo[16];
 #pragma unroll
                 for (int e = 0; e < 16; ++e) {
-                    const float x = tc_exp2((__uint_as_float(s[half * 32 + 2 * e]) - from) * kSaLog2e), y = tc_exp2((__uint_as_float(s[half * 32 + 2 * e + 1]) - from) * kSaLog2e);
+                    const float x = tc_exp2(fmaf(__uint_as_float(s[half * 32 + 2 * e]), mul, -from)), y = tc_exp2(fmaf(__uint_as_float(s[half * 32 + 2 * e + 1]), mul, -from));
                     l0 += x;
                     l1 += y;
                     hi[e] = tc_pack(x, y);
-                    lo[e] = tc_pack(x - __uint_as_float(hi[e] << 16), y - __uint_as_float(hi[e] & 0xffff0000u));
+                    const float rx = x - __uint_as_float(hi[e] << 16), ry = y - __uint_as_float(hi[e] & 0xffff0000u);
+                    mid[e] = tc_pack(rx, ry);
+                    lo[e] = tc_pack(rx - __uint_as_float(mid[e] << 16), ry - __uint_as_float(mid[e] & 0xffff0000u));
                 }
                 tc_st16(s_tmem + half * 16, hi);
-                tc_st16(s_tmem + 32 + half * 16, lo);
+                tc_st16(s_tmem + 32 + half * 16, mid);
+                tc_st16(s_tmem + 64 + half * 16, lo);
             }
             l += l0 + l1;
             tc_wait_st();
             tc_fence_before();
             mb_arrive(pready);
         }
+        if (live && n > kSaFlush) prefetch_flushed();
         if (ok && n > 0) ok = tc_wait(odone, (uint32_t)(n - 1) & 1, gave_up);
         tc_fence_after();
-        const bool direct = p.out || p.out16;
-        const float inv = direct ? 1.0f / l : 1.0f;
+        float inv = direct ? 1.0f / l : 1.0f;
         const int t = tok0 + qi;
-        float* rec = direct ? nullptr : p.ws + (((size_t)t * p.heads + h) * p.nsplit + split) * (HD + 2);
         if (ok && live && !direct) {
-            rec[0] = ref;
-            rec[1] = l;
+            // the reference as a logarithm to the base e, and what its rounding leaves of it in the sums
+            constexpr float ln2 = 0.693147181f, ln2_rest = -1.90465421e-9f;
+            const float m = ref * ln2;
+            if (ref != -INFINITY) inv = 1.0f + fmaf(ref, ln2_rest, fmaf(ref, ln2, -m));
+            rec_of(lane)[0] = m;
+            rec_of(lane)[1] = l * inv;
         }
+        float* mine = reinterpret_cast<float*>(smem) + warp * (32 * 33);        // the rings' place: every tile has been read
         // fp32 results: where this lane's column of the first row goes, and how far the next query and the next head are
-        float* to = lane + (p.out ? p.out + (size_t)tok0 * p.ldo + (size_t)h0 * HD : p.ws + (((size_t)tok0 * p.heads + h0) * p.nsplit + split) * (HD + 2) + 2);
-        const int step_h = p.out ? HD : p.nsplit * (HD + 2), step_q = p.out ? p.ldo : p.heads * step_h;
+        float* to = lane + (p.out ? p.out + (size_t)tok0 * p.ldo + (size_t)h0 * HD : recs + 2);
+        const int step_h = p.out ? HD : rec_h, step_q = p.out ? p.ldo : rec_q;
 #pragma unroll 1
         for (int c = 0; ok && c < HD; c += 32) {
             uint32_t o[32];
@@ -288,6 +368,11 @@ __global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const _
 #pragma unroll
                 for (int e = 0; e < 32; ++e) o[e] = 0u;
             }
+            if (n > kSaFlush && live) {
+                add_flushed(o, c);
+                add_flushed(o + 16, c + 16);
+            }
+            __syncwarp();
 #pragma unroll
             for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * inv);
             if (live && p.out16) {
@@ -298,13 +383,11 @@ __global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const _
                     dst[x] = make_uint4(two(0), two(2), two(4), two(6));
                 }
             }
-            if (p.out || !direct) {     // fp32 rows: through shared memory (the rings' place, every tile has been read), so that a store covers neighbouring columns of one row
-                float* mine = reinterpret_cast<float*>(smem) + warp * (32 * 33);
+            if (p.out || !direct) {     // fp32 rows: through shared memory, so that a store covers neighbouring columns of one row
                 __syncwarp();
 #pragma unroll
                 for (int e = 0; e < 32; ++e) mine[lane * 33 + e] = __uint_as_float(o[e]);
                 __syncwarp();
-                const int rows = min(32, (nq << sa.hpc_log2) - warp * 32);
 #pragma unroll 8
                 for (int r = 0; r < 32; ++r)
                     if (r < rows) {
