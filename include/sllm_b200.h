@@ -44,12 +44,16 @@ extern "C" {
 #define SLLM_ENOMEM (-3)   /* device allocation failed */
 #define SLLM_ESTATE (-4)   /* call sequence error (e.g. decode before weights are loaded) */
 #define SLLM_ECOMM (-5)    /* NCCL / peer-memory error */
+#define SLLM_ETIMEOUT (-6) /* a kernel gave up a bounded wait: results of an earlier launch are incomplete */
 
 enum { SLLM_F32 = 0, SLLM_BF16 = 1, SLLM_INT8 = 2 };
 
 typedef void* sllm_stream_t;
 
 const char* sllm_last_error(void);
+/* SLLM_ETIMEOUT, once, after a kernel of this library has given up one of its bounded waits (its result rows are then unwritten), else SLLM_OK. Every call
+ * that launches kernels or waits for them reports the same, so a program needs this only behind a synchronisation of its own. */
+int sllm_status(void);
 int sllm_abi_version(void);
 /* development knobs (not part of the drop-in surface): key 0 = GEMV CTAs per SM (0 = built-in choice); prefill GEMM: key 1 = force
  * the N extent of a tile (multiple of 32, 0 = cost model), key 2 = two-SM tiles (1 / 0 force / forbid, -1 = by T), key 3 = programmatic
@@ -59,7 +63,8 @@ int sllm_abi_version(void);
  * are live than whole rows fit shared memory, so that Wdown is read once (all 0 by default: experimental until measured); key 8 = decode
  * megakernel MEASUREMENT aid, results are garbage: bit 0 = skip the grid barriers, bit 1 = skip the dot products,
  * bit 4 = tensor-parallel prefill without its peer-memory exchanges (the GEMM / attention time alone); key 9 = ragged-batch attention
- * (sllm_seq_attention): 1 (default) tensor-core body for bf16 pools on steps that hold a prompt portion, 0 = always the fp32 body */
+ * (sllm_seq_attention): 1 (default) tensor-core body for bf16 pools on steps that hold a prompt portion, 0 = always the fp32 body;
+ * key 10 = polls after which a wait inside the tcgen05 attention kernels is given up (default 2^24, seconds; 0 gives up at once: for tests of the report) */
 int sllm_tune(int32_t key, int32_t value);
 /* device facts the host side sizes things by: sm count, max opt-in shared memory per block, total/free HBM */
 int sllm_device_info(int32_t* sm_count, int32_t* smem_optin_bytes, size_t* hbm_total, size_t* hbm_free);

@@ -32,7 +32,7 @@ class EngineConfig(C.Structure):
 ENGINE_UNFUSED, ENGINE_NO_GRAPH, ENGINE_PDL, ENGINE_P2P_ALLREDUCE, ENGINE_MEGAKERNEL, ENGINE_MEGA_LL = 1, 2, 4, 8, 16, 32
 ENGINE_MEGA_FUSE_DOWN = 64
 ENGINE_MEGA_V2 = 128
-EINVAL, ENOTSUP, ENOMEM, ESTATE, ECOMM = -1, -2, -3, -4, -5   # SLLM_E* of include/sllm_b200.h
+EINVAL, ENOTSUP, ENOMEM, ESTATE, ECOMM, ETIMEOUT = -1, -2, -3, -4, -5, -6   # SLLM_E* of include/sllm_b200.h
 
 _P = C.c_void_p
 _I = C.c_int32
@@ -42,6 +42,7 @@ _F = C.c_float
 # name -> (restype, argtypes); every symbol include/sllm_b200.h declares
 SIGNATURES = {
     "sllm_last_error": (C.c_char_p, []),
+    "sllm_status": (C.c_int, []),
     "sllm_abi_version": (C.c_int, []),
     "sllm_tune": (C.c_int, [_I, _I]),
     "sllm_device_info": (C.c_int, [C.POINTER(_I), C.POINTER(_I), C.POINTER(C.c_size_t), C.POINTER(C.c_size_t)]),
@@ -196,7 +197,7 @@ SIGNATURES.update({
 # sllm_seq_* kernels, the tensor-core GEMM, the page bookkeeping, the sampler): a model made of those blocks then needs seventeen
 # translation units compiled, not all of them. The full library contains the same objects and is preferred when it exists.
 SEQ_LIB_PATH = os.path.join(HERE, "lib", "libsllm_b200_seq.so")
-SEQ_SYMBOL_PREFIXES = ("sllm_seq_", "sllm_kvpages_", "sllm_sample_", "sllm_last_error", "sllm_abi_version", "sllm_tune", "sllm_device_info",
+SEQ_SYMBOL_PREFIXES = ("sllm_seq_", "sllm_kvpages_", "sllm_sample_", "sllm_last_error", "sllm_status", "sllm_abi_version", "sllm_tune", "sllm_device_info",
                        "sllm_prefill_gemm_")
 
 _lib = None

@@ -695,7 +695,7 @@ int sllm_batch_read(sllm_batch* b, int32_t slot, int32_t* tokens_out_host, int32
     const int n = std::min((int)max_tokens, b->host_pos[slot]);
     if (n > 0)
         SLLM_CUDA(cudaMemcpyAsync(tokens_out_host, b->history + (size_t)slot * b->S, sizeof(int32_t) * (size_t)n, cudaMemcpyDeviceToHost, b->stream));
-    SLLM_CUDA(cudaStreamSynchronize(b->stream));
+    SLLM_WAIT(b->stream);
     if (n_out) *n_out = n;
     return SLLM_OK;
 }
@@ -703,7 +703,7 @@ int sllm_batch_read(sllm_batch* b, int32_t slot, int32_t* tokens_out_host, int32
 int sllm_batch_logits(sllm_batch* b, int32_t slot, float* logits_host) {
     SLLM_REQUIRE(b && logits_host && slot >= 0 && slot < b->max_seqs && b->host_pos[slot] > 0, SLLM_EINVAL, "batch_logits: slot %d has not stepped", slot);
     SLLM_CUDA(cudaMemcpyAsync(logits_host, b->logits + (size_t)slot * b->V, sizeof(float) * (size_t)b->V, cudaMemcpyDeviceToHost, b->stream));
-    SLLM_CUDA(cudaStreamSynchronize(b->stream));
+    SLLM_WAIT(b->stream);
     return SLLM_OK;
 }
 
@@ -722,7 +722,7 @@ int sllm_batch_buffer(sllm_batch* b, int32_t id, void** dev_ptr, int64_t* n_elem
         case 16: *dev_ptr = b->logits; *n_elems = ms * b->V; break;
         default: SLLM_REQUIRE(false, SLLM_EINVAL, "batch_buffer: unknown buffer id %d", id);
     }
-    SLLM_CUDA(cudaStreamSynchronize(b->stream));
+    SLLM_WAIT(b->stream);
     return SLLM_OK;
 }
 

@@ -28,8 +28,26 @@ int cuda_fail(cudaError_t e, const char* what, const char* file, int line);
         }                                  \
     } while (0)
 
+// What kernels have to report. A kernel that gives up a bounded wait stores kStatusWait in a word of mapped host memory, since it returns like any other;
+// the library's next call that launches or waits returns SLLM_ETIMEOUT for it, once.
+constexpr int32_t kStatusWait = 1;
+extern int32_t* g_status;          // the word, nullptr until a kernel that may set it has been launched
+int status_word(int32_t** word);   // makes it (also while a stream is being captured)
+int status_take();                 // reports and clears
+inline int status_check() { return g_status && *reinterpret_cast<volatile int32_t*>(g_status) ? status_take() : SLLM_OK; }
+
 // Every launcher ends with this: a launch-configuration error surfaces here, not at the next sync.
-#define SLLM_LAUNCH_CHECK() SLLM_CUDA(cudaGetLastError())
+#define SLLM_LAUNCH_CHECK()                              \
+    do {                                                 \
+        SLLM_CUDA(cudaGetLastError());                   \
+        if (int _s = ::sllm::status_check()) return _s;  \
+    } while (0)
+// A wait of the library for a stream whose results it hands out.
+#define SLLM_WAIT(stream)                                \
+    do {                                                 \
+        SLLM_CUDA(cudaStreamSynchronize(stream));        \
+        if (int _s = ::sllm::status_check()) return _s;  \
+    } while (0)
 
 inline cudaStream_t as_stream(sllm_stream_t s) { return reinterpret_cast<cudaStream_t>(s); }
 

@@ -1015,7 +1015,7 @@ int sllm_engine_read_tokens(sllm_engine* e, int32_t* out, int32_t n) {
     const int first = e->h_state[7] - n;
     SLLM_REQUIRE(first >= 0, SLLM_EINVAL, "asked for %d tokens, only %d steps taken", n, e->h_state[7]);
     SLLM_CUDA(cudaMemcpyAsync(out, e->history_dev + first, sizeof(int32_t) * (size_t)n, cudaMemcpyDeviceToHost, e->stream));
-    SLLM_CUDA(cudaStreamSynchronize(e->stream));
+    SLLM_WAIT(e->stream);
     return SLLM_OK;
 }
 
@@ -1033,7 +1033,7 @@ int sllm_engine_forward(sllm_engine* e, int32_t token, int32_t pos, float* logit
     e->h_state[7] = pos + 1;
     if (logits_host) SLLM_CUDA(cudaMemcpyAsync(logits_host, e->logits, sizeof(float) * (size_t)e->V_loc, cudaMemcpyDeviceToHost, e->stream));
     if (next_token_host) SLLM_CUDA(cudaMemcpyAsync(e->h_state + 4, &e->state->next, 4, cudaMemcpyDeviceToHost, e->stream));
-    SLLM_CUDA(cudaStreamSynchronize(e->stream));
+    SLLM_WAIT(e->stream);
     if (next_token_host) *next_token_host = e->h_state[4];
     return SLLM_OK;
 }

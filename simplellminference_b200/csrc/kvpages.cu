@@ -48,6 +48,7 @@ const int32_t* sllm_kvpages_table(const sllm_kvpages* kp) { return kp ? kp->tabl
 int64_t sllm_seq_step_fill(int32_t* out, int64_t capacity, int32_t nseg, const int32_t* segments, const int32_t* tokens, const int32_t* rows, int32_t n_rows,
                            const sllm_kvpages* kp, int32_t tile, int64_t* offsets, int32_t* n_qtiles) {
     SLLM_REQUIRE(nseg > 0 && segments && tokens && kp && tile > 0 && offsets && n_qtiles && n_rows >= 0 && (n_rows == 0 || rows), SLLM_EINVAL, "seq_step_fill: bad argument");
+    if (int rc = status_check()) return rc;          // what an earlier step left unfinished
     int64_t T = 0, tiles = 0;
     for (int i = 0; i < nseg; ++i) {
         const int32_t len = segments[4 * i + 2];

@@ -38,6 +38,7 @@ struct TaArgs {
     int T, pos0, ldq, heads, group, pair_heads;     // pair_heads: a CTA's two tiles are two heads of a kv head; else two query tiles of one head
     int tiles, items;                               // query tiles of the prompt; tiles of a CTA (1 or 2)
     float scale_log2;
+    int32_t* status; unsigned polls;                // where a wait that was given up is reported, and after how many polls it is
 };
 
 template <int HD>
@@ -96,10 +97,10 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
             for (int kt = 0; kt < kts; ++kt) {
                 const int s = kt % ST;
                 const uint32_t ph = (uint32_t)(kt / ST) & 1;
-                if (!tc_wait(kempty + s, ph ^ 1, gave_up)) break;
+                if (!tc_wait(kempty + s, ph ^ 1, gave_up, p.polls)) break;
                 mb_expect(kfull + s, Sh::kTileBytes);
                 for (int c = 0; c < Sh::kBlocks; ++c) tma_load_3d(sK + s * Sh::kTileBytes + c * Sh::kBlockBytes, &tmK, 64 * c, kt * kTaTile, kvh, kfull + s);
-                if (!tc_wait(vempty + s, ph ^ 1, gave_up)) break;
+                if (!tc_wait(vempty + s, ph ^ 1, gave_up, p.polls)) break;
                 mb_expect(vfull + s, Sh::kTileBytes);
                 for (int c = 0; c < Sh::kBlocks; ++c) tma_load_3d(sV + s * Sh::kTileBytes + c * Sh::kBlockBytes, &tmV, 64 * c, kt * kTaTile, kvh, vfull + s);
             }
@@ -122,28 +123,28 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
                     tc_mma_bf16_ts(tmem + 256 + 128 * j, tmem + 128 * j + 8 * ks, umma_desc_mn_sw128(v + ks * 16 * 128, Sh::kBlockBytes), idesc_o, (kt | ks) != 0);
                 tc_commit(odone + j);
             };
-            bool ok = tc_wait(qfull, 0, gave_up) && tc_wait(kfull, 0, gave_up);
+            bool ok = tc_wait(qfull, 0, gave_up, p.polls) && tc_wait(kfull, 0, gave_up, p.polls);
             if (ok) {
                 tc_fence_after();
                 for (int j = 0; j < items; ++j) scores(j, 0);
                 tc_commit(kempty);
             }
             for (int kt = 0; ok && kt < kts; ++kt) {
-                ok = tc_wait(vfull + kt % ST, (uint32_t)(kt / ST) & 1, gave_up);
+                ok = tc_wait(vfull + kt % ST, (uint32_t)(kt / ST) & 1, gave_up, p.polls);
                 bool keys = false;
                 for (int j = 0; ok && j < items; ++j) {
                     if (kt >= nkt[j]) continue;
-                    ok = tc_wait(pready + j, (uint32_t)kt & 1, gave_up);
+                    ok = tc_wait(pready + j, (uint32_t)kt & 1, gave_up, p.polls);
                     if (!ok) break;
                     tc_fence_after();
                     values(j, kt);
                     if (kt + 1 >= nkt[j]) continue;
                     if (!keys) {
-                        ok = tc_wait(kfull + (kt + 1) % ST, (uint32_t)((kt + 1) / ST) & 1, gave_up);
+                        ok = tc_wait(kfull + (kt + 1) % ST, (uint32_t)((kt + 1) / ST) & 1, gave_up, p.polls);
                         keys = true;
                     }
                     // the next scores land where the weights lie that this product is still reading
-                    ok = ok && tc_wait(odone + j, (uint32_t)kt & 1, gave_up);
+                    ok = ok && tc_wait(odone + j, (uint32_t)kt & 1, gave_up, p.polls);
                     if (!ok) break;
                     tc_fence_after();
                     scores(j, kt + 1);
@@ -161,7 +162,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
             float ref = -INFINITY, l = 0.0f;            // what the weights are relative to (log2 units); their sum
             bool ok = true;
             for (int kt = 0; kt < nkt[j]; ++kt) {
-                ok = tc_wait(sfull + j, (uint32_t)kt & 1, gave_up);
+                ok = tc_wait_warp(sfull + j, (uint32_t)kt & 1, gave_up, p.polls);
                 if (!ok) break;
                 tc_fence_after();
                 const bool masked = kt * kTaTile + kTaTile - 1 > first_pos;       // some row of this warp does not see every key of the tile
@@ -234,7 +235,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
                 tc_fence_before();
                 mb_arrive(pready + j);
             }
-            ok = ok && tc_wait(odone + j, (uint32_t)(nkt[j] - 1) & 1, gave_up);
+            ok = ok && tc_wait_warp(odone + j, (uint32_t)(nkt[j] - 1) & 1, gave_up, p.polls);
             tc_fence_after();
             const float inv = 1.0f / l;
 #pragma unroll 1
@@ -256,11 +257,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
     }
     tc_fence_before();
     __syncthreads();
-    if (*gave_up) {        // copies may still be on their way into this CTA's memory: give them time before it is handed on
-        const long long until = clock64() + 4000000;
-        while (clock64() < until) {}
-        __syncthreads();
-    }
+    if (*gave_up) tc_gave_up(p.status);
     if (warp == 1) {
         tc_fence_after();
         tc_dealloc(tmem, kTaTmem);
@@ -293,11 +290,14 @@ static int ta_launch(const uint16_t* q, const void* kc, const void* vc, uint16_t
     a.tiles = (T + kTaTile - 1) / kTaTile;
     // two tiles per CTA hide each other's softmax and share their loads, unless single ones would still leave SMs idle
     a.items = (long long)a.tiles * heads > sm_count() ? 2 : 1;
+    if (int rc = status_word(&a.status)) return rc;
+    a.polls = (unsigned)g_tune_tc_polls;
     a.scale_log2 = (1.0f / sqrtf((float)HD)) * 1.4426950408889634f;
     const dim3 grid(a.items == 2 && !a.pair_heads ? (a.tiles + 1) / 2 : a.tiles, a.items == 2 && a.pair_heads ? heads / 2 : heads);
     LaunchCfg lc(grid, dim3(kTaThreads), Sh::kSmem, st, g_tune_pf_pdl != 0);
     SLLM_CUDA(cudaLaunchKernelEx(&lc.cfg, pf_attn_tc_kernel<HD>, tmQ, tmK, tmV, a));
     g_launches++;
+    SLLM_LAUNCH_CHECK();
     return SLLM_OK;
 }
 

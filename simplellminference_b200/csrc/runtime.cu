@@ -1,6 +1,7 @@
 // csrc/runtime.cu — error reporting and device facts behind include/sllm_b200.h.
 #include <cstdarg>
 #include <cstring>
+#include <mutex>
 
 #include "common.cuh"
 
@@ -17,6 +18,7 @@ int g_tune_batch_rows4 = 0;   // batched decode GEMV: 1 = four weight rows per w
 int g_tune_batch_ksplit = 0;  // batched decode, with rows4: down projection with K cut in two over grid.y when more vectors are live than fit whole rows (experimental)
 int g_tune_mega_debug = 0;   // decode megakernel measurement aid (MegaParams::debug): bit 0 = no grid barriers, bit 1 = no dot products; results are garbage
 int g_tune_seq_attn_mma = 1;   // ragged-batch attention: 1 = tensor-core body for bf16 pools on steps with prompt portions, 0 = always the fp32 body
+int g_tune_tc_polls = 1 << 24;   // tcgen05 attention kernels: polls after which a wait is given up
 int g_tune_pf_pair = -1;   // prefill GEMM: 1 / 0 = force / forbid the two-SM (cta_group::2) kernel, -1 = heuristic
 
 void set_error(const char* fmt, ...) {
@@ -29,6 +31,32 @@ void set_error(const char* fmt, ...) {
 int cuda_fail(cudaError_t e, const char* what, const char* file, int line) {
     set_error("CUDA error %d (%s) at %s:%d in %s", (int)e, cudaGetErrorString(e), file, line, what);
     return (int)e;
+}
+
+int32_t* g_status = nullptr;
+
+int status_word(int32_t** word) {
+    static std::mutex lock;
+    std::lock_guard<std::mutex> hold(lock);
+    if (!g_status) {
+        // an allocation would end a capture that runs in this thread; this one takes no part in it
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        SLLM_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+        void* p = nullptr;
+        const cudaError_t e = cudaHostAlloc(&p, sizeof(int32_t), cudaHostAllocMapped | cudaHostAllocPortable);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        SLLM_CUDA(e);
+        *static_cast<int32_t*>(p) = 0;
+        g_status = static_cast<int32_t*>(p);      // unified addressing: the same address on every device
+    }
+    *word = g_status;
+    return SLLM_OK;
+}
+
+int status_take() {
+    if (!g_status || __atomic_exchange_n(g_status, 0, __ATOMIC_ACQ_REL) == 0) return SLLM_OK;
+    set_error("a kernel gave up waiting for its copies or products: the results of an earlier launch are incomplete");
+    return SLLM_ETIMEOUT;
 }
 
 int sm_count() {
@@ -58,6 +86,7 @@ int smem_optin_bytes() {
 extern "C" {
 
 const char* sllm_last_error(void) { return sllm::g_err; }
+int sllm_status(void) { return sllm::status_check(); }
 int sllm_abi_version(void) { return 1; }
 
 int sllm_tune(int32_t key, int32_t value) {
@@ -72,6 +101,10 @@ int sllm_tune(int32_t key, int32_t value) {
         case 7: sllm::g_tune_batch_ksplit = value; return SLLM_OK;
         case 8: sllm::g_tune_mega_debug = value; return SLLM_OK;
         case 9: sllm::g_tune_seq_attn_mma = value; return SLLM_OK;
+        case 10:
+            SLLM_REQUIRE(value >= 0, SLLM_EINVAL, "a limit of %d polls", value);
+            sllm::g_tune_tc_polls = value;
+            return SLLM_OK;
         default: sllm::set_error("unknown tunable %d", key); return SLLM_EINVAL;
     }
 }

@@ -576,6 +576,7 @@ static int launch_attention_decode(Kernel* kernel, int G, int smem, const sllm::
     cfg.numAttrs = 1;
     SLLM_CUDA(cudaLaunchKernelEx(&cfg, kernel, p, args...));
     ++g_launches;
+    SLLM_LAUNCH_CHECK();
     return SLLM_OK;
 }
 

@@ -61,6 +61,7 @@ struct SaArgs {
     AttnArgs a;
     int hpc, hpc_log2, queries;          // query heads and queries of a CTA: hpc * queries = 128
     int vec_q;
+    int32_t* status; unsigned polls;     // where a wait that was given up is reported, and after how many polls it is
 };
 
 template <int HD, bool kOpts>
@@ -112,12 +113,12 @@ __global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const _
                     at[x] = pos <= last_pos ? in_page : b.page_len;                           // behind the last position: outside the map, zeros
                     row[x] = pos <= last_pos ? table[idx] * p.kv_heads + gkv : 0;
                 }
-                if (!tc_wait(kempty + s, ph ^ 1, gave_up)) break;
+                if (!tc_wait(kempty + s, ph ^ 1, gave_up, sa.polls)) break;
                 mb_expect(kfull + s, Sh::kTile);
 #pragma unroll
                 for (int x = 0; x < 2; ++x)
                     for (int c = 0; c < Sh::kBlocks; ++c) tma_load_3d(sK + s * Sh::kTile + c * Sh::kKBlock + x * kSaBox * 128, &tmK, 64 * c, at[x], row[x], kfull + s);
-                if (!tc_wait(vempty + s, ph ^ 1, gave_up)) break;
+                if (!tc_wait(vempty + s, ph ^ 1, gave_up, sa.polls)) break;
                 mb_expect(vfull + s, Sh::kTile);
 #pragma unroll
                 for (int x = 0; x < 2; ++x)
@@ -136,13 +137,13 @@ __global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const _
                 tc_commit(sfull);
                 tc_commit(kempty + i % ST);
             };
-            bool ok = n > 0 && tc_wait(qready, 0, gave_up) && tc_wait(kfull, 0, gave_up);
+            bool ok = n > 0 && tc_wait(qready, 0, gave_up, sa.polls) && tc_wait(kfull, 0, gave_up, sa.polls);
             if (ok) {
                 tc_fence_after();
                 scores(0);
             }
             for (int i = 0; ok && i < n; ++i) {
-                ok = tc_wait(vready + i % ST, (uint32_t)(i / ST) & 1, gave_up) && tc_wait(pready, (uint32_t)i & 1, gave_up);
+                ok = tc_wait(vready + i % ST, (uint32_t)(i / ST) & 1, gave_up, sa.polls) && tc_wait(pready, (uint32_t)i & 1, gave_up, sa.polls);
                 if (!ok) break;
                 tc_fence_after();
                 const uint8_t* v = sV + (i % ST) * Sh::kTile;
@@ -152,7 +153,7 @@ __global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const _
                 tc_commit(odone);
                 tc_commit(vempty + i % ST);
                 if (i + 1 < n) {        // the next scores land where the weights lie that this product is still reading
-                    ok = tc_wait(kfull + (i + 1) % ST, (uint32_t)((i + 1) / ST) & 1, gave_up) && tc_wait(odone, (uint32_t)i & 1, gave_up);
+                    ok = tc_wait(kfull + (i + 1) % ST, (uint32_t)((i + 1) / ST) & 1, gave_up, sa.polls) && tc_wait(odone, (uint32_t)i & 1, gave_up, sa.polls);
                     if (!ok) break;
                     tc_fence_after();
                     scores(i + 1);
@@ -162,7 +163,7 @@ __global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const _
     } else if (warp == 6) {   // ===== value rows that the sequence does not have yet =====
         for (int i = 0; i < n; ++i) {
             const int s = i % ST, have = last_pos + 1 - tiles.tile_of(split + i * p.nsplit) * kSaKeys;
-            if (!tc_wait(vfull + s, (uint32_t)(i / ST) & 1, gave_up)) break;
+            if (!tc_wait_warp(vfull + s, (uint32_t)(i / ST) & 1, gave_up, sa.polls)) break;
             if (have < kSaKeys) {
                 for (int x = lane; x < (kSaKeys - have) * 8 * Sh::kBlocks; x += 32) {
                     const int c = x / ((kSaKeys - have) * 8), y = x % ((kSaKeys - have) * 8);
@@ -248,7 +249,7 @@ __global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const _
         bool ok = true;
         for (int i = 0; i < n; ++i) {
             const int j0 = tiles.tile_of(split + i * p.nsplit) * kSaKeys;
-            ok = tc_wait(sfull, (uint32_t)i & 1, gave_up);
+            ok = tc_wait_warp(sfull, (uint32_t)i & 1, gave_up, sa.polls);
             if (!ok) break;
             tc_fence_after();
             uint32_t s[64];
@@ -342,7 +343,7 @@ __global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const _
             mb_arrive(pready);
         }
         if (live && n > kSaFlush) prefetch_flushed();
-        if (ok && n > 0) ok = tc_wait(odone, (uint32_t)(n - 1) & 1, gave_up);
+        if (ok && n > 0) ok = tc_wait_warp(odone, (uint32_t)(n - 1) & 1, gave_up, sa.polls);
         tc_fence_after();
         float inv = direct ? 1.0f / l : 1.0f;
         const int t = tok0 + qi;
@@ -400,11 +401,7 @@ __global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const _
     }
     tc_fence_before();
     __syncthreads();
-    if (*gave_up) {        // copies may still be on their way into this CTA's memory: give them time before it is handed on
-        const long long until = clock64() + 4000000;
-        while (clock64() < until) {}
-        __syncthreads();
-    }
+    if (*gave_up) tc_gave_up(sa.status);
     if (warp == 5) {
         tc_fence_after();
         tc_dealloc(tmem, kSaTmem);
@@ -426,6 +423,8 @@ static int sa_launch(const AttnArgs& p, cudaStream_t st) {
     a.hpc = group % 4 == 0 ? 4 : group % 2 == 0 ? 2 : 1;
     a.hpc_log2 = a.hpc / 2;
     a.queries = kSaRows / a.hpc;
+    if (int rc = status_word(&a.status)) return rc;
+    a.polls = (unsigned)g_tune_tc_polls;
     a.vec_q = p.ldq % 4 == 0 && ((uintptr_t)p.q % 16) == 0;
     // a pool [pages][kv_heads][page_len][HD]: how many pages it has is the caller's knowledge, the block table names existing ones only
     CUtensorMap tmK, tmV;

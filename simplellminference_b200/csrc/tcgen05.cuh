@@ -10,6 +10,8 @@ namespace sllm {
 // tensor map of bf16 elements, boxes with 128-byte rows in the 128B swizzle, zeros outside the tensor (prefill_gemm.cu)
 int tc_encode_bf16(CUtensorMap* tm, const void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides_bytes, const cuuint32_t* box);
 
+extern int g_tune_tc_polls;   // runtime.cu: polls after which the kernels below give up a wait
+
 #ifdef __CUDACC__
 
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* tm, int c0, int c1, uint64_t* bar) {
@@ -119,24 +121,36 @@ __device__ __forceinline__ uint32_t tc_pack(float lo, float hi) {
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
     return r;
 }
-// Bounded wait on a barrier; false once some thread of this CTA has given up (a flag in shared memory): the kernel then tears down without its result
-constexpr unsigned kTcSpin = 1u << 24;              // polls, seconds: nothing legitimate waits that long
-__device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile int* gave_up) {
-    uint32_t done;
-    unsigned spins = 0;
-    while (true) {
+// Bounded wait on a barrier. False once this thread's polls have run out or another one of the CTA has given up (a flag in shared memory): the kernel then
+// tears down without its result and says so in the library's status word (tc_gave_up).
+__device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile int* gave_up, unsigned polls) {
+    for (unsigned i = 0; i < polls; ++i) {
+        uint32_t done;
         asm volatile(
             "{\n.reg .pred p;\n"
             "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
             "selp.u32 %0, 1, 0, p;\n}\n"
             : "=r"(done) : "r"(s_addr(bar)), "r"(parity) : "memory");
         if (done) return true;
-        if ((++spins & 1023) == 0 && *gave_up) return false;
-        if (spins > kTcSpin) {
-            *gave_up = 1;
-            return false;
-        }
+        if ((i & 1023) == 1023 && *gave_up) return false;
     }
+    *gave_up = 1;
+    return false;
+}
+// The same for all lanes of a warp, which go on or give up together (what follows are instructions of the whole warp).
+__device__ __forceinline__ bool tc_wait_warp(uint64_t* bar, uint32_t parity, volatile int* gave_up, unsigned polls) {
+    return __all_sync(0xffffffffu, tc_wait(bar, parity, gave_up, polls));
+}
+// By all threads of a CTA some of which has given up, behind a barrier of the CTA: copies and products may still be on their way into this CTA's memory, so they
+// get time before it is handed on.
+__device__ __forceinline__ void tc_gave_up(int32_t* status) {
+    if (threadIdx.x == 0) {
+        *reinterpret_cast<volatile int32_t*>(status) = kStatusWait;
+        __threadfence_system();
+    }
+    const long long until = clock64() + 4000000;
+    while (clock64() < until) {}
+    __syncthreads();
 }
 
 #endif

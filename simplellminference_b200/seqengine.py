@@ -401,5 +401,6 @@ class SequenceDecoder:
                 eng.ops.sample(logits.data_ptr() + 4 * i * logits.shape[1], logits.shape[1], temperature, top_k, top_p, seed, eng.pos[slot] - 1,
                                self._idx.data_ptr() + 4 * i, st)
             drawn = self._idx[:len(drawing)].cpu().numpy()
+            _lib.check_seq(_lib.load_seq().sllm_status())      # the copy has waited for the step
             for i, slot in enumerate(drawing):
                 self._req[slot]["out"].append(int(drawn[i]))
