@@ -412,7 +412,8 @@ typedef struct {
     const int32_t* seg_pos0;     /* [nseg] position of the segment's first token */
     const int32_t* block_table;  /* [slots][max_pages] page of positions i*page_len.., -1 = none */
     int32_t max_pages, page_len; /* page_len: a multiple of 32 */
-    int32_t n_qtiles;            /* attention work list: tiles of up to 32 consecutive queries of one segment, offsets multiples of 32; every query is in one */
+    int32_t n_qtiles;            /* attention work list: tiles of up to 32 consecutive queries of one segment, no query in two of them. Attention works on
+                                  * the listed ones, whichever they are; the block and range forms of the recurrent layers need every token in one, at offsets that are multiples of 32 */
     const int32_t* qt_seg;       /* [n_qtiles] segment of the tile */
     const int32_t* qt_off;       /* [n_qtiles] offset of its first query inside the segment */
     const int32_t* seg_tile0;    /* [nseg] running count of tiles of the segments before this one (tile ids in segment order) */

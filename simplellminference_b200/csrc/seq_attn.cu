@@ -665,8 +665,7 @@ static int attention_run(const sllm_seq_batch* b, const float* q, int32_t ldq, i
         // 1000, 311, 700 and 37 tokens, 16 heads over 4 of 128 170 | 50, capped 218 | 74; one of 4096, 32 heads over 8 2050 | 377; one of 512 51 | 33 (heads of
         // 64, 32 over 32: 54 | 49); 256 tokens from the start and behind 2000 34 | 31 and 96 | 39 (heads of 64: 32 | 40); 128 and 16 tokens from the
         // start 15 | 21 and 7.7 | 16 (a fixed part of some 14 us: queries, TMEM, barriers, rows out): below that size this body stays.
-        // (It takes several neighbouring tiles of the list as one, so the list has to hold every query: at least T / 32 tiles.)
-        const bool tc = dk == dv && (dk == 64 || dk == 128) && b->n_qtiles >= (dk == 128 ? 8 : 16) && (long long)b->n_qtiles * kBQ >= b->T && !p.cross && !v_in_k &&
+        const bool tc = dk == dv && (dk == 64 || dk == 128) && b->n_qtiles >= (dk == 128 ? 8 : 16) && !p.cross && !v_in_k &&
                         (((uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)out16 | (uintptr_t)ws) % 16) == 0;
         // shares are for steps whose query tiles leave SMs idle (the tcgen05 body takes 128 rows of query heads and queries at a time)
         if (tc && (out || out16) && (long long)b->n_qtiles * kBQ * heads / 128 >= 2LL * sm_count()) p.nsplit = 1;

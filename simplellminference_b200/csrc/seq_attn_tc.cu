@@ -71,7 +71,27 @@ __global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const _
     const AttnArgs& p = sa.a;
     const sllm_seq_batch& b = p.b;
     const int seg = b.qt_seg[blockIdx.x], off = b.qt_off[blockIdx.x], split = blockIdx.z;
-    if (off % sa.queries) return;        // the first 32-query tile of a run of `queries` stands for all of it
+    // The work list may hold any tiles of 32 queries. Those of one aligned run of `queries` that are in it are done together, by the CTA of the first of them:
+    // bit i of `parts` says that the tile i behind this CTA's own is one of them.
+    uint32_t parts = 1;
+    const bool in_run = sa.queries > kBQ && off % kBQ == 0;
+    if (in_run) {
+        __shared__ uint32_t found;
+        const int run = off & ~(sa.queries - 1);
+        uint32_t mine = 0;
+        for (int i = threadIdx.x; i < b.n_qtiles; i += kSaThreads) {
+            const uint32_t d = (uint32_t)(b.qt_off[i] - run);
+            if (b.qt_seg[i] == seg && d < (uint32_t)sa.queries && d % kBQ == 0) mine |= 1u << (d / kBQ);
+        }
+        if (threadIdx.x == 0) found = 0;
+        __syncthreads();
+        mine = __reduce_or_sync(0xffffffffu, mine);
+        if (mine && threadIdx.x % 32 == 0) atomicOr(&found, mine);
+        __syncthreads();
+        const uint32_t own = 1u << ((off - run) / kBQ);
+        if (found & (own - 1)) return;
+        parts = found / own;
+    }
     extern __shared__ uint8_t sa_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(sa_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t *sK = smem, *sV = sK + ST * Sh::kTile, *sQ = sV + ST * Sh::kTile;
@@ -80,7 +100,7 @@ __global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const _
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(odone + 1);
     volatile int* gave_up = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nq = min(sa.queries, b.seg_len[seg] - off), tok0 = b.seg_start[seg] + off, pos0 = b.seg_pos0[seg] + off, slot = b.seg_slot[seg];
+    const int nq = min((32 - __clz(parts)) * kBQ, b.seg_len[seg] - off), tok0 = b.seg_start[seg] + off, pos0 = b.seg_pos0[seg] + off, slot = b.seg_slot[seg];
     const int group = p.heads / p.kv_heads, sets = group / sa.hpc, gkv = blockIdx.y / sets, h0 = gkv * group + (blockIdx.y % sets) * sa.hpc;
     const int last_pos = pos0 + nq - 1;
     const TileList tiles(pos0, last_pos, seq_row_window(pos0, p.window, p.chunk), p.keep_first, kSaKeys);
@@ -176,7 +196,7 @@ __global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const _
         }
     } else if (warp < 4) {   // ===== softmax: row = warp * 32 + lane = query * hpc + head =====
         const int row = threadIdx.x, qi = row >> sa.hpc_log2, h = h0 + (row & (sa.hpc - 1));
-        const bool live = qi < nq;
+        const bool live = qi < nq && (parts >> (qi / kBQ) & 1);
         const int qpos = pos0 + qi;
         {   // the warp's 32 rows, one row (or two) per load so that neighbouring lanes read neighbouring columns
             constexpr int kLanes = HD / 4, kPer = 32 / kLanes;                  // lanes of a row, rows of a load
@@ -198,7 +218,7 @@ __global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const _
         const bool plain = !kOpts && p.scale > 0.0f;
         const float mul = plain ? p.scale * kSaLog2e : kSaLog2e;
         float ref = -INFINITY, l = 0.0f, flushed = -INFINITY;      // what the weights are relative to; their sum; the reference of what has been flushed
-        const int rows = min(32, (nq << sa.hpc_log2) - warp * 32);
+        const int rows = parts >> ((warp * 32 >> sa.hpc_log2) / kBQ) & 1 ? min(32, (nq << sa.hpc_log2) - warp * 32) : 0;      // a warp's rows belong to one tile
         // the records of this warp's rows, and how far the next head's and the next query's are
         float* recs = p.ws + (((size_t)tok0 * p.heads + h0) * p.nsplit + split) * (HD + 2);
         const int rec_h = p.nsplit * (HD + 2), rec_q = p.heads * rec_h;
