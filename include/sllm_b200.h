@@ -51,8 +51,9 @@ enum { SLLM_F32 = 0, SLLM_BF16 = 1, SLLM_INT8 = 2 };
 typedef void* sllm_stream_t;
 
 const char* sllm_last_error(void);
-/* SLLM_ETIMEOUT, once, after a kernel of this library has given up one of its bounded waits (its result rows are then unwritten), else SLLM_OK. Every call
- * that launches kernels or waits for them reports the same, so a program needs this only behind a synchronisation of its own. */
+/* SLLM_ETIMEOUT, once, after a kernel of this library has given up one of its bounded waits (its result rows are then unwritten), SLLM_EINVAL, once, after one
+ * has found index arrays that contradict the host's counts, else SLLM_OK. Every call that launches kernels or waits for them reports the same, so a program
+ * needs this only behind a synchronisation of its own. */
 int sllm_status(void);
 int sllm_abi_version(void);
 /* development knobs (not part of the drop-in surface): key 0 = GEMV CTAs per SM (0 = built-in choice); prefill GEMM: key 1 = force

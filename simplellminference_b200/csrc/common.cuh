@@ -29,8 +29,8 @@ int cuda_fail(cudaError_t e, const char* what, const char* file, int line);
     } while (0)
 
 // What kernels have to report. A kernel that gives up a bounded wait stores kStatusWait in a word of mapped host memory, since it returns like any other;
-// the library's next call that launches or waits returns SLLM_ETIMEOUT for it, once.
-constexpr int32_t kStatusWait = 1;
+// the library's next call that launches or waits returns SLLM_ETIMEOUT for it, once. kStatusBatch: index arrays on the device contradict the host's counts (SLLM_EINVAL).
+constexpr int32_t kStatusWait = 1, kStatusBatch = 2;
 extern int32_t* g_status;          // the word, nullptr until a kernel that may set it has been launched
 int status_word(int32_t** word);   // makes it (also while a stream is being captured)
 int status_take();                 // reports and clears

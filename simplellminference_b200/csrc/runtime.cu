@@ -54,7 +54,9 @@ int status_word(int32_t** word) {
 }
 
 int status_take() {
-    if (!g_status || __atomic_exchange_n(g_status, 0, __ATOMIC_ACQ_REL) == 0) return SLLM_OK;
+    const int32_t what = g_status ? __atomic_exchange_n(g_status, 0, __ATOMIC_ACQ_REL) : 0;
+    if (what == 0) return SLLM_OK;
+    SLLM_REQUIRE(what != kStatusBatch, SLLM_EINVAL, "seq_ssd_blocks: n_qtiles of an earlier launch does not count the tiles of all its tokens; its results are incomplete");
     set_error("a kernel gave up waiting for its copies or products: the results of an earlier launch are incomplete");
     return SLLM_ETIMEOUT;
 }

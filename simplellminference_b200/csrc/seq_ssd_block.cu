@@ -33,10 +33,18 @@ template <int NK>
 __global__ void __launch_bounds__(kSsdThreads) seq_ssd_prepare_kernel(SsdBlockArgs p, int vec) {
     extern __shared__ __align__(16) float sp_sm[];
     const sllm_seq_batch& b = p.b;
-    const int tile = blockIdx.x, seg = b.qt_seg[tile], off = b.qt_off[tile];
-    if (off % kSsdBlock) return;                             // a block is two query tiles; the first of them stands for it
-    const int n = min(kSsdBlock, b.seg_len[seg] - off), start = b.seg_start[seg] + off;
-    const size_t id = ssd_block_id(b.seg_tile0[seg], seg, off / kSsdBlock);
+    const size_t id = blockIdx.x;                            // this block's number in the scratch: whose is it?
+    __shared__ int owner;
+    if (threadIdx.x == 0) owner = -1;
+    __syncthreads();
+    for (int i = threadIdx.x; i < b.nseg; i += kSsdThreads) {
+        const size_t first = ssd_block_id(b.seg_tile0[i], i, 0);
+        if (id >= first && id < first + (b.seg_len[i] + kSsdBlock - 1) / kSsdBlock) owner = i;
+    }
+    __syncthreads();
+    const int seg = owner;
+    if (seg < 0) return;
+    const int off = (int)(id - ssd_block_id(b.seg_tile0[seg], seg, 0)) * kSsdBlock, n = min(kSsdBlock, b.seg_len[seg] - off), start = b.seg_start[seg] + off;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if ((int)blockIdx.y >= p.groups) {                       // step sizes and running sums, a warp per head
         const int h = ((int)blockIdx.y - p.groups) * (kSsdThreads / 32) + warp;
@@ -175,6 +183,10 @@ __global__ void __launch_bounds__(kSsdWalk, 1) seq_ssd_walk_kernel(SsdBlockArgs 
     const int start = b.seg_start[seg], len = b.seg_len[seg], slot = b.seg_slot[seg], blocks = (len + kSsdBlock - 1) / kSsdBlock;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3, ct = warp & 1, qu = warp >> 1;
     const size_t id0 = ssd_block_id(b.seg_tile0[seg], seg, 0);
+    if (id0 + blocks > p.slots) {       // the scratch was sized by a tile count that leaves tokens out
+        if (threadIdx.x == 0) *reinterpret_cast<volatile int32_t*>(p.status) = kStatusBatch;
+        return;
+    }
     const float* xs = p.x + (size_t)start * p.ldx + (size_t)h * p.dv + col0;
     auto issue = [&](int blk) {
         uint8_t* dst = sw_sm + (blk & 1) * kStage;
@@ -369,7 +381,7 @@ static int launch_ssd(SsdBlockArgs p, cudaStream_t st) {
         sized = true;
     }
     const int per = kSsdThreads / 32;
-    seq_ssd_prepare_kernel<NK><<<dim3(p.b.n_qtiles, p.groups + (p.heads + per - 1) / per), kSsdThreads, smem_prep, st>>>(p, vec_prep);
+    seq_ssd_prepare_kernel<NK><<<dim3((unsigned)p.slots, p.groups + (p.heads + per - 1) / per), kSsdThreads, smem_prep, st>>>(p, vec_prep);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     seq_ssd_walk_kernel<NK><<<dim3(p.b.nseg, p.heads, (p.dv + kSsdCols - 1) / kSsdCols), kSsdWalk, smem, st>>>(p, vec);
@@ -391,16 +403,16 @@ extern "C" int sllm_seq_ssd_blocks(const sllm_seq_batch* b, const float* x, int3
                                    int32_t lda, const float* A_log, const float* dt_bias, const float* skip, int32_t heads, int32_t groups, int32_t n_state, int32_t dv,
                                    float* state, float* y, int32_t ldy, const float* conv_x, int32_t ld_conv, int32_t channels, int32_t taps, float* ring, void* block_ws,
                                    sllm_stream_t stream) {
-    SLLM_REQUIRE(b && b->T > 0 && b->nseg > 0 && b->seg_start && b->seg_len && b->seg_slot && b->seg_tile0 && b->qt_seg && b->qt_off && b->n_qtiles > 0, SLLM_EINVAL,
+    SLLM_REQUIRE(b && b->T > 0 && b->nseg > 0 && b->seg_start && b->seg_len && b->seg_slot && b->seg_tile0 && (long long)b->n_qtiles * 32 >= b->T, SLLM_EINVAL,
                  "seq_ssd_blocks: incomplete batch description");
     SLLM_REQUIRE(x && B && C && step_logit && A_log && dt_bias && state && y && block_ws && ((uintptr_t)block_ws % 16) == 0, SLLM_EINVAL, "seq_ssd_blocks: bad argument");
     SLLM_REQUIRE(heads > 0 && groups > 0 && heads % groups == 0 && n_state > 0 && dv > 0, SLLM_EINVAL, "seq_ssd_blocks: %d heads over %d groups", heads, groups);
     SLLM_REQUIRE(n_state <= kSsdMaxState && heads <= 65535 && groups + heads / 8 < 65535, SLLM_ENOTSUP, "seq_ssd_blocks: %d states per channel beyond %d", n_state, kSsdMaxState);
     SLLM_REQUIRE(!ring || taps <= 1 || conv_x, SLLM_EINVAL, "seq_ssd_blocks: a ring without its inputs");
-    SsdBlockArgs p{*b, x, B, C, step_logit, ldx, ldb, ldc, lda, A_log, dt_bias, skip, heads, groups, n_state, dv, state, y, ldy, nullptr, nullptr};
-    const size_t slots = ssd_block_count(b->n_qtiles, b->nseg);
+    SsdBlockArgs p{*b, x, B, C, step_logit, ldx, ldb, ldc, lda, A_log, dt_bias, skip, heads, groups, n_state, dv, state, y, ldy, nullptr, ssd_block_count(b->n_qtiles, b->nseg), nullptr, nullptr};
+    if (int rc = status_word(&p.status)) return rc;
     p.group_ws = reinterpret_cast<uint8_t*>(block_ws);
-    p.head_ws = reinterpret_cast<float*>(p.group_ws + slots * groups * ssd_block_group_bytes(n_state <= 64 ? 64 : 128));
+    p.head_ws = reinterpret_cast<float*>(p.group_ws + p.slots * groups * ssd_block_group_bytes(n_state <= 64 ? 64 : 128));
     if (int rc = n_state <= 64 ? launch_ssd<64>(p, as_stream(stream)) : launch_ssd<128>(p, as_stream(stream))) return rc;
     return ring && taps > 1 ? sllm_seq_ring_store(b, conv_x, ld_conv, channels, taps, ring, stream) : SLLM_OK;
 }

@@ -14,6 +14,7 @@ struct SsdBlockArgs {
     int heads, groups, n_state, dv;
     float* state; float* y; int ldy;
     uint8_t* group_ws;                 // per (block, group): fragments of C and B, products C_i . B_j
+    size_t slots; int32_t* status;     // blocks the scratch has room for; where a batch that needs more is reported
     float* head_ws;                    // per (block, head): running sums of the decays' base-2 logarithms [64] and their second terms [64], step sizes [64]
 };
 

@@ -1,5 +1,5 @@
-"""State-space duality in blocks of tokens (sllm_seq_ssd_blocks) keeps what the token-by-token form (sllm_seq_ssd_scan) has: its accuracy, and which tokens a value
-reaches. Three bf16 terms per operand leave 2^-24 of a product; fp32 sums of up to 128 + 64
+"""State-space duality in blocks of tokens (sllm_seq_ssd_blocks) keeps what the token-by-token form (sllm_seq_ssd_scan) has: its accuracy, which tokens a value
+reaches, and an error where index arrays and counts contradict each other. Three bf16 terms per operand leave 2^-24 of a product; fp32 sums of up to 128 + 64
 products and 16 blocks of carried state stay within 5e-7."""
 import math
 
@@ -80,3 +80,16 @@ def test_a_value_that_is_not_finite_reaches_no_earlier_token(value):
     rest[0, 1, :, 5] = False
     assert torch.equal(S[rest], clean[1][rest])
     assert torch.equal(torch.isfinite(y[at:128, col]), torch.isfinite(y2[at:128, col]))      # (infinite or no number: the two forms sum in different orders)
+
+
+def test_a_tile_count_that_leaves_tokens_out_is_reported():
+    from simplellminference_b200 import _lib
+    lens, shape = [33] * 16, (2, 1, 64, 32)
+    t = _inputs(lens, *shape, 0.0)
+    with pytest.raises(_lib.SllmError) as e:          # fewer tiles than tokens need at all: refused at once
+        _run(t, lens, *shape, n_qtiles=16)
+    assert e.value.code == _lib.EINVAL
+    lib = _lib.load_seq()
+    assert lib.sllm_status() == 0
+    _run(t, lens, *shape, n_qtiles=17)                # two tiles a segment are needed: seen on the device
+    assert lib.sllm_status() == _lib.EINVAL and lib.sllm_status() == 0
