@@ -2,6 +2,8 @@
 #pragma once
 #include <cooperative_groups.h>
 
+#include <type_traits>
+
 #include "seq_attn.cuh"
 
 namespace sllm {
@@ -376,9 +378,9 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, 2) seq_attention_decode_mma
         }
         cp_async_commit();
     };
-    int run = (split * CS + rank) * kDecodeWarps + warp;
+    const int first_run = (split * CS + rank) * kDecodeWarps + warp;
 #pragma unroll
-    for (int i = 0; i < kRing - 1; ++i) issue(run + i * workers, i);
+    for (int i = 0; i < kRing - 1; ++i) issue(first_run + i * workers, i);
 
     uint32_t qa[kSteps][4];
     {
@@ -401,83 +403,105 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, 2) seq_attention_decode_mma
     // ldmatrix rows: keys as they lie (two key tiles x two halves of a k-step), values transposed (two value tiles x two halves of the keys)
     const uint32_t k_at = (((lane & 7) + (lane & 16 ? 8 : 0)) * D * 2) | (((lane & 8 ? 1 : 0) ^ (lane & 7)) << 4);
     const uint32_t v_at = ((kRun + (lane & 15)) * D * 2) | (((lane & 16 ? 1 : 0) ^ (lane & 7)) << 4);
-    int stage = 0;
-    for (; run < n_runs; run += workers) {
-        cp_async_wait<kRing - 2>();
+    // Several terms times an infinite value are no number, where the fp32 product would be infinite: a warp whose sums come out like that walks its runs once
+    // more with the later terms' products left out wherever they are not finite. The first terms then give what fp32 gives.
+    auto finite = [](float x) { return fabsf(x) <= 3.402823466e38f ? x : 0.0f; };
+    auto walk = [&](auto careful_) {
+        constexpr bool careful = decltype(careful_)::value;
+        int stage = 0;
+        for (int run = first_run; run < n_runs; run += workers) {
+            cp_async_wait<kRing - 2>();
+            __syncwarp();
+            const int j0 = first_key(run);
+            const uint32_t base = ring + stage * Tile::kStage * 2;
+            float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+            for (int ks = 0; ks < kSteps; ks += 2) {
+                float part[2][4];
+                uint32_t ka[4], kb[4];
+                ldmatrix4(ka, base + (k_at ^ (ks * 32)));
+                ldmatrix4(kb, base + (k_at ^ ((ks + 1) * 32)));
+                mma_bf16_zero(part[0], qa[ks], ka[0], ka[1]);
+                mma_bf16_zero(part[1], qa[ks], ka[2], ka[3]);
+                mma_bf16_16816(part[0], qa[ks + 1], kb[0], kb[1]);
+                mma_bf16_16816(part[1], qa[ks + 1], kb[2], kb[3]);
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) s[i][e] += part[i][e];
+            }
+            // first + third term here, the second on the neighbouring lane: both then hold the head's scores of keys 2c, 2c + 1 (+ 8)
+            float w[4], mx = -INFINITY;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float here = s[i >> 1][i & 1], third = s[i >> 1][2 + (i & 1)];
+                const float mine = careful ? (second ? finite(here) : here) + finite(third) : here + third;
+                w[i] = mine + __shfl_xor_sync(0xffffffffu, mine, 4);
+                w[i] = kOpts ? seq_score(w[i], p.scale, p.softcap, slope, r1, r2, pos, j0 + (i >> 1) * 8 + 2 * c + (i & 1)) : w[i] * p.scale;
+            }
+            if (j0 + kRun - 1 > pos || (pos - j0 >= wnd && j0 + kRun > p.keep_first)) {      // some key of the run is hidden
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (!seq_sees(pos, j0 + (i >> 1) * 8 + 2 * c + (i & 1), wnd, p.keep_first)) w[i] = -INFINITY;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) mx = fmaxf(mx, w[i]);
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+            const float mn = fmaxf(m, mx);
+            if (__any_sync(0xffffffffu, mn != m)) {
+                const float corr = mn == -INFINITY ? 1.0f : expf(m - mn);
+                l *= corr;
+#pragma unroll
+                for (int i = 0; i < kTiles; ++i)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) o[i][e] *= corr;
+                m = mn;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                w[i] = w[i] == -INFINITY ? 0.0f : expf(w[i] - mn);
+                l += w[i];
+            }
+            uint32_t pa[4];
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                uint32_t t1, t2, t3;
+                split3_bf16(w[half * 2], w[half * 2 + 1], t1, t2, t3);
+                pa[half * 2] = second ? t2 : t1;
+                pa[half * 2 + 1] = second ? 0u : t3;
+            }
+#pragma unroll
+            for (int nt = 0; nt < kTiles; nt += 2) {
+                uint32_t vb[4];
+                ldmatrix4_trans(vb, base + (v_at ^ (nt * 16)));
+                float part[2][4];
+                mma_bf16_zero(part[0], pa, vb[0], vb[1]);
+                mma_bf16_zero(part[1], pa, vb[2], vb[3]);
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) o[nt + i][e] += careful ? (second ? finite(part[i][e]) : part[i][e]) + finite(part[i][2 + e]) : part[i][e] + part[i][2 + e];
+            }
+            __syncwarp();                       // every lane has read the stage that is filled next
+            issue(run + (kRing - 1) * workers, stage == 0 ? kRing - 1 : stage - 1);
+            stage = stage + 1 == kRing ? 0 : stage + 1;
+        }
+    };
+    walk(std::false_type{});
+    bool wild = false;
+#pragma unroll
+    for (int i = 0; i < kTiles; ++i) wild |= o[i][0] != o[i][0] || o[i][1] != o[i][1];
+    if (__any_sync(0xffffffffu, wild)) {
+        cp_async_wait<0>();
         __syncwarp();
-        const int j0 = first_key(run);
-        const uint32_t base = ring + stage * Tile::kStage * 2;
-        float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
-        for (int ks = 0; ks < kSteps; ks += 2) {
-            float part[2][4];
-            uint32_t ka[4], kb[4];
-            ldmatrix4(ka, base + (k_at ^ (ks * 32)));
-            ldmatrix4(kb, base + (k_at ^ ((ks + 1) * 32)));
-            mma_bf16_zero(part[0], qa[ks], ka[0], ka[1]);
-            mma_bf16_zero(part[1], qa[ks], ka[2], ka[3]);
-            mma_bf16_16816(part[0], qa[ks + 1], kb[0], kb[1]);
-            mma_bf16_16816(part[1], qa[ks + 1], kb[2], kb[3]);
+        for (int i = 0; i < kRing - 1; ++i) issue(first_run + i * workers, i);
+        m = -INFINITY;
+        l = 0.0f;
 #pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) s[i][e] += part[i][e];
-        }
-        // first + third term here, the second on the neighbouring lane: both then hold the head's scores of keys 2c, 2c + 1 (+ 8)
-        float w[4], mx = -INFINITY;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float mine = s[i >> 1][i & 1] + s[i >> 1][2 + (i & 1)];
-            w[i] = mine + __shfl_xor_sync(0xffffffffu, mine, 4);
-            w[i] = kOpts ? seq_score(w[i], p.scale, p.softcap, slope, r1, r2, pos, j0 + (i >> 1) * 8 + 2 * c + (i & 1)) : w[i] * p.scale;
-        }
-        if (j0 + kRun - 1 > pos || (pos - j0 >= wnd && j0 + kRun > p.keep_first)) {      // some key of the run is hidden
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-                if (!seq_sees(pos, j0 + (i >> 1) * 8 + 2 * c + (i & 1), wnd, p.keep_first)) w[i] = -INFINITY;
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) mx = fmaxf(mx, w[i]);
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-        const float mn = fmaxf(m, mx);
-        if (__any_sync(0xffffffffu, mn != m)) {
-            const float corr = mn == -INFINITY ? 1.0f : expf(m - mn);
-            l *= corr;
-#pragma unroll
-            for (int i = 0; i < kTiles; ++i)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) o[i][e] *= corr;
-            m = mn;
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            w[i] = w[i] == -INFINITY ? 0.0f : expf(w[i] - mn);
-            l += w[i];
-        }
-        uint32_t pa[4];
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            uint32_t t1, t2, t3;
-            split3_bf16(w[half * 2], w[half * 2 + 1], t1, t2, t3);
-            pa[half * 2] = second ? t2 : t1;
-            pa[half * 2 + 1] = second ? 0u : t3;
-        }
-#pragma unroll
-        for (int nt = 0; nt < kTiles; nt += 2) {
-            uint32_t vb[4];
-            ldmatrix4_trans(vb, base + (v_at ^ (nt * 16)));
-            float part[2][4];
-            mma_bf16_zero(part[0], pa, vb[0], vb[1]);
-            mma_bf16_zero(part[1], pa, vb[2], vb[3]);
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) o[nt + i][e] += part[i][e] + part[i][2 + e];
-        }
-        __syncwarp();                       // every lane has read the stage that is filled next
-        issue(run + (kRing - 1) * workers, stage == 0 ? kRing - 1 : stage - 1);
-        stage = stage + 1 == kRing ? 0 : stage + 1;
+        for (int i = 0; i < kTiles; ++i) o[i][0] = o[i][1] = 0.0f;
+        walk(std::true_type{});
     }
     // The terms' results meet on neighbouring lanes: the lane of the first and third terms keeps the first half of the columns, the other the second.
     float v[kTiles / 2][2];
