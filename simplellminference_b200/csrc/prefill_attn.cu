@@ -209,11 +209,12 @@ static int attn_launch(const uint16_t* q, const void* kc, const void* vc, uint16
 int pf_attention(const uint16_t* q, const void* kc, const void* vc, int kv_dtype, uint16_t* out, int T, int pos0, int S, int hd, int heads,
                  int kv_heads, cudaStream_t st) {
     SLLM_REQUIRE(q && kc && vc && out && T > 0 && pos0 >= 0 && pos0 + T <= S, SLLM_EINVAL, "pf_attention: bad argument");
+    SLLM_REQUIRE((((uintptr_t)q | (uintptr_t)kc | (uintptr_t)vc) % 16) == 0 && ((uintptr_t)out % 4) == 0, SLLM_EINVAL,
+                 "pf_attention: queries and caches are read 16 bytes at a time and the result is written 4 at a time: their addresses have to be such multiples");
     // bf16 caches: tcgen05. Measured, mma.sync | tcgen05: 2048 queries behind 6144 positions, 32 heads over 8 of 128 1062 | 350 us (687 TFLOP/s); 2048 and 512
     // queries from position 0, 32 heads 180 | 83 and 23 | 14 us; 64 and 128 queries of 32 and 8 heads 11.5 | 11.8 and 12.0 | 11.9 us. The kernel below keeps fp32
     // caches, and results that do not start at a multiple of 16 bytes.
-    const bool aligned = (((uintptr_t)q | (uintptr_t)kc | (uintptr_t)vc | (uintptr_t)out) % 16) == 0;
-    if (kv_dtype == SLLM_BF16 && aligned && (hd == 64 || hd == 128)) return pf_attention_tc(q, kc, vc, out, T, pos0, S, hd, heads, kv_heads, st);
+    if (kv_dtype == SLLM_BF16 && ((uintptr_t)out % 16) == 0 && (hd == 64 || hd == 128)) return pf_attention_tc(q, kc, vc, out, T, pos0, S, hd, heads, kv_heads, st);
     if (hd == 128) return kv_dtype == SLLM_F32 ? attn_launch<128, SLLM_F32>(q, kc, vc, out, T, pos0, S, heads, kv_heads, st)
                                                : attn_launch<128, SLLM_BF16>(q, kc, vc, out, T, pos0, S, heads, kv_heads, st);
     if (hd == 64) return kv_dtype == SLLM_F32 ? attn_launch<64, SLLM_F32>(q, kc, vc, out, T, pos0, S, heads, kv_heads, st)
