@@ -488,7 +488,9 @@ extern "C" int sllm_seq_linear(const float* A, int32_t lda, const void* W, int32
     LinArgs p{A, W, bias, C, lda, ldw, ldc, T, N, K, w_dtype, accumulate, round_a, alpha, a_bs, w_bs, bias_bs, c_bs, rows_dev, nullptr, 0, 0};
     if (T <= kRowsMax) return launch_rows(p, batch, st);
     // tensor cores: bf16 weights, a dense bf16 copy of A, rows that TMA can address (16-byte multiples) and enough work to fill tiles
-    if (a16 && sllm_seq_linear_on_tensor_cores(T, N, K, w_dtype, ldw, batch, round_a) && (((uintptr_t)W | (uintptr_t)a16) % 16) == 0) {
+    const bool tensor_cores = a16 && sllm_seq_linear_on_tensor_cores(T, N, K, w_dtype, ldw, batch, round_a) && ((uintptr_t)W % 16) == 0;
+    SLLM_REQUIRE(!tensor_cores || !a16_ready || ((uintptr_t)a16 % 16) == 0, SLLM_EINVAL, "seq_linear: bf16 rows that do not start at a multiple of 16 bytes");
+    if (tensor_cores && ((uintptr_t)a16 % 16) == 0) {
         static PfCache* cache = pf_cache_create();
         if (!a16_ready) {   // else the kernel that produced A has left its bf16 rows in a16 already
             const size_t n = (size_t)T * K / 8;
