@@ -661,14 +661,19 @@ static int attention_run(const sllm_seq_batch* b, const float* q, int32_t ldq, i
         grid.y = p.heads / hpc;
         const dim3 block(64 * hpc);
         cudaStream_t st = as_stream(stream);
-        // Heads of 64 or 128 and steps of some size: tcgen05 (seq_attn_tc.cu). Measured, this body | tcgen05 with the merge where there is one, us: prompts of
-        // 1000, 311, 700 and 37 tokens, 16 heads over 4 of 128 170 | 50, capped 218 | 74; one of 4096, 32 heads over 8 2050 | 377; one of 512 51 | 33 (heads of
-        // 64, 32 over 32: 54 | 49); 256 tokens from the start and behind 2000 34 | 31 and 96 | 39 (heads of 64: 32 | 40); 128 and 16 tokens from the
-        // start 15 | 21 and 7.7 | 16 (a fixed part of some 14 us: queries, TMEM, barriers, rows out): below that size this body stays.
-        const bool tc = dk == dv && (dk == 64 || dk == 128) && b->n_qtiles >= (dk == 128 ? 8 : 16) && !p.cross && !v_in_k &&
-                        (((uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)out16 | (uintptr_t)ws) % 16) == 0;
-        // shares are for steps whose query tiles leave SMs idle (the tcgen05 body takes 128 rows of query heads and queries at a time)
-        if (tc && (out || out16) && (long long)b->n_qtiles * kBQ * heads / 128 >= 2LL * sm_count()) p.nsplit = 1;
+        // Heads of 64 or 128 and steps of some size: tcgen05 (seq_attn_tc.cu), which has a fixed part of some 14 us (queries, TMEM, barriers, rows out). Measured, us, this
+        // body | tcgen05, each with the merge where there is one. Prompts of 1000, 311, 700 and 37 tokens, 16 heads over 4 of 128: 168 | 54, capped 215 | 81; one of 4096,
+        // 32 heads over 8 2050 | 468. Prompts from the start, heads of 128: 16 tiles 4 heads 25 | 23, 8 heads 31 | 30, 16 heads 50 | 33; 8 tiles 32 heads 58 | 53, 16 heads
+        // 33 | 31, but 8 heads 19.5 | 25.6 and 4 heads 14 | 20, 12 tiles of 4 heads 20 | 21. Heads of 64: 16 tiles 8 heads 24 | 23, 16 heads 31 | 33; 19 tiles 34 | 25 and
+        // 42 | 34. Longer contexts are always better off (8 heads, 256 tokens behind 1000 39 | 31, behind 4000 97 | 46), decoding requests beside a portion most of
+        // all: 4 behind 2500 to 6900 positions with 128 tokens, 32 heads 202 | 85, 8 heads 117 | 54; 8 with 16 tokens 242 | 83 and 169 | 110; 32 with 64 tokens 1309 | 335
+        // and 992 | 349. Contexts are not known here, but a list half of whose tiles hold one token tells such a step.
+        const bool mixed = b->T <= 17LL * b->n_qtiles;
+        const bool large = dk == 128 ? b->n_qtiles >= 16 || (b->n_qtiles >= 8 && ((long long)b->n_qtiles * heads >= 128 || mixed)) : b->n_qtiles >= 18 || (b->n_qtiles >= 16 && mixed);
+        const bool tc = dk == dv && (dk == 64 || dk == 128) && large && !p.cross && !v_in_k && (((uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)out16 | (uintptr_t)ws) % 16) == 0;
+        // Shares are for steps whose rows leave SMs idle (the tcgen05 body takes 128 rows of query heads and queries at a time). Rows, not tiles: a decoding request is a
+        // tile of one query with a long context.
+        if (tc && (out || out16) && (long long)b->T * heads / 128 >= 2LL * sm_count()) p.nsplit = 1;
         if (p.nsplit == 1 && !p.cross && (out || out16)) {
             p.out = out; p.ldo = ldo; p.out16 = out16;
             *merged = true;
