@@ -6,7 +6,7 @@
 // CTA = 64 queries of one head (4 warps x 16 rows), K/V tiles of 64 positions double-buffered in shared memory
 // with cp.async, XOR-swizzled 16-byte chunks (conflict-free ldmatrix), S = QK^T and O += PV with the P fragments
 // taken straight from the S accumulators. Heaviest query tiles are scheduled first (causal imbalance). bf16 caches go to the
-// tcgen05 kernel of prefill_attn_tc.cu.
+// tcgen05 kernel of prefill_attn_tc.cu where its larger tiles pay (pf_attention).
 #include "mega_common.cuh"
 #include "prefill.cuh"
 
@@ -211,10 +211,15 @@ int pf_attention(const uint16_t* q, const void* kc, const void* vc, int kv_dtype
     SLLM_REQUIRE(q && kc && vc && out && T > 0 && pos0 >= 0 && pos0 + T <= S, SLLM_EINVAL, "pf_attention: bad argument");
     SLLM_REQUIRE((((uintptr_t)q | (uintptr_t)kc | (uintptr_t)vc) % 16) == 0 && ((uintptr_t)out % 4) == 0, SLLM_EINVAL,
                  "pf_attention: queries and caches are read 16 bytes at a time and the result is written 4 at a time: their addresses have to be such multiples");
-    // bf16 caches: tcgen05. Measured, mma.sync | tcgen05: 2048 queries behind 6144 positions, 32 heads over 8 of 128 1062 | 350 us (687 TFLOP/s); 2048 and 512
-    // queries from position 0, 32 heads 180 | 83 and 23 | 14 us; 64 and 128 queries of 32 and 8 heads 11.5 | 11.8 and 12.0 | 11.9 us. The kernel below keeps fp32
-    // caches, and results that do not start at a multiple of 16 bytes.
-    if (kv_dtype == SLLM_BF16 && ((uintptr_t)out % 16) == 0 && (hd == 64 || hd == 128)) return pf_attention_tc(q, kc, vc, out, T, pos0, S, hd, heads, kv_heads, st);
+    // bf16 caches: tcgen05 (128 queries x 128 keys a tile), where its tiles are not mostly padding. Measured, us, mma.sync | tcgen05, heads of 128, 32 over 8: 2048 queries
+    // behind 6144 positions 1061 | 390, 512 from the start 22.4 | 14.9, 256 9.8 | 9.2, one query behind 250, 1000 and 2000 9.4 | 7.8, 29.5 | 22.5 and 55.9 | 41.4; 192
+    // keys and 64 or fewer, where the last tile is half empty: 64 queries behind 128 7.9 | 8.2, 192 from the start 8.0 | 8.4, 64 4.9 | 5.7, one 4.6 | 5.3, but 16 behind
+    // 64 6.2 | 5.3 and 128 from the start 6.3 | 6.1. Heads of 64 fill a tile's time with half the products, so there it pays only where the 64-query tiles of the other
+    // kernel make more than one wave: 2048 queries, 32 heads 119 | 80, 700 of 16 heads behind 1234 51 | 39, but 256 of 32 heads behind 0 and 2000 6.6 | 8.0 and
+    // 42.2 | 44.3, 1000 of 8 heads behind 5000 106 | 107. The kernel below keeps the rest, fp32 caches, and results that do not start at a multiple of 16 bytes.
+    const int keys = pos0 + T;
+    const bool fills = hd == 128 ? keys > 192 || (keys > 64 && keys <= 128) : (long long)((T + kPaBQ - 1) / kPaBQ) * heads > sm_count();
+    if (kv_dtype == SLLM_BF16 && ((uintptr_t)out % 16) == 0 && (hd == 64 || hd == 128) && fills) return pf_attention_tc(q, kc, vc, out, T, pos0, S, hd, heads, kv_heads, st);
     if (hd == 128) return kv_dtype == SLLM_F32 ? attn_launch<128, SLLM_F32>(q, kc, vc, out, T, pos0, S, heads, kv_heads, st)
                                                : attn_launch<128, SLLM_BF16>(q, kc, vc, out, T, pos0, S, heads, kv_heads, st);
     if (hd == 64) return kv_dtype == SLLM_F32 ? attn_launch<64, SLLM_F32>(q, kc, vc, out, T, pos0, S, heads, kv_heads, st)
