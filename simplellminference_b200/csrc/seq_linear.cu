@@ -440,10 +440,15 @@ static int launch_rows(const sllm::LinArgs& p, int batch, cudaStream_t st) {
     const int e = bf16 ? 8 : 4;   // elements per 16-byte weight load
     const bool vec = p.K % e == 0 && p.ldw % e == 0 && (p.w_bs % e) == 0 && p.lda % 4 == 0 && (p.a_bs % 4) == 0 && ((uintptr_t)p.W % 16) == 0 &&
                      ((uintptr_t)p.A % 16) == 0;
-    // The streaming body starts 1.4 to 2 us later than the small one (its ring, its activations, more code) and is faster from about 2 million
-    // weights on. Measured, bf16, old | new: 1024 x 1024 3.8 | 4.1 us (one row) and 4.7 | 6.4 (four), 2048 x 2048 6.4 | 4.7 and 9.4 | 7.4, 32 matrices of
-    // 512 x 128 13.4 | 8.7 (four), 6144 x 4096 19.4 | 11.4 (one), 46.9 | 14.6 (four) and 85.4 | 21.7 (eight), 32000 x 2048 40.1 | 24.5 (one row).
-    if (vec && (long long)p.N * batch * p.K >= 1500000LL) {
+    // The streaming body needs a few us to start (its ring, its activations, more code). Measured, us, small body | streaming. Up to four rows it is ahead from 1.5 million
+    // weights on: 1536 x 1024 bf16 5.2 | 4.2 (one row), 6.1 | 6.0 (three), 6.6 | 6.3 (four), fp32 5.8 | 4.7 and 6.1 | 5.0; 512 x 8192 bf16 5.4 | 5.2 and 8.6 | 7.5; 6144 x
+    // 4096 19.4 | 11.4 and 46.9 | 14.6. From five rows on its CTAs hold half the warps and read eight rows of activations each, whatever share of the weights they have:
+    // bf16 2048 x 1024 7.8 | 8.2 (five), 512 x 8192 9.7 | 11.9 and 13.0 | 12.8 (eight), but 2800 x 1024 9.5 | 8.8, 768 x 8192 15.9 | 13.2, 6144 x 4096 85.4 | 21.7 (eight);
+    // fp32 2048 x 1024 7.0 | 7.7, 1024 x 4096 9.7 | 11.0, 1024 x 11008 20.5 | 23.4, but 2800 x 1024 8.6 | 8.4, 1500 x 11008 34.0 | 29.0. Several products in a launch: 74 of
+    // 512 x 512 24 | 9.9 (one row) and 57 | 21 (eight), 80, which leave 68 SMs without one, 26 | 15 and 61 | 33, 160 of 128 x 2048 29 | 24 and 107 | 59.
+    const long long rows = (long long)p.N * batch;
+    const bool stream = vec && (p.T <= 4 ? rows * p.K >= 1500000LL : rows * p.K >= 2800000LL && rows >= (bf16 ? 5LL : 10LL) * sm_count());
+    if (stream) {
         int rc;
         if (p.T == 1) rc = bf16 ? launch_rows_body<SLLM_BF16, 1>(p, batch, st) : launch_rows_body<SLLM_F32, 1>(p, batch, st);
         else if (p.T == 2) rc = bf16 ? launch_rows_body<SLLM_BF16, 2>(p, batch, st) : launch_rows_body<SLLM_F32, 2>(p, batch, st);
