@@ -538,7 +538,7 @@ class StateSpaceDuality:
         y = step.scratch("ssd_y", T * inner)
         args = (step.b, u.data_ptr(), C, u.data_ptr() + inner * F32B, C, u.data_ptr() + (inner + gn) * F32B, C, dt, ld, self.a_log, self.dt_bias,
                 self.skip, c.heads, c.groups, c.state, c.vdim, state["S"], y, inner, xbc, ld, C, c.conv, ring, step.st)
-        blocks = step.ssd_block_scratch(c.heads, c.groups, c.state)
+        blocks = step.ssd_block_scratch(c.heads, c.groups, c.state, c.vdim)
         if blocks is not None:
             ops.ssd_blocks(*args, block_ws=blocks)
         else:
