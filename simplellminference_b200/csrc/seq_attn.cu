@@ -598,7 +598,7 @@ static int attention_decode_bf16(const sllm::AttnArgs& p, cudaStream_t st) {
 template <int L, int G, int S>      // loads per lane of a row, query heads of a CTA, rows in flight per lane
 static int attention_decode_f32(const sllm::AttnArgs& p, cudaStream_t st) {
     using namespace sllm;
-    auto* kernel = seq_attention_decode_kernel<float, L, L, G, S>;
+    auto* kernel = seq_attention_decode_kernel<L, G, S>;
     static bool ready = false;
     if (!ready) {
         SLLM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));

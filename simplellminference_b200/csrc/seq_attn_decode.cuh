@@ -52,13 +52,7 @@ __device__ __forceinline__ int page_of(int pos, int page_len, uint32_t magic, in
 }
 
 // 16 bytes of a cache row as pairs of floats
-__device__ __forceinline__ void cache_pairs(const uint4& u, uint64_t (&p)[4], const uint16_t*) {
-    p[0] = pair_f32(u.x << 16, u.x & 0xffff0000u);
-    p[1] = pair_f32(u.y << 16, u.y & 0xffff0000u);
-    p[2] = pair_f32(u.z << 16, u.z & 0xffff0000u);
-    p[3] = pair_f32(u.w << 16, u.w & 0xffff0000u);
-}
-__device__ __forceinline__ void cache_pairs(const uint4& u, uint64_t (&p)[2], const float*) {
+__device__ __forceinline__ void cache_pairs(const uint4& u, uint64_t (&p)[2]) {
     p[0] = pair_f32(u.x, u.y);
     p[1] = pair_f32(u.z, u.w);
 }
@@ -72,16 +66,16 @@ constexpr int kDecodeWarps = 4, kDecodeCluster = 16;     // warps of a CTA, CTAs
 // every score on one lane for its exponential. A sequence's rows are dealt in runs of 4 x kSteps keys to all warps of a thread-block cluster, so that
 // the longest context of a step is spread over up to 16 CTAs whatever the step's share count; every warp sends its sums to the CTAs that own the
 // columns (distributed shared memory, one barrier), which merge them and write the result (or one record per share when something still follows).
-template <typename KV, int KL, int VL, int G, int kSteps>     // 16-byte loads per lane of a key / value row: dk = 8 * KL * E, dv = 8 * VL * E
+template <int L, int G, int kSteps>     // 16-byte loads per lane of a key or value row: heads of D = 32 L
 __global__ void __launch_bounds__(kDecodeWarps * 32) seq_attention_decode_kernel(AttnArgs p) {
     namespace cg = cooperative_groups;
-    constexpr int E = 16 / sizeof(KV), PE = E / 2, dk = 8 * KL * E, dv = 8 * VL * E, VAL = G * kSteps;
+    constexpr int E = 4, PE = E / 2, D = 8 * L * E, VAL = G * kSteps;
     constexpr int kPer = VAL >= 8 ? VAL / 8 : 1, kDup = VAL >= 8 ? 1 : 8 / VAL;      // scores per lane after the exchange, lanes that hold the same one
     constexpr int kRun = 4 * kSteps;                                                  // keys of one step of a warp
     static_assert(kBK % kRun == 0, "a run of keys lies inside one tile");
-    constexpr int kPairs = G * VL * PE;                  // pairs of sums a lane keeps
-    // what the cluster's warps send this CTA: their sums for its share of the G * dv results, and every warp's (maximum, sum) per head
-    __shared__ __align__(16) float got_o[kDecodeWarps * G * dv];
+    constexpr int kPairs = G * L * PE;                  // pairs of sums a lane keeps
+    // what the cluster's warps send this CTA: their sums for its share of the G * D results, and every warp's (maximum, sum) per head
+    __shared__ __align__(16) float got_o[kDecodeWarps * G * D];
     __shared__ __align__(16) float2 got_ml[kDecodeCluster * kDecodeWarps][G];
     __shared__ float weight[kDecodeCluster * kDecodeWarps][G], total[G][2];
     const sllm_seq_batch& b = p.b;
@@ -95,16 +89,16 @@ __global__ void __launch_bounds__(kDecodeWarps * 32) seq_attention_decode_kernel
     const TileList tiles(pos, pos, wnd, p.keep_first, kBK);
     constexpr int kRuns = kBK / kRun;
     const int n_runs = tiles.n * kRuns, workers = p.nsplit * CS * kDecodeWarps;
-    const KV* kp = reinterpret_cast<const KV*>(p.k_pool);
-    const KV* vp = reinterpret_cast<const KV*>(p.v_pool);
+    const float* kp = reinterpret_cast<const float*>(p.k_pool);
+    const float* vp = reinterpret_cast<const float*>(p.v_pool);
     const int32_t* table = b.block_table + (size_t)slot * b.max_pages;
 
-    uint64_t qv[G][KL * PE];
+    uint64_t qv[G][L * PE];
 #pragma unroll
     for (int g = 0; g < G; ++g)
 #pragma unroll
-        for (int i = 0; i < KL; ++i) {
-            const float* src = p.q + (size_t)t * p.ldq + (size_t)(h0 + g) * dk + (i * 8 + j8) * E;
+        for (int i = 0; i < L; ++i) {
+            const float* src = p.q + (size_t)t * p.ldq + (size_t)(h0 + g) * D + (i * 8 + j8) * E;
 #pragma unroll
             for (int e = 0; e < PE; ++e) qv[g][i * PE + e] = pair_f32(src[2 * e], src[2 * e + 1]);
         }
@@ -113,31 +107,31 @@ __global__ void __launch_bounds__(kDecodeWarps * 32) seq_attention_decode_kernel
     const float slope = p.slopes ? p.slopes[h0 + og] : 0.0f;
     const float r1 = p.logdist ? p.logdist[h0 + og] : 0.0f, r2 = p.logdist ? p.logdist[p.heads + h0 + og] : 0.0f;
     float m[G], l = 0.0f;                       // running maxima (all lanes alike); this lane's share of the sum of head og
-    uint64_t acc[G][VL * PE];
+    uint64_t acc[G][L * PE];
 #pragma unroll
     for (int g = 0; g < G; ++g) {
         m[g] = -INFINITY;
 #pragma unroll
-        for (int i = 0; i < VL * PE; ++i) acc[g][i] = 0ull;
+        for (int i = 0; i < L * PE; ++i) acc[g][i] = 0ull;
     }
     auto first_key = [&](int run) { return tiles.tile_of(run / kRuns) * kBK + run % kRuns * kRun; };
     // rows the sequence does not have yet read as zeros (their memory may hold anything)
-    auto load_keys = [&](uint4 (&u)[kSteps][KL], int j0, int page) {
-        const KV* row = kp + seq_pool_row(page, p.kv_heads, gkv, b.page_len, j0 % b.page_len + kg, dk) + j8 * E;
+    auto load_keys = [&](uint4 (&u)[kSteps][L], int j0, int page) {
+        const float* row = kp + seq_pool_row(page, p.kv_heads, gkv, b.page_len, j0 % b.page_len + kg, D) + j8 * E;
 #pragma unroll
         for (int s = 0; s < kSteps; ++s)
 #pragma unroll
-            for (int i = 0; i < KL; ++i) u[s][i] = j0 + 4 * s + kg <= pos ? ldg_stream(row + (size_t)(4 * s) * dk + i * 8 * E) : make_uint4(0u, 0u, 0u, 0u);
+            for (int i = 0; i < L; ++i) u[s][i] = j0 + 4 * s + kg <= pos ? ldg_stream(row + (size_t)(4 * s) * D + i * 8 * E) : make_uint4(0u, 0u, 0u, 0u);
     };
-    auto load_values = [&](uint4 (&u)[kSteps][VL], int j0, int page) {
-        const KV* row = vp + seq_pool_row(page, p.kv_heads, gkv, b.page_len, j0 % b.page_len + kg, dv) + j8 * E;
+    auto load_values = [&](uint4 (&u)[kSteps][L], int j0, int page) {
+        const float* row = vp + seq_pool_row(page, p.kv_heads, gkv, b.page_len, j0 % b.page_len + kg, D) + j8 * E;
 #pragma unroll
         for (int s = 0; s < kSteps; ++s)
 #pragma unroll
-            for (int i = 0; i < VL; ++i) u[s][i] = j0 + 4 * s + kg <= pos ? ldg_stream(row + (size_t)(4 * s) * dv + i * 8 * E) : make_uint4(0u, 0u, 0u, 0u);
+            for (int i = 0; i < L; ++i) u[s][i] = j0 + 4 * s + kg <= pos ? ldg_stream(row + (size_t)(4 * s) * D + i * 8 * E) : make_uint4(0u, 0u, 0u, 0u);
     };
     // A run's keys are asked for as soon as the previous run's have been multiplied, its values likewise: one of the two is always on its way.
-    uint4 ku[kSteps][KL], vu[kSteps][VL];
+    uint4 ku[kSteps][L], vu[kSteps][L];
     int run = (split * CS + rank) * kDecodeWarps + warp, page = 0;
     if (run < n_runs) {
         const int j0 = first_key(run);
@@ -156,9 +150,9 @@ __global__ void __launch_bounds__(kDecodeWarps * 32) seq_attention_decode_kernel
 #pragma unroll
             for (int g = 0; g < G; ++g) d[g] = 0ull;
 #pragma unroll
-            for (int i = 0; i < KL; ++i) {
+            for (int i = 0; i < L; ++i) {
                 uint64_t kk[PE];
-                cache_pairs(ku[s][i], kk, kp);
+                cache_pairs(ku[s][i], kk);
 #pragma unroll
                 for (int g = 0; g < G; ++g)
 #pragma unroll
@@ -205,7 +199,7 @@ __global__ void __launch_bounds__(kDecodeWarps * 32) seq_attention_decode_kernel
                 const float corr = mn[g] == -INFINITY ? 1.0f : expf(m[g] - mn[g]);
                 const uint64_t c2 = pair_f32(corr, corr);
 #pragma unroll
-                for (int i = 0; i < VL * PE; ++i) asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(acc[g][i]) : "l"(c2));
+                for (int i = 0; i < L * PE; ++i) asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(acc[g][i]) : "l"(c2));
                 m[g] = mn[g];
             }
         }
@@ -224,9 +218,9 @@ __global__ void __launch_bounds__(kDecodeWarps * 32) seq_attention_decode_kernel
                 w2[g] = pair_f32(w, w);
             }
 #pragma unroll
-            for (int i = 0; i < VL; ++i) {
+            for (int i = 0; i < L; ++i) {
                 uint64_t vv[PE];
-                cache_pairs(vu[s][i], vv, vp);
+                cache_pairs(vu[s][i], vv);
 #pragma unroll
                 for (int g = 0; g < G; ++g)
 #pragma unroll
@@ -239,7 +233,7 @@ __global__ void __launch_bounds__(kDecodeWarps * 32) seq_attention_decode_kernel
     // The warp's four groups of keys: in two exchanges a lane gives away three quarters of its pairs and gets the others' parts of the rest.
     uint64_t v[kPairs];
 #pragma unroll
-    for (int i = 0; i < kPairs; ++i) v[i] = acc[i / (VL * PE)][i % (VL * PE)];
+    for (int i = 0; i < kPairs; ++i) v[i] = acc[i / (L * PE)][i % (L * PE)];
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
         const int bit = half ? 8 : 16, n = half ? kPairs / 4 : kPairs / 2;
@@ -255,12 +249,12 @@ __global__ void __launch_bounds__(kDecodeWarps * 32) seq_attention_decode_kernel
 #pragma unroll
     for (int g = 0; g < G; ++g) lg[g] = warp_sum(og == g ? l : 0.0f);
     // every CTA of the cluster gets the sums of its own share of the results, and everybody's maxima
-    const int share = G * dv / CS, worker = rank * kDecodeWarps + warp;
+    const int share = G * D / CS, worker = rank * kDecodeWarps + warp;
     cluster.barrier_wait();
 #pragma unroll
     for (int i = 0; i < kPairs / 4; ++i) {
-        const int at = kg * (kPairs / 4) + i, g = at / (VL * PE), r = at % (VL * PE);
-        const int item = g * dv + (r / PE * 8 + j8) * E + r % PE * 2, to = item / share;
+        const int at = kg * (kPairs / 4) + i, g = at / (L * PE), r = at % (L * PE);
+        const int item = g * D + (r / PE * 8 + j8) * E + r % PE * 2, to = item / share;
         *reinterpret_cast<uint64_t*>(cluster.map_shared_rank(got_o, to) + worker * share + item % share) = v[i];
     }
     if (lane < CS) {
@@ -271,32 +265,32 @@ __global__ void __launch_bounds__(kDecodeWarps * 32) seq_attention_decode_kernel
     cluster.sync();
     if (warp < G) {
         const int n = CS * kDecodeWarps;
-        float M = -INFINITY, L = 0.0f;
+        float M = -INFINITY, sum = 0.0f;
         for (int i = lane; i < n; i += 32) M = fmaxf(M, got_ml[i][warp].x);
         M = warp_max(M);
         for (int i = lane; i < n; i += 32) {
             const float f = got_ml[i][warp].x == -INFINITY ? 0.0f : expf(got_ml[i][warp].x - M);
             weight[i][warp] = f;
-            L = fmaf(got_ml[i][warp].y, f, L);
+            sum = fmaf(got_ml[i][warp].y, f, sum);
         }
-        L = warp_sum(L);
+        sum = warp_sum(sum);
         if (lane == 0) {
             total[warp][0] = M;
-            total[warp][1] = L;
+            total[warp][1] = sum;
         }
     }
     __syncthreads();
     for (int i = threadIdx.x; i < share; i += kDecodeWarps * 32) {
-        const int item = rank * share + i, g = item / dv, c = item % dv;
+        const int item = rank * share + i, g = item / D, c = item % D;
         float o = 0.0f;
 #pragma unroll 4
         for (int w = 0; w < CS * kDecodeWarps; ++w) o = fmaf(got_o[w * share + i], weight[w][g], o);
         if (p.out || p.out16) {
             o *= 1.0f / total[g][1];
-            if (p.out) p.out[(size_t)t * p.ldo + (size_t)(h0 + g) * dv + c] = o;
-            if (p.out16) p.out16[((size_t)t * p.heads + h0 + g) * dv + c] = f32_to_bf16_bits(o);
+            if (p.out) p.out[(size_t)t * p.ldo + (size_t)(h0 + g) * D + c] = o;
+            if (p.out16) p.out16[((size_t)t * p.heads + h0 + g) * D + c] = f32_to_bf16_bits(o);
         } else {
-            float* rec = p.ws + (((size_t)t * p.heads + h0 + g) * p.nsplit + split) * (dv + 2);
+            float* rec = p.ws + (((size_t)t * p.heads + h0 + g) * p.nsplit + split) * (D + 2);
             rec[2 + c] = o;
             if (c == 0) {
                 rec[0] = total[g][0];

@@ -157,7 +157,6 @@ class SequenceEngine:
         self._meta_dev = None
         self._meta_host = None
         self._meta_event = None
-        self._meta_used = False
         self._meta_offsets = np.zeros(13, np.int64)
         self.step_obj = Step(self)
         self.steps_run = 0
@@ -223,7 +222,7 @@ class SequenceEngine:
                 _lib.check_seq(int(n))
             return int(n)
 
-        if self._meta_used:
+        if self._meta_event is not None:
             self._meta_event.synchronize()          # the previous step's copy has left the pinned buffer
         total = run(self._meta_host)
         if self._meta_host is None or self._meta_host.numel() < total:
@@ -238,7 +237,6 @@ class SequenceEngine:
             if self._meta_event is None:
                 self._meta_event = torch.cuda.Event()
             self._meta_event.record()
-            self._meta_used = True
         base = self._meta_dev.data_ptr()
         return [base + 4 * o for o in self._meta_offsets.tolist()], n_tiles.value
 

@@ -1,7 +1,7 @@
-"""Attention of single-token steps (sllm_seq_attention / sllm_seq_attention_out with one query per sequence) in the body that reads the pools straight
-into registers: contexts that end anywhere in a run, a tile or a page, every number of query heads a CTA can hold, both pool types, every way in which a
-score can be changed or hidden, shares merged by the caller and results written by the launch. Cache rows beyond a context hold NaN.
-Against float64 on the same operands; fp32 sums over at most 3000 keys stay within 2e-6."""
+"""Attention of single-token steps (sllm_seq_attention / sllm_seq_attention_out with one query per sequence): over fp32 pools in the body that reads them straight
+into registers, over bf16 pools in the one whose tensor-core products take three bf16 terms. Contexts that end anywhere in a run, a tile or a page, every number
+of query heads a CTA can hold, every way in which a score can be changed or hidden, shares merged by the caller and results written by the launch. Cache rows
+beyond a context hold NaN. Against float64 on the same operands; fp32 sums over at most 3000 keys stay within 2e-6."""
 import math
 
 import numpy as np
