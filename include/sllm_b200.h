@@ -617,8 +617,8 @@ int sllm_seq_ssd_scan(const sllm_seq_batch* b, const float* x, int32_t ldx, cons
                       const float* step_logit, int32_t lda, const float* A_log, const float* dt_bias, const float* skip, int32_t heads, int32_t groups,
                       int32_t n_state, int32_t dv, float* state, float* y, int32_t ldy, const float* conv_x, int32_t ld_conv, int32_t channels,
                       int32_t taps, float* ring, float* scratch, sllm_stream_t stream);
-/* sllm_seq_ssd_scan in blocks of 64 tokens on the tensor cores, for steps that hold portions of prompts: state and sums fp32, operands as two bf16 terms each
- * (the fp32 form stays sllm_seq_ssd_scan). n_state <= 128; block_ws: sllm_seq_ssd_block_ws_bytes of scratch, 16-byte aligned. */
+/* sllm_seq_ssd_scan in blocks of 64 tokens on the tensor cores, for steps that hold portions of prompts: state and sums fp32, operands as three bf16
+ * terms each (24 bits). n_qtiles has to count every token's tile: it sizes the scratch. n_state <= 128; block_ws: sllm_seq_ssd_block_ws_bytes of scratch, 16-byte aligned. */
 int64_t sllm_seq_ssd_block_ws_bytes(int32_t n_qtiles, int32_t nseg, int32_t heads, int32_t groups, int32_t n_state);
 int sllm_seq_ssd_blocks(const sllm_seq_batch* b, const float* x, int32_t ldx, const float* B, int32_t ldb, const float* C, int32_t ldc,
                         const float* step_logit, int32_t lda, const float* A_log, const float* dt_bias, const float* skip, int32_t heads, int32_t groups,

@@ -1,7 +1,8 @@
 """Attention of prompt portions on tcgen05 (sllm_seq_attention / sllm_seq_attention_out, bf16 pools): portions that end anywhere in a tile, several at once and
 behind a cached context, one, two and four query heads of a kv head in a CTA, pages of other lengths than a tile, every option, shares merged by the caller
 and results written by the launch, maxima that keep growing. Cache rows beyond a portion hold NaN. Against float64 on the bf16-rounded queries: the
-weights keep 2^-17 (two bf16 terms), the fp32 sums of at most 1400 keys far less; 2e-5 of the result's norm."""
+weights keep 2^-24 (three bf16 terms), the sums of at most 1400 keys a few 2^-23 a tile; 2e-5 of the result's norm is generous (tighter:
+test_attention_forms_gpu.py)."""
 import math
 
 import numpy as np

@@ -1,7 +1,7 @@
 """State-space duality in blocks of 64 tokens on the tensor cores (sllm_seq_ssd_blocks): portions that end anywhere in a block, several portions in one
 step that go on from a state, states and columns that are multiples of nothing, groups, with and without the skip term, decays that forget within a
-token and ones that hardly forget. Against float64 on the same fp32 inputs; two bf16 terms per operand leave 2^-17 of each product, whose signs differ:
-2e-5 of the result at most, as in the block form of the delta rule. The ring afterwards is that of sllm_seq_ssd_scan, bit for bit."""
+token and ones that hardly forget. Against float64 on the same fp32 inputs; three bf16 terms per operand leave 2^-24 of each product:
+2e-5 of the result is generous (tighter: test_ssd_blocks_terms_gpu.py). The ring afterwards is that of sllm_seq_ssd_scan, bit for bit."""
 import numpy as np
 import pytest
 
