@@ -218,7 +218,9 @@ constexpr int kInFlight = 2;   // 16-byte weight loads per batch and lane; two b
 
 // Small matrices (launch_rows says which) and accesses that are not 16 bytes wide: `wpr` warps (1, 2, 4 or 8) share one output column and cut K among them, so that a matrix with few rows and long rows still fills the
 // machine; a lane keeps two batches of 16-byte weight loads in flight (the next batch travels while this one is multiplied). The partial sums of a column meet in shared memory in a fixed order.
-template <int WD>
+// kShort: a load's products are summed before they join the sum of a lane, as many roundings in a row as in the streaming body (error of fp32 1000 x 11008 at five rows
+// 1.13e-7, else 1.2e-7; streaming 1.08e-7), for the larger ones of these products; 2 to 8 % slower, so not for the others.
+template <int WD, bool kShort>
 __global__ void __launch_bounds__(256, 4) seq_linear_rows_small_kernel(LinArgs p, int vec, int wpr) {
     __shared__ float part_sum[8][kRowsMax];
     const int b = blockIdx.y;
@@ -261,13 +263,15 @@ __global__ void __launch_bounds__(256, 4) seq_linear_rows_small_kernel(LinArgs p
                         for (int t = 0; t < kRowsMax; ++t) {
                             if (t < p.T) {
                                 const float* ar = A + (size_t)t * p.lda + k;
+                                float sum = kShort ? 0.0f : acc[t];
 #pragma unroll
                                 for (int e = 0; e < E; e += 4) {
                                     const float4 a4 = *reinterpret_cast<const float4*>(ar + e);
                                     const float av[4] = {a4.x, a4.y, a4.z, a4.w};
 #pragma unroll
-                                    for (int i = 0; i < 4; ++i) acc[t] = fmaf(p.round_a ? seq_round_bf16(av[i]) : av[i], wv[e + i], acc[t]);
+                                    for (int i = 0; i < 4; ++i) sum = fmaf(p.round_a ? seq_round_bf16(av[i]) : av[i], wv[e + i], sum);
                                 }
+                                acc[t] = kShort ? acc[t] + sum : sum;
                             }
                         }
                     }
@@ -442,12 +446,15 @@ static int launch_rows(const sllm::LinArgs& p, int batch, cudaStream_t st) {
                      ((uintptr_t)p.A % 16) == 0;
     // The streaming body needs a few us to start (its ring, its activations, more code). Measured, us, small body | streaming. Up to four rows it is ahead from 1.5 million
     // weights on: 1536 x 1024 bf16 5.2 | 4.2 (one row), 6.1 | 6.0 (three), 6.6 | 6.3 (four), fp32 5.8 | 4.7 and 6.1 | 5.0; 512 x 8192 bf16 5.4 | 5.2 and 8.6 | 7.5; 6144 x
-    // 4096 19.4 | 11.4 and 46.9 | 14.6. From five rows on its CTAs hold half the warps and read eight rows of activations each, whatever share of the weights they have:
-    // bf16 2048 x 1024 7.8 | 8.2 (five), 512 x 8192 9.7 | 11.9 and 13.0 | 12.8 (eight), but 2800 x 1024 9.5 | 8.8, 768 x 8192 15.9 | 13.2, 6144 x 4096 85.4 | 21.7 (eight);
-    // fp32 2048 x 1024 7.0 | 7.7, 1024 x 4096 9.7 | 11.0, 1024 x 11008 20.5 | 23.4, but 2800 x 1024 8.6 | 8.4, 1500 x 11008 34.0 | 29.0. Several products in a launch: 74 of
-    // 512 x 512 24 | 9.9 (one row) and 57 | 21 (eight), 80, which leave 68 SMs without one, 26 | 15 and 61 | 33, 160 of 128 x 2048 29 | 24 and 107 | 59.
-    const long long rows = (long long)p.N * batch;
-    const bool stream = vec && (p.T <= 4 ? rows * p.K >= 1500000LL : rows * p.K >= 2800000LL && rows >= (bf16 ? 5LL : 10LL) * sm_count());
+    // 4096 19.4 | 11.4 and 46.9 | 14.6. From five rows on its CTAs hold half the warps and read eight rows of activations each, whatever share of the weights they have.
+    // bf16, five rows | eight rows: 2048 x 1024 7.8 | 8.2, 9.5 | 8.7; 512 x 8192 9.7 | 11.9, 13.0 | 12.8; 2800 x 1024 9.5 | 8.8, 12.5 | 9.3; 700 x 8000 16.2 | 13.1, 23.7 | 14.0;
+    // 6144 x 4096 85.4 | 21.7 (eight). fp32: 2048 x 1024 7.0 | 7.7, 7.7 | 8.2; 1024 x 4096 9.7 | 11.0, 11.3 | 11.9; 512 x 8192 8.8 | 13.8, 10.2 | 15.7; 600 x 8000 13.6 | 15.2,
+    // 18.8 | 16.9; 1000 x 11008 22.0 | 23.4, 26.3 | 26.2; 2800 x 1024 8.6 | 8.4, 9.6 | 8.9; 1500 x 11008 34.0 | 29.0, 43.7 | 32.1. Several products in a launch: 74 of 512 x
+    // 512 24 | 9.9 (one row) and 57 | 21 (eight), 80, which leave 68 SMs without one, 26 | 15 and 61 | 33, 160 of 128 x 2048 29 | 24 and 107 | 59.
+    const long long rows = (long long)p.N * batch, weights = rows * p.K, sms = sm_count();
+    const bool stream = vec && (p.T <= 4          ? weights >= 1500000LL
+                                : bf16 ? p.T <= 6 ? weights >= 2800000LL && rows >= 4 * sms : weights >= 2000000LL
+                                                  : (weights >= 2800000LL && rows >= 10 * sms) || (p.T >= 7 && weights >= 4500000LL && rows >= 4 * sms));
     if (stream) {
         int rc;
         if (p.T == 1) rc = bf16 ? launch_rows_body<SLLM_BF16, 1>(p, batch, st) : launch_rows_body<SLLM_F32, 1>(p, batch, st);
@@ -459,8 +466,11 @@ static int launch_rows(const sllm::LinArgs& p, int batch, cudaStream_t st) {
         int wpr = 1;   // warps per output column: enough CTAs for ~4 per SM, and no warp with less than 256 weights
         while (wpr < 8 && (long long)p.N * batch * wpr / 8 < 4LL * sm_count() && p.K / (2 * wpr) >= 256) wpr *= 2;
         dim3 grid(((long long)p.N * wpr + 7) / 8, batch);
-        if (bf16) seq_linear_rows_small_kernel<SLLM_BF16><<<grid, 256, 0, st>>>(p, vec, wpr);
-        else seq_linear_rows_small_kernel<SLLM_F32><<<grid, 256, 0, st>>>(p, vec, wpr);
+        const bool brief = weights >= 1500000LL;
+        if (bf16 && brief) seq_linear_rows_small_kernel<SLLM_BF16, true><<<grid, 256, 0, st>>>(p, vec, wpr);
+        else if (bf16) seq_linear_rows_small_kernel<SLLM_BF16, false><<<grid, 256, 0, st>>>(p, vec, wpr);
+        else if (brief) seq_linear_rows_small_kernel<SLLM_F32, true><<<grid, 256, 0, st>>>(p, vec, wpr);
+        else seq_linear_rows_small_kernel<SLLM_F32, false><<<grid, 256, 0, st>>>(p, vec, wpr);
     }
     ++g_launches;
     SLLM_LAUNCH_CHECK();
