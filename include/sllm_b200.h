@@ -55,6 +55,10 @@ const char* sllm_last_error(void);
  * has found index arrays that contradict the host's counts, else SLLM_OK. Every call that launches kernels or waits for them reports the same, so a program
  * needs this only behind a synchronisation of its own. */
 int sllm_status(void);
+/* Turns edges of a captured graph (cudaGraph_t, not yet instantiated) into programmatic ones: a kernel of this library that waits for its predecessor itself, and has
+ * one predecessor, a kernel, may become resident while that one still runs. What it reads and writes behind that wait, and so every result, is the same. *edges (or
+ * NULL): how many were changed. */
+int sllm_graph_overlap(void* graph, int32_t* edges);
 int sllm_abi_version(void);
 /* development knobs (not part of the drop-in surface): key 0 = GEMV CTAs per SM (0 = built-in choice); prefill GEMM: key 1 = force
  * the N extent of a tile (multiple of 32, 0 = cost model), key 2 = two-SM tiles (1 / 0 force / forbid, -1 = by T), key 3 = programmatic
@@ -448,7 +452,9 @@ int sllm_seq_hyper_write_read(float* x, int32_t streams, int32_t T, int32_t d, c
  * its rows in a16 as dense bf16 [T][K] (sllm_seq_depth_average, sllm_seq_layernorm and sllm_seq_clamped_glu can), so that the copy is
  * skipped; only meaningful when sllm_seq_linear_on_tensor_cores says the product goes there. rows_dev (device memory or NULL): a row
  * count an earlier kernel left; rows from *rows_dev on (of the T the call names) are not computed and their outputs stay as they are
- * (steps of more than 8 tokens; smaller steps compute all T rows). */
+ * (steps of more than 8 tokens; smaller steps compute all T rows). round_a may carry SLLM_SEQ_W_FIXED: nothing enqueued since the start of the graph that is being
+ * captured writes W, so that the weights may be read before the kernel in front of this one has completed (sllm_graph_overlap). */
+#define SLLM_SEQ_W_FIXED 0x100
 int sllm_seq_linear(const float* A, int32_t lda, const void* W, int32_t w_dtype, int32_t ldw, const float* bias, float* C, int32_t ldc,
                     int32_t T, int32_t N, int32_t K, float alpha, int32_t accumulate, int32_t round_a, int32_t batch, int64_t a_bs,
                     int64_t w_bs, int64_t bias_bs, int64_t c_bs, void* a16, int32_t a16_ready, const int32_t* rows_dev, sllm_stream_t stream);

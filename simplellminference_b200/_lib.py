@@ -32,6 +32,7 @@ class EngineConfig(C.Structure):
 ENGINE_UNFUSED, ENGINE_NO_GRAPH, ENGINE_PDL, ENGINE_P2P_ALLREDUCE, ENGINE_MEGAKERNEL, ENGINE_MEGA_LL = 1, 2, 4, 8, 16, 32
 ENGINE_MEGA_FUSE_DOWN = 64
 ENGINE_MEGA_V2 = 128
+SEQ_W_FIXED = 0x100       # SLLM_SEQ_W_FIXED
 EINVAL, ENOTSUP, ENOMEM, ESTATE, ECOMM, ETIMEOUT = -1, -2, -3, -4, -5, -6   # SLLM_E* of include/sllm_b200.h
 
 _P = C.c_void_p
@@ -43,6 +44,7 @@ _F = C.c_float
 SIGNATURES = {
     "sllm_last_error": (C.c_char_p, []),
     "sllm_status": (C.c_int, []),
+    "sllm_graph_overlap": (C.c_int, [_P, _P]),
     "sllm_abi_version": (C.c_int, []),
     "sllm_tune": (C.c_int, [_I, _I]),
     "sllm_device_info": (C.c_int, [C.POINTER(_I), C.POINTER(_I), C.POINTER(C.c_size_t), C.POINTER(C.c_size_t)]),
@@ -198,7 +200,7 @@ SIGNATURES.update({
 # translation units compiled, not all of them. The full library contains the same objects and is preferred when it exists.
 SEQ_LIB_PATH = os.path.join(HERE, "lib", "libsllm_b200_seq.so")
 SEQ_SYMBOL_PREFIXES = ("sllm_seq_", "sllm_kvpages_", "sllm_sample_", "sllm_last_error", "sllm_status", "sllm_abi_version", "sllm_tune", "sllm_device_info",
-                       "sllm_prefill_gemm_")
+                       "sllm_prefill_gemm_", "sllm_graph_")
 
 _lib = None
 _seq_lib = None

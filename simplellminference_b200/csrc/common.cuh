@@ -72,6 +72,15 @@ struct LaunchCfg {
     }
 };
 
+// A kernel that calls after_previous() on every path: in a captured step it may become resident while the kernel before it still runs (sllm_graph_overlap). The
+// launch itself is an ordinary one.
+void overlap_kernel(const void* kernel);
+template <class F>
+inline F* overlapping(F* kernel) {
+    overlap_kernel(reinterpret_cast<const void*>(kernel));
+    return kernel;
+}
+
 // ------------------------------------------------------------------------------------- device --------
 #ifdef __CUDACC__
 
@@ -80,6 +89,14 @@ constexpr int kWarp = 32;
 // PDL: let the next kernel in the stream start its prologue / wait for the previous kernel's results.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// What a kernel launched through overlapping() does before it touches memory that another kernel writes or reads: every thread, on every path. It waits until the
+// kernel in front has completed and then lets the one behind become resident. In that order: with the two exchanged a captured Nelutar step took 15 us longer (CTAs
+// that only wait hold places which the step's other branches need). Data from other kernels are read without the read-only path (no __restrict__ in these
+// kernels): those loads need not stay behind the wait.
+__device__ __forceinline__ void after_previous() {
+    pdl_wait();
+    pdl_launch_dependents();
+}
 
 // 128-bit streaming load of weights: read-only path, do not pollute L1 (each byte is used exactly once).
 __device__ __forceinline__ uint4 ldg_stream(const void* p) {
@@ -87,6 +104,12 @@ __device__ __forceinline__ uint4 ldg_stream(const void* p) {
     asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
                  : "l"(p));
+    return r;
+}
+// the same for data that the kernel in front may still have been writing when this one became resident (after_previous())
+__device__ __forceinline__ uint4 ld_stream(const void* p) {
+    uint4 r;
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
     return r;
 }
 __device__ __forceinline__ uint2 ldg_stream8(const void* p) {

@@ -1,7 +1,9 @@
 // csrc/runtime.cu — error reporting and device facts behind include/sllm_b200.h.
+#include <atomic>
 #include <cstdarg>
 #include <cstring>
 #include <mutex>
+#include <vector>
 
 #include "common.cuh"
 
@@ -61,6 +63,29 @@ int status_take() {
     return SLLM_ETIMEOUT;
 }
 
+// Kernels launched through overlapping(): a set that only grows, to at most as many as the library has instantiations; looked up on every launch, so without a lock.
+static constexpr size_t kOverlapSlots = 1024;
+static std::atomic<const void*> g_overlap[kOverlapSlots];
+static bool overlap_find(const void* kernel, bool add) {
+    for (size_t i = reinterpret_cast<uintptr_t>(kernel) >> 4, n = 0; n < kOverlapSlots; ++i, ++n) {
+        std::atomic<const void*>& slot = g_overlap[i % kOverlapSlots];
+        const void* held = slot.load(std::memory_order_acquire);
+        if (held == nullptr && add && slot.compare_exchange_strong(held, kernel, std::memory_order_acq_rel)) return true;
+        if (held == kernel) return true;      // compare_exchange has left what another thread put there
+        if (held == nullptr && !add) return false;
+    }
+    return false;                             // a full table: this kernel's edges stay as they are
+}
+void overlap_kernel(const void* kernel) { overlap_find(kernel, true); }
+static bool overlaps(cudaGraphNode_t node) {
+    cudaKernelNodeParams p{};
+    if (cudaGraphKernelNodeGetParams(node, &p) != cudaSuccess) {   // another library's kernel
+        cudaGetLastError();
+        return false;
+    }
+    return overlap_find(p.func, false);
+}
+
 int sm_count() {
     static int n = 0;
     if (!n) {
@@ -109,6 +134,39 @@ int sllm_tune(int32_t key, int32_t value) {
             return SLLM_OK;
         default: sllm::set_error("unknown tunable %d", key); return SLLM_EINVAL;
     }
+}
+
+int sllm_graph_overlap(void* graph, int32_t* edges) {
+    using namespace sllm;
+    SLLM_REQUIRE(graph, SLLM_EINVAL, "graph_overlap: no graph");
+    const cudaGraph_t g = reinterpret_cast<cudaGraph_t>(graph);
+    int32_t changed = 0;
+    size_t n = 0;
+    SLLM_CUDA(cudaGraphGetNodes(g, nullptr, &n));
+    std::vector<cudaGraphNode_t> nodes(n);
+    SLLM_CUDA(cudaGraphGetNodes(g, nodes.data(), &n));
+    for (size_t i = 0; i < n; ++i) {
+        cudaGraphNodeType type;
+        SLLM_CUDA(cudaGraphNodeGetType(nodes[i], &type));
+        if (type != cudaGraphNodeTypeKernel || !overlaps(nodes[i])) continue;
+        // One predecessor, a kernel: this node's own wait takes the place of the edge. Joins of several branches keep theirs (a step of Nelutar measured the same with
+        // those converted too).
+        size_t deps = 0;
+        SLLM_CUDA(cudaGraphNodeGetDependencies_v2(nodes[i], nullptr, nullptr, &deps));
+        if (deps != 1) continue;
+        cudaGraphNode_t from = nullptr;
+        cudaGraphEdgeData edge{}, early{};
+        SLLM_CUDA(cudaGraphNodeGetDependencies_v2(nodes[i], &from, &edge, &deps));
+        SLLM_CUDA(cudaGraphNodeGetType(from, &type));
+        if (type != cudaGraphNodeTypeKernel || edge.type != cudaGraphDependencyTypeDefault || edge.from_port != cudaGraphKernelNodePortDefault) continue;
+        early.type = cudaGraphDependencyTypeProgrammatic;
+        early.from_port = cudaGraphKernelNodePortProgrammatic;
+        SLLM_CUDA(cudaGraphRemoveDependencies_v2(g, &from, &nodes[i], &edge, 1));
+        SLLM_CUDA(cudaGraphAddDependencies_v2(g, &from, &nodes[i], &early, 1));
+        ++changed;
+    }
+    if (edges) *edges = changed;
+    return SLLM_OK;
 }
 
 int sllm_device_info(int32_t* sms, int32_t* smem, size_t* total, size_t* free_) {

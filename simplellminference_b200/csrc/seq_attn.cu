@@ -23,6 +23,7 @@ constexpr int kQW = 4;   // queries per warp of the fp32 body
 
 template <typename KV, int kMaxDvChunks>   // dv <= 32 * kMaxDvChunks
 __global__ void __launch_bounds__(256) seq_attention_kernel(AttnArgs p) {
+    after_previous();
     extern __shared__ __align__(16) float sm[];
     const int dk = p.dk, dv = p.dv, dkp = ((dk + 3) & ~3) + 4;   // padded row of q / k in floats
     float* sq = sm;                      // [kBQ][dkp]
@@ -381,9 +382,10 @@ __global__ void __launch_bounds__(128) seq_attention_mma_kernel(AttnArgs p) {
 // one CTA per (token, head), one thread per value column: merge the shares, normalise, turn back by the token's position, gate.
 // Warp 0 turns the shares' (max, sum) into one weight per share (exp(m_s - max) / total, zero for a share that saw no key); every thread
 // then adds its column over the shares with coalesced loads; pairs meet through shared memory for the rotation.
-__global__ void seq_attention_finish_kernel(sllm_seq_batch b, const float* __restrict__ ws, int nsplit, int heads, int dv, const double* __restrict__ vfreq,
-                                            int layout, const float* __restrict__ gate, int ldg, int gate_channels, const float* __restrict__ sink, float* __restrict__ out,
-                                            int ldo, uint16_t* __restrict__ out16) {
+__global__ void seq_attention_finish_kernel(sllm_seq_batch b, const float* ws, int nsplit, int heads, int dv, const double* vfreq,
+                                            int layout, const float* gate, int ldg, int gate_channels, const float* sink, float* out,
+                                            int ldo, uint16_t* out16) {
+    after_previous();
     extern __shared__ float fsm[];
     float* s_w = fsm;            // [nsplit]
     float* s_o = fsm + nsplit;   // [groups][dv]
@@ -446,9 +448,10 @@ __global__ void seq_attention_finish_kernel(sllm_seq_batch b, const float* __res
 
 // one CTA per token: rotate q in place, rotate k and v and store them into the pools
 template <typename KV>
-__global__ void seq_rotary_kv_kernel(sllm_seq_batch b, float* __restrict__ q, int ldq, int heads, int dk, const float* __restrict__ k, int ldk, int kv_heads,
-                                     const float* __restrict__ v, int ldv, int dv, const double* __restrict__ freq, int n_freq, float magnitude,
-                                     const double* __restrict__ vfreq, int layout, KV* __restrict__ k_pool, KV* __restrict__ v_pool) {
+__global__ void seq_rotary_kv_kernel(sllm_seq_batch b, float* q, int ldq, int heads, int dk, const float* k, int ldk, int kv_heads,
+                                     const float* v, int ldv, int dv, const double* freq, int n_freq, float magnitude,
+                                     const double* vfreq, int layout, KV* k_pool, KV* v_pool) {
+    after_previous();
     const int t = blockIdx.x, posi = b.tok_pos[t], slot = b.tok_slot[t];
     const int pos = posi;
     // gridDim.y CTAs share a token: CTA y takes the work items y, y + gridDim.y, ... of each of the three loops (single tokens would
@@ -519,7 +522,7 @@ int sllm::launch_attention_finish(const sllm_seq_batch* b, const float* ws, int 
     SLLM_REQUIRE(dv <= 1024 && nsplit <= 8192, SLLM_ENOTSUP, "seq_attention_finish: value width %d / %d shares beyond what one CTA merges", dv, nsplit);
     // many shares (single tokens): up to eight groups of threads add them side by side, each at least four
     const int cols = (dv + 31) / 32 * 32, groups = std::max(1, std::min({8, 1024 / cols, nsplit / 4})), threads = cols * groups;
-    seq_attention_finish_kernel<<<b->T * heads, threads, (size_t)(nsplit + groups * dv) * sizeof(float), st>>>(*b, ws, nsplit, heads, dv, vfreq, layout, gate, ldg, gate_channels,
+    overlapping(seq_attention_finish_kernel)<<<b->T * heads, threads, (size_t)(nsplit + groups * dv) * sizeof(float), st>>>(*b, ws, nsplit, heads, dv, vfreq, layout, gate, ldg, gate_channels,
                                                                                                      sink, out, ldo, out16);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
@@ -541,10 +544,10 @@ int sllm_seq_rotary_kv(const sllm_seq_batch* b, float* q, int32_t ldq, int32_t h
     const int work = std::max(heads * n_freq, kv_heads * std::max(dk, dv));
     const dim3 rgrid(b->T, std::max(1, std::min((work + 127) / 128, b->T >= 64 ? 1 : 16)));
     if (kv_dtype == SLLM_F32)
-        seq_rotary_kv_kernel<float><<<rgrid, 128, 0, as_stream(stream)>>>(*b, q, ldq, heads, dk, k, ldk, kv_heads, v, ldv, dv, freq, n_freq, magnitude, vfreq,
+        overlapping(seq_rotary_kv_kernel<float>)<<<rgrid, 128, 0, as_stream(stream)>>>(*b, q, ldq, heads, dk, k, ldk, kv_heads, v, ldv, dv, freq, n_freq, magnitude, vfreq,
                                                                          layout, (float*)k_pool, (float*)v_pool);
     else
-        seq_rotary_kv_kernel<uint16_t><<<rgrid, 128, 0, as_stream(stream)>>>(*b, q, ldq, heads, dk, k, ldk, kv_heads, v, ldv, dv, freq, n_freq, magnitude,
+        overlapping(seq_rotary_kv_kernel<uint16_t>)<<<rgrid, 128, 0, as_stream(stream)>>>(*b, q, ldq, heads, dk, k, ldk, kv_heads, v, ldv, dv, freq, n_freq, magnitude,
                                                                             vfreq, layout, (uint16_t*)k_pool, (uint16_t*)v_pool);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
@@ -574,7 +577,7 @@ static int launch_attention_decode(Kernel* kernel, int G, int smem, const sllm::
     attr[0].val.clusterDim.z = cs;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    SLLM_CUDA(cudaLaunchKernelEx(&cfg, kernel, p, args...));
+    SLLM_CUDA(cudaLaunchKernelEx(&cfg, overlapping(kernel), p, args...));
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;
@@ -708,7 +711,7 @@ static int attention_run(const sllm_seq_batch* b, const float* q, int32_t ldq, i
 #define SLLM_ATTN_LAUNCH(KV, NC)                                                                                                              \
     do {                                                                                                                                      \
         if (smem > 48 * 1024) SLLM_CUDA(cudaFuncSetAttribute(seq_attention_kernel<KV, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-        seq_attention_kernel<KV, NC><<<grid, 256, smem, as_stream(stream)>>>(p);                                                              \
+        overlapping(seq_attention_kernel<KV, NC>)<<<grid, 256, smem, as_stream(stream)>>>(p);                                                              \
     } while (0)
     if (kv_dtype == SLLM_F32) {
         if (chunks == 4) SLLM_ATTN_LAUNCH(float, 4); else if (chunks == 8) SLLM_ATTN_LAUNCH(float, 8); else SLLM_ATTN_LAUNCH(float, 16);

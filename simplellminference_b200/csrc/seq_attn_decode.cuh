@@ -68,6 +68,7 @@ constexpr int kDecodeWarps = 4, kDecodeCluster = 16;     // warps of a CTA, CTAs
 // columns (distributed shared memory, one barrier), which merge them and write the result (or one record per share when something still follows).
 template <int L, int G, int kSteps>     // 16-byte loads per lane of a key or value row: heads of D = 32 L
 __global__ void __launch_bounds__(kDecodeWarps * 32) seq_attention_decode_kernel(AttnArgs p) {
+    after_previous();
     namespace cg = cooperative_groups;
     constexpr int E = 4, PE = E / 2, D = 8 * L * E, VAL = G * kSteps;
     constexpr int kPer = VAL >= 8 ? VAL / 8 : 1, kDup = VAL >= 8 ? 1 : 8 / VAL;      // scores per lane after the exchange, lanes that hold the same one
@@ -121,14 +122,14 @@ __global__ void __launch_bounds__(kDecodeWarps * 32) seq_attention_decode_kernel
 #pragma unroll
         for (int s = 0; s < kSteps; ++s)
 #pragma unroll
-            for (int i = 0; i < L; ++i) u[s][i] = j0 + 4 * s + kg <= pos ? ldg_stream(row + (size_t)(4 * s) * D + i * 8 * E) : make_uint4(0u, 0u, 0u, 0u);
+            for (int i = 0; i < L; ++i) u[s][i] = j0 + 4 * s + kg <= pos ? ld_stream(row + (size_t)(4 * s) * D + i * 8 * E) : make_uint4(0u, 0u, 0u, 0u);
     };
     auto load_values = [&](uint4 (&u)[kSteps][L], int j0, int page) {
         const float* row = vp + seq_pool_row(page, p.kv_heads, gkv, b.page_len, j0 % b.page_len + kg, D) + j8 * E;
 #pragma unroll
         for (int s = 0; s < kSteps; ++s)
 #pragma unroll
-            for (int i = 0; i < L; ++i) u[s][i] = j0 + 4 * s + kg <= pos ? ldg_stream(row + (size_t)(4 * s) * D + i * 8 * E) : make_uint4(0u, 0u, 0u, 0u);
+            for (int i = 0; i < L; ++i) u[s][i] = j0 + 4 * s + kg <= pos ? ld_stream(row + (size_t)(4 * s) * D + i * 8 * E) : make_uint4(0u, 0u, 0u, 0u);
     };
     // A run's keys are asked for as soon as the previous run's have been multiplied, its values likewise: one of the two is always on its way.
     uint4 ku[kSteps][L], vu[kSteps][L];
@@ -324,6 +325,7 @@ __device__ __forceinline__ void ldmatrix4_trans(uint32_t (&r)[4], uint32_t addr)
 
 template <int D, bool kOpts>     // kOpts: capped scores or charges on the distance (a window, kept positions and chunks are part of both)
 __global__ void __launch_bounds__(kDecodeWarps * 32, 2) seq_attention_decode_mma_kernel(AttnArgs p, int G) {
+    after_previous();
     namespace cg = cooperative_groups;
     using Tile = DecodeTile<D>;
     constexpr int kRun = Tile::kRun, kRing = Tile::kRing, kSteps = D / 16, kTiles = D / 8;

@@ -313,6 +313,7 @@ __host__ __device__ inline size_t talk_smem(int nq, int gs, int heads, int dkq, 
 
 template <typename KV>
 __global__ void __launch_bounds__(kTalkWarps * 32) seq_attention_talk_kernel(TalkArgs p) {
+    after_previous();
     extern __shared__ __align__(16) float sm[];
     const int H = p.heads, G = p.kv_heads, group = H / G, dk = p.dk, dv = p.dv, NQ = p.nq;
     float* sT = sm;                                                                  // [H][H]
@@ -579,10 +580,10 @@ int sllm_seq_attention_talk(const sllm_seq_batch* b, const float* q, int32_t ldq
     const dim3 grid(b->T == b->nseg ? b->n_qtiles : b->n_qtiles * (kBQ / p.nq), nsplit);
     if (kv_dtype == SLLM_F32) {
         SLLM_CUDA(cudaFuncSetAttribute(seq_attention_talk_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        seq_attention_talk_kernel<float><<<grid, kTalkWarps * 32, smem, st>>>(p);
+        overlapping(seq_attention_talk_kernel<float>)<<<grid, kTalkWarps * 32, smem, st>>>(p);
     } else {
         SLLM_CUDA(cudaFuncSetAttribute(seq_attention_talk_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        seq_attention_talk_kernel<uint16_t><<<grid, kTalkWarps * 32, smem, st>>>(p);
+        overlapping(seq_attention_talk_kernel<uint16_t>)<<<grid, kTalkWarps * 32, smem, st>>>(p);
     }
     ++g_launches;
     SLLM_LAUNCH_CHECK();

@@ -27,8 +27,9 @@
 namespace sllm {
 
 // thread = (token, channel): out = act(cb[c] + sum_j w[c][j] * x[t - taps + 1 + j][c]); act 0 = none, 1 = silu
-__global__ void seq_conv_ring_kernel(sllm_seq_batch b, const float* __restrict__ x, int ldx, int channels, int taps, const float* __restrict__ w,
-                                     const float* __restrict__ cb, const float* __restrict__ ring, int act, float* __restrict__ out, int ldo) {
+__global__ void seq_conv_ring_kernel(sllm_seq_batch b, const float* x, int ldx, int channels, int taps, const float* w,
+                                     const float* cb, const float* ring, int act, float* out, int ldo) {
+    after_previous();
     const int t = blockIdx.y, c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= channels) return;
     const int slot = b.tok_slot[t], pos = b.tok_pos[t];
@@ -47,8 +48,9 @@ __global__ void seq_conv_ring_kernel(sllm_seq_batch b, const float* __restrict__
 // stay in registers while the thread walks its tokens.
 constexpr int kConvTile = 8;
 template <int TAPS>
-__global__ void seq_conv_ring_vec_kernel(sllm_seq_batch b, const float* __restrict__ x, int ldx, int channels, const float* __restrict__ w, const float* __restrict__ cb,
-                                         const float* __restrict__ ring, int act, float* __restrict__ out, int ldo) {
+__global__ void seq_conv_ring_vec_kernel(sllm_seq_batch b, const float* x, int ldx, int channels, const float* w, const float* cb,
+                                         const float* ring, int act, float* out, int ldo) {
+    after_previous();
     const int ch = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
     if (ch >= channels) return;
     float4 wt[TAPS];                                     // wt[back]: the weights of the input `back` positions before the token
@@ -137,6 +139,7 @@ __device__ __forceinline__ void delta_cp4(void* dst, const void* src, bool take)
 // 4: the delta rule with a decay per key channel. 5 / 6 / 7: as 1 / 2 / 3 with a constant decay per head (qscale then multiplies k).
 template <int kDeltaKP, int kMaxThreads, int kForm>
 __global__ void __launch_bounds__(kMaxThreads) seq_delta_kernel(DeltaArgs p) {
+    after_previous();
     constexpr int kDeltaRS = kDeltaKP + 4;
     constexpr bool kChannel = kForm == 4, kFixed = kForm >= 5, kSsd = kForm != 0 && !kChannel;
     constexpr bool kFromZero = kForm == 2 || kForm == 6, kFromStart = kForm == 3 || kForm == 7, kRanges = kFromZero || kFromStart;
@@ -370,6 +373,7 @@ __global__ void __launch_bounds__(kMaxThreads) seq_delta_kernel(DeltaArgs p) {
 
 // thread = one state element of one head of one portion: its ranges in order, end state from zero -> start state
 __global__ void seq_ssd_carry_kernel(DeltaArgs p) {
+    after_previous();
     const sllm_seq_batch& b = p.b;
     const int seg = blockIdx.z, h = blockIdx.y, per = p.dk * p.dv, e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= per) return;
@@ -412,14 +416,14 @@ int sllm_seq_conv_ring(const sllm_seq_batch* b, const float* x, int32_t ldx, int
     auto aligned = [](const void* q) { return q == nullptr || ((uintptr_t)q % 16) == 0; };
     if (b->T > b->nseg && taps >= 2 && taps <= 4 && channels % 4 == 0 && ldx % 4 == 0 && ldo % 4 == 0 && aligned(x) && aligned(w) && aligned(cb) && aligned(ring) && aligned(out)) {
         const dim3 grid((channels / 4 + 127) / 128, (b->T + kConvTile - 1) / kConvTile);
-        if (taps == 2) seq_conv_ring_vec_kernel<2><<<grid, 128, 0, as_stream(stream)>>>(*b, x, ldx, channels, w, cb, ring, act, out, ldo);
-        else if (taps == 3) seq_conv_ring_vec_kernel<3><<<grid, 128, 0, as_stream(stream)>>>(*b, x, ldx, channels, w, cb, ring, act, out, ldo);
-        else seq_conv_ring_vec_kernel<4><<<grid, 128, 0, as_stream(stream)>>>(*b, x, ldx, channels, w, cb, ring, act, out, ldo);
+        if (taps == 2) overlapping(seq_conv_ring_vec_kernel<2>)<<<grid, 128, 0, as_stream(stream)>>>(*b, x, ldx, channels, w, cb, ring, act, out, ldo);
+        else if (taps == 3) overlapping(seq_conv_ring_vec_kernel<3>)<<<grid, 128, 0, as_stream(stream)>>>(*b, x, ldx, channels, w, cb, ring, act, out, ldo);
+        else overlapping(seq_conv_ring_vec_kernel<4>)<<<grid, 128, 0, as_stream(stream)>>>(*b, x, ldx, channels, w, cb, ring, act, out, ldo);
         ++g_launches;
         SLLM_LAUNCH_CHECK();
         return SLLM_OK;
     }
-    seq_conv_ring_kernel<<<dim3((channels + 127) / 128, b->T), 128, 0, as_stream(stream)>>>(*b, x, ldx, channels, taps, w, cb, ring, act, out, ldo);
+    overlapping(seq_conv_ring_kernel)<<<dim3((channels + 127) / 128, b->T), 128, 0, as_stream(stream)>>>(*b, x, ldx, channels, taps, w, cb, ring, act, out, ldo);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;
@@ -493,14 +497,14 @@ static int delta_run(bool ssd, const float* skip, const DeltaExtra& ex, const sl
 #define SLLM_DELTA_LAUNCH_AS(KPV, MAXT, FORM)                                                                                                             \
     do {                                                                                                                                                  \
         if (smem > 48 * 1024) SLLM_CUDA(cudaFuncSetAttribute(seq_delta_kernel<KPV, MAXT, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-        seq_delta_kernel<KPV, MAXT, FORM><<<grid, threads, smem, as_stream(stream)>>>(p);                                                                 \
+        overlapping(seq_delta_kernel<KPV, MAXT, FORM>)<<<grid, threads, smem, as_stream(stream)>>>(p);                                                                 \
         ++g_launches;                                                                                                                                     \
         SLLM_LAUNCH_CHECK();                                                                                                                              \
     } while (0)
 #define SLLM_DELTA_RANGES(KPV, MAXT, FIRST, THIRD)                                                                                    \
     do {                                                                                                                              \
         SLLM_DELTA_LAUNCH_AS(KPV, MAXT, FIRST);                                                                                       \
-        seq_ssd_carry_kernel<<<dim3((dk * dv + 255) / 256, heads, b->nseg), 256, 0, as_stream(stream)>>>(p);                          \
+        overlapping(seq_ssd_carry_kernel)<<<dim3((dk * dv + 255) / 256, heads, b->nseg), 256, 0, as_stream(stream)>>>(p);                          \
         ++g_launches;                                                                                                                 \
         SLLM_LAUNCH_CHECK();                                                                                                          \
         SLLM_DELTA_LAUNCH_AS(KPV, MAXT, THIRD);                                                                                       \

@@ -7,8 +7,9 @@
 
 namespace sllm {
 
-__global__ void seq_embed_kernel(const int32_t* __restrict__ ids, const void* __restrict__ table, int w_dtype, int vocab, int d, int streams,
-                                 float scale, float* __restrict__ out, int T) {
+__global__ void seq_embed_kernel(const int32_t* ids, const void* table, int w_dtype, int vocab, int d, int streams,
+                                 float scale, float* out, int T) {
+    after_previous();
     const int t = blockIdx.x;
     int id = ids[t];
     id = id < 0 ? 0 : (id >= vocab ? vocab - 1 : id);
@@ -19,8 +20,9 @@ __global__ void seq_embed_kernel(const int32_t* __restrict__ ids, const void* __
 }
 
 // grid (T, groups): one CTA normalises one part of one token's vector
-__global__ void seq_hyper_read_kernel(const float* __restrict__ x, int streams, int T, int d, const float* __restrict__ coef,
-                                      const float* __restrict__ norm_w, int groups, float eps, float* __restrict__ y) {
+__global__ void seq_hyper_read_kernel(const float* x, int streams, int T, int d, const float* coef,
+                                      const float* norm_w, int groups, float eps, float* y) {
+    after_previous();
     __shared__ float red[33];
     const int t = blockIdx.x, g = blockIdx.y, n = d / groups, j0 = g * n;
     float ss = 0.0f;
@@ -41,8 +43,9 @@ __global__ void seq_hyper_read_kernel(const float* __restrict__ x, int streams, 
 
 constexpr int kMaxStreams = 8;
 
-__global__ void seq_hyper_write_kernel(float* __restrict__ x, int streams, int T, int d, const float* __restrict__ mix,
-                                       const float* __restrict__ outc, const float* __restrict__ y) {
+__global__ void seq_hyper_write_kernel(float* x, int streams, int T, int d, const float* mix,
+                                       const float* outc, const float* y) {
+    after_previous();
     const size_t n = (size_t)T * d;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         float old[kMaxStreams];
@@ -63,9 +66,10 @@ __global__ void seq_hyper_write_kernel(float* __restrict__ x, int streams, int T
 
 // hyper-connection write of one sublayer and read (+ grouped norm) of the next in one pass over the streams: grid (T, groups), a CTA owns
 // one part of one token's vector in every stream — it stores the mixed streams and normalises their weighted sum for the next sublayer
-__global__ void seq_hyper_write_read_kernel(float* __restrict__ x, int streams, int T, int d, const float* __restrict__ mix, const float* __restrict__ outc,
-                                            const float* __restrict__ y_in, const float* __restrict__ coef, const float* __restrict__ norm_w, int groups,
-                                            float eps, float* __restrict__ y_out) {
+__global__ void seq_hyper_write_read_kernel(float* x, int streams, int T, int d, const float* mix, const float* outc,
+                                            const float* y_in, const float* coef, const float* norm_w, int groups,
+                                            float eps, float* y_out) {
+    after_previous();
     __shared__ float red[33];
     __shared__ float s_mix[kMaxStreams * kMaxStreams], s_outc[kMaxStreams], s_coef[kMaxStreams];   // the small matrices once per CTA, not per element
     const int t = blockIdx.x, g = blockIdx.y, n = d / groups, j0 = g * n;
@@ -107,8 +111,9 @@ __global__ void seq_hyper_write_read_kernel(float* __restrict__ x, int streams, 
     }
 }
 
-__global__ void seq_polynorm_kernel(const float* z, int ldz, const float* __restrict__ coef, float eps, float* out,
+__global__ void seq_polynorm_kernel(const float* z, int ldz, const float* coef, float eps, float* out,
                                     int ldo, int n) {
+    after_previous();
     __shared__ float red[33];
     const int t = blockIdx.x;
     const float* zr = z + (size_t)t * ldz;
@@ -130,7 +135,8 @@ __global__ void seq_polynorm_kernel(const float* z, int ldz, const float* __rest
     }
 }
 
-__global__ void seq_gather_rows_kernel(const float* __restrict__ x, int ldx, const int32_t* __restrict__ rows, int d, float* __restrict__ out) {
+__global__ void seq_gather_rows_kernel(const float* x, int ldx, const int32_t* rows, int d, float* out) {
+    after_previous();
     const int i = blockIdx.x;
     const float* src = x + (size_t)rows[i] * ldx;
     for (int j = threadIdx.x; j < d; j += blockDim.x) out[(size_t)i * d + j] = src[j];
@@ -141,8 +147,9 @@ __global__ void seq_gather_rows_kernel(const float* __restrict__ x, int ldx, con
 __device__ __forceinline__ float headnorm_gate_of(float g, int mode) { return (mode & 4) ? seq_sigmoid(g) : g / (1.0f + expf(-g)); }
 
 // one warp per (token, head)
-__global__ void seq_headnorm_gate_kernel(const float* __restrict__ o, int ldo, const float* __restrict__ g, int ldg, const float* __restrict__ w,
-                                         int heads, int dv, float eps, float* __restrict__ out, int ldout, uint16_t* __restrict__ out16, int T, int mode) {
+__global__ void seq_headnorm_gate_kernel(const float* o, int ldo, const float* g, int ldg, const float* w,
+                                         int heads, int dv, float eps, float* out, int ldout, uint16_t* out16, int T, int mode) {
+    after_previous();
     const int item = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (item >= T * heads) return;
     const int t = item / heads, h = item % heads;
@@ -168,9 +175,10 @@ __global__ void seq_headnorm_gate_kernel(const float* __restrict__ o, int ldo, c
 // the same with one CTA per (token, part), for parts too wide for a warp (a norm over a few parts of a wide row): the part's gated values
 // wait in registers between the sum of squares and the scaling, kNormPer per thread
 constexpr int kNormPer = 8;
-__global__ void __launch_bounds__(1024) seq_headnorm_gate_wide_kernel(const float* __restrict__ o, int ldo, const float* __restrict__ g, int ldg,
-                                                                     const float* __restrict__ w, int heads, int dv, float eps, float* __restrict__ out, int ldout,
-                                                                     uint16_t* __restrict__ out16, int mode) {
+__global__ void __launch_bounds__(1024) seq_headnorm_gate_wide_kernel(const float* o, int ldo, const float* g, int ldg,
+                                                                     const float* w, int heads, int dv, float eps, float* out, int ldout,
+                                                                     uint16_t* out16, int mode) {
+    after_previous();
     __shared__ float red[33];
     const int t = blockIdx.x / heads, h = blockIdx.x % heads;
     const float* orow = o + (size_t)t * ldo + (size_t)h * dv;
@@ -206,9 +214,10 @@ __global__ void __launch_bounds__(1024) seq_headnorm_gate_wide_kernel(const floa
 // the same four columns at a time: a team of `team` threads (a warp, or the whole CTA) per (token, part), R groups of four columns per thread,
 // everything in registers between the sum of squares and the scaling
 template <int R>
-__global__ void __launch_bounds__(1024) seq_headnorm_gate_vec_kernel(const float* __restrict__ o, int ldo, const float* __restrict__ g, int ldg, const float* __restrict__ w,
-                                                                     int heads, int dv, float eps, float* __restrict__ out, int ldout, uint16_t* __restrict__ out16, int items,
+__global__ void __launch_bounds__(1024) seq_headnorm_gate_vec_kernel(const float* o, int ldo, const float* g, int ldg, const float* w,
+                                                                     int heads, int dv, float eps, float* out, int ldout, uint16_t* out16, int items,
                                                                      int team, int mode) {
+    after_previous();
     __shared__ float red[33];
     const int per_cta = blockDim.x / team, item = blockIdx.x * per_cta + threadIdx.x / team, me = threadIdx.x % team;
     const bool live = item < items;                      // (a CTA that is one team has one item: no thread leaves before the barriers)
@@ -247,8 +256,8 @@ __global__ void __launch_bounds__(1024) seq_headnorm_gate_vec_kernel(const float
 
 // (row - mean) / sqrt(variance + eps) * w + b of one row that the CTA's threads hold strided; the variance is the mean of the squared
 // deviations (two passes: the mean first), as the definition says
-__device__ __forceinline__ void seq_layernorm_row(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias, float eps,
-                                                  float* __restrict__ y, uint16_t* __restrict__ y16, int d, float* red) {
+__device__ __forceinline__ void seq_layernorm_row(const float* x, const float* w, const float* bias, float eps,
+                                                  float* y, uint16_t* y16, int d, float* red) {
     float s = 0.0f;
     for (int j = threadIdx.x; j < d; j += blockDim.x) s += x[j];
     const float mean = block_sum(s, red) / (float)d;
@@ -265,8 +274,9 @@ __device__ __forceinline__ void seq_layernorm_row(const float* __restrict__ x, c
     }
 }
 
-__global__ void seq_layernorm_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ w, const float* __restrict__ bias, float eps,
-                                     float* __restrict__ y, int ldy, uint16_t* __restrict__ y16, int d) {
+__global__ void seq_layernorm_kernel(const float* x, int ldx, const float* w, const float* bias, float eps,
+                                     float* y, int ldy, uint16_t* y16, int d) {
+    after_previous();
     __shared__ float red[33];
     seq_layernorm_row(x + (size_t)blockIdx.x * ldx, w, bias, eps, y + (size_t)blockIdx.x * ldy, y16 ? y16 + (size_t)blockIdx.x * d : nullptr, d, red);
 }
@@ -277,8 +287,9 @@ constexpr int kMaxDepth = 256;
 // The new row stays in shared memory for the norm's passes; with rows of a multiple of four floats everything moves as 16-byte words and
 // the loads of the earlier results are issued together, before the store into the same array.
 template <typename V>
-__global__ void seq_depth_average_kernel(float* __restrict__ x, const float* __restrict__ y, float* hist, int n_prev, const float* __restrict__ coef,
-                                         const float* __restrict__ norm_w, const float* __restrict__ norm_b, float eps, float* __restrict__ h, uint16_t* __restrict__ h16, int T, int d) {
+__global__ void seq_depth_average_kernel(float* x, const float* y, float* hist, int n_prev, const float* coef,
+                                         const float* norm_w, const float* norm_b, float eps, float* h, uint16_t* h16, int T, int d) {
+    after_previous();
     extern __shared__ __align__(16) float s_row[];   // [d]
     __shared__ float red[33];
     __shared__ float s_coef[kMaxDepth + 1];
@@ -334,8 +345,9 @@ __global__ void seq_depth_average_kernel(float* __restrict__ x, const float* __r
 }
 
 // out = g * sigmoid(alpha * g) * (u + 1) with g = min(gate, limit), u = clamp(up, -limit, limit)
-__global__ void seq_clamped_glu_kernel(const float* __restrict__ gate, int ldg, const float* __restrict__ up, int ldu, float limit, float alpha,
-                                       float* __restrict__ out, int ldo, uint16_t* __restrict__ out16, int T, int n) {
+__global__ void seq_clamped_glu_kernel(const float* gate, int ldg, const float* up, int ldu, float limit, float alpha,
+                                       float* out, int ldo, uint16_t* out16, int T, int n) {
+    after_previous();
     const size_t total = (size_t)T * n;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const size_t t = i / n, j = i % n;
@@ -348,8 +360,9 @@ __global__ void seq_clamped_glu_kernel(const float* __restrict__ gate, int ldg, 
 }
 
 // the same four columns at a time: grid (T, parts of a row)
-__global__ void seq_clamped_glu_vec_kernel(const float* __restrict__ gate, int ldg, const float* __restrict__ up, int ldu, float limit, float alpha, float* __restrict__ out,
-                                           int ldo, uint16_t* __restrict__ out16, int n) {
+__global__ void seq_clamped_glu_vec_kernel(const float* gate, int ldg, const float* up, int ldu, float limit, float alpha, float* out,
+                                           int ldo, uint16_t* out16, int n) {
+    after_previous();
     const size_t t = blockIdx.x;
     auto one = [&](float g, float u) {
         g = fminf(g, limit);
@@ -366,9 +379,10 @@ __global__ void seq_clamped_glu_vec_kernel(const float* __restrict__ gate, int l
 
 // token embedding plus a hashed embedding of the (previous token, token) pair: row (prev * mul_prev + id * mul_cur) mod buckets of
 // `pairs`, and row `buckets` (the table's last) for a sequence's first token (prev < 0)
-__global__ void seq_embed_pair_kernel(const int32_t* __restrict__ ids, const int32_t* __restrict__ prev, const void* __restrict__ table,
-                                      const void* __restrict__ pairs, int w_dtype, int vocab, int d, int buckets, long long mul_prev, long long mul_cur,
-                                      float* __restrict__ out) {
+__global__ void seq_embed_pair_kernel(const int32_t* ids, const int32_t* prev, const void* table,
+                                      const void* pairs, int w_dtype, int vocab, int d, int buckets, long long mul_prev, long long mul_cur,
+                                      float* out) {
+    after_previous();
     const int t = blockIdx.x;
     int id = ids[t];
     id = id < 0 ? 0 : (id >= vocab ? vocab - 1 : id);
@@ -379,7 +393,8 @@ __global__ void seq_embed_pair_kernel(const int32_t* __restrict__ ids, const int
 }
 
 // one warp per row: y = x / sqrt(mean(x^2) + eps) * w (w NULL = no weight)
-__global__ void seq_rmsnorm_rows_kernel(const float* x, int ldx, const float* __restrict__ w, float eps, float* y, int ldy, int T, int n) {   // y may be x
+__global__ void seq_rmsnorm_rows_kernel(const float* x, int ldx, const float* w, float eps, float* y, int ldy, int T, int n) {
+    after_previous();   // y may be x
     const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (t >= T) return;
     const float* xr = x + (size_t)t * ldx;
@@ -390,7 +405,8 @@ __global__ void seq_rmsnorm_rows_kernel(const float* x, int ldx, const float* __
 }
 
 // the same with one CTA per row, for steps of few rows (one warp would walk a long row alone)
-__global__ void seq_rmsnorm_row_cta_kernel(const float* x, int ldx, const float* __restrict__ w, float eps, float* y, int ldy, int n) {   // y may be x
+__global__ void seq_rmsnorm_row_cta_kernel(const float* x, int ldx, const float* w, float eps, float* y, int ldy, int n) {
+    after_previous();   // y may be x
     __shared__ float red[33];
     const float* xr = x + (size_t)blockIdx.x * ldx;
     float ss = 0.0f;
@@ -400,8 +416,9 @@ __global__ void seq_rmsnorm_row_cta_kernel(const float* x, int ldx, const float*
 }
 
 // out = act(gate) * up; act 0 = silu
-__global__ void seq_gated_act_kernel(const float* __restrict__ gate, int ldg, const float* __restrict__ up, int ldu, int act, float* __restrict__ out,
-                                     int ldo, uint16_t* __restrict__ out16, int T, int n) {
+__global__ void seq_gated_act_kernel(const float* gate, int ldg, const float* up, int ldu, int act, float* out,
+                                     int ldo, uint16_t* out16, int T, int n) {
+    after_previous();
     const size_t total = (size_t)T * n;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const size_t t = i / n, j = i % n;
@@ -413,8 +430,9 @@ __global__ void seq_gated_act_kernel(const float* __restrict__ gate, int ldg, co
 }
 
 // the same four columns at a time: grid (T, parts of a row), 16-byte loads
-__global__ void seq_gated_act_vec_kernel(const float* __restrict__ gate, int ldg, const float* __restrict__ up, int ldu, float* __restrict__ out, int ldo,
-                                         uint16_t* __restrict__ out16, int n) {
+__global__ void seq_gated_act_vec_kernel(const float* gate, int ldg, const float* up, int ldu, float* out, int ldo,
+                                         uint16_t* out16, int n) {
+    after_previous();
     const size_t t = blockIdx.x;
     for (int j = (blockIdx.y * blockDim.x + threadIdx.x) * 4; j < n; j += gridDim.y * blockDim.x * 4) {
         const float4 g = *reinterpret_cast<const float4*>(gate + t * ldg + j), u = *reinterpret_cast<const float4*>(up + t * ldu + j);
@@ -427,7 +445,8 @@ __global__ void seq_gated_act_vec_kernel(const float* __restrict__ gate, int ldg
 }
 
 // x <- cap * tanh(x / cap)
-__global__ void seq_softcap_kernel(float* __restrict__ x, size_t n, float cap) {
+__global__ void seq_softcap_kernel(float* x, size_t n, float cap) {
+    after_previous();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) x[i] = cap * tanhf(x[i] / cap);
 }
 
@@ -448,7 +467,7 @@ int sllm_seq_embed(const int32_t* ids, const void* table, int32_t w_dtype, int32
                    int32_t T, sllm_stream_t stream) {
     SLLM_REQUIRE(ids && table && out && T > 0 && d > 0 && vocab > 0 && streams >= 1, SLLM_EINVAL, "seq_embed: bad argument");
     SLLM_REQUIRE(w_dtype == SLLM_F32 || w_dtype == SLLM_BF16, SLLM_ENOTSUP, "seq_embed: fp32 or bf16 tables");
-    seq_embed_kernel<<<T, row_threads(T, d, 128), 0, as_stream(stream)>>>(ids, table, w_dtype, vocab, d, streams, scale, out, T);
+    overlapping(seq_embed_kernel)<<<T, row_threads(T, d, 128), 0, as_stream(stream)>>>(ids, table, w_dtype, vocab, d, streams, scale, out, T);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;
@@ -460,7 +479,7 @@ int sllm_seq_hyper_read(const float* x, int32_t streams, int32_t T, int32_t d, c
     if (!norm_w) groups = 1;
     SLLM_REQUIRE(groups >= 1 && d % groups == 0, SLLM_EINVAL, "seq_hyper_read: %d does not divide into %d parts", d, groups);
     const int n = d / groups, threads = n >= 1024 ? 256 : (n >= 256 ? 128 : 64);
-    seq_hyper_read_kernel<<<dim3(T, groups), threads, 0, as_stream(stream)>>>(x, streams, T, d, coef, norm_w, groups, eps, y);
+    overlapping(seq_hyper_read_kernel)<<<dim3(T, groups), threads, 0, as_stream(stream)>>>(x, streams, T, d, coef, norm_w, groups, eps, y);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;
@@ -471,7 +490,7 @@ int sllm_seq_hyper_write(float* x, int32_t streams, int32_t T, int32_t d, const 
     SLLM_REQUIRE(streams >= 1 && streams <= kMaxStreams, SLLM_ENOTSUP, "seq_hyper_write: 1..%d streams", kMaxStreams);
     const size_t n = (size_t)T * d;
     const int blocks = (int)std::min<size_t>((n + 255) / 256, (size_t)sm_count() * 8);
-    seq_hyper_write_kernel<<<blocks, 256, 0, as_stream(stream)>>>(x, streams, T, d, mix, outc, y);
+    overlapping(seq_hyper_write_kernel)<<<blocks, 256, 0, as_stream(stream)>>>(x, streams, T, d, mix, outc, y);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;
@@ -484,7 +503,7 @@ int sllm_seq_hyper_write_read(float* x, int32_t streams, int32_t T, int32_t d, c
     if (!norm_w) groups = 1;
     SLLM_REQUIRE(groups >= 1 && d % groups == 0, SLLM_EINVAL, "seq_hyper_write_read: %d does not divide into %d parts", d, groups);
     const int n = d / groups, threads = n >= 1024 ? 256 : (n >= 256 ? 128 : 64);
-    seq_hyper_write_read_kernel<<<dim3(T, groups), threads, 0, as_stream(stream)>>>(x, streams, T, d, mix, outc, y_in, coef, norm_w, groups, eps, y_out);
+    overlapping(seq_hyper_write_read_kernel)<<<dim3(T, groups), threads, 0, as_stream(stream)>>>(x, streams, T, d, mix, outc, y_in, coef, norm_w, groups, eps, y_out);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;
@@ -492,7 +511,7 @@ int sllm_seq_hyper_write_read(float* x, int32_t streams, int32_t T, int32_t d, c
 
 int sllm_seq_polynorm(const float* z, int32_t ldz, const float* coef, float eps, float* out, int32_t ldo, int32_t T, int32_t n, sllm_stream_t stream) {
     SLLM_REQUIRE(z && coef && out && T > 0 && n > 0 && ldz >= n && ldo >= n, SLLM_EINVAL, "seq_polynorm: bad argument");
-    seq_polynorm_kernel<<<T, n >= 8192 ? 1024 : (n >= 2048 ? 512 : 256), 0, as_stream(stream)>>>(z, ldz, coef, eps, out, ldo, n);
+    overlapping(seq_polynorm_kernel)<<<T, n >= 8192 ? 1024 : (n >= 2048 ? 512 : 256), 0, as_stream(stream)>>>(z, ldz, coef, eps, out, ldo, n);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;
@@ -500,7 +519,7 @@ int sllm_seq_polynorm(const float* z, int32_t ldz, const float* coef, float eps,
 
 int sllm_seq_gather_rows(const float* x, int32_t ldx, const int32_t* rows, int32_t n, int32_t d, float* out, sllm_stream_t stream) {
     SLLM_REQUIRE(x && rows && out && n > 0 && d > 0, SLLM_EINVAL, "seq_gather_rows: bad argument");
-    seq_gather_rows_kernel<<<n, row_threads(n, d, 128), 0, as_stream(stream)>>>(x, ldx, rows, d, out);
+    overlapping(seq_gather_rows_kernel)<<<n, row_threads(n, d, 128), 0, as_stream(stream)>>>(x, ldx, rows, d, out);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;
@@ -514,16 +533,16 @@ int sllm_seq_headnorm_gate(const float* o, int32_t ldo, const float* g, int32_t 
     if (dv % 4 == 0 && ldo % 4 == 0 && ldg % 4 == 0 && (!out || ldout % 4 == 0) && dv <= 8192 && aligned(o) && aligned(g) && aligned(w) && aligned(out) && aligned(out16)) {
         cudaStream_t st = as_stream(stream);
         const int team = dv <= 256 ? 32 : std::min(1024, ((dv + 7) / 8 + 31) / 32 * 32), cta = team == 32 ? 128 : team, grid = team == 32 ? (items + 3) / 4 : items;
-        seq_headnorm_gate_vec_kernel<2><<<grid, cta, 0, st>>>(o, ldo, g, ldg, w, heads, dv, eps, out, ldout, (uint16_t*)out16, items, team, mode);
+        overlapping(seq_headnorm_gate_vec_kernel<2>)<<<grid, cta, 0, st>>>(o, ldo, g, ldg, w, heads, dv, eps, out, ldout, (uint16_t*)out16, items, team, mode);
         ++g_launches;
         SLLM_LAUNCH_CHECK();
         return SLLM_OK;
     }
     if (dv >= 512 && dv <= 1024 * kNormPer)       // a warp per part would walk such a part in 16 and more rounds, twice
-        seq_headnorm_gate_wide_kernel<<<items, std::max(256, ((dv + kNormPer - 1) / kNormPer + 31) / 32 * 32), 0, as_stream(stream)>>>(o, ldo, g, ldg, w, heads, dv, eps, out, ldout,
+        overlapping(seq_headnorm_gate_wide_kernel)<<<items, std::max(256, ((dv + kNormPer - 1) / kNormPer + 31) / 32 * 32), 0, as_stream(stream)>>>(o, ldo, g, ldg, w, heads, dv, eps, out, ldout,
                                                                                                                     (uint16_t*)out16, mode);
     else
-        seq_headnorm_gate_kernel<<<(items + 3) / 4, 128, 0, as_stream(stream)>>>(o, ldo, g, ldg, w, heads, dv, eps, out, ldout, (uint16_t*)out16, T, mode);
+        overlapping(seq_headnorm_gate_kernel)<<<(items + 3) / 4, 128, 0, as_stream(stream)>>>(o, ldo, g, ldg, w, heads, dv, eps, out, ldout, (uint16_t*)out16, T, mode);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;
@@ -532,7 +551,7 @@ int sllm_seq_headnorm_gate(const float* o, int32_t ldo, const float* g, int32_t 
 int sllm_seq_layernorm(const float* x, int32_t ldx, const float* w, const float* bias, float eps, float* y, int32_t ldy, void* y16, int32_t T,
                        int32_t d, sllm_stream_t stream) {
     SLLM_REQUIRE(x && w && y && T > 0 && d > 0 && ldx >= d && ldy >= d, SLLM_EINVAL, "seq_layernorm: bad argument");
-    seq_layernorm_kernel<<<T, row_threads(T, d, d >= 2048 ? 256 : 128), 0, as_stream(stream)>>>(x, ldx, w, bias, eps, y, ldy, (uint16_t*)y16, d);
+    overlapping(seq_layernorm_kernel)<<<T, row_threads(T, d, d >= 2048 ? 256 : 128), 0, as_stream(stream)>>>(x, ldx, w, bias, eps, y, ldy, (uint16_t*)y16, d);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;
@@ -548,10 +567,10 @@ int sllm_seq_depth_average(float* x, const float* y, float* hist, int32_t n_prev
     const int threads = row_threads(T, vec ? d / 4 : d, d >= 2048 ? 256 : 128);
     if (vec) {
         if (smem > 48 * 1024) SLLM_CUDA(cudaFuncSetAttribute(seq_depth_average_kernel<float4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        seq_depth_average_kernel<float4><<<T, threads, smem, as_stream(stream)>>>(x, y, hist, n_prev, coef, norm_w, norm_b, eps, h, (uint16_t*)h16, T, d);
+        overlapping(seq_depth_average_kernel<float4>)<<<T, threads, smem, as_stream(stream)>>>(x, y, hist, n_prev, coef, norm_w, norm_b, eps, h, (uint16_t*)h16, T, d);
     } else {
         if (smem > 48 * 1024) SLLM_CUDA(cudaFuncSetAttribute(seq_depth_average_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        seq_depth_average_kernel<float><<<T, threads, smem, as_stream(stream)>>>(x, y, hist, n_prev, coef, norm_w, norm_b, eps, h, (uint16_t*)h16, T, d);
+        overlapping(seq_depth_average_kernel<float>)<<<T, threads, smem, as_stream(stream)>>>(x, y, hist, n_prev, coef, norm_w, norm_b, eps, h, (uint16_t*)h16, T, d);
     }
     ++g_launches;
     SLLM_LAUNCH_CHECK();
@@ -563,14 +582,14 @@ int sllm_seq_clamped_glu(const float* gate, int32_t ldg, const float* up, int32_
     SLLM_REQUIRE(gate && up && (out || out16) && T > 0 && n > 0 && ldg >= n && ldu >= n && (!out || ldo >= n), SLLM_EINVAL, "seq_clamped_glu: bad argument");
     auto aligned = [](const void* q) { return q == nullptr || ((uintptr_t)q % 16) == 0; };
     if (n % 4 == 0 && ldg % 4 == 0 && ldu % 4 == 0 && (!out || ldo % 4 == 0) && aligned(gate) && aligned(up) && aligned(out) && aligned(out16)) {
-        seq_clamped_glu_vec_kernel<<<dim3(T, std::min(64, (n / 4 + 255) / 256)), n >= 1024 ? 256 : 64, 0, as_stream(stream)>>>(gate, ldg, up, ldu, limit, alpha, out, ldo,
+        overlapping(seq_clamped_glu_vec_kernel)<<<dim3(T, std::min(64, (n / 4 + 255) / 256)), n >= 1024 ? 256 : 64, 0, as_stream(stream)>>>(gate, ldg, up, ldu, limit, alpha, out, ldo,
                                                                                                                            (uint16_t*)out16, n);
         ++g_launches;
         SLLM_LAUNCH_CHECK();
         return SLLM_OK;
     }
     const size_t total = (size_t)T * n;
-    seq_clamped_glu_kernel<<<(int)std::min<size_t>((total + 255) / 256, (size_t)sm_count() * 8), 256, 0, as_stream(stream)>>>(gate, ldg, up, ldu, limit, alpha, out,
+    overlapping(seq_clamped_glu_kernel)<<<(int)std::min<size_t>((total + 255) / 256, (size_t)sm_count() * 8), 256, 0, as_stream(stream)>>>(gate, ldg, up, ldu, limit, alpha, out,
                                                                                                                        ldo, (uint16_t*)out16, T, n);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
@@ -581,7 +600,7 @@ int sllm_seq_embed_pair(const int32_t* ids, const int32_t* prev_ids, const void*
                         int32_t buckets, int64_t mul_prev, int64_t mul_cur, float* out, int32_t T, sllm_stream_t stream) {
     SLLM_REQUIRE(ids && prev_ids && table && pairs && out && T > 0 && d > 0 && vocab > 0 && buckets > 0, SLLM_EINVAL, "seq_embed_pair: bad argument");
     SLLM_REQUIRE(w_dtype == SLLM_F32 || w_dtype == SLLM_BF16, SLLM_ENOTSUP, "seq_embed_pair: fp32 or bf16 tables");
-    seq_embed_pair_kernel<<<T, row_threads(T, d, 128), 0, as_stream(stream)>>>(ids, prev_ids, table, pairs, w_dtype, vocab, d, buckets, mul_prev, mul_cur, out);
+    overlapping(seq_embed_pair_kernel)<<<T, row_threads(T, d, 128), 0, as_stream(stream)>>>(ids, prev_ids, table, pairs, w_dtype, vocab, d, buckets, mul_prev, mul_cur, out);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;
@@ -589,8 +608,8 @@ int sllm_seq_embed_pair(const int32_t* ids, const int32_t* prev_ids, const void*
 
 int sllm_seq_rmsnorm_rows(const float* x, int32_t ldx, const float* w, float eps, float* y, int32_t ldy, int32_t T, int32_t n, sllm_stream_t stream) {
     SLLM_REQUIRE(x && y && T > 0 && n > 0 && ldx >= n && ldy >= n, SLLM_EINVAL, "seq_rmsnorm_rows: bad argument");
-    if (T < 64 && n > 128) seq_rmsnorm_row_cta_kernel<<<T, std::min(1024, (n + 31) / 32 * 32), 0, as_stream(stream)>>>(x, ldx, w, eps, y, ldy, n);
-    else seq_rmsnorm_rows_kernel<<<(T + 3) / 4, 128, 0, as_stream(stream)>>>(x, ldx, w, eps, y, ldy, T, n);
+    if (T < 64 && n > 128) overlapping(seq_rmsnorm_row_cta_kernel)<<<T, std::min(1024, (n + 31) / 32 * 32), 0, as_stream(stream)>>>(x, ldx, w, eps, y, ldy, n);
+    else overlapping(seq_rmsnorm_rows_kernel)<<<(T + 3) / 4, 128, 0, as_stream(stream)>>>(x, ldx, w, eps, y, ldy, T, n);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;
@@ -603,13 +622,13 @@ int sllm_seq_gated_act(const float* gate, int32_t ldg, const float* up, int32_t 
     auto aligned = [](const void* q) { return q == nullptr || ((uintptr_t)q % 16) == 0; };
     if (n % 4 == 0 && ldg % 4 == 0 && ldu % 4 == 0 && (!out || ldo % 4 == 0) && aligned(gate) && aligned(up) && aligned(out) && aligned(out16)) {
         const int parts = std::min(64, (n / 4 + 255) / 256);
-        seq_gated_act_vec_kernel<<<dim3(T, parts), n >= 1024 ? 256 : 64, 0, as_stream(stream)>>>(gate, ldg, up, ldu, out, ldo, (uint16_t*)out16, n);
+        overlapping(seq_gated_act_vec_kernel)<<<dim3(T, parts), n >= 1024 ? 256 : 64, 0, as_stream(stream)>>>(gate, ldg, up, ldu, out, ldo, (uint16_t*)out16, n);
         ++g_launches;
         SLLM_LAUNCH_CHECK();
         return SLLM_OK;
     }
     const size_t total = (size_t)T * n;
-    seq_gated_act_kernel<<<(int)std::min<size_t>((total + 255) / 256, (size_t)sm_count() * 8), 256, 0, as_stream(stream)>>>(gate, ldg, up, ldu, act, out, ldo,
+    overlapping(seq_gated_act_kernel)<<<(int)std::min<size_t>((total + 255) / 256, (size_t)sm_count() * 8), 256, 0, as_stream(stream)>>>(gate, ldg, up, ldu, act, out, ldo,
                                                                                                                      (uint16_t*)out16, T, n);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
@@ -618,7 +637,7 @@ int sllm_seq_gated_act(const float* gate, int32_t ldg, const float* up, int32_t 
 
 int sllm_seq_softcap(float* x, int64_t n, float cap, sllm_stream_t stream) {
     SLLM_REQUIRE(x && n > 0 && cap > 0.0f, SLLM_EINVAL, "seq_softcap: bad argument");
-    seq_softcap_kernel<<<(int)std::min<size_t>(((size_t)n + 255) / 256, (size_t)sm_count() * 8), 256, 0, as_stream(stream)>>>(x, (size_t)n, cap);
+    overlapping(seq_softcap_kernel)<<<(int)std::min<size_t>(((size_t)n + 255) / 256, (size_t)sm_count() * 8), 256, 0, as_stream(stream)>>>(x, (size_t)n, cap);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;

@@ -22,6 +22,7 @@ struct LinArgs {
     const int32_t* w_index;    // rows body, device memory or NULL: product b of the batch uses matrix w_index[b] (W + w_index[b] * w_bs); -1 = no matrix, zeros
     int a_div;                 // rows body: product b reads the activations of batch element b / a_div (0 or 1: its own)
     int rows_bs;               // tile body: 1 = a row count per product of the batch
+    int w_fixed;               // rows bodies: no kernel enqueued shortly before writes W, its first rows are asked for before the wait for those kernels
 };
 
 constexpr int kRowsMax = 8;
@@ -52,6 +53,8 @@ __global__ void __launch_bounds__(RowsShape<TT>::kWarps * 32, 1) seq_linear_rows
     constexpr int C = Shape::kChunks, RG = Shape::kGroup, D = Shape::kDeep, V = RG * TT;
     extern __shared__ __align__(16) uint8_t rows_smem[];
     const int b = blockIdx.y;
+    const bool early = p.w_fixed && !p.w_index;
+    if (!early) after_previous();
     const int wb = p.w_index ? p.w_index[b] : b;               // which matrix of W; negative: none (the outputs are zeros)
     const float* A = p.A + (size_t)(p.a_div > 1 ? b / p.a_div : b) * p.a_bs;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -123,10 +126,9 @@ __global__ void __launch_bounds__(RowsShape<TT>::kWarps * 32, 1) seq_linear_rows
     };
     if (blocks) begin_run(); else pad = 1 << 30;
 #pragma unroll
-    for (int i = 0; i < D / 2; ++i) issue();
+    for (int i = 0; i < D; ++i) issue();
+    if (early) after_previous();
     load_act(0);
-#pragma unroll
-    for (int i = D / 2; i < D; ++i) issue();
 
     // after the exchange a lane holds the sum of row `which / TT` of the group and activation row `which % TT`
     int which = 0;
@@ -224,6 +226,8 @@ template <int WD, bool kShort>
 __global__ void __launch_bounds__(256, 4) seq_linear_rows_small_kernel(LinArgs p, int vec, int wpr) {
     __shared__ float part_sum[8][kRowsMax];
     const int b = blockIdx.y;
+    const bool early = p.w_fixed && !p.w_index && vec;
+    if (!early) after_previous();
     const int wb = p.w_index ? p.w_index[b] : b;             // which matrix of W; negative: none (the outputs are zeros)
     const float* A = p.A + (size_t)(p.a_div > 1 ? b / p.a_div : b) * p.a_bs;
     const float* bias = p.bias ? p.bias + (size_t)b * p.bias_bs : nullptr;
@@ -281,6 +285,7 @@ __global__ void __launch_bounds__(256, 4) seq_linear_rows_small_kernel(LinArgs p
             int k0 = k_lo + lane * E;
             uint4 cur[kInFlight];
             load(cur, k0);
+            if (early) after_previous();
             for (; k0 < k_hi; k0 += kStep) {
                 uint4 nxt[kInFlight];
                 load(nxt, k0 + kStep);
@@ -300,6 +305,8 @@ __global__ void __launch_bounds__(256, 4) seq_linear_rows_small_kernel(LinArgs p
                     }
             }
         }
+    } else if (early) {
+        after_previous();
     }
 #pragma unroll
     for (int t = 0; t < kRowsMax; ++t) {
@@ -320,6 +327,7 @@ constexpr int kTM = 64, kTN = 64, kTK = 16;
 
 template <int WD>
 __global__ void __launch_bounds__(256) seq_linear_tile_kernel(LinArgs p) {
+    after_previous();
     __shared__ float As[kTK][kTM + 4];
     __shared__ float Ws[kTK][kTN + 4];
     const int b = blockIdx.z;
@@ -383,7 +391,8 @@ __global__ void __launch_bounds__(256) seq_linear_tile_kernel(LinArgs p) {
 
 // A (fp32, row stride lda) -> bf16 [T][K] dense, K a multiple of 8: eight values per thread, 16-byte accesses where A allows them. Bound: HBM. Element by
 // element, with a 64-bit division each, 2048 x 2048 took 13.1 us; 5 us like this.
-__global__ void __launch_bounds__(256) seq_to_bf16_kernel(const float* __restrict__ A, int lda, uint16_t* __restrict__ out, int T, int K, int vec) {
+__global__ void __launch_bounds__(256) seq_to_bf16_kernel(const float* A, int lda, uint16_t* out, int T, int K, int vec) {
+    after_previous();
     const int per_row = K / 8;
     const long long n = (long long)T * per_row, stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -403,8 +412,9 @@ __global__ void __launch_bounds__(256) seq_to_bf16_kernel(const float* __restric
 }
 
 // C = alpha * (P + bias) (+ C) where P [T][N] dense holds the plain product
-__global__ void seq_linear_epilogue_kernel(const float* __restrict__ P, const float* __restrict__ bias, float* __restrict__ C, int ldc, int T, int N,
+__global__ void seq_linear_epilogue_kernel(const float* P, const float* bias, float* C, int ldc, int T, int N,
                                            float alpha, int accumulate) {
+    after_previous();
     const size_t n = (size_t)T * N;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const size_t t = i / N, j = i % N;
@@ -433,7 +443,7 @@ static int launch_rows_body(const sllm::LinArgs& p, int batch, cudaStream_t st) 
         sized = true;
     }
     const dim3 grid(std::max(1, std::min(p.N, sm_count() / batch)), batch);      // one CTA per SM, however many products share the launch
-    seq_linear_rows_kernel<WD, TT><<<grid, Shape::kWarps * 32, smem, st>>>(p, wk_log2);
+    overlapping(seq_linear_rows_kernel<WD, TT>)<<<grid, Shape::kWarps * 32, smem, st>>>(p, wk_log2);
     return SLLM_OK;
 }
 
@@ -467,10 +477,10 @@ static int launch_rows(const sllm::LinArgs& p, int batch, cudaStream_t st) {
         while (wpr < 8 && (long long)p.N * batch * wpr / 8 < 4LL * sm_count() && p.K / (2 * wpr) >= 256) wpr *= 2;
         dim3 grid(((long long)p.N * wpr + 7) / 8, batch);
         const bool brief = weights >= 1500000LL;
-        if (bf16 && brief) seq_linear_rows_small_kernel<SLLM_BF16, true><<<grid, 256, 0, st>>>(p, vec, wpr);
-        else if (bf16) seq_linear_rows_small_kernel<SLLM_BF16, false><<<grid, 256, 0, st>>>(p, vec, wpr);
-        else if (brief) seq_linear_rows_small_kernel<SLLM_F32, true><<<grid, 256, 0, st>>>(p, vec, wpr);
-        else seq_linear_rows_small_kernel<SLLM_F32, false><<<grid, 256, 0, st>>>(p, vec, wpr);
+        if (bf16 && brief) overlapping(seq_linear_rows_small_kernel<SLLM_BF16, true>)<<<grid, 256, 0, st>>>(p, vec, wpr);
+        else if (bf16) overlapping(seq_linear_rows_small_kernel<SLLM_BF16, false>)<<<grid, 256, 0, st>>>(p, vec, wpr);
+        else if (brief) overlapping(seq_linear_rows_small_kernel<SLLM_F32, true>)<<<grid, 256, 0, st>>>(p, vec, wpr);
+        else overlapping(seq_linear_rows_small_kernel<SLLM_F32, false>)<<<grid, 256, 0, st>>>(p, vec, wpr);
     }
     ++g_launches;
     SLLM_LAUNCH_CHECK();
@@ -484,7 +494,7 @@ extern "C" int sllm_seq_linear_indexed(const float* A, int32_t lda, int64_t a_bs
     SLLM_REQUIRE(A && W && C && w_index && batch > 0 && batch <= 65535 && N > 0 && K > 0 && a_div >= 1, SLLM_EINVAL, "seq_linear_indexed: bad argument");
     SLLM_REQUIRE(lda >= K && ldw >= K && ldc >= N, SLLM_EINVAL, "seq_linear_indexed: row strides shorter than the rows");
     SLLM_REQUIRE(w_dtype == SLLM_F32 || w_dtype == SLLM_BF16, SLLM_ENOTSUP, "seq_linear_indexed: fp32 or bf16 weights");
-    LinArgs p{A, W, nullptr, C, lda, ldw, ldc, 1, N, K, w_dtype, 0, round_a, 1.0f, a_bs, w_bs, 0, c_bs, nullptr, w_index, a_div, 0};
+    LinArgs p{A, W, nullptr, C, lda, ldw, ldc, 1, N, K, w_dtype, 0, round_a, 1.0f, a_bs, w_bs, 0, c_bs, nullptr, w_index, a_div, 0, 0};
     return launch_rows(p, batch, as_stream(stream));
 }
 
@@ -500,7 +510,9 @@ extern "C" int sllm_seq_linear(const float* A, int32_t lda, const void* W, int32
     SLLM_REQUIRE(lda >= K && ldw >= K && ldc >= N, SLLM_EINVAL, "seq_linear: row strides shorter than the rows");
     SLLM_REQUIRE(w_dtype == SLLM_F32 || w_dtype == SLLM_BF16, SLLM_ENOTSUP, "seq_linear: fp32 or bf16 weights");
     cudaStream_t st = as_stream(stream);
-    LinArgs p{A, W, bias, C, lda, ldw, ldc, T, N, K, w_dtype, accumulate, round_a, alpha, a_bs, w_bs, bias_bs, c_bs, rows_dev, nullptr, 0, 0};
+    const int w_fixed = (round_a & SLLM_SEQ_W_FIXED) != 0;
+    round_a &= ~SLLM_SEQ_W_FIXED;
+    LinArgs p{A, W, bias, C, lda, ldw, ldc, T, N, K, w_dtype, accumulate, round_a, alpha, a_bs, w_bs, bias_bs, c_bs, rows_dev, nullptr, 0, 0, w_fixed};
     if (T <= kRowsMax) return launch_rows(p, batch, st);
     // tensor cores: bf16 weights, a dense bf16 copy of A, rows that TMA can address (16-byte multiples) and enough work to fill tiles
     const bool tensor_cores = a16 && sllm_seq_linear_on_tensor_cores(T, N, K, w_dtype, ldw, batch, round_a) && ((uintptr_t)W % 16) == 0;
@@ -510,7 +522,7 @@ extern "C" int sllm_seq_linear(const float* A, int32_t lda, const void* W, int32
         if (!a16_ready) {   // else the kernel that produced A has left its bf16 rows in a16 already
             const size_t n = (size_t)T * K / 8;
             const int vec = lda % 4 == 0 && ((uintptr_t)A % 16) == 0;
-            seq_to_bf16_kernel<<<(int)std::min<size_t>((n + 255) / 256, (size_t)sm_count() * 8), 256, 0, st>>>(A, lda, reinterpret_cast<uint16_t*>(a16), T, K, vec);
+            overlapping(seq_to_bf16_kernel)<<<(int)std::min<size_t>((n + 255) / 256, (size_t)sm_count() * 8), 256, 0, st>>>(A, lda, reinterpret_cast<uint16_t*>(a16), T, K, vec);
             ++g_launches;
             SLLM_LAUNCH_CHECK();
         }
@@ -527,14 +539,14 @@ extern "C" int sllm_seq_linear(const float* A, int32_t lda, const void* W, int32
         const int rc = pf_gemm(cache, a, st);
         if (rc != SLLM_OK) return rc;
         const size_t m = (size_t)T * N;
-        seq_linear_epilogue_kernel<<<(int)std::min<size_t>((m + 255) / 256, (size_t)sm_count() * 8), 256, 0, st>>>(P, bias, C, ldc, T, N, alpha, accumulate);
+        overlapping(seq_linear_epilogue_kernel)<<<(int)std::min<size_t>((m + 255) / 256, (size_t)sm_count() * 8), 256, 0, st>>>(P, bias, C, ldc, T, N, alpha, accumulate);
         ++g_launches;
         SLLM_LAUNCH_CHECK();
         return SLLM_OK;
     }
     dim3 grid((N + kTN - 1) / kTN, (T + kTM - 1) / kTM, batch);
-    if (w_dtype == SLLM_BF16) seq_linear_tile_kernel<SLLM_BF16><<<grid, 256, 0, st>>>(p);
-    else seq_linear_tile_kernel<SLLM_F32><<<grid, 256, 0, st>>>(p);
+    if (w_dtype == SLLM_BF16) overlapping(seq_linear_tile_kernel<SLLM_BF16>)<<<grid, 256, 0, st>>>(p);
+    else overlapping(seq_linear_tile_kernel<SLLM_F32>)<<<grid, 256, 0, st>>>(p);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;
@@ -557,10 +569,10 @@ extern "C" int sllm_seq_linear_grouped(const void* A, int32_t a_bf16, const void
         return pf_gemm(cache, a, st);
     }
     LinArgs p{(const float*)A, W, nullptr, C, K, K, N, cap, N, K, w_dtype, 0, w_dtype == SLLM_BF16, 1.0f, (long long)cap * K, (long long)N * K, 0, (long long)cap * N,
-              counts, nullptr, 0, 1};
+              counts, nullptr, 0, 1, 0};
     dim3 grid((N + kTN - 1) / kTN, (cap + kTM - 1) / kTM, groups);
-    if (w_dtype == SLLM_BF16) seq_linear_tile_kernel<SLLM_BF16><<<grid, 256, 0, st>>>(p);
-    else seq_linear_tile_kernel<SLLM_F32><<<grid, 256, 0, st>>>(p);
+    if (w_dtype == SLLM_BF16) overlapping(seq_linear_tile_kernel<SLLM_BF16>)<<<grid, 256, 0, st>>>(p);
+    else overlapping(seq_linear_tile_kernel<SLLM_F32>)<<<grid, 256, 0, st>>>(p);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;

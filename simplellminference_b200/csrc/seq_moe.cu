@@ -34,7 +34,7 @@ __device__ __forceinline__ float moe_glu(float g, float u, int kind, float limit
 
 // One warp routes a token: scores and choice scores to shared memory (softmax over all router outputs, or every output's own sigmoid), experts
 // outside the best groups out of the choice. s_group: [2 * groups] floats.
-__device__ __forceinline__ void moe_scores(const float* __restrict__ z, int n_route, const float* __restrict__ correction, int mode, const sllm_seq_moe_opts& o,
+__device__ __forceinline__ void moe_scores(const float* z, int n_route, const float* correction, int mode, const sllm_seq_moe_opts& o,
                                            float* s_score, float* s_choice, float* s_group, int lane) {
     float inv = 1.0f;
     if (mode & kMoeSigmoid) {
@@ -111,10 +111,11 @@ __device__ __forceinline__ float moe_weight_factor(float sum, int mode, const sl
 }
 
 // one CTA per token; shared: scores [n_route], weights [n_route]
-__global__ void seq_moe_act_kernel(const float* __restrict__ logits, int ldl, int n_route, int experts, int top, const float* __restrict__ correction,
-                                   const float* __restrict__ up, int ldu, int ff, int act, const float* __restrict__ h, int ldh, int d,
-                                   float* __restrict__ out, uint16_t* __restrict__ out16, float* __restrict__ y, int ldy, float* __restrict__ route_w,
-                                   const float* __restrict__ shared_up, int ld_shared, int shared_ff, sllm_seq_moe_opts o) {
+__global__ void seq_moe_act_kernel(const float* logits, int ldl, int n_route, int experts, int top, const float* correction,
+                                   const float* up, int ldu, int ff, int act, const float* h, int ldh, int d,
+                                   float* out, uint16_t* out16, float* y, int ldy, float* route_w,
+                                   const float* shared_up, int ld_shared, int shared_ff, sllm_seq_moe_opts o) {
+    after_previous();
     extern __shared__ float msm[];
     float* s_score = msm;
     float* s_choice = msm + n_route;
@@ -198,7 +199,7 @@ extern "C" int sllm_seq_moe_act(const float* logits, int32_t ldl, int32_t n_rout
     SLLM_REQUIRE(n_route <= 2048, SLLM_ENOTSUP, "seq_moe_act: %d router outputs beyond 2048", n_route);
     const int work = std::max(experts * ff + shared_ff, d);
     const int threads = T >= 64 ? 256 : std::min(1024, std::max(128, (work + 31) / 32 * 32));
-    seq_moe_act_kernel<<<T, threads, (3 * (size_t)n_route + 2 * std::max(o.groups, 0)) * sizeof(float), as_stream(stream)>>>(
+    overlapping(seq_moe_act_kernel)<<<T, threads, (3 * (size_t)n_route + 2 * std::max(o.groups, 0)) * sizeof(float), as_stream(stream)>>>(
         logits, ldl, n_route, experts, top, correction, up, ldu, ff, act, h, ldh, d, out, (uint16_t*)out16, y, ldy, route_w, shared_up, ld_shared, shared_ff, o);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
@@ -212,10 +213,11 @@ extern "C" int sllm_seq_moe_act(const float* logits, int32_t ldl, int32_t n_rout
 // the device: sllm_seq_linear's rows_dev); the combine kernel adds each token's rows, times their scores, to (identity scores) * input.
 namespace sllm {
 
-__global__ void seq_moe_route_kernel(int act, const float* __restrict__ logits, int ldl, int n_route, int experts, int top, const float* __restrict__ correction,
-                                     const float* __restrict__ h, int ldh, int d, int32_t* __restrict__ counts, int cap, int32_t* __restrict__ sel_e,
-                                     int32_t* __restrict__ sel_pos, float* __restrict__ sel_w, float* __restrict__ ident_out, uint16_t* __restrict__ rows16,
-                                     float* __restrict__ rows32, const uint16_t* __restrict__ h16, sllm_seq_moe_opts o) {
+__global__ void seq_moe_route_kernel(int act, const float* logits, int ldl, int n_route, int experts, int top, const float* correction,
+                                     const float* h, int ldh, int d, int32_t* counts, int cap, int32_t* sel_e,
+                                     int32_t* sel_pos, float* sel_w, float* ident_out, uint16_t* rows16,
+                                     float* rows32, const uint16_t* h16, sllm_seq_moe_opts o) {
+    after_previous();
     extern __shared__ float msm[];
     float* s_score = msm;
     float* s_choice = msm + n_route;
@@ -283,13 +285,15 @@ __global__ void seq_moe_route_kernel(int act, const float* __restrict__ logits, 
 }
 
 // x <- act(x) over n floats
-__global__ void seq_act_kernel(float* __restrict__ x, size_t n, int act) {
+__global__ void seq_act_kernel(float* x, size_t n, int act) {
+    after_previous();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) x[i] = moe_act(x[i], act);
 }
 
 // grid (cap, experts): rows in use only
-__global__ void seq_moe_expert_act_kernel(const float* __restrict__ up, const int32_t* __restrict__ counts, int cap, int ff, int act,
-                                          uint16_t* __restrict__ out16, float* __restrict__ out32, float limit) {
+__global__ void seq_moe_expert_act_kernel(const float* up, const int32_t* counts, int cap, int ff, int act,
+                                          uint16_t* out16, float* out32, float limit) {
+    after_previous();
     const int e = blockIdx.y, r = blockIdx.x;
     if (r >= counts[e]) return;
     const size_t row = ((size_t)e * cap + r) * ff;
@@ -315,8 +319,9 @@ __global__ void seq_moe_expert_act_kernel(const float* __restrict__ up, const in
 // grid (pairs, parts of a row), rows in the (token, choice) pairs' own order: out = act(s * up) or act(s * gate) * (s * up), with s the pair's
 // score when the score multiplies what the expert reads (the products are linear: the score is applied to their results) and 1 otherwise;
 // w_out takes what the combine kernel has to multiply the pair's down row by: 1 in the first case, the score in the second
-__global__ void seq_moe_pair_act_kernel(const float* __restrict__ up, const float* __restrict__ sel_w, int ff, int act, float* __restrict__ out,
-                                        float* __restrict__ w_out, float limit) {
+__global__ void seq_moe_pair_act_kernel(const float* up, const float* sel_w, int ff, int act, float* out,
+                                        float* w_out, float limit) {
+    after_previous();
     const int p = blockIdx.x;
     const bool gated = act & kMoeGated, on_input = act & kMoeScaleInput;
     const float score = sel_w[p], s = on_input ? score : 1.0f;
@@ -326,9 +331,10 @@ __global__ void seq_moe_pair_act_kernel(const float* __restrict__ up, const floa
     if (threadIdx.x == 0 && blockIdx.y == 0) w_out[p] = on_input ? 1.0f : score;
 }
 
-__global__ void seq_moe_combine_kernel(const float* __restrict__ down, const int32_t* __restrict__ sel_e, const int32_t* __restrict__ sel_pos,
-                                       const float* __restrict__ sel_w, int top, const float* __restrict__ ident, const float* __restrict__ h, int ldh,
-                                       int cap, int d, float* __restrict__ y, int ldy) {
+__global__ void seq_moe_combine_kernel(const float* down, const int32_t* sel_e, const int32_t* sel_pos,
+                                       const float* sel_w, int top, const float* ident, const float* h, int ldh,
+                                       int cap, int d, float* y, int ldy) {
+    after_previous();
     extern __shared__ float csm[];                           // [top] score (0 = no row), [top] row offset
     float* s_w = csm;
     long long* s_row = reinterpret_cast<long long*>(csm + ((top + 1) & ~1));
@@ -354,7 +360,7 @@ extern "C" {
 
 int sllm_seq_act(float* x, int64_t n, int32_t act, sllm_stream_t stream) {
     SLLM_REQUIRE(x && n > 0 && act >= 0 && act <= 2, SLLM_EINVAL, "seq_act: bad argument");
-    seq_act_kernel<<<(int)std::min<size_t>(((size_t)n + 255) / 256, (size_t)sm_count() * 8), 256, 0, as_stream(stream)>>>(x, (size_t)n, act);
+    overlapping(seq_act_kernel)<<<(int)std::min<size_t>(((size_t)n + 255) / 256, (size_t)sm_count() * 8), 256, 0, as_stream(stream)>>>(x, (size_t)n, act);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;
@@ -378,7 +384,7 @@ int sllm_seq_moe_route(const float* logits, int32_t ldl, int32_t n_route, int32_
     if (int rc = moe_options(opts, n_route, mode, "seq_moe_route", &o)) return rc;
     SLLM_REQUIRE(n_route <= 2048 && top <= 1024, SLLM_ENOTSUP, "seq_moe_route: %d router outputs / top %d beyond what one CTA routes", n_route, top);
     const size_t smem = (2 * (size_t)n_route + 3 * (size_t)top + 2 * (size_t)std::max(o.groups, 0)) * sizeof(float);
-    seq_moe_route_kernel<<<T, 256, smem, as_stream(stream)>>>(mode, logits, ldl, n_route, experts, top, correction, h, ldh, d, counts, cap, sel_e, sel_pos, sel_w, ident,
+    overlapping(seq_moe_route_kernel)<<<T, 256, smem, as_stream(stream)>>>(mode, logits, ldl, n_route, experts, top, correction, h, ldh, d, counts, cap, sel_e, sel_pos, sel_w, ident,
                                                                (uint16_t*)rows16, rows32, (const uint16_t*)h16, o);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
@@ -390,7 +396,7 @@ int sllm_seq_moe_expert_act(const float* up, const int32_t* counts, int32_t expe
     SLLM_REQUIRE(up && counts && (out16 || out32) && experts > 0 && cap > 0 && cap <= 65535 * 32 && ff > 0 && act >= 0 && ((act & 3) <= 2 || (act & kMoeGated)), SLLM_EINVAL,
                  "seq_moe_expert_act: bad argument");
     SLLM_REQUIRE(experts <= 65535, SLLM_ENOTSUP, "seq_moe_expert_act: %d experts", experts);
-    seq_moe_expert_act_kernel<<<dim3(cap, experts), 256, 0, as_stream(stream)>>>(up, counts, cap, ff, act, (uint16_t*)out16, out32, limit);
+    overlapping(seq_moe_expert_act_kernel)<<<dim3(cap, experts), 256, 0, as_stream(stream)>>>(up, counts, cap, ff, act, (uint16_t*)out16, out32, limit);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;
@@ -399,7 +405,7 @@ int sllm_seq_moe_expert_act(const float* up, const int32_t* counts, int32_t expe
 int sllm_seq_moe_pair_act(const float* up, const float* sel_w, int32_t pairs, int32_t ff, int32_t act, float* out, float* w_out, float limit,
                           sllm_stream_t stream) {
     SLLM_REQUIRE(up && sel_w && out && w_out && pairs > 0 && ff > 0 && act >= 0 && ((act & 3) <= 2 || (act & kMoeGated)) && act < 64, SLLM_EINVAL, "seq_moe_pair_act: bad argument");
-    seq_moe_pair_act_kernel<<<dim3(pairs, std::min(64, (ff + 255) / 256)), 256, 0, as_stream(stream)>>>(up, sel_w, ff, act, out, w_out, limit);
+    overlapping(seq_moe_pair_act_kernel)<<<dim3(pairs, std::min(64, (ff + 255) / 256)), 256, 0, as_stream(stream)>>>(up, sel_w, ff, act, out, w_out, limit);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;
@@ -411,7 +417,7 @@ int sllm_seq_moe_combine(const float* down, const int32_t* sel_e, const int32_t*
     SLLM_REQUIRE(top <= 2048, SLLM_ENOTSUP, "seq_moe_combine: top %d beyond 2048", top);
     const int threads = T >= 64 ? 256 : std::min(1024, std::max(128, (d + 31) / 32 * 32));
     const size_t smem = (size_t)((top + 1) & ~1) * sizeof(float) + (size_t)top * sizeof(long long);
-    seq_moe_combine_kernel<<<T, threads, smem, as_stream(stream)>>>(down, sel_e, sel_pos, sel_w, top, ident, h, ldh, cap, d, y, ldy);
+    overlapping(seq_moe_combine_kernel)<<<T, threads, smem, as_stream(stream)>>>(down, sel_e, sel_pos, sel_w, top, ident, h, ldh, cap, d, y, ldy);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;

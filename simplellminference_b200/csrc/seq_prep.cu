@@ -20,9 +20,10 @@ namespace sllm {
 
 // grid (T, ceil(items / 4)), 4 warps: warp = one head of q, k or v of one token
 template <typename KV>
-__global__ void seq_unit_kv_kernel(sllm_seq_batch b, float* __restrict__ q, int ldq, int heads, int dk, const float* __restrict__ k, int ldk, int kv_heads,
-                                   const float* __restrict__ v, int ldv, int dv, float eps, int unit, float* __restrict__ v_shared, int share, float lambda,
-                                   float q_temp_coef, int q_temp_every, KV* __restrict__ k_pool, KV* __restrict__ v_pool) {
+__global__ void seq_unit_kv_kernel(sllm_seq_batch b, float* q, int ldq, int heads, int dk, const float* k, int ldk, int kv_heads,
+                                   const float* v, int ldv, int dv, float eps, int unit, float* v_shared, int share, float lambda,
+                                   float q_temp_coef, int q_temp_every, KV* k_pool, KV* v_pool) {
+    after_previous();
     const int t = blockIdx.x, item = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (item >= heads + 2 * kv_heads) return;
     const int pos = b.tok_pos[t], slot = b.tok_slot[t];
@@ -72,9 +73,10 @@ __global__ void seq_unit_kv_kernel(sllm_seq_batch b, float* __restrict__ q, int 
 
 // one CTA per token
 template <typename KV>
-__global__ void seq_latent_kv_kernel(sllm_seq_batch b, const float* __restrict__ q, int ldq, int heads, int dn, int dr, const float* __restrict__ low, int ldlow,
-                                     int rank, const float* __restrict__ norm_w, float eps, const double* __restrict__ freq, int n_freq, float magnitude,
-                                     float* __restrict__ q_out, int ldqo, KV* __restrict__ pool) {
+__global__ void seq_latent_kv_kernel(sllm_seq_batch b, const float* q, int ldq, int heads, int dn, int dr, const float* low, int ldlow,
+                                     int rank, const float* norm_w, float eps, const double* freq, int n_freq, float magnitude,
+                                     float* q_out, int ldqo, KV* pool) {
+    after_previous();
     __shared__ float red[33];
     const int t = blockIdx.x, pos = b.tok_pos[t], slot = b.tok_slot[t];
     const int page = b.block_table[(size_t)slot * b.max_pages + pos / b.page_len], in_page = pos % b.page_len;
@@ -118,9 +120,10 @@ __global__ void seq_latent_kv_kernel(sllm_seq_batch b, const float* __restrict__
 // grid (T, ceil(items / 4)), 4 warps: warp = one query head (normed and rotated in place), one key head (normed, rotated -> pool) or one
 // value head (-> pool as it is); the head's row sits in shared memory while its pairs turn
 template <typename KV>
-__global__ void seq_normed_rotary_kv_kernel(sllm_seq_batch b, float* __restrict__ q, int ldq, int heads, int dk, const float* __restrict__ k, int ldk, int kv_heads,
-                                            const float* __restrict__ v, int ldv, int dv, const float* __restrict__ q_w, const float* __restrict__ k_w, float eps,
-                                            const double* __restrict__ freq, int n_freq, int layout, KV* __restrict__ k_pool, KV* __restrict__ v_pool) {
+__global__ void seq_normed_rotary_kv_kernel(sllm_seq_batch b, float* q, int ldq, int heads, int dk, const float* k, int ldk, int kv_heads,
+                                            const float* v, int ldv, int dv, const float* q_w, const float* k_w, float eps,
+                                            const double* freq, int n_freq, int layout, KV* k_pool, KV* v_pool) {
+    after_previous();
     extern __shared__ float nr_sm[];                     // [4][dk]
     const int t = blockIdx.x, item = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (item >= heads + 2 * kv_heads) return;
@@ -171,7 +174,8 @@ __device__ __forceinline__ void seq_st4(uint16_t* p, float4 v) {
 }
 
 // thread = (token, frequency)
-__global__ void seq_angles_kernel(sllm_seq_batch b, const double* __restrict__ freq, int n_freq, float2* __restrict__ out) {
+__global__ void seq_angles_kernel(sllm_seq_batch b, const double* freq, int n_freq, float2* out) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= b.T * n_freq) return;
     float sn, cs;
@@ -184,12 +188,13 @@ __global__ void seq_angles_kernel(sllm_seq_batch b, const double* __restrict__ f
 constexpr int kMixGroup = 8;   // query heads of a key head whose values a thread holds at once while it mixes
 
 template <typename KV>
-__global__ void __launch_bounds__(256) seq_wide_normed_rotary_kv_kernel(sllm_seq_batch b, float* __restrict__ q, int ldq, int heads, int dk, const float* __restrict__ k,
-                                                                        int ldk, int kv_heads, const float* __restrict__ v, int ldv, int dv, const float* __restrict__ q_w,
-                                                                        const float* __restrict__ k_w, float eps, const float2* __restrict__ angles, int n_freq, int layout,
-                                                                        float* __restrict__ v_shared, int share, float lambda, const float* __restrict__ talk,
-                                                                        uint16_t* __restrict__ q_mixed, int k_joint, KV* __restrict__ k_pool, KV* __restrict__ v_pool,
+__global__ void __launch_bounds__(256) seq_wide_normed_rotary_kv_kernel(sllm_seq_batch b, float* q, int ldq, int heads, int dk, const float* k,
+                                                                        int ldk, int kv_heads, const float* v, int ldv, int dv, const float* q_w,
+                                                                        const float* k_w, float eps, const float2* angles, int n_freq, int layout,
+                                                                        float* v_shared, int share, float lambda, const float* talk,
+                                                                        uint16_t* q_mixed, int k_joint, KV* k_pool, KV* v_pool,
                                                                         int vec) {
+    after_previous();
     extern __shared__ __align__(16) float wr_sm[];       // the row, and for the mix talk [heads][heads]
     __shared__ float red[33];
     const int t = blockIdx.x, pos = b.tok_pos[t], slot = b.tok_slot[t];
@@ -344,6 +349,7 @@ struct ConvRotaryArgs {
 // sits in shared memory while its pairs turn
 template <typename KV>
 __global__ void __launch_bounds__(128) seq_conv_rotary_kv_kernel(ConvRotaryArgs p) {
+    after_previous();
     extern __shared__ __align__(16) float cr_sm[];       // [4][max(dk, dv)]
     const sllm_seq_batch& b = p.b;
     const int item = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -445,6 +451,7 @@ __global__ void __launch_bounds__(128) seq_conv_rotary_kv_kernel(ConvRotaryArgs 
 // registers — the weights over the tile of tokens, the pairs that turn — and nothing passes through shared memory.
 template <typename KV, int TAPS>   // TAPS 0: no convolution
 __global__ void __launch_bounds__(128) seq_conv_rotary_kv_row_kernel(ConvRotaryArgs p) {
+    after_previous();
     const sllm_seq_batch& b = p.b;
     const int item = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (item >= p.heads + 2 * p.kv_heads) return;
@@ -509,8 +516,9 @@ __global__ void __launch_bounds__(128) seq_conv_rotary_kv_row_kernel(ConvRotaryA
 
 // thread = (token, head, column): out[t][h][c] = sum_g mix[h][g] * in[t][(h / group) * heads + g][c], group = heads / kv_heads: `in` holds,
 // for every key/value head, the result of EVERY query head's weights on that head's values
-__global__ void seq_head_mix_kernel(const float* __restrict__ in, int ldi, const float* __restrict__ mix, int heads, int kv_heads, int dv,
-                                    float* __restrict__ out, int ldo, uint16_t* __restrict__ out16, int T) {
+__global__ void seq_head_mix_kernel(const float* in, int ldi, const float* mix, int heads, int kv_heads, int dv,
+                                    float* out, int ldo, uint16_t* out16, int T) {
+    after_previous();
     extern __shared__ float hm_sm[];                     // [heads][heads]
     for (int i = threadIdx.x; i < heads * heads; i += blockDim.x) hm_sm[i] = mix[i];
     __syncthreads();
@@ -541,10 +549,10 @@ int sllm_seq_unit_kv(const sllm_seq_batch* b, float* q, int32_t ldq, int32_t hea
     SLLM_REQUIRE(kv_dtype == SLLM_F32 || kv_dtype == SLLM_BF16, SLLM_ENOTSUP, "seq_unit_kv: fp32 or bf16 pools");
     const dim3 grid(b->T, (heads + 2 * kv_heads + 3) / 4);
     if (kv_dtype == SLLM_F32)
-        seq_unit_kv_kernel<float><<<grid, 128, 0, as_stream(stream)>>>(*b, q, ldq, heads, dk, k, ldk, kv_heads, v, ldv, dv, eps, unit, v_shared, share, lambda,
+        overlapping(seq_unit_kv_kernel<float>)<<<grid, 128, 0, as_stream(stream)>>>(*b, q, ldq, heads, dk, k, ldk, kv_heads, v, ldv, dv, eps, unit, v_shared, share, lambda,
                                                                        q_temp_coef, q_temp_every, (float*)k_pool, (float*)v_pool);
     else
-        seq_unit_kv_kernel<uint16_t><<<grid, 128, 0, as_stream(stream)>>>(*b, q, ldq, heads, dk, k, ldk, kv_heads, v, ldv, dv, eps, unit, v_shared, share, lambda,
+        overlapping(seq_unit_kv_kernel<uint16_t>)<<<grid, 128, 0, as_stream(stream)>>>(*b, q, ldq, heads, dk, k, ldk, kv_heads, v, ldv, dv, eps, unit, v_shared, share, lambda,
                                                                           q_temp_coef, q_temp_every, (uint16_t*)k_pool, (uint16_t*)v_pool);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
@@ -560,10 +568,10 @@ int sllm_seq_latent_kv(const sllm_seq_batch* b, const float* q, int32_t ldq, int
     SLLM_REQUIRE(kv_dtype == SLLM_F32 || kv_dtype == SLLM_BF16, SLLM_ENOTSUP, "seq_latent_kv: fp32 or bf16 pools");
     const int threads = rank >= 512 ? 256 : 128;
     if (kv_dtype == SLLM_F32)
-        seq_latent_kv_kernel<float><<<b->T, threads, 0, as_stream(stream)>>>(*b, q, ldq, heads, dn, dr, low, ldlow, rank, norm_w, eps, freq, n_freq, magnitude, q_out, ldqo,
+        overlapping(seq_latent_kv_kernel<float>)<<<b->T, threads, 0, as_stream(stream)>>>(*b, q, ldq, heads, dn, dr, low, ldlow, rank, norm_w, eps, freq, n_freq, magnitude, q_out, ldqo,
                                                                              (float*)pool);
     else
-        seq_latent_kv_kernel<uint16_t><<<b->T, threads, 0, as_stream(stream)>>>(*b, q, ldq, heads, dn, dr, low, ldlow, rank, norm_w, eps, freq, n_freq, magnitude, q_out,
+        overlapping(seq_latent_kv_kernel<uint16_t>)<<<b->T, threads, 0, as_stream(stream)>>>(*b, q, ldq, heads, dn, dr, low, ldlow, rank, norm_w, eps, freq, n_freq, magnitude, q_out,
                                                                                 ldqo, (uint16_t*)pool);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
@@ -582,10 +590,10 @@ int sllm_seq_normed_rotary_kv(const sllm_seq_batch* b, float* q, int32_t ldq, in
     const dim3 grid(b->T, (heads + 2 * kv_heads + 3) / 4);
     const size_t smem = 4 * (size_t)dk * sizeof(float);
     if (kv_dtype == SLLM_F32)
-        seq_normed_rotary_kv_kernel<float><<<grid, 128, smem, as_stream(stream)>>>(*b, q, ldq, heads, dk, k, ldk, kv_heads, v, ldv, dv, q_norm_w, k_norm_w, eps, freq,
+        overlapping(seq_normed_rotary_kv_kernel<float>)<<<grid, 128, smem, as_stream(stream)>>>(*b, q, ldq, heads, dk, k, ldk, kv_heads, v, ldv, dv, q_norm_w, k_norm_w, eps, freq,
                                                                                  n_freq, layout, (float*)k_pool, (float*)v_pool);
     else
-        seq_normed_rotary_kv_kernel<uint16_t><<<grid, 128, smem, as_stream(stream)>>>(*b, q, ldq, heads, dk, k, ldk, kv_heads, v, ldv, dv, q_norm_w, k_norm_w, eps, freq,
+        overlapping(seq_normed_rotary_kv_kernel<uint16_t>)<<<grid, 128, smem, as_stream(stream)>>>(*b, q, ldq, heads, dk, k, ldk, kv_heads, v, ldv, dv, q_norm_w, k_norm_w, eps, freq,
                                                                                     n_freq, layout, (uint16_t*)k_pool, (uint16_t*)v_pool);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
@@ -594,7 +602,7 @@ int sllm_seq_normed_rotary_kv(const sllm_seq_batch* b, float* q, int32_t ldq, in
 
 int sllm_seq_angles(const sllm_seq_batch* b, const double* freq, int32_t n_freq, float* out, sllm_stream_t stream) {
     SLLM_REQUIRE(b && b->T > 0 && b->tok_pos && freq && out && n_freq > 0 && (uintptr_t)out % 8 == 0, SLLM_EINVAL, "seq_angles: bad argument");
-    seq_angles_kernel<<<(b->T * n_freq + 127) / 128, 128, 0, as_stream(stream)>>>(*b, freq, n_freq, (float2*)out);
+    overlapping(seq_angles_kernel)<<<(b->T * n_freq + 127) / 128, 128, 0, as_stream(stream)>>>(*b, freq, n_freq, (float2*)out);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;
@@ -621,7 +629,7 @@ int sllm_seq_wide_normed_rotary_kv(const sllm_seq_batch* b, float* q, int32_t ld
     do {                                                                                                                                                   \
         if (smem > 48 * 1024)                                                                                                                              \
             SLLM_CUDA(cudaFuncSetAttribute(seq_wide_normed_rotary_kv_kernel<KV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));                 \
-        seq_wide_normed_rotary_kv_kernel<KV><<<dim3(b->T, 2), 256, smem, as_stream(stream)>>>(*b, q, ldq, heads, dk, k, ldk, kv_heads, v, ldv, dv, q_norm_w, \
+        overlapping(seq_wide_normed_rotary_kv_kernel<KV>)<<<dim3(b->T, 2), 256, smem, as_stream(stream)>>>(*b, q, ldq, heads, dk, k, ldk, kv_heads, v, ldv, dv, q_norm_w, \
                                                                                              k_norm_w, eps, (const float2*)angles, n_freq, layout, v_shared, share, lambda, talk, \
                                                                                              (uint16_t*)q_mixed, k_joint, (KV*)k_pool, (KV*)v_pool, vec);   \
     } while (0)
@@ -655,8 +663,8 @@ int sllm_seq_conv_rotary_kv(const sllm_seq_batch* b, const float* q, int32_t ldq
     if (vec && layout == 0 && dk <= 128 && dv <= 128 && (!conv_w || taps <= 4)) {
 #define SLLM_ROW_LAUNCH(TAPS)                                                                                               \
     do {                                                                                                                    \
-        if (kv_dtype == SLLM_F32) seq_conv_rotary_kv_row_kernel<float, TAPS><<<grid, 128, 0, as_stream(stream)>>>(p);       \
-        else seq_conv_rotary_kv_row_kernel<uint16_t, TAPS><<<grid, 128, 0, as_stream(stream)>>>(p);                         \
+        if (kv_dtype == SLLM_F32) overlapping(seq_conv_rotary_kv_row_kernel<float, TAPS>)<<<grid, 128, 0, as_stream(stream)>>>(p);       \
+        else overlapping(seq_conv_rotary_kv_row_kernel<uint16_t, TAPS>)<<<grid, 128, 0, as_stream(stream)>>>(p);                         \
     } while (0)
         if (!conv_w) SLLM_ROW_LAUNCH(0);
         else if (taps == 1) SLLM_ROW_LAUNCH(1);
@@ -668,8 +676,8 @@ int sllm_seq_conv_rotary_kv(const sllm_seq_batch* b, const float* q, int32_t ldq
         SLLM_LAUNCH_CHECK();
         return SLLM_OK;
     }
-    if (kv_dtype == SLLM_F32) seq_conv_rotary_kv_kernel<float><<<grid, 128, smem, as_stream(stream)>>>(p);
-    else seq_conv_rotary_kv_kernel<uint16_t><<<grid, 128, smem, as_stream(stream)>>>(p);
+    if (kv_dtype == SLLM_F32) overlapping(seq_conv_rotary_kv_kernel<float>)<<<grid, 128, smem, as_stream(stream)>>>(p);
+    else overlapping(seq_conv_rotary_kv_kernel<uint16_t>)<<<grid, 128, smem, as_stream(stream)>>>(p);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;
@@ -680,7 +688,7 @@ int sllm_seq_head_mix(const float* in, int32_t ldi, const float* mix, int32_t he
     SLLM_REQUIRE(in && mix && (out || out16) && T > 0 && heads > 0 && kv_heads > 0 && heads % kv_heads == 0 && dv > 0, SLLM_EINVAL, "seq_head_mix: bad argument");
     SLLM_REQUIRE(heads <= 96, SLLM_ENOTSUP, "seq_head_mix: %d heads beyond 96", heads);
     const int threads = T >= 64 ? 256 : std::min(1024, std::max(128, (heads * dv + 31) / 32 * 32));
-    seq_head_mix_kernel<<<T, threads, (size_t)heads * heads * sizeof(float), as_stream(stream)>>>(in, ldi, mix, heads, kv_heads, dv, out, ldo, (uint16_t*)out16, T);
+    overlapping(seq_head_mix_kernel)<<<T, threads, (size_t)heads * heads * sizeof(float), as_stream(stream)>>>(in, ldi, mix, heads, kv_heads, dv, out, ldo, (uint16_t*)out16, T);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;

@@ -7,8 +7,9 @@
 namespace sllm {
 
 // thread = (token, channel); the taps-1 inputs before a segment come from the sequence's tail
-__global__ void seq_conv_kernel(sllm_seq_batch b, const float* __restrict__ x, int ldx, int channels, int taps, const float* __restrict__ w,
-                                const float* __restrict__ cb, const float* __restrict__ tail, float* __restrict__ u, int ldu) {
+__global__ void seq_conv_kernel(sllm_seq_batch b, const float* x, int ldx, int channels, int taps, const float* w,
+                                const float* cb, const float* tail, float* u, int ldu) {
+    after_previous();
     const int t = blockIdx.y, c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= channels) return;
     const int slot = b.tok_slot[t];
@@ -34,10 +35,11 @@ __global__ void seq_conv_kernel(sllm_seq_batch b, const float* __restrict__ x, i
 constexpr int kMaxTaps = 16;
 
 // thread = (segment, channel)
-__global__ void seq_rglru_scan_kernel(sllm_seq_batch b, const float* __restrict__ u, int ldu, const float* __restrict__ lr, const float* __restrict__ li,
-                                      int ldg, const float* __restrict__ ypre, int ldy, const float* __restrict__ lam, float cc, int channels,
-                                      float* __restrict__ state, const float* __restrict__ xconv, int ldx, int taps, float* __restrict__ tail,
-                                      float* __restrict__ out, int ldo) {
+__global__ void seq_rglru_scan_kernel(sllm_seq_batch b, const float* u, int ldu, const float* lr, const float* li,
+                                      int ldg, const float* ypre, int ldy, const float* lam, float cc, int channels,
+                                      float* state, const float* xconv, int ldx, int taps, float* tail,
+                                      float* out, int ldo) {
+    after_previous();
     const int seg = blockIdx.y, c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= channels) return;
     const int start = b.seg_start[seg], len = b.seg_len[seg], slot = b.seg_slot[seg];
@@ -92,8 +94,9 @@ __device__ __forceinline__ void rg_coeffs(float lr, float li, float uu, float sp
 }
 
 // thread = (tile, channel)
-__global__ void seq_rglru_tile_kernel(sllm_seq_batch b, const float* __restrict__ u, int ldu, const float* __restrict__ lr, const float* __restrict__ li,
-                                      int ldg, const float* __restrict__ lam, float cc, int channels, double* __restrict__ PQ) {
+__global__ void seq_rglru_tile_kernel(sllm_seq_batch b, const float* u, int ldu, const float* lr, const float* li,
+                                      int ldg, const float* lam, float cc, int channels, double* PQ) {
+    after_previous();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= channels) return;
     const RgTile tl = rg_tile(b, blockIdx.y);
@@ -111,8 +114,9 @@ __global__ void seq_rglru_tile_kernel(sllm_seq_batch b, const float* __restrict_
 }
 
 // thread = (segment, channel): the tiles of the segment in order; PQ[cid][0] becomes the tile's start state
-__global__ void seq_rglru_carry_kernel(sllm_seq_batch b, int channels, double* __restrict__ PQ, float* __restrict__ state, const float* __restrict__ xconv,
-                                       int ldx, int taps, float* __restrict__ tail) {
+__global__ void seq_rglru_carry_kernel(sllm_seq_batch b, int channels, double* PQ, float* state, const float* xconv,
+                                       int ldx, int taps, float* tail) {
+    after_previous();
     const int seg = blockIdx.y, c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= channels) return;
     const int start = b.seg_start[seg], len = b.seg_len[seg], slot = b.seg_slot[seg], cid0 = b.seg_tile0[seg];
@@ -138,9 +142,10 @@ __global__ void seq_rglru_carry_kernel(sllm_seq_batch b, int channels, double* _
 }
 
 // thread = (tile, channel): the tile again from its start state, outputs written
-__global__ void seq_rglru_emit_kernel(sllm_seq_batch b, const float* __restrict__ u, int ldu, const float* __restrict__ lr, const float* __restrict__ li,
-                                      int ldg, const float* __restrict__ ypre, int ldy, const float* __restrict__ lam, float cc, int channels,
-                                      const double* __restrict__ PQ, float* __restrict__ out, int ldo) {
+__global__ void seq_rglru_emit_kernel(sllm_seq_batch b, const float* u, int ldu, const float* lr, const float* li,
+                                      int ldg, const float* ypre, int ldy, const float* lam, float cc, int channels,
+                                      const double* PQ, float* out, int ldo) {
+    after_previous();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= channels) return;
     const RgTile tl = rg_tile(b, blockIdx.y);
@@ -163,10 +168,11 @@ __global__ void seq_rglru_emit_kernel(sllm_seq_batch b, const float* __restrict_
 // leaves the tile's (P = product of the decays per key channel, Q = its state) in `pbuf` / `qbuf`; seq_gla_carry_kernel turns Q into the
 // tile's start state; pass 2 redoes the tile from there and writes the outputs.
 template <int KP, int MODE>
-__global__ void __launch_bounds__(1024) seq_gla_scan_kernel(sllm_seq_batch b, const float* __restrict__ q, int ldq, const float* __restrict__ k, int ldk,
-                                                            const float* __restrict__ v, int ldv, const float* __restrict__ z, int ldz, int heads, int dk,
-                                                            int dv, float qscale, float inv_tau, float* __restrict__ state, float* __restrict__ o,
-                                                            int ldo, int chunk, float* __restrict__ pbuf, float* __restrict__ qbuf) {
+__global__ void __launch_bounds__(1024) seq_gla_scan_kernel(sllm_seq_batch b, const float* q, int ldq, const float* k, int ldk,
+                                                            const float* v, int ldv, const float* z, int ldz, int heads, int dk,
+                                                            int dv, float qscale, float inv_tau, float* state, float* o,
+                                                            int ldo, int chunk, float* pbuf, float* qbuf) {
+    after_previous();
     extern __shared__ float sm[];
     const int h = blockIdx.y;
     int seg, start, len, cid = 0;
@@ -248,8 +254,9 @@ __global__ void __launch_bounds__(1024) seq_gla_scan_kernel(sllm_seq_batch b, co
 }
 
 // thread = one element (key channel, value column) of one head's state of one segment: the segment's tiles in order, Q -> start state
-__global__ void seq_gla_carry_kernel(sllm_seq_batch b, int heads, int dk, int dv, const float* __restrict__ pbuf, float* __restrict__ qbuf,
-                                     float* __restrict__ state) {
+__global__ void seq_gla_carry_kernel(sllm_seq_batch b, int heads, int dk, int dv, const float* pbuf, float* qbuf,
+                                     float* state) {
+    after_previous();
     const int seg = blockIdx.z, h = blockIdx.y, e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= dk * dv) return;
     const int kr = e / dv;
@@ -285,7 +292,7 @@ int sllm_seq_conv(const sllm_seq_batch* b, const float* x, int32_t ldx, int32_t 
     SLLM_REQUIRE(x && w && u && channels > 0 && taps >= 1 && taps <= kMaxTaps, SLLM_EINVAL, "seq_conv: bad argument (1..%d taps)", kMaxTaps);
     SLLM_REQUIRE(taps == 1 || tail, SLLM_EINVAL, "seq_conv: a convolution over more than one tap needs the sequences' tails");
     SLLM_REQUIRE(b->T <= 65535, SLLM_ENOTSUP, "seq_conv: at most 65535 tokens per step");
-    seq_conv_kernel<<<dim3((channels + 127) / 128, b->T), 128, 0, as_stream(stream)>>>(*b, x, ldx, channels, taps, w, cb, tail, u, ldu);
+    overlapping(seq_conv_kernel)<<<dim3((channels + 127) / 128, b->T), 128, 0, as_stream(stream)>>>(*b, x, ldx, channels, taps, w, cb, tail, u, ldu);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;
@@ -300,14 +307,14 @@ int sllm_seq_rglru_scan(const sllm_seq_batch* b, const float* u, int32_t ldu, co
     if (scratch && b->n_qtiles > b->nseg && b->qt_seg && b->qt_off && b->seg_tile0) {   // some portion is longer than a tile: three passes
         double* PQ = reinterpret_cast<double*>(scratch);
         const dim3 tiles((channels + 127) / 128, b->n_qtiles), segs((channels + 127) / 128, b->nseg);
-        seq_rglru_tile_kernel<<<tiles, 128, 0, as_stream(stream)>>>(*b, u, ldu, lr, li, ldg, lam, c, channels, PQ);
-        seq_rglru_carry_kernel<<<segs, 128, 0, as_stream(stream)>>>(*b, channels, PQ, state, xconv, ldx, taps, tail);
-        seq_rglru_emit_kernel<<<tiles, 128, 0, as_stream(stream)>>>(*b, u, ldu, lr, li, ldg, ypre, ldy, lam, c, channels, PQ, out, ldo);
+        overlapping(seq_rglru_tile_kernel)<<<tiles, 128, 0, as_stream(stream)>>>(*b, u, ldu, lr, li, ldg, lam, c, channels, PQ);
+        overlapping(seq_rglru_carry_kernel)<<<segs, 128, 0, as_stream(stream)>>>(*b, channels, PQ, state, xconv, ldx, taps, tail);
+        overlapping(seq_rglru_emit_kernel)<<<tiles, 128, 0, as_stream(stream)>>>(*b, u, ldu, lr, li, ldg, ypre, ldy, lam, c, channels, PQ, out, ldo);
         g_launches += 3;
         SLLM_LAUNCH_CHECK();
         return SLLM_OK;
     }
-    seq_rglru_scan_kernel<<<dim3((channels + 63) / 64, b->nseg), 64, 0, as_stream(stream)>>>(*b, u, ldu, lr, li, ldg, ypre, ldy, lam, c, channels, state, xconv,
+    overlapping(seq_rglru_scan_kernel)<<<dim3((channels + 63) / 64, b->nseg), 64, 0, as_stream(stream)>>>(*b, u, ldu, lr, li, ldg, ypre, ldy, lam, c, channels, state, xconv,
                                                                                               ldx, taps, tail, out, ldo);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
@@ -339,16 +346,16 @@ if (smem > 48 * 1024) {
         float* pbuf = reinterpret_cast<float*>(scratch);
         float* qbuf = pbuf + (((size_t)b->n_qtiles * heads * dk + 63) / 64) * 64;
         const dim3 tiles(b->n_qtiles, heads);
-        seq_gla_scan_kernel<kp, 1><<<tiles, threads, smem, st>>>(*b, q, ldq, k, ldk, v, ldv, z, ldz, heads, dk, dv, qscale, 1.0f / tau, state, o, ldo, chunk,
+        overlapping(seq_gla_scan_kernel<kp, 1>)<<<tiles, threads, smem, st>>>(*b, q, ldq, k, ldk, v, ldv, z, ldz, heads, dk, dv, qscale, 1.0f / tau, state, o, ldo, chunk,
                                                                    pbuf, qbuf);
-        seq_gla_carry_kernel<<<dim3((dk * dv + 255) / 256, heads, b->nseg), 256, 0, st>>>(*b, heads, dk, dv, pbuf, qbuf, state);
-        seq_gla_scan_kernel<kp, 2><<<tiles, threads, smem, st>>>(*b, q, ldq, k, ldk, v, ldv, z, ldz, heads, dk, dv, qscale, 1.0f / tau, state, o, ldo, chunk,
+        overlapping(seq_gla_carry_kernel)<<<dim3((dk * dv + 255) / 256, heads, b->nseg), 256, 0, st>>>(*b, heads, dk, dv, pbuf, qbuf, state);
+        overlapping(seq_gla_scan_kernel<kp, 2>)<<<tiles, threads, smem, st>>>(*b, q, ldq, k, ldk, v, ldv, z, ldz, heads, dk, dv, qscale, 1.0f / tau, state, o, ldo, chunk,
                                                                    pbuf, qbuf);
         g_launches += 3;
         SLLM_LAUNCH_CHECK();
         return SLLM_OK;
     }
-    seq_gla_scan_kernel<kp, 0><<<grid, threads, smem, st>>>(*b, q, ldq, k, ldk, v, ldv, z, ldz, heads, dk, dv, qscale, 1.0f / tau, state, o, ldo, chunk,
+    overlapping(seq_gla_scan_kernel<kp, 0>)<<<grid, threads, smem, st>>>(*b, q, ldq, k, ldk, v, ldv, z, ldz, heads, dk, dv, qscale, 1.0f / tau, state, o, ldo, chunk,
                                                               nullptr, nullptr);
     ++g_launches;
     SLLM_LAUNCH_CHECK();

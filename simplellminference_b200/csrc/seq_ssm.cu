@@ -37,6 +37,7 @@ __device__ __forceinline__ size_t scan_range_id(const sllm_seq_batch& b, int seg
 // from zero, leaving its end state and its sum of dt in the workspace; MODE 2: a range from the start state the carry kernel left there.
 template <int R, int MODE>
 __global__ void __launch_bounds__(kScanLanes * kScanChannels) seq_selective_scan_kernel(ScanArgs p) {
+    after_previous();
     extern __shared__ __align__(16) float ssm_sm[];
     const sllm_seq_batch& b = p.b;
     const int seg = MODE == 0 ? blockIdx.x : blockIdx.x / p.nrange, rg = MODE == 0 ? 0 : blockIdx.x % p.nrange, c0 = blockIdx.y * kScanChannels;
@@ -141,6 +142,7 @@ __global__ void __launch_bounds__(kScanLanes * kScanChannels) seq_selective_scan
 // thread = one state element (channel c, state n) of one portion: its ranges in order, end state from zero -> start state; the last
 // start state, moved on over the last range, is the sequence's new state
 __global__ void seq_selective_scan_carry_kernel(ScanArgs p) {
+    after_previous();
     const sllm_seq_batch& b = p.b;
     const int seg = blockIdx.y;
     const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x, per = (size_t)p.inner * p.N;
@@ -172,7 +174,8 @@ __global__ void seq_selective_scan_carry_kernel(ScanArgs p) {
 }
 
 // ring[slot][p % (taps-1)][c] <- x[t][c] for the last taps-1 tokens of every portion (position p); grid (nseg, blocks of channels)
-__global__ void seq_ring_store_kernel(sllm_seq_batch b, const float* __restrict__ x, int ldx, int channels, int taps, float* __restrict__ ring) {
+__global__ void seq_ring_store_kernel(sllm_seq_batch b, const float* x, int ldx, int channels, int taps, float* ring) {
+    after_previous();
     const int seg = blockIdx.x;
     const int start = b.seg_start[seg], len = b.seg_len[seg], slot = b.seg_slot[seg], pos0 = b.seg_pos0[seg];
     const int keep = min(len, taps - 1);
@@ -209,12 +212,12 @@ int sllm_seq_selective_scan(const sllm_seq_batch* b, const float* x, int32_t ldx
     const int per_lane = (n_state + kScanLanes - 1) / kScanLanes;
 #define SLLM_SCAN_LAUNCH(MODE, GRID)                                                          \
     do {                                                                                      \
-        if (per_lane <= 1) seq_selective_scan_kernel<1, MODE><<<GRID, threads, smem, st>>>(p);       \
-        else if (per_lane <= 2) seq_selective_scan_kernel<2, MODE><<<GRID, threads, smem, st>>>(p);  \
-        else if (per_lane <= 4) seq_selective_scan_kernel<4, MODE><<<GRID, threads, smem, st>>>(p);  \
-        else if (per_lane <= 8) seq_selective_scan_kernel<8, MODE><<<GRID, threads, smem, st>>>(p);  \
-        else if (per_lane <= 16) seq_selective_scan_kernel<16, MODE><<<GRID, threads, smem, st>>>(p); \
-        else seq_selective_scan_kernel<32, MODE><<<GRID, threads, smem, st>>>(p);                    \
+        if (per_lane <= 1) overlapping(seq_selective_scan_kernel<1, MODE>)<<<GRID, threads, smem, st>>>(p);       \
+        else if (per_lane <= 2) overlapping(seq_selective_scan_kernel<2, MODE>)<<<GRID, threads, smem, st>>>(p);  \
+        else if (per_lane <= 4) overlapping(seq_selective_scan_kernel<4, MODE>)<<<GRID, threads, smem, st>>>(p);  \
+        else if (per_lane <= 8) overlapping(seq_selective_scan_kernel<8, MODE>)<<<GRID, threads, smem, st>>>(p);  \
+        else if (per_lane <= 16) overlapping(seq_selective_scan_kernel<16, MODE>)<<<GRID, threads, smem, st>>>(p); \
+        else overlapping(seq_selective_scan_kernel<32, MODE>)<<<GRID, threads, smem, st>>>(p);                    \
         ++g_launches;                                                                         \
         SLLM_LAUNCH_CHECK();                                                                  \
     } while (0)
@@ -223,7 +226,7 @@ int sllm_seq_selective_scan(const sllm_seq_batch* b, const float* x, int32_t ldx
         const dim3 grid(b->nseg * p.nrange, blocks);
         SLLM_SCAN_LAUNCH(1, grid);
         const size_t per = (size_t)inner * n_state;
-        seq_selective_scan_carry_kernel<<<dim3((unsigned)((per + 255) / 256), b->nseg), 256, 0, st>>>(p);
+        overlapping(seq_selective_scan_carry_kernel)<<<dim3((unsigned)((per + 255) / 256), b->nseg), 256, 0, st>>>(p);
         ++g_launches;
         SLLM_LAUNCH_CHECK();
         SLLM_SCAN_LAUNCH(2, grid);
@@ -240,7 +243,7 @@ int sllm_seq_ring_store(const sllm_seq_batch* b, const float* x, int32_t ldx, in
     SLLM_REQUIRE(x && channels > 0 && taps >= 1 && (taps == 1 || ring), SLLM_EINVAL, "seq_ring_store: bad argument");
     if (taps == 1) return SLLM_OK;
     const int blocks = std::max(1, std::min(64, ((taps - 1) * channels + 255) / 256));
-    seq_ring_store_kernel<<<dim3(b->nseg, blocks), 256, 0, as_stream(stream)>>>(*b, x, ldx, channels, taps, ring);
+    overlapping(seq_ring_store_kernel)<<<dim3(b->nseg, blocks), 256, 0, as_stream(stream)>>>(*b, x, ldx, channels, taps, ring);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;

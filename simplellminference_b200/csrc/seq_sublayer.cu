@@ -43,6 +43,7 @@ __device__ __forceinline__ bool seam_is_last(const sllm_seq_batch& b, int t, int
 }
 
 __global__ void seq_seam_kernel(SeamArgs p) {
+    after_previous();
     extern __shared__ __align__(16) float seam_sm[];   // [d] the row at hand, [d] the convolution's sums
     __shared__ float red[33];
     float* s_row = seam_sm;
@@ -116,6 +117,7 @@ __global__ void seq_seam_kernel(SeamArgs p) {
 // CTA = token, R groups of four channels per thread; x and y are read once, in flight together, and everything is stored once.
 template <int R>
 __global__ void __launch_bounds__(1024) seq_seam_row_kernel(SeamArgs p) {
+    after_previous();
     __shared__ float red[33];
     const int d4 = p.d / 4;
     const size_t r = (size_t)blockIdx.x * p.d;
@@ -180,7 +182,8 @@ __global__ void __launch_bounds__(1024) seq_seam_row_kernel(SeamArgs p) {
 // (1) one CTA per token: the residual sum and the scale of the next norm, scale[t] = g_pre / rms(x_new[t]);
 // (2) element-wise over (token, channel): h = n + conv(n) with n = scale * x_new read from the step's rows (complete after launch 1) or
 //     the ring, the stash and the flush as in the one-launch form.
-__global__ void seq_seam_sum_kernel(SeamArgs p, float* __restrict__ scale) {
+__global__ void seq_seam_sum_kernel(SeamArgs p, float* scale) {
+    after_previous();
     extern __shared__ __align__(16) float seam_sm[];   // [d] the sublayer's output row
     __shared__ float red[33];
     const int t = blockIdx.x, d = p.d;
@@ -210,7 +213,8 @@ constexpr int kSeamMaxTaps = 64;
 
 // The rows a token's convolution reads are found once per CTA (the step's own rows with their scales, or ring rows), then the channels
 // are walked four at a time with 16-byte loads where the row length allows.
-__global__ void seq_seam_conv_kernel(SeamArgs p, const float* __restrict__ scale, int vec) {
+__global__ void seq_seam_conv_kernel(SeamArgs p, const float* scale, int vec) {
+    after_previous();
     __shared__ const float* s_src[kSeamMaxTaps];   // [back] row that lies `back` positions before the token, NULL = before the sequence's start
     __shared__ float s_mul[kSeamMaxTaps];
     __shared__ bool back_is_step[kSeamMaxTaps];    // the row is one of this step's (not yet normed) rather than a ring row
@@ -303,6 +307,7 @@ struct BranchSeamArgs {
 
 template <int E, int R>
 __global__ void __launch_bounds__(E * R <= 8 ? 1024 : 512) seq_branch_seam_kernel(BranchSeamArgs p) {
+    after_previous();
     __shared__ float s_part[kMaxBranches][33];
     __shared__ float red[33];
     const int groups = p.d / E, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
@@ -422,7 +427,7 @@ extern "C" int sllm_seq_branch_seam(const float* x_in, float* x_out, int32_t n, 
     const int per = (items + cta - 1) / cta;
     SLLM_REQUIRE(per <= (vec ? 8 : 32), SLLM_ENOTSUP, "seq_branch_seam: rows of %d floats", d);
     cudaStream_t st = as_stream(stream);
-#define SLLM_BRANCH_LAUNCH(E, R) seq_branch_seam_kernel<E, R><<<T, cta, 0, st>>>(p)
+#define SLLM_BRANCH_LAUNCH(E, R) overlapping(seq_branch_seam_kernel<E, R>)<<<T, cta, 0, st>>>(p)
     if (vec) {
         if (per == 1) SLLM_BRANCH_LAUNCH(4, 1);
         else if (per == 2) SLLM_BRANCH_LAUNCH(4, 2);
@@ -457,24 +462,24 @@ extern "C" int sllm_seq_seam(const sllm_seq_batch* b, const float* x_in, float* 
         aligned(post_w)) {
         // many tokens: CTAs of 256 threads with up to four groups of channels each; few: a thread per group of channels
         const int d4 = d / 4, cta = std::min(1024, (((b->T >= 64 ? std::max(std::min(d4, 256), (d4 + 3) / 4) : d4) + 31) / 32) * 32), per = (d4 + cta - 1) / cta;
-        if (per == 1) seq_seam_row_kernel<1><<<b->T, cta, 0, as_stream(stream)>>>(p);
-        else if (per == 2) seq_seam_row_kernel<2><<<b->T, cta, 0, as_stream(stream)>>>(p);
-        else seq_seam_row_kernel<4><<<b->T, cta, 0, as_stream(stream)>>>(p);
+        if (per == 1) overlapping(seq_seam_row_kernel<1>)<<<b->T, cta, 0, as_stream(stream)>>>(p);
+        else if (per == 2) overlapping(seq_seam_row_kernel<2>)<<<b->T, cta, 0, as_stream(stream)>>>(p);
+        else overlapping(seq_seam_row_kernel<4>)<<<b->T, cta, 0, as_stream(stream)>>>(p);
         ++g_launches;
         SLLM_LAUNCH_CHECK();
         return SLLM_OK;
     }
     const int threads = b->T >= 64 ? (d >= 2048 ? 256 : 128) : std::min(1024, std::max(128, (d + 31) / 32 * 32));
     if (scales && has_pre && conv_w && b->T >= 64 && b->T <= 65535) {       // many tokens: two launches, every row normed once
-        seq_seam_sum_kernel<<<b->T, threads, smem / 2, as_stream(stream)>>>(p, scales);
+        overlapping(seq_seam_sum_kernel)<<<b->T, threads, smem / 2, as_stream(stream)>>>(p, scales);
         const int vec = d % 4 == 0 && aligned(x_in) && aligned(x_out) && aligned(ring) && aligned(h) && aligned(stash) && aligned(flush_ring) &&
                         (h16 == nullptr || ((uintptr_t)h16 % 8) == 0);
-        seq_seam_conv_kernel<<<dim3(b->T, std::max(1, std::min(4, d / 4096))), 256, 0, as_stream(stream)>>>(p, scales, vec);
+        overlapping(seq_seam_conv_kernel)<<<dim3(b->T, std::max(1, std::min(4, d / 4096))), 256, 0, as_stream(stream)>>>(p, scales, vec);
         g_launches += 2;
         SLLM_LAUNCH_CHECK();
         return SLLM_OK;
     }
-    seq_seam_kernel<<<b->T, threads, smem, as_stream(stream)>>>(p);
+    overlapping(seq_seam_kernel)<<<b->T, threads, smem, as_stream(stream)>>>(p);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;

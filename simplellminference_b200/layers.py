@@ -92,11 +92,12 @@ class FusedLinear:
     def __call__(self, step, a_ptr, lda, c_ptr, ldc, alpha=1.0, accumulate=False, a16_ready=False, a16=None):
         """``a16``: dense bf16 rows [T][K] of the input that the caller keeps (only where ``takes_rows16`` says so; the fp32 rows are not read)."""
         if a16 is not None:
-            self.ops.linear(a16.data_ptr(), self.K, self.w, self.K, self.bias, c_ptr, ldc, step.T, self.N, self.K, step.st, accumulate=accumulate, scratch=a16, a16_ready=True)
+            self.ops.linear(a16.data_ptr(), self.K, self.w, self.K, self.bias, c_ptr, ldc, step.T, self.N, self.K, step.st, accumulate=accumulate, scratch=a16, a16_ready=True,
+                            w_fixed=True)
             return
         scratch = step.gemm_scratch(self.K, self.N)
         self.ops.linear(a_ptr, lda, self.w, self.K, self.bias, c_ptr, ldc, step.T, self.N, self.K, step.st, alpha=alpha, accumulate=accumulate,
-                        scratch=scratch, a16_ready=a16_ready and scratch is not None)
+                        scratch=scratch, a16_ready=a16_ready and scratch is not None, w_fixed=True)
 
     def takes_rows16(self, step) -> bool:
         """Whether this step's product runs on the tensor cores and can read bf16 rows kept by the caller (``a16``)."""
@@ -242,12 +243,12 @@ class LatentAttention:
         qa = step.scratch("latent_q", T * H * wide)
         ops.latent_kv(step.b, q, ldq, H, dn, dr, low, ld, R, self.norm_w, self.eps, self.freq, c.rot.dims // 2, qa, H * wide, state["row"], step.st,
                       magnitude=self.magnitude)
-        ops.linear(q, ldq, self.uk_t, dn, None, qa.data_ptr(), H * wide, T, R, dn, step.st, batch=H, a_bs=dn + dr, w_bs=R * dn, c_bs=wide)
+        ops.linear(q, ldq, self.uk_t, dn, None, qa.data_ptr(), H * wide, T, R, dn, step.st, batch=H, a_bs=dn + dr, w_bs=R * dn, c_bs=wide, w_fixed=True)
         ws = step.scratch("attn_ws", T * H * step.nsplit * (R + 2))
         ops.attention(step.b, qa.data_ptr(), H * wide, H, 1, wide, R, c.scale, state["row"], None, step.nsplit, ws, step.st, opts=self.opts)
         mixed = step.scratch("latent_o", T * H * R)
         ops.attention_finish(step.b, ws, step.nsplit, H, R, None, 0, g, ld, mixed, H * R, step.st, sink=self.sink)
-        ops.linear(mixed.data_ptr(), H * R, self.uv, R, None, out.data_ptr(), self.width, T, dv, R, step.st, batch=H, a_bs=R, w_bs=dv * R, c_bs=dv)
+        ops.linear(mixed.data_ptr(), H * R, self.uv, R, None, out.data_ptr(), self.width, T, dv, R, step.st, batch=H, a_bs=R, w_bs=dv * R, c_bs=dv, w_fixed=True)
 
 
 class GatedLinearRecurrence:
@@ -284,7 +285,7 @@ class GatedLinearRecurrence:
         bs = W // c.blocks
         for which in range(2):   # block-diagonal products: one launch per gate, the blocks as its batch
             ops.linear(u.data_ptr(), W, self.gates_w[which], bs, self.gates_b[which], gates.data_ptr() + which * T * W * F32B, W, T, bs, bs, step.st,
-                       batch=c.blocks, a_bs=bs, w_bs=bs * bs, bias_bs=bs, c_bs=bs)
+                       batch=c.blocks, a_bs=bs, w_bs=bs * bs, bias_bs=bs, c_bs=bs, w_fixed=True)
         tiles = step.b.n_qtiles
         scan_ws = step.scratch("rg_tiles", 4 * tiles * W) if tiles > step.nseg else None      # (P, Q) per tile and channel, doubles
         ops.rglru_scan(step.b, u, W, gates.data_ptr(), gates.data_ptr() + T * W * F32B, W, y, ld, self.lam, self.decay_scale, W, state["S"],

@@ -296,7 +296,7 @@ class SequenceEngine:
             entry = self._graphs[key]
             if entry is None:                               # second step of this kind: capture it (a capture does not execute)
                 meta_addr = self._meta_dev.data_ptr()
-                g = torch.cuda.CUDAGraph()
+                g = torch.cuda.CUDAGraph(keep_graph=True)
                 collecting = gc.isenabled()
                 gc.disable()        # a finaliser that frees device memory (another engine's graphs, say) must not run inside the capture
                 try:
@@ -306,6 +306,8 @@ class SequenceEngine:
                 finally:
                     if collecting:
                         gc.enable()
+                self.ops.overlap(g.raw_cuda_graph())
+                g.instantiate()
                 entry = self._graphs[key] = (g, out, meta_addr, p[0], p[9])
             g, logits, meta_addr, ids_addr, rows_addr = entry
             if meta_addr != self._meta_dev.data_ptr() or ids_addr != p[0] or rows_addr != p[9]:

@@ -26,6 +26,7 @@ class Ops:
         self.lib = _lib.load_seq(build=build)
         self.w_dtype = w_dtype
         self.round_a = 1 if w_dtype == BF16 else 0
+        self.round_a_fixed = self.round_a | _lib.SEQ_W_FIXED
         self.kv_dtype = BF16 if w_dtype == BF16 else F32
         self.tensor_cores = w_dtype == BF16
         self.launches = 0
@@ -34,6 +35,13 @@ class Ops:
         self.launches += 1
         if rc != 0:
             raise _lib.SllmError(rc, self.lib.sllm_last_error().decode(errors="replace"))
+
+    def overlap(self, graph: int) -> int:
+        """Lets kernels of a captured graph (``raw_cuda_graph()``, not instantiated yet) start while the one in front of them ends; how many edges that is."""
+        n = C.c_int32()
+        if self.lib.sllm_graph_overlap(graph, C.byref(n)) != 0:
+            raise _lib.SllmError(_lib.ESTATE, self.lib.sllm_last_error().decode(errors="replace"))
+        return n.value
 
     # ---- rows ----
     def embed(self, ids, table, vocab, d, streams, out, T, st, scale=1.0):
@@ -62,11 +70,12 @@ class Ops:
         self._ck(self.lib.sllm_seq_hyper_write_read(_p(x), streams, T, d, _p(mix), _p(outc), _p(y_in), _p(coef), _p(norm_w), groups, eps, _p(y_out), st))
 
     def linear(self, a_ptr, lda, w, ldw, bias, c_ptr, ldc, T, N, K, st, alpha=1.0, accumulate=False, batch=1, a_bs=0, w_bs=0, bias_bs=0,
-               c_bs=0, scratch=None, a16_ready=False, rows_dev=None, w_ptr=None):
+               c_bs=0, scratch=None, a16_ready=False, rows_dev=None, w_ptr=None, w_fixed=False):
         """``w_ptr``: an address inside ``w`` to use instead of its start (one matrix of several stored back to back);
-        ``rows_dev``: device address of a row count, rows beyond it are skipped."""
+        ``rows_dev``: device address of a row count, rows beyond it are skipped; ``w_fixed``: no kernel of the same captured step writes ``w``, so that in a
+        step whose kernels overlap (``overlap``) its rows may be read before the kernel in front has completed."""
         self._ck(self.lib.sllm_seq_linear(a_ptr, lda, _p(w) if w_ptr is None else w_ptr, self.w_dtype, ldw, _p(bias), c_ptr, ldc, T, N, K, alpha, int(accumulate),
-                                          self.round_a, batch, a_bs, w_bs, bias_bs, c_bs,
+                                          self.round_a_fixed if w_fixed else self.round_a, batch, a_bs, w_bs, bias_bs, c_bs,
                                           (scratch if isinstance(scratch, int) else _p(scratch)) if self.tensor_cores else None, int(a16_ready), rows_dev, st))
 
     def linear_grouped(self, a_ptr, a_bf16, w, c_ptr, counts_ptr, groups, cap, rows_hint, N, K, st):

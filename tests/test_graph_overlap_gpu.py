@@ -1,0 +1,84 @@
+"""Captured steps whose kernels become resident while the one in front still runs (sllm_graph_overlap): the same kernels on the same inputs, so the same bits
+as launches one behind the other; weights that the graph itself writes; joins, other libraries' kernels and copies keep their edges."""
+import os
+import sys
+
+import numpy as np
+import pytest
+
+sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
+import nelutar_testlib as L  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("requests", [1, 3])
+def test_captured_steps_equal_direct_ones(tmp_path, dtype, requests):
+    from simplellminference_b200.models import build_model
+    from simplellminference_b200.seqengine import SequenceEngine
+    cfg = L.make_config([L.lightning_pair(), L.delta_pair(mlp=L.moe()), L.retention_layer(mlp=L.moe(experts=6, top=2, groups=3, keep=1))])
+    w = L.random_weights(cfg, seed=3)
+    rng = np.random.default_rng(4)
+    reqs = [rng.integers(0, cfg["vocab"], size=20 + 7 * i).tolist() for i in range(requests)]
+    got = []
+    for graphs in (True, False):
+        model = build_model(L.write_model(str(tmp_path / f"m{graphs}"), cfg, w), dtype, "cuda")
+        edges, plain = [], model.ops.overlap
+        model.ops.overlap = lambda g: edges.append(plain(g))
+        eng = SequenceEngine(model, max_tokens=256, max_seqs=4, page_len=32, graphs=graphs)
+        slots = [eng.admit() for _ in reqs]
+        rows = [eng.run([(s, r[:10], [9])]).clone() for s, r in zip(slots, reqs)]
+        for k in range(10, 20):
+            rows.append(eng.run([(s, [r[k]], [0]) for s, r in zip(slots, reqs)]).clone())
+        got.append(rows)
+        assert bool(edges) == graphs == bool(eng.graph_replays) and all(e >= 10 for e in edges), (edges, eng.graph_replays)
+    for a, b in zip(*got):
+        assert (a == b).all()
+
+
+def test_weights_written_by_the_graph_itself():
+    import torch
+    from simplellminference_b200.config import F32
+    from simplellminference_b200.seqops import Ops
+    ops = Ops(F32)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    K, N = 2048, 1024
+    a, w1 = torch.randn(1, K, generator=g, device="cuda"), torch.randn(8, K, K, generator=g, device="cuda")
+    mid, out, far = torch.zeros(N, K, device="cuda"), torch.zeros(1, N, device="cuda"), torch.zeros(1, N, device="cuda")
+
+    def step(st):
+        for i in range(8):       # K outputs each: rows of the matrix that the next kernels multiply by
+            ops.linear(a.data_ptr(), K, w1[i], K, None, mid[i].data_ptr(), K, 1, K, K, st, w_fixed=True)
+        ops.linear(a.data_ptr(), K, mid, K, None, out.data_ptr(), N, 1, N, K, st)
+        far.copy_(out)           # a copy between two of them
+        ops.linear(a.data_ptr(), K, mid, K, None, out.data_ptr(), N, 1, N, K, st, accumulate=True)
+
+    step(torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    want = out.clone()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        step(torch.cuda.current_stream().cuda_stream)
+    assert ops.overlap(graph.raw_cuda_graph()) == 8      # not the first, not the one behind the copy
+    assert ops.overlap(graph.raw_cuda_graph()) == 0
+    graph.instantiate()
+    for seed in (2, 3):
+        g.manual_seed(seed)
+        a.copy_(torch.randn(1, K, generator=g, device="cuda"))
+        mid.fill_(float("nan"))
+        mid[8:] = 1.0
+        graph.replay()
+        torch.cuda.synchronize()
+        have = out.clone()
+        step(torch.cuda.current_stream().cuda_stream)
+        assert torch.equal(have, out) and torch.equal(far * 2, out) and not torch.equal(have, want)
+
+
+def test_no_graph_is_refused():
+    from simplellminference_b200.config import F32
+    from simplellminference_b200.seqops import Ops
+    from simplellminference_b200._lib import SllmError
+    with pytest.raises(SllmError):
+        Ops(F32).overlap(0)
