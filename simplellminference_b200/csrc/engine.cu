@@ -105,6 +105,7 @@ struct sllm_engine {
     int cls_grid = 0;
     // pinned host staging
     int32_t* h_state = nullptr;   // 8 ints
+    float* h_logits = nullptr;    // [V_loc], pinned: a forward()'s logits on their way to the caller
     // graph
     cudaGraphExec_t graph_exec = nullptr;
     int step_launches = 0;
@@ -496,7 +497,7 @@ static int build_graph(sllm_engine* e) {
 }
 
 // *done = steps actually enqueued (the host shadow of the position must follow the device, also when a launch fails half way)
-static int enqueue_steps(sllm_engine* e, int n, int host_pos, int* done) {
+static int enqueue_steps(sllm_engine* e, int n, int host_pos, int* done, const MegaCall& call = MegaCall()) {
     *done = 0;
     SLLM_REQUIRE(e->weights_loaded, SLLM_ESTATE, "weights not loaded");
     if (!e->fused) {
@@ -508,10 +509,13 @@ static int enqueue_steps(sllm_engine* e, int n, int host_pos, int* done) {
     }
     if (e->mega) {
         SLLM_REQUIRE(!e->mega_ll || e->ll_ready, SLLM_ESTATE, "tensor-parallel megakernel: peer areas not exchanged yet (sllm_engine_p2p_import)");
+        MegaParams p = e->mega_params;
+        Mega2Params P = e->mega2_params;
+        p.call = P.m.call = call;
         for (int i = 0; i < n; ++i) {
             const int rc = e->mega_ll ? mega_ll_launch(e->ll_params, e->H_loc / e->KVH_loc, e->ll_plan.grid, e->ll_plan.smem, e->stream)
-                           : e->mega2 ? mega2_launch(e->mega2_params, e->H_loc / e->KVH_loc, e->mega_plan_.grid, e->mega_plan_.smem, e->stream, e->mega_fuse)
-                                      : mega_launch(e->mega_params, e->H_loc / e->KVH_loc, e->mega_plan_.grid, e->mega_plan_.smem, e->stream, e->mega_fuse);
+                           : e->mega2 ? mega2_launch(P, e->H_loc / e->KVH_loc, e->mega_plan_.grid, e->mega_plan_.smem, e->stream, e->mega_fuse)
+                                      : mega_launch(p, e->H_loc / e->KVH_loc, e->mega_plan_.grid, e->mega_plan_.smem, e->stream, e->mega_fuse);
             if (rc) return rc;
             e->total_launches++;
             ++*done;
@@ -831,6 +835,7 @@ int sllm_engine_create(const sllm_engine_config* cfg, sllm_stream_t stream, sllm
     // zero everything that is read before it is written: KV cache, workspaces, state
     cudaError_t ce = cudaMemsetAsync(e->key_cache, 0, e->arena + e->arena_used - reinterpret_cast<uint8_t*>(e->key_cache), e->stream);
     if (ce == cudaSuccess) ce = cudaMallocHost(reinterpret_cast<void**>(&e->h_state), 64);
+    if (ce == cudaSuccess && e->mega && !e->mega_ll) ce = cudaMallocHost(reinterpret_cast<void**>(&e->h_logits), sizeof(float) * (size_t)e->V_loc);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->stream);
     if (ce != cudaSuccess) { cuda_fail(ce, "engine init", __FILE__, __LINE__); sllm_engine_destroy(e); return (int)ce; }
     *out = e;
@@ -842,6 +847,7 @@ void sllm_engine_destroy(sllm_engine* e) {
     if (e->graph_exec) cudaGraphExecDestroy(e->graph_exec);
     if (e->comm) ncclCommDestroy(e->comm);
     if (e->h_state) cudaFreeHost(e->h_state);
+    if (e->h_logits) cudaFreeHost(e->h_logits);
     for (int r = 0; r < kMaxTp; ++r) if (e->p2p_peer[r]) cudaIpcCloseMemHandle(e->p2p_peer[r]);
     if (e->p2p_dev) cudaFree(e->p2p_dev);
     if (e->p2p_block) cudaFree(e->p2p_block);
@@ -1022,10 +1028,29 @@ int sllm_engine_read_tokens(sllm_engine* e, int32_t* out, int32_t n) {
 int sllm_engine_forward(sllm_engine* e, int32_t token, int32_t pos, float* logits_host, int32_t* next_token_host) {
     SLLM_REQUIRE(e, SLLM_EINVAL, "null engine");
     SLLM_REQUIRE(e->tp == 1 || e->comm || e->p2p_ready, SLLM_ESTATE, "tensor-parallel engine without a communicator");
-    // host -> device: token and position travel through pinned memory like any other input
-    e->h_state[0] = token; e->h_state[1] = pos; e->h_state[2] = 0; e->h_state[3] = 0;
     SLLM_REQUIRE(pos >= 0 && pos < e->S, SLLM_EINVAL, "position %d outside [0, %d)", pos, e->S);
     SLLM_REQUIRE(token >= 0 && token < e->V, SLLM_EINVAL, "Token index %d is outside the vocabulary [0, %d).", token, e->V);
+    if (e->fused && e->mega && !e->mega_ll) {
+        // What was around the kernel cost more than the bytes it moved (stories110M, fp32, position 200, us a call: 408): a copy of 16 bytes in front (the launch carries
+        // token and position now), the next token's copy behind (the kernel leaves it in pinned memory, with the reduction behind it 386 -> 370 without logits), the
+        // logits staged into pageable memory by the driver (390; into pinned memory and from there to the caller 385; stored by the kernel itself, 8 bytes a
+        // thread over PCIe, 410).
+        MegaCall call;
+        call.token = token;
+        call.pos = pos;
+        call.next = next_token_host ? e->h_state + 4 : nullptr;
+        e->h_state[7] = pos;
+        int done = 0;
+        if (int rc = enqueue_steps(e, 1, pos, &done, call)) return rc;
+        e->h_state[7] = pos + 1;
+        if (logits_host) SLLM_CUDA(cudaMemcpyAsync(e->h_logits, e->logits, sizeof(float) * (size_t)e->V_loc, cudaMemcpyDeviceToHost, e->stream));
+        SLLM_WAIT(e->stream);
+        if (logits_host) std::memcpy(logits_host, e->h_logits, sizeof(float) * (size_t)e->V_loc);
+        if (next_token_host) *next_token_host = e->h_state[4];
+        return SLLM_OK;
+    }
+    // host -> device: token and position travel through pinned memory like any other input
+    e->h_state[0] = token; e->h_state[1] = pos; e->h_state[2] = 0; e->h_state[3] = 0;
     SLLM_CUDA(cudaMemcpyAsync(e->state, e->h_state, 16, cudaMemcpyHostToDevice, e->stream));
     e->h_state[7] = pos;
     int done = 0;

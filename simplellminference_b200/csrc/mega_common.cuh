@@ -162,11 +162,99 @@ __device__ __forceinline__ void phase_tiles(const PhaseDesc& ph, int cta, int nc
     }
 }
 
+// The CTA's share of a phase ([first, last) tile rows; for PH_WO_T of its item), worked out once per launch and kept where the descriptor's table pointer was: from
+// the table, an L2 round trip, or by 64-bit divisions it stood on the path of every producer that came to a new phase, as good as every tile of a small model.
+__device__ __forceinline__ const uint32_t* pack_share(int first, int last) {
+    return reinterpret_cast<const uint32_t*>((uint64_t)(uint32_t)first | ((uint64_t)(uint32_t)last << 32));
+}
+__device__ __forceinline__ void share_of(const PhaseDesc& ph, int& first, int& last) {
+    const uint64_t v = reinterpret_cast<uint64_t>(ph.cum);
+    first = (int)(uint32_t)v;
+    last = (int)(uint32_t)(v >> 32);
+}
+template <bool FUSE>
+__device__ __forceinline__ void keep_share(PhaseDesc& ph, int cta, int ncta, int nsplit) {
+    int first, last;
+    if (ph.kind == PH_WO_T) {
+        const int part = cta % nsplit;
+        first = (int)(((int64_t)ph.ntr * part) / nsplit);
+        last = (int)(((int64_t)ph.ntr * (part + 1)) / nsplit);
+    } else {
+        phase_tiles<FUSE>(ph, cta, ncta, first, last);
+    }
+    ph.cum = pack_share(first, last);
+}
+
 // tile rows [a, b) of the transposed down matrix that row group rg of RG takes out of a CTA's [g0, g1): contiguous shares
 __device__ __forceinline__ void down_t_rows(int g0, int g1, int rg, int RG, int& a, int& b) {
     const int cnt = g1 - g0;
     a = g0 + (cnt * rg) / RG;
     b = g0 + (cnt * (rg + 1)) / RG;
+}
+
+// Attention output of `heads` heads from h0 on, their splits' partial records merged, into xs. A thread takes every ngrp-th split of one 16-byte piece, so that all records
+// are asked for at once; the splits' maxima and sums travel beside them. (Two dependent loops over the splits in every thread took 2.5 us for the 12 of
+// stories110M, of a layer's 28.) wgt: the partial table, idle here; xs_bytes: what lies behind xs.
+__device__ __forceinline__ void merge_splits(const MegaParams& p, int h0, int heads, float* xs, size_t xs_bytes, float* wgt) {
+    const int tid = threadIdx.x, rec = p.hd + kAttRecPad, n = heads * p.nsplit, width = heads * p.hd, nc = width / 4;
+    const float* base = p.att_part + (size_t)h0 * p.nsplit * rec;
+    const int ngrp = max(1, min(min(kMegaThreads / nc, p.nsplit), (int)(xs_bytes / ((size_t)width * 4)) - 1));
+    const int grp = ngrp > 1 ? tid / nc : 0, per = ngrp > 1 ? nc : kMegaThreads;
+    float* share = xs + width;                  // [ngrp][nc] pieces
+    float* sums = wgt + (2 * n + 3) / 4 * 4;    // [ngrp][nc] their shares of the sums of weights
+    const int c0 = tid - grp * nc;
+    const bool takes = grp < ngrp && c0 < nc;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto piece = [&](int c4, int s) {
+        const int h = c4 * 4 / p.hd;
+        return __ldcg(reinterpret_cast<const float4*>(base + ((size_t)h * p.nsplit + s) * rec + (c4 * 4 - h * p.hd)));
+    };
+    if (takes) v = piece(c0, grp);
+    for (int i = tid; i < n; i += kMegaThreads) {
+        wgt[2 * i] = __ldcg(base + (size_t)i * rec + p.hd);
+        wgt[2 * i + 1] = __ldcg(base + (size_t)i * rec + p.hd + 1);
+    }
+    __syncthreads();
+    if (takes) {
+        for (int c4 = c0; c4 < nc; c4 += per) {
+            const float* ml = wgt + 2 * (c4 * 4 / p.hd) * p.nsplit;
+            float M = -INFINITY, Ls = 0.f;
+            for (int s = 0; s < p.nsplit; ++s) M = fmaxf(M, ml[2 * s]);
+            float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+            for (int s = grp; s < p.nsplit; s += ngrp) {
+                if (s != grp || c4 != c0) v = piece(c4, s);
+                const float w = (ml[2 * s] == -INFINITY) ? 0.f : expf(ml[2 * s] - M);
+                o.x = fmaf(v.x, w, o.x); o.y = fmaf(v.y, w, o.y); o.z = fmaf(v.z, w, o.z); o.w = fmaf(v.w, w, o.w);
+                Ls = fmaf(ml[2 * s + 1], w, Ls);
+            }
+            if (ngrp == 1) {
+                reinterpret_cast<float4*>(xs)[c4] = make_float4(o.x / Ls, o.y / Ls, o.z / Ls, o.w / Ls);
+            } else {
+                reinterpret_cast<float4*>(share)[grp * nc + c4] = o;
+                sums[grp * nc + c4] = Ls;
+            }
+        }
+    }
+    if (ngrp == 1) return;                      // callers synchronise
+    __syncthreads();
+    if (tid < nc) {
+        float4 o = reinterpret_cast<const float4*>(share)[tid];
+        float Ls = sums[tid];
+        for (int g = 1; g < ngrp; ++g) {
+            const float4 q = reinterpret_cast<const float4*>(share)[g * nc + tid];
+            o.x += q.x; o.y += q.y; o.z += q.z; o.w += q.w;
+            Ls += sums[g * nc + tid];
+        }
+        reinterpret_cast<float4*>(xs)[tid] = make_float4(o.x / Ls, o.y / Ls, o.z / Ls, o.w / Ls);
+    }
+}
+
+// Norm weights of this layer's second half and of the next layer, asked into L2 while it is early: a phase needs them right behind a barrier.
+__device__ __forceinline__ void prefetch_norms(const MegaParams& p, int l, int cta, int ncta) {
+    const int lines = (p.d * 8 + 127) / 128;
+    for (int i = cta + threadIdx.x * ncta; i < lines; i += ncta * kMegaThreads)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t*>(p.norms + (size_t)(2 * l + 1) * p.d) + min(i * 128, p.d * 8 - 4)));
 }
 
 // ---- L2 prefetch of the weight stream: built twice, measured, removed ------------------------------------------------------
@@ -233,6 +321,55 @@ __device__ __forceinline__ float reg_dot(const uint4 w, const float* x, float ac
 }
 
 
+// The larger logit, the smaller index among equals (candidates are never NaN).
+__device__ __forceinline__ void take_better(float& v, int& i, float ov, int oi) {
+    if (ov > v || (ov == v && oi < i)) { v = ov; i = oi; }
+}
+__device__ __forceinline__ void warp_better(float& v, int& i) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) take_better(v, i, __shfl_xor_sync(0xffffffffu, v, o), __shfl_xor_sync(0xffffffffu, i, o));
+}
+// (v, i) of every thread -> the CTA's best in all threads of warp 0; red: 2 * kMegaWarps words of shared memory
+__device__ __forceinline__ void cta_better(float& v, int& i, float* red) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int* ri = reinterpret_cast<int*>(red + kMegaWarps);
+    warp_better(v, i);
+    if (lane == 0) { red[warp] = v; ri[warp] = i; }
+    __syncthreads();
+    if (warp == 0) {
+        v = lane < kMegaWarps ? red[lane] : -INFINITY;
+        i = lane < kMegaWarps ? ri[lane] : 0x7fffffff;
+        warp_better(v, i);
+    }
+}
+// End of the classifier phase: every CTA leaves its best logit, the CTA that comes last picks the arg max and advances the step state. True in the one thread that has
+// done so (it stores the counters that its kernel keeps). All threads of the last CTA read the candidates: by one thread, a chain of 148 reads of L2, that end took
+// several us.
+__device__ __forceinline__ bool mega_finish(const MegaParams& p, float v, int i, float* red, int* s_last, int cta, int ncta) {
+    cta_better(v, i, red);
+    if (threadIdx.x == 0) {
+        p.blk_val[cta] = v;
+        p.blk_idx[cta] = i;
+        __threadfence();
+        *s_last = (atomicAdd(&p.st->ticket, 1) == ncta - 1);
+        __threadfence();
+    }
+    __syncthreads();
+    if (!*s_last) return false;
+    v = -INFINITY;
+    i = 0x7fffffff;
+    for (int b = threadIdx.x; b < ncta; b += kMegaThreads) take_better(v, i, __ldcg(p.blk_val + b), __ldcg(p.blk_idx + b));
+    cta_better(v, i, red);
+    if (threadIdx.x != 0) return false;
+    if (i == 0x7fffffff) i = 0;
+    p.blk_val[ncta] = v;
+    p.blk_idx[ncta] = i;
+    p.st->ticket = 0;
+    if (p.call.token >= 0) { p.st->pos = p.call.pos; p.st->n_prompt = 0; }
+    if (p.call.next) *p.call.next = i;
+    ClsPolicy<SLLM_F32>::step_feedback(p.st, p.prompt, p.history, i);
+    return true;
+}
 static __device__ __noinline__ void mega_timeout(const char* what) {
     printf("sllm mega: %s timed out (cta %d warp %d)\n", what, (int)blockIdx.x, (int)(threadIdx.x >> 5));
     __trap();

@@ -44,13 +44,7 @@ __device__ __forceinline__ unsigned long long gtime() {
         if (p.trace && threadIdx.x == 0 && (ev) < kTraceEvents) p.trace[((size_t)blockIdx.x * kTraceEvents + (ev)) * 8 + (slot)] = gtime(); \
     } while (0)
 
-// producer state of one warp (meaningful in lane 0): constants of the phase it is currently feeding
-struct ProdState {
-    int wp, j;                 // phase and next slot index (j < 0: phase not entered yet)
-    unsigned count;            // slots issued so far
-    const uint8_t* W;          // phase matrix + this warp's column offset
-    int row_bytes, sbytes, u0, u1, upp, RG, nslots, kind;
-};
+constexpr int kPhaseCache = 56;   // as many as fit beside the largest plan (8 query heads per kv head of 256)
 
 // FUSE (experimental, SLLM_ENGINE_MEGA_FUSE_DOWN): the down projection runs inside the gate_up phase's CTA as a K-split over the
 // values that CTA produced (megakernel.cuh "PH_DOWN_T"): four grid barriers per layer instead of five, no staging of swi.
@@ -70,11 +64,27 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega_step_kernel(const MegaPa
     uint8_t* ring = smem + SL.ring;
     float* xs = reinterpret_cast<float*>(smem + SL.att_k);    // activation staging: aliases the (idle) K/V stages
     __shared__ int s_last;
+    // the phase descriptors with this CTA's shares (deeper models read the rest from global memory, an L2 round trip in front of every phase and every producer that
+    // comes to one)
+    __shared__ __align__(16) PhaseDesc s_ph[kPhaseCache];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int cta = blockIdx.x, ncta = gridDim.x;
     const int nwp = 4 * p.L + 1;
 
+    {
+        static_assert(sizeof(PhaseDesc) % 16 == 0, "PhaseDesc is copied in 16-byte words");
+        const int n = min(nwp, kPhaseCache), n16 = n * (int)(sizeof(PhaseDesc) / 16);
+        for (int i = tid; i < n16; i += kMegaThreads) reinterpret_cast<uint4*>(s_ph)[i] = __ldg(reinterpret_cast<const uint4*>(p.phases) + i);
+        __syncthreads();
+        for (int i = tid; i < n; i += kMegaThreads) keep_share<FUSE>(s_ph[i], cta, ncta, p.nsplit);
+    }
+    auto phase = [&](int i) -> PhaseDesc {
+        if (i < kPhaseCache) return s_ph[i];
+        PhaseDesc ph = p.phases[i];
+        keep_share<FUSE>(ph, cta, ncta, p.nsplit);
+        return ph;
+    };
     if (tid < kMegaWarps * kSlots + 2) mb_init(ring_bar + tid, 1);
     if (tid == 0) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     __syncthreads();
@@ -84,8 +94,8 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega_step_kernel(const MegaPa
         asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
         p.trace[((size_t)blockIdx.x * kTraceEvents) * 8 + 7] = smid;
     }
-    const int pos = p.st->pos;
-    const int token = min(max(p.st->token, 0), p.V - 1);
+    const int pos = p.call.token >= 0 ? p.call.pos : p.st->pos;
+    const int token = p.call.token >= 0 ? p.call.token : min(max(p.st->token, 0), p.V - 1);
     const unsigned bar_base = (unsigned)p.st->pad[0];
     unsigned bar_idx = 0;
 
@@ -101,10 +111,10 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega_step_kernel(const MegaPa
     auto produce_one = [&]() {   // lane 0 only: arm the next slot of this warp's stream (if any is left)
         while (pr_left <= 0) {                            // enter the next phase this warp has work in
             if (++pr_wp >= nwp) { pr_wp = nwp; return; }
-            const PhaseDesc ph = p.phases[pr_wp];
+            const PhaseDesc ph = phase(pr_wp);
             const int ks = warp & (ph.KS - 1), rg = warp / ph.KS, RG = kMegaWarps / ph.KS;
             int g0, g1;
-            phase_tiles<FUSE>(ph, cta, ncta, g0, g1);
+            share_of(ph, g0, g1);
             if constexpr (FUSE) {
                 pr_tail = 0;
                 if (ph.kind == PH_DOWN_T) {   // stripe-major matrix: this warp's tile rows [a, b) are ONE contiguous byte range, copied a slot at a time
@@ -144,7 +154,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega_step_kernel(const MegaPa
 #pragma unroll 1
     for (int wp = 0; wp < nwp; ++wp) {
         // =============================== weight phase wp ===============================================
-        const PhaseDesc ph = p.phases[wp];
+        const PhaseDesc ph = phase(wp);
         const int l = ph.layer;
         const int ks = warp & (ph.KS - 1), rg = warp / ph.KS, RG = kMegaWarps / ph.KS;
         const int c0 = ks * ph.SC;
@@ -158,7 +168,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega_step_kernel(const MegaPa
                 // x += Wdown[:, this CTA's units] . swi[this CTA's units]: the gate_up epilogue left the values in shared memory (xs),
                 // the wo epilogue left h in x. A lane owns E outputs; its warp streams the (tile row, stripe) tiles of stripe ks.
                 int g0, g1;
-                cta_tiles(ph, cta, ncta, g0, g1);
+                share_of(ph, g0, g1);
                 MEGA_STAMP(ev, 1);   // no prologue: nothing to stage
                 float acc[E];
 #pragma unroll
@@ -215,11 +225,12 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega_step_kernel(const MegaPa
                 }
             }
         }
+        if (ph.kind == PH_QKV) prefetch_norms(p, l, cta, ncta);
         // ---- 1. stage the activation vector in shared memory (plain loops, all 512 threads) -------------
         float ss = 0.f;
         if (ph.kind == PH_QKV && l == 0) {                                   // embedding gather (model.cpp:48)
             // row `token` of the (tiled) embedding/classifier matrix: tile row token/R, row token%R inside the tile
-            const PhaseDesc em = p.phases[nwp - 1];
+            const PhaseDesc em = phase(nwp - 1);
             const uint8_t* trow = p.emb + (size_t)(token / em.R) * em.KS * em.tile_bytes + (size_t)(token % em.R) * em.SC * 16;
             for (int c = tid; c < ph.nchunks; c += kMegaThreads) {
                 const int eks = c / em.SC, ecc = c - eks * em.SC;
@@ -247,24 +258,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega_step_kernel(const MegaPa
                 }
             }
         } else if (ph.kind == PH_WO) {                                       // merge the attention splits
-            const int rec = p.hd + kAttRecPad;
-            for (int c4 = tid; c4 < cols / 4; c4 += kMegaThreads) {
-                const int col = c4 * 4;
-                const int head = col / p.hd, j = col - head * p.hd;
-                const float* base = p.att_part + (size_t)head * p.nsplit * rec;
-                float M = -INFINITY;
-                for (int s = 0; s < p.nsplit; ++s) M = fmaxf(M, __ldcg(base + (size_t)s * rec + p.hd));
-                float Ls = 0.f;
-                float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-                for (int s = 0; s < p.nsplit; ++s) {
-                    const float m = __ldcg(base + (size_t)s * rec + p.hd);
-                    const float w = (m == -INFINITY) ? 0.f : expf(m - M);
-                    Ls = fmaf(__ldcg(base + (size_t)s * rec + p.hd + 1), w, Ls);
-                    const float4 v = __ldcg(reinterpret_cast<const float4*>(base + (size_t)s * rec + j));
-                    o.x = fmaf(v.x, w, o.x); o.y = fmaf(v.y, w, o.y); o.z = fmaf(v.z, w, o.z); o.w = fmaf(v.w, w, o.w);
-                }
-                reinterpret_cast<float4*>(xs)[c4] = make_float4(o.x / Ls, o.y / Ls, o.z / Ls, o.w / Ls);
-            }
+            merge_splits(p, 0, p.H_loc, xs, SL.total - SL.att_k, part);
         } else {
             const float* src = (ph.kind == PH_GATEUP) ? p.h : (ph.kind == PH_DOWN) ? p.swi : p.x;
             for (int c4 = tid; c4 < cols / 4; c4 += kMegaThreads) {
@@ -334,7 +328,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega_step_kernel(const MegaPa
         MEGA_STAMP(ev, 1);   // prologue done
         // ---- 2. stream this CTA's tile rows through the rings, round by round ------------------------------
         int g0, g1;
-        phase_tiles<FUSE>(ph, cta, ncta, g0, g1);
+        share_of(ph, g0, g1);
         const int upp = ph.R >> 1;
         const int u0 = g0 * upp;
         const int n = max(0, min(ph.nunits, g1 * upp) - u0);   // real units of this CTA
@@ -489,41 +483,8 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega_step_kernel(const MegaPa
         }
 
         if (ph.kind == PH_CLS) {   // CTA best -> global; the last CTA picks the arg max and advances the step state
-            float* sv = part;
-            int* si = reinterpret_cast<int*>(part + kMegaThreads);
-            sv[tid] = best_v;
-            si[tid] = best_i;
-            __syncthreads();
-            for (int o = kMegaThreads / 2; o > 0; o >>= 1) {
-                if (tid < o) {
-                    const float ov = sv[tid + o];
-                    const int oi = si[tid + o];
-                    if (ov > sv[tid] || (ov == sv[tid] && oi < si[tid])) { sv[tid] = ov; si[tid] = oi; }
-                }
-                __syncthreads();
-            }
-            if (tid == 0) {
-                p.blk_val[cta] = sv[0];
-                p.blk_idx[cta] = si[0];
-                __threadfence();
-                s_last = (atomicAdd(&p.st->ticket, 1) == ncta - 1);
-            }
-            __syncthreads();
-            if (s_last && tid == 0) {
-                __threadfence();
-                float v = -INFINITY;
-                int idx = 0x7fffffff;
-                for (int b = 0; b < ncta; ++b) {
-                    const float ov = __ldcg(p.blk_val + b);
-                    const int oi = __ldcg(p.blk_idx + b);
-                    if (ov > v || (ov == v && oi < idx)) { v = ov; idx = oi; }
-                }
-                if (idx == 0x7fffffff) idx = 0;
-                p.st->ticket = 0;
+            if (mega_finish(p, best_v, best_i, part, &s_last, cta, ncta)) {
                 p.st->pad[0] = (int32_t)(bar_base + bar_idx * (unsigned)ncta);   // barrier epoch for the next launch
-                p.blk_val[ncta] = v;
-                p.blk_idx[ncta] = idx;
-                ClsPolicy<SLLM_F32>::step_feedback(p.st, p.prompt, p.history, idx);
             }
             break;
         }

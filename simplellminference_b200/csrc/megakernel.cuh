@@ -55,6 +55,12 @@ inline TileGeom mega_tile_geom(int rows_phys, int cols, int w_dtype) {
 // bytes of one [rows][cols] matrix of phase kind `kind` in the tiled layout
 size_t mega_matrix_bytes(int rows, int cols, int kind, int w_dtype);
 
+// One step asked for by value (sllm_engine_forward): its token and position come with the launch, its arg max goes into pinned host memory, so that nothing is
+// copied for them. token < 0: both are the device's (StepState), which is advanced either way.
+struct MegaCall {
+    int32_t token = -1, pos = 0;
+    int32_t* next = nullptr;      // or NULL
+};
 struct MegaParams {
     const PhaseDesc* phases;   // [4L+1]
     int32_t d, hd, L, S, V, V_loc, v0, q_loc, kv_loc, I_loc, H_loc, KVH_loc, nsplit;
@@ -73,6 +79,7 @@ struct MegaParams {
     int32_t* history;
     unsigned* bar_counter;
     unsigned long long* trace;  // optional [grid][512][8] %globaltimer stamps (nullptr = off)
+    MegaCall call;
     int32_t debug;              // measurement aid (sllm_tune key 8; results are garbage): bit 0 = skip the grid barriers, bit 1 = skip the dot products
 };
 

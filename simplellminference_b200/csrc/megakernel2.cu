@@ -138,6 +138,8 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega2_step_kernel(const Mega2
         static_assert(sizeof(PhaseDesc) % 16 == 0, "PhaseDesc is copied in 16-byte words");
         const int n16 = min(nwp, kPhaseCache) * (int)(sizeof(PhaseDesc) / 16);
         for (int i = tid; i < n16; i += kMegaThreads) reinterpret_cast<uint4*>(s_ph)[i] = __ldg(reinterpret_cast<const uint4*>(p.phases) + i);
+        __syncthreads();
+        for (int i = tid; i < min(nwp, kPhaseCache); i += kMegaThreads) keep_share<FUSE>(s_ph[i], cta, ncta, p.nsplit);
     }
     if (tid < kMegaWarps * kSlots + 3) mb_init(ring_bar + tid, 1);
     if (tid == 0) {
@@ -151,9 +153,14 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega2_step_kernel(const Mega2
         asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
         p.trace[((size_t)blockIdx.x * kTraceEvents2) * 8 + 7] = smid;
     }
-    auto phase = [&](int i) -> PhaseDesc { return i < kPhaseCache ? s_ph[i] : p.phases[i]; };
-    const int pos = p.st->pos;
-    const int token = min(max(p.st->token, 0), p.V - 1);
+    auto phase = [&](int i) -> PhaseDesc {
+        if (i < kPhaseCache) return s_ph[i];
+        PhaseDesc ph = p.phases[i];
+        keep_share<FUSE>(ph, cta, ncta, p.nsplit);
+        return ph;
+    };
+    const int pos = p.call.token >= 0 ? p.call.pos : p.st->pos;
+    const int token = p.call.token >= 0 ? p.call.token : min(max(p.st->token, 0), p.V - 1);
     const unsigned bar_base = (unsigned)p.st->pad[0];
     const unsigned epoch = (unsigned)p.st->pad[2];          // launches of THIS kernel so far: every counter below is monotonic
     unsigned bar_idx = 0;
@@ -172,7 +179,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega2_step_kernel(const Mega2
     {
         const PhaseDesc ph0 = phase(0);
         int g0, g1;
-        cta_tiles(ph0, cta, ncta, g0, g1);
+        share_of(ph0, g0, g1);
         const int upp = ph0.R >> 1;
         const int a = g0 * upp, b = min(ph0.nunits, g1 * upp);
         if (tid < p.KVH_loc && b > a) {
@@ -203,7 +210,8 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega2_step_kernel(const Mega2
             const PhaseDesc ph = phase(pr_wp);
             if (ph.kind == PH_WO_T) {   // this CTA's row range of its kv head group's block: tiles T0 + warp, + 16, ...
                 if (!has_item) continue;
-                const int T0 = (int)(((int64_t)ph.ntr * my_part) / p.nsplit), T1 = (int)(((int64_t)ph.ntr * (my_part + 1)) / p.nsplit);
+                int T0, T1;
+                share_of(ph, T0, T1);
                 pr_left = (T1 - T0 - warp + kMegaWarps - 1) / kMegaWarps;
                 pr_ptr = ph.W + ((size_t)my_kvh * ph.ntr + T0 + warp) * ph.tile_bytes;
                 pr_step = (uint32_t)kMegaWarps * ph.tile_bytes;
@@ -213,7 +221,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega2_step_kernel(const Mega2
             }
             const int ks = warp & (ph.KS - 1), rg = warp / ph.KS, RG = kMegaWarps / ph.KS;
             int g0, g1;
-            phase_tiles<FUSE>(ph, cta, ncta, g0, g1);
+            share_of(ph, g0, g1);
             pr_tail = 0;
             if constexpr (FUSE) {
                 if (ph.kind == PH_DOWN_T) {
@@ -274,9 +282,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega2_step_kernel(const Mega2
                 const int ghd = G * p.hd;
                 if (tid == 0 && !(p.debug & 1)) flag_wait(att_cnt + (size_t)my_kvh * 32, abase + (unsigned)((l + 1) * p.nsplit));
                 __syncthreads();
-                // merge the group's attention splits: weights of the splits per head first, then the columns
                 const int rec = p.hd + kAttRecPad;
-                float* wgt = part;                              // [G][nsplit + 1] (the partial table is idle here)
                 if (p.nsplit <= 8) {   // every record word a thread needs, requested at once: ONE L2 round trip, the weights recomputed per thread
                     for (int c4 = tid; c4 < ghd / 4; c4 += kMegaThreads) {
                         const int col = c4 * 4;
@@ -307,33 +313,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega2_step_kernel(const Mega2
                         reinterpret_cast<float4*>(xs)[c4] = make_float4(o.x / Ls, o.y / Ls, o.z / Ls, o.w / Ls);
                     }
                 } else {
-                if (tid < G) {
-                    const float* base = p.att_part + (size_t)(my_kvh * G + tid) * p.nsplit * rec + p.hd;
-                    float M = -INFINITY;
-                    for (int s = 0; s < p.nsplit; ++s) M = fmaxf(M, __ldcg(base + (size_t)s * rec));
-                    float Ls = 0.f;
-                    for (int s = 0; s < p.nsplit; ++s) {
-                        const float m = __ldcg(base + (size_t)s * rec);
-                        const float w = (m == -INFINITY) ? 0.f : expf(m - M);
-                        Ls = fmaf(__ldcg(base + (size_t)s * rec + 1), w, Ls);
-                        wgt[tid * (p.nsplit + 1) + s] = w;
-                    }
-                    wgt[tid * (p.nsplit + 1) + p.nsplit] = Ls;
-                }
-                __syncthreads();
-                for (int c4 = tid; c4 < ghd / 4; c4 += kMegaThreads) {
-                    const int col = c4 * 4;
-                    const int gi = col / p.hd, j = col - gi * p.hd;
-                    const float* base = p.att_part + (size_t)(my_kvh * G + gi) * p.nsplit * rec + j;
-                    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-                    for (int s = 0; s < p.nsplit; ++s) {
-                        const float w = wgt[gi * (p.nsplit + 1) + s];
-                        const float4 v = __ldcg(reinterpret_cast<const float4*>(base + (size_t)s * rec));
-                        o.x = fmaf(v.x, w, o.x); o.y = fmaf(v.y, w, o.y); o.z = fmaf(v.z, w, o.z); o.w = fmaf(v.w, w, o.w);
-                    }
-                    const float Ls = wgt[gi * (p.nsplit + 1) + p.nsplit];
-                    reinterpret_cast<float4*>(xs)[c4] = make_float4(o.x / Ls, o.y / Ls, o.z / Ls, o.w / Ls);
-                }
+                    merge_splits(p, my_kvh * G, G, xs, SL.total - SL.att_k, part);
                 }
                 __syncthreads();
                 // this lane's chunk(s) of the merged vector -> registers
@@ -354,7 +334,8 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega2_step_kernel(const Mega2
                 }
                 M2_STAMP(ev, 1);
                 const int NR = ph.R;
-                const int T0 = (int)(((int64_t)ph.ntr * my_part) / p.nsplit), T1 = (int)(((int64_t)ph.ntr * (my_part + 1)) / p.nsplit);
+                int T0, T1;
+                share_of(ph, T0, T1);
 #pragma unroll 1
                 for (int t = T0 + warp; t < T1; t += kMegaWarps) {
                     const int si = cons_count & (kSlots - 1);
@@ -401,7 +382,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega2_step_kernel(const Mega2
                 // x_out += Wdown[:, this CTA's units] . swi[this CTA's units] (values left in xs by the gate_up epilogue); x_out was zeroed
                 // during the qkv phase, CTA 0 adds the residual h once
                 int g0, g1;
-                cta_tiles(ph, cta, ncta, g0, g1);
+                share_of(ph, g0, g1);
                 M2_STAMP(ev, 1);
                 float acc[E];
 #pragma unroll
@@ -470,7 +451,9 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega2_step_kernel(const Mega2
         if (ph.kind == PH_QKV) {
             // zero, a layer / a phase ahead, the vectors the reductions of the NEXT dependency points land on: the next layer's h and
             // (fused down) this layer's x_out. Their last readers finished before the grid barrier this CTA has just passed.
-            const int n4 = p.d >> 2, z0 = (int)(((int64_t)n4 * cta) / ncta), z1 = (int)(((int64_t)n4 * (cta + 1)) / ncta);
+            const unsigned n4 = (unsigned)p.d >> 2;
+            const int z0 = (int)(n4 * (unsigned)cta / (unsigned)ncta), z1 = (int)(n4 * (unsigned)(cta + 1) / (unsigned)ncta);
+            prefetch_norms(p, l, cta, ncta);
             for (int i = z0 + tid; i < z1; i += kMegaThreads) {
                 reinterpret_cast<float4*>(P.hbuf[par ^ 1])[i] = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (FUSE) reinterpret_cast<float4*>(x_out)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -564,7 +547,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega2_step_kernel(const Mega2
         M2_STAMP(ev, 1);   // prologue done
         // ---- 2. stream this CTA's tile rows through the rings, round by round ------------------------------
         int g0, g1;
-        phase_tiles<FUSE>(ph, cta, ncta, g0, g1);
+        share_of(ph, g0, g1);
         const int upp = ph.R >> 1;
         const int u0 = g0 * upp;
         const int n = max(0, min(ph.nunits, g1 * upp) - u0);
@@ -702,42 +685,9 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega2_step_kernel(const Mega2
         }
 
         if (ph.kind == PH_CLS) {
-            float* sv = part;
-            int* si = reinterpret_cast<int*>(part + kMegaThreads);
-            sv[tid] = best_v;
-            si[tid] = best_i;
-            __syncthreads();
-            for (int o = kMegaThreads / 2; o > 0; o >>= 1) {
-                if (tid < o) {
-                    const float ov = sv[tid + o];
-                    const int oi = si[tid + o];
-                    if (ov > sv[tid] || (ov == sv[tid] && oi < si[tid])) { sv[tid] = ov; si[tid] = oi; }
-                }
-                __syncthreads();
-            }
-            if (tid == 0) {
-                p.blk_val[cta] = sv[0];
-                p.blk_idx[cta] = si[0];
-                __threadfence();
-                s_last = (atomicAdd(&p.st->ticket, 1) == ncta - 1);
-            }
-            __syncthreads();
-            if (s_last && tid == 0) {
-                __threadfence();
-                float v = -INFINITY;
-                int idx = 0x7fffffff;
-                for (int b = 0; b < ncta; ++b) {
-                    const float ov = __ldcg(p.blk_val + b);
-                    const int oi = __ldcg(p.blk_idx + b);
-                    if (ov > v || (ov == v && oi < idx)) { v = ov; idx = oi; }
-                }
-                if (idx == 0x7fffffff) idx = 0;
-                p.st->ticket = 0;
-                p.st->pad[0] = (int32_t)(bar_base + bar_idx * (unsigned)ncta);
+            if (mega_finish(p, best_v, best_i, part, &s_last, cta, ncta)) {
+                p.st->pad[0] = (int32_t)(bar_base + bar_idx * (unsigned)ncta);   // barrier epoch for the next launch
                 p.st->pad[2] = (int32_t)(epoch + 1u);
-                p.blk_val[ncta] = v;
-                p.blk_idx[ncta] = idx;
-                ClsPolicy<SLLM_F32>::step_feedback(p.st, p.prompt, p.history, idx);
             }
             break;
         }
