@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega_step_kernel(const MegaPa
         while (pr_left <= 0) {                            // enter the next phase this warp has work in
             if (++pr_wp >= nwp) { pr_wp = nwp; return; }
             const PhaseDesc ph = phase(pr_wp);
-            const int ks = warp & (ph.KS - 1), rg = warp / ph.KS, RG = kMegaWarps / ph.KS;
+            const int ks_log2 = __ffs(ph.KS) - 1, ks = warp & (ph.KS - 1), rg = warp >> ks_log2, RG = kMegaWarps >> ks_log2;   // KS: a power of two
             int g0, g1;
             share_of(ph, g0, g1);
             if constexpr (FUSE) {
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega_step_kernel(const MegaPa
                     continue;
                 }
             }
-            pr_left = (g1 - g0 - rg + RG - 1) / RG;       // tile rows g0+rg, g0+rg+RG, ... < g1
+            pr_left = (g1 - g0 - rg + RG - 1) >> (4 - ks_log2);       // tile rows g0+rg, g0+rg+RG, ... < g1
             pr_ptr = ph.W + ((size_t)(g0 + rg) * ph.KS + ks) * ph.tile_bytes;
             pr_step = (uint32_t)RG * ph.KS * ph.tile_bytes;
             pr_bytes = (uint32_t)ph.tile_bytes;
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega_step_kernel(const MegaPa
         // =============================== weight phase wp ===============================================
         const PhaseDesc ph = phase(wp);
         const int l = ph.layer;
-        const int ks = warp & (ph.KS - 1), rg = warp / ph.KS, RG = kMegaWarps / ph.KS;
+        const int ks_log2 = __ffs(ph.KS) - 1, ks = warp & (ph.KS - 1), rg = warp >> ks_log2, RG = kMegaWarps >> ks_log2;   // KS: a power of two
         const int c0 = ks * ph.SC;
         const int nsc = max(0, min(ph.SC, ph.nchunks - c0));   // real chunks of this slice (the tile is zero padded to SC)
         const int cols = ph.nchunks * E;
@@ -340,10 +340,10 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega_step_kernel(const MegaPa
 
 #pragma unroll 1
         for (int rbase = 0; rbase < n || rbase == 0; rbase += kRoundUnits) {
-            const int jend = min(nslots, (rbase + kRoundUnits) / upp);
+            const int jend = min(nslots, (rbase + kRoundUnits) >> (upp - 1));   // upp: 1 or 2
             {
 #pragma unroll 1
-                for (int j = rbase / upp + rg; j < jend; j += RG) {
+                for (int j = (rbase >> (upp - 1)) + rg; j < jend; j += RG) {
                     const int si = cons_count & (kSlots - 1);
                     mb_wait_fast(my_bar + si, (cons_count / kSlots) & 1);
                     const uint8_t* sp = my_ring + (size_t)si * kSlotBytes + lane * 16;

@@ -173,6 +173,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega2_step_kernel(const Mega2
     unsigned* const att_cnt = P.flags + (size_t)p.KVH_loc * 32;
     const int my_kvh = cta / p.nsplit, my_part = cta - my_kvh * p.nsplit;   // this CTA's item (meaningful when cta < nitems)
     const bool has_item = cta < nitems;
+    const int att_per = (pos + p.nsplit) / p.nsplit;        // positions of a split
 
     // which kv head groups this CTA's qkv units belong to (the same in every layer): group g owns q units [g*G*half, (g+1)*G*half),
     // k units q_units + [g*half, (g+1)*half), v units rope_units + [g*half, (g+1)*half)
@@ -219,7 +220,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega2_step_kernel(const Mega2
                 pr_tail = 0;
                 continue;
             }
-            const int ks = warp & (ph.KS - 1), rg = warp / ph.KS, RG = kMegaWarps / ph.KS;
+            const int ks_log2 = __ffs(ph.KS) - 1, ks = warp & (ph.KS - 1), rg = warp >> ks_log2, RG = kMegaWarps >> ks_log2;   // KS: a power of two
             int g0, g1;
             share_of(ph, g0, g1);
             pr_tail = 0;
@@ -236,7 +237,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega2_step_kernel(const Mega2
                     continue;
                 }
             }
-            pr_left = (g1 - g0 - rg + RG - 1) / RG;
+            pr_left = (g1 - g0 - rg + RG - 1) >> (4 - ks_log2);
             pr_ptr = ph.W + ((size_t)(g0 + rg) * ph.KS + ks) * ph.tile_bytes;
             pr_step = (uint32_t)RG * ph.KS * ph.tile_bytes;
             pr_bytes = (uint32_t)ph.tile_bytes;
@@ -371,7 +372,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega2_step_kernel(const Mega2
             continue;
         }
 
-        const int ks = warp & (ph.KS - 1), rg = warp / ph.KS, RG = kMegaWarps / ph.KS;
+        const int ks_log2 = __ffs(ph.KS) - 1, ks = warp & (ph.KS - 1), rg = warp >> ks_log2, RG = kMegaWarps >> ks_log2;   // KS: a power of two
         const int c0 = ks * ph.SC;
         const int nsc = max(0, min(ph.SC, ph.nchunks - c0));
         const int cols = ph.nchunks * E;
@@ -528,7 +529,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega2_step_kernel(const Mega2
             if (warp == 0 && lane == 0) {
                 fence_async_smem();
                 const int row_bytes = p.hd * KESZ;
-                const int npos = pos + 1, per = (npos + p.nsplit - 1) / p.nsplit;
+                const int npos = pos + 1, per = att_per;
                 const int t0 = my_part * per, t1 = min(npos, t0 + per);
                 const size_t head_off = ((size_t)l * p.KVH_loc + my_kvh) * p.S * row_bytes;   // [L][KVH][S][hd]
                 for (int tile = 0; tile < 2; ++tile) {
@@ -575,9 +576,9 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega2_step_kernel(const Mega2
 
 #pragma unroll 1
         for (int rbase = 0; rbase < n || rbase == 0; rbase += kRoundUnits) {
-            const int jend = min(nslots, (rbase + kRoundUnits) / upp);
+            const int jend = min(nslots, (rbase + kRoundUnits) >> (upp - 1));   // upp: 1 or 2
 #pragma unroll 1
-            for (int j = rbase / upp + rg; j < jend; j += RG) {
+            for (int j = (rbase >> (upp - 1)) + rg; j < jend; j += RG) {
                 const int si = cons_count & (kSlots - 1);
                 mb_wait_fast(my_bar + si, (cons_count / kSlots) & 1);
                 const uint8_t* sp = my_ring + (size_t)si * kSlotBytes + lane * 16;
@@ -712,7 +713,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega2_step_kernel(const Mega2
         const int tail_cap = min(kAttTile, (kRoundUnits * 2 * kMegaWarps * 4) / (2 * att_row_bytes));
         int att_t0 = 0, att_rows = 0;
         if (has_item) {
-            const int npos_ = pos + 1, per_ = (npos_ + p.nsplit - 1) / p.nsplit;
+            const int npos_ = pos + 1, per_ = att_per;
             att_t0 = my_part * per_;
             att_rows = max(0, min(npos_, att_t0 + per_) - att_t0);
         }
@@ -747,7 +748,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega2_step_kernel(const Mega2
             const int row_bytes = p.hd * KESZ;
             const int cpr = row_bytes / 16;
             const int npos = pos + 1;
-            const int per = (npos + p.nsplit - 1) / p.nsplit;
+            const int per = att_per;
             const float scale = 1.0f / sqrtf((float)p.hd);
             constexpr int kStripes = 16;
             const int pv_chunk = tid % cpr, pv_stripe = tid / cpr;
@@ -776,6 +777,16 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega2_step_kernel(const Mega2
                     }
                 }
             };
+            auto krow = [&](int r) -> uint8_t* { return r < 2 * AT ? k_s + (size_t)r * stride : tail_k + (size_t)(r - 2 * AT) * row_bytes; };
+            auto vrow = [&](int r) -> uint8_t* { return r < 2 * AT ? v_s + (size_t)r * stride : tail_v + (size_t)(r - 2 * AT) * row_bytes; };
+            // the newest row (generic stores of this launch) bypasses the async proxy; it lies behind what the copies write, so it travels beside q
+            if (att_single && pos >= t0 && pos < t1 && warp == kMegaWarps - 1) {
+                const size_t g_off = head_off + (size_t)pos * row_bytes;
+                for (int c = lane; c < cpr; c += 32) {
+                    *reinterpret_cast<uint4*>(krow(pos - t0) + c * 16) = __ldcg(reinterpret_cast<const uint4*>(p.kc + g_off + c * 16));
+                    *reinterpret_cast<uint4*>(vrow(pos - t0) + c * 16) = __ldcg(reinterpret_cast<const uint4*>(p.vc + g_off + c * 16));
+                }
+            }
             fence_async_smem();
             __syncthreads();
             float acc[G][KVEC];
@@ -786,19 +797,9 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega2_step_kernel(const Mega2
 
             if (att_single) {
                 const int nrows = att_rows;
-                auto krow = [&](int r) -> const uint8_t* { return r < 2 * AT ? k_s + (size_t)r * stride : tail_k + (size_t)(r - 2 * AT) * row_bytes; };
-                auto vrow = [&](int r) -> const uint8_t* { return r < 2 * AT ? v_s + (size_t)r * stride : tail_v + (size_t)(r - 2 * AT) * row_bytes; };
-                if (pos >= t0 && pos < t1 && warp == 1) {   // the newest row (generic stores of this launch) bypasses the async proxy
-                    const size_t g_off = head_off + (size_t)pos * row_bytes;
-                    for (int c = lane; c < cpr; c += 32) {
-                        *reinterpret_cast<uint4*>(const_cast<uint8_t*>(krow(pos - t0)) + c * 16) = __ldcg(reinterpret_cast<const uint4*>(p.kc + g_off + c * 16));
-                        *reinterpret_cast<uint4*>(const_cast<uint8_t*>(vrow(pos - t0)) + c * 16) = __ldcg(reinterpret_cast<const uint4*>(p.vc + g_off + c * 16));
-                    }
-                }
                 if (nrows > 0) { mb_wait_fast(att_bar, kv_use0 & 1); kv_use0++; }
                 if (nrows > AT) { mb_wait_fast(att_bar + 1, kv_use1 & 1); kv_use1++; }
                 if (att_tail > 0) { mb_wait_fast(att_bar + 2, kv_use2 & 1); kv_use2++; }
-                __syncthreads();
 #pragma unroll 1
                 for (int kb = 0; kb < nrows; kb += kAttTile) {        // scores of all rows, 8 threads per key
                     const int r = kb + key;
