@@ -42,6 +42,9 @@ inline int status_check() { return g_status && *reinterpret_cast<volatile int32_
         SLLM_CUDA(cudaGetLastError());                   \
         if (int _s = ::sllm::status_check()) return _s;  \
     } while (0)
+// The same without the word: for a kernel that may set it, whose launcher has looked at it before (status_check), and for launches behind one in the same call, which would
+// otherwise report this very call, or not, by how fast the kernel gives up.
+#define SLLM_LAUNCH_CHECK_ONLY() SLLM_CUDA(cudaGetLastError())
 // A wait of the library for a stream whose results it hands out.
 #define SLLM_WAIT(stream)                                \
     do {                                                 \

@@ -8,21 +8,26 @@
 //                       prompt lie outside the tensor map and read as zeros);
 //   warp 1 (one lane)   MMA issuer: S = Q K^T (both K-major) into TMEM; O += P V with P read from TMEM, V as the MN-major operand as it lies;
 //   warps 4-7, 8-11     softmax of tile 0 / 1, a thread per query row: tcgen05.ld the scores (once for the maximum, the second half once more for the
-//                       weights), exponentials in powers of two, weights packed as bf16 over the scores' own TMEM columns. O stays in TMEM and is
-//                       rescaled whenever the maximum of one of the warp's rows has grown: a row's largest weights, which decide its error, are then
-//                       rounded to bf16 next to 1, where they lose least, and their sum is that of the rounded ones. (With a reference that lagged by up to
-//                       2^8 and the sum of the unrounded ones the result was off by 2.34e-3 instead of 2.29e-3 on the case below and by 2.12e-3 instead
+//                       weights), exponentials in powers of two, weights packed as bf16 over the scores' own TMEM columns; two values per instruction
+//                       where there is one (fma, add), three in the maximum;
+//   warps 12-15         O of both tiles: stays in TMEM and is rescaled whenever the maximum of one of the rows of a warp has grown, while the softmax
+//                       warps take their exponentials. The reference is the maximum so far: a row's largest weights, which decide its error, are
+//                       rounded to bf16 next to 1, where they lose least, and their sum is that of the rounded ones. (With a reference that lagged by up
+//                       to 2^8 and the sum of the unrounded ones the result was off by 2.34e-3 instead of 2.29e-3 on the case below and by 2.12e-3 instead
 //                       of 1.72e-3 with scores four times as wide; mma.sync 2.29e-3 and 1.73e-3.)
-// TMEM: S0 | S1 | O0 | O1, 128 columns each. Bound: the tensor pipe and the exponentials, 1024 clocks each per pair of 128 x 128 tiles at head_dim 128;
-// mma.sync, which it replaces for bf16 caches, spent them one after the other in the same warps. Measured, 2048 queries behind 6144 positions, 32 heads
-// over 8 of 128: 390 us, 617 TFLOP/s (mma.sync 1061 us, 227; with the lagging reference 348); 256 CTAs on 148 SMs leave a last wave of 108.
+// TMEM: S0 | S1 | O0 | O1, 128 columns each. Bound: the tensor pipe and the exponentials, 1024 clocks each per 128 x 128 tile at head_dim 128, and the chain
+// scores -> softmax -> product of a tile; mma.sync, which it replaces for bf16 caches, spent them one after the other in the same warps. Measured, 2048
+// queries behind 6144 positions, 32 heads over 8 of 128: 317 us, 760 TFLOP/s (mma.sync 1061 us, 227; rescaling in the softmax warps, one body for masked and other
+// tiles and one value per instruction 391); 256 CTAs on 148 SMs leave a last wave of 108.
+#include <type_traits>
+
 #include "prefill.cuh"
 #include "tcgen05.cuh"
 
 namespace sllm {
 extern int g_tune_pf_pdl;
 
-constexpr int kTaThreads = 384, kTaTile = 128;      // queries of a tile = keys of a tile
+constexpr int kTaThreads = 512, kTaTile = 128;      // queries of a tile = keys of a tile
 constexpr uint32_t kTaTmem = 512;
 
 template <int HD>
@@ -30,7 +35,7 @@ struct TaShape {
     static constexpr int kBlocks = HD / 64;                                   // 64-column blocks (128-byte rows) of a tile
     static constexpr int kBlockBytes = kTaTile * 128, kTileBytes = kBlocks * kBlockBytes;
     static constexpr int kStages = HD == 128 ? 2 : 4;
-    static constexpr int kSmem = 1024 + (2 + 2 * kStages) * kTileBytes + 512;
+    static constexpr int kSmem = 1024 + (2 + 2 * kStages) * kTileBytes + 512 + 2 * kTaTile * (int)sizeof(float);
 };
 
 struct TaArgs {
@@ -53,8 +58,10 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
     uint8_t* sQ = sV + ST * Sh::kTileBytes;
     uint64_t* bars = reinterpret_cast<uint64_t*>(sQ + 2 * Sh::kTileBytes);
     uint64_t *kfull = bars, *kempty = kfull + ST, *vfull = kempty + ST, *vempty = vfull + ST, *qfull = vempty + ST;
-    uint64_t *sfull = qfull + 1, *pready = sfull + 2, *odone = pready + 2;      // per tile: scores written / weights written / product with the values done
+    // per tile: scores written / factors for O written / weights written and O rescaled / product with the values done
+    uint64_t *sfull = qfull + 1, *factors = sfull + 2, *pready = factors + 2, *odone = pready + 2;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(odone + 2);
+    float* factor = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 512);       // [2][kTaTile]
     volatile int* gave_up = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -77,7 +84,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
         tma_prefetch_desc(&tmV);
         for (int i = 0; i < ST; ++i) { mb_init(kfull + i, 1); mb_init(kempty + i, 1); mb_init(vfull + i, 1); mb_init(vempty + i, 1); }
         mb_init(qfull, 1);
-        for (int j = 0; j < 2; ++j) { mb_init(sfull + j, 1); mb_init(pready + j, 128); mb_init(odone + j, 1); }
+        for (int j = 0; j < 2; ++j) { mb_init(sfull + j, 1); mb_init(factors + j, 128); mb_init(pready + j, 256); mb_init(odone + j, 1); }
         *gave_up = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -154,19 +161,55 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
                 if (kt + 1 < kts) tc_commit(kempty + (kt + 1) % ST);
             }
         }
+    } else if (warp >= 12) {   // ===== O of both tiles: rescaled while the softmax warps take their exponentials =====
+        const int quad = warp & 3, row = quad * 32 + lane;
+        bool ok = true;
+        for (int kt = 0; ok && kt < kts; ++kt)
+            for (int j = 0; ok && j < items; ++j) {
+                if (kt >= nkt[j]) continue;
+                ok = tc_wait_warp(factors + j, (uint32_t)kt & 1, gave_up, p.polls);
+                if (ok && kt > 0) ok = tc_wait_warp(odone + j, (uint32_t)(kt - 1) & 1, gave_up, p.polls);     // long since: the scores follow that product
+                if (!ok) break;
+                tc_fence_after();
+                const float f = factor[j * kTaTile + row];
+                if (kt > 0 && __any_sync(0xffffffffu, f != 1.0f)) {
+                    const uint32_t o_tmem = tmem + ((uint32_t)(quad * 32) << 16) + 256 + 128 * j;
+                    const uint64_t ff = tc_two(__float_as_uint(f), __float_as_uint(f));
+#pragma unroll 1
+                    for (int c = 0; c < HD; c += 64) {
+                        uint32_t o[2][32];
+                        tc_ld32_async(o_tmem + c, o[0]);
+                        tc_ld32_async(o_tmem + c + 32, o[1]);
+                        tc_arrived(o[0]);
+                        tc_arrived(o[1]);
+#pragma unroll
+                        for (int i = 0; i < 64; i += 2) {
+                            float x, y;
+                            tc_split(tc_mul2(tc_two(o[i / 32][i % 32], o[i / 32][i % 32 + 1]), ff), x, y);
+                            o[i / 32][i % 32] = __float_as_uint(x);
+                            o[i / 32][i % 32 + 1] = __float_as_uint(y);
+                        }
+                        tc_st32(o_tmem + c, o[0]);
+                        tc_st32(o_tmem + c + 32, o[1]);
+                    }
+                    tc_wait_st();
+                }
+                tc_fence_before();
+                mb_arrive(pready + j);
+            }
     } else if (warp >= 4) {   // ===== softmax: TMEM lane quadrant = warp % 4 =====
         const int j = (warp - 4) >> 2, quad = warp & 3, row = quad * 32 + lane;
         if (j < items) {
             const uint32_t lanes = (uint32_t)(quad * 32) << 16, s_tmem = tmem + lanes + 128 * j, o_tmem = tmem + lanes + 256 + 128 * j;
             const int t = t0[j] + row, qpos = p.pos0 + t, first_pos = p.pos0 + t0[j] + quad * 32;
+            const uint64_t scale2 = tc_two(__float_as_uint(p.scale_log2), __float_as_uint(p.scale_log2));
             float ref = -INFINITY, l = 0.0f;            // what the weights are relative to (log2 units); their sum
             bool ok = true;
-            for (int kt = 0; kt < nkt[j]; ++kt) {
-                ok = tc_wait_warp(sfull + j, (uint32_t)kt & 1, gave_up, p.polls);
-                if (!ok) break;
-                tc_fence_after();
-                const bool masked = kt * kTaTile + kTaTile - 1 > first_pos;       // some row of this warp does not see every key of the tile
-                const int seen = qpos - kt * kTaTile;                             // columns 0 .. seen are visible to this row
+            // One tile of scores. kMasked: some row of this warp does not see every key of it (columns 0 .. seen are visible); in a body of its own, since
+            // comparing and choosing cost as much as everything else a score needs (1700 issue slots a warp and tile, 800 without)
+            auto step = [&](auto masked, int kt) {
+                constexpr bool kMasked = decltype(masked)::value;
+                const int seen = qpos - kt * kTaTile;
                 uint32_t a[32], b[32];
                 tc_ld32_async(s_tmem + 64, a);
                 tc_ld32_async(s_tmem + 96, b);
@@ -175,10 +218,12 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
                 float m0 = -INFINITY, m1 = -INFINITY;
                 auto top = [&](const uint32_t* v, int c0) {
 #pragma unroll
-                    for (int i = 0; i < 32; i += 2) {
-                        const float x = !masked || c0 + i <= seen ? __uint_as_float(v[i]) : -INFINITY, y = !masked || c0 + i + 1 <= seen ? __uint_as_float(v[i + 1]) : -INFINITY;
-                        m0 = fmaxf(m0, x);
-                        m1 = fmaxf(m1, y);
+                    for (int i = 0; i < 32; i += 4) {
+                        float x[4];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) x[e] = !kMasked || c0 + i + e <= seen ? __uint_as_float(v[i + e]) : -INFINITY;
+                        m0 = tc_max3(m0, x[0], x[1]);
+                        m1 = tc_max3(m1, x[2], x[3]);
                     }
                 };
                 top(a, 64);
@@ -189,36 +234,28 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
                 tc_arrived(b);
                 top(a, 0);
                 top(b, 32);
-                const float mx = fmaxf(m0, m1) * p.scale_log2;
-                if (kt == 0) {
-                    ref = mx;
-                } else if (__any_sync(0xffffffffu, mx > ref)) {                   // the product before this one has completed: these scores follow it
-                    const float nr = fmaxf(ref, mx), f = tc_exp2(ref - nr);
-                    l *= f;
-                    ref = nr;
-#pragma unroll 1
-                    for (int c = 0; c < HD; c += 32) {
-                        uint32_t o[32];
-                        tc_ld32_async(o_tmem + c, o);
-                        tc_arrived(o);
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f);
-                        tc_st32(o_tmem + c, o);
-                    }
-                }
-                float l0 = 0.0f, l1 = 0.0f;
+                const float nr = fmaxf(ref, fmaxf(m0, m1) * p.scale_log2), f = kt == 0 || nr == ref ? 1.0f : tc_exp2(ref - nr);
+                factor[j * kTaTile + row] = f;
+                mb_arrive(factors + j);
+                l *= f;
+                ref = nr;
+                const uint64_t neg2 = tc_two(__float_as_uint(-ref), __float_as_uint(-ref));
+                uint64_t sum0 = 0, sum1 = 0;                                      // (0, 0)
                 auto weigh = [&](const uint32_t* v, int c0) {                     // 32 scores -> 16 columns of weights
                     uint32_t w[16];
 #pragma unroll
                     for (int i = 0; i < 32; i += 2) {
-                        float x = tc_exp2(fmaf(__uint_as_float(v[i]), p.scale_log2, -ref)), y = tc_exp2(fmaf(__uint_as_float(v[i + 1]), p.scale_log2, -ref));
-                        if (masked) {
+                        float x, y;
+                        tc_split(tc_fma2(tc_two(v[i], v[i + 1]), scale2, neg2), x, y);
+                        x = tc_exp2(x);
+                        y = tc_exp2(y);
+                        if (kMasked) {
                             x = c0 + i <= seen ? x : 0.0f;
                             y = c0 + i + 1 <= seen ? y : 0.0f;
                         }
                         w[i / 2] = tc_pack(x, y);
-                        l0 += __uint_as_float(w[i / 2] << 16);                    // the weights as they are used
-                        l1 += __uint_as_float(w[i / 2] & 0xffff0000u);
+                        uint64_t& sum = (i & 2) ? sum1 : sum0;
+                        sum = tc_add2(sum, tc_two(w[i / 2] << 16, w[i / 2] & 0xffff0000u));      // the weights as they are used
                     }
                     tc_st16(s_tmem + c0 / 2, w);
                 };
@@ -230,7 +267,16 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
                 tc_arrived(b);
                 weigh(a, 64);
                 weigh(b, 96);
+                float l0, l1;
+                tc_split(tc_add2(sum0, sum1), l0, l1);
                 l += l0 + l1;
+            };
+            for (int kt = 0; kt < nkt[j]; ++kt) {
+                ok = tc_wait_warp(sfull + j, (uint32_t)kt & 1, gave_up, p.polls);
+                if (!ok) break;
+                tc_fence_after();
+                if (kt * kTaTile + kTaTile - 1 > first_pos) step(std::true_type{}, kt);
+                else step(std::false_type{}, kt);
                 tc_wait_st();
                 tc_fence_before();
                 mb_arrive(pready + j);
@@ -290,6 +336,7 @@ static int ta_launch(const uint16_t* q, const void* kc, const void* vc, uint16_t
     a.tiles = (T + kTaTile - 1) / kTaTile;
     // two tiles per CTA hide each other's softmax and share their loads, unless single ones would still leave SMs idle
     a.items = (long long)a.tiles * heads > sm_count() ? 2 : 1;
+    if (int rc = status_check()) return rc;
     if (int rc = status_word(&a.status)) return rc;
     a.polls = (unsigned)g_tune_tc_polls;
     a.scale_log2 = (1.0f / sqrtf((float)HD)) * 1.4426950408889634f;
@@ -297,7 +344,7 @@ static int ta_launch(const uint16_t* q, const void* kc, const void* vc, uint16_t
     LaunchCfg lc(grid, dim3(kTaThreads), Sh::kSmem, st, g_tune_pf_pdl != 0);
     SLLM_CUDA(cudaLaunchKernelEx(&lc.cfg, pf_attn_tc_kernel<HD>, tmQ, tmK, tmV, a));
     g_launches++;
-    SLLM_LAUNCH_CHECK();
+    SLLM_LAUNCH_CHECK_ONLY();
     return SLLM_OK;
 }
 

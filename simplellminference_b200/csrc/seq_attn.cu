@@ -525,7 +525,7 @@ int sllm::launch_attention_finish(const sllm_seq_batch* b, const float* ws, int 
     overlapping(seq_attention_finish_kernel)<<<b->T * heads, threads, (size_t)(nsplit + groups * dv) * sizeof(float), st>>>(*b, ws, nsplit, heads, dv, vfreq, layout, gate, ldg, gate_channels,
                                                                                                      sink, out, ldo, out16);
     ++g_launches;
-    SLLM_LAUNCH_CHECK();
+    SLLM_LAUNCH_CHECK_ONLY();
     return SLLM_OK;
 }
 
@@ -746,6 +746,7 @@ int sllm_seq_attention_out(const sllm_seq_batch* b, const float* q, int32_t ldq,
 int sllm_seq_attention_finish(const sllm_seq_batch* b, const float* ws, int32_t nsplit, int32_t heads, int32_t dv, const double* vfreq, int32_t layout,
                               const float* gate, int32_t ldg, int32_t gate_channels, const float* sink, float* out, int32_t ldo, void* out16,
                               sllm_stream_t stream) {
+    if (int rc = status_check()) return rc;
     return launch_attention_finish(b, ws, nsplit, heads, dv, vfreq, layout, gate, ldg, gate_channels, sink, out, ldo, (uint16_t*)out16, as_stream(stream));
 }
 

@@ -443,6 +443,7 @@ static int sa_launch(const AttnArgs& p, cudaStream_t st) {
     a.hpc = group % 4 == 0 ? 4 : group % 2 == 0 ? 2 : 1;
     a.hpc_log2 = a.hpc / 2;
     a.queries = kSaRows / a.hpc;
+    if (int rc = status_check()) return rc;
     if (int rc = status_word(&a.status)) return rc;
     a.polls = (unsigned)g_tune_tc_polls;
     a.vec_q = p.ldq % 4 == 0 && ((uintptr_t)p.q % 16) == 0;
@@ -455,7 +456,7 @@ static int sa_launch(const AttnArgs& p, cudaStream_t st) {
     if (int rc = tc_encode_bf16(&tmV, p.v_pool, 3, dims, strides, box)) return rc;
     kernel<<<dim3(p.b.n_qtiles, p.heads / a.hpc, p.nsplit), kSaThreads, Sh::kSmem, st>>>(tmK, tmV, a);
     ++g_launches;
-    SLLM_LAUNCH_CHECK();
+    SLLM_LAUNCH_CHECK_ONLY();
     return SLLM_OK;
 }
 
