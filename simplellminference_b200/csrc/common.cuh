@@ -149,6 +149,47 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
     return r;
 }
 
+// Index of the largest of n values (the first of equals), in thread 0 of a CTA of up to 1024 threads; NaN is never chosen, 0 if nothing is. Bound: what one SM reads; sixteen
+// bytes a load and eight loads on their way per thread (one value a load took 10.8 us for 32000 values).
+__device__ __forceinline__ void better_of(float& v, int& i, float ov, int oi) {
+    if (ov > v || (ov == v && oi < i)) { v = ov; i = oi; }
+}
+__device__ __forceinline__ int block_argmax(const float* x, int n, float* sv, int* si) {     // sv, si: 32 values of shared memory each
+    float v = -INFINITY;
+    int idx = 0x7fffffff;
+    const int body = (reinterpret_cast<uintptr_t>(x) & 15) ? 0 : n / 4;
+    constexpr int kAhead = 8;
+    for (int c = threadIdx.x; c < body; c += kAhead * blockDim.x) {
+        float4 q[kAhead];
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) {
+            const int at = c + k * (int)blockDim.x;
+            q[k] = at < body ? reinterpret_cast<const float4*>(x)[at] : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+        }
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) {
+            const int at = c + k * (int)blockDim.x;
+            if (at >= body) break;          // a value of -infinity may be the largest there is, but not one that stands in for nothing
+            better_of(v, idx, q[k].x, 4 * at);
+            better_of(v, idx, q[k].y, 4 * at + 1);
+            better_of(v, idx, q[k].z, 4 * at + 2);
+            better_of(v, idx, q[k].w, 4 * at + 3);
+        }
+    }
+    for (int i = 4 * body + threadIdx.x; i < n; i += blockDim.x) better_of(v, idx, x[i], i);
+    for (int o = 16; o > 0; o >>= 1) better_of(v, idx, __shfl_xor_sync(0xffffffffu, v, o), __shfl_xor_sync(0xffffffffu, idx, o));
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0) { sv[warp] = v; si[warp] = idx; }
+    __syncthreads();
+    if (warp == 0) {
+        const int nw = blockDim.x >> 5;
+        v = lane < nw ? sv[lane] : -INFINITY;
+        idx = lane < nw ? si[lane] : 0x7fffffff;
+        for (int o = 16; o > 0; o >>= 1) better_of(v, idx, __shfl_xor_sync(0xffffffffu, v, o), __shfl_xor_sync(0xffffffffu, idx, o));
+    }
+    return idx == 0x7fffffff ? 0 : idx;
+}
+
 // bf16 <-> fp32 by bit manipulation (RNE), identical to oracle/synth_weights.c:syn_round_bf16
 __device__ __forceinline__ float bf16_lo(uint32_t packed) { return __uint_as_float(packed << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t packed) { return __uint_as_float(packed & 0xffff0000u); }

@@ -95,28 +95,13 @@ __global__ void rope_kernel(float* __restrict__ q, float* __restrict__ k, const 
 
 // ------------------------------------------------------------------------------------------ argmax ----
 // first maximum (std::max_element, argmax.cpp:11): ties resolve to the lowest index.
-__device__ __forceinline__ void argmax_combine(float& v, int& i, float ov, int oi) {
-    if (ov > v || (ov == v && oi < i)) { v = ov; i = oi; }
-}
-__global__ void __launch_bounds__(1024) argmax_kernel(const float* __restrict__ logits, int n, int32_t* __restrict__ idx_out) {
+__global__ void __launch_bounds__(1024) argmax_kernel(const float* logits, int n, int32_t* idx_out) {
     __shared__ float sv[32];
     __shared__ int si[32];
     pdl_launch_dependents();
     pdl_wait();
-    float v = -INFINITY;
-    int idx = 0x7fffffff;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) argmax_combine(v, idx, logits[i], i);
-    for (int o = 16; o > 0; o >>= 1) argmax_combine(v, idx, __shfl_xor_sync(0xffffffffu, v, o), __shfl_xor_sync(0xffffffffu, idx, o));
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) { sv[warp] = v; si[warp] = idx; }
-    __syncthreads();
-    if (warp == 0) {
-        const int nw = blockDim.x >> 5;
-        v = lane < nw ? sv[lane] : -INFINITY;
-        idx = lane < nw ? si[lane] : 0x7fffffff;
-        for (int o = 16; o > 0; o >>= 1) argmax_combine(v, idx, __shfl_xor_sync(0xffffffffu, v, o), __shfl_xor_sync(0xffffffffu, idx, o));
-        if (lane == 0) *idx_out = (idx == 0x7fffffff) ? 0 : idx;
-    }
+    const int idx = block_argmax(logits, n, sv, si);
+    if (threadIdx.x == 0) *idx_out = idx;
 }
 
 // ------------------------------------------------------------------------------------ kv row store ----

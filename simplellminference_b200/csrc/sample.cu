@@ -137,21 +137,11 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(const float* __r
     }
 }
 
-__global__ void __launch_bounds__(1024) sample_argmax_kernel(const float* __restrict__ logits, int n, int32_t* __restrict__ idx_out) {
+__global__ void __launch_bounds__(1024) sample_argmax_kernel(const float* logits, int n, int32_t* idx_out) {
     __shared__ float sv[32];
     __shared__ int si[32];
-    float v = -INFINITY;
-    int idx = 0x7fffffff;
-    auto comb = [](float& a, int& ai, float b, int bi) { if (b > a || (b == a && bi < ai)) { a = b; ai = bi; } };
-    for (int i = threadIdx.x; i < n; i += blockDim.x) comb(v, idx, logits[i], i);
-    for (int o = 16; o > 0; o >>= 1) comb(v, idx, __shfl_xor_sync(0xffffffffu, v, o), __shfl_xor_sync(0xffffffffu, idx, o));
-    if ((threadIdx.x & 31) == 0) { sv[threadIdx.x >> 5] = v; si[threadIdx.x >> 5] = idx; }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        v = sv[threadIdx.x]; idx = si[threadIdx.x];
-        for (int o = 16; o > 0; o >>= 1) comb(v, idx, __shfl_xor_sync(0xffffffffu, v, o), __shfl_xor_sync(0xffffffffu, idx, o));
-        if (threadIdx.x == 0) *idx_out = (idx == 0x7fffffff) ? 0 : idx;
-    }
+    const int idx = block_argmax(logits, n, sv, si);
+    if (threadIdx.x == 0) *idx_out = idx;
 }
 
 }  // namespace sllm

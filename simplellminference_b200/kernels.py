@@ -11,8 +11,14 @@ from . import _lib
 from .config import F32, BF16, INT8
 
 
+# The handle of the current stream of the current device, without the Python object around it: building that took 3 us of a call's 11 (matmul, 256 x 256).
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    if _raw_stream is None or not torch.cuda.is_initialized():
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(torch._C._cuda_getDevice())
 
 
 def _p(t):
