@@ -13,7 +13,10 @@
 //   warp 5     (one lane) tcgen05.mma issuer: S = Q K^T, O += (hi + mid + lo) V with the weights read from TMEM, V MN-major as it lies;
 //   warp 6     zeros the value rows between the last position and the end of its box (the pool may hold anything there).
 // Bound: the fp32 work per score; the tensor pipe needs 1024 clocks per 128 x 64 scores at heads of 128. Caps and charges are applied in loops of
-// their own: with tanhf and log1pf inlined 64 times the code left the instruction cache (210 us where the loops take 81). Measured: attention_run.
+// their own: with tanhf and log1pf inlined 64 times the code left the instruction cache (210 us where the loops take 81). Two scores per instruction where there is one that
+// takes two, and scores within a quarter of a cap through the series alone: capped prompts of 1000, 311, 700 and 37 tokens, 16 heads over 4 of 128, 84 -> 65 us; the queries
+// and the results moved in batches 65 -> 58. Clocks of a tile there: capping 1300, weights 1000, maximum 400, waiting for the products 2000; beside 4000 before the first
+// and 6000 behind the last. Further figures: attention_run.
 #include "seq_attn_decode.cuh"
 #include "tcgen05.cuh"
 
@@ -200,13 +203,26 @@ __global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const _
         const int qpos = pos0 + qi;
         {   // the warp's 32 rows, one row (or two) per load so that neighbouring lanes read neighbouring columns
             constexpr int kLanes = HD / 4, kPer = 32 / kLanes;                  // lanes of a row, rows of a load
-#pragma unroll 16
-            for (int r0 = 0; r0 < 32; r0 += kPer) {
-                const int r = warp * 32 + r0 + lane / kLanes, col = (lane % kLanes) * 4;
-                const float* src = p.q + (size_t)(tok0 + min(r >> sa.hpc_log2, nq - 1)) * p.ldq + (size_t)(h0 + (r & (sa.hpc - 1))) * HD + col;
-                const float4 x = sa.vec_q ? *reinterpret_cast<const float4*>(src) : make_float4(src[0], src[1], src[2], src[3]);
-                *reinterpret_cast<uint2*>(sQ + (col / 64) * Sh::kQBlock + r * 128 + ((((col % 64) / 8) ^ (r & 7)) << 4) + (col % 8) * 2) =
-                    make_uint2(tc_pack(x.x, x.y), tc_pack(x.z, x.w));
+            // Sixteen loads on their way before the first of them is stored: left to itself the compiler keeps every load behind the store before it, since both could be
+            // the same memory, and the queries of a CTA took 11000 to 21000 clocks.
+            constexpr int kAhead = 16;
+            const int col = (lane % kLanes) * 4;
+#pragma unroll 1
+            for (int r0 = 0; r0 < 32; r0 += kPer * kAhead) {
+                float4 x[kAhead];
+#pragma unroll
+                for (int k = 0; k < kAhead; ++k) {
+                    const int r = warp * 32 + r0 + k * kPer + lane / kLanes;
+                    const float* src = p.q + (size_t)(tok0 + min(r >> sa.hpc_log2, nq - 1)) * p.ldq + (size_t)(h0 + (r & (sa.hpc - 1))) * HD + col;
+                    if (sa.vec_q) x[k] = *reinterpret_cast<const float4*>(src);
+                    else x[k] = make_float4(src[0], src[1], src[2], src[3]);
+                }
+#pragma unroll
+                for (int k = 0; k < kAhead; ++k) {
+                    const int r = warp * 32 + r0 + k * kPer + lane / kLanes;
+                    *reinterpret_cast<uint2*>(sQ + (col / 64) * Sh::kQBlock + r * 128 + ((((col % 64) / 8) ^ (r & 7)) << 4) + (col % 8) * 2) =
+                        make_uint2(tc_pack(x[k].x, x[k].y), tc_pack(x[k].z, x[k].w));
+                }
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             mb_arrive(qready);
@@ -281,8 +297,34 @@ __global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const _
             const bool all = __all_sync(0xffffffffu, j0 + kSaKeys - 1 <= qpos && (qpos - j0 < wnd || j0 + kSaKeys <= p.keep_first));
             if (kOpts && p.softcap > 0.0f) {
                 const float inv = p.scale / p.softcap;
+                const uint64_t inv2 = tc_two(__float_as_uint(inv), __float_as_uint(inv));
+                float top0 = 0.0f, top1 = 0.0f;
 #pragma unroll
-                for (int e = 0; e < 64; ++e) s[e] = __float_as_uint(p.softcap * sa_tanh(__uint_as_float(s[e]) * inv));
+                for (int e = 0; e < 64; e += 2) {
+                    float x, y;
+                    tc_split(tc_mul2(tc_two(s[e], s[e + 1]), inv2), x, y);
+                    s[e] = __float_as_uint(x);
+                    s[e + 1] = __float_as_uint(y);
+                    if (e & 2) top1 = tc_max3(top1, fabsf(x), fabsf(y));
+                    else top0 = tc_max3(top0, fabsf(x), fabsf(y));
+                }
+                // Scores within a quarter of the cap, as nearly all are: the series alone, two at a time. It is the one sa_tanh takes for them, so which of the two loops a tile
+                // goes through shows in no bit (NaN stays NaN in both).
+                if (__any_sync(0xffffffffu, fmaxf(top0, top1) >= 0.25f)) {
+#pragma unroll
+                    for (int e = 0; e < 64; ++e) s[e] = __float_as_uint(p.softcap * sa_tanh(__uint_as_float(s[e])));
+                } else {
+                    auto both = [](float v) { return tc_two(__float_as_uint(v), __float_as_uint(v)); };
+                    const uint64_t c4 = both(62.0f / 2835.0f), c3 = both(-17.0f / 315.0f), c2 = both(2.0f / 15.0f), c1 = both(-1.0f / 3.0f), c0 = both(1.0f), cap2 = both(p.softcap);
+#pragma unroll
+                    for (int e = 0; e < 64; e += 2) {
+                        const uint64_t x = tc_two(s[e], s[e + 1]), x2 = tc_mul2(x, x);
+                        float a, c;
+                        tc_split(tc_mul2(cap2, tc_mul2(x, tc_fma2(x2, tc_fma2(x2, tc_fma2(x2, tc_fma2(x2, c4, c3), c2), c1), c0))), a, c);
+                        s[e] = __float_as_uint(a);
+                        s[e + 1] = __float_as_uint(c);
+                    }
+                }
             } else if (!plain) {
 #pragma unroll
                 for (int e = 0; e < 64; ++e) s[e] = __float_as_uint(__uint_as_float(s[e]) * p.scale);
@@ -302,13 +344,10 @@ __global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const _
                 for (int e = 0; e < 64; ++e)
                     if (!seq_sees(qpos, j0 + e, wnd, p.keep_first)) s[e] = 0xff800000u;       // -inf
             }
-            float m0 = -INFINITY, m1 = -INFINITY;
+            float m[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-            for (int e = 0; e < 64; e += 2) {
-                m0 = fmaxf(m0, __uint_as_float(s[e]));
-                m1 = fmaxf(m1, __uint_as_float(s[e + 1]));
-            }
-            const float mx = fmaxf(m0, m1) * mul;
+            for (int e = 0; e < 64; e += 2) m[(e / 2) & 3] = tc_max3(m[(e / 2) & 3], __uint_as_float(s[e]), __uint_as_float(s[e + 1]));
+            const float mx = tc_max3(fmaxf(m[0], m[1]), m[2], m[3]) * mul;
             if (i % kSaFlush == 0 && i > 0) {           // the product before this tile has completed: these scores follow it
                 if (live && i > kSaFlush) prefetch_flushed();
 #pragma unroll 1
@@ -338,25 +377,35 @@ __global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const _
                     tc_st16(o_tmem + c, o);
                 }
             }
-            float l0 = 0.0f, l1 = 0.0f;
+            uint64_t sum = 0;                                                   // (0, 0)
             const float from = ref == -INFINITY ? 0.0f : ref;                   // nothing seen yet: every weight is exp(-inf) = 0
+            const uint64_t mul2 = tc_two(__float_as_uint(mul), __float_as_uint(mul)), from2 = tc_two(__float_as_uint(-from), __float_as_uint(-from));
+            const uint64_t less = tc_two(__float_as_uint(-1.0f), __float_as_uint(-1.0f));
+            auto terms = [](uint32_t w) { return tc_two(w << 16, w & 0xffff0000u); };
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
                 uint32_t hi[16], mid[16], lo[16];
 #pragma unroll
                 for (int e = 0; e < 16; ++e) {
-                    const float x = tc_exp2(fmaf(__uint_as_float(s[half * 32 + 2 * e]), mul, -from)), y = tc_exp2(fmaf(__uint_as_float(s[half * 32 + 2 * e + 1]), mul, -from));
-                    l0 += x;
-                    l1 += y;
+                    float x, y;
+                    tc_split(tc_fma2(tc_two(s[half * 32 + 2 * e], s[half * 32 + 2 * e + 1]), mul2, from2), x, y);
+                    x = tc_exp2(x);
+                    y = tc_exp2(y);
+                    const uint64_t w = tc_two(__float_as_uint(x), __float_as_uint(y));
+                    sum = tc_add2(sum, w);
                     hi[e] = tc_pack(x, y);
-                    const float rx = x - __uint_as_float(hi[e] << 16), ry = y - __uint_as_float(hi[e] & 0xffff0000u);
-                    mid[e] = tc_pack(rx, ry);
-                    lo[e] = tc_pack(rx - __uint_as_float(mid[e] << 16), ry - __uint_as_float(mid[e] & 0xffff0000u));
+                    const uint64_t r = tc_fma2(terms(hi[e]), less, w);          // what the first terms leave: exact
+                    tc_split(r, x, y);
+                    mid[e] = tc_pack(x, y);
+                    tc_split(tc_fma2(terms(mid[e]), less, r), x, y);
+                    lo[e] = tc_pack(x, y);
                 }
                 tc_st16(s_tmem + half * 16, hi);
                 tc_st16(s_tmem + 32 + half * 16, mid);
                 tc_st16(s_tmem + 64 + half * 16, lo);
             }
+            float l0, l1;
+            tc_split(sum, l0, l1);
             l += l0 + l1;
             tc_wait_st();
             tc_fence_before();
@@ -409,12 +458,17 @@ __global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const _
 #pragma unroll
                 for (int e = 0; e < 32; ++e) mine[lane * 33 + e] = __uint_as_float(o[e]);
                 __syncwarp();
-#pragma unroll 8
-                for (int r = 0; r < 32; ++r)
-                    if (r < rows) {
-                        const int rr = warp * 32 + r;
-                        to[(size_t)(uint32_t)((rr >> sa.hpc_log2) * step_q + (rr & (sa.hpc - 1)) * step_h + c)] = mine[r * 33 + lane];
+#pragma unroll 1
+                for (int r0 = 0; r0 < rows; r0 += 16) {                        // sixteen rows read before the first is stored, as above
+                    float x[16];
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) x[k] = mine[(r0 + k) * 33 + lane];
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) {
+                        const int rr = warp * 32 + r0 + k;
+                        if (r0 + k < rows) to[(size_t)(uint32_t)((rr >> sa.hpc_log2) * step_q + (rr & (sa.hpc - 1)) * step_h + c)] = x[k];
                     }
+                }
             }
             __syncwarp();
         }

@@ -79,3 +79,14 @@ def test_sums_over_long_contexts(segs, heads, kv_heads, dim, nsplit):
     for _, n in segs:        # each portion by itself: the norms of long contexts' results are small
         assert _close(out[at:at + n], want[at:at + n], 4e-6)
         at += n
+
+
+@pytest.mark.parametrize("cap", [0.5, 9.0, 14.0, 60.0])
+@pytest.mark.parametrize("heads,kv_heads,dim", [(8, 2, 64), (3, 3, 128), (8, 2, 128)])
+def test_portions_with_caps_near_and_far_from_the_scores(heads, kv_heads, dim, cap):
+    """Scores of up to about five: all tiles beyond a quarter of the cap, some, hardly any, none (the two loops of the capped body)."""
+    segs = [(0, 500), (130, 333), (700, 40)]
+    q, k, v, rows, b, keep = _inputs(segs, heads, kv_heads, dim, 64)
+    ops = _ops()
+    want = _want(q, rows, segs, heads, kv_heads, dim, dim ** -0.5, softcap=cap)
+    assert _close(_run(ops, b, q, k, v, heads, kv_heads, dim, ops.attention_options(softcap=cap)), want, 4e-6)
