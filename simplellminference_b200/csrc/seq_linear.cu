@@ -22,7 +22,7 @@ struct LinArgs {
     const int32_t* w_index;    // rows body, device memory or NULL: product b of the batch uses matrix w_index[b] (W + w_index[b] * w_bs); -1 = no matrix, zeros
     int a_div;                 // rows body: product b reads the activations of batch element b / a_div (0 or 1: its own)
     int rows_bs;               // tile body: 1 = a row count per product of the batch
-    int w_fixed;               // rows bodies: no kernel enqueued shortly before writes W, its first rows are asked for before the wait for those kernels
+    int w_fixed;               // rows bodies: no kernel of the same captured graph writes W, whose first rows are asked for before the wait for the kernel in front (and for all before it)
 };
 
 constexpr int kRowsMax = 8;
@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(256, 4) seq_linear_rows_small_kernel(LinArgs p
 #pragma unroll
                 for (int j = 0; j < kInFlight; ++j) {
                     const int k = k0 + j * 32 * E;
-                    u[j] = k < k_hi ? ldg_stream(w + (size_t)k * (16 / E)) : make_uint4(0u, 0u, 0u, 0u);
+                    u[j] = k < k_hi ? ld_stream(w + (size_t)k * (16 / E)) : make_uint4(0u, 0u, 0u, 0u);     // W may be the work of the kernel in front
                 }
             };
             auto consume = [&](const uint4 (&u)[kInFlight], int k0) {

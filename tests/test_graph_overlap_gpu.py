@@ -76,6 +76,55 @@ def test_weights_written_by_the_graph_itself():
         assert torch.equal(have, out) and torch.equal(far * 2, out) and not torch.equal(have, want)
 
 
+@pytest.mark.parametrize("N,K", [(256, 2048), (250, 1000), (96, 510)], ids=["whole-warps", "ragged", "single-values"])
+@pytest.mark.parametrize("T", [1, 8])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_small_matrices_written_by_the_kernel_in_front(dtype, T, N, K):
+    """Below 1.5 million weights, where the products go through the body for small matrices. fp32: written, then added to, by tiles of 64 x 64, so that CTAs side by side
+    write parts of the same rows; bf16: the rows of a norm."""
+    import torch
+    from simplellminference_b200.config import BF16, F32
+    from simplellminference_b200.seqops import Ops
+    ops = Ops(F32 if dtype == "float32" else BF16)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(K + T)
+    a, x = torch.randn(T, K, generator=g, device="cuda"), torch.randn(N, K, generator=g, device="cuda")
+    w1, ones = torch.randn(K, K, generator=g, device="cuda") / K ** 0.5, torch.ones(K, device="cuda")
+    mid, y = torch.zeros(N, K, device="cuda", dtype=getattr(torch, dtype)), torch.zeros(N, K, device="cuda")
+    out = torch.zeros(T, N, device="cuda")
+
+    def step(st):
+        if dtype == "float32":
+            ops.linear(x.data_ptr(), K, w1, K, None, mid.data_ptr(), K, N, K, K, st)
+            ops.linear(x.data_ptr(), K, w1, K, None, mid.data_ptr(), K, N, K, K, st, accumulate=True)
+        else:
+            ops.layernorm(x, K, ones, None, 1e-5, y, K, N, K, st, y16=mid)
+        ops.linear(a.data_ptr(), K, mid, K, None, out.data_ptr(), N, T, N, K, st)
+        ops.linear(a.data_ptr(), K, mid, K, None, out.data_ptr(), N, T, N, K, st, accumulate=True)
+
+    step(torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        step(torch.cuda.current_stream().cuda_stream)
+    assert ops.overlap(graph.raw_cuda_graph()) == (3 if dtype == "float32" else 2)
+    graph.instantiate()
+    for seed in (2, 3, 4):
+        g.manual_seed(seed)
+        x.copy_(torch.randn(N, K, generator=g, device="cuda"))
+        mid.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        have = out.clone()
+        out.fill_(float("nan"))
+        mid.fill_(float("nan"))
+        step(torch.cuda.current_stream().cuda_stream)
+        assert torch.equal(have, out) and bool(torch.isfinite(out).all()), seed
+        # sums of K products in another order, doubled; operands as the kernel takes them (bf16: both rounded to it)
+        rows = a.to(torch.bfloat16).double() if dtype == "bfloat16" else a.double()
+        assert float((out.double() - 2 * rows @ mid.double().T).norm() / out.double().norm()) < 1e-6
+
+
 def test_no_graph_is_refused():
     from simplellminference_b200.config import F32
     from simplellminference_b200.seqops import Ops
