@@ -77,13 +77,29 @@ static bool overlap_find(const void* kernel, bool add) {
     return false;                             // a full table: this kernel's edges stay as they are
 }
 void overlap_kernel(const void* kernel) { overlap_find(kernel, true); }
-static bool overlaps(cudaGraphNode_t node) {
+static bool quiet(cudaError_t e) {               // a refusal that is no error of the caller's
+    if (e != cudaSuccess) cudaGetLastError();
+    return e == cudaSuccess;
+}
+// The edge in front of one node: 1 = programmatic now; 0 = as it was, being of another kind or because the runtime will not exchange it; -1 = lost.
+static int overlap_edge(cudaGraph_t g, cudaGraphNode_t node) {
+    cudaGraphNodeType type;
+    if (!quiet(cudaGraphNodeGetType(node, &type)) || type != cudaGraphNodeTypeKernel) return 0;
     cudaKernelNodeParams p{};
-    if (cudaGraphKernelNodeGetParams(node, &p) != cudaSuccess) {   // another library's kernel
-        cudaGetLastError();
-        return false;
-    }
-    return overlap_find(p.func, false);
+    if (!quiet(cudaGraphKernelNodeGetParams(node, &p)) || !overlap_find(p.func, false)) return 0;     // another library's kernel, or one that does not wait
+    // One predecessor, a kernel: this node's own wait takes the place of the edge. Joins of several branches keep theirs (a step of Nelutar measured the same with
+    // those converted too).
+    size_t deps = 0;
+    if (!quiet(cudaGraphNodeGetDependencies_v2(node, nullptr, nullptr, &deps)) || deps != 1) return 0;
+    cudaGraphNode_t from = nullptr;
+    cudaGraphEdgeData edge{}, early{};
+    if (!quiet(cudaGraphNodeGetDependencies_v2(node, &from, &edge, &deps)) || !quiet(cudaGraphNodeGetType(from, &type))) return 0;
+    if (type != cudaGraphNodeTypeKernel || edge.type != cudaGraphDependencyTypeDefault || edge.from_port != cudaGraphKernelNodePortDefault) return 0;
+    early.type = cudaGraphDependencyTypeProgrammatic;
+    early.from_port = cudaGraphKernelNodePortProgrammatic;
+    if (!quiet(cudaGraphRemoveDependencies_v2(g, &from, &node, &edge, 1))) return 0;
+    if (quiet(cudaGraphAddDependencies_v2(g, &from, &node, &early, 1))) return 1;
+    return quiet(cudaGraphAddDependencies_v2(g, &from, &node, &edge, 1)) ? 0 : -1;
 }
 
 int sm_count() {
@@ -146,24 +162,9 @@ int sllm_graph_overlap(void* graph, int32_t* edges) {
     std::vector<cudaGraphNode_t> nodes(n);
     SLLM_CUDA(cudaGraphGetNodes(g, nodes.data(), &n));
     for (size_t i = 0; i < n; ++i) {
-        cudaGraphNodeType type;
-        SLLM_CUDA(cudaGraphNodeGetType(nodes[i], &type));
-        if (type != cudaGraphNodeTypeKernel || !overlaps(nodes[i])) continue;
-        // One predecessor, a kernel: this node's own wait takes the place of the edge. Joins of several branches keep theirs (a step of Nelutar measured the same with
-        // those converted too).
-        size_t deps = 0;
-        SLLM_CUDA(cudaGraphNodeGetDependencies_v2(nodes[i], nullptr, nullptr, &deps));
-        if (deps != 1) continue;
-        cudaGraphNode_t from = nullptr;
-        cudaGraphEdgeData edge{}, early{};
-        SLLM_CUDA(cudaGraphNodeGetDependencies_v2(nodes[i], &from, &edge, &deps));
-        SLLM_CUDA(cudaGraphNodeGetType(from, &type));
-        if (type != cudaGraphNodeTypeKernel || edge.type != cudaGraphDependencyTypeDefault || edge.from_port != cudaGraphKernelNodePortDefault) continue;
-        early.type = cudaGraphDependencyTypeProgrammatic;
-        early.from_port = cudaGraphKernelNodePortProgrammatic;
-        SLLM_CUDA(cudaGraphRemoveDependencies_v2(g, &from, &nodes[i], &edge, 1));
-        SLLM_CUDA(cudaGraphAddDependencies_v2(g, &from, &nodes[i], &early, 1));
-        ++changed;
+        const int done = overlap_edge(g, nodes[i]);
+        SLLM_REQUIRE(done >= 0, SLLM_ESTATE, "graph_overlap: the runtime took an edge and would not have it back; the graph has to be captured again");
+        changed += done;
     }
     if (edges) *edges = changed;
     return SLLM_OK;

@@ -296,18 +296,17 @@ class SequenceEngine:
             entry = self._graphs[key]
             if entry is None:                               # second step of this kind: capture it (a capture does not execute)
                 meta_addr = self._meta_dev.data_ptr()
-                g = torch.cuda.CUDAGraph(keep_graph=True)
+                def forward():
+                    step.turned.clear()
+                    step.st = torch.cuda.current_stream(self.device).cuda_stream
+                    return self.model.forward(step, ids_t, self.states, rows_t, n_rows)
                 collecting = gc.isenabled()
                 gc.disable()        # a finaliser that frees device memory (another engine's graphs, say) must not run inside the capture
                 try:
-                    with torch.cuda.graph(g):
-                        step.st = torch.cuda.current_stream(self.device).cuda_stream
-                        out = self.model.forward(step, ids_t, self.states, rows_t, n_rows)
+                    g, out = _captured(self.ops, forward)
                 finally:
                     if collecting:
                         gc.enable()
-                self.ops.overlap(g.raw_cuda_graph())
-                g.instantiate()
                 entry = self._graphs[key] = (g, out, meta_addr, p[0], p[9])
             g, logits, meta_addr, ids_addr, rows_addr = entry
             if meta_addr != self._meta_dev.data_ptr() or ids_addr != p[0] or rows_addr != p[9]:
@@ -324,6 +323,27 @@ class SequenceEngine:
             self.last_token[slot] = int(toks[-1])
         self.steps_run += 1
         return logits
+
+
+def _captured(ops, launch):
+    """A graph of what ``launch()`` enqueues, ready to replay, and what it returns. Its kernels overlap (``ops.overlap``) where the runtime allows that; where it does not,
+    or torch cannot hand out a graph before it is instantiated, the plain graph does."""
+    for overlap in (True, False):
+        try:
+            g = torch.cuda.CUDAGraph(keep_graph=True) if overlap else torch.cuda.CUDAGraph()
+        except TypeError:
+            continue
+        with torch.cuda.graph(g):
+            out = launch()
+        if not overlap:
+            break
+        try:
+            ops.overlap(g.raw_cuda_graph())
+            g.instantiate()
+            break
+        except RuntimeError:        # its edges may be incomplete: once more without
+            del g
+    return g, out
 
 
 class _PtrView:

@@ -1,0 +1,112 @@
+"""sllm_graph_overlap where the runtime refuses: an edge that cannot be exchanged stays what it was and is not counted, a lost one is reported; and the capture of a step
+that goes on with a plain graph then. The library's own code against a stand-in for the runtime's graph calls (tests/cpp/fake_graph_runtime.c), in a process of its own."""
+import contextlib
+import os
+import subprocess
+import sys
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+LIB = os.path.join(ROOT, "simplellminference_b200", "lib", "libsllm_b200.so")
+
+CHILD = """
+import ctypes as C, sys
+fake = C.CDLL(sys.argv[1], mode=C.RTLD_GLOBAL)          # in front of the runtime's own symbols
+lib = C.CDLL(sys.argv[2])
+add = getattr(lib, "_ZN4sllm14overlap_kernelEPKv")
+add.argtypes = [C.c_void_p]
+for kernel in (2, 3, 4, 6):                              # node 5's kernel is not one that waits
+    add(kernel << 8)
+lib.sllm_graph_overlap.argtypes = [C.c_void_p, C.c_void_p]
+fake.fake_reset(6, *map(int, sys.argv[3:7]))
+n = C.c_int32(-7)
+rc = lib.sllm_graph_overlap(1, C.byref(n))
+print(rc, n.value, *[fake.fake_edge(i) for i in range(2, 7)])
+"""
+
+
+@pytest.mark.parametrize("look,remove,add,add_from,want", [
+    (0, 0, 0, 0, [0, 4, 2, 2, 2, 1, 2]),            # nothing fails: nodes 2, 3, 4 and 6
+    (2, 0, 0, 0, [0, 3, 1, 2, 2, 1, 2]),            # the first node's edge cannot be looked at
+    (0, 2, 0, 0, [0, 3, 2, 1, 2, 1, 2]),            # the second removal is refused
+    (0, 0, 1, 0, [0, 3, 1, 2, 2, 1, 2]),            # the first programmatic edge is refused and the ordinary one put back
+    (0, 0, 3, 0, [0, 3, 2, 2, 1, 1, 2]),
+    (0, 0, 0, 2, [-4, -7, 2, 0, 1, 1, 1]),          # from the second on none can be added, nor put back: reported
+])
+def test_refused_edges(tmp_path, look, remove, add, add_from, want):
+    if not os.path.exists(LIB):
+        pytest.skip("library not built")
+    fake = str(tmp_path / "libfake.so")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-Wall", "-Werror", "-I/usr/local/cuda/include", "-o", fake, os.path.join(ROOT, "tests", "cpp", "fake_graph_runtime.c")], check=True)
+    out = subprocess.run([sys.executable, "-c", CHILD, fake, LIB, *map(str, (look, remove, add, add_from))], capture_output=True, text=True)
+    assert out.returncode == 0, out.stderr
+    assert [int(x) for x in out.stdout.split()] == want
+
+
+class _Graph:
+    made = []
+
+    def __init__(self, keep_graph=False):
+        self.keep, self.instantiated = keep_graph, not keep_graph
+        _Graph.made.append(self)
+
+    def raw_cuda_graph(self):
+        assert self.keep
+        return 1
+
+    def instantiate(self):
+        self.instantiated = True
+
+
+class _PlainGraph(_Graph):
+    """As of a torch that does not hand graphs out."""
+    def __init__(self):
+        super().__init__()
+
+
+class _Ops:
+    def __init__(self, error=None):
+        self.error, self.asked = error, 0
+
+    def overlap(self, graph):
+        self.asked += 1
+        if self.error:
+            raise self.error
+
+
+@pytest.mark.parametrize("case", ["overlaps", "refused", "not-instantiated", "old-torch"])
+def test_a_step_is_captured_either_way(monkeypatch, case):
+    import torch
+    from simplellminference_b200 import _lib, seqengine
+    _Graph.made = []
+    kind = _PlainGraph if case == "old-torch" else _Graph
+    monkeypatch.setattr(torch.cuda, "CUDAGraph", kind)
+    monkeypatch.setattr(torch.cuda, "graph", lambda g: contextlib.nullcontext())
+    if case == "not-instantiated":
+        def refuse(self):
+            raise RuntimeError("CUDA error: operation not supported")
+        monkeypatch.setattr(_Graph, "instantiate", refuse)
+    ops, launches = _Ops(_lib.SllmError(_lib.ESTATE, "lost") if case == "refused" else None), []
+
+    def launch():
+        launches.append(1)
+        return len(launches)
+
+    g, out = seqengine._captured(ops, launch)
+    again = case in ("refused", "not-instantiated")
+    assert len(launches) == (2 if again else 1) and out == len(launches)
+    assert g is _Graph.made[-1] and g.instantiated and g.keep == (case == "overlaps")
+    assert ops.asked == (0 if case == "old-torch" else 1)
+
+
+def test_errors_of_the_step_itself_are_not_swallowed(monkeypatch):
+    import torch
+    from simplellminference_b200 import seqengine
+    monkeypatch.setattr(torch.cuda, "CUDAGraph", _Graph)
+    monkeypatch.setattr(torch.cuda, "graph", lambda g: contextlib.nullcontext())
+
+    def launch():
+        raise RuntimeError("the step")
+    with pytest.raises(RuntimeError, match="the step"):
+        seqengine._captured(_Ops(), launch)

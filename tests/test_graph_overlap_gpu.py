@@ -37,6 +37,33 @@ def test_captured_steps_equal_direct_ones(tmp_path, dtype, requests):
         assert (a == b).all()
 
 
+def test_a_step_whose_edges_are_refused_is_captured_without(tmp_path):
+    from simplellminference_b200 import _lib
+    from simplellminference_b200.models import build_model
+    from simplellminference_b200.seqengine import SequenceEngine
+    cfg = L.make_config([L.lightning_pair(), L.delta_pair(mlp=L.moe())])
+    path = L.write_model(str(tmp_path / "m"), cfg, L.random_weights(cfg, seed=3))
+    got = []
+    for refuse in (False, True):
+        model = build_model(path, "float32", "cuda")
+        if refuse:
+            plain = model.ops.overlap
+
+            def lose(graph):
+                plain(graph)
+                raise _lib.SllmError(_lib.ESTATE, "an edge is lost")
+            model.ops.overlap = lose
+        eng = SequenceEngine(model, max_tokens=64, max_seqs=2, page_len=32)
+        slot = eng.admit()
+        rows = [eng.run([(slot, [5, 6, 7], [2])]).clone()]
+        for k in range(6):
+            rows.append(eng.run([(slot, [8 + k], [0])]).clone())
+        assert eng.graph_replays >= 4
+        got.append(rows)
+    for a, b in zip(*got):
+        assert (a == b).all()
+
+
 def test_weights_written_by_the_graph_itself():
     import torch
     from simplellminference_b200.config import F32
