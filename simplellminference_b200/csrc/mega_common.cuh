@@ -28,14 +28,14 @@ struct MegaSmem {
     int att_tile;   // cache positions per K/V stage: 64, or 32 when a row is wider than 256 bytes (fp32 cache with 128-wide heads), so that
                     // two K and two V stages always fit in 64 KB next to the weight rings
 };
-__host__ __device__ inline int mega_att_tile(int hd, int kv_esz) { return hd * kv_esz > 256 ? kAttTile / 2 : kAttTile; }
+__host__ __device__ constexpr int mega_att_tile(int hd, int kv_esz) { return hd * kv_esz > 256 ? kAttTile / 2 : kAttTile; }
 __host__ __device__ inline int mega_kv_stride(int row_bytes) {
     int s = (row_bytes / 128) * 128 + 32;
     if (s < row_bytes) s += 128;
     return s;
 }
-__host__ __device__ inline MegaSmem mega_smem_layout(int hd, int g, int kv_esz) {
-    MegaSmem L;
+__host__ __device__ constexpr MegaSmem mega_smem_layout(int hd, int g, int kv_esz) {
+    MegaSmem L{};
     size_t off = 0;
     L.bars = off; off += 512;
     L.red = off; off += 256;

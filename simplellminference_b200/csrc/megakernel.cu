@@ -44,7 +44,9 @@ __device__ __forceinline__ unsigned long long gtime() {
         if (p.trace && threadIdx.x == 0 && (ev) < kTraceEvents) p.trace[((size_t)blockIdx.x * kTraceEvents + (ev)) * 8 + (slot)] = gtime(); \
     } while (0)
 
-constexpr int kPhaseCache = 56;   // as many as fit beside the largest plan (8 query heads per kv head of 256)
+constexpr int kPhaseCache = 56;   // phase descriptors kept in shared memory: 14 layers; deeper models read the rest from global memory
+constexpr size_t kMegaStatic = sizeof(PhaseDesc) * kPhaseCache + 128;   // the kernel's static shared memory: descriptors, a word, up to the next 128 bytes
+static_assert(mega_smem_layout(128, 8, 2).total + kMegaStatic <= 227 * 1024, "the largest plan and the kernel's static shared memory fit an SM together");
 
 // FUSE (experimental, SLLM_ENGINE_MEGA_FUSE_DOWN): the down projection runs inside the gate_up phase's CTA as a K-split over the
 // values that CTA produced (megakernel.cuh "PH_DOWN_T"): four grid barriers per layer instead of five, no staging of swi.
@@ -705,7 +707,7 @@ MegaPlan mega_plan_for(int sms, int smem_optin, int w_dtype, int group, int kv_d
     const int kesz = kv_dtype == SLLM_F32 ? 4 : 2;
     if ((hd * kesz / 16) > 32) { pl.why = "head_dim chunking"; return pl; }
     const MegaSmem SL = mega_smem_layout(hd, g, kesz);
-    if (SL.total > (size_t)smem_optin) { pl.why = "shared memory"; return pl; }
+    if (SL.total + kMegaStatic > (size_t)smem_optin) { pl.why = "shared memory"; return pl; }
     if ((size_t)16 * g * hd * 4 > (size_t)4 * SL.att_tile * SL.kv_stride) { pl.why = "attention scratch"; return pl; }   // the cross-stripe reduction buffer spans the (drained, contiguous) K and V stages
     if ((size_t)std::max(d, I_loc) * 4 > (size_t)4 * SL.att_tile * SL.kv_stride) { pl.why = "activation staging"; return pl; }
     if (q_loc % 2 || kv_loc % 2) { pl.why = "odd dims"; return pl; }

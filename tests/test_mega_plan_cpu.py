@@ -145,3 +145,16 @@ def test_tile_geometry_rejects_bad_arguments():
     assert lib.sllm_mega_tile_geometry(0, 4096, 0, BF16, None, None, None, None, None, None) != 0
     assert lib.sllm_mega_tile_geometry(16, 4100, 0, BF16, None, None, None, None, None, None) != 0     # not whole 16-byte chunks
     assert lib.sllm_mega_tile_geometry(16, 4096, 7, BF16, None, None, None, None, None, None) != 0
+
+
+@pytest.mark.parametrize("kvd,hd,group", [(BF16, 128, 8), (BF16, 256, 4), (F32, 128, 1)])
+def test_plan_counts_the_kernels_static_shared_memory(kvd, hd, group):
+    """The largest plan, the widest heads, a small one. The descriptors of 56 phases of 64 bytes and a word, rounded up to 128 bytes, lie beside the dynamic part."""
+    static = 56 * 64 + 128
+    ms = dataclasses.replace(PRESETS["llama2-7b"], head_dim=hd, hidden=group * hd, heads=group, kv_heads=1, kv_hidden=hd, inter=2048)
+    ok, _, nbytes, _, why = plan(ms, BF16, kvd)
+    assert ok and nbytes + static <= B200_SMEM, why
+    assert plan(ms, BF16, kvd, smem=nbytes + static)[0]
+    for short in (nbytes + static - 1, nbytes):
+        ok, _, _, _, why = plan(ms, BF16, kvd, smem=short)
+        assert not ok and "shared memory" in why
