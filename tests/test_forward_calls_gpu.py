@@ -9,16 +9,21 @@ from simplellminference_b200.engine import Engine
 pytestmark = pytest.mark.gpu
 
 MODES = {"mega": dict(mega=True), "mega_v2": dict(mega=True, mega_v2=True), "mega_v2_fuse": dict(mega=True, mega_v2=True, mega_fuse_down=True)}
-# (shape, weights): one kv head, 16 splits of it, eight query heads; 8 kv heads, 16 splits; more heads than one pass of the merge has threads for
-SHAPES = [(ModelShape(320, 32, 256, 32, 512, 1024, 2, 8, 1), F32), (ModelShape(512, 64, 512, 512, 768, 1024, 2, 8, 8), INT8),
-          (ModelShape(512, 64, 1024, 512, 512, 1024, 2, 16, 8), BF16), (ModelShape(300, 128, 2048, 256, 256, 600, 1, 16, 2), F32)]
+V1, V1F, V2, V2F = "megakernel", "megakernel(fused-down)", "megakernel(v2)", "megakernel(v2,fused-down)"
+# (shape, weights, the kernel each mode gets: the one with per-head counters takes neither int8 weights nor kv head groups of more than 128 16-byte
+# chunks, nor the largest plans): one kv head,
+# 16 splits of it, eight query heads; 8 kv heads, 16 splits; two query heads a kv head; a merge whose pieces are as many as its threads; one with twice as many, 9 splits
+SHAPES = [(ModelShape(320, 32, 256, 32, 512, 1024, 2, 8, 1), F32, (V1, V2, V2F)), (ModelShape(512, 64, 512, 512, 768, 1024, 2, 8, 8), INT8, (V1, V1, V1)),
+          (ModelShape(512, 64, 1024, 512, 512, 1024, 2, 16, 8), BF16, (V1, V2, V2F)), (ModelShape(300, 128, 2048, 256, 256, 600, 1, 16, 2), F32, (V1, V1, V1F)),
+          (ModelShape(300, 128, 4096, 512, 512, 576, 1, 32, 4), BF16, (V1, V1, V1F))]
 
 
 @pytest.mark.parametrize("mode", list(MODES))
-@pytest.mark.parametrize("shape,wd", SHAPES)
-def test_calls_follow_a_greedy_run(mode, shape, wd):
+@pytest.mark.parametrize("shape,wd,kernels", SHAPES)
+def test_calls_follow_a_greedy_run(mode, shape, wd, kernels):
     kw = dict(w_dtype=wd, kv_dtype=F32, group=64)
     a = Engine(shape, **kw, **MODES[mode]).load_synthetic(5)
+    assert a.mode == kernels[list(MODES).index(mode)], a.mode
     b = Engine(shape, **kw).load_synthetic(5)             # the kernels of one op each, in a graph
     prompt, n = np.arange(1, 40, dtype=np.int32), 90
     want = b.greedy(prompt, n)
