@@ -56,9 +56,10 @@ const char* sllm_last_error(void);
  * needs this only behind a synchronisation of its own. */
 int sllm_status(void);
 /* Turns edges of a captured graph (cudaGraph_t, not yet instantiated) into programmatic ones: a kernel of this library that waits for its predecessor itself, and has
- * one predecessor, a kernel, may become resident while that one still runs. What it reads and writes behind that wait, and so every result, is the same. *edges (or
- * NULL): how many were changed. An edge that the runtime will not exchange stays as it was; SLLM_ESTATE: one could not be put back either, and the graph must not
- * be used. */
+ * one predecessor, a kernel that nothing else follows, may become resident while that one still runs. What it reads and writes behind that wait, and so every result, is
+ * the same. Left as they are: all edges of nodes beside which the graph has a parallel branch; programmatic edges that the
+ * capture has made from one branch to another become ordinary ones. *edges (or NULL): how many were made programmatic. An edge that the runtime will not exchange stays as it was, and so does a graph it will not describe; SLLM_ESTATE: an edge could not be put back either, and
+ * the graph must not be used. */
 int sllm_graph_overlap(void* graph, int32_t* edges);
 int sllm_abi_version(void);
 /* development knobs (not part of the drop-in surface): key 0 = GEMV CTAs per SM (0 = built-in choice); prefill GEMM: key 1 = force

@@ -3,6 +3,7 @@
 #include <cstdarg>
 #include <cstring>
 #include <mutex>
+#include <unordered_map>
 #include <vector>
 
 #include "common.cuh"
@@ -64,42 +65,125 @@ int status_take() {
 }
 
 // Kernels launched through overlapping(): a set that only grows, to at most as many as the library has instantiations; looked up on every launch, so without a lock.
-static constexpr size_t kOverlapSlots = 1024;
-static std::atomic<const void*> g_overlap[kOverlapSlots];
-static bool overlap_find(const void* kernel, bool add) {
-    for (size_t i = reinterpret_cast<uintptr_t>(kernel) >> 4, n = 0; n < kOverlapSlots; ++i, ++n) {
-        std::atomic<const void*>& slot = g_overlap[i % kOverlapSlots];
-        const void* held = slot.load(std::memory_order_acquire);
-        if (held == nullptr && add && slot.compare_exchange_strong(held, kernel, std::memory_order_acq_rel)) return true;
-        if (held == kernel) return true;      // compare_exchange has left what another thread put there
-        if (held == nullptr && !add) return false;
+struct KernelSet {
+    static constexpr size_t kSlots = 1024;
+    std::atomic<const void*> slots[kSlots];
+    bool find(const void* kernel, bool add) {
+        for (size_t i = reinterpret_cast<uintptr_t>(kernel) >> 4, n = 0; n < kSlots; ++i, ++n) {
+            std::atomic<const void*>& slot = slots[i % kSlots];
+            const void* held = slot.load(std::memory_order_acquire);
+            if (held == nullptr && add && slot.compare_exchange_strong(held, kernel, std::memory_order_acq_rel)) return true;
+            if (held == kernel) return true;      // compare_exchange has left what another thread put there
+            if (held == nullptr && !add) return false;
+        }
+        return false;                             // a full table: this kernel's edges stay as they are
     }
-    return false;                             // a full table: this kernel's edges stay as they are
-}
-void overlap_kernel(const void* kernel) { overlap_find(kernel, true); }
+};
+static KernelSet g_overlap;
+void overlap_kernel(const void* kernel) { g_overlap.find(kernel, true); }
 static bool quiet(cudaError_t e) {               // a refusal that is no error of the caller's
     if (e != cudaSuccess) cudaGetLastError();
     return e == cudaSuccess;
 }
-// The edge in front of one node: 1 = programmatic now; 0 = as it was, being of another kind or because the runtime will not exchange it; -1 = lost.
-static int overlap_edge(cudaGraph_t g, cudaGraphNode_t node) {
-    cudaGraphNodeType type;
-    if (!quiet(cudaGraphNodeGetType(node, &type)) || type != cudaGraphNodeTypeKernel) return 0;
-    cudaKernelNodeParams p{};
-    if (!quiet(cudaGraphKernelNodeGetParams(node, &p)) || !overlap_find(p.func, false)) return 0;     // another library's kernel, or one that does not wait
-    // One predecessor, a kernel: this node's own wait takes the place of the edge. Joins of several branches keep theirs (a step of Nelutar measured the same with
-    // those converted too).
-    size_t deps = 0;
-    if (!quiet(cudaGraphNodeGetDependencies_v2(node, nullptr, nullptr, &deps)) || deps != 1) return 0;
-    cudaGraphNode_t from = nullptr;
-    cudaGraphEdgeData edge{}, early{};
-    if (!quiet(cudaGraphNodeGetDependencies_v2(node, &from, &edge, &deps)) || !quiet(cudaGraphNodeGetType(from, &type))) return 0;
-    if (type != cudaGraphNodeTypeKernel || edge.type != cudaGraphDependencyTypeDefault || edge.from_port != cudaGraphKernelNodePortDefault) return 0;
+
+// A captured graph as sllm_graph_overlap sees it.
+struct StepGraph {
+    struct Node {
+        cudaGraphNode_t node;
+        std::vector<size_t> from, to;        // predecessors, successors
+        std::vector<cudaGraphEdgeData> edges;    // from its predecessors
+        bool kernel = false, waits = false;  // waits: a kernel that may become resident early
+        size_t before = 0, after = 0;        // nodes that have to complete before it, nodes that wait for it
+    };
+    std::vector<Node> nodes;
+    bool read(cudaGraph_t g);
+    int overlap(cudaGraph_t g, size_t i) const;
+    int separate(cudaGraph_t g, size_t i) const;
+};
+
+bool StepGraph::read(cudaGraph_t g) {        // false: the runtime will not say all of it
+    size_t n = 0;
+    if (!quiet(cudaGraphGetNodes(g, nullptr, &n))) return false;
+    std::vector<cudaGraphNode_t> handles(n);
+    if (!quiet(cudaGraphGetNodes(g, handles.data(), &n))) return false;
+    std::unordered_map<cudaGraphNode_t, size_t> index;
+    for (size_t i = 0; i < n; ++i) index[handles[i]] = i;
+    nodes.resize(n);
+    for (size_t i = 0; i < n; ++i) {
+        Node& x = nodes[i];
+        x.node = handles[i];
+        size_t deps = 0;
+        if (!quiet(cudaGraphNodeGetDependencies_v2(x.node, nullptr, nullptr, &deps))) return false;
+        std::vector<cudaGraphNode_t> from(deps);
+        x.edges.resize(deps);
+        if (deps && !quiet(cudaGraphNodeGetDependencies_v2(x.node, from.data(), x.edges.data(), &deps))) return false;
+        for (size_t k = 0; k < deps; ++k) {
+            const auto at = index.find(from[k]);
+            if (at == index.end()) return false;
+            x.from.push_back(at->second);
+            nodes[at->second].to.push_back(i);
+        }
+        cudaGraphNodeType type;
+        if (!quiet(cudaGraphNodeGetType(x.node, &type))) return false;
+        x.kernel = type == cudaGraphNodeTypeKernel;
+        cudaKernelNodeParams p{};
+        if (!x.kernel || !quiet(cudaGraphKernelNodeGetParams(x.node, &p))) continue;     // or another library's kernel
+        x.waits = g_overlap.find(p.func, false);
+    }
+    // how many nodes each one follows: a row of bits per node, predecessors first; every node it follows is followed by it
+    const size_t words = (n + 63) / 64;
+    std::vector<uint64_t> bits(n * words, 0);
+    std::vector<size_t> order, open(n);
+    for (size_t i = 0; i < n; ++i)
+        if ((open[i] = nodes[i].from.size()) == 0) order.push_back(i);
+    for (size_t k = 0; k < order.size(); ++k) {
+        const size_t i = order[k];
+        for (size_t w = 0; w < words; ++w)
+            for (uint64_t rest = bits[i * words + w]; rest; rest &= rest - 1) {
+                ++nodes[i].before;
+                ++nodes[w * 64 + __builtin_ctzll(rest)].after;
+            }
+        for (size_t j : nodes[i].to) {
+            for (size_t w = 0; w < words; ++w) bits[j * words + w] |= bits[i * words + w];
+            bits[j * words + i / 64] |= uint64_t(1) << (i % 64);
+            if (--open[j] == 0) order.push_back(j);
+        }
+    }
+    return true;
+}
+
+// One edge for another: 1 = done; 0 = as it was, since the runtime will not exchange it; -1 = lost.
+static int exchange(cudaGraph_t g, cudaGraphNode_t from, cudaGraphNode_t to, const cudaGraphEdgeData& old, const cudaGraphEdgeData& edge) {
+    if (!quiet(cudaGraphRemoveDependencies_v2(g, &from, &to, &old, 1))) return 0;
+    if (quiet(cudaGraphAddDependencies_v2(g, &from, &to, &edge, 1))) return 1;
+    return quiet(cudaGraphAddDependencies_v2(g, &from, &to, &old, 1)) ? 0 : -1;
+}
+
+// The edge in front of node i made programmatic: as exchange(), 0 also where it has to stay.
+int StepGraph::overlap(cudaGraph_t g, size_t i) const {
+    const Node& x = nodes[i];
+    // One predecessor, a kernel with no other successor, and no node in a parallel branch of the step (every other one completes before it or waits for it): its own wait takes the
+    // place of the edge, as between two launches of one stream. Where there are branches a CTA that only waits keeps another branch's off its SM. Measured, us a step of Nelutar,
+    // whose layers have branches, edges as captured | exchanged there too | only outside: width 1024, one request 388 | 368 | 376, four 503 | 503 | 491, eight 689 | 713 | 677;
+    // width 2048 537 | 498 | 525, 893 | 975 | 880, 1443 | 1490 | 1430; and at nine requests replays with edges exchanged there came to a stand.
+    if (!x.waits || x.from.size() != 1 || x.edges[0].type != cudaGraphDependencyTypeDefault || x.edges[0].from_port != cudaGraphKernelNodePortDefault) return 0;
+    const Node& previous = nodes[x.from[0]];
+    if (!previous.kernel || previous.to.size() != 1 || x.before + x.after + 1 != nodes.size()) return 0;
+    cudaGraphEdgeData early{};
     early.type = cudaGraphDependencyTypeProgrammatic;
     early.from_port = cudaGraphKernelNodePortProgrammatic;
-    if (!quiet(cudaGraphRemoveDependencies_v2(g, &from, &node, &edge, 1))) return 0;
-    if (quiet(cudaGraphAddDependencies_v2(g, &from, &node, &early, 1))) return 1;
-    return quiet(cudaGraphAddDependencies_v2(g, &from, &node, &edge, 1)) ? 0 : -1;
+    return exchange(g, previous.node, x.node, x.edges[0], early);
+}
+
+// Programmatic edges that the capture itself has made (products are launched with that attribute) from one branch to another, made ordinary: a launch at the start of a branch or behind
+// a join is not one behind another in a stream either. 0 or -1.
+int StepGraph::separate(cudaGraph_t g, size_t i) const {
+    const Node& x = nodes[i];
+    for (size_t k = 0; k < x.from.size(); ++k) {
+        if (x.edges[k].type != cudaGraphDependencyTypeProgrammatic || (x.from.size() == 1 && nodes[x.from[k]].to.size() == 1)) continue;
+        if (exchange(g, nodes[x.from[k]].node, x.node, x.edges[k], cudaGraphEdgeData{}) < 0) return -1;
+    }
+    return 0;
 }
 
 int sm_count() {
@@ -157,14 +241,13 @@ int sllm_graph_overlap(void* graph, int32_t* edges) {
     SLLM_REQUIRE(graph, SLLM_EINVAL, "graph_overlap: no graph");
     const cudaGraph_t g = reinterpret_cast<cudaGraph_t>(graph);
     int32_t changed = 0;
-    size_t n = 0;
-    SLLM_CUDA(cudaGraphGetNodes(g, nullptr, &n));
-    std::vector<cudaGraphNode_t> nodes(n);
-    SLLM_CUDA(cudaGraphGetNodes(g, nodes.data(), &n));
-    for (size_t i = 0; i < n; ++i) {
-        const int done = overlap_edge(g, nodes[i]);
-        SLLM_REQUIRE(done >= 0, SLLM_ESTATE, "graph_overlap: the runtime took an edge and would not have it back; the graph has to be captured again");
-        changed += done;
+    StepGraph step;
+    if (step.read(g)) {
+        for (size_t i = 0; i < step.nodes.size(); ++i) {
+            const int done = step.separate(g, i) < 0 ? -1 : step.overlap(g, i);
+            SLLM_REQUIRE(done >= 0, SLLM_ESTATE, "graph_overlap: the runtime took an edge and would not have it back; the graph has to be captured again");
+            changed += done;
+        }
     }
     if (edges) *edges = changed;
     return SLLM_OK;

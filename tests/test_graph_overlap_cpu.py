@@ -1,6 +1,7 @@
-"""sllm_graph_overlap where the runtime refuses: an edge that cannot be exchanged stays what it was and is not counted, a lost one is reported; and the capture of a step
-that goes on with a plain graph then. The library's own code against a stand-in for the runtime's graph calls (tests/cpp/fake_graph_runtime.c), in a process of its own."""
+"""Which edges sllm_graph_overlap exchanges, by the kernels and the branches of a step; what it does where the runtime refuses: an edge that cannot be exchanged stays what it
+was and is not counted, a lost one is reported; and the capture of a step that goes on with a plain graph then. The library's own code against a stand-in for the runtime's graph calls (tests/cpp/fake_graph_runtime.c), in a process of its own."""
 import contextlib
+import json
 import os
 import subprocess
 import sys
@@ -11,37 +12,67 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 LIB = os.path.join(ROOT, "simplellminference_b200", "lib", "libsllm_b200.so")
 
 CHILD = """
-import ctypes as C, sys
+import ctypes as C, json, sys
 fake = C.CDLL(sys.argv[1], mode=C.RTLD_GLOBAL)          # in front of the runtime's own symbols
 lib = C.CDLL(sys.argv[2])
-add = getattr(lib, "_ZN4sllm14overlap_kernelEPKv")
-add.argtypes = [C.c_void_p]
-for kernel in (2, 3, 4, 6):                              # node 5's kernel is not one that waits
-    add(kernel << 8)
+case = json.loads(sys.argv[3])
+register = getattr(lib, "_ZN4sllm14overlap_kernelEPKv")
+register.argtypes = [C.c_void_p]
+for node in case["waits"]:
+    register(node << 8)
 lib.sllm_graph_overlap.argtypes = [C.c_void_p, C.c_void_p]
-fake.fake_reset(6, *map(int, sys.argv[3:7]))
+fake.fake_reset(case["nodes"], *case.get("fails", [0, 0, 0, 0]))
+for edges in case.get("from", []):
+    fake.fake_from(*edges)
 n = C.c_int32(-7)
 rc = lib.sllm_graph_overlap(1, C.byref(n))
-print(rc, n.value, *[fake.fake_edge(i) for i in range(2, 7)])
+print(json.dumps([[rc, n.value], [fake.fake_edge(i, 0) + 10 * fake.fake_edge(i, 1) for i in range(2, case["nodes"] + 1)]]))
 """
 
 
-@pytest.mark.parametrize("look,remove,add,add_from,want", [
-    (0, 0, 0, 0, [0, 4, 2, 2, 2, 1, 2]),            # nothing fails: nodes 2, 3, 4 and 6
-    (2, 0, 0, 0, [0, 3, 1, 2, 2, 1, 2]),            # the first node's edge cannot be looked at
-    (0, 2, 0, 0, [0, 3, 2, 1, 2, 1, 2]),            # the second removal is refused
-    (0, 0, 1, 0, [0, 3, 1, 2, 2, 1, 2]),            # the first programmatic edge is refused and the ordinary one put back
-    (0, 0, 3, 0, [0, 3, 2, 2, 1, 1, 2]),
-    (0, 0, 0, 2, [-4, -7, 2, 0, 1, 1, 1]),          # from the second on none can be added, nor put back: reported
-])
-def test_refused_edges(tmp_path, look, remove, add, add_from, want):
+def _overlapped(tmp_path, **case):
+    """[return code, edges changed], the states of the edges in front of nodes 2, 3, ...: 1 ordinary, 2 programmatic, 10 times that for a second one."""
     if not os.path.exists(LIB):
         pytest.skip("library not built")
     fake = str(tmp_path / "libfake.so")
     subprocess.run(["gcc", "-shared", "-fPIC", "-Wall", "-Werror", "-I/usr/local/cuda/include", "-o", fake, os.path.join(ROOT, "tests", "cpp", "fake_graph_runtime.c")], check=True)
-    out = subprocess.run([sys.executable, "-c", CHILD, fake, LIB, *map(str, (look, remove, add, add_from))], capture_output=True, text=True)
+    out = subprocess.run([sys.executable, "-c", CHILD, fake, LIB, json.dumps(case)], capture_output=True, text=True)
     assert out.returncode == 0, out.stderr
-    assert [int(x) for x in out.stdout.split()] == want
+    return json.loads(out.stdout)
+
+
+@pytest.mark.parametrize("fails,want", [
+    ([0, 0, 0, 0], [[0, 4], [2, 2, 2, 1, 2]]),            # nothing fails: nodes 2, 3, 4 and 6 (5's kernel is not one that waits)
+    ([4, 0, 0, 0], [[0, 0], [1, 1, 1, 1, 1]]),            # the runtime will not describe the graph
+    ([0, 2, 0, 0], [[0, 3], [2, 1, 2, 1, 2]]),            # the second removal is refused
+    ([0, 0, 1, 0], [[0, 3], [1, 2, 2, 1, 2]]),            # the first programmatic edge is refused and the ordinary one put back
+    ([0, 0, 3, 0], [[0, 3], [2, 2, 1, 1, 2]]),
+    ([0, 0, 0, 2], [[-4, -7], [2, 0, 1, 1, 1]]),          # from the second on none can be added, nor put back: reported
+])
+def test_refused_edges(tmp_path, fails, want):
+    assert _overlapped(tmp_path, nodes=6, waits=[2, 3, 4, 6], fails=fails) == want
+
+
+@pytest.mark.parametrize("nodes,edges,want", [
+    # 1 -> 2 -> 3 -> 4 -> 7 -> 8 with 2 -> 5 -> 6 -> 7 beside 3 and 4: only the edges outside the branches
+    (8, [[5, 2, 1, 0, 0], [7, 4, 1, 6, 1]], [2, 1, 1, 1, 1, 11, 2]),
+    # a branch of one kernel that nothing follows
+    (5, [[5, 2, 1, 0, 0]], [2, 1, 1, 1]),
+    # no branch, but an edge beside the chain: 3 follows 1 and 2, 1 has two successors
+    (4, [[3, 2, 1, 1, 1]], [1, 11, 2]),
+    # made by the capture: across a fork and into a join they become ordinary, inside a branch they stay
+    (8, [[3, 2, 2, 0, 0], [4, 3, 2, 0, 0], [5, 2, 2, 0, 0], [7, 4, 2, 6, 1]], [2, 1, 2, 1, 1, 11, 2]),
+], ids=["fork-join", "loose-end", "shortcut", "captured"])
+def test_parallel_branches_keep_their_edges(tmp_path, nodes, edges, want):
+    kept = sum(e[2] == 2 and w == 2 for e, w in ((e, want[e[0] - 2]) for e in edges))
+    assert _overlapped(tmp_path, nodes=nodes, waits=list(range(2, nodes + 1)), **{"from": edges}) == [[0, want.count(2) - kept], want]
+
+
+def test_refused_while_branches_are_separated(tmp_path):
+    case = dict(nodes=5, waits=[2], **{"from": [[3, 2, 2, 0, 0], [5, 2, 1, 0, 0]]})
+    assert _overlapped(tmp_path, fails=[0, 0, 0, 0], **case) == [[0, 1], [2, 1, 1, 1]]
+    assert _overlapped(tmp_path, fails=[0, 0, 2, 0], **case) == [[0, 1], [2, 2, 1, 1]]      # the captured edge is put back
+    assert _overlapped(tmp_path, fails=[0, 0, 0, 2], **case)[0][0] == -4
 
 
 class _Graph:
