@@ -57,7 +57,7 @@ const char* sllm_last_error(void);
 int sllm_status(void);
 /* Turns edges of a captured graph (cudaGraph_t, not yet instantiated) into programmatic ones: a kernel of this library that waits for its predecessor itself, and has
  * one predecessor, a kernel that nothing else follows, may become resident while that one still runs. What it reads and writes behind that wait, and so every result, is
- * the same. Left as they are: all edges of nodes beside which the graph has a parallel branch; programmatic edges that the
+ * the same. Left as they are: edges in front of kernels of few heavy CTAs, and all edges of nodes beside which the graph has a parallel branch; programmatic edges that the
  * capture has made from one branch to another become ordinary ones. *edges (or NULL): how many were made programmatic. An edge that the runtime will not exchange stays as it was, and so does a graph it will not describe; SLLM_ESTATE: an edge could not be put back either, and
  * the graph must not be used. */
 int sllm_graph_overlap(void* graph, int32_t* edges);

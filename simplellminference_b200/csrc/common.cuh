@@ -77,10 +77,20 @@ struct LaunchCfg {
 
 // A kernel that calls after_previous() on every path: in a captured step it may become resident while the kernel before it still runs (sllm_graph_overlap). The
 // launch itself is an ordinary one.
-void overlap_kernel(const void* kernel);
+void overlap_kernel(const void* kernel, bool alone);
 template <class F>
 inline F* overlapping(F* kernel) {
-    overlap_kernel(reinterpret_cast<const void*>(kernel));
+    overlap_kernel(reinterpret_cast<const void*>(kernel), false);
+    return kernel;
+}
+// The same, but early only where the launch is a single CTA: for kernels of few CTAs with much work each. Becoming resident while the kernel in front still holds most SMs, they
+// end up several to an SM and take that much longer. Measured, us a step with the edge in front of them early | not: attention in latent heads (Vasosun, width 1024, four
+// requests) 1017 | 927, a seam that convolves 1017 | 1003, experts' activation 1017 | 1005 (with one request, where those two are one CTA, 572 | 577 and 575), attention whose
+// heads are mixed (Lovulix, width 1024, 64 requests) 1369 | 1092, rotation of latent queries (Sopetar, width 2048, 64) 1410 | 1397, products in tiles of 64 x 64 (Munazen, width
+// 2048, 32) 14590 | 11400.
+template <class F>
+inline F* overlapping_alone(F* kernel) {
+    overlap_kernel(reinterpret_cast<const void*>(kernel), true);
     return kernel;
 }
 

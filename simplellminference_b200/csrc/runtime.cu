@@ -64,7 +64,8 @@ int status_take() {
     return SLLM_ETIMEOUT;
 }
 
-// Kernels launched through overlapping(): a set that only grows, to at most as many as the library has instantiations; looked up on every launch, so without a lock.
+// Kernels launched through overlapping() and overlapping_alone(): sets that only grow, to at most as many as the library has instantiations; looked up on every launch, so
+// without a lock.
 struct KernelSet {
     static constexpr size_t kSlots = 1024;
     std::atomic<const void*> slots[kSlots];
@@ -79,8 +80,8 @@ struct KernelSet {
         return false;                             // a full table: this kernel's edges stay as they are
     }
 };
-static KernelSet g_overlap;
-void overlap_kernel(const void* kernel) { g_overlap.find(kernel, true); }
+static KernelSet g_overlap, g_overlap_alone;
+void overlap_kernel(const void* kernel, bool alone) { (alone ? g_overlap_alone : g_overlap).find(kernel, true); }
 static bool quiet(cudaError_t e) {               // a refusal that is no error of the caller's
     if (e != cudaSuccess) cudaGetLastError();
     return e == cudaSuccess;
@@ -128,7 +129,7 @@ bool StepGraph::read(cudaGraph_t g) {        // false: the runtime will not say 
         x.kernel = type == cudaGraphNodeTypeKernel;
         cudaKernelNodeParams p{};
         if (!x.kernel || !quiet(cudaGraphKernelNodeGetParams(x.node, &p))) continue;     // or another library's kernel
-        x.waits = g_overlap.find(p.func, false);
+        x.waits = g_overlap.find(p.func, false) || (g_overlap_alone.find(p.func, false) && (size_t)p.gridDim.x * p.gridDim.y * p.gridDim.z == 1);
     }
     // how many nodes each one follows: a row of bits per node, predecessors first; every node it follows is followed by it
     const size_t words = (n + 63) / 64;

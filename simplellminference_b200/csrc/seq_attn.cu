@@ -711,7 +711,7 @@ static int attention_run(const sllm_seq_batch* b, const float* q, int32_t ldq, i
 #define SLLM_ATTN_LAUNCH(KV, NC)                                                                                                              \
     do {                                                                                                                                      \
         if (smem > 48 * 1024) SLLM_CUDA(cudaFuncSetAttribute(seq_attention_kernel<KV, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-        overlapping(seq_attention_kernel<KV, NC>)<<<grid, 256, smem, as_stream(stream)>>>(p);                                                              \
+        overlapping_alone(seq_attention_kernel<KV, NC>)<<<grid, 256, smem, as_stream(stream)>>>(p);                                                              \
     } while (0)
     if (kv_dtype == SLLM_F32) {
         if (chunks == 4) SLLM_ATTN_LAUNCH(float, 4); else if (chunks == 8) SLLM_ATTN_LAUNCH(float, 8); else SLLM_ATTN_LAUNCH(float, 16);

@@ -580,10 +580,10 @@ int sllm_seq_attention_talk(const sllm_seq_batch* b, const float* q, int32_t ldq
     const dim3 grid(b->T == b->nseg ? b->n_qtiles : b->n_qtiles * (kBQ / p.nq), nsplit);
     if (kv_dtype == SLLM_F32) {
         SLLM_CUDA(cudaFuncSetAttribute(seq_attention_talk_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        overlapping(seq_attention_talk_kernel<float>)<<<grid, kTalkWarps * 32, smem, st>>>(p);
+        overlapping_alone(seq_attention_talk_kernel<float>)<<<grid, kTalkWarps * 32, smem, st>>>(p);
     } else {
         SLLM_CUDA(cudaFuncSetAttribute(seq_attention_talk_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        overlapping(seq_attention_talk_kernel<uint16_t>)<<<grid, kTalkWarps * 32, smem, st>>>(p);
+        overlapping_alone(seq_attention_talk_kernel<uint16_t>)<<<grid, kTalkWarps * 32, smem, st>>>(p);
     }
     ++g_launches;
     SLLM_LAUNCH_CHECK();

@@ -545,8 +545,8 @@ extern "C" int sllm_seq_linear(const float* A, int32_t lda, const void* W, int32
         return SLLM_OK;
     }
     dim3 grid((N + kTN - 1) / kTN, (T + kTM - 1) / kTM, batch);
-    if (w_dtype == SLLM_BF16) overlapping(seq_linear_tile_kernel<SLLM_BF16>)<<<grid, 256, 0, st>>>(p);
-    else overlapping(seq_linear_tile_kernel<SLLM_F32>)<<<grid, 256, 0, st>>>(p);
+    if (w_dtype == SLLM_BF16) overlapping_alone(seq_linear_tile_kernel<SLLM_BF16>)<<<grid, 256, 0, st>>>(p);
+    else overlapping_alone(seq_linear_tile_kernel<SLLM_F32>)<<<grid, 256, 0, st>>>(p);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;
@@ -571,8 +571,8 @@ extern "C" int sllm_seq_linear_grouped(const void* A, int32_t a_bf16, const void
     LinArgs p{(const float*)A, W, nullptr, C, K, K, N, cap, N, K, w_dtype, 0, w_dtype == SLLM_BF16, 1.0f, (long long)cap * K, (long long)N * K, 0, (long long)cap * N,
               counts, nullptr, 0, 1, 0};
     dim3 grid((N + kTN - 1) / kTN, (cap + kTM - 1) / kTM, groups);
-    if (w_dtype == SLLM_BF16) overlapping(seq_linear_tile_kernel<SLLM_BF16>)<<<grid, 256, 0, st>>>(p);
-    else overlapping(seq_linear_tile_kernel<SLLM_F32>)<<<grid, 256, 0, st>>>(p);
+    if (w_dtype == SLLM_BF16) overlapping_alone(seq_linear_tile_kernel<SLLM_BF16>)<<<grid, 256, 0, st>>>(p);
+    else overlapping_alone(seq_linear_tile_kernel<SLLM_F32>)<<<grid, 256, 0, st>>>(p);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;

@@ -199,7 +199,7 @@ extern "C" int sllm_seq_moe_act(const float* logits, int32_t ldl, int32_t n_rout
     SLLM_REQUIRE(n_route <= 2048, SLLM_ENOTSUP, "seq_moe_act: %d router outputs beyond 2048", n_route);
     const int work = std::max(experts * ff + shared_ff, d);
     const int threads = T >= 64 ? 256 : std::min(1024, std::max(128, (work + 31) / 32 * 32));
-    overlapping(seq_moe_act_kernel)<<<T, threads, (3 * (size_t)n_route + 2 * std::max(o.groups, 0)) * sizeof(float), as_stream(stream)>>>(
+    overlapping_alone(seq_moe_act_kernel)<<<T, threads, (3 * (size_t)n_route + 2 * std::max(o.groups, 0)) * sizeof(float), as_stream(stream)>>>(
         logits, ldl, n_route, experts, top, correction, up, ldu, ff, act, h, ldh, d, out, (uint16_t*)out16, y, ldy, route_w, shared_up, ld_shared, shared_ff, o);
     ++g_launches;
     SLLM_LAUNCH_CHECK();

@@ -568,10 +568,10 @@ int sllm_seq_latent_kv(const sllm_seq_batch* b, const float* q, int32_t ldq, int
     SLLM_REQUIRE(kv_dtype == SLLM_F32 || kv_dtype == SLLM_BF16, SLLM_ENOTSUP, "seq_latent_kv: fp32 or bf16 pools");
     const int threads = rank >= 512 ? 256 : 128;
     if (kv_dtype == SLLM_F32)
-        overlapping(seq_latent_kv_kernel<float>)<<<b->T, threads, 0, as_stream(stream)>>>(*b, q, ldq, heads, dn, dr, low, ldlow, rank, norm_w, eps, freq, n_freq, magnitude, q_out, ldqo,
+        overlapping_alone(seq_latent_kv_kernel<float>)<<<b->T, threads, 0, as_stream(stream)>>>(*b, q, ldq, heads, dn, dr, low, ldlow, rank, norm_w, eps, freq, n_freq, magnitude, q_out, ldqo,
                                                                              (float*)pool);
     else
-        overlapping(seq_latent_kv_kernel<uint16_t>)<<<b->T, threads, 0, as_stream(stream)>>>(*b, q, ldq, heads, dn, dr, low, ldlow, rank, norm_w, eps, freq, n_freq, magnitude, q_out,
+        overlapping_alone(seq_latent_kv_kernel<uint16_t>)<<<b->T, threads, 0, as_stream(stream)>>>(*b, q, ldq, heads, dn, dr, low, ldlow, rank, norm_w, eps, freq, n_freq, magnitude, q_out,
                                                                                 ldqo, (uint16_t*)pool);
     ++g_launches;
     SLLM_LAUNCH_CHECK();

@@ -479,7 +479,7 @@ extern "C" int sllm_seq_seam(const sllm_seq_batch* b, const float* x_in, float* 
         SLLM_LAUNCH_CHECK();
         return SLLM_OK;
     }
-    overlapping(seq_seam_kernel)<<<b->T, threads, smem, as_stream(stream)>>>(p);
+    overlapping_alone(seq_seam_kernel)<<<b->T, threads, smem, as_stream(stream)>>>(p);
     ++g_launches;
     SLLM_LAUNCH_CHECK();
     return SLLM_OK;

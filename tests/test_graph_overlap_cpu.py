@@ -16,14 +16,18 @@ import ctypes as C, json, sys
 fake = C.CDLL(sys.argv[1], mode=C.RTLD_GLOBAL)          # in front of the runtime's own symbols
 lib = C.CDLL(sys.argv[2])
 case = json.loads(sys.argv[3])
-register = getattr(lib, "_ZN4sllm14overlap_kernelEPKv")
-register.argtypes = [C.c_void_p]
+register = getattr(lib, "_ZN4sllm14overlap_kernelEPKvb")
+register.argtypes = [C.c_void_p, C.c_bool]
 for node in case["waits"]:
-    register(node << 8)
+    register(node << 8, False)
+for node in case.get("alone", []):
+    register(node << 8, True)
 lib.sllm_graph_overlap.argtypes = [C.c_void_p, C.c_void_p]
 fake.fake_reset(case["nodes"], *case.get("fails", [0, 0, 0, 0]))
 for edges in case.get("from", []):
     fake.fake_from(*edges)
+for node, grid in case.get("grids", []):
+    fake.fake_grid(node, grid)
 n = C.c_int32(-7)
 rc = lib.sllm_graph_overlap(1, C.byref(n))
 print(json.dumps([[rc, n.value], [fake.fake_edge(i, 0) + 10 * fake.fake_edge(i, 1) for i in range(2, case["nodes"] + 1)]]))
@@ -73,6 +77,12 @@ def test_refused_while_branches_are_separated(tmp_path):
     assert _overlapped(tmp_path, fails=[0, 0, 0, 0], **case) == [[0, 1], [2, 1, 1, 1]]
     assert _overlapped(tmp_path, fails=[0, 0, 2, 0], **case) == [[0, 1], [2, 2, 1, 1]]      # the captured edge is put back
     assert _overlapped(tmp_path, fails=[0, 0, 0, 2], **case)[0][0] == -4
+
+
+@pytest.mark.parametrize("grid", [1, 2, 4])
+def test_kernels_of_few_heavy_ctas_are_early_only_alone(tmp_path, grid):
+    want = [2, 2 if grid == 1 else 1, 2]
+    assert _overlapped(tmp_path, nodes=4, waits=[2, 4], alone=[3], grids=[[3, grid], [4, 148]]) == [[0, want.count(2)], want]
 
 
 class _Graph:

@@ -113,7 +113,7 @@ def test_weights_written_by_the_graph_itself():
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_small_matrices_written_by_the_kernel_in_front(dtype, T, N, K):
     """Below 1.5 million weights, where the products go through the body for small matrices. fp32: written, then added to, by tiles of 64 x 64, so that CTAs side by side
-    write parts of the same rows; bf16: the rows of a norm."""
+    write parts of the same rows (tiles that start when the kernel in front has ended); bf16: the rows of a norm."""
     import torch
     from simplellminference_b200.config import BF16, F32
     from simplellminference_b200.seqops import Ops
@@ -139,7 +139,7 @@ def test_small_matrices_written_by_the_kernel_in_front(dtype, T, N, K):
     graph = torch.cuda.CUDAGraph(keep_graph=True)
     with torch.cuda.graph(graph):
         step(torch.cuda.current_stream().cuda_stream)
-    assert ops.overlap(graph.raw_cuda_graph()) == (3 if dtype == "float32" else 2)
+    assert ops.overlap(graph.raw_cuda_graph()) == 2
     graph.instantiate()
     for seed in (2, 3, 4):
         g.manual_seed(seed)
