@@ -18,6 +18,20 @@
 
 namespace sllm {
 
+// The lanes' values of a row, four loads on their way before the first is handed on: stored one by one, each load would stand behind the store before it, which could be the
+// same memory (unit_kv of 2048 tokens, 8 heads over 2 of 128, 7.4 -> 6.1 us; of five 2.6 -> 2.4).
+template <class F>
+__device__ __forceinline__ void seq_each(const float* row, int n, int lane, F use) {
+    for (int j0 = lane; j0 < n; j0 += 128) {
+        float x[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x[k] = j0 + 32 * k < n ? row[j0 + 32 * k] : 0.0f;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (j0 + 32 * k < n) use(j0 + 32 * k, x[k]);
+    }
+}
+
 // grid (T, ceil(items / 4)), 4 warps: warp = one head of q, k or v of one token
 template <typename KV>
 __global__ void seq_unit_kv_kernel(sllm_seq_batch b, float* q, int ldq, int heads, int dk, const float* k, int ldk, int kv_heads,
@@ -39,7 +53,7 @@ __global__ void seq_unit_kv_kernel(sllm_seq_batch b, float* q, int ldq, int head
             for (int j = lane; j < dk; j += 32) ss = fmaf(row[j], row[j], ss);
             inv = temp / sqrtf(warp_sum(ss) / (float)dk + eps);
         }
-        for (int j = lane; j < dk; j += 32) row[j] *= inv;
+        seq_each(row, dk, lane, [&](int j, float x) { row[j] = x * inv; });
     } else if (item < heads + kv_heads) {                // a key head -> pool
         const int g = item - heads;
         const float* row = k + (size_t)t * ldk + (size_t)g * dk;
@@ -50,7 +64,7 @@ __global__ void seq_unit_kv_kernel(sllm_seq_batch b, float* q, int ldq, int head
             inv = 1.0f / sqrtf(warp_sum(ss) / (float)dk + eps);
         }
         const size_t dst = seq_pool_row(page, kv_heads, g, b.page_len, in_page, dk);
-        for (int j = lane; j < dk; j += 32) seq_st(k_pool, dst + j, row[j] * inv);
+        seq_each(row, dk, lane, [&](int j, float x) { seq_st(k_pool, dst + j, x * inv); });
     } else {                                             // a value head -> (blend) -> pool
         const int g = item - heads - kv_heads;
         const float* row = v + (size_t)t * ldv + (size_t)g * dv;
@@ -62,12 +76,12 @@ __global__ void seq_unit_kv_kernel(sllm_seq_batch b, float* q, int ldq, int head
         }
         const size_t dst = seq_pool_row(page, kv_heads, g, b.page_len, in_page, dv);
         float* sh = v_shared ? v_shared + ((size_t)t * kv_heads + g) * dv : nullptr;
-        for (int j = lane; j < dv; j += 32) {
-            float val = row[j] * inv;
+        seq_each(row, dv, lane, [&](int j, float x) {
+            float val = x * inv;
             if (share == 1) sh[j] = val;
             else if (share == 2) val = (1.0f - lambda) * val + lambda * sh[j];
             seq_st(v_pool, dst + j, val);
-        }
+        });
     }
 }
 
