@@ -17,7 +17,7 @@ pos) per token with host buffers: H2D of token+position, D2H of the next token, 
 `roofline` = the dominant kernel (gate_up GEMV) timed alone with CUDA events, cycling over the layers so its
 weights always come from HBM; `step_roofline` = whole-step algorithmic bytes B(p) / step time.
 Secondary keys measured in child processes AFTER every timed region (N = 1; a failure there costs only its own key):
-`batch_decode` (tools/batch_bench.py) and `experiments` (tools/fuse_bench.py, tools/microbench/fusion_probe); --no-batch skips them.
+`batch_decode` (tools/batch_bench.py) and `experiments` (tools/fuse_bench.py, tools/mega_trace.py); --no-batch skips them.
 """
 from __future__ import annotations
 
@@ -58,7 +58,7 @@ def parse():
                                                            "the default: csrc/megakernel2.cu with the fused down projection and the calibrated partition")
     ap.add_argument("--no-calibrate", action="store_true", help="skip sllm_engine_calibrate (per-CTA shares of every phase sized by the measured streaming rate of each SM)")
     ap.add_argument("--extras", action="store_true", help="after the timed regions, also run the secondary measurements in child processes (batched multi-sequence decode, "
-                                                          "microbenchmarks, per-phase timelines); their JSON goes under batch_decode / experiments")
+                                                          "per-phase timelines); their JSON goes under batch_decode / experiments")
     ap.add_argument("--nccl", action="store_true", help="tensor parallel: NCCL all-reduce instead of the fused peer-memory one")
     ap.add_argument("--kernel-only", default=None, help="profiling aid: loop one fused kernel kind and exit")
     ap.add_argument("--hybrid", default=None, metavar="SIZES",
@@ -97,7 +97,7 @@ def tensor_peak():
         with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
             return float(json.load(f)["bf16_tflops_sustained"]), "measured (MEASURED_PEAKS.json bf16_tflops_sustained)"
     except Exception:
-        return 1350.0, "fallback (B200_PROFILING.md sustained cuBLAS bf16)"
+        return 1350.0, "fallback (sustained cuBLAS bf16)"
 
 
 def prefill_flops(ms, T):
@@ -112,7 +112,7 @@ def peaks():
         with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
             return float(json.load(f)["hbm_gbs"]), "measured (MEASURED_PEAKS.json hbm_gbs)"
     except Exception:
-        return 6650.0, "fallback (B200_PROFILING.md 6.65 TB/s)"
+        return 6650.0, "fallback (6.65 TB/s)"
 
 
 def prompt_ids(n, vocab):
@@ -124,7 +124,7 @@ def prompt_ids(n, vocab):
 
 
 class ClockSampler:
-    """nvidia-smi sampled while the GPU runs the measured kernel (B200_PROFILING.md 'clocks' line). The timed region of a default run is
+    """nvidia-smi sampled while the GPU runs the measured kernel (clocks and the reasons for their events). The timed region of a default run is
     ~55 ms — shorter than nvidia-smi's start-up — so the sampler starts before the (untimed) prompt feed, which runs the very same
     kernel back to back for > 1 s, and runs through warm-up, timed steps and the end-to-end leg; every sample carries a timestamp and
     the record says how many fell inside the timed region itself."""
@@ -346,9 +346,7 @@ def _child_text(cmd, timeout, max_lines=60):
 def experiments_sample(args, main_checksum, K, W):
     """Secondary, N = 1 only, each in its own child process after every timed region of the main arm (nothing here can touch the headline):
     (1) the experimental megakernel with the down projection fused into the gate_up phase on the main arm's exact workload — tokens/s and
-    whether its tokens equal the main arm's; (2) tools/microbench/fusion_probe — what combining 148 partial vectors with vector reductions
-    costs against the grid barrier, cluster co-residency, TMA ingest from L2-resident against HBM-resident tiles;
-    (3) the per-phase timelines of both kernels."""
+    whether its tokens equal the main arm's; (2) the per-phase timelines of both kernels (trace_sample)."""
     out = {}
     if args.wdtype in ("f32", "bf16"):
         lines, note = _child_json_lines([sys.executable, os.path.join(ROOT, "tools", "fuse_bench.py"), "--config", args.config, "--wdtype", args.wdtype,
@@ -361,17 +359,13 @@ def experiments_sample(args, main_checksum, K, W):
             # something is off with the never-before-run kernel: bring back WHERE (layout of the transposed matrix alone; one forward of a
             # one-layer model through the verified and the fused kernel, buffer by buffer, for 1 / 2 / 16 stripes; the reference's golden stream)
             out["fused_down_diagnosis"] = _child_text([sys.executable, os.path.join(ROOT, "tests", "fuse_check.py"), "--quick", "/tmp/sllm_fuse_check.log"], 60, max_lines=40)
-    probe = os.path.join(ROOT, "tools", "microbench", "_build", "fusion_probe")
-    if os.path.exists(probe):
-        lines, note = _child_json_lines([probe, "1000"], 60)
-        out["fusion_probe"] = lines if lines else {"error": note or "no output"}
     return out
 
 
 def trace_sample(args):
-    """(3) where the time of a decode step goes: per-phase timeline (%globaltimer stamps) of the default megakernel and of the fused one,
+    """(2) where the time of a decode step goes: per-phase timeline (%globaltimer stamps) of the default megakernel and of the fused one,
     four layers of the same widths (tools/mega_trace.py). Last in line for the shared budget: the longest-running child (the batched
-    decoder) goes before it, the two short experiments before that."""
+    decoder) goes before it, the short experiment before that."""
     if not (args.config == "llama2-7b" and args.wdtype == "bf16" and args.kvdtype == "bf16"):
         return None
     trace = [sys.executable, os.path.join(ROOT, "tools", "mega_trace.py"), "--pos", str(args.prompt_len)]
@@ -621,7 +615,7 @@ def run_ours(args):
     batch = experiments = None
     if world == 1 and args.extras:
         eng.close()
-        try:   # secondary: never lose the line over any of it. Order = cost: the two short experiments, the batched decoder, the timelines
+        try:   # secondary: never lose the line over any of it. Order = cost: the short experiment, the batched decoder, the timelines
             if mode == "megakernel":   # the grid-barrier kernel: measure its fused-down variant beside it
                 experiments = experiments_sample(args, int(np.sum(tokens.astype(np.int64)) % 1000003), K, W)
             batch = batch_decode_sample(args)

@@ -284,11 +284,10 @@ __device__ __forceinline__ void prefetch_norms(const MegaParams& p, int l, int c
 // ---- L2 prefetch of the weight stream: built twice, measured, removed ------------------------------------------------------
 // The rings hold 128 KB per SM; at a dependency point (grid barrier, attention, per-head counters) the consumers stall and HBM runs dry
 // (with the dot products removed the step takes exactly as long, with the barriers removed it is 20 % shorter: r02_mega_debug_v1.jsonl).
-// Asking the L2 for the tiles beyond the ring with cp.async.bulk.prefetch.L2 works IN ISOLATION (r02_prefetch_probe.jsonl: 39 MB asked
+// Asking the L2 for the tiles beyond the ring with cp.async.bulk.prefetch.L2 works IN ISOLATION (39 MB asked
 // for, 10 us of idling, then streamed through the rings in 2.1 us instead of 4.2 us = 120-130 GB/s per SM against 49-63 from HBM), and
-// loses in the kernel in both forms tried: (1) a continuous look-ahead of 2-16 tiles per warp during streaming: -5 % to -30 %
-// (r02_l2_lookahead_sweep.jsonl); (2) 2-12 tiles per warp asked for right before a grid barrier and / or before the attention chain:
-// -4 % to -13 % (r02_l2_prefetch_at_stalls_sweep.jsonl). A CTA's "stall" is the time the slowest CTAs still stream (the bulk prefetches
+// loses in the kernel in both forms tried: (1) a continuous look-ahead of 2-16 tiles per warp during streaming: -5 % to -30 %; (2) 2-12 tiles per warp asked for right before a grid barrier and / or before the attention chain:
+// -4 % to -13 %. A CTA's "stall" is the time the slowest CTAs still stream (the bulk prefetches
 // of the early ones take HBM bandwidth from exactly the copies the barrier is waiting for), and the attention / counter chain is a
 // sequence of small latency-critical L2 round trips that queue behind 40 MB of prefetch traffic. HBM is the shared resource: anything
 // that is not on the critical path and uses it lengthens the critical path.
@@ -345,13 +344,9 @@ __device__ __forceinline__ float reg_dot(const uint4 w, const float* x, float ac
 }
 
 
-// The larger logit, the smaller index among equals (candidates are never NaN).
-__device__ __forceinline__ void take_better(float& v, int& i, float ov, int oi) {
-    if (ov > v || (ov == v && oi < i)) { v = ov; i = oi; }
-}
 __device__ __forceinline__ void warp_better(float& v, int& i) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) take_better(v, i, __shfl_xor_sync(0xffffffffu, v, o), __shfl_xor_sync(0xffffffffu, i, o));
+    for (int o = 16; o > 0; o >>= 1) better_of(v, i, __shfl_xor_sync(0xffffffffu, v, o), __shfl_xor_sync(0xffffffffu, i, o));
 }
 // (v, i) of every thread -> the CTA's best in all threads of warp 0; red: 2 * kMegaWarps words of shared memory
 __device__ __forceinline__ void cta_better(float& v, int& i, float* red) {
@@ -382,7 +377,7 @@ __device__ __forceinline__ bool mega_finish(const MegaParams& p, float v, int i,
     if (!*s_last) return false;
     v = -INFINITY;
     i = 0x7fffffff;
-    for (int b = threadIdx.x; b < ncta; b += kMegaThreads) take_better(v, i, __ldcg(p.blk_val + b), __ldcg(p.blk_idx + b));
+    for (int b = threadIdx.x; b < ncta; b += kMegaThreads) better_of(v, i, __ldcg(p.blk_val + b), __ldcg(p.blk_idx + b));
     cta_better(v, i, red);
     if (threadIdx.x != 0) return false;
     if (i == 0x7fffffff) i = 0;

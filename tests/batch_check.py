@@ -1,10 +1,11 @@
-"""Stand-alone runner of the batched-decode GPU checks (tests/test_zz_batch_gpu.py) with a progressive log, for a GPU
-box on a short lease: `python tests/batch_check.py [logfile]`. First a one-step localisation (every per-slot buffer
+"""Stand-alone runner of the batched-decode GPU checks (tests/test_zz_batch_gpu.py) with a progressive log:
+`python tests/batch_check.py [logfile]`. First a one-step localisation (every per-slot buffer
 of the batch against the per-kernel engine at position 0, so a wrong kernel is named), then each test function in
 turn (`--quick`: only the never-run cases that take seconds). Not collected by pytest (no test_ prefix); the assertions live in the
 test module."""
 import os
 import sys
+import tempfile
 import time
 import traceback
 
@@ -13,7 +14,7 @@ sys.path.insert(0, ROOT)
 sys.path.insert(0, os.path.join(ROOT, "tests"))
 QUICK = "--quick" in sys.argv      # only the cases that have never run on a GPU and finish in seconds (bench.py's diagnostic child)
 _args = [a for a in sys.argv[1:] if a != "--quick"]
-LOG = _args[0] if _args else os.path.join(ROOT, "gpurun_out", "batch_check.log")
+LOG = _args[0] if _args else os.path.join(tempfile.gettempdir(), "sllm_batch_check.log")
 os.makedirs(os.path.dirname(LOG), exist_ok=True)
 _t0 = time.time()
 _f = open(LOG, "w")

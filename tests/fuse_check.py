@@ -7,6 +7,7 @@ stage is named; then every case of tests/test_zzz_mega_fuse_gpu.py in turn (`--q
 import dataclasses
 import os
 import sys
+import tempfile
 import time
 import traceback
 
@@ -15,7 +16,7 @@ sys.path.insert(0, ROOT)
 sys.path.insert(0, os.path.join(ROOT, "tests"))
 QUICK = "--quick" in sys.argv      # localisation + the cases that need no oracle run (bench.py's diagnostic child: about 20 s)
 _args = [a for a in sys.argv[1:] if a != "--quick"]
-LOG = _args[0] if _args else os.path.join(ROOT, "gpurun_out", "fuse_check.log")
+LOG = _args[0] if _args else os.path.join(tempfile.gettempdir(), "sllm_fuse_check.log")
 os.makedirs(os.path.dirname(LOG), exist_ok=True)
 _t0 = time.time()
 _f = open(LOG, "w")

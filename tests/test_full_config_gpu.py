@@ -24,7 +24,7 @@ max|logits_strict_i| (the sensitivity is a property of the state at that positio
 positions): the CUDA path
 must stay within max(5e-3, 8 * yard_i) of the strict oracle, i.e. no further from the reference than a legal re-association of the
 reference's own arithmetic is (times 8: the envelope is two samples per position; measured yard_i ~ 1e-2 at 32 layers, and every
-CUDA path measured between 0.5x and 4.2x of it, profiles/r02_full_config_parity.log). The K row
+CUDA path measured between 0.5x and 4.2x of it). The K row
 the engine writes for layer 0 (no depth amplification) must match the oracle's to a bf16 ulp. Every engine mode that serves the configuration is checked: the default megakernel(s), the word-based
 megakernel (the kernel behind every N > 1 number) and the per-kernel CUDA-graph path. bf16 KV on both sides (orc_set_kv_bf16).
 """

@@ -71,7 +71,7 @@ def main():
         with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
             peak, peak_src = float(json.load(f)["hbm_gbs"]), "measured (MEASURED_PEAKS.json hbm_gbs)"
     except Exception:
-        peak, peak_src = 6650.0, "fallback (B200_PROFILING.md 6.65 TB/s)"
+        peak, peak_src = 6650.0, "fallback (6.65 TB/s)"
 
     stream = torch.cuda.Stream()
     torch.cuda.set_stream(stream)

@@ -1,5 +1,5 @@
 import os, sys, numpy as np, torch
-sys.path.insert(0, '/root/repo')
+sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
 from oracle import loader
 from simplellminference_b200.config import ModelShape, BF16, F32
 from simplellminference_b200.engine import Engine

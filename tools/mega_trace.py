@@ -69,6 +69,5 @@ print("slowest CTAs (cta, smid, relative time):", [(int(c), int(smid[c]), round(
 print("fastest CTAs:", [(int(c), int(smid[c]), round(float(allm[c]), 3)) for c in order[:10]])
 print("relative time by smid parity / half:", {"smid<74": round(float(allm[smid < 74].mean()), 4), "smid>=74": round(float(allm[smid >= 74].mean()), 4),
       "even": round(float(allm[smid % 2 == 0].mean()), 4), "odd": round(float(allm[smid % 2 == 1].mean()), 4)})
-np.save("gpurun_out/mega_rel_time.npy", np.stack([smid.astype(np.float64), allm], 1)) if (os.path.isdir("gpurun_out") and rank == 0) else None
 if world > 1:
     torch.cuda.synchronize(); dist.barrier(); eng.close(); dist.destroy_process_group()
