@@ -665,7 +665,7 @@ static int attention_run(const sllm_seq_batch* b, const float* q, int32_t ldq, i
         const dim3 block(64 * hpc);
         cudaStream_t st = as_stream(stream);
         // Heads of 64 or 128 and steps of some size: tcgen05 (seq_attn_tc.cu), which has a fixed part of some 14 us (queries, TMEM, barriers, rows out). Measured, us, this
-        // body | tcgen05, each with the merge where there is one. Prompts of 1000, 311, 700 and 37 tokens, 16 heads over 4 of 128: 168 | 54, capped 215 | 57; one of 4096,
+        // body | tcgen05, each with the merge where there is one. Prompts of 1000, 311, 700 and 37 tokens, 16 heads over 4 of 128: 168 | 54, capped at 30 215 | 63; one of 4096,
         // 32 heads over 8 2050 | 468. Prompts from the start, heads of 128: 16 tiles 4 heads 25 | 23, 8 heads 31 | 30, 16 heads 50 | 33; 8 tiles 32 heads 58 | 53, 16 heads
         // 33 | 31, but 8 heads 19.5 | 25.6 and 4 heads 14 | 20, 12 tiles of 4 heads 20 | 21. Heads of 64: 16 tiles 8 heads 24 | 23, 16 heads 31 | 33; 19 tiles 34 | 25 and
         // 42 | 34. Longer contexts are always better off (8 heads, 256 tokens behind 1000 39 | 31, behind 4000 97 | 46), decoding requests beside a portion most of

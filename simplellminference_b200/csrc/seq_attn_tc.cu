@@ -13,9 +13,10 @@
 //   warp 5     (one lane) tcgen05.mma issuer: S = Q K^T, O += (hi + mid + lo) V with the weights read from TMEM, V MN-major as it lies;
 //   warp 6     zeros the value rows between the last position and the end of its box (the pool may hold anything there).
 // Bound: the fp32 work per score; the tensor pipe needs 1024 clocks per 128 x 64 scores at heads of 128. Caps and charges are applied in loops of
-// their own: with tanhf and log1pf inlined 64 times the code left the instruction cache (210 us where the loops take 81). Two scores per instruction where there is one that
-// takes two, and scores within a quarter of a cap through the series alone: capped prompts of 1000, 311, 700 and 37 tokens, 16 heads over 4 of 128, 84 -> 65 us; the queries
-// and the results moved in batches 65 -> 58. Clocks of a tile there: capping 1300, weights 1000, maximum 400, waiting for the products 2000; beside 4000 before the first
+// their own: with tanhf and log1pf inlined 64 times the code left the instruction cache (210 us, then, where the loops took 81). Two scores per instruction where there is one
+// that takes two, scores within a quarter of a cap through the series alone, the queries and the results moved in batches: prompts of 1000, 311, 700 and 37 tokens, 16 heads over 4
+// of 128, capped at 30, 85 -> 63 us (launches one behind the other in a captured graph; capped at 2, where most tiles are beyond a quarter of it, 85 -> 81; not capped 57 -> 54).
+// Clocks of a tile, capped: capping 1300, weights 1000, maximum 400, waiting for the products 2000; beside 4000 before the first
 // and 6000 behind the last. Further figures: attention_run.
 #include "seq_attn_decode.cuh"
 #include "tcgen05.cuh"

@@ -11,7 +11,7 @@ from . import _lib
 from .config import F32, BF16, INT8
 
 
-# The handle of the current stream of the current device, without the Python object around it: building that took 3 us of a call's 11 (matmul, 256 x 256).
+# The handle of the current stream of the current device, without the Python object around it: building that took 3 us of a call's 11 (matmul, int8, 2048 x 5632).
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
