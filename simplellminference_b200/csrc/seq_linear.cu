@@ -125,10 +125,16 @@ __global__ void __launch_bounds__(RowsShape<TT>::kWarps * 32, 1) seq_linear_rows
             }
     };
     if (blocks) begin_run(); else pad = 1 << 30;
+    // Half of the ring is asked for before the activations, the rest behind them; eight rows, whose activations take longer, ask for all of it. Measured against asking for all of it,
+    // launches one behind the other, means over nine shapes: one to four bf16 rows 2 to 3 % shorter, fp32 1 to 2 %; captured steps of one to four requests 0.3 to 3 % shorter, of
+    // eight (half, then the rest) 0 to 2 % longer.
+    constexpr int kFirst = TT == 8 ? D : D / 2;
 #pragma unroll
-    for (int i = 0; i < D; ++i) issue();
+    for (int i = 0; i < kFirst; ++i) issue();
     if (early) after_previous();
     load_act(0);
+#pragma unroll
+    for (int i = kFirst; i < D; ++i) issue();
 
     // after the exchange a lane holds the sum of row `which / TT` of the group and activation row `which % TT`
     int which = 0;
