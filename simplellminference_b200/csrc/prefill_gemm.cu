@@ -17,9 +17,11 @@
 // {k inside a K slice, row inside a tile, K slice, tile row}: prefill and decode share one copy of the weights.
 // Rows of the tiled layout are in unit order, so the two values an epilogue needs together (RoPE partners,
 // (up, gate)) sit in ADJACENT accumulator columns of the same thread.
-// The one-SM tile took its operands in at ~65 GB/s per SM with the tensor pipe half busy (profiles/r01_prefill_ncu_raw.md) — hence the two-SM tile; L2
-// prefetch and stream-K were measured and dropped. Two-SM tiles, 2048 x 12288 x 4096: 440 tiles fill the waves; 164 us alone and cold with the tensor pipe 79 % busy, 188 to
-// 194 us back to back.
+// Bound: the tensor pipe inside a tile (a 256 x 224 tile's k-block of 64 takes 461 clocks of the 448 its products need), beside that some 2 us until the first operands are there and
+// 4 us for the last tile's rows. What it took, measured back to back on matrices larger than L2 in turn, before | after: issuing loops without divisions (560 | 290 clocks per
+// k-block), rows written by whole lines (a k-block beside an epilogue 2400 | 600 clocks), and an epilogue without a loop that indexes the accumulator registers, which had put them
+// into local memory (1600 | 900 clocks per 32 columns). 2048 x 12288 x 4096: 186 | 143 us; 512 x 12288 x 4096: 65 | 46; 512 x 4096 x 4096: 31 | 20; 512 x 4096 x 11008: 64 | 41;
+// 2048 x 6176 x 2048: 66 | 43; 2048 x 2048 x 2048: 26 | 19. L2 prefetch and stream-K were measured and dropped, and so was asking for the next k-block's barrier in advance.
 #include <map>
 #include <tuple>
 
@@ -39,8 +41,9 @@ constexpr uint32_t kPfABytes = kPfBM * kPfBK * 2;
 // the host picks the BN that fills the last wave best, e.g. 192 instead of 256 for a 512 x 12288 output on 74 SM pairs.
 constexpr int kPfMaxStages = 12;
 constexpr uint32_t kPfRingBytes = 192 * 1024;          // operand ring; stages = ring / (A box + this CTA's W box)
+constexpr long long kPfWaitClocks = 1ll << 33;         // some 4 seconds
 constexpr uint32_t kPfTmemCols = 512;                  // two accumulators of up to 256 fp32 columns
-constexpr size_t kPfSmem = 1024 /*alignment slack*/ + kPfRingBytes + 512 /*barriers + tmem slot*/;
+constexpr size_t kPfSmem = 1024 /*alignment slack*/ + kPfRingBytes + 512 /*barriers + tmem slot*/ + 4 * 4096 /*rows on their way through the epilogue*/;
 
 struct PfDev {           // kernel-side view of PfGemmArgs
     int32_t T, N, m_tiles, n_tiles, BN;
@@ -50,28 +53,55 @@ struct PfDev {           // kernel-side view of PfGemmArgs
     int32_t epilogue;
     int32_t a_rows;       // rows of A one CTA stages per k-block: 128, or (one-SM kernel, T < 128) T rounded up to the 8-row swizzle period —
                           // the rest of the 128-row operand tile is never loaded (its accumulator rows are never stored)
-    float* out; int32_t ld_out, n_valid;
+    float* out; int32_t ld_out, n_valid, vec_out;   // vec_out: rows of out may be written 16 bytes at a time
     uint16_t* q_out; uint8_t *kc, *vc; int32_t kv_dtype, q_loc, kv_loc, hd, S, pos0;
     const float *sin_t, *cos_t;
     uint16_t* s_out; int32_t I_loc;
     const float* bias;
     const int32_t* rows_dev;   // the row tiles beyond ceil(*rows_dev / tile rows) are skipped by every role alike
     int32_t groups;            // matrices one behind the other, each with its own count in rows_dev; T and N are then those of one group
+    int32_t* status;           // where a wait that was given up is reported
 };
 
+// Bounded wait on a barrier: false once some seconds have passed or another thread of the CTA has given up. The kernel then tears down without its result and says so in the
+// library's status word. (By the clock and not by polls: a poll may sleep.)
+__device__ __forceinline__ bool pf_wait(uint64_t* bar, uint32_t parity, volatile int* gave_up) {
+    uint32_t done;
+    long long since = 0;
+    while (true) {
+        asm volatile(
+            "{\n.reg .pred p;\n"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+            "selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(done) : "r"(s_addr(bar)), "r"(parity) : "memory");
+        if (done) return true;
+        const long long now = clock64();
+        if (!since) since = now;
+        if (*gave_up || now - since > kPfWaitClocks) break;
+    }
+    *gave_up = 1;
+    return false;
+}
+
 // ------------------------------------------------------------------------------------------ PTX -------
-__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* tm, int c0, int c1, int c2, int c3, uint64_t* bar) {
-    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-                 ::"r"(s_addr(dst)), "l"(tm), "r"(s_addr(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+// PAIR: the cta_group::2 forms. The destination is this CTA's shared memory, the mbarrier may live in the peer CTA (shared::cluster address)
+template <bool PAIR>
+__device__ __forceinline__ void pf_load_2d(uint32_t dst, const CUtensorMap* tm, int c0, int c1, uint32_t bar) {
+    if constexpr (PAIR)
+        asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+                     ::"r"(dst), "l"(tm), "r"(bar), "r"(c0), "r"(c1) : "memory");
+    else
+        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+                     ::"r"(dst), "l"(tm), "r"(bar), "r"(c0), "r"(c1) : "memory");
 }
-// cta_group::2 forms: the destination is this CTA's shared memory, the mbarrier may live in the peer CTA (shared::cluster address)
-__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* tm, int c0, int c1, uint32_t bar_cluster_addr) {
-    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-                 ::"r"(s_addr(dst)), "l"(tm), "r"(bar_cluster_addr), "r"(c0), "r"(c1) : "memory");
-}
-__device__ __forceinline__ void tma_load_4d_pair(void* dst, const CUtensorMap* tm, int c0, int c1, int c2, int c3, uint32_t bar_cluster_addr) {
-    asm volatile("cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-                 ::"r"(s_addr(dst)), "l"(tm), "r"(bar_cluster_addr), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+template <bool PAIR>
+__device__ __forceinline__ void pf_load_4d(uint32_t dst, const CUtensorMap* tm, int c0, int c1, int c2, int c3, uint32_t bar) {
+    if constexpr (PAIR)
+        asm volatile("cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+                     ::"r"(dst), "l"(tm), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+    else
+        asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+                     ::"r"(dst), "l"(tm), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
 }
 __device__ __forceinline__ uint32_t cluster_ctarank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
 __device__ __forceinline__ uint32_t mapa_u32(const void* local, uint32_t cta) {   // shared::cluster address of `local` in CTA `cta`
@@ -107,40 +137,81 @@ __device__ __forceinline__ void tc_mma_bf16_pair(uint32_t d_tmem, uint64_t adesc
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) { return (uint32_t)f32_to_bf16_bits(lo) | ((uint32_t)f32_to_bf16_bits(hi) << 16); }
 
 // ------------------------------------------------------------------------------- fused epilogues ------
-// v[0..31] = accumulator columns n0 .. n0+31 of token row t (n0 is a multiple of 32)
-__device__ __forceinline__ void epi_store(const PfDev& p, int t, int n0, const uint32_t* v, bool add) {
-    float* dst = p.out + (size_t)t * p.ld_out + n0;
-    if (n0 + 32 <= p.n_valid && (p.ld_out & 3) == 0) {
+// All lanes of an epilogue warp call them together. v[0..31] = accumulator columns n0 .. n0+31 (n0 is a multiple of 32) of this lane's token row; `valid`: there is such a token.
+// A store of 16 bytes into each of 32 rows reaches the L2 as 32 half sectors, and while they were written that way the operands of the next tile waited behind them: a
+// k-block took 2400 clocks beside an epilogue and 580 without one. So rows change lanes first and whole lines (fp32) or sectors (bf16) are written.
+
+// fp32 rows: through `tr`, 4 KB of shared memory of this warp (16-byte pieces of a row in the XOR swizzle); eight lanes then write the 128 bytes of one row
+template <int MODE>      // 0 = store, 1 = add to what is there, 2 = reduction in L2 (no return value): for the partial sums of a split K
+__device__ __forceinline__ void epi_rows(const PfDev& p, uint32_t tr, int t0, int t_limit, int t_shift, int n0, const uint32_t* v, bool bias) {
+    const int lane = threadIdx.x & 31, sub = lane >> 3, c = lane & 7;
 #pragma unroll
-        for (int i = 0; i < 32; i += 4) {
-            float4 o = make_float4(__uint_as_float(v[i]), __uint_as_float(v[i + 1]), __uint_as_float(v[i + 2]), __uint_as_float(v[i + 3]));
-            if (add) {
-                const float4 r = *reinterpret_cast<const float4*>(dst + i);
-                o = make_float4(r.x + o.x, r.y + o.y, r.z + o.z, r.w + o.w);   // residual + projection (add_kernel.cpp:10-13)
-            }
-            *reinterpret_cast<float4*>(dst + i) = o;
+    for (int i = 0; i < 8; ++i)
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(tr + lane * 128 + ((i ^ c) << 4)), "r"(v[4 * i]), "r"(v[4 * i + 1]), "r"(v[4 * i + 2]), "r"(v[4 * i + 3]) : "memory");
+    __syncwarp();
+    const int n = n0 + 4 * c;
+    float4 x[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        const int row = 4 * r + sub;
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x[r].x), "=f"(x[r].y), "=f"(x[r].z), "=f"(x[r].w) : "r"(tr + row * 128 + ((c ^ (row & 7)) << 4)) : "memory");
+    }
+    __syncwarp();
+    if (bias) {
+        const float4 b = make_float4(n < p.n_valid ? p.bias[n] : 0.f, n + 1 < p.n_valid ? p.bias[n + 1] : 0.f, n + 2 < p.n_valid ? p.bias[n + 2] : 0.f, n + 3 < p.n_valid ? p.bias[n + 3] : 0.f);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) x[r] = make_float4(x[r].x + b.x, x[r].y + b.y, x[r].z + b.z, x[r].w + b.w);
+    }
+    float* dst = p.out + (size_t)(t0 + t_shift + sub) * p.ld_out + n;
+    const size_t step = 4 * (size_t)p.ld_out;
+    if (p.vec_out && n0 + 32 <= p.n_valid) {
+        if (MODE == 1) {                                   // residual + projection (add_kernel.cpp:10-13)
+            float4 y[8];
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+                if (t0 + 4 * r + sub < t_limit) y[r] = *reinterpret_cast<const float4*>(dst + r * step);
+#pragma unroll
+            for (int r = 0; r < 8; ++r) x[r] = make_float4(y[r].x + x[r].x, y[r].y + x[r].y, y[r].z + x[r].z, y[r].w + x[r].w);
+        }
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            if (t0 + 4 * r + sub >= t_limit) break;
+            if (MODE == 2)
+                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + r * step), "f"(x[r].x), "f"(x[r].y), "f"(x[r].z), "f"(x[r].w) : "memory");
+            else
+                *reinterpret_cast<float4*>(dst + r * step) = x[r];
         }
     } else {
-        for (int i = 0; i < 32; ++i)
-            if (n0 + i < p.n_valid) dst[i] = (add ? dst[i] : 0.f) + __uint_as_float(v[i]);
-    }
-}
-
-// split-K residual epilogue: out[t][n0..n0+31] += v, one vector reduction per 16 bytes (no return value, resolved in L2)
-__device__ __forceinline__ void epi_red_add(const PfDev& p, int t, int n0, const uint32_t* v) {
-    float* dst = p.out + (size_t)t * p.ld_out + n0;
-    if (n0 + 32 <= p.n_valid && (p.ld_out & 3) == 0) {
 #pragma unroll
-        for (int i = 0; i < 32; i += 4)
-            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + i), "f"(__uint_as_float(v[i])), "f"(__uint_as_float(v[i + 1])),
-                         "f"(__uint_as_float(v[i + 2])), "f"(__uint_as_float(v[i + 3])) : "memory");
-    } else {
-        for (int i = 0; i < 32; ++i)
-            if (n0 + i < p.n_valid) atomicAdd(dst + i, __uint_as_float(v[i]));
+        for (int r = 0; r < 8; ++r) {
+            if (t0 + 4 * r + sub >= t_limit) break;
+            const float e[4] = {x[r].x, x[r].y, x[r].z, x[r].w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (n + i < p.n_valid) {
+                    if (MODE == 2) atomicAdd(dst + r * step + i, e[i]);
+                    else dst[r * step + i] = MODE == 1 ? dst[r * step + i] + e[i] : e[i];
+                }
+        }
     }
 }
 
-__device__ __forceinline__ void epi_gateup(const PfDev& p, int t, int n0, const uint32_t* v) {
+// 32 bytes of every lane's own row at `own` (16-byte aligned; the neighbour's row lies `stride` bytes further for even lanes, before it for odd ones): a pair of lanes
+// writes the even lane's row first, then the odd one's, 32 bytes each time
+__device__ __forceinline__ void put_pair(uint8_t* own, ptrdiff_t stride, const uint4& a, const uint4& b, bool valid, bool peer_valid) {
+    const bool odd = threadIdx.x & 1;
+    uint4 s = odd ? a : b;
+    s.x = __shfl_xor_sync(0xffffffffu, s.x, 1);
+    s.y = __shfl_xor_sync(0xffffffffu, s.y, 1);
+    s.z = __shfl_xor_sync(0xffffffffu, s.z, 1);
+    s.w = __shfl_xor_sync(0xffffffffu, s.w, 1);
+    uint8_t* even_row = odd ? own - stride + 16 : own;
+    if (odd ? peer_valid : valid) *reinterpret_cast<uint4*>(even_row) = odd ? s : a;
+    if (odd ? valid : peer_valid) *reinterpret_cast<uint4*>(even_row + stride) = odd ? b : s;
+}
+__device__ __forceinline__ uint4 pack_bf16x8(const float* x) { return make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7])); }
+
+__device__ __forceinline__ void epi_gateup(const PfDev& p, int t, int n0, const uint32_t* v, bool valid, bool peer_valid) {
     const int u0 = n0 >> 1;
     float s[16];
 #pragma unroll
@@ -150,23 +221,22 @@ __device__ __forceinline__ void epi_gateup(const PfDev& p, int t, int n0, const 
     }
     uint16_t* dst = p.s_out + (size_t)t * p.I_loc + u0;
     if (u0 + 16 <= p.I_loc && (p.I_loc & 7) == 0) {
-        *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf16x2(s[0], s[1]), pack_bf16x2(s[2], s[3]), pack_bf16x2(s[4], s[5]), pack_bf16x2(s[6], s[7]));
-        *reinterpret_cast<uint4*>(dst + 8) = make_uint4(pack_bf16x2(s[8], s[9]), pack_bf16x2(s[10], s[11]), pack_bf16x2(s[12], s[13]), pack_bf16x2(s[14], s[15]));
-    } else {
+        put_pair(reinterpret_cast<uint8_t*>(dst), 2 * (ptrdiff_t)p.I_loc, pack_bf16x8(s), pack_bf16x8(s + 8), valid, peer_valid);
+    } else if (valid) {
+#pragma unroll
         for (int i = 0; i < 16; ++i)
             if (u0 + i < p.I_loc) dst[i] = f32_to_bf16_bits(s[i]);
     }
 }
 
-__device__ __forceinline__ void kv_store16(uint8_t* cache, int kv_dtype, size_t elem, const float* x) {   // 16 consecutive elements
-    if (kv_dtype == SLLM_BF16) {
-        uint4* d = reinterpret_cast<uint4*>(cache + elem * 2);
-        d[0] = make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));
-        d[1] = make_uint4(pack_bf16x2(x[8], x[9]), pack_bf16x2(x[10], x[11]), pack_bf16x2(x[12], x[13]), pack_bf16x2(x[14], x[15]));
+// 16 consecutive elements of a cache row per lane; the neighbour's row is the next position
+__device__ __forceinline__ void kv_store16(uint8_t* cache, const PfDev& p, size_t elem, const float* x, bool valid, bool peer_valid) {
+    if (p.kv_dtype == SLLM_BF16) {
+        put_pair(cache + elem * 2, 2 * (ptrdiff_t)p.hd, pack_bf16x8(x), pack_bf16x8(x + 8), valid, peer_valid);
     } else {
-        float4* d = reinterpret_cast<float4*>(cache + elem * 4);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) d[i] = make_float4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
+        const uint4* q = reinterpret_cast<const uint4*>(x);
+        put_pair(cache + elem * 4, 4 * (ptrdiff_t)p.hd, q[0], q[1], valid, peer_valid);
+        put_pair(cache + elem * 4 + 32, 4 * (ptrdiff_t)p.hd, q[2], q[3], valid, peer_valid);
     }
 }
 __device__ __forceinline__ void kv_store1(uint8_t* cache, int kv_dtype, size_t elem, float x) {
@@ -174,7 +244,7 @@ __device__ __forceinline__ void kv_store1(uint8_t* cache, int kv_dtype, size_t e
     else reinterpret_cast<float*>(cache)[elem] = x;
 }
 
-__device__ __forceinline__ void epi_qkv(const PfDev& p, int t, int n0, const uint32_t* v) {
+__device__ __forceinline__ void epi_qkv(const PfDev& p, int t, int n0, const uint32_t* v, bool valid, bool peer_valid) {
     const int half = p.hd >> 1, rope_units = (p.q_loc + p.kv_loc) >> 1, nunits = (p.q_loc + 2 * p.kv_loc) >> 1;
     const int u0 = n0 >> 1;
     const int pos = p.pos0 + t;
@@ -183,9 +253,10 @@ __device__ __forceinline__ void epi_qkv(const PfDev& p, int t, int n0, const uin
         // 16 units = 16 consecutive j of ONE head (half is a multiple of 16) or 32 consecutive V elements
         if (u0 < rope_units) {
             const int head = u0 / half, j0 = u0 - head * half;
-            const float4* sp = reinterpret_cast<const float4*>(p.sin_t + (size_t)pos * half + j0);
-            const float4* cp = reinterpret_cast<const float4*>(p.cos_t + (size_t)pos * half + j0);
-            float lo[16], hi[16];
+            const size_t at = (size_t)(valid ? pos : p.pos0) * half + j0;
+            const float4* sp = reinterpret_cast<const float4*>(p.sin_t + at);
+            const float4* cp = reinterpret_cast<const float4*>(p.cos_t + at);
+            alignas(16) float lo[16], hi[16];
 #pragma unroll
             for (int i4 = 0; i4 < 4; ++i4) {
                 const float4 s4 = sp[i4], c4 = cp[i4];
@@ -200,34 +271,32 @@ __device__ __forceinline__ void epi_qkv(const PfDev& p, int t, int n0, const uin
             }
             const int r0 = head * p.hd + j0;
             if (r0 < p.q_loc) {
-                uint16_t* q = p.q_out + (size_t)t * p.q_loc + r0;
-                uint4* a = reinterpret_cast<uint4*>(q);
-                uint4* b = reinterpret_cast<uint4*>(q + half);
-                a[0] = make_uint4(pack_bf16x2(lo[0], lo[1]), pack_bf16x2(lo[2], lo[3]), pack_bf16x2(lo[4], lo[5]), pack_bf16x2(lo[6], lo[7]));
-                a[1] = make_uint4(pack_bf16x2(lo[8], lo[9]), pack_bf16x2(lo[10], lo[11]), pack_bf16x2(lo[12], lo[13]), pack_bf16x2(lo[14], lo[15]));
-                b[0] = make_uint4(pack_bf16x2(hi[0], hi[1]), pack_bf16x2(hi[2], hi[3]), pack_bf16x2(hi[4], hi[5]), pack_bf16x2(hi[6], hi[7]));
-                b[1] = make_uint4(pack_bf16x2(hi[8], hi[9]), pack_bf16x2(hi[10], hi[11]), pack_bf16x2(hi[12], hi[13]), pack_bf16x2(hi[14], hi[15]));
+                uint8_t* q = reinterpret_cast<uint8_t*>(p.q_out + (size_t)t * p.q_loc + r0);
+                put_pair(q, 2 * (ptrdiff_t)p.q_loc, pack_bf16x8(lo), pack_bf16x8(lo + 8), valid, peer_valid);
+                put_pair(q + 2 * half, 2 * (ptrdiff_t)p.q_loc, pack_bf16x8(hi), pack_bf16x8(hi + 8), valid, peer_valid);
             } else {
                 const int kvh = (r0 - p.q_loc) / p.hd;
                 const size_t e0 = ((size_t)kvh * p.S + pos) * p.hd + j0;
-                kv_store16(p.kc, p.kv_dtype, e0, lo);
-                kv_store16(p.kc, p.kv_dtype, e0 + half, hi);
+                kv_store16(p.kc, p, e0, lo, valid, peer_valid);
+                kv_store16(p.kc, p, e0 + half, hi, valid, peer_valid);
             }
         } else {
             const int b2 = 2 * (u0 - rope_units);
             const int kvh = b2 / p.hd, j = b2 - kvh * p.hd;
             const size_t e0 = ((size_t)kvh * p.S + pos) * p.hd + j;
-            float x[32];
+            alignas(16) float x[32];
 #pragma unroll
             for (int i = 0; i < 32; ++i) x[i] = __uint_as_float(v[i]);
-            kv_store16(p.vc, p.kv_dtype, e0, x);
-            kv_store16(p.vc, p.kv_dtype, e0 + 16, x + 16);
+            kv_store16(p.vc, p, e0, x, valid, peer_valid);
+            kv_store16(p.vc, p, e0 + 16, x + 16, valid, peer_valid);
         }
         return;
     }
+    if (!valid) return;
+#pragma unroll                       // (a loop that indexes v would put it into local memory)
     for (int i = 0; i < 16; ++i) {   // generic shapes: unit by unit
         const int u = u0 + i;
-        if (u >= nunits) break;
+        if (u >= nunits) continue;
         const float a = __uint_as_float(v[2 * i]), b = __uint_as_float(v[2 * i + 1]);
         if (u < rope_units) {
             const int head = u / half, j = u - head * half;
@@ -274,6 +343,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
     uint64_t* tfull = empty + kPfMaxStages;     // [2] accumulator ready for the epilogue
     uint64_t* tempty = tfull + 2;     // [2] accumulator drained
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
+    volatile int* gave_up = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (warp == 0 && lane == 0) {
@@ -281,6 +351,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
         tma_prefetch_desc(&tmB);
         for (int s = 0; s < ST; ++s) { mb_init(full + s, 1); mb_init(empty + s, 1); }
         for (int a = 0; a < 2; ++a) { mb_init(tfull + a, 1); mb_init(tempty + a, PAIR ? 8 : 4); }
+        *gave_up = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) { if (PAIR) tc_alloc_pair(tmem_slot, kPfTmemCols); else tc_alloc(tmem_slot, kPfTmemCols); }
@@ -312,104 +383,111 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
     };
     Walk walk(p);
 
+    // One elected lane of either issuing warp runs its loop, with nothing in it that need not be: with an integer division and addresses made anew for every k-block either warp
+    // took 560 clocks for one, whatever its width (a 256 x 256 tile's products need 512, a 256 x 128 tile's 256); like this some 290. The lane waits by itself: a lane that
+    // only looked on could miss a phase while the elected one goes on.
     if (warp == 0) {
-        if (lane == 0) {   // ===== TMA producer =====
+        if (elect_one()) {     // ===== TMA producer =====
+            const uint32_t full_at = PAIR ? mapa_u32(full, 0) : s_addr(full), a_at = s_addr(sA), b_at = s_addr(sB);   // pair: both CTAs' bytes are counted on the LEADER's barriers
             int stage = 0;
             uint32_t phase = 0;
-            for (int unit = worker; walk.reach(unit); unit += nworkers) {
+            bool ok = true;
+            for (int unit = worker; ok && walk.reach(unit); unit += nworkers) {
                 const int tile = (unit - walk.base) / p.ksplit, part = (unit - walk.base) - tile * p.ksplit;
                 const int kb0 = (p.nkb * part) / p.ksplit, kb1 = (p.nkb * (part + 1)) / p.ksplit;
                 const int m_tile = tile % walk.m_tiles, n_tile = tile / walk.m_tiles;   // consecutive workers share the weight tile (L2)
                 const int row0 = walk.g * p.T + m_tile * BM + (int)rank * kPfBM;   // this CTA's 128 rows of A
                 const int n0 = walk.g * p.N + n_tile * BN + (int)rank * b_rows;    // this CTA's rows of W
+                const int w_row = p.tiled ? 0 : n0, w_tile = p.tiled ? n0 / p.R : 0;
+                int ks = kb0 / p.kb_per_seg, kk = kb0 - ks * p.kb_per_seg;
                 for (int kb = kb0; kb < kb1; ++kb) {
-                    mb_wait(empty + stage, phase ^ 1);
-                    const int ks = kb / p.kb_per_seg, kk = kb - ks * p.kb_per_seg;
-                    uint8_t* a_dst = sA + (size_t)stage * kPfABytes;
-                    uint8_t* b_dst = sB + (size_t)stage * b_bytes;
-                    if (PAIR) {
-                        // both CTAs' bytes are counted on the LEADER's barrier (it is the leader that issues the MMAs)
-                        if (rank == 0) mb_expect(full + stage, 2 * tx_bytes);
-                        const uint32_t bar = mapa_u32(full + stage, 0);
-                        tma_load_2d_pair(a_dst, &tmA, ks * p.seg_elems + kk * kPfBK, row0, bar);
-                        if (p.tiled) tma_load_4d_pair(b_dst, &tmB, kk * kPfBK, 0, ks, n0 / p.R, bar);
-                        else tma_load_4d_pair(b_dst, &tmB, kk * kPfBK, n0, 0, 0, bar);
-                    } else {
-                        mb_expect(full + stage, tx_bytes);
-                        tma_load_2d(a_dst, &tmA, ks * p.seg_elems + kk * kPfBK, row0, full + stage);
-                        if (p.tiled) tma_load_4d(b_dst, &tmB, kk * kPfBK, 0, ks, n0 / p.R, full + stage);
-                        else tma_load_4d(b_dst, &tmB, kk * kPfBK, n0, 0, 0, full + stage);
-                    }
+                    ok = pf_wait(empty + stage, phase ^ 1, gave_up);
+                    if (!ok) break;
+                    const uint32_t bar = full_at + 8 * stage;
+                    if (!PAIR) mb_expect(full + stage, tx_bytes);
+                    else if (rank == 0) mb_expect(full + stage, 2 * tx_bytes);
+                    pf_load_2d<PAIR>(a_at + (uint32_t)stage * kPfABytes, &tmA, ks * p.seg_elems + kk * kPfBK, row0, bar);
+                    pf_load_4d<PAIR>(b_at + (uint32_t)stage * b_bytes, &tmB, kk * kPfBK, w_row, ks, w_tile, bar);
+                    if (++kk == p.kb_per_seg) { kk = 0; ++ks; }
                     if (++stage == ST) { stage = 0; phase ^= 1; }
                 }
             }
         }
+        __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {   // ===== MMA issuer (pair: the leader CTA only) =====
+        if (rank == 0 && elect_one()) {   // ===== MMA issuer (pair: the leader CTA only) =====
             const uint32_t idesc = umma_idesc_bf16(BM, BN);
+            const uint64_t a_desc = umma_desc_sw128(sA), b_desc = umma_desc_sw128(sB);
             int stage = 0, acc = 0;
             uint32_t phase = 0, acc_phase = 0;
-            for (int unit = worker; walk.reach(unit); unit += nworkers) {
+            bool ok = true;
+            for (int unit = worker; ok && walk.reach(unit); unit += nworkers) {
                 const int part = (unit - walk.base) % p.ksplit;
-                const int kb0 = (p.nkb * part) / p.ksplit, kb1 = (p.nkb * (part + 1)) / p.ksplit;
-                mb_wait(tempty + acc, acc_phase ^ 1);   // the epilogue has drained this accumulator
+                const int n_kb = (p.nkb * (part + 1)) / p.ksplit - (p.nkb * part) / p.ksplit;
+                ok = pf_wait(tempty + acc, acc_phase ^ 1, gave_up);   // the epilogue has drained this accumulator
+                if (!ok) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + (uint32_t)(acc * 256);
-                for (int kb = kb0; kb < kb1; ++kb) {
-                    mb_wait(full + stage, phase);
+                for (int kb = 0; kb < n_kb; ++kb) {
+                    ok = pf_wait(full + stage, phase, gave_up);
+                    if (!ok) break;
                     tc_fence_after();
-                    const uint64_t ad = umma_desc_sw128(sA + (size_t)stage * kPfABytes);
-                    const uint64_t bd = umma_desc_sw128(sB + (size_t)stage * b_bytes);
+                    const uint64_t ad = a_desc + (uint64_t)((uint32_t)stage * (kPfABytes >> 4)), bd = b_desc + (uint64_t)((uint32_t)stage * (b_bytes >> 4));
 #pragma unroll
                     for (int k = 0; k < kPfBK / 16; ++k) {   // +32 bytes along K inside the 128-byte swizzle atom = +2 in the address field
-                        if (PAIR) tc_mma_bf16_pair(d_tmem, ad + (uint64_t)(2 * k), bd + (uint64_t)(2 * k), idesc, ((kb - kb0) | k) != 0);
-                        else tc_mma_bf16(d_tmem, ad + (uint64_t)(2 * k), bd + (uint64_t)(2 * k), idesc, ((kb - kb0) | k) != 0);
+                        if (PAIR) tc_mma_bf16_pair(d_tmem, ad + (uint64_t)(2 * k), bd + (uint64_t)(2 * k), idesc, (kb | k) != 0);
+                        else tc_mma_bf16(d_tmem, ad + (uint64_t)(2 * k), bd + (uint64_t)(2 * k), idesc, (kb | k) != 0);
                     }
                     if (PAIR) tc_commit_pair(empty + stage); else tc_commit(empty + stage);   // stage reusable once these MMAs have read it
                     if (++stage == ST) { stage = 0; phase ^= 1; }
                 }
+                if (!ok) break;
                 if (PAIR) tc_commit_pair(tfull + acc); else tc_commit(tfull + acc);           // accumulator complete
                 if (++acc == 2) { acc = 0; acc_phase ^= 1; }
             }
         }
+        __syncwarp();
     } else {               // ===== epilogue warps 2..5: TMEM lane quadrant = warp % 4 =====
         const int quad = warp & 3;
-        const int row = quad * 32 + lane;
+        const uint32_t tr = s_addr(smem + kPfRingBytes + 512 + quad * 4096);
         int acc = 0;
         uint32_t acc_phase = 0;
         const uint32_t tempty_leader[2] = {PAIR ? mapa_u32(tempty, 0) : 0u, PAIR ? mapa_u32(tempty + 1, 0) : 0u};
         for (int unit = worker; walk.reach(unit); unit += nworkers) {
             const int tile = (unit - walk.base) / p.ksplit;
             const int m_tile = tile % walk.m_tiles, n_tile = tile / walk.m_tiles;
-            const int t = m_tile * BM + (int)rank * kPfBM + row;
-            const int t_out = walk.g * p.T + t;
-            mb_wait(tfull + acc, acc_phase);
+            const int t0 = m_tile * BM + (int)rank * kPfBM + quad * 32, t = t0 + lane;
+            const bool bias = p.bias && (unit - walk.base) % p.ksplit == 0;   // the bias rides on the first share of K
+            // the warp goes on as one: what follows are instructions of all its lanes
+            if (!__all_sync(0xffffffffu, pf_wait(tfull + acc, acc_phase, gave_up))) break;
             tc_fence_after();
+            const uint32_t src = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * 256);
 #pragma unroll 1
             for (int c0 = 0; c0 < BN; c0 += 32) {
                 uint32_t v[32];
-                tc_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * 256 + c0), v);
+                __syncwarp();
+                tc_ld32(src + (uint32_t)c0, v);
+                if (c0 + 32 >= BN) {                     // the accumulator has been read: the next tile may have it
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) { if (PAIR) mb_arrive_cluster(tempty_leader[acc]); else mb_arrive(tempty + acc); }
+                }
                 const int n0 = n_tile * BN + c0;
-                if (t < p.T && n0 < p.N) {
-                    if (p.bias && (unit - walk.base) % p.ksplit == 0) {   // the bias rides on the first share of K
-#pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            if (n0 + i < p.n_valid) v[i] = __float_as_uint(__uint_as_float(v[i]) + p.bias[n0 + i]);
-                    }
-                    if (p.epilogue == PF_EPI_QKV) epi_qkv(p, t, n0, v);
-                    else if (p.epilogue == PF_EPI_GATEUP) epi_gateup(p, t, n0, v);
-                    else if (p.ksplit > 1) epi_red_add(p, t_out, n0, v);
-                    else epi_store(p, t_out, n0, v, p.epilogue == PF_EPI_RESID);
+                if (t0 < p.T && n0 < p.N) {
+                    if (p.epilogue == PF_EPI_QKV) epi_qkv(p, t, n0, v, t < p.T, (t ^ 1) < p.T);
+                    else if (p.epilogue == PF_EPI_GATEUP) epi_gateup(p, t, n0, v, t < p.T, (t ^ 1) < p.T);
+                    else if (p.ksplit > 1) epi_rows<2>(p, tr, t0, p.T, walk.g * p.T, n0, v, bias);
+                    else if (p.epilogue == PF_EPI_RESID) epi_rows<1>(p, tr, t0, p.T, walk.g * p.T, n0, v, bias);
+                    else epi_rows<0>(p, tr, t0, p.T, walk.g * p.T, n0, v, bias);
                 }
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) { if (PAIR) mb_arrive_cluster(tempty_leader[acc]); else mb_arrive(tempty + acc); }
             if (++acc == 2) { acc = 0; acc_phase ^= 1; }
         }
+        __syncwarp();
     }
     tc_fence_before();
     if (PAIR) cluster_sync_all(); else __syncthreads();   // pair: nobody leaves while the peer may still signal its barriers / read its operands
+    if (__syncthreads_or(*gave_up)) tc_gave_up(p.status);
     if (warp == 1) {
         tc_fence_after();
         if (PAIR) tc_dealloc_pair(tmem_base, kPfTmemCols); else tc_dealloc(tmem_base, kPfTmemCols);
@@ -546,11 +624,14 @@ int pf_gemm(PfCache* cache, const PfGemmArgs& a, cudaStream_t st) {
     p.BN = bn;
     p.n_tiles = pl.n_tiles;
     p.out = a.out; p.ld_out = a.ld_out; p.n_valid = a.n_valid;
+    p.vec_out = a.ld_out % 4 == 0 && ((uintptr_t)a.out % 16) == 0;
     p.q_out = a.q_out; p.kc = a.k_cache; p.vc = a.v_cache; p.kv_dtype = a.kv_dtype; p.q_loc = a.q_loc; p.kv_loc = a.kv_loc; p.hd = a.hd; p.S = a.S;
     p.pos0 = a.pos0; p.sin_t = a.sin_t; p.cos_t = a.cos_t; p.s_out = a.s_out; p.I_loc = a.I_loc;
     p.bias = (a.epilogue == PF_EPI_STORE || a.epilogue == PF_EPI_RESID || a.epilogue == PF_EPI_ACCUM) ? a.bias : nullptr;
     p.rows_dev = a.rows_dev;
     p.groups = groups;
+    if (int rc = status_check()) return rc;
+    if (int rc = status_word(&p.status)) return rc;
 
     CUtensorMap tmA;
     {
