@@ -17,8 +17,8 @@
 //                       of 1.72e-3 with scores four times as wide; mma.sync 2.29e-3 and 1.73e-3.)
 // TMEM: S0 | S1 | O0 | O1, 128 columns each. Bound: the tensor pipe and the exponentials, 1024 clocks each per 128 x 128 tile at head_dim 128, and the chain
 // scores -> softmax -> product of a tile; mma.sync, which it replaces for bf16 caches, spent them one after the other in the same warps. Measured, 2048
-// queries behind 6144 positions, 32 heads over 8 of 128: 317 us, 760 TFLOP/s (mma.sync 1061 us, 227; rescaling in the softmax warps, one body for masked and other
-// tiles and one value per instruction 391); 256 CTAs on 148 SMs leave a last wave of 108.
+// queries behind 6144 positions, 32 heads over 8 of 128: 292 us, 822 TFLOP/s (mma.sync 1061 us, 227; rescaling in the softmax warps, one body for masked and other
+// tiles and one value per instruction 391; descriptors made anew for every product 315); 256 CTAs on 148 SMs leave a last wave of 108.
 #include <type_traits>
 
 #include "prefill.cuh"
@@ -67,7 +67,8 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
 
     // this CTA's tiles: (head, first query) and the key tiles each has to see; the longest first
     const int bx = (int)gridDim.x - 1 - (int)blockIdx.x;
-    int head[2], t0[2], nkt[2], items = p.items;
+    int head[2], t0[2], nkt[2], items = p.items;       // (every loop over the tiles is unrolled: an index that is not a constant would put these into local memory)
+#pragma unroll
     for (int j = 0; j < 2; ++j) {
         head[j] = p.items == 2 && p.pair_heads ? 2 * (int)blockIdx.y + j : (int)blockIdx.y;
         const int tile = p.items == 2 && !p.pair_heads ? 2 * bx + j : bx;
@@ -97,10 +98,11 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
     pdl_launch_dependents();
 
     if (warp == 0) {
-        if (lane == 0) {   // ===== TMA producer =====
+        if (elect_one()) {   // ===== TMA producer =====
             mb_expect(qfull, (uint32_t)(items * Sh::kTileBytes));
-            for (int j = 0; j < items; ++j)
-                for (int c = 0; c < Sh::kBlocks; ++c) tma_load_2d(sQ + j * Sh::kTileBytes + c * Sh::kBlockBytes, &tmQ, head[j] * HD + 64 * c, t0[j], qfull);
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                for (int c = 0; j < items && c < Sh::kBlocks; ++c) tma_load_2d(sQ + j * Sh::kTileBytes + c * Sh::kBlockBytes, &tmQ, head[j] * HD + 64 * c, t0[j], qfull);
             for (int kt = 0; kt < kts; ++kt) {
                 const int s = kt % ST;
                 const uint32_t ph = (uint32_t)(kt / ST) & 1;
@@ -113,36 +115,41 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {   // ===== MMA issuer =====
+        if (elect_one()) {   // ===== MMA issuer: with descriptors at hand (made anew for each product they took 60 clocks apiece, as long as the product itself) =====
+            const uint64_t q_desc = umma_desc_sw128(sQ), k_desc = umma_desc_sw128(sK), v_desc = umma_desc_mn_sw128(sV, Sh::kBlockBytes);      // + bytes / 16: another place
             constexpr uint32_t idesc_s = umma_idesc_bf16(kTaTile, kTaTile), idesc_o = umma_idesc_bf16(kTaTile, HD) | (1u << 16);      // B MN-major
             auto scores = [&](int j, int kt) {
-                const uint8_t *q = sQ + j * Sh::kTileBytes, *k = sK + (kt % ST) * Sh::kTileBytes;
+                const uint64_t q = q_desc + (uint32_t)j * (Sh::kTileBytes / 16), k = k_desc + (uint32_t)(kt % ST) * (Sh::kTileBytes / 16);
 #pragma unroll
-                for (int ks = 0; ks < HD / 16; ++ks)
-                    tc_mma_bf16(tmem + 128 * j, umma_desc_sw128(q + (ks / 4) * Sh::kBlockBytes) + (uint64_t)(2 * (ks % 4)),
-                                umma_desc_sw128(k + (ks / 4) * Sh::kBlockBytes) + (uint64_t)(2 * (ks % 4)), idesc_s, ks != 0);
+                for (int ks = 0; ks < HD / 16; ++ks) {
+                    const uint32_t at = (ks / 4) * (Sh::kBlockBytes / 16) + 2 * (ks % 4);
+                    tc_mma_bf16(tmem + 128 * j, q + at, k + at, idesc_s, ks != 0);
+                }
                 tc_commit(sfull + j);
             };
             auto values = [&](int j, int kt) {
-                const uint8_t* v = sV + (kt % ST) * Sh::kTileBytes;
+                const uint64_t v = v_desc + (uint32_t)(kt % ST) * (Sh::kTileBytes / 16);
 #pragma unroll
                 for (int ks = 0; ks < kTaTile / 16; ++ks)
-                    tc_mma_bf16_ts(tmem + 256 + 128 * j, tmem + 128 * j + 8 * ks, umma_desc_mn_sw128(v + ks * 16 * 128, Sh::kBlockBytes), idesc_o, (kt | ks) != 0);
+                    tc_mma_bf16_ts(tmem + 256 + 128 * j, tmem + 128 * j + 8 * ks, v + (uint32_t)(ks * 128), idesc_o, (kt | ks) != 0);
                 tc_commit(odone + j);
             };
             bool ok = tc_wait(qfull, 0, gave_up, p.polls) && tc_wait(kfull, 0, gave_up, p.polls);
             if (ok) {
                 tc_fence_after();
-                for (int j = 0; j < items; ++j) scores(j, 0);
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+                    if (j < items) scores(j, 0);
                 tc_commit(kempty);
             }
             for (int kt = 0; ok && kt < kts; ++kt) {
                 ok = tc_wait(vfull + kt % ST, (uint32_t)(kt / ST) & 1, gave_up, p.polls);
                 bool keys = false;
-                for (int j = 0; ok && j < items; ++j) {
-                    if (kt >= nkt[j]) continue;
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    if (!ok || kt >= nkt[j]) continue;       // (a CTA's second tile has no key tiles where there is none)
                     ok = tc_wait(pready + j, (uint32_t)kt & 1, gave_up, p.polls);
-                    if (!ok) break;
+                    if (!ok) continue;
                     tc_fence_after();
                     values(j, kt);
                     if (kt + 1 >= nkt[j]) continue;
@@ -152,7 +159,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
                     }
                     // the next scores land where the weights lie that this product is still reading
                     ok = ok && tc_wait(odone + j, (uint32_t)kt & 1, gave_up, p.polls);
-                    if (!ok) break;
+                    if (!ok) continue;
                     tc_fence_after();
                     scores(j, kt + 1);
                 }
@@ -165,11 +172,12 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
         const int quad = warp & 3, row = quad * 32 + lane;
         bool ok = true;
         for (int kt = 0; ok && kt < kts; ++kt)
-            for (int j = 0; ok && j < items; ++j) {
-                if (kt >= nkt[j]) continue;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                if (!ok || kt >= nkt[j]) continue;
                 ok = tc_wait_warp(factors + j, (uint32_t)kt & 1, gave_up, p.polls);
                 if (ok && kt > 0) ok = tc_wait_warp(odone + j, (uint32_t)(kt - 1) & 1, gave_up, p.polls);     // long since: the scores follow that product
-                if (!ok) break;
+                if (!ok) continue;
                 tc_fence_after();
                 const float f = factor[j * kTaTile + row];
                 if (kt > 0 && __any_sync(0xffffffffu, f != 1.0f)) {
@@ -198,10 +206,10 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
                 mb_arrive(pready + j);
             }
     } else if (warp >= 4) {   // ===== softmax: TMEM lane quadrant = warp % 4 =====
-        const int j = (warp - 4) >> 2, quad = warp & 3, row = quad * 32 + lane;
+        const int j = (warp - 4) >> 2, quad = warp & 3, row = quad * 32 + lane, my_t0 = j ? t0[1] : t0[0], my_nkt = j ? nkt[1] : nkt[0], my_head = j ? head[1] : head[0];
         if (j < items) {
             const uint32_t lanes = (uint32_t)(quad * 32) << 16, s_tmem = tmem + lanes + 128 * j, o_tmem = tmem + lanes + 256 + 128 * j;
-            const int t = t0[j] + row, qpos = p.pos0 + t, first_pos = p.pos0 + t0[j] + quad * 32;
+            const int t = my_t0 + row, qpos = p.pos0 + t, first_pos = p.pos0 + my_t0 + quad * 32;
             const uint64_t scale2 = tc_two(__float_as_uint(p.scale_log2), __float_as_uint(p.scale_log2));
             float ref = -INFINITY, l = 0.0f;            // what the weights are relative to (log2 units); their sum
             bool ok = true;
@@ -271,7 +279,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
                 tc_split(tc_add2(sum0, sum1), l0, l1);
                 l += l0 + l1;
             };
-            for (int kt = 0; kt < nkt[j]; ++kt) {
+            for (int kt = 0; kt < my_nkt; ++kt) {
                 ok = tc_wait_warp(sfull + j, (uint32_t)kt & 1, gave_up, p.polls);
                 if (!ok) break;
                 tc_fence_after();
@@ -281,7 +289,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
                 tc_fence_before();
                 mb_arrive(pready + j);
             }
-            ok = ok && tc_wait_warp(odone + j, (uint32_t)(nkt[j] - 1) & 1, gave_up, p.polls);
+            ok = ok && tc_wait_warp(odone + j, (uint32_t)(my_nkt - 1) & 1, gave_up, p.polls);
             tc_fence_after();
             const float inv = 1.0f / l;
 #pragma unroll 1
@@ -290,7 +298,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
                 tc_ld32_async(o_tmem + c, o);
                 tc_arrived(o);
                 if (t < p.T) {
-                    uint4* dst = reinterpret_cast<uint4*>(p.out + (size_t)t * p.ldq + (size_t)head[j] * HD + c);
+                    uint4* dst = reinterpret_cast<uint4*>(p.out + (size_t)t * p.ldq + (size_t)my_head * HD + c);
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         auto two = [&](int e) { return tc_pack(__uint_as_float(o[8 * i + e]) * inv, __uint_as_float(o[8 * i + e + 1]) * inv); };

@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const _
     const int32_t* table = b.block_table + (size_t)slot * b.max_pages;
 
     if (warp == 4) {
-        if (lane == 0) {   // ===== TMA producer =====
+        if (elect_one()) {   // ===== TMA producer =====
             for (int i = 0; i < n; ++i) {
                 const int s = i % ST, j0 = tiles.tile_of(split + i * p.nsplit) * kSaKeys;
                 const uint32_t ph = (uint32_t)(i / ST) & 1;
@@ -150,14 +150,15 @@ __global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const _
             }
         }
     } else if (warp == 5) {
-        if (lane == 0) {   // ===== MMA issuer =====
+        if (elect_one()) {   // ===== MMA issuer: products of a tile leave one after the other only where their descriptors are at hand (made anew for each they took 60 clocks apiece, =====
+                             // a tile's scores twice as long as the tensor pipe needs for them) =====
             constexpr uint32_t idesc_s = umma_idesc_bf16(kSaRows, kSaKeys), idesc_o = umma_idesc_bf16(kSaRows, HD) | (1u << 16);      // B MN-major
+            const uint64_t q_desc = umma_desc_sw128(sQ), k_desc = umma_desc_sw128(sK), v_desc = umma_desc_mn_sw128(sV, Sh::kKBlock);  // + bytes / 16: another place
             auto scores = [&](int i) {
-                const uint8_t* k = sK + (i % ST) * Sh::kTile;
+                const uint64_t k = k_desc + (uint32_t)(i % ST) * (Sh::kTile / 16);
 #pragma unroll
                 for (int ks = 0; ks < HD / 16; ++ks)
-                    tc_mma_bf16(tmem, umma_desc_sw128(sQ + (ks / 4) * Sh::kQBlock) + (uint64_t)(2 * (ks % 4)), umma_desc_sw128(k + (ks / 4) * Sh::kKBlock) + (uint64_t)(2 * (ks % 4)),
-                                idesc_s, ks != 0);
+                    tc_mma_bf16(tmem, q_desc + (uint32_t)((ks / 4) * (Sh::kQBlock / 16) + 2 * (ks % 4)), k + (uint32_t)((ks / 4) * (Sh::kKBlock / 16) + 2 * (ks % 4)), idesc_s, ks != 0);
                 tc_commit(sfull);
                 tc_commit(kempty + i % ST);
             };
@@ -170,10 +171,10 @@ __global__ void __launch_bounds__(kSaThreads, 2) seq_attention_tc_kernel(const _
                 ok = tc_wait(vready + i % ST, (uint32_t)(i / ST) & 1, gave_up, sa.polls) && tc_wait(pready, (uint32_t)i & 1, gave_up, sa.polls);
                 if (!ok) break;
                 tc_fence_after();
-                const uint8_t* v = sV + (i % ST) * Sh::kTile;
+                const uint64_t v = v_desc + (uint32_t)(i % ST) * (Sh::kTile / 16);
 #pragma unroll
                 for (int ks = 0; ks < 3 * kSaKeys / 16; ++ks)                    // first terms, then second ones, then third ones, against the same values
-                    tc_mma_bf16_ts(tmem + 128, tmem + 8 * ks, umma_desc_mn_sw128(v + (ks % (kSaKeys / 16)) * 16 * 128, Sh::kKBlock), idesc_o, (i % kSaFlush | ks) != 0);
+                    tc_mma_bf16_ts(tmem + 128, tmem + 8 * ks, v + (uint32_t)((ks % (kSaKeys / 16)) * 128), idesc_o, (i % kSaFlush | ks) != 0);
                 tc_commit(odone);
                 tc_commit(vempty + i % ST);
                 if (i + 1 < n) {        // the next scores land where the weights lie that this product is still reading
