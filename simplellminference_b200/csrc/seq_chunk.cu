@@ -1,37 +1,40 @@
-// csrc/seq_chunk.cu — the delta rule (decay per head or per key channel) and linear attention with a constant decay, in blocks of 16 tokens
+// csrc/seq_chunk.cu — the delta rule (decay per head or per key channel) and linear attention with a constant decay, in blocks of 32 tokens
 // on the tensor cores: portions of prompts in bf16 mode. Within a block that starts from the state S0 [dk][dv], with G_i the running sum of
 // the logarithms of the decays (a vector over the key channels) up to token i,
 //     u_i = beta_i (v_i - S0^T (e^G_i k_i) - sum_{j<i} A_ij u_j),       A_ij = sum_c k_ic k_jc e^(G_ic - G_jc)
 //     o_i = S0^T (e^G_i q_i) + sum_{j<=i} B_ij u_j,                     B_ij = sum_c q_ic k_jc e^(G_ic - G_jc)
 //     S'  = e^G_n S0 + sum_j (e^(G_n - G_j) k_j) u_j^T
-// (e^G per key channel, i.e. on the rows of S). The u of a block solve a 16 x 16 triangular system, u = M (v - S0^T (e^G k)); linear attention
-// is the case M = 1, no S0 term in u. No factor exceeds 1: a difference of sums is formed before its exponential.
+// (e^G per key channel, i.e. on the rows of S). The u of a block solve a 32 x 32 triangular system, u = M (v - S0^T (e^G k)); linear attention
+// is the case M = 1, no S0 term in u. No factor exceeds 1: a difference of sums is formed before its exponential. The sums start anew at a block's middle, so that they stay as
+// small, and their differences as exact, as over 16 tokens.
 //
-// (1) seq_chunk_prepare_kernel, CTA = (block, head), all blocks of the step in parallel: silu / rotation / unit vectors, G, A and B (fp32,
-// a pair of threads per entry), M by forward substitution; leaves e^G k, e^G q, e^(G_n - G) k, M and B as the tensor-core fragments the walk
-// will load, each as two bf16 terms (x = hi + lo, |x - hi - lo| <= 2^-17 |x|), and e^G_n in fp32.
+// (1) seq_chunk_prepare_kernel, CTA = (block, head), all blocks of the step in parallel: silu / rotation / unit vectors, G, A and B (fp32, 4 x 4 entries and an eighth of the channels
+// per thread), M from the inverses of its two 16 x 16 triangles; leaves e^G k, e^G q, e^(G_n - G) k, M and B as the tensor-core fragments the walk
+// will load, each as two bf16 terms (x = hi + lo, |x - hi - lo| <= 2^-17 |x|), and e^G_n in fp32. Bound: shared memory's bandwidth and the exponentials: decays that are one number per
+// head multiply finished sums and whole rows (2048 tokens of 16 heads: 58 us with the decays inside the sums and blocks of 16 in two threads per entry, 43 like this).
 // (2) seq_chunk_walk_kernel, CTA = (portion, head, 16 or 32 value columns), two or four warps = 16 value columns, a share of the key channels each: their part of
 // S^T [16][dk] stays in the accumulators (fp32) from the portion's first token to its last. An accumulator fragment is register for register
 // an A fragment of the next product, so state and u never leave the registers; all products take both operands as two bf16 terms (three products, fp32 accumulation), which keeps
-// the recurrence at fp32 working accuracy. The blocks' records arrive by cp.async, three stages.
+// the recurrence at fp32 working accuracy (against float64 in the mean over 36 shapes and decays 0.85 of the error of blocks of 16 without the products of second terms). The blocks' records arrive by one bulk copy each, three stages. Bound: latency of a block's chain (products with the state, their exchange
+// between the warps, u, the state); a block of 32 takes hardly longer than one of 16 did (2048 tokens of 16 heads: 1.05 us for 16, 1.6 for 32, a walk 137 -> 103 us).
 #include "seq_attn.cuh"
 #include "seq_chunk.cuh"
+#include "mega_common.cuh"
 
 namespace sllm {
 
-constexpr int kPrepThreads = 288;    // two threads per entry of a triangle of 16 x 16
+constexpr int kPrepThreads = 288;    // eight threads per 4 x 4 entries of a triangle of 32 x 32
 constexpr int kWalkStages = 3;
 constexpr float kLog2e = 1.4426950408889634f;
 
 struct ChunkPlace { int seg, start, n, id; };      // segment, first token in the batch, tokens, number of the block in segment order
-__device__ __forceinline__ ChunkPlace chunk_place(const sllm_seq_batch& b, int item) {
+__device__ __forceinline__ ChunkPlace chunk_place(const sllm_seq_batch& b, int tile) {
     ChunkPlace c;
-    const int tile = item >> 1, half = item & 1;
     c.seg = b.qt_seg[tile];
-    const int off = b.qt_off[tile] + half * kChunk;
+    const int off = b.qt_off[tile];
     c.n = min(kChunk, b.seg_len[c.seg] - off);
     c.start = b.seg_start[c.seg] + off;
-    c.id = 2 * (b.seg_tile0[c.seg] + b.qt_off[tile] / 32) + half;
+    c.id = b.seg_tile0[c.seg] + off / kChunk;
     return c;
 }
 
@@ -43,20 +46,45 @@ __device__ __forceinline__ void chunk_put(uint8_t* hi, uint8_t* lo, int at, cons
     reinterpret_cast<uint4*>(hi)[at] = make_uint4(h[0], h[1], h[2], h[3]);
     reinterpret_cast<uint4*>(lo)[at] = make_uint4(l[0], l[1], l[2], l[3]);
 }
+__device__ __forceinline__ float4 chunk_scale(const float4& a, const float4& e) { return make_float4(a.x * e.x, a.y * e.y, a.z * e.z, a.w * e.w); }
+__device__ __forceinline__ float4 chunk_decay(const float4& a, const float4& b) { return make_float4(exp2f(a.x - b.x), exp2f(a.y - b.y), exp2f(a.z - b.z), exp2f(a.w - b.w)); }
+__device__ __forceinline__ float chunk_dot(const float4& a, const float4& b, float c) { return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, c)))); }
+
+// lanes with `bit` set keep (and complete) the upper half of 2 K values, the others the lower half
+template <int K, int N>
+__device__ __forceinline__ void chunk_halve(float (&v)[N], bool up, int bit) {
+#pragma unroll
+    for (int x = 0; x < K; ++x) {
+        const float give = up ? v[x] : v[x + K], keep = up ? v[x + K] : v[x];
+        v[x] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+    }
+}
+
+enum { kDecayConstant = 0, kDecayHead = 1, kDecayChannel = 2 };      // linear attention; the delta rule with one decay per head, per key channel
+template <int kMode, int dkp> struct ChunkPrepShared {               // floats
+    static constexpr int ld = dkp + 8, kRows = kChunk * ld, kTri = kChunk * (kChunk + 1);
+    static constexpr int kBytes = ((kMode == kDecayChannel ? 3 : 2) * kRows + (kMode == kDecayConstant ? 1 : 3) * kTri + 16 * 17) * 4;
+};
 
 // vec: rows of q, k, v (and of the channels' steps) may be read 16 bytes at a time
-template <bool kDelta, int dkp>
-__global__ void __launch_bounds__(kPrepThreads) seq_chunk_prepare_kernel(ChunkArgs p, int vec) {
+template <int kMode, int dkp>
+__global__ void __launch_bounds__(kPrepThreads, kMode == kDecayChannel ? 2 : 3) seq_chunk_prepare_kernel(ChunkArgs p, int vec) {
+    constexpr bool kDelta = kMode != kDecayConstant, kChannel = kMode == kDecayChannel;
+    using Sh = ChunkPrepShared<kMode, dkp>;
+    constexpr int ld = Sh::ld, H = kChunk / 2;
     extern __shared__ __align__(16) float cp_sm[];
-    __shared__ float s_A[kChunk][kChunk + 1], s_B[kChunk][kChunk + 1], s_M[kChunk][kChunk + 1], s_beta[kChunk];
+    __shared__ float s_beta[kChunk], s_g[kChunk], s_pre[kChunk], s_end[kChunk];
     const sllm_seq_batch& b = p.b;
     const ChunkPlace c = chunk_place(b, blockIdx.x);
     if (c.n <= 0) return;
     const int h = blockIdx.y, kvh = h / (p.heads / p.kv_heads), dk = p.dk;
-    constexpr int ld = dkp + 4;
-    float* s_k = cp_sm;                 // [16][ld]
-    float* s_q = s_k + kChunk * ld;     // [16][ld]
-    float* s_G = s_q + kChunk * ld;     // [16][ld], delta rule only
+    float* s_k = cp_sm;                             // [32][ld]
+    float* s_q = s_k + Sh::kRows;                   // [32][ld]
+    float* s_G = s_q + Sh::kRows;                   // [32][ld], a decay per channel only: sums of a half
+    float (*s_B)[kChunk + 1] = reinterpret_cast<float (*)[kChunk + 1]>(s_q + (kChannel ? 2 : 1) * Sh::kRows);
+    float (*s_A)[kChunk + 1] = s_B + kChunk;        // the delta rule only
+    float (*s_M)[kChunk + 1] = s_A + kChunk;
+    float (*s_T)[17] = reinterpret_cast<float (*)[17]>(s_M + kChunk);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const float rate = kDelta ? expf(p.A_log[h]) : p.rate[h];
     const float lg = -rate * kLog2e;    // constant decay: its base-2 logarithm
@@ -82,14 +110,12 @@ __global__ void __launch_bounds__(kPrepThreads) seq_chunk_prepare_kernel(ChunkAr
         }
         *reinterpret_cast<float4*>(s_k + tok * ld + ch) = kv;
         *reinterpret_cast<float4*>(s_q + tok * ld + ch) = qv;
-        if (kDelta) {
+        if (kChannel) {
             float4 g = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (has && p.channel) {
+            if (has) {
                 const float4 a = load4(p.al + t * p.lda + (size_t)h * dk, ch, true), bias = load4(p.dt_bias + (size_t)h * dk, ch, true);
                 g = make_float4(ch < dk ? lg * seq_softplus(a.x + bias.x) : 0.0f, ch + 1 < dk ? lg * seq_softplus(a.y + bias.y) : 0.0f,
                                 ch + 2 < dk ? lg * seq_softplus(a.z + bias.z) : 0.0f, ch + 3 < dk ? lg * seq_softplus(a.w + bias.w) : 0.0f);
-            } else if (has) {
-                g.x = g.y = g.z = g.w = lg * seq_softplus(p.al[t * p.lda + h] + p.dt_bias[h]);
             }
             *reinterpret_cast<float4*>(s_G + tok * ld + ch) = g;
         }
@@ -103,7 +129,28 @@ __global__ void __launch_bounds__(kPrepThreads) seq_chunk_prepare_kernel(ChunkAr
             else
                 for (int j = lane; j < p.dv; j += 32) dst[j] = src[j] * seq_sigmoid(src[j]);
         }
-    if (kDelta && threadIdx.x < kChunk) s_beta[threadIdx.x] = (int)threadIdx.x < c.n ? seq_sigmoid(p.bl[(size_t)(c.start + threadIdx.x) * p.ldb + h]) : 0.0f;
+    if (kDelta && warp == 8) {
+        const bool has = lane < c.n;
+        s_beta[lane] = has ? seq_sigmoid(p.bl[(size_t)(c.start + lane) * p.ldb + h]) : 0.0f;
+        if (!kChannel) {                                 // sums over either half, one token behind the other
+            const float g = has ? lg * seq_softplus(p.al[(size_t)(c.start + lane) * p.lda + h] + p.dt_bias[h]) : 0.0f;
+            float sum = 0.0f;
+#pragma unroll
+            for (int i = 0; i < H; ++i) {
+                const float x = __shfl_sync(0xffffffffu, g, (lane & H) + i);
+                if (i <= lane % H) sum += x;
+            }
+            const float first = __shfl_sync(0xffffffffu, sum, H - 1), second = __shfl_sync(0xffffffffu, sum, kChunk - 1);
+            s_g[lane] = sum;
+            s_pre[lane] = exp2f(lane < H ? sum : first + sum);
+            s_end[lane] = exp2f(lane < H ? (first - sum) + second : second - sum);
+        }
+    }
+    const int last = c.n - 1;
+    if (!kDelta && warp == 8) {
+        s_pre[lane] = exp2f(lg * (float)(min(lane, last) + 1));
+        s_end[lane] = exp2f(lg * (float)(last - min(lane, last)));
+    }
     __syncthreads();
     for (int tok = warp; tok < c.n; tok += kPrepThreads / 32) {
         float* kr = s_k + tok * ld;
@@ -134,68 +181,110 @@ __global__ void __launch_bounds__(kPrepThreads) seq_chunk_prepare_kernel(ChunkAr
                 for (int ch = lane; ch < dk; ch += 32) kr[ch] *= p.scale;
         }
     }
-    if (kDelta && threadIdx.x >= kPrepThreads - 128 && (int)threadIdx.x - (kPrepThreads - 128) < dkp) {   // running sums (a column no other thread touches)
-        float* col = s_G + threadIdx.x - (kPrepThreads - 128);
+    if (kChannel && (int)threadIdx.x < 2 * dkp) {        // running sums of a half (a column no other thread touches)
+        float* col = s_G + (threadIdx.x / dkp) * H * ld + threadIdx.x % dkp;
         float sum = 0.0f;
 #pragma unroll
-        for (int i = 0; i < kChunk; ++i) {
+        for (int i = 0; i < H; ++i) {
             sum += col[i * ld];
             col[i * ld] = sum;
         }
     }
     __syncthreads();
-    // the two matrices: two threads per entry (i >= j), each half of the channels in groups of four
+    // The two matrices: eight threads per 4 x 4 entries (rows ti, columns tj <= ti), each every eighth group of four channels. The sums of A and B change lanes in a halving
+    // exchange, after which a lane has N / 8 of them.
     {
-        const int e = threadIdx.x >> 1, part = threadIdx.x & 1;
-        int i = (int)((sqrtf(8.0f * e + 1.0f) - 1.0f) * 0.5f);
-        while ((i + 1) * (i + 2) / 2 <= e) ++i;
-        while (i * (i + 1) / 2 > e) --i;
-        const int j = e - i * (i + 1) / 2;
-        float a = 0.0f, bb = 0.0f;
-        if (i < kChunk) {
-            const float4 *ki = reinterpret_cast<const float4*>(s_k + i * ld), *kj = reinterpret_cast<const float4*>(s_k + j * ld), *qi = reinterpret_cast<const float4*>(s_q + i * ld);
-            const float4 *Gi = reinterpret_cast<const float4*>(s_G + i * ld), *Gj = reinterpret_cast<const float4*>(s_G + j * ld);
-            for (int g = part; g < dkp / 4; g += 2) {
-                float4 x = kj[g];
-                const float4 y = qi[g];
-                if (kDelta) {
-                    const float4 ga = Gi[g], gb = Gj[g], z = ki[g];
-                    x = make_float4(x.x * exp2f(ga.x - gb.x), x.y * exp2f(ga.y - gb.y), x.z * exp2f(ga.z - gb.z), x.w * exp2f(ga.w - gb.w));
-                    a = fmaf(z.x, x.x, fmaf(z.y, x.y, fmaf(z.z, x.z, fmaf(z.w, x.w, a))));
+        constexpr int N = kDelta ? 32 : 16;
+        const int e = threadIdx.x >> 3, kg = threadIdx.x & 7;
+        int ti = 0;
+        while ((ti + 1) * (ti + 2) / 2 <= e) ++ti;
+        const int tj = e - ti * (ti + 1) / 2;
+        const float *ki = s_k + 4 * ti * ld, *kj = s_k + 4 * tj * ld, *qi = s_q + 4 * ti * ld, *Gi = s_G + 4 * ti * ld, *Gj = s_G + 4 * tj * ld;
+        const bool cross = ti >= H / 4 && tj < H / 4;
+        float v[N];
+#pragma unroll
+        for (int x = 0; x < N; ++x) v[x] = 0.0f;
+        auto at = [](const float* row, int ch) { return *reinterpret_cast<const float4*>(row + ch); };
+        for (int ch = 4 * kg; ch < dkp; ch += 32) {
+            float4 x[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) x[j] = at(kj + j * ld, ch);
+            if (kChannel && ti != tj) {                  // decays from token j to the end of the first half, or to the tile's first row; from there on to token i
+                const float4 to = cross ? at(s_G + (H - 1) * ld, ch) : at(Gi, ch);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) x[j] = chunk_scale(x[j], chunk_decay(to, at(Gj + j * ld, ch)));
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float4 y = at(qi + i * ld, ch), z = y;
+                if (kDelta) z = at(ki + i * ld, ch);
+                if (kChannel) {
+                    const float4 g = at(Gi + i * ld, ch);
+                    if (ti != tj) {
+                        const float4 f = chunk_decay(g, cross ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : at(Gi, ch));
+                        y = chunk_scale(y, f);
+                        z = chunk_scale(z, f);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            if (j > i) continue;
+                            const float4 f = chunk_scale(x[j], chunk_decay(g, at(Gj + j * ld, ch)));
+                            v[4 * i + j] = chunk_dot(z, f, v[4 * i + j]);
+                            v[N - 16 + 4 * i + j] = chunk_dot(y, f, v[N - 16 + 4 * i + j]);
+                        }
+                        continue;
+                    }
                 }
-                bb = fmaf(y.x, x.x, fmaf(y.y, x.y, fmaf(y.z, x.z, fmaf(y.w, x.w, bb))));
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (kDelta) v[4 * i + j] = chunk_dot(z, x[j], v[4 * i + j]);
+                    v[N - 16 + 4 * i + j] = chunk_dot(y, x[j], v[N - 16 + 4 * i + j]);
+                }
             }
         }
-        a += __shfl_xor_sync(0xffffffffu, a, 1);
-        bb += __shfl_xor_sync(0xffffffffu, bb, 1);
-        if (i < kChunk && part == 0) {
-            s_A[i][j] = a;
-            s_B[i][j] = kDelta ? bb : bb * exp2f(lg * (float)(i - j));
-            if (i != j) s_B[j][i] = 0.0f;
+        chunk_halve<N / 2>(v, lane & 4, 4);
+        chunk_halve<N / 4>(v, lane & 2, 2);
+        chunk_halve<N / 8>(v, lane & 1, 1);
+#pragma unroll
+        for (int x = 0; x < N / 8; ++x) {
+            const int idx = (lane & 7) * (N / 8) + x, i = 4 * ti + idx / 4 % 4, j = 4 * tj + idx % 4;
+            float w = v[x];
+            if (kMode == kDecayConstant) w *= exp2f(lg * (float)(i - j));
+            if (kMode == kDecayHead) w *= exp2f(i >= H && j < H ? s_g[i] + (s_g[H - 1] - s_g[j]) : s_g[i] - s_g[j]);
+            if (kDelta && idx < 16) {
+                s_A[i][j] = w;
+            } else {
+                s_B[i][j] = i >= j ? w : 0.0f;
+                if (ti != tj) s_B[j][i] = 0.0f;
+            }
         }
     }
     __syncthreads();
     uint8_t* rec = p.ws + ((size_t)c.id * p.heads + h) * chunk_record_bytes(dkp);
-    const size_t plane = (size_t)kChunk * dkp * 2;
-    uint8_t* mats = rec + 6 * plane;                     // M hi, M lo, B hi, B lo: 512 bytes each
-    float* D = reinterpret_cast<float*>(mats + 4 * kChunk * kChunk * 2);
-    if (kDelta && warp == 0) {                           // M = (1 + diag(beta) A)^-1 diag(beta), lane = column
-        float m[kChunk];
+    constexpr size_t plane = (size_t)kChunk * dkp * 2;
+    uint8_t* mats = rec + 6 * plane;                     // M hi, M lo, B hi, B lo: the 16 x 16 blocks (0, 0), (1, 0) and (1, 1) of each, 512 bytes a block
+    float* D = reinterpret_cast<float*>(mats + 12 * 512);
+    if (kDelta && warp < 2) {                            // M = (1 + diag(beta) A)^-1 diag(beta) of either half, lane = column
+        const int o = warp * H;
+        float m[H];
 #pragma unroll
-        for (int i = 0; i < kChunk; ++i) {
+        for (int i = 0; i < H; ++i) {
             float acc = 0.0f;
 #pragma unroll
-            for (int l = 0; l < i; ++l) acc = fmaf(s_A[i][l], m[l], acc);
-            m[i] = s_beta[i] * ((i == lane ? 1.0f : 0.0f) - acc);
-            if (lane < kChunk) s_M[i][lane] = m[i];
+            for (int l = 0; l < i; ++l) acc = fmaf(s_A[o + i][o + l], m[l], acc);
+            m[i] = s_beta[o + i] * ((i == lane ? 1.0f : 0.0f) - acc);
+            if (lane < H) s_M[o + i][o + lane] = m[i];
         }
     }
-    const int last = c.n - 1;
-    // logarithm of the decay from the block's start to after token i, and from after token i to the block's end
-    auto G = [&](int i, int ch) { return kDelta ? s_G[i * ld + ch] : lg * (float)(min(i, last) + 1); };
-    constexpr int granules = dkp * 2;                    // 16-byte pieces of a plane: [k-step][lane]
-    for (int x = threadIdx.x; x < 3 * granules; x += kPrepThreads) {
-        const int which = x / granules, at = x % granules, ks = at >> 5, gr = (at & 31) >> 2, cc = at & 3;
+    // the decay from the block's start to after token i, and from after token i to the block's end
+    auto before = [&](int i, int ch) { return !kChannel ? s_pre[i] : exp2f(i < H ? s_G[i * ld + ch] : s_G[(H - 1) * ld + ch] + s_G[i * ld + ch]); };
+    auto behind = [&](int i, int ch) {
+        if (!kChannel) return s_end[i];
+        return exp2f(i < H ? (s_G[(H - 1) * ld + ch] - s_G[i * ld + ch]) + s_G[(kChunk - 1) * ld + ch] : s_G[(kChunk - 1) * ld + ch] - s_G[i * ld + ch]);
+    };
+    constexpr int granules = dkp * 4;                    // 16-byte pieces of a plane: [half of the tokens][k-step of channels][lane]
+    for (int x = threadIdx.x + (kDelta ? 0 : granules); x < 3 * granules; x += kPrepThreads) {     // (without a correction there is no S0 term in u)
+        const int which = x / granules, at = x % granules, pr = at / (granules / 2), ks = (at >> 5) % (dkp / 16), gr = (at & 31) >> 2, cc = at & 3;
         float v[8];
 #pragma unroll
         for (int y = 0; y < 4; ++y) {                    // pairs: (first / second group of 8) x (first / second half of the k-step)
@@ -203,47 +292,66 @@ __global__ void __launch_bounds__(kPrepThreads) seq_chunk_prepare_kernel(ChunkAr
             for (int half = 0; half < 2; ++half) {
                 const int outer = (y >> 1) * 8 + gr, inner = (y & 1) * 8 + 2 * cc + half;
                 if (which < 2) {
-                    const int tok = outer, ch = ks * 16 + inner;
-                    v[2 * y + half] = (which == 0 ? s_k : s_q)[tok * ld + ch] * exp2f(G(tok, ch));
+                    const int tok = pr * H + outer, ch = ks * 16 + inner;
+                    v[2 * y + half] = (which == 0 ? s_k : s_q)[tok * ld + ch] * before(tok, ch);
                 } else {
-                    const int tok = inner, ch = ks * 16 + outer;
-                    v[2 * y + half] = s_k[tok * ld + ch] * exp2f(G(last, ch) - G(tok, ch));
+                    const int tok = pr * H + inner, ch = ks * 16 + outer;
+                    v[2 * y + half] = s_k[tok * ld + ch] * behind(tok, ch);
                 }
             }
         }
-        if (!kDelta && which == 0) continue;             // no S0 term in u
         chunk_put(rec + 2 * which * plane, rec + (2 * which + 1) * plane, at, v);
     }
-    for (int ch = threadIdx.x; ch < dkp; ch += kPrepThreads) D[ch] = exp2f(G(last, ch));
-    __syncthreads();
-    for (int x = threadIdx.x; x < 64; x += kPrepThreads) {
-        const int which = x >> 5, gr = (x & 31) >> 2, cc = x & 3;
-        if (!kDelta && which == 0) continue;
+    for (int ch = threadIdx.x; ch < dkp; ch += kPrepThreads) D[ch] = before(kChannel ? kChunk - 1 : last, ch);
+    if (kDelta) {                                        // the block (1, 0) of M: -M(1,1) A(1,0) M(0,0)
+        __syncthreads();
+        const int i = threadIdx.x / H, j = threadIdx.x % H;
+        if (i < H) {
+            float acc = 0.0f;
+#pragma unroll
+            for (int l = 0; l < H; ++l) acc = fmaf(s_A[H + i][l], l >= j ? s_M[l][j] : 0.0f, acc);
+            s_T[i][j] = acc;
+        }
+        __syncthreads();
+        if (i < H) {
+            float acc = 0.0f;
+#pragma unroll
+            for (int l = 0; l < H; ++l) acc = fmaf(l <= i ? s_M[H + i][H + l] : 0.0f, s_T[l][j], acc);
+            s_M[H + i][j] = -acc;
+        }
+        __syncthreads();
+    }
+    for (int x = threadIdx.x + (kDelta ? 0 : 96); x < 192; x += kPrepThreads) {
+        const int which = x / 96, blk = (x >> 5) % 3, i0 = blk > 0 ? H : 0, j0 = blk > 1 ? H : 0, gr = (x & 31) >> 2, cc = x & 3;
         float v[8];
 #pragma unroll
         for (int y = 0; y < 4; ++y)
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
-                const int i = (y >> 1) * 8 + gr, j = (y & 1) * 8 + 2 * cc + half;
+                const int i = i0 + (y >> 1) * 8 + gr, j = j0 + (y & 1) * 8 + 2 * cc + half;
                 v[2 * y + half] = which == 0 ? s_M[i][j] : s_B[i][j];
             }
-        chunk_put(mats + 2 * which * 512, mats + (2 * which + 1) * 512, x & 31, v);
+        chunk_put(mats + (2 * which * 3 + blk) * 512, mats + ((2 * which + 1) * 3 + blk) * 512, x & 31, v);
     }
 }
 
-// three products of two-term operands: (ah + al) (bh + bl) without al * bl, each into an accumulator of its own (no product waits for another)
+// Products of two-term operands: (ah + al) (bh + bl), each term's into an accumulator of its own as far as there are three (no product waits for another). The product of the second
+// terms, as large as what two terms leave of an operand, is kept where u is an operand (kAll), and left out of the products with the old state.
+template <bool kAll>
 __device__ __forceinline__ void mma_split(float (&d)[4], float (&dl)[4], float (&dm)[4], const uint32_t (&ah)[4], const uint32_t (&al)[4], uint32_t h0, uint32_t h1, uint32_t l0, uint32_t l1) {
     mma_bf16_16816(d, ah, h0, h1);
     mma_bf16_16816(dl, al, h0, h1);
     mma_bf16_16816(dm, ah, l0, l1);
+    if (kAll) mma_bf16_16816(dl, al, l0, l1);
 }
 
 // KS: k-steps of 16 key channels. PARTS warps share 16 value columns, each owning KS / PARTS of the k-steps; they add their parts of the
-// products with the old state through shared memory and finish 16 / PARTS outputs per column each. GROUPS: how many times 16 columns a CTA takes.
+// products with the old state through shared memory and finish 32 / PARTS tokens each. GROUPS: how many times 16 columns a CTA takes.
 template <int KS, int PARTS, int GROUPS, bool kDelta>
-__global__ void __launch_bounds__(PARTS * GROUPS * 32) seq_chunk_walk_kernel(ChunkArgs p, int vec) {
+__global__ void __launch_bounds__(PARTS * GROUPS * 32, 1) seq_chunk_walk_kernel(ChunkArgs p, int vec) {
     extern __shared__ __align__(16) uint8_t cw_sm[];
-    constexpr int dkp = KS * 16, HS = KS / PARTS, kThreads = PARTS * GROUPS * 32, kCols = GROUPS * 16;
+    __shared__ uint64_t landed[kWalkStages];             // the records
+    constexpr int dkp = KS * 16, HS = KS / PARTS, kThreads = PARTS * GROUPS * 32, kCols = GROUPS * 16, kTiles = kChunk / 8;
     constexpr uint32_t kPlane = kChunk * dkp * 2;
     constexpr uint32_t rec_bytes = (uint32_t)chunk_record_bytes(dkp), stage_bytes = rec_bytes + kChunk * kCols * 4;
     const sllm_seq_batch& b = p.b;
@@ -254,19 +362,22 @@ __global__ void __launch_bounds__(PARTS * GROUPS * 32) seq_chunk_walk_kernel(Chu
     const int group = warp % GROUPS, part = warp / GROUPS, k0 = part * HS;   // this warp's value columns and first k-step
     const int cl = group * 16 + g, r0 = col0 + cl, r1 = r0 + 8;              // this thread's two value columns
     const bool ok0 = r0 < p.dv, ok1 = r1 < p.dv;
-    // what the warps of a group hand each other: [group][part][x, x, o, o][lane]
-    float4* exchange = reinterpret_cast<float4*>(cw_sm + kWalkStages * stage_bytes) + group * (PARTS * 4 * 32) + lane;
-    const size_t first = 2 * (size_t)b.seg_tile0[seg];   // number of the portion's first block
+    // what the warps of a group hand each other: [group][part][x of four tiles of 8 tokens, o of four][lane]
+    float4* exchange = reinterpret_cast<float4*>(cw_sm + kWalkStages * stage_bytes) + group * (PARTS * 2 * kTiles * 32) + lane;
+    const size_t first = (size_t)b.seg_tile0[seg];       // number of the portion's first block
     const uint8_t* recs = p.ws + (first * p.heads + h) * rec_bytes;
-    // values: the batch's rows, or those the preparation left (passed through silu), 16 rows per block
+    // values: the batch's rows, or those the preparation left (passed through silu), 32 rows per block
     const bool own_v = !kDelta && p.silu;
     const float* vsrc = own_v ? p.v_ws + first * kChunk * p.heads * p.dv + (size_t)h * p.dv + col0 : p.v + (size_t)start * p.ldv + (size_t)h * p.dv + col0;
     const size_t ldv = own_v ? (size_t)p.heads * p.dv : (size_t)p.ldv;
     auto issue = [&](int blk) {
         uint8_t* dst = cw_sm + (blk % kWalkStages) * stage_bytes;
-        const uint8_t* src = recs + (size_t)blk * p.heads * rec_bytes;
-#pragma unroll 4
-        for (uint32_t i = threadIdx.x + (kDelta ? 0 : 2 * kPlane / 16); i < rec_bytes / 16; i += kThreads) cp_async16(dst + 16 * i, src + 16 * i, 16);
+        if (threadIdx.x == 0) {
+            constexpr uint32_t skip = kDelta ? 0 : 2 * kPlane;
+            const uint8_t* src = recs + (size_t)blk * p.heads * rec_bytes;
+            mb_expect(landed + blk % kWalkStages, rec_bytes - skip);
+            tma_g2s(dst + skip, src + skip, rec_bytes - skip, landed + blk % kWalkStages);
+        }
         float* dv = reinterpret_cast<float*>(dst + rec_bytes);
         const int n = min(kChunk, len - blk * kChunk);
         const float* vb = vsrc + (size_t)blk * kChunk * ldv;
@@ -285,7 +396,12 @@ __global__ void __launch_bounds__(PARTS * GROUPS * 32) seq_chunk_walk_kernel(Chu
         }
         cp_async_commit();
     };
-    issue(0);
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kWalkStages; ++i) mb_init(landed + i, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    if (blocks > 0) issue(0);
     if (blocks > 1) issue(1);
     else cp_async_commit();
     float* st = p.state + ((size_t)slot * p.heads + h) * p.dk * p.dv;
@@ -298,26 +414,25 @@ __global__ void __launch_bounds__(PARTS * GROUPS * 32) seq_chunk_walk_kernel(Chu
             S[nt][e] = (e < 2 ? ok0 : ok1) && ch < p.dk ? st[(size_t)ch * p.dv + (e < 2 ? r0 : r1)] : 0.0f;
         }
     const bool work = col0 + group * 16 < p.dv;          // the same answer in all warps of a group
-    // the outputs this warp finishes: tokens mt * 8 + 2c and + 1 of columns r0 and r1 (two parts) or of one of them (four)
-    const int mt = PARTS == 4 ? part >> 1 : part, mrow = PARTS == 4 ? part & 1 : 0;
-    float* orow = p.o + (size_t)(start + mt * 8 + 2 * c) * p.ldo + (size_t)h * p.dv + (mrow ? r1 : r0);
+    float* orow = p.o + (size_t)(start + 2 * c) * p.ldo + (size_t)h * p.dv + r0;
     for (int blk = 0; blk < blocks; ++blk, orow += (size_t)kChunk * p.ldo) {
         cp_async_wait<1>();
+        mb_wait(landed + blk % kWalkStages, (uint32_t)(blk / kWalkStages) & 1);
         __syncthreads();                                 // this block has landed for everyone, and everyone has left the block before
         if (blk + 2 < blocks) issue(blk + 2);
         else cp_async_commit();
         if (!work) continue;
         const uint8_t* rec = cw_sm + (blk % kWalkStages) * stage_bytes;
-        const uint4* Kh = reinterpret_cast<const uint4*>(rec) + k0 * 32 + lane;
+        const uint4* Kh = reinterpret_cast<const uint4*>(rec) + k0 * 32 + lane;                 // second half of the tokens: KS * 32 pieces further
         const uint4* Kl = Kh + kPlane / 16;
         const uint4* Qh = Kl + kPlane / 16;
         const uint4* Ql = Qh + kPlane / 16;
         const uint4* Eh = Ql + kPlane / 16;              // keys decayed to the block's end
         const uint4* El = Eh + kPlane / 16;
-        const uint4* Mh = reinterpret_cast<const uint4*>(rec + 6 * kPlane) + lane;              // M hi, M lo, B hi, B lo: 32 pieces each
-        const float* D = reinterpret_cast<const float*>(rec + 6 * kPlane + 4 * kChunk * kChunk * 2) + k0 * 16 + 2 * c;
+        const uint4* Mh = reinterpret_cast<const uint4*>(rec + 6 * kPlane) + lane;              // M hi, M lo, B hi, B lo: three blocks of 32 pieces each
+        const float* D = reinterpret_cast<const float*>(rec + 6 * kPlane + 12 * 512) + k0 * 16 + 2 * c;
         const float* sv = reinterpret_cast<const float*>(rec + rec_bytes) + 2 * c * kCols + cl;
-        float x[2][4] = {}, xl[2][4] = {}, xm[2][4] = {}, o[2][4] = {}, ol[2][4] = {}, om[2][4] = {};     // rows r0 / r1, columns (tokens) nt * 8 + 2c, + 1
+        float x[kTiles][4] = {}, xl[kTiles][4] = {}, xm[kTiles][4] = {}, o[kTiles][4] = {}, ol[kTiles][4] = {}, om[kTiles][4] = {};     // rows r0 / r1, columns (tokens) nt * 8 + 2c, + 1
 #pragma unroll
         for (int ks = 0; ks < HS; ++ks) {
             uint32_t ah[4], al[4];
@@ -325,25 +440,27 @@ __global__ void __launch_bounds__(PARTS * GROUPS * 32) seq_chunk_walk_kernel(Chu
             split_bf16(S[2 * ks][2], S[2 * ks][3], &ah[1], &al[1]);
             split_bf16(S[2 * ks + 1][0], S[2 * ks + 1][1], &ah[2], &al[2]);
             split_bf16(S[2 * ks + 1][2], S[2 * ks + 1][3], &ah[3], &al[3]);
-            if (kDelta) {
-                const uint4 kh = Kh[ks * 32], kl = Kl[ks * 32];
-                mma_split(x[0], xl[0], xm[0], ah, al, kh.x, kh.y, kl.x, kl.y);
-                mma_split(x[1], xl[1], xm[1], ah, al, kh.z, kh.w, kl.z, kl.w);
+#pragma unroll
+            for (int pr = 0; pr < 2; ++pr) {
+                if (kDelta) {
+                    const uint4 kh = Kh[(pr * KS + ks) * 32], kl = Kl[(pr * KS + ks) * 32];
+                    mma_split<false>(x[2 * pr], xl[2 * pr], xm[2 * pr], ah, al, kh.x, kh.y, kl.x, kl.y);
+                    mma_split<false>(x[2 * pr + 1], xl[2 * pr + 1], xm[2 * pr + 1], ah, al, kh.z, kh.w, kl.z, kl.w);
+                }
+                const uint4 qh = Qh[(pr * KS + ks) * 32], ql = Ql[(pr * KS + ks) * 32];
+                mma_split<false>(o[2 * pr], ol[2 * pr], om[2 * pr], ah, al, qh.x, qh.y, ql.x, ql.y);
+                mma_split<false>(o[2 * pr + 1], ol[2 * pr + 1], om[2 * pr + 1], ah, al, qh.z, qh.w, ql.z, ql.w);
             }
-            const uint4 qh = Qh[ks * 32], ql = Ql[ks * 32];
-            mma_split(o[0], ol[0], om[0], ah, al, qh.x, qh.y, ql.x, ql.y);
-            mma_split(o[1], ol[1], om[1], ah, al, qh.z, qh.w, ql.z, ql.w);
         }
         auto sum3 = [](const float (&p0)[4], const float (&p1)[4], const float (&p2)[4]) {
             return make_float4(p0[0] + (p1[0] + p2[0]), p0[1] + (p1[1] + p2[1]), p0[2] + (p1[2] + p2[2]), p0[3] + (p1[3] + p2[3]));
         };
-        float4* mine = exchange + part * 4 * 32;
-        if (kDelta) {
-            mine[0] = sum3(x[0], xl[0], xm[0]);
-            mine[32] = sum3(x[1], xl[1], xm[1]);
+        float4* mine = exchange + part * 2 * kTiles * 32;
+#pragma unroll
+        for (int nt = 0; nt < kTiles; ++nt) {
+            if (kDelta) mine[nt * 32] = sum3(x[nt], xl[nt], xm[nt]);
+            mine[(kTiles + nt) * 32] = sum3(o[nt], ol[nt], om[nt]);
         }
-        mine[64] = sum3(o[0], ol[0], om[0]);
-        mine[96] = sum3(o[1], ol[1], om[1]);
 #pragma unroll
         for (int nt = 0; nt < 2 * HS; ++nt) {            // the old state decays to the block's end
             const float2 d = *reinterpret_cast<const float2*>(D + nt * 8);
@@ -352,19 +469,19 @@ __global__ void __launch_bounds__(PARTS * GROUPS * 32) seq_chunk_walk_kernel(Chu
             S[nt][2] *= d.x;
             S[nt][3] *= d.y;
         }
-        float v[2][4];
+        float v[kTiles][4];
 #pragma unroll
-        for (int nt = 0; nt < 2; ++nt)
+        for (int nt = 0; nt < kTiles; ++nt)
 #pragma unroll
             for (int e = 0; e < 4; ++e) v[nt][e] = sv[(nt * 8 + (e & 1)) * kCols + (e < 2 ? 0 : 8)];
         asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(PARTS * 32) : "memory");   // the warps of the group
         if (kDelta) {
 #pragma unroll
-            for (int nt = 0; nt < 2; ++nt) {
+            for (int nt = 0; nt < kTiles; ++nt) {
                 float4 y = exchange[nt * 32];
 #pragma unroll
                 for (int q = 1; q < PARTS; ++q) {
-                    const float4 z = exchange[(q * 4 + nt) * 32];
+                    const float4 z = exchange[(q * 2 * kTiles + nt) * 32];
                     y = make_float4(y.x + z.x, y.y + z.y, y.z + z.z, y.w + z.w);
                 }
                 v[nt][0] -= y.x;
@@ -373,60 +490,77 @@ __global__ void __launch_bounds__(PARTS * GROUPS * 32) seq_chunk_walk_kernel(Chu
                 v[nt][3] -= y.w;
             }
         }
-        uint32_t uh[4], ul[4];
-        auto operand = [&](const float (&y)[2][4]) {     // rows x 16 tokens as an A fragment
-            split_bf16(y[0][0], y[0][1], &uh[0], &ul[0]);
-            split_bf16(y[0][2], y[0][3], &uh[1], &ul[1]);
-            split_bf16(y[1][0], y[1][1], &uh[2], &ul[2]);
-            split_bf16(y[1][2], y[1][3], &uh[3], &ul[3]);
+        uint32_t uh[2][4], ul[2][4];
+        auto operand = [&](const float (&y)[kTiles][4]) {     // rows x 2 times 16 tokens as A fragments
+#pragma unroll
+            for (int pr = 0; pr < 2; ++pr) {
+                split_bf16(y[2 * pr][0], y[2 * pr][1], &uh[pr][0], &ul[pr][0]);
+                split_bf16(y[2 * pr][2], y[2 * pr][3], &uh[pr][1], &ul[pr][1]);
+                split_bf16(y[2 * pr + 1][0], y[2 * pr + 1][1], &uh[pr][2], &ul[pr][2]);
+                split_bf16(y[2 * pr + 1][2], y[2 * pr + 1][3], &uh[pr][3], &ul[pr][3]);
+            }
         };
         operand(v);
         if (kDelta) {
-            float u[2][4] = {}, lo[2][4] = {}, mid[2][4] = {};
-            const uint4 mh = Mh[0], ml = Mh[32];
-            mma_split(u[0], lo[0], mid[0], uh, ul, mh.x, mh.y, ml.x, ml.y);
-            mma_split(u[1], lo[1], mid[1], uh, ul, mh.z, mh.w, ml.z, ml.w);
+            float u[kTiles][4] = {}, lo[kTiles][4] = {}, mid[kTiles][4] = {};
 #pragma unroll
-            for (int nt = 0; nt < 2; ++nt)
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j <= i; ++j) {
+                    const uint4 mh = Mh[(i + j) * 32], ml = Mh[(3 + i + j) * 32];
+                    mma_split<true>(u[2 * i], lo[2 * i], mid[2 * i], uh[j], ul[j], mh.x, mh.y, ml.x, ml.y);
+                    mma_split<true>(u[2 * i + 1], lo[2 * i + 1], mid[2 * i + 1], uh[j], ul[j], mh.z, mh.w, ml.z, ml.w);
+                }
+#pragma unroll
+            for (int nt = 0; nt < kTiles; ++nt)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) u[nt][e] += lo[nt][e] + mid[nt][e];
             operand(u);
         }
+        float add[2 * HS][4] = {};                       // the products of second terms, in accumulators of their own: half as long a chain
 #pragma unroll
-        for (int ks = 0; ks < HS; ++ks) {
-            const uint4 eh = Eh[ks * 32], el = El[ks * 32];
-            mma_bf16_16816(S[2 * ks], uh, eh.x, eh.y);
-            mma_bf16_16816(S[2 * ks + 1], uh, eh.z, eh.w);
-            mma_bf16_16816(S[2 * ks], ul, eh.x, eh.y);
-            mma_bf16_16816(S[2 * ks + 1], ul, eh.z, eh.w);
-            mma_bf16_16816(S[2 * ks], uh, el.x, el.y);
-            mma_bf16_16816(S[2 * ks + 1], uh, el.z, el.w);
-        }
-        const uint4 bh = Mh[64], bl = Mh[96];
-        float y[4] = {}, yl[4] = {}, ym[4] = {};
-        if (mt == 0) mma_split(y, yl, ym, uh, ul, bh.x, bh.y, bl.x, bl.y);
-        else mma_split(y, yl, ym, uh, ul, bh.z, bh.w, bl.z, bl.w);
-        const int n = min(kChunk, len - blk * kChunk), tok = mt * 8 + 2 * c;
-        if (PARTS == 4) {                                // two tokens of one column
-            const float* at = reinterpret_cast<const float*>(exchange + (2 + mt) * 32) + 2 * mrow;
-            float2 z = *reinterpret_cast<const float2*>(at);
+        for (int pr = 0; pr < 2; ++pr)
+#pragma unroll
+            for (int ks = 0; ks < HS; ++ks) {
+                const uint4 eh = Eh[(pr * KS + ks) * 32], el = El[(pr * KS + ks) * 32];
+                mma_bf16_16816(S[2 * ks], uh[pr], eh.x, eh.y);
+                mma_bf16_16816(S[2 * ks + 1], uh[pr], eh.z, eh.w);
+                mma_bf16_16816(add[2 * ks], ul[pr], eh.x, eh.y);
+                mma_bf16_16816(add[2 * ks + 1], ul[pr], eh.z, eh.w);
+                mma_bf16_16816(add[2 * ks], uh[pr], el.x, el.y);
+                mma_bf16_16816(add[2 * ks + 1], uh[pr], el.z, el.w);
+                mma_bf16_16816(add[2 * ks], ul[pr], el.x, el.y);
+                mma_bf16_16816(add[2 * ks + 1], ul[pr], el.z, el.w);
+            }
+        // the outputs this warp finishes: tokens mt * 8 + 2c and + 1 of columns r0 and r1
+        const int n = min(kChunk, len - blk * kChunk);
+#pragma unroll
+        for (int m = 0; m < kTiles / PARTS; ++m) {
+            const int mt = m * PARTS + part, tok = mt * 8 + 2 * c, i = mt >> 1;
+            float y[4] = {}, yl[4] = {}, ym[4] = {};
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                if (j > i) continue;
+                const uint4 bh = Mh[(6 + i + j) * 32], bl = Mh[(9 + i + j) * 32];
+                if (mt & 1) mma_split<true>(y, yl, ym, uh[j], ul[j], bh.z, bh.w, bl.z, bl.w);
+                else mma_split<true>(y, yl, ym, uh[j], ul[j], bh.x, bh.y, bl.x, bl.y);
+            }
+            float4 z = exchange[(kTiles + mt) * 32];
 #pragma unroll
             for (int q = 1; q < PARTS; ++q) {
-                const float2 w = *reinterpret_cast<const float2*>(at + q * 4 * 32 * 4);
-                z = make_float2(z.x + w.x, z.y + w.y);
+                const float4 w = exchange[(q * 2 * kTiles + kTiles + mt) * 32];
+                z = make_float4(z.x + w.x, z.y + w.y, z.z + w.z, z.w + w.w);
             }
-            const float o0 = (mrow ? y[2] + (yl[2] + ym[2]) : y[0] + (yl[0] + ym[0])) + z.x, o1 = (mrow ? y[3] + (yl[3] + ym[3]) : y[1] + (yl[1] + ym[1])) + z.y;
-            if (mrow ? ok1 : ok0) {
-                if (tok < n) orow[0] = o0;
-                if (tok + 1 < n) orow[p.ldo] = o1;
-            }
-        } else {                                         // two tokens of both columns
-            const float4 z0 = exchange[(2 + mt) * 32], z1 = exchange[(4 + 2 + mt) * 32];
-            if (ok0 && tok < n) orow[0] = y[0] + (yl[0] + ym[0]) + (z0.x + z1.x);
-            if (ok0 && tok + 1 < n) orow[p.ldo] = y[1] + (yl[1] + ym[1]) + (z0.y + z1.y);
-            if (ok1 && tok < n) orow[8] = y[2] + (yl[2] + ym[2]) + (z0.z + z1.z);
-            if (ok1 && tok + 1 < n) orow[p.ldo + 8] = y[3] + (yl[3] + ym[3]) + (z0.w + z1.w);
+            float* to = orow + (size_t)(mt * 8) * p.ldo;
+            if (ok0 && tok < n) to[0] = y[0] + (yl[0] + ym[0]) + z.x;
+            if (ok0 && tok + 1 < n) to[p.ldo] = y[1] + (yl[1] + ym[1]) + z.y;
+            if (ok1 && tok < n) to[8] = y[2] + (yl[2] + ym[2]) + z.z;
+            if (ok1 && tok + 1 < n) to[p.ldo + 8] = y[3] + (yl[3] + ym[3]) + z.w;
         }
+#pragma unroll
+        for (int nt = 0; nt < 2 * HS; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) S[nt][e] += add[nt][e];
     }
 #pragma unroll
     for (int nt = 0; nt < 2 * HS; ++nt)
@@ -439,7 +573,7 @@ __global__ void __launch_bounds__(PARTS * GROUPS * 32) seq_chunk_walk_kernel(Chu
 
 template <int KS, int PARTS, int GROUPS, bool kDelta>
 static int launch_walk(const ChunkArgs& p, int vec, cudaStream_t st) {
-    constexpr size_t smem = kWalkStages * (chunk_record_bytes(KS * 16) + kChunk * GROUPS * 16 * 4) + GROUPS * PARTS * 4 * 32 * sizeof(float4);
+    constexpr size_t smem = kWalkStages * (chunk_record_bytes(KS * 16) + kChunk * GROUPS * 16 * 4) + GROUPS * PARTS * 2 * (kChunk / 8) * 32 * sizeof(float4);
     SLLM_CUDA(cudaFuncSetAttribute(seq_chunk_walk_kernel<KS, PARTS, GROUPS, kDelta>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     seq_chunk_walk_kernel<KS, PARTS, GROUPS, kDelta><<<dim3(p.b.nseg, p.heads, (p.dv + GROUPS * 16 - 1) / (GROUPS * 16)), PARTS * GROUPS * 32, smem, st>>>(p, vec);
     ++g_launches;
@@ -447,21 +581,30 @@ static int launch_walk(const ChunkArgs& p, int vec, cudaStream_t st) {
     return SLLM_OK;
 }
 
+template <int kMode, int dkp>
+static int launch_prepare_as(const ChunkArgs& p, int vec, cudaStream_t st) {
+    constexpr int smem = ChunkPrepShared<kMode, dkp>::kBytes;
+    SLLM_CUDA(cudaFuncSetAttribute(seq_chunk_prepare_kernel<kMode, dkp>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    seq_chunk_prepare_kernel<kMode, dkp><<<dim3(p.b.n_qtiles, p.heads), kPrepThreads, smem, st>>>(p, vec);
+    ++g_launches;
+    SLLM_LAUNCH_CHECK();
+    return SLLM_OK;
+}
+template <int kMode>
+static int launch_prepare(const ChunkArgs& p, int vec, cudaStream_t st) {
+    const int dkp = chunk_key(p.dk);
+    return dkp == 32 ? launch_prepare_as<kMode, 32>(p, vec, st) : dkp == 64 ? launch_prepare_as<kMode, 64>(p, vec, st) : dkp == 96 ? launch_prepare_as<kMode, 96>(p, vec, st)
+                                                                                                                                : launch_prepare_as<kMode, 128>(p, vec, st);
+}
+
 template <bool kDelta>
 static int launch_chunk_as(ChunkArgs p, cudaStream_t st) {
     const int dkp = chunk_key(p.dk);
-    p.v_ws = reinterpret_cast<float*>(p.ws + 2 * (size_t)p.b.n_qtiles * p.heads * chunk_record_bytes(dkp));
+    p.v_ws = reinterpret_cast<float*>(p.ws + (size_t)p.b.n_qtiles * p.heads * chunk_record_bytes(dkp));
     auto aligned = [](const void* q) { return ((uintptr_t)q % 16) == 0; };
     const int vec_prep = p.dk % 4 == 0 && p.dv % 4 == 0 && p.ldq % 4 == 0 && p.ldk % 4 == 0 && p.ldv % 4 == 0 && aligned(p.q) && aligned(p.k) && aligned(p.v) &&
                          (!p.channel || (p.lda % 4 == 0 && aligned(p.al) && aligned(p.dt_bias)));
-    const dim3 grid(2 * p.b.n_qtiles, p.heads);
-    const size_t smem = (size_t)3 * kChunk * (dkp + 4) * sizeof(float);
-    if (dkp == 32) seq_chunk_prepare_kernel<kDelta, 32><<<grid, kPrepThreads, smem, st>>>(p, vec_prep);
-    else if (dkp == 64) seq_chunk_prepare_kernel<kDelta, 64><<<grid, kPrepThreads, smem, st>>>(p, vec_prep);
-    else if (dkp == 96) seq_chunk_prepare_kernel<kDelta, 96><<<grid, kPrepThreads, smem, st>>>(p, vec_prep);
-    else seq_chunk_prepare_kernel<kDelta, 128><<<grid, kPrepThreads, smem, st>>>(p, vec_prep);
-    ++g_launches;
-    SLLM_LAUNCH_CHECK();
+    if (int rc = kDelta ? (p.channel ? launch_prepare<kDecayChannel>(p, vec_prep, st) : launch_prepare<kDecayHead>(p, vec_prep, st)) : launch_prepare<kDecayConstant>(p, vec_prep, st)) return rc;
     const bool own_v = !kDelta && p.silu;
     const int vec = p.dv % 4 == 0 && (own_v || (p.ldv % 4 == 0 && ((uintptr_t)p.v % 16) == 0));
     // a walk is a chain of dependent blocks: few heads are spread over the machine 16 value columns a CTA, many take 32 (every CTA of a head

@@ -1,0 +1,22 @@
+"""The recurrences in blocks of 32 tokens at the edges of a block and of its halves, whose sums and triangles are made apart: portions that end in the first half, at the middle, behind it
+and at the end, every width of key head that has a body of its own, against the restatement."""
+import numpy as np
+import pytest
+from test_nelutar_gpu import L, _rel, _scan_oracle, _scan_stub
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kind", ["head", "channel", "lightning"])
+@pytest.mark.parametrize("dk,dv", [(32, 16), (64, 64), (96, 33), (128, 128)])
+def test_portions_that_end_anywhere_in_a_block(kind, dk, dv):
+    rng = np.random.default_rng(dk + dv)
+    H, portions = 2, [16, 17, 31, 32, 33, 47, 48, 49, 64, 65]
+    decay = np.linspace(0.9, 0.99, H).astype(np.float32)
+    consts = {"A_log": rng.uniform(-3, 1, size=H).astype(np.float32), "decay": decay, "decay64": decay.astype(np.float64), "rate": (-np.log(decay.astype(np.float64))).astype(np.float32),
+              "dt_bias": rng.uniform(-3, 3, size=H * dk if kind == "channel" else H).astype(np.float32)}
+    stub, sizes, rot = _scan_stub(kind, H, H, dk, dv, consts, True)
+    x = rng.standard_normal((sum(portions), sum(sizes))).astype(np.float32)
+    got = L.feed(stub, x, portions)[0]
+    # two bf16 terms leave 2^-17 of an operand, three operands stand between the state and a result: as the test of whole recurrences
+    assert _rel(got, _scan_oracle(kind, x, sizes, H, H, dk, dv, consts, rot)) < 5e-5
