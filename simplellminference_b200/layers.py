@@ -391,7 +391,9 @@ class GatedDeltaRule:
         ops.delta_rule(step.b, u.data_ptr(), C, u.data_ptr() + nk * F32B, C, u.data_ptr() + 2 * nk * F32B, C, bl, ld, al, ld, self.a_log, self.dt_bias,
                        c.heads, c.kv_heads, c.dim, c.vdim, self.unit_eps, c.dim ** -0.5, state["S"], o, self.width, q, ld, C, c.conv, ring, step.st,
                        chunk_ws=step.chunk_scratch(c.heads, c.dim, c.vdim))
-        ops.headnorm_gate(o.data_ptr(), self.width, g, ld, self.norm_w, c.heads, c.vdim, self.eps, out, self.width, T, step.st)
+        rows16 = self.out.operand_rows(step)
+        ops.headnorm_gate(o.data_ptr(), self.width, g, ld, self.norm_w, c.heads, c.vdim, self.eps, None if rows16 is not None else out, self.width, T, step.st, out16=rows16)
+        return rows16 is not None
 
 
 class ChannelDeltaRule:
