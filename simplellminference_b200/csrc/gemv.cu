@@ -31,6 +31,71 @@ struct PlainPolicyT : PlainPolicy {
 template <int WD>
 __global__ void __launch_bounds__(kGemvThreads) gemv_plain_kernel(PlainPolicyT<WD> pol) { gemv_body<WD>(pol); }
 
+// Few rows: `parts` (2, 4 or 8) neighbouring warps cut the columns of a pair of rows among themselves, so that all of the matrix is asked for at once where a warp per pair leaves SMs
+// without work and takes its rows in several trips. Bound: the latency of one trip behind the launch. The partial sums meet in shared memory in a fixed order.
+template <int WD>
+__global__ void __launch_bounds__(kGemvThreads, 2) gemv_split_kernel(PlainPolicyT<WD> pol, int parts, int group_shift) {
+    extern __shared__ __align__(16) float smem[];
+    __shared__ float2 part_sum[kGemvWarps];
+    constexpr int E = WInfo<WD>::E;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, part = warp % parts;
+    const int unit = (blockIdx.x * kGemvWarps + warp) / parts;
+    const int nchunks = pol.ncols / E, per = (nchunks + parts - 1) / parts, lo = part * per, hi = min(nchunks, lo + per);
+    const int cpg = WD == SLLM_INT8 ? pol.grp / 16 : 1, groups = WD == SLLM_INT8 ? pol.ncols / pol.grp : 0;
+    const bool live = unit < pol.units();
+    int64_t r0 = 0, r1 = 0;
+    if (live) pol.rows(unit, r0, r1);
+    const uint4 *w0 = reinterpret_cast<const uint4*>(pol.W_) + r0 * nchunks, *w1 = reinterpret_cast<const uint4*>(pol.W_) + r1 * nchunks;
+    const float *sc0 = pol.sc + r0 * groups, *sc1 = pol.sc + r1 * groups;
+    Batch<WD> cur;
+    auto load = [&](int base) {
+#pragma unroll
+        for (int u = 0; u < kGemvU; ++u) {
+            const int c = base + u * 32 + lane;
+            const bool has = live && c < hi;
+            cur.w0[u] = has ? ldg_stream(w0 + c) : make_uint4(0, 0, 0, 0);
+            cur.w1[u] = has ? ldg_stream(w1 + c) : make_uint4(0, 0, 0, 0);
+            if (WD == SLLM_INT8) {
+                const int g = group_shift >= 0 ? c >> group_shift : c / cpg;
+                cur.s0[u] = has ? __ldg(sc0 + g) : 0.0f;
+                cur.s1[u] = has ? __ldg(sc1 + g) : 0.0f;
+            }
+        }
+    };
+    load(lo);
+    pol.stage(smem, smem + pol.ncols);
+    __syncthreads();
+    const float4* xs4 = reinterpret_cast<const float4*>(smem);
+    float a0 = 0.0f, a1 = 0.0f;
+    for (int base = lo; base < hi; base += 32 * kGemvU) {
+#pragma unroll
+        for (int u = 0; u < kGemvU; ++u) {
+            const int c = base + u * 32 + lane;
+            if (c < hi) {
+                if (WD == SLLM_INT8) {
+                    a0 = fmaf(chunk_dot<WD>(cur.w0[u], xs4, c, nchunks, 0.0f), cur.s0[u], a0);
+                    a1 = fmaf(chunk_dot<WD>(cur.w1[u], xs4, c, nchunks, 0.0f), cur.s1[u], a1);
+                } else {
+                    a0 = chunk_dot<WD>(cur.w0[u], xs4, c, nchunks, a0);
+                    a1 = chunk_dot<WD>(cur.w1[u], xs4, c, nchunks, a1);
+                }
+            }
+        }
+        if (base + 32 * kGemvU < hi) load(base + 32 * kGemvU);
+    }
+    a0 = warp_sum(a0);
+    a1 = warp_sum(a1);
+    if (lane == 0) part_sum[warp] = make_float2(a0, a1);
+    __syncthreads();
+    if (live && part == 0 && lane == 0) {
+        for (int i = 1; i < parts; ++i) {
+            a0 += part_sum[warp + i].x;
+            a1 += part_sum[warp + i].y;
+        }
+        pol.emit(unit, a0, a1);
+    }
+}
+
 template <int WD>
 static int launch_plain(const PlainPolicy& p, cudaStream_t st) {
     const size_t smem = gemv_smem_bytes(p.ncols);
@@ -42,7 +107,25 @@ static int launch_plain(const PlainPolicy& p, cudaStream_t st) {
     }
     PlainPolicyT<WD> pt;
     static_cast<PlainPolicy&>(pt) = p;
-    const int grid = gemv_grid((p.nrows + 1) / 2, 2);
+    // As many warps a pair of rows as still fit two CTAs per SM at once and leave each lane a load of 16 bytes. Measured, us a call one behind the other, a warp per pair | like this: fp32 2048 x 5632
+    // 13.9 | 11.8, 1500 x 5632 12.2 | 9.9, 2300 x 11008 22.1 | 20.0; bf16 1500 x 5632 9.7 | 8.2, 2300 x 11008 15.9 | 13.9; int8 1500 x 5632 9.7 | 7.8, 2300 x 11008 12.7 | 12.4; the kernel alone,
+    // int8 256 x 4096 5.0 | 3.9, 2048 x 5632 7.0 | 6.5. One warp a pair from 2369 rows on: 4096 x 4096 the same.
+    const int units = (p.nrows + 1) / 2, chunks = p.ncols / WInfo<WD>::E, warps = 2 * kGemvWarps * sm_count();
+    int parts = 1;
+    while (parts < kGemvWarps && 2LL * parts * units <= warps && chunks / (2 * parts) >= 32) parts *= 2;
+    if (parts > 1 && g_tune_ctas_per_sm == 0) {
+        static size_t split_configured = 0;
+        if (smem + 64 > 48 * 1024 && smem > split_configured) {
+            SLLM_CUDA(cudaFuncSetAttribute(gemv_split_kernel<WD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            split_configured = smem;
+        }
+        const int cpg = WD == SLLM_INT8 ? p.grp / 16 : 1;
+        gemv_split_kernel<WD><<<(units * parts + kGemvWarps - 1) / kGemvWarps, kGemvThreads, smem, st>>>(pt, parts, (cpg & (cpg - 1)) == 0 ? __builtin_ctz(cpg) : -1);
+        g_launches++;
+        SLLM_LAUNCH_CHECK();
+        return SLLM_OK;
+    }
+    const int grid = gemv_grid(units, 2);
     gemv_plain_kernel<WD><<<grid, kGemvThreads, smem, st>>>(pt);
     g_launches++;
     SLLM_LAUNCH_CHECK();
