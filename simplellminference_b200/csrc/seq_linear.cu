@@ -1,5 +1,5 @@
 // csrc/seq_linear.cu — sllm_seq_linear: C = alpha * (A . W^T + bias) (+ C) for the ragged token batch. Three bodies:
-//   * rows_kernel  (T <= 8, decode-sized steps): every weight streamed once, the activations of a lane's columns in registers; a body without that
+//   * rows kernels (T <= 8, decode-sized steps): every weight streamed once past activations in registers, bf16 ones of several rows through the tensor cores; a body without that
 //     set-up for small matrices, with scalar loads where 16-byte accesses do not fit;
 //   * tile_kernel  (any shape): 64 x 64 x 16 shared-memory tiles, 4 x 4 outputs per thread, fp32 FMAs with fp32 accumulation. This is
 //     the body of the all-fp32 mode, and of bf16 products whose shape the tensor-core tiles do not take;
@@ -8,8 +8,10 @@
 //     run as a short epilogue kernel over C.
 // In bf16 mode (round_a) the activations are rounded to bf16 as they are loaded, so all three bodies multiply the same operands and
 // differ only in summation order.
+#include <type_traits>
+
 #include "prefill.cuh"
-#include "seq_common.cuh"
+#include "seq_attn.cuh"
 
 namespace sllm {
 
@@ -218,6 +220,158 @@ __global__ void __launch_bounds__(RowsShape<TT>::kWarps * 32, 1) seq_linear_rows
             const float val = p.alpha * (sum + (bias ? bias[n] : 0.0f));
             float* c = out + (size_t)t * p.ldc + n;
             *c = p.accumulate ? *c + val : val;
+        }
+    }
+}
+
+// Up to 8 activation rows, rounded to bf16, against a stream of bf16 weight rows on the tensor cores: mma.sync m16n8k16 with 8 weight rows as the columns. Bound: HBM, every weight is read
+// once. One CTA per SM takes a contiguous share of the weight rows; WK = 2^wk_log2 of its 16 warps cut K among themselves, 256 columns each of a panel of K, the others take other
+// tiles of 8 rows. The activations stay in registers; the weights arrive through cp.async in a ring of each warp's own, 16 rows of 512 bytes (128 KB an SM), and leave it through ldmatrix.
+// A weight costs a fortieth of an instruction of each kind where fma.rn.f32x2 and the exchange between lanes took a tenth, and the same for one row as for eight.
+// Accuracy: the tensor core truncates its sums. So an activation is split into its upper and its lower four significant bits, which go through as rows 0..7 and 8..15: products of 12
+// bits, whose sums of 16 fit a result's 24 but for columns 2^8 below the largest; each starts from zero and is added with ordinary rounding, and the warps' sums meet in double.
+// Error against float64, streaming body | this one: 8.2e-8 | 5.4e-8 (K = 4096), 1.03e-7 | 6.4e-8 (11008), 5.5e-8 | 5.1e-8 (264); unsplit it was 9.9e-8.
+constexpr int kMmaWarps = 16, kMmaSlice = 256, kMmaSteps = kMmaSlice / 32, kMmaHalves = 4, kMmaHalf = 4 * 2 * kMmaSlice, kMmaRing = kMmaHalves * kMmaHalf, kMmaStage = 8 * kMmaSlice;      // bytes: half a tile, ring of a warp, half of its columns' activations
+__host__ __device__ __forceinline__ int mma_block_rows(int WR) { return WR <= 2 ? 48 : WR <= 8 ? 64 : 128; }      // weight rows between two flushes of the partial sums: whole rounds of tiles
+// a pair of bf16 values as a pair of their upper four significant bits and one of the lower four
+__device__ __forceinline__ void mma_halves(uint32_t a, uint32_t& hi, uint32_t& lo) {
+    hi = a & 0xfff0fff0u;
+    asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(lo) : "r"(a), "r"(hi));
+}
+__device__ __forceinline__ void mma_fragments(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__global__ void __launch_bounds__(kMmaWarps * 32, 1) seq_linear_rows_mma_kernel(LinArgs p, int wk_log2) {
+    extern __shared__ __align__(16) uint8_t mma_smem[];        // rings, 2 KB a warp for activations on their way, then [2][WK][8 activation rows][block + 8] partial sums
+    const int b = blockIdx.y;
+    const bool early = p.w_fixed && !p.w_index;
+    if (!early) after_previous();
+    const int wb = p.w_index ? p.w_index[b] : b;               // which matrix of W; negative: none (the outputs are zeros)
+    const float* A = p.A + (size_t)(p.a_div > 1 ? b / p.a_div : b) * p.a_bs;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
+    const int WK = 1 << wk_log2, WR = kMmaWarps >> wk_log2, wk = warp & (WK - 1), wr = warp >> wk_log2, block = mma_block_rows(WR), ldt = block + 8;
+    const int n_lo = (int)((long long)p.N * blockIdx.x / gridDim.x), rows = (int)((long long)p.N * (blockIdx.x + 1) / gridDim.x) - n_lo;
+    const int K = wb >= 0 ? p.K : 0, panel = WK * kMmaSlice, panels = max(1, (K + panel - 1) / panel), blocks = (rows + block - 1) / block;
+    const uint32_t ring = smem_u32(mma_smem) + warp * kMmaRing;
+    float* table = reinterpret_cast<float*>(mma_smem + kMmaWarps * (kMmaRing + kMmaStage));
+
+    struct Unit { int blk, pan, row; };                        // a tile of this warp: block, panel, first row in the block
+    auto settle = [&](Unit& x) {                               // on to one that has rows, or past the last block
+        while (x.blk < blocks && x.row >= min(block, rows - x.blk * block)) {
+            x.row = 8 * wr;
+            if (++x.pan == panels) {
+                x.pan = 0;
+                ++x.blk;
+            }
+        }
+    };
+    Unit u{0, 0, 8 * wr};
+    settle(u);
+    Unit ahead = u;                                            // the tile being asked for, half by half
+    int half = 0;
+    uint32_t fill = ring;
+    // this lane's 16 bytes of weight row 0
+    const uint8_t* W = reinterpret_cast<const uint8_t*>(p.W) + (((size_t)max(wb, 0) * p.w_bs + (size_t)n_lo * p.ldw + wk * kMmaSlice + 8 * lane) << 1);
+    const size_t row_bytes = (size_t)p.ldw * 2;
+    const int K0 = K - wk * kMmaSlice - 8 * lane;              // columns from there on
+    auto issue = [&]() {
+        if (ahead.blk < blocks) {
+            const int row = ahead.blk * block + ahead.row + 4 * half;
+            const int left = ahead.pan * panel < K0 ? rows - row : 0;      // rows that are there
+            const uint8_t* src = left > 0 ? W + row * row_bytes + (size_t)(2 * ahead.pan * panel) : reinterpret_cast<const uint8_t*>(p.W);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(fill + r * (2 * kMmaSlice) + ((lane ^ (4 * half + r)) << 4)), "l"(src), "r"(r < left ? 16 : 0) : "memory");
+                if (r + 1 < left) src += row_bytes;
+            }
+            if (half) {
+                ahead.row += 8 * WR;
+                settle(ahead);
+            }
+            half ^= 1;
+            fill = fill + kMmaHalf == ring + kMmaRing ? ring : fill + kMmaHalf;
+        }
+        cp_async_commit();
+    };
+    const int mr = lane & 7;                                   // row of this lane's addresses for ldmatrix, and its 16-byte piece, swizzled
+    const uint32_t piece = (uint32_t)(((lane >> 3) ^ mr) << 4);
+    // The activations of this warp's columns as fragments: rows of 128 columns at a time through shared memory (a load of 8 bytes per lane and fragment touched eight lines each: 2 us
+    // for eight rows of 4096). Rows from T on hold what is there: they meet no other row.
+    uint32_t act[kMmaSteps][4];
+    auto load_act = [&](int pan) {
+        const uint32_t stage = smem_u32(mma_smem) + kMmaWarps * kMmaRing + warp * kMmaStage;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int k = pan * panel + wk * kMmaSlice + h * (kMmaSlice / 2) + 4 * lane;
+            float4 x[8];
+#pragma unroll
+            for (int t = 0; t < 8; ++t) x[t] = t < p.T && k < K ? *reinterpret_cast<const float4*>(A + (size_t)t * p.lda + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+            __syncwarp();
+#pragma unroll
+            for (int t = 0; t < 8; ++t)
+                asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(stage + t * kMmaSlice + (((lane >> 1) ^ t) << 4) + (lane & 1) * 8), "r"(pack_bf16(x[t].x, x[t].y)),
+                             "r"(pack_bf16(x[t].z, x[t].w)) : "memory");
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < kMmaSteps / 2; ++i) mma_fragments(act[h * (kMmaSteps / 2) + i], stage + mr * kMmaSlice + (piece ^ (64u * i)));
+        }
+    };
+#pragma unroll
+    for (int i = 0; i < kMmaHalves; ++i) issue();
+    if (early) after_previous();
+    load_act(0);
+    uint32_t take = ring;
+    for (int blk = 0; blk < blocks; ++blk) {
+        const int n = min(block, rows - blk * block);
+        float* tab = table + (size_t)(blk & 1) * WK * 8 * ldt;
+        for (int pan = 0; pan < panels; ++pan) {
+            if (panels > 1 && pan + blk > 0) load_act(pan);
+            while (u.blk == blk && u.pan == pan) {
+                cp_async_wait<kMmaHalves - 2>();
+                __syncwarp();
+                const uint32_t second = take + kMmaHalf == ring + kMmaRing ? ring : take + kMmaHalf;
+                const uint32_t from = (mr < 4 ? take : second) + (mr & 3) * (2 * kMmaSlice);
+                float s[4] = {};
+#pragma unroll
+                for (int i = 0; i < kMmaSteps; ++i) {
+                    uint32_t w[4];                             // columns 32 i + 8 m + 2 c, + 1 of weight row g
+                    mma_fragments(w, from + (piece ^ (64u * i)));
+#pragma unroll
+                    for (int m = 0; m < 4; m += 2) {
+                        float d[4];
+                        uint32_t a[4];
+                        mma_halves(act[i][m], a[0], a[1]);
+                        mma_halves(act[i][m + 1], a[2], a[3]);
+                        mma_bf16_zero(d, a, w[m], w[m + 1]);
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) s[q] += d[q];
+                    }
+                }
+                __syncwarp();
+                issue();
+                issue();
+                take = second + kMmaHalf == ring + kMmaRing ? ring : second + kMmaHalf;
+                float2* cell = reinterpret_cast<float2*>(tab + (size_t)(wk * 8 + g) * ldt + u.row + 2 * c);
+                float2 v = make_float2(s[0] + s[2], s[1] + s[3]);
+                if (pan) {
+                    const float2 o = *cell;
+                    v = make_float2(o.x + v.x, o.y + v.y);
+                }
+                *cell = v;
+                u.row += 8 * WR;
+                settle(u);
+            }
+        }
+        __syncthreads();
+        const float* bias = p.bias ? p.bias + (size_t)b * p.bias_bs : nullptr;
+        float* out = p.C + (size_t)b * p.c_bs;
+        for (int o = threadIdx.x; o < n * p.T; o += kMmaWarps * 32) {
+            const int t = o / n, r = o % n, at = n_lo + blk * block + r;
+            double sum = 0.0;
+            for (int k = 0; k < WK; ++k) sum += (double)tab[(size_t)(k * 8 + t) * ldt + r];
+            const float val = p.alpha * ((float)sum + (bias ? bias[at] : 0.0f));
+            float* to = out + (size_t)t * p.ldc + at;
+            *to = p.accumulate ? *to + val : val;
         }
     }
 }
@@ -453,6 +607,21 @@ static int launch_rows_body(const sllm::LinArgs& p, int batch, cudaStream_t st) 
     return SLLM_OK;
 }
 
+static int launch_rows_mma(const sllm::LinArgs& p, int batch, cudaStream_t st) {
+    using namespace sllm;
+    int wk_log2 = 0;      // as many warps along K as one panel of it needs
+    while ((1 << wk_log2) < kMmaWarps && (kMmaSlice << wk_log2) < p.K) ++wk_log2;
+    auto smem = [](int wk) { return kMmaWarps * (kMmaRing + kMmaStage) + 2 * ((8 * (mma_block_rows(kMmaWarps >> wk) + 8) * (int)sizeof(float)) << wk); };
+    static bool sized = false;
+    if (!sized) {
+        SLLM_CUDA(cudaFuncSetAttribute(seq_linear_rows_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem(4)));
+        sized = true;
+    }
+    const dim3 grid(std::max(1, std::min(p.N, sm_count() / batch)), batch);
+    overlapping(seq_linear_rows_mma_kernel)<<<grid, kMmaWarps * 32, smem(wk_log2), st>>>(p, wk_log2);
+    return SLLM_OK;
+}
+
 // the rows body: up to 8 activation rows per product, `batch` products
 static int launch_rows(const sllm::LinArgs& p, int batch, cudaStream_t st) {
     using namespace sllm;
@@ -471,9 +640,16 @@ static int launch_rows(const sllm::LinArgs& p, int batch, cudaStream_t st) {
     const bool stream = vec && (p.T <= 4          ? weights >= 1500000LL
                                 : bf16 ? p.T <= 6 ? weights >= 2800000LL && rows >= 4 * sms : weights >= 2000000LL
                                                   : (weights >= 2800000LL && rows >= 10 * sms) || (p.T >= 7 && weights >= 4500000LL && rows >= 4 * sms));
-    if (stream) {
+    // bf16 rows on the tensor cores. Measured in a captured graph, us, small body | streaming | this one: two rows 1024 x 1024 3.9 | 4.5 | 4.3, 1536 x 1024 5.3 | 4.6 | 4.3, 2800 x 1024
+    // 6.6 | 5.8 | 5.2, 2048 x 2048 7.3 | 5.9 | 5.9, 6144 x 4096 26.6 | 12.1 | 13.4; three rows 512 x 4096 5.3 | 6.3 | 5.5, 1024 x 1024 4.3 | 5.7 | 4.4, 2048 x 1024 6.6 | 6.2 | 4.9;
+    // four rows 512 x 1024 3.6 | 5.8 | 4.4, 1024 x 1024 4.6 | 5.9 | 4.4, 6144 x 4096 45 | 14.1 | 13.9, 2048 x 5632, which takes two panels of K, 20.6 | 10.6 | 11.5; six rows 512 x 1024 4.1 | 7.6 | 4.6; eight rows 512 x 1024 4.7 | 8.0 | 4.7,
+    // 2048 x 2048 13.3 | 11.8 | 6.5, 6144 x 4096 84 | 23.5 | 14.7, 16384 x 4096 140 | 46.5 | 27.8, 1000 x 11008 34 | 24.9 | 13.9. One row is streamed: 6144 x 4096 18.7 | 11.5 | 13.3.
+    const bool mma = vec && bf16 && p.round_a && (p.T >= 5 || (p.K <= kMmaWarps * kMmaSlice && (p.T == 4 || (p.T >= 2 && rows >= 4 * sms && (p.T == 3 || weights <= 3000000LL)))));
+    const long long mma_from = p.T <= 3 ? 1200000LL : p.T == 4 ? 900000LL : p.T <= 6 ? 750000LL : 500000LL;
+    if (mma ? weights >= mma_from : stream) {
         int rc;
-        if (p.T == 1) rc = bf16 ? launch_rows_body<SLLM_BF16, 1>(p, batch, st) : launch_rows_body<SLLM_F32, 1>(p, batch, st);
+        if (mma) rc = launch_rows_mma(p, batch, st);
+        else if (p.T == 1) rc = bf16 ? launch_rows_body<SLLM_BF16, 1>(p, batch, st) : launch_rows_body<SLLM_F32, 1>(p, batch, st);
         else if (p.T == 2) rc = bf16 ? launch_rows_body<SLLM_BF16, 2>(p, batch, st) : launch_rows_body<SLLM_F32, 2>(p, batch, st);
         else if (p.T <= 4) rc = bf16 ? launch_rows_body<SLLM_BF16, 4>(p, batch, st) : launch_rows_body<SLLM_F32, 4>(p, batch, st);
         else rc = bf16 ? launch_rows_body<SLLM_BF16, 8>(p, batch, st) : launch_rows_body<SLLM_F32, 8>(p, batch, st);
