@@ -561,13 +561,21 @@ int sllm_seq_rotary_kv(const sllm_seq_batch* b, float* q, int32_t ldq, int32_t h
 // time, so they pay only when the step has no more of them than fit at once. Measured (us) at 16 | 8 | 4 CTAs: one request of 8000 positions, 8 kv
 // heads 17.9 | 23.4 | 35.0; four of 2048, 4 kv heads 17.6 | 11.2 | 13.1; with twice as many CTAs 32 requests of 2048 take 54 instead of 47.
 template <typename Kernel, typename... Args>
-static int launch_attention_decode(Kernel* kernel, int G, int smem, const sllm::AttnArgs& p, cudaStream_t st, Args... args) {
+static int launch_attention_decode(Kernel* kernel, int G, int smem, sllm::AttnArgs p, bool foldable, cudaStream_t st, Args... args) {
     using namespace sllm;
     const long long items = (long long)p.b.n_qtiles * (p.heads / G) * p.nsplit;
     int cs = items * kDecodeCluster <= sm_count() ? kDecodeCluster : kDecodeCluster / 2;
     while (cs > 1 && (items * cs > 2LL * sm_count() || (long long)p.nsplit * cs > 65535)) cs /= 2;
+    // clusters of up to eight CTAs, two rounds of them at most, that the kernel may fold to those of one round (it looks at the contexts)
+    const bool heads_first = foldable && p.b.n_qtiles <= 65535;
+    p.fold = heads_first ? 1 : 0;
+    p.slots = 2 * sm_count();
+    while (heads_first && p.b.n_qtiles > 1 && p.b.n_qtiles <= kDecodeWarps * 32 && cs < kDecodeCluster / 2 && items * 2 * cs <= 4LL * sm_count() && (long long)p.nsplit * 2 * cs <= 65535) {
+        cs *= 2;
+        p.fold *= 2;
+    }
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(p.b.n_qtiles, p.heads / G, p.nsplit * cs);
+    cfg.gridDim = heads_first ? dim3(p.heads / G, p.b.n_qtiles, p.nsplit * cs) : dim3(p.b.n_qtiles, p.heads / G, p.nsplit * cs);
     cfg.blockDim = dim3(kDecodeWarps * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -595,7 +603,7 @@ static int attention_decode_bf16(const sllm::AttnArgs& p, cudaStream_t st) {
     }
     const int group = p.heads / p.kv_heads;
     const int G = group % 4 == 0 ? 4 : group % 3 == 0 ? 3 : group % 2 == 0 ? 2 : 1;
-    return launch_attention_decode(kernel, G, DecodeTile<D>::kSmem, p, st, G);
+    return launch_attention_decode(kernel, G, DecodeTile<D>::kSmem, p, true, st, G);
 }
 
 template <int L, int G, int S>      // loads per lane of a row, query heads of a CTA, rows in flight per lane
@@ -607,7 +615,7 @@ static int attention_decode_f32(const sllm::AttnArgs& p, cudaStream_t st) {
         SLLM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         ready = true;
     }
-    return launch_attention_decode(kernel, G, 0, p, st);
+    return launch_attention_decode(kernel, G, 0, p, false, st);
 }
 
 static int attention_decode(const sllm::AttnArgs& p, int kv_dtype, cudaStream_t st) {

@@ -25,6 +25,8 @@ struct AttnArgs {
     int chunk;                // > 0: a query sees its own chunk of `chunk` positions only (then window / keep_first are not used)
     float* out; int ldo; uint16_t* out16;   // one share: the normalised result goes here (fp32 [T][ldo] and / or dense bf16) instead of ws
     uint32_t page_magic;      // ceil(2^32 / page_len): the page of a position without a division (page_of)
+    // Decode over bf16 pools: a cluster may be folded, i.e. serve `fold` items (a request and a set of heads) with 1 / fold of its CTAs each; 1 = it serves one. 0: the grid has the requests in x (more of them than y takes). `slots`: CTAs that are resident at once.
+    int fold, slots;
 };
 
 // prompt portions over bf16 pools on tcgen05: dk = dv = 64 or 128, pools 16-byte aligned, no values inside keys, no cross values (seq_attn_tc.cu)
@@ -325,6 +327,7 @@ __device__ __forceinline__ void ldmatrix4_trans(uint32_t (&r)[4], uint32_t addr)
 
 template <int D, bool kOpts>     // kOpts: capped scores or charges on the distance (a window, kept positions and chunks are part of both)
 __global__ void __launch_bounds__(kDecodeWarps * 32, 2) seq_attention_decode_mma_kernel(AttnArgs p, int G) {
+    static_assert(kDecodeWarps == 4, "sums of a column");
     after_previous();
     namespace cg = cooperative_groups;
     using Tile = DecodeTile<D>;
@@ -335,11 +338,61 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, 2) seq_attention_decode_mma
     __shared__ float weight[kDecodeCluster * kDecodeWarps][4], total[4][2];
     const sllm_seq_batch& b = p.b;
     cg::cluster_group cluster = cg::this_cluster();
-    const int CS = (int)cluster.num_blocks(), rank = (int)cluster.block_rank(), split = blockIdx.z / CS;
-    cluster.barrier_arrive();       // waited for before anything is sent: every CTA of the cluster runs by then
-    const int seg = b.qt_seg[blockIdx.x], t = b.seg_start[seg], pos = b.seg_pos0[seg], slot = b.seg_slot[seg];
-    const int group = p.heads / p.kv_heads, subsets = group / G, gkv = blockIdx.y / subsets, h0 = gkv * group + (blockIdx.y % subsets) * G;
+    const int full = (int)cluster.num_blocks(), split = blockIdx.z / full;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3, h = g >> 1;
+    // Items in the caller's order of requests (the longest context first), all heads of one before the next. Few long requests among short ones keep the last CTAs busy long after the others:
+    // then a cluster per item, more than fit at once, is better; requests alike are better off when every item starts at once in a part of a cluster. The longest share of a
+    // warp, in runs, stands against all the runs a warp gets and what an item costs beside them (5.7 runs). Measured, us, folded | unfolded | as chosen: eight requests of 77 to 8000 positions
+    // 41 | 30 | 31, eight of 2048 18.4 | 28 | 19.1, eight of 6000 38.5 | 47 | 38.4, 13 of 16 to 8000 61 | 36 | 39, 32 of them 90 | 57 | 57, 32 of 2048 47 | 54 | 48, 16 of 1000 17.9 | 24 | 18.5.
+    int CS = full, sub = 0, item_x = p.fold ? blockIdx.y : blockIdx.x, item_y = p.fold ? blockIdx.x : blockIdx.y;
+    int seg = b.qt_seg[item_x], t = b.seg_start[seg], pos = b.seg_pos0[seg], slot = b.seg_slot[seg];
+    bool present = true;
+    if (p.fold > 1) {
+        // both places this CTA may have are looked up beside the contexts
+        const int small = full / p.fold, folded_sub = (int)cluster.block_rank() / small, item = (blockIdx.y * gridDim.x + blockIdx.x) * p.fold + folded_sub;
+        const int folded_x = min(item / (int)gridDim.x, (int)gridDim.y - 1), fseg = b.qt_seg[folded_x], ft = b.seg_start[fseg], fpos = b.seg_pos0[fseg], fslot = b.seg_slot[fseg];
+        __shared__ float part[kDecodeWarps][2];
+        float most = 0.0f, all = 0.0f;
+        if ((int)threadIdx.x < b.n_qtiles) {
+            const int at = b.seg_pos0[b.qt_seg[threadIdx.x]];
+            most = all = (float)(TileList(at, at, seq_row_window(at, p.window, p.chunk), p.keep_first, kBK).n * (kBK / kRun));
+        }
+        most = warp_max(most);
+        all = warp_sum(all);
+        if (lane == 0) {
+            part[warp][0] = most;
+            part[warp][1] = all;
+        }
+        __syncthreads();
+        most = all = 0.0f;
+#pragma unroll
+        for (int i = 0; i < kDecodeWarps; ++i) {
+            most = fmaxf(most, part[i][0]);
+            all += part[i][1];
+        }
+        const float per = (float)(full * kDecodeWarps * p.nsplit);      // warps of an item
+        const float apart = (all / per + 5.7f * (float)b.n_qtiles) * (float)(gridDim.x * full * p.nsplit) / (float)p.slots;
+        if (fmaxf(apart, most / per) >= 0.9f * most * (float)p.fold / per) {
+            if (item - folded_sub >= (int)(gridDim.x * gridDim.y)) return;                // the whole cluster
+            present = item < (int)(gridDim.x * gridDim.y);
+            CS = small;
+            sub = folded_sub;
+            item_x = folded_x;
+            item_y = item % (int)gridDim.x;
+            seg = fseg;
+            t = ft;
+            pos = fpos;
+            slot = fslot;
+        }
+    }
+    const int base_rank = sub * CS, rank = (int)cluster.block_rank() - base_rank;
+    cluster.barrier_arrive();       // waited for before anything is sent: every CTA of the cluster runs by then
+    if (!present) {
+        cluster.barrier_wait();
+        cluster.sync();
+        return;
+    }
+    const int group = p.heads / p.kv_heads, subsets = group / G, gkv = item_y / subsets, h0 = gkv * group + (item_y % subsets) * G;
     const bool live = h < G, second = g & 1;           // this lane's head exists; it holds the second terms (and no third ones)
     const int wnd = seq_row_window(pos, p.window, p.chunk);
     const TileList tiles(pos, pos, wnd, p.keep_first, kBK);
@@ -516,11 +569,11 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, 2) seq_attention_decode_mma
     if (live) {
 #pragma unroll
         for (int i = 0; i < kTiles / 2; ++i) {
-            const int item = h * D + (second ? D / 2 : 0) + i * 8 + 2 * c, to = item / share;
-            *reinterpret_cast<float2*>(cluster.map_shared_rank(got_o, to) + worker * share + item % share) = make_float2(v[i][0], v[i][1]);
+            const int at = h * D + (second ? D / 2 : 0) + i * 8 + 2 * c, to = at / share;
+            *reinterpret_cast<float2*>(cluster.map_shared_rank(got_o, base_rank + to) + worker * share + at % share) = make_float2(v[i][0], v[i][1]);
         }
         if (!second)
-            for (int r = c; r < CS; r += 4) cluster.map_shared_rank(got_ml, r)[worker * 4 + h] = make_float2(m, l);
+            for (int r = c; r < CS; r += 4) cluster.map_shared_rank(got_ml, base_rank + r)[worker * 4 + h] = make_float2(m, l);
     }
     cluster.sync();
     if (warp < G) {
@@ -542,11 +595,13 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, 2) seq_attention_decode_mma
     }
     __syncthreads();
     for (int i = threadIdx.x; i < share; i += kDecodeWarps * 32) {
-        const int item = rank * share + i, hh = item / D, col = item % D;
-        if (item >= columns) break;
-        float acc = 0.0f;
-#pragma unroll 4
-        for (int wkr = 0; wkr < CS * kDecodeWarps; ++wkr) acc = fmaf(got_o[wkr * share + i], weight[wkr][hh], acc);
+        const int at = rank * share + i, hh = at / D, col = at % D;
+        if (at >= columns) break;
+        float sums[kDecodeWarps] = {};                  // (several: fewer roundings in a row)
+        for (int wkr = 0; wkr < CS * kDecodeWarps; wkr += kDecodeWarps)
+#pragma unroll
+            for (int e = 0; e < kDecodeWarps; ++e) sums[e] = fmaf(got_o[(wkr + e) * share + i], weight[wkr + e][hh], sums[e]);
+        float acc = (sums[0] + sums[1]) + (sums[2] + sums[3]);
         if (p.out || p.out16) {
             acc *= 1.0f / total[hh][1];
             if (p.out) p.out[(size_t)t * p.ldo + (size_t)(h0 + hh) * D + col] = acc;
