@@ -11,7 +11,7 @@
 // (1) seq_chunk_prepare_kernel, CTA = (block, head), all blocks of the step in parallel: silu / rotation / unit vectors, G, A and B (fp32, 4 x 4 entries and an eighth of the channels
 // per thread), M from the inverses of its two 16 x 16 triangles; leaves e^G k, e^G q, e^(G_n - G) k, M and B as the tensor-core fragments the walk
 // will load, each as two bf16 terms (x = hi + lo, |x - hi - lo| <= 2^-17 |x|), and e^G_n in fp32. Bound: shared memory's bandwidth and the exponentials: decays that are one number per
-// head multiply finished sums and whole rows (2048 tokens of 16 heads: 58 us with the decays inside the sums and blocks of 16 in two threads per entry, 43 like this).
+// head multiply finished sums and whole rows (2048 tokens of 16 heads: 58 us with the decays inside the sums and blocks of 16 in two threads per entry, 42 like this).
 // (2) seq_chunk_walk_kernel, CTA = (portion, head, 16 or 32 value columns), two or four warps = 16 value columns, a share of the key channels each: their part of
 // S^T [16][dk] stays in the accumulators (fp32) from the portion's first token to its last. An accumulator fragment is register for register
 // an A fragment of the next product, so state and u never leave the registers; all products take both operands as two bf16 terms (three products, fp32 accumulation), which keeps
@@ -99,25 +99,38 @@ __global__ void __launch_bounds__(kPrepThreads, kMode == kDecayChannel ? 2 : 3) 
         return v;
     };
     auto silu4 = [](float4 v) { return make_float4(v.x * seq_sigmoid(v.x), v.y * seq_sigmoid(v.y), v.z * seq_sigmoid(v.z), v.w * seq_sigmoid(v.w)); };
-    for (int i = threadIdx.x; i < kChunk * dkp / 4; i += kPrepThreads) {
-        const int tok = i / (dkp / 4), ch = (i % (dkp / 4)) * 4;
-        const bool has = tok < c.n;
-        const size_t t = (size_t)(c.start + (has ? tok : 0));
-        float4 kv = load4(p.k + t * p.ldk + (size_t)kvh * dk, ch, has), qv = load4(p.q + t * p.ldq + (size_t)kvh * dk, ch, has);
-        if (!kDelta && p.silu) {
-            kv = silu4(kv);
-            qv = silu4(qv);
-        }
-        *reinterpret_cast<float4*>(s_k + tok * ld + ch) = kv;
-        *reinterpret_cast<float4*>(s_q + tok * ld + ch) = qv;
-        if (kChannel) {
-            float4 g = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (has) {
-                const float4 a = load4(p.al + t * p.lda + (size_t)h * dk, ch, true), bias = load4(p.dt_bias + (size_t)h * dk, ch, true);
-                g = make_float4(ch < dk ? lg * seq_softplus(a.x + bias.x) : 0.0f, ch + 1 < dk ? lg * seq_softplus(a.y + bias.y) : 0.0f,
-                                ch + 2 < dk ? lg * seq_softplus(a.z + bias.z) : 0.0f, ch + 3 < dk ? lg * seq_softplus(a.w + bias.w) : 0.0f);
+    // all of a thread's rows are asked for before the first of them is worked on
+    constexpr int kWords = kChunk * dkp / 4, kRounds = (kWords + kPrepThreads - 1) / kPrepThreads;
+    {
+        float4 kv[kRounds], qv[kRounds], a[kRounds], bias[kRounds];
+#pragma unroll
+        for (int x = 0; x < kRounds; ++x) {
+            const int i = threadIdx.x + x * kPrepThreads, tok = i / (dkp / 4), ch = (i % (dkp / 4)) * 4;
+            const bool has = i < kWords && tok < c.n;
+            const size_t t = (size_t)(c.start + (has ? tok : 0));
+            kv[x] = load4(p.k + t * p.ldk + (size_t)kvh * dk, ch, has);
+            qv[x] = load4(p.q + t * p.ldq + (size_t)kvh * dk, ch, has);
+            if (kChannel) {
+                a[x] = load4(p.al + t * p.lda + (size_t)h * dk, ch, has);
+                bias[x] = load4(p.dt_bias + (size_t)h * dk, ch, has);
             }
-            *reinterpret_cast<float4*>(s_G + tok * ld + ch) = g;
+        }
+#pragma unroll
+        for (int x = 0; x < kRounds; ++x) {
+            const int i = threadIdx.x + x * kPrepThreads, tok = i / (dkp / 4), ch = (i % (dkp / 4)) * 4;
+            if (i >= kWords) break;
+            if (!kDelta && p.silu) {
+                kv[x] = silu4(kv[x]);
+                qv[x] = silu4(qv[x]);
+            }
+            *reinterpret_cast<float4*>(s_k + tok * ld + ch) = kv[x];
+            *reinterpret_cast<float4*>(s_q + tok * ld + ch) = qv[x];
+            if (kChannel) {
+                const bool has = tok < c.n;
+                *reinterpret_cast<float4*>(s_G + tok * ld + ch) =
+                    make_float4(has && ch < dk ? lg * seq_softplus(a[x].x + bias[x].x) : 0.0f, has && ch + 1 < dk ? lg * seq_softplus(a[x].y + bias[x].y) : 0.0f,
+                                has && ch + 2 < dk ? lg * seq_softplus(a[x].z + bias[x].z) : 0.0f, has && ch + 3 < dk ? lg * seq_softplus(a[x].w + bias[x].w) : 0.0f);
+            }
         }
     }
     if (!kDelta && p.silu)                               // the values too, for the walk

@@ -211,17 +211,17 @@ __global__ void __launch_bounds__(1024) seq_headnorm_gate_wide_kernel(const floa
     }
 }
 
-// the same four columns at a time: a team of `team` threads (a warp, or the whole CTA) per (token, part), R groups of four columns per thread,
-// everything in registers between the sum of squares and the scaling
-template <int R>
+// the same four columns at a time: a team of threads (a warp, or the whole CTA) per (token, part), R groups of four columns per thread,
+// everything in registers between the sum of squares and the scaling. Bound: issue slots (the gate's exponential and division beside three accesses): 95 instructions
+// an element with a team size and two groups that only the launch knew, 16.2 us for 2048 x 16 parts of 128, now 12.6 (2048 x 2 parts of 2048: 24 | 19).
+template <int R, bool kWarp>
 __global__ void __launch_bounds__(1024) seq_headnorm_gate_vec_kernel(const float* o, int ldo, const float* g, int ldg, const float* w,
-                                                                     int heads, int dv, float eps, float* out, int ldout, uint16_t* out16, int items,
-                                                                     int team, int mode) {
+                                                                     int heads, int dv, float eps, float* out, int ldout, uint16_t* out16, int items, int mode) {
     after_previous();
     __shared__ float red[33];
-    const int per_cta = blockDim.x / team, item = blockIdx.x * per_cta + threadIdx.x / team, me = threadIdx.x % team;
+    const int item = kWarp ? blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5) : blockIdx.x, me = kWarp ? threadIdx.x & 31 : threadIdx.x, team = kWarp ? 32 : blockDim.x;
     const bool live = item < items;                      // (a CTA that is one team has one item: no thread leaves before the barriers)
-    const int t = live ? item / heads : 0, h = live ? item % heads : 0;
+    const int t = live ? item / heads : 0, h = live ? item - t * heads : 0;
     const float* orow = o + (size_t)t * ldo + (size_t)h * dv;
     const float* grow = g + (size_t)t * ldg + (size_t)h * dv;
     const float* wrow = (w && (mode & 2)) ? w + (size_t)h * dv : w;
@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(1024) seq_headnorm_gate_vec_kernel(const float
             ss = fmaf(v[i].x, v[i].x, fmaf(v[i].y, v[i].y, fmaf(v[i].z, v[i].z, fmaf(v[i].w, v[i].w, ss))));
         }
     }
-    ss = team == 32 ? warp_sum(ss) : block_sum(ss, red);
+    ss = kWarp ? warp_sum(ss) : block_sum(ss, red);
     const float inv = 1.0f / sqrtf(ss / (float)dv + eps);
 #pragma unroll
     for (int i = 0; i < R; ++i) {
@@ -533,7 +533,9 @@ int sllm_seq_headnorm_gate(const float* o, int32_t ldo, const float* g, int32_t 
     if (dv % 4 == 0 && ldo % 4 == 0 && ldg % 4 == 0 && (!out || ldout % 4 == 0) && dv <= 8192 && aligned(o) && aligned(g) && aligned(w) && aligned(out) && aligned(out16)) {
         cudaStream_t st = as_stream(stream);
         const int team = dv <= 256 ? 32 : std::min(1024, ((dv + 7) / 8 + 31) / 32 * 32), cta = team == 32 ? 128 : team, grid = team == 32 ? (items + 3) / 4 : items;
-        overlapping(seq_headnorm_gate_vec_kernel<2>)<<<grid, cta, 0, st>>>(o, ldo, g, ldg, w, heads, dv, eps, out, ldout, (uint16_t*)out16, items, team, mode);
+        if (team == 32 && dv <= 128) overlapping(seq_headnorm_gate_vec_kernel<1, true>)<<<grid, cta, 0, st>>>(o, ldo, g, ldg, w, heads, dv, eps, out, ldout, (uint16_t*)out16, items, mode);
+        else if (team == 32) overlapping(seq_headnorm_gate_vec_kernel<2, true>)<<<grid, cta, 0, st>>>(o, ldo, g, ldg, w, heads, dv, eps, out, ldout, (uint16_t*)out16, items, mode);
+        else overlapping(seq_headnorm_gate_vec_kernel<2, false>)<<<grid, cta, 0, st>>>(o, ldo, g, ldg, w, heads, dv, eps, out, ldout, (uint16_t*)out16, items, mode);
         ++g_launches;
         SLLM_LAUNCH_CHECK();
         return SLLM_OK;
