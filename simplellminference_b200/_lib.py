@@ -85,6 +85,8 @@ SIGNATURES = {
     "sllm_mega_repack_down_t": (C.c_int, [_P, _P, _I, _I, _I, _P]),
     "sllm_mega_tile_geometry": (C.c_int, [_I, _I, _I, _I, C.POINTER(_I), C.POINTER(_I), C.POINTER(_I), C.POINTER(_I), C.POINTER(_I), C.POINTER(_L)]),
     "sllm_prefill_attention": (C.c_int, [_P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I, _P]),
+    "sllm_prefill_attention_scratch": (_L, [_I, _I, _I, _I, _I, _I]),
+    "sllm_prefill_attention_in": (C.c_int, [_P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I, _P, _L, _P]),
     "sllm_kvpages_create": (_P, [_I, _I, _I, _I]),
     "sllm_kvpages_destroy": (None, [_P]),
     "sllm_kvpages_reserve": (_I, [_P, _I, _I]),

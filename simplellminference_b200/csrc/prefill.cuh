@@ -52,10 +52,14 @@ const char* pf_unsupported_reason(int w_dtype, int hd, int d, int q_loc, int I_l
 int pf_gemm(PfCache* cache, const PfGemmArgs& a, cudaStream_t st);
 // causal attention of T queries at positions pos0.. over cache rows [0, pos0+T): q bf16 [T][q_loc] -> out bf16 [T][q_loc]
 int pf_attention(const uint16_t* q, const void* k_cache, const void* v_cache, int kv_dtype, uint16_t* out, int T, int pos0, int S, int hd,
-                 int heads, int kv_heads, cudaStream_t st);
+                 int heads, int kv_heads, cudaStream_t st, float* scratch = nullptr);
+// fp32 values of scratch with which such a call divides its work evenly; 0: it has no use for any
+size_t pf_attention_scratch(int kv_dtype, int T, int pos0, int hd, int heads, int kv_heads);
 // the same on tcgen05: bf16 cache, head_dim 64 or 128, 16-byte aligned pointers (prefill_attn_tc.cu)
 int pf_attention_tc(const uint16_t* q, const void* k_cache, const void* v_cache, uint16_t* out, int T, int pos0, int S, int hd, int heads, int kv_heads,
-                    cudaStream_t st);
+                    float* scratch, cudaStream_t st);
+bool pf_attention_fills(int T, int keys, int hd, int heads);      // without scratch: tcgen05 rather than mma.sync
+size_t pf_attention_tc_scratch(int T, int pos0, int hd, int heads, int kv_heads);
 // x[t][:] = E[ids[t]][:] from the tiled embedding matrix (emb_kernel.cpp:9-16), fp32
 int pf_embed(const int32_t* ids_dev, const void* emb_tiled, int vocab, int d, float* x, int T, cudaStream_t st);
 // x[t] += add[t] (optional), y[t] = bf16(rmsnorm(x[t]) * w)   (rms_kernel.cpp:12-22)

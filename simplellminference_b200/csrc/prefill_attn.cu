@@ -206,20 +206,27 @@ static int attn_launch(const uint16_t* q, const void* kc, const void* vc, uint16
     return SLLM_OK;
 }
 
+// bf16 caches: tcgen05 (128 queries x 128 keys a tile), where its tiles are not mostly padding. Measured, us, mma.sync | tcgen05, heads of 128, 32 over 8: 2048 queries
+// behind 6144 positions 1061 | 390, 512 from the start 22.4 | 14.9, 256 9.8 | 9.2, one query behind 250, 1000 and 2000 9.4 | 7.8, 29.5 | 22.5 and 55.9 | 41.4; 192
+// keys and 64 or fewer, where the last tile is half empty: 64 queries behind 128 7.9 | 8.2, 192 from the start 8.0 | 8.4, 64 4.9 | 5.7, one 4.6 | 5.3, but 16 behind
+// 64 6.2 | 5.3 and 128 from the start 6.3 | 6.1. Heads of 64 fill a tile's time with half the products, so there it pays only where the 64-query tiles of the other
+// kernel make more than one wave: 2048 queries, 32 heads 119 | 80, 700 of 16 heads behind 1234 51 | 39, but 256 of 32 heads behind 0 and 2000 6.6 | 8.0 and
+// 42.2 | 44.3, 1000 of 8 heads behind 5000 106 | 107 (with scratch, and so with shares: prefill_attn_tc.cu). The mma.sync kernel keeps the rest, fp32 caches, and results that do not start at a multiple of 16 bytes.
+bool pf_attention_fills(int T, int keys, int hd, int heads) {
+    return hd == 128 ? keys > 192 || (keys > 64 && keys <= 128) : (hd == 64 && (long long)((T + kPaBQ - 1) / kPaBQ) * heads > sm_count());
+}
+size_t pf_attention_scratch(int kv_dtype, int T, int pos0, int hd, int heads, int kv_heads) {
+    const bool tc = kv_dtype == SLLM_BF16 && (hd == 64 || pf_attention_fills(T, pos0 + T, hd, heads));
+    return tc ? pf_attention_tc_scratch(T, pos0, hd, heads, kv_heads) : 0;
+}
+
 int pf_attention(const uint16_t* q, const void* kc, const void* vc, int kv_dtype, uint16_t* out, int T, int pos0, int S, int hd, int heads,
-                 int kv_heads, cudaStream_t st) {
+                 int kv_heads, cudaStream_t st, float* scratch) {
     SLLM_REQUIRE(q && kc && vc && out && T > 0 && pos0 >= 0 && pos0 + T <= S, SLLM_EINVAL, "pf_attention: bad argument");
     SLLM_REQUIRE((((uintptr_t)q | (uintptr_t)kc | (uintptr_t)vc) % 16) == 0 && ((uintptr_t)out % 4) == 0, SLLM_EINVAL,
                  "pf_attention: queries and caches are read 16 bytes at a time and the result is written 4 at a time: their addresses have to be such multiples");
-    // bf16 caches: tcgen05 (128 queries x 128 keys a tile), where its tiles are not mostly padding. Measured, us, mma.sync | tcgen05, heads of 128, 32 over 8: 2048 queries
-    // behind 6144 positions 1061 | 390, 512 from the start 22.4 | 14.9, 256 9.8 | 9.2, one query behind 250, 1000 and 2000 9.4 | 7.8, 29.5 | 22.5 and 55.9 | 41.4; 192
-    // keys and 64 or fewer, where the last tile is half empty: 64 queries behind 128 7.9 | 8.2, 192 from the start 8.0 | 8.4, 64 4.9 | 5.7, one 4.6 | 5.3, but 16 behind
-    // 64 6.2 | 5.3 and 128 from the start 6.3 | 6.1. Heads of 64 fill a tile's time with half the products, so there it pays only where the 64-query tiles of the other
-    // kernel make more than one wave: 2048 queries, 32 heads 119 | 80, 700 of 16 heads behind 1234 51 | 39, but 256 of 32 heads behind 0 and 2000 6.6 | 8.0 and
-    // 42.2 | 44.3, 1000 of 8 heads behind 5000 106 | 107. The kernel below keeps the rest, fp32 caches, and results that do not start at a multiple of 16 bytes.
-    const int keys = pos0 + T;
-    const bool fills = hd == 128 ? keys > 192 || (keys > 64 && keys <= 128) : (long long)((T + kPaBQ - 1) / kPaBQ) * heads > sm_count();
-    if (kv_dtype == SLLM_BF16 && ((uintptr_t)out % 16) == 0 && (hd == 64 || hd == 128) && fills) return pf_attention_tc(q, kc, vc, out, T, pos0, S, hd, heads, kv_heads, st);
+    if (kv_dtype == SLLM_BF16 && ((uintptr_t)out % 16) == 0 && (hd == 64 || hd == 128) && (scratch || pf_attention_fills(T, pos0 + T, hd, heads)))
+        return pf_attention_tc(q, kc, vc, out, T, pos0, S, hd, heads, kv_heads, scratch, st);
     if (hd == 128) return kv_dtype == SLLM_F32 ? attn_launch<128, SLLM_F32>(q, kc, vc, out, T, pos0, S, heads, kv_heads, st)
                                                : attn_launch<128, SLLM_BF16>(q, kc, vc, out, T, pos0, S, heads, kv_heads, st);
     if (hd == 64) return kv_dtype == SLLM_F32 ? attn_launch<64, SLLM_F32>(q, kc, vc, out, T, pos0, S, heads, kv_heads, st)
@@ -310,6 +317,20 @@ int pf_rmsnorm(float* x, const float* add, const float* w, uint16_t* y, int T, i
 
 }  // namespace sllm
 
+extern "C" int64_t sllm_prefill_attention_scratch(int32_t kv_dtype, int32_t T, int32_t pos0, int32_t head_dim, int32_t heads, int32_t kv_heads) {
+    if (T <= 0 || pos0 < 0 || heads <= 0 || kv_heads <= 0 || heads % kv_heads) return 0;
+    return 4 * (int64_t)sllm::pf_attention_scratch(kv_dtype, T, pos0, head_dim, heads, kv_heads);
+}
+extern "C" int sllm_prefill_attention_in(const void* q, const void* kc, const void* vc, int32_t kv_dtype, void* out, int32_t T, int32_t pos0, int32_t max_len,
+                                         int32_t head_dim, int32_t heads, int32_t kv_heads, void* scratch, int64_t scratch_bytes, sllm_stream_t stream) {
+    using namespace sllm;
+    SLLM_REQUIRE(heads > 0 && kv_heads > 0 && heads % kv_heads == 0, SLLM_EINVAL, "bad head counts");
+    SLLM_REQUIRE(T > 0 && pos0 >= 0, SLLM_EINVAL, "pf_attention: bad argument");
+    const int64_t wanted = sllm_prefill_attention_scratch(kv_dtype, T, pos0, head_dim, heads, kv_heads);
+    float* ws = wanted && scratch && scratch_bytes >= wanted && ((uintptr_t)scratch | (uintptr_t)out) % 16 == 0 ? reinterpret_cast<float*>(scratch) : nullptr;
+    return pf_attention(reinterpret_cast<const uint16_t*>(q), kc, vc, kv_dtype, reinterpret_cast<uint16_t*>(out), T, pos0, max_len, head_dim, heads,
+                        kv_heads, as_stream(stream), ws);
+}
 extern "C" int sllm_prefill_attention(const void* q, const void* kc, const void* vc, int32_t kv_dtype, void* out, int32_t T, int32_t pos0, int32_t max_len,
                                       int32_t head_dim, int32_t heads, int32_t kv_heads, sllm_stream_t stream) {
     using namespace sllm;
