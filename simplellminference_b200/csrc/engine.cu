@@ -1033,17 +1033,18 @@ int sllm_engine_forward(sllm_engine* e, int32_t token, int32_t pos, float* logit
     if (e->fused && e->mega && !e->mega_ll) {
         // What was around the kernel cost more than the bytes it moved (stories110M, fp32, position 200, us a call: 408): a copy of 16 bytes in front (the launch carries
         // token and position now), the next token's copy behind (the kernel leaves it in pinned memory, with the reduction behind it 386 -> 370 without logits), the
-        // logits staged into pageable memory by the driver (390; into pinned memory and from there to the caller 385; stored by the kernel itself, 8 bytes a
-        // thread over PCIe, 410).
+        // logits staged into pageable memory by the driver (390; into pinned memory and from there to the caller 385; stored by the kernel's own epilogue, 8 bytes a
+        // thread over PCIe and in front of the fence of its ticket, 410). With a faster kernel that copy was the end of every call: 329 us, 246 at 7B in bf16; the kernel's CTAs
+        // storing their rows 16 bytes a thread behind the ticket: 321 and 236 (without logits 312 and 228).
         MegaCall call;
         call.token = token;
         call.pos = pos;
         call.next = next_token_host ? e->h_state + 4 : nullptr;
+        call.logits = logits_host ? e->h_logits : nullptr;
         e->h_state[7] = pos;
         int done = 0;
         if (int rc = enqueue_steps(e, 1, pos, &done, call)) return rc;
         e->h_state[7] = pos + 1;
-        if (logits_host) SLLM_CUDA(cudaMemcpyAsync(e->h_logits, e->logits, sizeof(float) * (size_t)e->V_loc, cudaMemcpyDeviceToHost, e->stream));
         SLLM_WAIT(e->stream);
         if (logits_host) std::memcpy(logits_host, e->h_logits, sizeof(float) * (size_t)e->V_loc);
         if (next_token_host) *next_token_host = e->h_state[4];

@@ -361,10 +361,23 @@ __device__ __forceinline__ void cta_better(float& v, int& i, float* red) {
         warp_better(v, i);
     }
 }
+// Rows [r0, r1) of the logits into pinned host memory. A function of its own: written out in mega_finish it cost kernels that have no register to spare 2 % of a step.
+static __device__ __noinline__ void mega_logits_out(const float* from, float* to, int r0, int r1) {
+#pragma unroll 1
+    for (int r = (r0 & ~3) + 4 * (int)threadIdx.x; r < r1; r += 4 * kMegaThreads) {
+        if (r >= r0 && r + 4 <= r1) {
+            *reinterpret_cast<float4*>(to + r) = __ldcg(reinterpret_cast<const float4*>(from + r));
+        } else {
+#pragma unroll 1
+            for (int e = max(r, r0); e < min(r + 4, r1); ++e) to[e] = __ldcg(from + e);
+        }
+    }
+}
 // End of the classifier phase: every CTA leaves its best logit, the CTA that comes last picks the arg max and advances the step state. True in the one thread that has
 // done so (it stores the counters that its kernel keeps). All threads of the last CTA read the candidates: by one thread, a chain of 148 reads of L2, that end took
-// several us.
-__device__ __forceinline__ bool mega_finish(const MegaParams& p, float v, int i, float* red, int* s_last, int cta, int ncta) {
+// several us. A call that wants its logits on the host (p.call.logits, pinned) gets this CTA's rows [r0, r1) from here: read back from the device's copy, 16 bytes a thread,
+// so that a warp stores 512 bytes in a row over PCIe, and behind the ticket, so that no fence waits for them to arrive.
+__device__ __forceinline__ bool mega_finish(const MegaParams& p, float v, int i, float* red, int* s_last, int cta, int ncta, int r0, int r1) {
     cta_better(v, i, red);
     if (threadIdx.x == 0) {
         p.blk_val[cta] = v;
@@ -374,6 +387,7 @@ __device__ __forceinline__ bool mega_finish(const MegaParams& p, float v, int i,
         __threadfence();
     }
     __syncthreads();
+    if (p.call.logits) mega_logits_out(p.logits, p.call.logits, r0, r1);
     if (!*s_last) return false;
     v = -INFINITY;
     i = 0x7fffffff;

@@ -485,7 +485,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega_step_kernel(const MegaPa
         }
 
         if (ph.kind == PH_CLS) {   // CTA best -> global; the last CTA picks the arg max and advances the step state
-            if (mega_finish(p, best_v, best_i, part, &s_last, cta, ncta)) {
+            if (mega_finish(p, best_v, best_i, part, &s_last, cta, ncta, 2 * u0, min(ph.nrows, 2 * (u0 + n)))) {
                 p.st->pad[0] = (int32_t)(bar_base + bar_idx * (unsigned)ncta);   // barrier epoch for the next launch
             }
             break;

@@ -55,11 +55,12 @@ inline TileGeom mega_tile_geom(int rows_phys, int cols, int w_dtype) {
 // bytes of one [rows][cols] matrix of phase kind `kind` in the tiled layout
 size_t mega_matrix_bytes(int rows, int cols, int kind, int w_dtype);
 
-// One step asked for by value (sllm_engine_forward): its token and position come with the launch, its arg max goes into pinned host memory, so that nothing is
-// copied for them. token < 0: both are the device's (StepState), which is advanced either way.
+// One step asked for by value (sllm_engine_forward): its token and position come with the launch, its arg max and its logits go into pinned host memory, so that
+// nothing is copied for them. token < 0: both are the device's (StepState), which is advanced either way.
 struct MegaCall {
     int32_t token = -1, pos = 0;
     int32_t* next = nullptr;      // or NULL
+    float* logits = nullptr;      // [V_loc] in pinned host memory, or NULL
 };
 struct MegaParams {
     const PhaseDesc* phases;   // [4L+1]
