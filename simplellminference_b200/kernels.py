@@ -146,7 +146,10 @@ def prefill_attention(q_bf16: torch.Tensor, key_cache: torch.Tensor, value_cache
     out = torch.empty_like(q_bf16)
     lib = _lib.load()
     need = lib.sllm_prefill_attention_scratch(kvd, T, pos0, hd, heads, kv_heads) if T > 0 else 0
-    scratch = torch.empty(need, dtype=torch.uint8, device=q_bf16.device) if need else None
+    try:
+        scratch = torch.empty(need, dtype=torch.uint8, device=q_bf16.device) if need else None
+    except torch.OutOfMemoryError:      # the call runs without, only slower
+        need, scratch = 0, None
     _lib.check(lib.sllm_prefill_attention_in(_p(q_bf16), _p(key_cache), _p(value_cache), kvd, _p(out), T, pos0, max_len, hd, heads, kv_heads,
                                              scratch.data_ptr() if need else None, need, _stream()))
     return out
