@@ -298,7 +298,7 @@ int sllm_prefill_gemm_plan(int32_t T, int32_t N, int32_t K, int32_t residual_epi
 int sllm_prefill_attention(const void* q, const void* key_cache, const void* value_cache, int32_t kv_dtype, void* out,
                            int32_t T, int32_t pos0, int32_t max_len, int32_t head_dim, int32_t heads, int32_t kv_heads,
                            sllm_stream_t stream);
-/* The same with scratch memory, over which every SM gets an equal share of the key tiles. _scratch: the bytes of it that such a call
+/* The same with scratch memory, with which every SM gets an equal share of the key tiles and an fp32 cache is rounded to bf16 once. _scratch: the bytes of it that such a call
  * can use (0: none); with less, or none, the call runs without. 16-byte aligned, free again when the call's work on the stream is done. */
 int64_t sllm_prefill_attention_scratch(int32_t kv_dtype, int32_t T, int32_t pos0, int32_t head_dim, int32_t heads, int32_t kv_heads);
 int sllm_prefill_attention_in(const void* q, const void* key_cache, const void* value_cache, int32_t kv_dtype, void* out,

@@ -6,7 +6,7 @@
 // CTA = 64 queries of one head (4 warps x 16 rows), K/V tiles of 64 positions double-buffered in shared memory
 // with cp.async, XOR-swizzled 16-byte chunks (conflict-free ldmatrix), S = QK^T and O += PV with the P fragments
 // taken straight from the S accumulators. Heaviest query tiles are scheduled first (causal imbalance). bf16 caches go to the
-// tcgen05 kernel of prefill_attn_tc.cu where its larger tiles pay (pf_attention).
+// tcgen05 kernel of prefill_attn_tc.cu where its larger tiles pay (pf_attention), and so do fp32 ones where there is scratch to round them into.
 #include "mega_common.cuh"
 #include "prefill.cuh"
 
@@ -215,6 +215,23 @@ static int attn_launch(const uint16_t* q, const void* kc, const void* vc, uint16
 bool pf_attention_fills(int T, int keys, int hd, int heads) {
     return hd == 128 ? keys > 192 || (keys > 64 && keys <= 128) : (hd == 64 && (long long)((T + kPaBQ - 1) / kPaBQ) * heads > sm_count());
 }
+// fp32 cache rows as the bf16 values that pf_attn_kernel rounds them to, eight a thread; blockIdx.y: kv head, z: keys or values. Bound by HBM, 6 bytes a value (8192
+// positions of 8 heads of 128: 13 us with its launch).
+__global__ void __launch_bounds__(256) pf_rows16_kernel(const float* __restrict__ k, const float* __restrict__ v, uint16_t* __restrict__ k16, uint16_t* __restrict__ v16, int groups,
+                                                        long long head_stride) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    pdl_wait();
+    pdl_launch_dependents();
+    if (i >= groups) return;
+    const float4* src = reinterpret_cast<const float4*>((blockIdx.z ? v : k) + blockIdx.y * head_stride) + 2 * (size_t)i;
+    const float4 a = __ldcs(src), b = __ldcs(src + 1);
+    reinterpret_cast<uint4*>(blockIdx.z ? v16 : k16)[(size_t)blockIdx.y * groups + i] = make_uint4(bf16x2(a.x, a.y), bf16x2(a.z, a.w), bf16x2(b.x, b.y), bf16x2(b.z, b.w));
+}
+// Whether an fp32 cache is rounded once, in front of the kernels for bf16 ones, instead of by every CTA for itself, whose 16-byte copies of fp32 rows and conversions are what binds it
+// then. Measured, us, fp32 rows in the kernel | rounded first (with shares where they pay), heads of 128: 2048 queries behind 6144 positions, 32 heads over 8 2697 | 260, 512 from the
+// start 45 | 16, 256 behind 5000, 8 heads 356 | 35, 128 behind 100 19.2 | 10.0, 64 from the start 7.3 | 6.4; heads of 64: 2048 queries, 32 heads 202 | 55, 1000 behind 5000, 8 heads 215 | 39. With 64
+// keys and heads of 64 the kernel is done in 4.8 and the copy alone takes 2.5; the bf16 kernel saves that from some 128 keys on.
+static bool pf_rows16_pay(int T, int pos0, int hd) { return hd == 128 || (hd == 64 && pos0 + T > 128); }
 size_t pf_attention_scratch(int kv_dtype, int T, int pos0, int hd, int heads, int kv_heads) {
     const bool tc = kv_dtype == SLLM_BF16 && (hd == 64 || pf_attention_fills(T, pos0 + T, hd, heads));
     return tc ? pf_attention_tc_scratch(T, pos0, hd, heads, kv_heads) : 0;
@@ -319,7 +336,9 @@ int pf_rmsnorm(float* x, const float* add, const float* w, uint16_t* y, int T, i
 
 extern "C" int64_t sllm_prefill_attention_scratch(int32_t kv_dtype, int32_t T, int32_t pos0, int32_t head_dim, int32_t heads, int32_t kv_heads) {
     if (T <= 0 || pos0 < 0 || heads <= 0 || kv_heads <= 0 || heads % kv_heads) return 0;
-    return 4 * (int64_t)sllm::pf_attention_scratch(kv_dtype, T, pos0, head_dim, heads, kv_heads);
+    const int64_t shares = 4 * (int64_t)sllm::pf_attention_scratch(SLLM_BF16, T, pos0, head_dim, heads, kv_heads);
+    if (kv_dtype == SLLM_BF16) return shares;
+    return kv_dtype == SLLM_F32 && sllm::pf_rows16_pay(T, pos0, head_dim) ? shares + 4 * (int64_t)kv_heads * (pos0 + T) * head_dim : 0;
 }
 extern "C" int sllm_prefill_attention_in(const void* q, const void* kc, const void* vc, int32_t kv_dtype, void* out, int32_t T, int32_t pos0, int32_t max_len,
                                          int32_t head_dim, int32_t heads, int32_t kv_heads, void* scratch, int64_t scratch_bytes, sllm_stream_t stream) {
@@ -328,8 +347,20 @@ extern "C" int sllm_prefill_attention_in(const void* q, const void* kc, const vo
     SLLM_REQUIRE(T > 0 && pos0 >= 0, SLLM_EINVAL, "pf_attention: bad argument");
     const int64_t wanted = sllm_prefill_attention_scratch(kv_dtype, T, pos0, head_dim, heads, kv_heads);
     float* ws = wanted && scratch && scratch_bytes >= wanted && ((uintptr_t)scratch | (uintptr_t)out) % 16 == 0 ? reinterpret_cast<float*>(scratch) : nullptr;
-    return pf_attention(reinterpret_cast<const uint16_t*>(q), kc, vc, kv_dtype, reinterpret_cast<uint16_t*>(out), T, pos0, max_len, head_dim, heads,
-                        kv_heads, as_stream(stream), ws);
+    cudaStream_t st = as_stream(stream);
+    auto run = [&](const void* k, const void* v, int type, int rows, float* shares) {
+        return pf_attention(reinterpret_cast<const uint16_t*>(q), k, v, type, reinterpret_cast<uint16_t*>(out), T, pos0, rows, head_dim, heads, kv_heads, st, shares);
+    };
+    if (!ws || kv_dtype == SLLM_BF16 || pos0 + T > max_len || !q || !kc || !vc || ((uintptr_t)q | (uintptr_t)kc | (uintptr_t)vc) % 16) return run(kc, vc, kv_dtype, max_len, ws);
+    const int n = pos0 + T;
+    const size_t bytes = (size_t)2 * kv_heads * n * head_dim;
+    uint8_t *k16 = reinterpret_cast<uint8_t*>(scratch), *v16 = k16 + bytes;
+    const int groups = n * head_dim / 8;
+    LaunchCfg lc(dim3((unsigned)((groups + 255) / 256), (unsigned)kv_heads, 2), dim3(256), 0, st, g_tune_pf_pdl != 0);
+    SLLM_CUDA(cudaLaunchKernelEx(&lc.cfg, pf_rows16_kernel, reinterpret_cast<const float*>(kc), reinterpret_cast<const float*>(vc), reinterpret_cast<uint16_t*>(k16),
+                                 reinterpret_cast<uint16_t*>(v16), groups, (long long)max_len * head_dim));
+    g_launches++;
+    return run(k16, v16, SLLM_BF16, n, wanted > (int64_t)(2 * bytes) ? reinterpret_cast<float*>(v16 + bytes) : nullptr);
 }
 extern "C" int sllm_prefill_attention(const void* q, const void* kc, const void* vc, int32_t kv_dtype, void* out, int32_t T, int32_t pos0, int32_t max_len,
                                       int32_t head_dim, int32_t heads, int32_t kv_heads, sllm_stream_t stream) {

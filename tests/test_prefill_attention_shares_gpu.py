@@ -44,3 +44,23 @@ def test_shares(T, pos0, heads, kv_heads, hd, shape):
     none = torch.empty_like(q)
     _lib.check(lib.sllm_prefill_attention(q.data_ptr(), k.data_ptr(), v.data_ptr(), 1, none.data_ptr(), T, pos0, S, hd, heads, kv_heads, torch.cuda.current_stream().cuda_stream))
     assert torch.equal(run(4), none)
+
+
+@pytest.mark.parametrize("T,pos0,heads,kv_heads,hd", [(1, 0, 8, 2, 128), (64, 0, 8, 8, 128), (65, 100, 6, 2, 128), (300, 5000, 3, 1, 128), (700, 33, 16, 4, 128), (1, 128, 8, 2, 64),
+                                                      (257, 60, 5, 5, 64), (300, 4000, 24, 8, 64)])
+def test_fp32_rows_are_rounded_once(T, pos0, heads, kv_heads, hd):
+    """A cache in fp32 is rounded as the kernel without scratch rounds it: the results are those of the rounded cache, bit for bit."""
+    import torch
+
+    from simplellminference_b200 import _lib, kernels as K
+    g = torch.Generator(device="cuda").manual_seed(T + pos0)
+    n, S = pos0 + T, pos0 + T + 9
+    q = torch.randn(T, heads * hd, device="cuda", generator=g).to(torch.bfloat16)
+    k, v = (torch.randn(kv_heads, S, hd, device="cuda", generator=g) for _ in range(2))
+    k[:, n:], v[:, n:] = float("nan"), float("nan")
+    assert _lib.load().sllm_prefill_attention_scratch(0, T, pos0, hd, heads, kv_heads) >= 4 * kv_heads * n * hd
+    got = K.prefill_attention(q, k, v, pos0, heads, kv_heads)
+    assert torch.equal(got, K.prefill_attention(q, k.to(torch.bfloat16), v.to(torch.bfloat16), pos0, heads, kv_heads))
+    plain = torch.empty_like(q)
+    _lib.check(_lib.load().sllm_prefill_attention(q.data_ptr(), k.data_ptr(), v.data_ptr(), 0, plain.data_ptr(), T, pos0, S, hd, heads, kv_heads, torch.cuda.current_stream().cuda_stream))
+    assert float((got.double() - plain.double()).norm() / plain.double().norm()) < 8e-3      # two results within 4e-3 of the same sums
