@@ -241,7 +241,30 @@ __device__ __forceinline__ void mma_halves(uint32_t a, uint32_t& hi, uint32_t& l
 __device__ __forceinline__ void mma_fragments(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
-__global__ void __launch_bounds__(kMmaWarps * 32, 1) seq_linear_rows_mma_kernel(LinArgs p, int wk_log2) {
+// A warp's results whose sums (in `tab`) are no number, once more: in fp32 from operands that are not split, a result at a time by all lanes.
+static __device__ __noinline__ void mma_unsplit(const LinArgs& p, const float* a, const uint16_t* W, const float* bias, float* out, const float* tab, int ldt, int WK, int n, int n0, int K) {
+    const int lane = threadIdx.x & 31;
+    for (int r0 = 4 * ((threadIdx.x >> 5) & 8); r0 < n; r0 += 64) {
+        double sum = 0.0;
+        for (int k = 0; r0 + lane < n && k < WK; ++k) sum += (double)tab[(size_t)k * 8 * ldt + r0 + lane];
+        for (uint32_t none = __ballot_sync(0xffffffffu, sum != sum); none; none &= none - 1) {
+            const int at = n0 + r0 + __ffs(none) - 1;
+            const uint16_t* w = W + (size_t)at * p.ldw;
+            float acc = 0.0f;
+            for (int k = 4 * lane; k < K; k += 128) {
+                const float4 x = *reinterpret_cast<const float4*>(a + k);
+                const uint2 u = *reinterpret_cast<const uint2*>(w + k);
+                acc = fmaf(seq_round_bf16(x.x), bf16_lo(u.x), fmaf(seq_round_bf16(x.y), bf16_hi(u.x), fmaf(seq_round_bf16(x.z), bf16_lo(u.y), fmaf(seq_round_bf16(x.w), bf16_hi(u.y), acc))));
+            }
+            acc = warp_sum(acc);
+            if (lane == 0) {
+                const float val = p.alpha * (acc + (bias ? bias[at] : 0.0f));
+                out[at] = p.accumulate ? out[at] + val : val;
+            }
+        }
+    }
+}
+__global__ void __launch_bounds__(kMmaWarps * 32, 1) seq_linear_rows_mma_kernel(const __grid_constant__ LinArgs p, int wk_log2) {
     extern __shared__ __align__(16) uint8_t mma_smem[];        // rings, 2 KB a warp for activations on their way, then [2][WK][8 activation rows][block + 8] partial sums
     const int b = blockIdx.y;
     const bool early = p.w_fixed && !p.w_index;
@@ -365,14 +388,26 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 1) seq_linear_rows_mma_kernel(
         __syncthreads();
         const float* bias = p.bias ? p.bias + (size_t)b * p.bias_bs : nullptr;
         float* out = p.C + (size_t)b * p.c_bs;
-        for (int o = threadIdx.x; o < n * p.T; o += kMmaWarps * 32) {
-            const int t = o / n, r = o % n, at = n_lo + blk * block + r;
+        // a warp has one activation row and every other 32 columns
+        const int t = warp & 7;
+        bool missing = false;
+        for (int r = 4 * (warp & 8) + lane; t < p.T && r < n; r += 64) {
+            const int at = n_lo + blk * block + r;
             double sum = 0.0;
+#pragma unroll 4
             for (int k = 0; k < WK; ++k) sum += (double)tab[(size_t)(k * 8 + t) * ldt + r];
+            if (__builtin_expect(sum != sum, 0)) {
+                missing = true;
+                continue;
+            }
             const float val = p.alpha * ((float)sum + (bias ? bias[at] : 0.0f));
             float* to = out + (size_t)t * p.ldc + at;
             *to = p.accumulate ? *to + val : val;
         }
+        // An infinite activation has no lower half (inf - inf), and an infinite weight times a lower half of zero is no number either, where the product itself would be infinite
+        if (__builtin_expect(__any_sync(0xffffffffu, missing), 0))
+            mma_unsplit(p, A + (size_t)t * p.lda, reinterpret_cast<const uint16_t*>(p.W) + (size_t)max(wb, 0) * p.w_bs, bias, out + (size_t)t * p.ldc, tab + (size_t)t * ldt, ldt, WK, n,
+                        n_lo + blk * block, K);
     }
 }
 
