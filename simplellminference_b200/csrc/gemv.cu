@@ -96,6 +96,8 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_split_kernel(PlainPolicy
     }
 }
 
+constexpr size_t kCtaSharedReserve = 1024;      // what the system keeps of an SM's shared memory for every resident CTA
+
 template <int WD>
 static int launch_plain(const PlainPolicy& p, cudaStream_t st) {
     const size_t smem = gemv_smem_bytes(p.ncols);
@@ -107,15 +109,18 @@ static int launch_plain(const PlainPolicy& p, cudaStream_t st) {
     }
     PlainPolicyT<WD> pt;
     static_cast<PlainPolicy&>(pt) = p;
-    // As many warps a pair of rows as still fit two CTAs per SM at once and leave each lane a load of 16 bytes. Measured, us a call one behind the other, a warp per pair | like this: fp32 2048 x 5632
+    // As many warps a pair of rows as still fit two CTAs per SM (or one) at once and leave each lane a load of 16 bytes. Measured, us a call one behind the other, a warp per pair | like this: fp32 2048 x 5632
     // 13.9 | 11.8, 1500 x 5632 12.2 | 9.9, 2300 x 11008 22.1 | 20.0; bf16 1500 x 5632 9.7 | 8.2, 2300 x 11008 15.9 | 13.9; int8 1500 x 5632 9.7 | 7.8, 2300 x 11008 12.7 | 12.4; the kernel alone,
     // int8 256 x 4096 5.0 | 3.9, 2048 x 5632 7.0 | 6.5. One warp a pair from 2369 rows on: 4096 x 4096 the same.
-    const int units = (p.nrows + 1) / 2, chunks = p.ncols / WInfo<WD>::E, warps = 2 * kGemvWarps * sm_count();
+    // A vector that takes more than half of an SM's shared memory (28 700 columns) leaves it one CTA, and one that fills it no room for the partial sums beside it.
+    const size_t split_smem = smem + kGemvWarps * sizeof(float2), sm_smem = (size_t)smem_optin_bytes() + kCtaSharedReserve;
+    const int resident = 2 * (split_smem + kCtaSharedReserve) <= sm_smem ? 2 : split_smem + kCtaSharedReserve <= sm_smem ? 1 : 0;
+    const int units = (p.nrows + 1) / 2, chunks = p.ncols / WInfo<WD>::E, warps = resident * kGemvWarps * sm_count();
     int parts = 1;
     while (parts < kGemvWarps && 2LL * parts * units <= warps && chunks / (2 * parts) >= 32) parts *= 2;
     if (parts > 1 && g_tune_ctas_per_sm == 0) {
         static size_t split_configured = 0;
-        if (smem + 64 > 48 * 1024 && smem > split_configured) {
+        if (split_smem > 48 * 1024 && smem > split_configured) {
             SLLM_CUDA(cudaFuncSetAttribute(gemv_split_kernel<WD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             split_configured = smem;
         }

@@ -1,14 +1,11 @@
-"""kernel::matmul over few rows, whose columns several warps share: odd row counts, shares that end inside a load of 32 lanes, one and several loads a share, and the line where a warp
-takes a pair of rows alone."""
+"""kernel::matmul over few rows, whose columns several warps share: odd row counts, shares that end inside a load of 32 lanes, one and several loads a share, the line where a warp
+takes a pair of rows alone, and vectors up to the longest that shared memory holds."""
 import pytest
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("rows", [1, 2, 7, 255, 1184, 1185, 2367, 2369])
-@pytest.mark.parametrize("cols", [256, 1024, 1088, 4160, 11264])
-@pytest.mark.parametrize("dtype", ["f32", "bf16", "int8"])
-def test_product(rows, cols, dtype):
+def _check(rows, cols, dtype, in_a_row):
     import torch
 
     from simplellminference_b200 import kernels
@@ -24,6 +21,21 @@ def test_product(rows, cols, dtype):
         full = w.double()
     got = kernels.matmul(x, w, rows, cols, {"f32": F32, "bf16": BF16, "int8": INT8}[dtype], scales, 64, 0.125).double()
     want = full @ x.double() * 0.125
-    # fp32 sums of at most cols / 64 + 32 products in a row
-    bound = (cols / 64 + 40) * 2.0 ** -24 * (full.abs() @ x.double().abs()) * 0.125
+    bound = (in_a_row + 8) * 2.0 ** -24 * (full.abs() @ x.double().abs()) * 0.125
     assert bool(((got - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("rows", [1, 2, 7, 255, 1184, 1185, 2367, 2369])
+@pytest.mark.parametrize("cols", [256, 1024, 1088, 4160, 11264])
+@pytest.mark.parametrize("dtype", ["f32", "bf16", "int8"])
+def test_product(rows, cols, dtype):
+    # fp32 sums of at most cols / 64 + 32 products in a row
+    _check(rows, cols, dtype, cols / 64 + 32)
+
+
+@pytest.mark.parametrize("rows", [1, 5, 600])
+@pytest.mark.parametrize("cols", [14400, 28672, 28736, 57984, 58048])
+@pytest.mark.parametrize("dtype", ["f32", "bf16", "int8"])
+def test_long_rows(rows, cols, dtype):
+    """Two CTAs an SM, one, and no room for the sums of several warps beside the vector: a lane then takes a 32nd of the columns."""
+    _check(rows, cols, dtype, cols / 32)
