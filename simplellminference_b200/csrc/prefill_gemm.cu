@@ -41,7 +41,7 @@ constexpr uint32_t kPfABytes = kPfBM * kPfBK * 2;
 // the host picks the BN that fills the last wave best, e.g. 192 instead of 256 for a 512 x 12288 output on 74 SM pairs.
 constexpr int kPfMaxStages = 12;
 constexpr uint32_t kPfRingBytes = 192 * 1024;          // operand ring; stages = ring / (A box + this CTA's W box)
-constexpr long long kPfWaitClocks = 1ll << 33;         // some 4 seconds
+constexpr long long kPfPollClocks = 512;               // a poll that g_tune_tc_polls allows, in clocks: some 4 seconds in all by default
 constexpr uint32_t kPfTmemCols = 512;                  // two accumulators of up to 256 fp32 columns
 constexpr size_t kPfSmem = 1024 /*alignment slack*/ + kPfRingBytes + 512 /*barriers + tmem slot*/ + 4 * 4096 /*rows on their way through the epilogue*/;
 
@@ -61,14 +61,15 @@ struct PfDev {           // kernel-side view of PfGemmArgs
     const int32_t* rows_dev;   // the row tiles beyond ceil(*rows_dev / tile rows) are skipped by every role alike
     int32_t groups;            // matrices one behind the other, each with its own count in rows_dev; T and N are then those of one group
     int32_t* status;           // where a wait that was given up is reported
+    long long wait_clocks;     // and after how long it is
 };
 
-// Bounded wait on a barrier: false once some seconds have passed or another thread of the CTA has given up. The kernel then tears down without its result and says so in the
-// library's status word. (By the clock and not by polls: a poll may sleep.)
-__device__ __forceinline__ bool pf_wait(uint64_t* bar, uint32_t parity, volatile int* gave_up) {
+// Bounded wait on a barrier: false once `limit` clocks have passed (0: without a poll) or another thread of the CTA has given up. The kernel then tears down without its result and says
+// so in the library's status word. (By the clock and not by polls: a poll may sleep.)
+__device__ __forceinline__ bool pf_wait(uint64_t* bar, uint32_t parity, volatile int* gave_up, long long limit) {
     uint32_t done;
     long long since = 0;
-    while (true) {
+    while (limit) {
         asm volatile(
             "{\n.reg .pred p;\n"
             "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
@@ -77,7 +78,7 @@ __device__ __forceinline__ bool pf_wait(uint64_t* bar, uint32_t parity, volatile
         if (done) return true;
         const long long now = clock64();
         if (!since) since = now;
-        if (*gave_up || now - since > kPfWaitClocks) break;
+        if (*gave_up || now - since > limit) break;
     }
     *gave_up = 1;
     return false;
@@ -401,7 +402,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
                 const int w_row = p.tiled ? 0 : n0, w_tile = p.tiled ? n0 / p.R : 0;
                 int ks = kb0 / p.kb_per_seg, kk = kb0 - ks * p.kb_per_seg;
                 for (int kb = kb0; kb < kb1; ++kb) {
-                    ok = pf_wait(empty + stage, phase ^ 1, gave_up);
+                    ok = pf_wait(empty + stage, phase ^ 1, gave_up, p.wait_clocks);
                     if (!ok) break;
                     const uint32_t bar = full_at + 8 * stage;
                     if (!PAIR) mb_expect(full + stage, tx_bytes);
@@ -424,12 +425,12 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
             for (int unit = worker; ok && walk.reach(unit); unit += nworkers) {
                 const int part = (unit - walk.base) % p.ksplit;
                 const int n_kb = (p.nkb * (part + 1)) / p.ksplit - (p.nkb * part) / p.ksplit;
-                ok = pf_wait(tempty + acc, acc_phase ^ 1, gave_up);   // the epilogue has drained this accumulator
+                ok = pf_wait(tempty + acc, acc_phase ^ 1, gave_up, p.wait_clocks);   // the epilogue has drained this accumulator
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + (uint32_t)(acc * 256);
                 for (int kb = 0; kb < n_kb; ++kb) {
-                    ok = pf_wait(full + stage, phase, gave_up);
+                    ok = pf_wait(full + stage, phase, gave_up, p.wait_clocks);
                     if (!ok) break;
                     tc_fence_after();
                     const uint64_t ad = a_desc + (uint64_t)((uint32_t)stage * (kPfABytes >> 4)), bd = b_desc + (uint64_t)((uint32_t)stage * (b_bytes >> 4));
@@ -459,7 +460,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
             const int t0 = m_tile * BM + (int)rank * kPfBM + quad * 32, t = t0 + lane;
             const bool bias = p.bias && (unit - walk.base) % p.ksplit == 0;   // the bias rides on the first share of K
             // the warp goes on as one: what follows are instructions of all its lanes
-            if (!__all_sync(0xffffffffu, pf_wait(tfull + acc, acc_phase, gave_up))) break;
+            if (!__all_sync(0xffffffffu, pf_wait(tfull + acc, acc_phase, gave_up, p.wait_clocks))) break;
             tc_fence_after();
             const uint32_t src = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * 256);
 #pragma unroll 1
@@ -486,7 +487,12 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
         __syncwarp();
     }
     tc_fence_before();
-    if (PAIR) cluster_sync_all(); else __syncthreads();   // pair: nobody leaves while the peer may still signal its barriers / read its operands
+    if (PAIR) {       // what is on its way for a CTA of a pair that gave up may reach into the other one's memory: both take their time then
+        if (*gave_up) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(mapa_u32(const_cast<const int*>(gave_up), rank ^ 1)), "r"(1) : "memory");
+        cluster_sync_all();      // nobody leaves while the peer may still signal its barriers / read its operands
+    } else {
+        __syncthreads();
+    }
     if (__syncthreads_or(*gave_up)) tc_gave_up(p.status);
     if (warp == 1) {
         tc_fence_after();
@@ -632,6 +638,7 @@ int pf_gemm(PfCache* cache, const PfGemmArgs& a, cudaStream_t st) {
     p.groups = groups;
     if (int rc = status_check()) return rc;
     if (int rc = status_word(&p.status)) return rc;
+    p.wait_clocks = kPfPollClocks * g_tune_tc_polls;
 
     CUtensorMap tmA;
     {

@@ -772,7 +772,7 @@ extern "C" int sllm_seq_linear(const float* A, int32_t lda, const void* W, int32
         const size_t m = (size_t)T * N;
         overlapping(seq_linear_epilogue_kernel)<<<(int)std::min<size_t>((m + 255) / 256, (size_t)sm_count() * 8), 256, 0, st>>>(P, bias, C, ldc, T, N, alpha, accumulate);
         ++g_launches;
-        SLLM_LAUNCH_CHECK();
+        SLLM_LAUNCH_CHECK_ONLY();
         return SLLM_OK;
     }
     dim3 grid((N + kTN - 1) / kTN, (T + kTM - 1) / kTM, batch);

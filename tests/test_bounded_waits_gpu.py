@@ -1,4 +1,4 @@
-"""Waits inside the tcgen05 attention kernels that run out: the report, and that nothing of it stays behind."""
+"""Waits inside the tcgen05 kernels that run out: the report, and that nothing of it stays behind."""
 import pytest
 from test_attention_forms_gpu import _close, _inputs, _ops, _run
 from test_attention_tc_gpu import _want
@@ -36,3 +36,29 @@ def test_waits_that_run_out_are_reported(which):
     torch.cuda.synchronize()
     assert lib.sllm_status() == 0
     assert _close(call(), want, 4e-6 if which == "paged" else 4e-3)
+
+
+@pytest.mark.parametrize("T", [100, 700], ids=["one SM", "two SMs a tile"])
+def test_waits_of_a_product_that_run_out_are_reported(T):
+    """The same for the product, whose roles all give up and whose CTAs of a pair leave together."""
+    import torch
+
+    from simplellminference_b200 import _lib, kernels
+    lib, g = _lib.load(), torch.Generator(device="cuda").manual_seed(T)
+    a = torch.randn(T, 512, generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randn(4100, 512, generator=g, device="cuda").to(torch.bfloat16)
+    want = a.double() @ w.double().T
+    assert lib.sllm_status() == 0
+    assert lib.sllm_tune(10, 0) == 0
+    try:
+        kernels.prefill_gemm(a, w)
+        torch.cuda.synchronize()
+    finally:
+        assert lib.sllm_tune(10, 1 << 24) == 0
+    with pytest.raises(_lib.SllmError) as e:
+        kernels.prefill_gemm(a, w)
+    assert e.value.code == _lib.ETIMEOUT
+    torch.cuda.synchronize()
+    assert lib.sllm_status() == 0
+    for _ in range(3):                  # tensor memory and barriers of the SMs are free again
+        assert float((kernels.prefill_gemm(a, w).double() - want).norm() / want.norm()) < 1e-6
