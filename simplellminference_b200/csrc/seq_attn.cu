@@ -560,22 +560,18 @@ int sllm_seq_rotary_kv(const sllm_seq_batch* b, float* q, int32_t ldq, int32_t h
 // cluster of up to 16 CTAs per (sequence, G query heads of a kv head, share), two CTAs of 128 threads per SM in all. Clusters of 16 find few places at a
 // time, so they pay only when the step has no more of them than fit at once. Measured (us) at 16 | 8 | 4 CTAs: one request of 8000 positions, 8 kv
 // heads 17.9 | 23.4 | 35.0; four of 2048, 4 kv heads 17.6 | 11.2 | 13.1; with twice as many CTAs 32 requests of 2048 take 54 instead of 47.
+// `pairs`: kernels whose clusters take two requests each, of more than two CTAs and of two, or nullptr; pairs_fit: how many clusters of 2 .. 8 CTAs of them are resident at once,
+// -1 = to be asked. heads_first: the kernel takes all heads of the longest context first.
 template <typename Kernel, typename... Args>
-static int launch_attention_decode(Kernel* kernel, int G, int smem, sllm::AttnArgs p, bool foldable, cudaStream_t st, Args... args) {
+static int launch_attention_decode(Kernel* kernel, Kernel* const* pairs, int* pairs_fit, int G, int smem, sllm::AttnArgs p, bool heads_first, cudaStream_t st, Args... args) {
     using namespace sllm;
-    const long long items = (long long)p.b.n_qtiles * (p.heads / G) * p.nsplit;
+    const int n = p.b.n_qtiles, sets = p.heads / G;
+    const long long items = (long long)n * sets * p.nsplit;
     int cs = items * kDecodeCluster <= sm_count() ? kDecodeCluster : kDecodeCluster / 2;
     while (cs > 1 && (items * cs > 2LL * sm_count() || (long long)p.nsplit * cs > 65535)) cs /= 2;
-    // clusters of up to eight CTAs, two rounds of them at most, that the kernel may fold to those of one round (it looks at the contexts)
-    const bool heads_first = foldable && p.b.n_qtiles <= 65535;
-    p.fold = heads_first ? 1 : 0;
-    p.slots = 2 * sm_count();
-    while (heads_first && p.b.n_qtiles > 1 && p.b.n_qtiles <= kDecodeWarps * 32 && cs < kDecodeCluster / 2 && items * 2 * cs <= 4LL * sm_count() && (long long)p.nsplit * 2 * cs <= 65535) {
-        cs *= 2;
-        p.fold *= 2;
-    }
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = heads_first ? dim3(p.heads / G, p.b.n_qtiles, p.nsplit * cs) : dim3(p.b.n_qtiles, p.heads / G, p.nsplit * cs);
+    p.by_request = !heads_first || n > 65535;
+    cfg.gridDim = p.by_request ? dim3(n, sets, p.nsplit * cs) : dim3(sets, n, p.nsplit * cs);
     cfg.blockDim = dim3(kDecodeWarps * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -585,6 +581,27 @@ static int launch_attention_decode(Kernel* kernel, int G, int smem, sllm::AttnAr
     attr[0].val.clusterDim.z = cs;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    if (pairs && n > 1 && n <= 2 * 65535 && cs < kDecodeCluster / 2 && p.nsplit <= 65535 / 8) {
+        // the largest clusters, of any number of CTAs, of which all are resident at once
+        const long long clusters = (long long)sets * ((n + 1) / 2) * p.nsplit;
+        cudaLaunchConfig_t two = cfg;
+        for (int size = 8; size >= 2 * cs; --size) {
+            if (clusters * size > 2LL * sm_count()) continue;
+            Kernel* with = pairs[size == 2];
+            two.gridDim = dim3(sets, (n + 1) / 2, p.nsplit * size);
+            attr[0].val.clusterDim.z = size;
+            int& fit = pairs_fit[size];
+            if (fit < 0 && cudaOccupancyMaxActiveClusters(&fit, with, &two) != cudaSuccess) {
+                cudaGetLastError();
+                fit = 0;
+            }
+            if (clusters > fit) continue;
+            cfg = two;
+            kernel = with;
+            break;
+        }
+        if (kernel != pairs[0] && kernel != pairs[1]) attr[0].val.clusterDim.z = cs;
+    }
     SLLM_CUDA(cudaLaunchKernelEx(&cfg, overlapping(kernel), p, args...));
     ++g_launches;
     SLLM_LAUNCH_CHECK();
@@ -594,16 +611,20 @@ static int launch_attention_decode(Kernel* kernel, int G, int smem, sllm::AttnAr
 template <int D, bool kOpts>
 static int attention_decode_bf16(const sllm::AttnArgs& p, cudaStream_t st) {
     using namespace sllm;
-    auto* kernel = seq_attention_decode_mma_kernel<D, kOpts>;
+    auto* kernel = seq_attention_decode_mma_kernel<D, kOpts, 0>;
+    static decltype(kernel) const pairs[2] = {seq_attention_decode_mma_kernel<D, kOpts, 1>, seq_attention_decode_mma_kernel<D, kOpts, 2>};
     static bool ready = false;
+    static int pairs_fit[9] = {-1, -1, -1, -1, -1, -1, -1, -1, -1};
     if (!ready) {
-        SLLM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        SLLM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DecodeTile<D>::kSmem));
+        for (auto* k : {kernel, pairs[0], pairs[1]}) {
+            SLLM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            SLLM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, DecodeTile<D>::kSmem));
+        }
         ready = true;
     }
     const int group = p.heads / p.kv_heads;
     const int G = group % 4 == 0 ? 4 : group % 3 == 0 ? 3 : group % 2 == 0 ? 2 : 1;
-    return launch_attention_decode(kernel, G, DecodeTile<D>::kSmem, p, true, st, G);
+    return launch_attention_decode(kernel, pairs, pairs_fit, G, DecodeTile<D>::kSmem, p, true, st, G);
 }
 
 template <int L, int G, int S>      // loads per lane of a row, query heads of a CTA, rows in flight per lane
@@ -615,7 +636,7 @@ static int attention_decode_f32(const sllm::AttnArgs& p, cudaStream_t st) {
         SLLM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         ready = true;
     }
-    return launch_attention_decode(kernel, G, 0, p, false, st);
+    return launch_attention_decode(kernel, (decltype(kernel) const*)nullptr, nullptr, G, 0, p, false, st);
 }
 
 static int attention_decode(const sllm::AttnArgs& p, int kv_dtype, cudaStream_t st) {

@@ -25,8 +25,7 @@ struct AttnArgs {
     int chunk;                // > 0: a query sees its own chunk of `chunk` positions only (then window / keep_first are not used)
     float* out; int ldo; uint16_t* out16;   // one share: the normalised result goes here (fp32 [T][ldo] and / or dense bf16) instead of ws
     uint32_t page_magic;      // ceil(2^32 / page_len): the page of a position without a division (page_of)
-    // Decode over bf16 pools: a cluster may be folded, i.e. serve `fold` items (a request and a set of heads) with 1 / fold of its CTAs each; 1 = it serves one. 0: the grid has the requests in x (more of them than y takes). `slots`: CTAs that are resident at once.
-    int fold, slots;
+    int by_request;           // decode over bf16 pools: the grid has the requests in x (more of them than y takes)
 };
 
 // prompt portions over bf16 pools on tcgen05: dk = dv = 64 or 128, pools 16-byte aligned, no values inside keys, no cross values (seq_attn_tc.cu)
@@ -325,7 +324,18 @@ __device__ __forceinline__ void ldmatrix4_trans(uint32_t (&r)[4], uint32_t addr)
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
 
-template <int D, bool kOpts>     // kOpts: capped scores or charges on the distance (a window, kept positions and chunks are part of both)
+// What a second turn of a cluster costs, in runs of 16 keys a warp
+constexpr float kTurnRuns = 4.0f;
+
+// kOpts: capped scores or charges on the distance (a window, kept positions and chunks are part of both). kPair: 0 = a cluster has one item (a request and a set of heads), the grid is
+// (sets, requests) or, with by_request, (requests, sets); else it has those of two requests, the x-th and the x-th from the back of the caller's list (the longest context first), and
+// kPair = 2: it has two CTAs.
+// A step's clusters are all resident at once. With one item each, requests of unequal length leave most of the machine idle behind the longest; a pair divides its CTAs by what the two
+// contexts need and, where that leaves the longer one too few, takes them one behind the other with all of them. Clusters look at their own pair only. Measured, us in a captured graph, one item a
+// cluster | pairs, contexts of 16 to 8000 positions, 32 heads over 8 of 128: five requests 28.4 | 23.1, eight 36.1 | 27.4, 13 57.9 | 35.7, 32 95.5 | 61.9; requests alike, whose pairs only cost (barriers of larger
+// clusters): eight of 64, 1000 and 2048 7.0 | 7.0, 11.7 | 11.9, 18.0 | 18.1, 16 of 300 9.4 | 9.9, 13 of 6000 59.9 | 62.9; 8 heads over 8 of 64: eight of 64 and 1000 5.5 | 5.7, 8.2 | 8.5, 13 of 300 7.0 | 7.5, 32 of 64
+// 5.5 | 5.7. (Twice as many clusters as fit at once, half of which left again where requests are alike: 21.9, 25.6, 36.6, 58.5; alike 8.9, 13.2, 19.3, 11.3, 72.4; 7.4, 10.3, 8.4, 7.7.)
+template <int D, bool kOpts, int kPair>
 __global__ void __launch_bounds__(kDecodeWarps * 32, 2) seq_attention_decode_mma_kernel(AttnArgs p, int G) {
     static_assert(kDecodeWarps == 4, "sums of a column");
     after_previous();
@@ -333,67 +343,54 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, 2) seq_attention_decode_mma
     using Tile = DecodeTile<D>;
     constexpr int kRun = Tile::kRun, kRing = Tile::kRing, kSteps = D / 16, kTiles = D / 8;
     extern __shared__ __align__(16) uint16_t dsm[];
-    __shared__ __align__(16) float got_o[kDecodeWarps * 4 * D];
+    __shared__ __align__(16) float got_o[kDecodeWarps * (4 * D + (kPair ? 16 : 0))];      // (a cluster's share of an item may be any number of CTAs up to eight)
     __shared__ __align__(16) float2 got_ml[kDecodeCluster * kDecodeWarps * 4];
     __shared__ float weight[kDecodeCluster * kDecodeWarps][4], total[4][2];
     const sllm_seq_batch& b = p.b;
     cg::cluster_group cluster = cg::this_cluster();
     const int full = (int)cluster.num_blocks(), split = blockIdx.z / full;
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");      // waited for before anything is sent: every CTA of the cluster runs by then (nothing is handed over)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3, h = g >> 1;
-    // Items in the caller's order of requests (the longest context first), all heads of one before the next. Few long requests among short ones keep the last CTAs busy long after the others:
-    // then a cluster per item, more than fit at once, is better; requests alike are better off when every item starts at once in a part of a cluster. The longest share of a
-    // warp, in runs, stands against all the runs a warp gets and what an item costs beside them (5.7 runs). Measured, us, folded | unfolded | as chosen: eight requests of 77 to 8000 positions
-    // 41 | 30 | 31, eight of 2048 18.4 | 28 | 19.1, eight of 6000 38.5 | 47 | 38.4, 13 of 16 to 8000 61 | 36 | 39, 32 of them 90 | 57 | 57, 32 of 2048 47 | 54 | 48, 16 of 1000 17.9 | 24 | 18.5.
-    int CS = full, sub = 0, item_x = p.fold ? blockIdx.y : blockIdx.x, item_y = p.fold ? blockIdx.x : blockIdx.y;
-    int seg = b.qt_seg[item_x], t = b.seg_start[seg], pos = b.seg_pos0[seg], slot = b.seg_slot[seg];
-    bool present = true;
-    if (p.fold > 1) {
-        // both places this CTA may have are looked up beside the contexts
-        const int small = full / p.fold, folded_sub = (int)cluster.block_rank() / small, item = (blockIdx.y * gridDim.x + blockIdx.x) * p.fold + folded_sub;
-        const int folded_x = min(item / (int)gridDim.x, (int)gridDim.y - 1), fseg = b.qt_seg[folded_x], ft = b.seg_start[fseg], fpos = b.seg_pos0[fseg], fslot = b.seg_slot[fseg];
-        __shared__ float part[kDecodeWarps][2];
-        float most = 0.0f, all = 0.0f;
-        if ((int)threadIdx.x < b.n_qtiles) {
-            const int at = b.seg_pos0[b.qt_seg[threadIdx.x]];
-            most = all = (float)(TileList(at, at, seq_row_window(at, p.window, p.chunk), p.keep_first, kBK).n * (kBK / kRun));
-        }
-        most = warp_max(most);
-        all = warp_sum(all);
-        if (lane == 0) {
-            part[warp][0] = most;
-            part[warp][1] = all;
-        }
-        __syncthreads();
-        most = all = 0.0f;
-#pragma unroll
-        for (int i = 0; i < kDecodeWarps; ++i) {
-            most = fmaxf(most, part[i][0]);
-            all += part[i][1];
-        }
-        const float per = (float)(full * kDecodeWarps * p.nsplit);      // warps of an item
-        const float apart = (all / per + 5.7f * (float)b.n_qtiles) * (float)(gridDim.x * full * p.nsplit) / (float)p.slots;
-        if (fmaxf(apart, most / per) >= 0.9f * most * (float)p.fold / per) {
-            if (item - folded_sub >= (int)(gridDim.x * gridDim.y)) return;                // the whole cluster
-            present = item < (int)(gridDim.x * gridDim.y);
-            CS = small;
-            sub = folded_sub;
-            item_x = folded_x;
-            item_y = item % (int)gridDim.x;
-            seg = fseg;
-            t = ft;
-            pos = fpos;
-            slot = fslot;
+    struct Item { int t, pos, slot; };
+    auto look_up = [&](int x) {
+        const int seg = b.qt_seg[x];
+        return Item{b.seg_start[seg], b.seg_pos0[seg], b.seg_slot[seg]};
+    };
+    auto runs_of = [&](int pos) { return TileList(pos, pos, seq_row_window(pos, p.window, p.chunk), p.keep_first, kBK).n * (kBK / kRun); };
+    const bool swapped = !kPair && p.by_request;
+    Item item = look_up(swapped ? blockIdx.x : blockIdx.y), next{};
+    const int set = swapped ? blockIdx.y : blockIdx.x;
+    int CS = full, base_rank = 0, turns = 1;
+    if constexpr (kPair != 0) {
+        const int other = b.n_qtiles - 1 - (int)blockIdx.y;
+        next = look_up(other);
+        if (other != (int)blockIdx.y) {
+            const int a = runs_of(item.pos), z = runs_of(next.pos);
+            int first = full / 2;      // CTAs of the first item: as many as end it with the other, one at least for either
+            if (a != z) {
+                first = min(full - 1, max(1, (int)((float)(a * full) / (float)(a + z) + 0.5f)));
+                const float apart = fmaxf((float)a / (float)first, (float)z / (float)(full - first));
+                if (apart * (float)full - (float)(a + z) > kTurnRuns * (float)(full * kDecodeWarps * p.nsplit)) turns = 2;
+            }
+            if (turns == 1) {
+                const bool mine = (int)cluster.block_rank() < first;
+                CS = mine ? first : full - first;
+                base_rank = mine ? 0 : first;
+                if (!mine) item = next;
+            }
         }
     }
-    const int base_rank = sub * CS, rank = (int)cluster.block_rank() - base_rank;
-    cluster.barrier_arrive();       // waited for before anything is sent: every CTA of the cluster runs by then
-    if (!present) {
-        cluster.barrier_wait();
-        cluster.sync();
-        return;
-    }
-    const int group = p.heads / p.kv_heads, subsets = group / G, gkv = item_y / subsets, h0 = gkv * group + (item_y % subsets) * G;
+    const bool alone = kPair == 2 && CS == 1;       // nobody in the cluster waits for anybody
+    const int rank = (int)cluster.block_rank() - base_rank;
+    const int group = p.heads / p.kv_heads, subsets = group / G, gkv = set / subsets, h0 = gkv * group + (set % subsets) * G;
     const bool live = h < G, second = g & 1;           // this lane's head exists; it holds the second terms (and no third ones)
+#pragma unroll 1
+    for (int turn = 0; turn < (kPair ? turns : 1); ++turn) {
+    if (turn) {
+        cluster.barrier_arrive();   // what was sent to this thread in the turn before has been read
+        item = next;
+    }
+    const int t = item.t, pos = item.pos, slot = item.slot;
     const int wnd = seq_row_window(pos, p.window, p.chunk);
     const TileList tiles(pos, pos, wnd, p.keep_first, kBK);
     const int n_runs = tiles.n * (kBK / kRun), workers = p.nsplit * CS * kDecodeWarps;
@@ -565,7 +562,7 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, 2) seq_attention_decode_mma
     l += __shfl_xor_sync(0xffffffffu, l, 2);
     // every CTA of the cluster gets the sums of its own share of the results, and everybody's maxima
     const int share = (G * D + 2 * CS - 1) / (2 * CS) * 2, worker = rank * kDecodeWarps + warp, columns = G * D;
-    cluster.barrier_wait();
+    if (!alone) cluster.barrier_wait();
     if (live) {
 #pragma unroll
         for (int i = 0; i < kTiles / 2; ++i) {
@@ -575,7 +572,7 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, 2) seq_attention_decode_mma
         if (!second)
             for (int r = c; r < CS; r += 4) cluster.map_shared_rank(got_ml, base_rank + r)[worker * 4 + h] = make_float2(m, l);
     }
-    cluster.sync();
+    if (alone) __syncthreads(); else cluster.sync();
     if (warp < G) {
         const int n = CS * kDecodeWarps;
         float M = -INFINITY, L = 0.0f;
@@ -598,6 +595,7 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, 2) seq_attention_decode_mma
         const int at = rank * share + i, hh = at / D, col = at % D;
         if (at >= columns) break;
         float sums[kDecodeWarps] = {};                  // (several: fewer roundings in a row)
+#pragma unroll 4
         for (int wkr = 0; wkr < CS * kDecodeWarps; wkr += kDecodeWarps)
 #pragma unroll
             for (int e = 0; e < kDecodeWarps; ++e) sums[e] = fmaf(got_o[(wkr + e) * share + i], weight[wkr + e][hh], sums[e]);
@@ -614,6 +612,7 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, 2) seq_attention_decode_mma
                 rec[1] = total[hh][1];
             }
         }
+    }
     }
 }
 
