@@ -8,6 +8,7 @@
 //     run as a short epilogue kernel over C.
 // In bf16 mode (round_a) the activations are rounded to bf16 as they are loaded, so all three bodies multiply the same operands and
 // differ only in summation order.
+#include <climits>
 #include <type_traits>
 
 #include "prefill.cuh"
@@ -675,13 +676,25 @@ static int launch_rows(const sllm::LinArgs& p, int batch, cudaStream_t st) {
     const bool stream = vec && (p.T <= 4          ? weights >= 1500000LL
                                 : bf16 ? p.T <= 6 ? weights >= 2800000LL && rows >= 4 * sms : weights >= 2000000LL
                                                   : (weights >= 2800000LL && rows >= 10 * sms) || (p.T >= 7 && weights >= 4500000LL && rows >= 4 * sms));
-    // bf16 rows on the tensor cores. Measured in a captured graph, us, small body | streaming | this one: two rows 1024 x 1024 3.9 | 4.5 | 4.3, 1536 x 1024 5.3 | 4.6 | 4.3, 2800 x 1024
-    // 6.6 | 5.8 | 5.2, 2048 x 2048 7.3 | 5.9 | 5.9, 6144 x 4096 26.6 | 12.1 | 13.4; three rows 512 x 4096 5.3 | 6.3 | 5.5, 1024 x 1024 4.3 | 5.7 | 4.4, 2048 x 1024 6.6 | 6.2 | 4.9;
-    // four rows 512 x 1024 3.6 | 5.8 | 4.4, 1024 x 1024 4.6 | 5.9 | 4.4, 6144 x 4096 45 | 14.1 | 13.9, 2048 x 5632, which takes two panels of K, 20.6 | 10.6 | 11.5; six rows 512 x 1024 4.1 | 7.6 | 4.6; eight rows 512 x 1024 4.7 | 8.0 | 4.7,
-    // 2048 x 2048 13.3 | 11.8 | 6.5, 6144 x 4096 84 | 23.5 | 14.7, 16384 x 4096 140 | 46.5 | 27.8, 1000 x 11008 34 | 24.9 | 13.9. One row is streamed: 6144 x 4096 18.7 | 11.5 | 13.3.
-    const bool mma = vec && bf16 && p.round_a && (p.T >= 5 || (p.K <= kMmaWarps * kMmaSlice && (p.T == 4 || (p.T >= 2 && rows >= 4 * sms && (p.T == 3 || weights <= 3000000LL)))));
-    const long long mma_from = p.T <= 3 ? 1200000LL : p.T == 4 ? 900000LL : p.T <= 6 ? 750000LL : 500000LL;
-    if (mma ? weights >= mma_from : stream) {
+    // bf16 rows on the tensor cores, where they are ahead of the body that they would take else. That kernel takes 4.3 to 5 us up to some 1.2 million weights (its ring, the split, the last sums),
+    // 2 to 3 more where K is longer than one panel, and has tiles that are half empty below four rows an SM; the small body grows with rows times weights. Measured in a captured graph, us, other
+    // body | this one, s = the other one streams: two rows 1024 x 1024 3.9 | 4.3, 700 x 2048 5.2 | 4.5, 2048 x 1024 s 5.1 | 5.0, 2048 x 2048 s 5.9 | 6.0; three rows 1024 x 1024 4.3 | 4.4, 700 x 2048 5.7 | 4.6,
+    // 400 x 4096 s 5.8 | 5.3, 2048 x 1024 s 6.3 | 5.1; four rows 700 x 1024 3.9 | 4.4, 1024 x 1024 4.6 | 4.4, 256 x 4096 4.7 | 5.3, 400 x 4096 s 6.0 | 5.4, 6144 x 4096 s 14.1 | 13.7, 1024 x 5632 s 8.5 | 8.8; five rows
+    // 1500 x 512 4.2 | 4.5, 1024 x 1024 4.9 | 4.5, 256 x 4096 5.2 | 5.5, 512 x 4096 6.4 | 6.0, 512 x 5632 8.1 | 8.4, 256 x 8192 8.5 | 8.6, 512 x 8192 9.7 | 9.0, 140 x 11008 11.6 | 10.3; six rows 400 x 2048 4.5 | 4.9, 512 x 2048
+    // 5.1 | 4.9, 400 x 5632 8.2 | 8.4, 512 x 5632 8.9 | 8.5, 64 x 8192 8.5 | 8.1; seven rows 400 x 2048 4.7 | 5.0, 512 x 2048 5.4 | 5.0, 140 x 4096 5.9 | 5.7; eight rows 512 x 1024 4.7 | 4.7, 700 x 1024 5.0 | 4.7, 140 x 4096
+    // 6.5 | 5.8, 2048 x 2048 s 11.9 | 6.6, 6144 x 4096 s 23.5 | 14.6, 16384 x 4096 s 46.5 | 27.8. One row is streamed: 6144 x 4096 11.5 | 13.3.
+    const bool many = rows >= 4 * sms, one_panel = p.K <= kMmaWarps * kMmaSlice;
+    const long long never = LLONG_MAX;
+    const long long mma_from = p.T == 2   ? many && one_panel && weights <= 3100000LL ? 1300000LL : never
+                               : p.T == 3 ? !one_panel ? never : many ? 1200000LL : 1500000LL
+                               : p.T == 4 ? !one_panel ? never : many ? 1000000LL : 1500000LL
+                               : p.T == 5 ? many ? 900000LL : p.K > 8192 ? 700000LL : p.K == 8192 ? 3000000LL : one_panel ? 1500000LL : never
+                               : p.T == 6 ? many ? 850000LL : p.K >= 8192 ? 500000LL : one_panel ? 1000000LL : 2800000LL
+                               : p.T == 7 ? many ? 700000LL : p.K >= 4096 ? 500000LL : 1000000LL
+                               : p.T == 8 ? many ? 600000LL : p.K >= 4096 ? 500000LL : 900000LL
+                                          : never;
+    const bool mma = vec && bf16 && p.round_a && weights >= mma_from;
+    if (mma || stream) {
         int rc;
         if (mma) rc = launch_rows_mma(p, batch, st);
         else if (p.T == 1) rc = bf16 ? launch_rows_body<SLLM_BF16, 1>(p, batch, st) : launch_rows_body<SLLM_F32, 1>(p, batch, st);
