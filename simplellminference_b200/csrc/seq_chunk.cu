@@ -365,6 +365,7 @@ __global__ void __launch_bounds__(PARTS * GROUPS * 32, 1) seq_chunk_walk_kernel(
     extern __shared__ __align__(16) uint8_t cw_sm[];
     __shared__ uint64_t landed[kWalkStages];             // the records
     constexpr int dkp = KS * 16, HS = KS / PARTS, kThreads = PARTS * GROUPS * 32, kCols = GROUPS * 16, kTiles = kChunk / 8;
+    constexpr bool kThird = kDelta && KS == 2;           // u as three bf16 terms
     constexpr uint32_t kPlane = kChunk * dkp * 2;
     constexpr uint32_t rec_bytes = (uint32_t)chunk_record_bytes(dkp), stage_bytes = rec_bytes + kChunk * kCols * 4;
     const sllm_seq_batch& b = p.b;
@@ -503,7 +504,7 @@ __global__ void __launch_bounds__(PARTS * GROUPS * 32, 1) seq_chunk_walk_kernel(
                 v[nt][3] -= y.w;
             }
         }
-        uint32_t uh[2][4], ul[2][4];
+        uint32_t uh[2][4], ul[2][4], u3[2][4];
         auto operand = [&](const float (&y)[kTiles][4]) {     // rows x 2 times 16 tokens as A fragments
 #pragma unroll
             for (int pr = 0; pr < 2; ++pr) {
@@ -529,6 +530,20 @@ __global__ void __launch_bounds__(PARTS * GROUPS * 32, 1) seq_chunk_walk_kernel(
 #pragma unroll
                 for (int e = 0; e < 4; ++e) u[nt][e] += lo[nt][e] + mid[nt][e];
             operand(u);
+            if (kThird) {
+                auto rest = [](float a, float b) {
+                    uint32_t t1, t2, t3;
+                    split3_bf16(a, b, t1, t2, t3);
+                    return t3;
+                };
+#pragma unroll
+                for (int pr = 0; pr < 2; ++pr) {
+                    u3[pr][0] = rest(u[2 * pr][0], u[2 * pr][1]);
+                    u3[pr][1] = rest(u[2 * pr][2], u[2 * pr][3]);
+                    u3[pr][2] = rest(u[2 * pr + 1][0], u[2 * pr + 1][1]);
+                    u3[pr][3] = rest(u[2 * pr + 1][2], u[2 * pr + 1][3]);
+                }
+            }
         }
         float add[2 * HS][4] = {};                       // the products of second terms, in accumulators of their own: half as long a chain
 #pragma unroll
@@ -544,6 +559,10 @@ __global__ void __launch_bounds__(PARTS * GROUPS * 32, 1) seq_chunk_walk_kernel(
                 mma_bf16_16816(add[2 * ks + 1], uh[pr], el.z, el.w);
                 mma_bf16_16816(add[2 * ks], ul[pr], el.x, el.y);
                 mma_bf16_16816(add[2 * ks + 1], ul[pr], el.z, el.w);
+                if (kThird) {
+                    mma_bf16_16816(add[2 * ks], u3[pr], eh.x, eh.y);
+                    mma_bf16_16816(add[2 * ks + 1], u3[pr], eh.z, eh.w);
+                }
             }
         // the outputs this warp finishes: tokens mt * 8 + 2c and + 1 of columns r0 and r1
         const int n = min(kChunk, len - blk * kChunk);
@@ -557,6 +576,7 @@ __global__ void __launch_bounds__(PARTS * GROUPS * 32, 1) seq_chunk_walk_kernel(
                 const uint4 bh = Mh[(6 + i + j) * 32], bl = Mh[(9 + i + j) * 32];
                 if (mt & 1) mma_split<true>(y, yl, ym, uh[j], ul[j], bh.z, bh.w, bl.z, bl.w);
                 else mma_split<true>(y, yl, ym, uh[j], ul[j], bh.x, bh.y, bl.x, bl.y);
+                if (kThird) mma_bf16_16816(ym, u3[j], mt & 1 ? bh.z : bh.x, mt & 1 ? bh.w : bh.y);
             }
             float4 z = exchange[(kTiles + mt) * 32];
 #pragma unroll

@@ -20,3 +20,19 @@ def test_portions_that_end_anywhere_in_a_block(kind, dk, dv):
     got = L.feed(stub, x, portions)[0]
     # two bf16 terms leave 2^-17 of an operand, three operands stand between the state and a result: as the test of whole recurrences
     assert _rel(got, _scan_oracle(kind, x, sizes, H, H, dk, dv, consts, rot)) < 5e-5
+
+
+@pytest.mark.parametrize("kind", ["head", "channel"])
+def test_one_key_channel(kind):
+    """Weak decays, steps near one and a key of one channel: every u of a block takes back what the ones before it have added, so its rounding stays. The mean error over 24 inputs was 1.95e-5 in
+    blocks of 16 tokens and 2.05e-5 in blocks of 32 with u as two bf16 terms; a third term of u takes it to 1.6e-5."""
+    H, dk, dv, n, errors = 2, 1, 16, 150, []
+    for seed in range(24):
+        rng = np.random.default_rng(1000 * seed + dk + dv)
+        consts = {"A_log": rng.uniform(-9, -6, size=H).astype(np.float32), "dt_bias": rng.uniform(-3, 3, size=H).astype(np.float32),
+                  "decay": np.ones(H, np.float32), "rate": np.ones(H, np.float32)}
+        stub, sizes, rot = _scan_stub(kind, H, H, dk, dv, consts, True)
+        x = rng.standard_normal((n, sum(sizes))).astype(np.float32)
+        x[:, sum(sizes[:3]):sum(sizes[:4])] += 3.0
+        errors.append(_rel(L.feed(stub, x, [n])[0], _scan_oracle(kind, x, sizes, H, H, dk, dv, consts, rot)))
+    assert float(np.sqrt(np.mean(np.square(errors)))) < 1.85e-5
