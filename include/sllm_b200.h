@@ -598,7 +598,7 @@ int sllm_seq_ring_store(const sllm_seq_batch* b, const float* x, int32_t ldx, in
  * o = S^T q, with q, k (of key head h / (heads / kv_heads)) divided by sqrt(sum(x^2) + unit_eps), q times qscale,
  * beta = sigmoid(beta_logit), g = exp(-exp(A_log[h]) * softplus(step_logit + dt_bias[h])). ring (or NULL): the last taps-1 rows of
  * conv_x [T][channels] of every portion are stored there for the convolution of the next step. chunk_ws (NULL = token by token):
- * sllm_seq_chunk_ws_bytes of scratch, 16-byte aligned; with it the portions are walked in blocks of 32 tokens on the tensor cores (dk <= 128;
+ * sllm_seq_chunk_ws_bytes of scratch, 16-byte aligned; with it the portions are walked in blocks of 32 or 16 tokens on the tensor cores (dk <= 128;
  * state and sums fp32, operands as two bf16 terms each). */
 int sllm_seq_delta_rule(const sllm_seq_batch* b, const float* q, int32_t ldq, const float* k, int32_t ldk, const float* v, int32_t ldv,
                         const float* beta_logit, int32_t ldb, const float* step_logit, int32_t lda, const float* A_log, const float* dt_bias,

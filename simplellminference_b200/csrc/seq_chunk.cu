@@ -14,10 +14,10 @@
 // head multiply finished sums and whole rows (2048 tokens of 16 heads: 58 us with the decays inside the sums and blocks of 16 in two threads per entry, 42 like this).
 // (2) seq_chunk_walk_kernel, CTA = (portion, head, 16 or 32 value columns), two or four warps = 16 value columns, a share of the key channels each: their part of
 // S^T [16][dk] stays in the accumulators (fp32) from the portion's first token to its last. An accumulator fragment is register for register
-// an A fragment of the next product, so state and u never leave the registers; all products take both operands as two bf16 terms (three products, fp32 accumulation), which keeps
-// the recurrence at fp32 working accuracy (against float64 in the mean over 36 shapes and decays 0.85 of the error of blocks of 16 without the products of second terms). The blocks' records arrive by one bulk copy each, three stages. Bound: latency of a block's chain (products with the state, their exchange
-// between the warps, u, the state); a block of 32 takes hardly longer than one of 16 did (2048 tokens of 16 heads: 1.05 us for 16, 1.6 for 32, a walk 137 -> 103 us).
-#include "seq_attn.cuh"
+// an A fragment of the next product, so state and u never leave the registers; all products take both operands as two bf16 terms (three products, four where u is an operand, fp32 accumulation), which keeps
+// the recurrence at fp32 working accuracy (against float64 in the mean over 120 shapes and decays 0.78 of the error of blocks of 16 without the products of second terms, in none more). The blocks' records arrive by one bulk copy each, three stages. Bound: latency of a block's chain (products with the state, their exchange
+// between the warps, u, the state); a block of 32 takes hardly longer than one of 16 (2048 tokens of 16 heads: 1.05 us for 16, 1.6 for 32, a walk 137 | 103 us). Where blocks of 16 are
+// ahead all the same, the kernels of seq_chunk16.cu run (chunk_in_16).
 #include "seq_chunk.cuh"
 #include "mega_common.cuh"
 
@@ -25,7 +25,6 @@ namespace sllm {
 
 constexpr int kPrepThreads = 288;    // eight threads per 4 x 4 entries of a triangle of 32 x 32
 constexpr int kWalkStages = 3;
-constexpr float kLog2e = 1.4426950408889634f;
 
 struct ChunkPlace { int seg, start, n, id; };      // segment, first token in the batch, tokens, number of the block in segment order
 __device__ __forceinline__ ChunkPlace chunk_place(const sllm_seq_batch& b, int tile) {
@@ -38,14 +37,6 @@ __device__ __forceinline__ ChunkPlace chunk_place(const sllm_seq_batch& b, int t
     return c;
 }
 
-// eight values -> 16 bytes of hi terms and 16 bytes of lo terms
-__device__ __forceinline__ void chunk_put(uint8_t* hi, uint8_t* lo, int at, const float (&v)[8]) {
-    uint32_t h[4], l[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) split_bf16(v[2 * i], v[2 * i + 1], &h[i], &l[i]);
-    reinterpret_cast<uint4*>(hi)[at] = make_uint4(h[0], h[1], h[2], h[3]);
-    reinterpret_cast<uint4*>(lo)[at] = make_uint4(l[0], l[1], l[2], l[3]);
-}
 __device__ __forceinline__ float4 chunk_scale(const float4& a, const float4& e) { return make_float4(a.x * e.x, a.y * e.y, a.z * e.z, a.w * e.w); }
 __device__ __forceinline__ float4 chunk_decay(const float4& a, const float4& b) { return make_float4(exp2f(a.x - b.x), exp2f(a.y - b.y), exp2f(a.z - b.z), exp2f(a.w - b.w)); }
 __device__ __forceinline__ float chunk_dot(const float4& a, const float4& b, float c) { return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, c)))); }
@@ -348,16 +339,6 @@ __global__ void __launch_bounds__(kPrepThreads, kMode == kDecayChannel ? 2 : 3) 
     }
 }
 
-// Products of two-term operands: (ah + al) (bh + bl), each term's into an accumulator of its own as far as there are three (no product waits for another). The product of the second
-// terms, as large as what two terms leave of an operand, is kept where u is an operand (kAll), and left out of the products with the old state.
-template <bool kAll>
-__device__ __forceinline__ void mma_split(float (&d)[4], float (&dl)[4], float (&dm)[4], const uint32_t (&ah)[4], const uint32_t (&al)[4], uint32_t h0, uint32_t h1, uint32_t l0, uint32_t l1) {
-    mma_bf16_16816(d, ah, h0, h1);
-    mma_bf16_16816(dl, al, h0, h1);
-    mma_bf16_16816(dm, ah, l0, l1);
-    if (kAll) mma_bf16_16816(dl, al, l0, l1);
-}
-
 // KS: k-steps of 16 key channels. PARTS warps share 16 value columns, each owning KS / PARTS of the k-steps; they add their parts of the
 // products with the old state through shared memory and finish 32 / PARTS tokens each. GROUPS: how many times 16 columns a CTA takes.
 template <int KS, int PARTS, int GROUPS, bool kDelta>
@@ -649,9 +630,27 @@ static int launch_chunk_as(ChunkArgs p, cudaStream_t st) {
     return narrow ? launch_walk<8, 4, 1, kDelta>(p, vec, st) : launch_walk<8, 4, 2, kDelta>(p, vec, st);
 }
 
+// Whether a step goes in blocks of 16 tokens. The lengths of the portions are on the device: their mean stands for them. Measured, us, both kernels, 16 | 32 tokens a block.
+// - Many CTAs (a portion, head and 32 value columns each): those of blocks of 32 fill an SM alone (128 key channels) or in pairs. Heads of 128, 16 of them: 8 portions of 64, 128 and 300 43 | 41, 78 | 73,
+//   166 | 160, 32 portions of 16, 40 and 100 53 | 79, 111 | 138, 232 | 250; 8 heads of 64: 8 portions of 100 23 | 21, 32 portions of 40 and 100 33 | 39, 63 | 69; 8 heads of 32: 32 of 40 20 | 21.
+// - Portions that end in the first half of a block: one of 33 tokens 14 | 15, of 64 15 | 15, of 80 16 | 17, of 128 20 | 19, of 300 37 | 31; 8 of 40 37 | 40, of 50 42 | 40, of 70 52 | 54.
+// - A constant decay needs no triangle inverted, so the larger blocks' matrices weigh more (heads of 128): one of 64 12 | 14, of 128 15 | 16, of 160 18 | 17, of 2048 142 | 112; two of 64 14 | 16, of 150 22 | 22; 8
+//   of 100 and 300 47 | 54, 113 | 120.
+// - A decay per channel takes an exponential per channel and pair of rows: 16 heads of 128, one of 300 38 | 41, of 600 65 | 70, of 1000 105 | 100, two of 300 55 | 65, 8 of 100 71 | 94; 8 heads of 64, one of 200 22 | 23, of 300
+//   29 | 27, of 1000 74 | 59; 8 heads of 32, one of 200 18 | 19, of 400 28 | 26. What a longer chain costs (0.26 us a block of 16) stands against the work per block and head.
+static bool chunk_in_16(const ChunkArgs& p) {
+    const int dkp = chunk_key(p.dk);
+    const long long T = p.b.T, nseg = p.b.nseg, ctas = nseg * p.heads * ((p.dv + 31) / 32);
+    if (p.delta && p.channel) return nseg > 1 || T * (44 - (dkp > 64 ? 2 : 1) * p.heads) <= 11000;
+    if (!p.delta) return ctas > sm_count() || T < 140 * nseg;
+    if (ctas > (dkp > 96 ? 4LL : dkp > 64 ? 3LL : dkp > 32 ? 2LL : 1LL) * sm_count()) return true;
+    return T <= 90 * nseg && ((T + 16 * nseg - 1) / (16 * nseg)) % 2 == 1;
+}
+
 int launch_chunk_scan(const ChunkArgs& p, cudaStream_t st) {
     SLLM_REQUIRE(p.dk <= kChunkMaxKey && p.ws && ((uintptr_t)p.ws % 16) == 0 && p.b.seg_tile0 && p.b.qt_seg && p.b.qt_off && p.b.n_qtiles > 0, SLLM_EINVAL,
                  "chunk scan: heads of %d key channels, or an incomplete batch description", p.dk);
+    if (chunk_in_16(p)) return launch_chunk16_scan(p, st);
     return p.delta ? launch_chunk_as<true>(p, st) : launch_chunk_as<false>(p, st);
 }
 

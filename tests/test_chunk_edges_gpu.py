@@ -1,4 +1,4 @@
-"""The recurrences in blocks of 32 tokens at the edges of a block and of its halves, whose sums and triangles are made apart: portions that end in the first half, at the middle, behind it
+"""The recurrences in blocks of 32 and 16 tokens at the edges of a block and of its halves, whose sums and triangles are made apart: portions that end in the first half, at the middle, behind it
 and at the end, every width of key head that has a body of its own, against the restatement."""
 import numpy as np
 import pytest
@@ -9,9 +9,11 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("kind", ["head", "channel", "lightning"])
 @pytest.mark.parametrize("dk,dv", [(32, 16), (64, 64), (96, 33), (128, 128)])
-def test_portions_that_end_anywhere_in_a_block(kind, dk, dv):
+@pytest.mark.parametrize("portions", [[16, 17, 31, 32, 33, 47, 48, 49, 64, 65], [280, 303, 320]], ids=["short", "long"])
+def test_portions_that_end_anywhere_in_a_block(kind, dk, dv, portions):
+    """Short ones take either size of blocks, long ones (a decay per channel above all) the larger one."""
     rng = np.random.default_rng(dk + dv)
-    H, portions = 2, [16, 17, 31, 32, 33, 47, 48, 49, 64, 65]
+    H = 2
     decay = np.linspace(0.9, 0.99, H).astype(np.float32)
     consts = {"A_log": rng.uniform(-3, 1, size=H).astype(np.float32), "decay": decay, "decay64": decay.astype(np.float64), "rate": (-np.log(decay.astype(np.float64))).astype(np.float32),
               "dt_bias": rng.uniform(-3, 3, size=H * dk if kind == "channel" else H).astype(np.float32)}
@@ -36,3 +38,27 @@ def test_one_key_channel(kind):
         x[:, sum(sizes[:3]):sum(sizes[:4])] += 3.0
         errors.append(_rel(L.feed(stub, x, [n])[0], _scan_oracle(kind, x, sizes, H, H, dk, dv, consts, rot)))
     assert float(np.sqrt(np.mean(np.square(errors)))) < 1.85e-5
+
+
+@pytest.mark.parametrize("kind", ["head", "channel", "lightning"])
+@pytest.mark.parametrize("dk,dv", [(40, 24), (128, 64)])
+@pytest.mark.parametrize("portions", [[40, 16, 17, 1, 100], [130, 150], [20] * 40], ids=["mixed", "two", "many"])
+def test_portions_of_one_step(kind, dk, dv, portions):
+    """Several requests in one step, whose blocks, of either size, find their own state, rows and records."""
+    import torch
+
+    from simplellminference_b200.seqengine import SequenceEngine
+    rng = np.random.default_rng(sum(portions) + dk)
+    H, T = 4, sum(portions)
+    decay = np.linspace(0.9, 0.99, H).astype(np.float32)
+    consts = {"A_log": rng.uniform(-3, 1, size=H).astype(np.float32), "decay": decay, "decay64": decay.astype(np.float64), "rate": (-np.log(decay.astype(np.float64))).astype(np.float32),
+              "dt_bias": rng.uniform(-3, 3, size=H * dk if kind == "channel" else H).astype(np.float32)}
+    stub, sizes, rot = _scan_stub(kind, H, H, dk, dv, consts, True)
+    x = rng.standard_normal((T, sum(sizes))).astype(np.float32)
+    eng = SequenceEngine(stub, max_tokens=4096, max_seqs=len(portions), page_len=32, graphs=False)
+    stub.h = torch.tensor(x, device="cuda").view(-1)
+    eng.run([(eng.admit(), np.zeros(n, np.int32), []) for n in portions])
+    got, at = stub.outs[0].cpu().numpy(), 0
+    for n in portions:
+        assert _rel(got[at:at + n], _scan_oracle(kind, x[at:at + n], sizes, H, H, dk, dv, consts, rot)) < 5e-5, n
+        at += n
