@@ -376,7 +376,9 @@ static __device__ __noinline__ void mega_logits_out(const float* from, float* to
 // End of the classifier phase: every CTA leaves its best logit, the CTA that comes last picks the arg max and advances the step state. True in the one thread that has
 // done so (it stores the counters that its kernel keeps). All threads of the last CTA read the candidates: by one thread, a chain of 148 reads of L2, that end took
 // several us. A call that wants its logits on the host (p.call.logits, pinned) gets this CTA's rows [r0, r1) from here: read back from the device's copy, 16 bytes a thread,
-// so that a warp stores 512 bytes in a row over PCIe, and behind the ticket, so that no fence waits for them to arrive.
+// so that a warp stores 512 bytes in a row over PCIe, and behind the ticket, so that no fence waits for them to arrive. kLogits = false: no call asks for them. (Over int8 weights, whose
+// kernels have no register to spare, the call that is not taken cost a step of a model 2048 wide 226.5 us instead of 223.)
+template <bool kLogits>
 __device__ __forceinline__ bool mega_finish(const MegaParams& p, float v, int i, float* red, int* s_last, int cta, int ncta, int r0, int r1) {
     cta_better(v, i, red);
     if (threadIdx.x == 0) {
@@ -387,7 +389,7 @@ __device__ __forceinline__ bool mega_finish(const MegaParams& p, float v, int i,
         __threadfence();
     }
     __syncthreads();
-    if (p.call.logits) mega_logits_out(p.logits, p.call.logits, r0, r1);
+    if (kLogits && p.call.logits) mega_logits_out(p.logits, p.call.logits, r0, r1);
     if (!*s_last) return false;
     v = -INFINITY;
     i = 0x7fffffff;

@@ -50,7 +50,8 @@ static_assert(mega_smem_layout(128, 8, 2).total + kMegaStatic <= 227 * 1024, "th
 
 // FUSE (experimental, SLLM_ENGINE_MEGA_FUSE_DOWN): the down projection runs inside the gate_up phase's CTA as a K-split over the
 // values that CTA produced (megakernel.cuh "PH_DOWN_T"): four grid barriers per layer instead of five, no staging of swi.
-template <int WD, int KVD, int G, bool FUSE>
+// OUT: a call may want its logits in host memory (mega_finish).
+template <int WD, int KVD, int G, bool FUSE, bool OUT>
 __global__ void __launch_bounds__(kMegaThreads, 1) mega_step_kernel(const MegaParams p) {
     constexpr int E = WInfo<WD>::E;                 // weights per 16-byte chunk
     constexpr int CPL = (WD == SLLM_INT8) ? 2 : kCplMax;   // max chunks per lane per row slice (x of a lane: CPL * E = 32 registers)
@@ -485,7 +486,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega_step_kernel(const MegaPa
         }
 
         if (ph.kind == PH_CLS) {   // CTA best -> global; the last CTA picks the arg max and advances the step state
-            if (mega_finish(p, best_v, best_i, part, &s_last, cta, ncta, 2 * u0, min(ph.nrows, 2 * (u0 + n)))) {
+            if (mega_finish<OUT>(p, best_v, best_i, part, &s_last, cta, ncta, 2 * u0, min(ph.nrows, 2 * (u0 + n)))) {
                 p.st->pad[0] = (int32_t)(bar_base + bar_idx * (unsigned)ncta);   // barrier epoch for the next launch
             }
             break;
@@ -883,11 +884,12 @@ int mega_repack_down_t(const void* src, void* dst, int d, int I_loc, int w_dtype
     return SLLM_OK;
 }
 
-template <int WD, int KVD, int G, bool FUSE = false>
+template <int WD, int KVD, int G, bool FUSE = false, bool OUT = true>
 static int mega_launch_t(const MegaParams& p, int grid, size_t smem, cudaStream_t st) {
+    if (WD == SLLM_INT8 && OUT && !p.call.logits) return mega_launch_t<WD, KVD, G, FUSE, WD != SLLM_INT8>(p, grid, smem, st);
     static size_t configured = 0;
     if (smem > configured) {
-        SLLM_CUDA(cudaFuncSetAttribute(mega_step_kernel<WD, KVD, G, FUSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        SLLM_CUDA(cudaFuncSetAttribute(mega_step_kernel<WD, KVD, G, FUSE, OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         configured = smem;
     }
     cudaLaunchConfig_t cfg{};
@@ -900,7 +902,7 @@ static int mega_launch_t(const MegaParams& p, int grid, size_t smem, cudaStream_
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    SLLM_CUDA(cudaLaunchKernelEx(&cfg, mega_step_kernel<WD, KVD, G, FUSE>, p));
+    SLLM_CUDA(cudaLaunchKernelEx(&cfg, mega_step_kernel<WD, KVD, G, FUSE, OUT>, p));
     g_launches++;
     return SLLM_OK;
 }

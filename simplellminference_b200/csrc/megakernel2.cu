@@ -686,7 +686,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) mega2_step_kernel(const Mega2
         }
 
         if (ph.kind == PH_CLS) {
-            if (mega_finish(p, best_v, best_i, part, &s_last, cta, ncta, 2 * u0, min(ph.nrows, 2 * (u0 + n)))) {
+            if (mega_finish<true>(p, best_v, best_i, part, &s_last, cta, ncta, 2 * u0, min(ph.nrows, 2 * (u0 + n)))) {
                 p.st->pad[0] = (int32_t)(bar_base + bar_idx * (unsigned)ncta);   // barrier epoch for the next launch
                 p.st->pad[2] = (int32_t)(epoch + 1u);
             }
