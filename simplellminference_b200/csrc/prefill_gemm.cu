@@ -35,8 +35,7 @@ constexpr int kPfBM = 128, kPfBK = 64, kPfThreads = 192;
 constexpr uint32_t kPfABytes = kPfBM * kPfBK * 2;
 // PAIR = true: two CTAs of a cluster (the two SMs of a TPC) work on ONE 256 x BN tile with tcgen05.mma.cta_group::2 — each
 // CTA stages its own 128 rows of A and its own BN/2 rows of W, so shared-memory traffic (TMA writes + tensor-core reads) and
-// L2->SM traffic per flop are 2/3 of the single-CTA 128 x BN tile's (measured bound of the single-CTA kernel: 55 % tensor
-// pipe inside a tile, profiles/r01_prefill_ncu_raw.md).
+// L2->SM traffic per flop are 2/3 of the single-CTA 128 x BN tile's.
 // The N extent of a tile (BN) is a RUN-TIME multiple of 32 up to 256 (one tcgen05.mma takes any N that is a multiple of 16):
 // the host picks the BN that fills the last wave best, e.g. 192 instead of 256 for a 512 x 12288 output on 74 SM pairs.
 constexpr int kPfMaxStages = 12;
@@ -64,12 +63,12 @@ struct PfDev {           // kernel-side view of PfGemmArgs
     long long wait_clocks;     // and after how long it is
 };
 
-// Bounded wait on a barrier: false once `limit` clocks have passed (0: without a poll) or another thread of the CTA has given up. The kernel then tears down without its result and says
+// Bounded wait on a barrier: false once `limit` clocks have passed or another thread of the CTA has given up. The kernel then tears down without its result and says
 // so in the library's status word. (By the clock and not by polls: a poll may sleep.)
 __device__ __forceinline__ bool pf_wait(uint64_t* bar, uint32_t parity, volatile int* gave_up, long long limit) {
     uint32_t done;
     long long since = 0;
-    while (limit) {
+    while (true) {
         asm volatile(
             "{\n.reg .pred p;\n"
             "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
@@ -383,6 +382,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
         }
     };
     Walk walk(p);
+    const bool gone = p.wait_clocks == 0;      // no wait is allowed at all: every role gives up in front of its first one (asked once and not by every wait: a k-block's 290 clocks)
+    if (gone) *gave_up = 1;
 
     // One elected lane of either issuing warp runs its loop, with nothing in it that need not be: with an integer division and addresses made anew for every k-block either warp
     // took 560 clocks for one, whatever its width (a 256 x 256 tile's products need 512, a 256 x 128 tile's 256); like this some 290. The lane waits by itself: a lane that
@@ -392,7 +393,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
             const uint32_t full_at = PAIR ? mapa_u32(full, 0) : s_addr(full), a_at = s_addr(sA), b_at = s_addr(sB);   // pair: both CTAs' bytes are counted on the LEADER's barriers
             int stage = 0;
             uint32_t phase = 0;
-            bool ok = true;
+            bool ok = !gone;
             for (int unit = worker; ok && walk.reach(unit); unit += nworkers) {
                 const int tile = (unit - walk.base) / p.ksplit, part = (unit - walk.base) - tile * p.ksplit;
                 const int kb0 = (p.nkb * part) / p.ksplit, kb1 = (p.nkb * (part + 1)) / p.ksplit;
@@ -421,7 +422,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
             const uint64_t a_desc = umma_desc_sw128(sA), b_desc = umma_desc_sw128(sB);
             int stage = 0, acc = 0;
             uint32_t phase = 0, acc_phase = 0;
-            bool ok = true;
+            bool ok = !gone;
             for (int unit = worker; ok && walk.reach(unit); unit += nworkers) {
                 const int part = (unit - walk.base) % p.ksplit;
                 const int n_kb = (p.nkb * (part + 1)) / p.ksplit - (p.nkb * part) / p.ksplit;
@@ -454,7 +455,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
         int acc = 0;
         uint32_t acc_phase = 0;
         const uint32_t tempty_leader[2] = {PAIR ? mapa_u32(tempty, 0) : 0u, PAIR ? mapa_u32(tempty + 1, 0) : 0u};
-        for (int unit = worker; walk.reach(unit); unit += nworkers) {
+        for (int unit = worker; !gone && walk.reach(unit); unit += nworkers) {
             const int tile = (unit - walk.base) / p.ksplit;
             const int m_tile = tile % walk.m_tiles, n_tile = tile / walk.m_tiles;
             const int t0 = m_tile * BM + (int)rank * kPfBM + quad * 32, t = t0 + lane;
@@ -585,9 +586,9 @@ static PfPlan pf_plan(int T, int N, int K, int tiled, int epilogue, int bn_force
         pl.kb_per_seg = (K + kPfBK - 1) / kPfBK;
         pl.nkb = pl.kb_per_seg;
     }
-    // N extent of a tile (a multiple of 32 up to 256) and, for the residual epilogue, a split of K: a work unit costs about
-    // k-blocks x operand bytes per k-block (the kernel is bound by what an SM can ingest) plus the epilogue of its tile, and the
-    // GEMM takes ceil(units / workers) waves of it. Pick the cheapest combination.
+    // N extent of a tile (a multiple of 32 up to 256) and, for the residual epilogue, a split of K: a work unit is reckoned as k-blocks x operand rows per k-block plus the
+    // epilogue of its tile, and the GEMM takes ceil(units / workers) waves of it; the cheapest combination is taken. The operand rows stand in for what a k-block takes, which is max(2 BN,
+    // 290) clocks (measured, two SMs a tile): by those the choice is up to 6 % off, e.g. for 512 x 22016 x 4096 224 columns in three waves (86 016 clocks) where 160 in four take 81 920.
     int bn = bn_forced ? bn_forced : g_tune_pf_bn;
     int ksplit = 1;
     if (bn < 32 || bn > 256 || bn % 32) {
