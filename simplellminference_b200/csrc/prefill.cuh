@@ -53,8 +53,8 @@ int pf_gemm(PfCache* cache, const PfGemmArgs& a, cudaStream_t st);
 // causal attention of T queries at positions pos0.. over cache rows [0, pos0+T): q bf16 [T][q_loc] -> out bf16 [T][q_loc]
 int pf_attention(const uint16_t* q, const void* k_cache, const void* v_cache, int kv_dtype, uint16_t* out, int T, int pos0, int S, int hd,
                  int heads, int kv_heads, cudaStream_t st, float* scratch = nullptr);
-// fp32 values of scratch with which such a call divides its work evenly; 0: it has no use for any
-size_t pf_attention_scratch(int kv_dtype, int T, int pos0, int hd, int heads, int kv_heads);
+// fp32 values of scratch with which such a call over a bf16 cache (or one rounded to bf16 in front) divides its key tiles evenly; 0: it has no use for any
+size_t pf_attention_shares(int T, int pos0, int hd, int heads, int kv_heads);
 // the same on tcgen05: bf16 cache, head_dim 64 or 128, 16-byte aligned pointers (prefill_attn_tc.cu)
 int pf_attention_tc(const uint16_t* q, const void* k_cache, const void* v_cache, uint16_t* out, int T, int pos0, int S, int hd, int heads, int kv_heads,
                     float* scratch, cudaStream_t st);

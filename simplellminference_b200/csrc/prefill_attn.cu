@@ -232,9 +232,8 @@ __global__ void __launch_bounds__(256) pf_rows16_kernel(const float* __restrict_
 // start 45 | 16, 256 behind 5000, 8 heads 356 | 35, 128 behind 100 19.2 | 10.0, 64 from the start 7.3 | 6.4; heads of 64: 2048 queries, 32 heads 202 | 55, 1000 behind 5000, 8 heads 215 | 39. With 64
 // keys and heads of 64 the kernel is done in 4.8 and the copy alone takes 2.5; the bf16 kernel saves that from some 128 keys on.
 static bool pf_rows16_pay(int T, int pos0, int hd) { return hd == 128 || (hd == 64 && pos0 + T > 128); }
-size_t pf_attention_scratch(int kv_dtype, int T, int pos0, int hd, int heads, int kv_heads) {
-    const bool tc = kv_dtype == SLLM_BF16 && (hd == 64 || pf_attention_fills(T, pos0 + T, hd, heads));
-    return tc ? pf_attention_tc_scratch(T, pos0, hd, heads, kv_heads) : 0;
+size_t pf_attention_shares(int T, int pos0, int hd, int heads, int kv_heads) {
+    return hd == 64 || pf_attention_fills(T, pos0 + T, hd, heads) ? pf_attention_tc_scratch(T, pos0, hd, heads, kv_heads) : 0;
 }
 
 int pf_attention(const uint16_t* q, const void* kc, const void* vc, int kv_dtype, uint16_t* out, int T, int pos0, int S, int hd, int heads,
@@ -336,7 +335,7 @@ int pf_rmsnorm(float* x, const float* add, const float* w, uint16_t* y, int T, i
 
 extern "C" int64_t sllm_prefill_attention_scratch(int32_t kv_dtype, int32_t T, int32_t pos0, int32_t head_dim, int32_t heads, int32_t kv_heads) {
     if (T <= 0 || pos0 < 0 || heads <= 0 || kv_heads <= 0 || heads % kv_heads) return 0;
-    const int64_t shares = 4 * (int64_t)sllm::pf_attention_scratch(SLLM_BF16, T, pos0, head_dim, heads, kv_heads);
+    const int64_t shares = 4 * (int64_t)sllm::pf_attention_shares(T, pos0, head_dim, heads, kv_heads);
     if (kv_dtype == SLLM_BF16) return shares;
     return kv_dtype == SLLM_F32 && sllm::pf_rows16_pay(T, pos0, head_dim) ? shares + 4 * (int64_t)kv_heads * (pos0 + T) * head_dim : 0;
 }
