@@ -109,15 +109,21 @@ static int launch_plain(const PlainPolicy& p, cudaStream_t st) {
     }
     PlainPolicyT<WD> pt;
     static_cast<PlainPolicy&>(pt) = p;
-    // As many warps a pair of rows as still fit two CTAs per SM (or one) at once and leave each lane a load of 16 bytes. Measured, us a call one behind the other, a warp per pair | like this: fp32 2048 x 5632
-    // 13.9 | 11.8, 1500 x 5632 12.2 | 9.9, 2300 x 11008 22.1 | 20.0; bf16 1500 x 5632 9.7 | 8.2, 2300 x 11008 15.9 | 13.9; int8 1500 x 5632 9.7 | 7.8, 2300 x 11008 12.7 | 12.4; the kernel alone,
-    // int8 256 x 4096 5.0 | 3.9, 2048 x 5632 7.0 | 6.5. One warp a pair from 2369 rows on: 4096 x 4096 the same.
+    // More warps a pair of rows while all CTAs are resident at once and a warp keeps enough columns: the sums' way through shared memory costs 0.3 us, and a second CTA an SM, which stages the vector again,
+    // another 0.2 (int8 0.5). Measured in a captured graph, us, a warp per pair | 2, 4 and 8: fp32 256 x 512 2.3 | 2.5 2.5 2.6, 256 x 1024 2.6 | 2.6 2.5 2.6, 700 x 1024 2.7 | 2.6 2.9, 2048 x 1024 3.7 | 3.6, 500 x 4096 7.2 | 4.9 3.7 3.7,
+    // 2048 x 5632 12.2 | 10.2; bf16 500 x 1024 2.5 | 2.5 2.6 2.9, 2048 x 1024 3.0 | 3.1, 2048 x 1536 3.7 | 3.5, 700 x 2048 3.2 | 2.9 3.1, 256 x 4096 4.2 | 3.0 2.8 2.8, 2048 x 5632 8.5 | 7.1; int8 256 x 1024 2.8 | 2.9 3.0 3.0, 256 x 2048 3.5 | 3.2
+    // 3.1 3.2, 700 x 2048 3.5 | 3.2 3.7, 1200 x 2048 3.5 | 3.9, 2048 x 4096 4.9 | 5.2, 500 x 5632 6.2 | 4.4 3.9 4.6, 2048 x 5632 6.9 | 6.5 (a call of it 8.20 | 8.16: the launch and the host). One warp a pair from 2369 rows on.
     // A vector that takes more than half of an SM's shared memory (28 700 columns) leaves it one CTA, and one that fills it no room for the partial sums beside it.
     const size_t split_smem = smem + kGemvWarps * sizeof(float2), sm_smem = (size_t)smem_optin_bytes() + kCtaSharedReserve;
     const int resident = 2 * (split_smem + kCtaSharedReserve) <= sm_smem ? 2 : split_smem + kCtaSharedReserve <= sm_smem ? 1 : 0;
     const int units = (p.nrows + 1) / 2, chunks = p.ncols / WInfo<WD>::E, warps = resident * kGemvWarps * sm_count();
+    constexpr bool kInt8 = WD == SLLM_INT8;
     int parts = 1;
-    while (parts < kGemvWarps && 2LL * parts * units <= warps && chunks / (2 * parts) >= 32) parts *= 2;
+    while (parts < kGemvWarps && 2LL * parts * units <= warps && chunks >= (kInt8 ? 128 : 192)) {
+        const bool second = 2LL * parts * units > kGemvWarps * sm_count();
+        if (chunks / (2 * parts) < (second ? (kInt8 ? 160 : 96) : (kInt8 ? 32 : 64))) break;
+        parts *= 2;
+    }
     if (parts > 1 && g_tune_ctas_per_sm == 0) {
         static size_t split_configured = 0;
         if (split_smem > 48 * 1024 && smem > split_configured) {
