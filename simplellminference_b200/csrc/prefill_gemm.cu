@@ -65,6 +65,14 @@ struct PfDev {           // kernel-side view of PfGemmArgs
 
 // Bounded wait on a barrier: false once `limit` clocks have passed or another thread of the CTA has given up. The kernel then tears down without its result and says
 // so in the library's status word. (By the clock and not by polls: a poll may sleep.)
+// Of a pair, the other CTA is told at once: what is on its way for one may reach into the other's memory, so both take their time before they leave.
+__device__ __forceinline__ uint32_t cluster_ctarank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ uint32_t mapa_u32(const void* local, uint32_t cta) {   // shared::cluster address of `local` in CTA `cta`
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(s_addr(local)), "r"(cta));
+    return r;
+}
+template <bool PAIR>
 __device__ __forceinline__ bool pf_wait(uint64_t* bar, uint32_t parity, volatile int* gave_up, long long limit) {
     uint32_t done;
     long long since = 0;
@@ -80,6 +88,7 @@ __device__ __forceinline__ bool pf_wait(uint64_t* bar, uint32_t parity, volatile
         if (*gave_up || now - since > limit) break;
     }
     *gave_up = 1;
+    if (PAIR) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(mapa_u32(const_cast<const int*>(gave_up), cluster_ctarank() ^ 1)), "r"(1) : "memory");
     return false;
 }
 
@@ -102,12 +111,6 @@ __device__ __forceinline__ void pf_load_4d(uint32_t dst, const CUtensorMap* tm, 
     else
         asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
                      ::"r"(dst), "l"(tm), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
-}
-__device__ __forceinline__ uint32_t cluster_ctarank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
-__device__ __forceinline__ uint32_t mapa_u32(const void* local, uint32_t cta) {   // shared::cluster address of `local` in CTA `cta`
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(s_addr(local)), "r"(cta));
-    return r;
 }
 __device__ __forceinline__ void mb_arrive_cluster(uint32_t bar_cluster_addr) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
@@ -351,7 +354,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
         tma_prefetch_desc(&tmB);
         for (int s = 0; s < ST; ++s) { mb_init(full + s, 1); mb_init(empty + s, 1); }
         for (int a = 0; a < 2; ++a) { mb_init(tfull + a, 1); mb_init(tempty + a, PAIR ? 8 : 4); }
-        *gave_up = 0;
+        *gave_up = p.wait_clocks == 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) { if (PAIR) tc_alloc_pair(tmem_slot, kPfTmemCols); else tc_alloc(tmem_slot, kPfTmemCols); }
@@ -383,7 +386,6 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
     };
     Walk walk(p);
     const bool gone = p.wait_clocks == 0;      // no wait is allowed at all: every role gives up in front of its first one (asked once and not by every wait: a k-block's 290 clocks)
-    if (gone) *gave_up = 1;
 
     // One elected lane of either issuing warp runs its loop, with nothing in it that need not be: with an integer division and addresses made anew for every k-block either warp
     // took 560 clocks for one, whatever its width (a 256 x 256 tile's products need 512, a 256 x 128 tile's 256); like this some 290. The lane waits by itself: a lane that
@@ -403,7 +405,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
                 const int w_row = p.tiled ? 0 : n0, w_tile = p.tiled ? n0 / p.R : 0;
                 int ks = kb0 / p.kb_per_seg, kk = kb0 - ks * p.kb_per_seg;
                 for (int kb = kb0; kb < kb1; ++kb) {
-                    ok = pf_wait(empty + stage, phase ^ 1, gave_up, p.wait_clocks);
+                    ok = pf_wait<PAIR>(empty + stage, phase ^ 1, gave_up, p.wait_clocks);
                     if (!ok) break;
                     const uint32_t bar = full_at + 8 * stage;
                     if (!PAIR) mb_expect(full + stage, tx_bytes);
@@ -426,12 +428,12 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
             for (int unit = worker; ok && walk.reach(unit); unit += nworkers) {
                 const int part = (unit - walk.base) % p.ksplit;
                 const int n_kb = (p.nkb * (part + 1)) / p.ksplit - (p.nkb * part) / p.ksplit;
-                ok = pf_wait(tempty + acc, acc_phase ^ 1, gave_up, p.wait_clocks);   // the epilogue has drained this accumulator
+                ok = pf_wait<PAIR>(tempty + acc, acc_phase ^ 1, gave_up, p.wait_clocks);   // the epilogue has drained this accumulator
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + (uint32_t)(acc * 256);
                 for (int kb = 0; kb < n_kb; ++kb) {
-                    ok = pf_wait(full + stage, phase, gave_up, p.wait_clocks);
+                    ok = pf_wait<PAIR>(full + stage, phase, gave_up, p.wait_clocks);
                     if (!ok) break;
                     tc_fence_after();
                     const uint64_t ad = a_desc + (uint64_t)((uint32_t)stage * (kPfABytes >> 4)), bd = b_desc + (uint64_t)((uint32_t)stage * (b_bytes >> 4));
@@ -461,7 +463,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
             const int t0 = m_tile * BM + (int)rank * kPfBM + quad * 32, t = t0 + lane;
             const bool bias = p.bias && (unit - walk.base) % p.ksplit == 0;   // the bias rides on the first share of K
             // the warp goes on as one: what follows are instructions of all its lanes
-            if (!__all_sync(0xffffffffu, pf_wait(tfull + acc, acc_phase, gave_up, p.wait_clocks))) break;
+            if (!__all_sync(0xffffffffu, pf_wait<PAIR>(tfull + acc, acc_phase, gave_up, p.wait_clocks))) break;
             tc_fence_after();
             const uint32_t src = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * 256);
 #pragma unroll 1
@@ -488,12 +490,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
         __syncwarp();
     }
     tc_fence_before();
-    if (PAIR) {       // what is on its way for a CTA of a pair that gave up may reach into the other one's memory: both take their time then
-        if (*gave_up) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(mapa_u32(const_cast<const int*>(gave_up), rank ^ 1)), "r"(1) : "memory");
-        cluster_sync_all();      // nobody leaves while the peer may still signal its barriers / read its operands
-    } else {
-        __syncthreads();
-    }
+    if (PAIR) cluster_sync_all(); else __syncthreads();   // pair: nobody leaves while the peer may still signal its barriers / read its operands
     if (__syncthreads_or(*gave_up)) tc_gave_up(p.status);
     if (warp == 1) {
         tc_fence_after();
