@@ -341,7 +341,9 @@ __global__ void __launch_bounds__(kTaThreads, 1) pf_attn_tc_kernel(const __grid_
                 mb_arrive(factors + j);
                 l *= f;
                 ref = nr;
-                const uint64_t neg2 = tc_two(__float_as_uint(-ref), __float_as_uint(-ref));
+                // where every score so far is -inf, -inf - ref were no number: relative to 0 their weights are 0 (a share may start with such keys, in the middle of a row that sees others)
+                const uint32_t neg = __float_as_uint(ref == -INFINITY ? 0.0f : -ref);
+                const uint64_t neg2 = tc_two(neg, neg);
                 uint64_t sum0 = 0, sum1 = 0;                                      // (0, 0)
                 auto weigh = [&](const uint32_t* v, int c0) {                     // 32 scores -> 16 columns of weights
                     uint32_t w[16];

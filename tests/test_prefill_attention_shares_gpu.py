@@ -64,3 +64,32 @@ def test_fp32_rows_are_rounded_once(T, pos0, heads, kv_heads, hd):
     plain = torch.empty_like(q)
     _lib.check(_lib.load().sllm_prefill_attention(q.data_ptr(), k.data_ptr(), v.data_ptr(), 0, plain.data_ptr(), T, pos0, S, hd, heads, kv_heads, torch.cuda.current_stream().cuda_stream))
     assert float((got.double() - plain.double()).norm() / plain.double().norm()) < 8e-3      # two results within 4e-3 of the same sums
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("T,pos0,heads,kv_heads", [(1, 6000, 8, 2), (300, 5000, 3, 1), (1500, 3000, 16, 4)])
+def test_keys_at_minus_infinity(T, pos0, heads, kv_heads, hd):
+    """A long run of keys whose scores are -inf, with whole shares in it: they count for nothing, with scratch as without."""
+    import torch
+
+    from simplellminference_b200 import _lib
+    lib, g = _lib.load(), torch.Generator(device="cuda").manual_seed(T + hd)
+    n = pos0 + T
+    q = torch.randn(T, heads * hd, device="cuda", generator=g)
+    k, v = (torch.randn(kv_heads, n, hd, device="cuda", generator=g) for _ in range(2))
+    q[:, ::hd] = 1.0
+    k[:, 700:2900, 0] = float("-inf")
+    q, k, v = (t.to(torch.bfloat16) for t in (q, k, v))
+    need = lib.sllm_prefill_attention_scratch(1, T, pos0, hd, heads, kv_heads)
+    assert need > 0
+    scratch = torch.full((need // 4,), float("nan"), device="cuda")
+    hidden = torch.arange(n, device="cuda")[None] > (pos0 + torch.arange(T, device="cuda"))[:, None]
+    for room in (need, 0):
+        out = torch.full((T, heads * hd), 7.0, device="cuda", dtype=torch.bfloat16)
+        _lib.check(lib.sllm_prefill_attention_in(q.data_ptr(), k.data_ptr(), v.data_ptr(), 1, out.data_ptr(), T, pos0, n, hd, heads, kv_heads, scratch.data_ptr(), room,
+                                                 torch.cuda.current_stream().cuda_stream))
+        for h in range(heads):
+            kh, vh = k[h // (heads // kv_heads)].double(), v[h // (heads // kv_heads)].double()
+            s = (q.view(T, heads, hd)[:, h].double() @ kh.T) / hd ** 0.5
+            want = torch.softmax(s.masked_fill(hidden, float("-inf")), -1) @ vh
+            assert float((out.double().view(T, heads, hd)[:, h] - want).norm() / want.norm()) < 4e-3, (room, h)
