@@ -6,7 +6,7 @@
  * functions kernel::<op>_kernel_cuda (include/kernel/cuda/<op>_kernel.cuh) that the op layers call (source/op/<op>.cpp) plus
  * model::LlamaModel::forward (source/model/model.cpp:40-140). Each entry point below names the reference
  * interface it replaces. The C++ host mirror in simplellminference_b200/host/ (mem::Tensor, op::*Layer,
- * kernel::*_cuda, model::LlamaModel) is a thin layer over exactly these functions; INTEGRATION.md shows the
+ * kernel::*_cuda, model::LlamaModel) is a thin layer over exactly these functions; the integration guide shows the
  * binding a maintainer of the reference would add.
  *
  * Conventions
@@ -71,7 +71,7 @@ int sllm_abi_version(void);
  * megakernel MEASUREMENT aid, results are garbage: bit 0 = skip the grid barriers, bit 1 = skip the dot products,
  * bit 4 = tensor-parallel prefill without its peer-memory exchanges (the GEMM / attention time alone); key 9 = ragged-batch attention
  * (sllm_seq_attention): 1 (default) tensor-core body for bf16 pools on steps that hold a prompt portion, 0 = always the fp32 body;
- * key 10 = polls after which a wait inside the tcgen05 kernels (products: 512 clocks apiece) is given up (default 2^24, seconds; 0 gives up at once: for tests of the report) */
+ * key 10 = after how many times 512 clocks a wait inside the tcgen05 kernels is given up (default 2^24, some 4 seconds; 0 gives up at once: for tests of the report) */
 int sllm_tune(int32_t key, int32_t value);
 /* device facts the host side sizes things by: sm count, max opt-in shared memory per block, total/free HBM */
 int sllm_device_info(int32_t* sm_count, int32_t* smem_optin_bytes, size_t* hbm_total, size_t* hbm_free);

@@ -40,7 +40,6 @@ constexpr uint32_t kPfABytes = kPfBM * kPfBK * 2;
 // the host picks the BN that fills the last wave best, e.g. 192 instead of 256 for a 512 x 12288 output on 74 SM pairs.
 constexpr int kPfMaxStages = 12;
 constexpr uint32_t kPfRingBytes = 192 * 1024;          // operand ring; stages = ring / (A box + this CTA's W box)
-constexpr long long kPfPollClocks = 512;               // a poll that g_tune_tc_polls allows, in clocks: some 4 seconds in all by default
 constexpr uint32_t kPfTmemCols = 512;                  // two accumulators of up to 256 fp32 columns
 constexpr size_t kPfSmem = 1024 /*alignment slack*/ + kPfRingBytes + 512 /*barriers + tmem slot*/ + 4 * 4096 /*rows on their way through the epilogue*/;
 
@@ -636,7 +635,7 @@ int pf_gemm(PfCache* cache, const PfGemmArgs& a, cudaStream_t st) {
     p.groups = groups;
     if (int rc = status_check()) return rc;
     if (int rc = status_word(&p.status)) return rc;
-    p.wait_clocks = kPfPollClocks * g_tune_tc_polls;
+    p.wait_clocks = kPollClocks * g_tune_tc_polls;
 
     CUtensorMap tmA;
     {

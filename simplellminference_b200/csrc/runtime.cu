@@ -21,7 +21,7 @@ int g_tune_batch_rows4 = 0;   // batched decode GEMV: 1 = four weight rows per w
 int g_tune_batch_ksplit = 0;  // batched decode, with rows4: down projection with K cut in two over grid.y when more vectors are live than fit whole rows (experimental)
 int g_tune_mega_debug = 0;   // decode megakernel measurement aid (MegaParams::debug): bit 0 = no grid barriers, bit 1 = no dot products; results are garbage
 int g_tune_seq_attn_mma = 1;   // ragged-batch attention: 1 = tensor-core body for bf16 pools on steps with prompt portions, 0 = always the fp32 body
-int g_tune_tc_polls = 1 << 24;   // tcgen05 kernels: polls after which a wait is given up
+int g_tune_tc_polls = 1 << 24;   // tcgen05 kernels: 512 clocks apiece (4 seconds in all) after which a wait is given up
 int g_tune_pf_pair = -1;   // prefill GEMM: 1 / 0 = force / forbid the two-SM (cta_group::2) kernel, -1 = heuristic
 
 void set_error(const char* fmt, ...) {

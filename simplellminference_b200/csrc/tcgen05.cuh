@@ -160,10 +160,13 @@ __device__ __forceinline__ uint32_t tc_pack(float lo, float hi) {
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
     return r;
 }
-// Bounded wait on a barrier. False once this thread's polls have run out or another one of the CTA has given up (a flag in shared memory): the kernel then
-// tears down without its result and says so in the library's status word (tc_gave_up).
+// Bounded wait on a barrier. False once this thread has waited for kPollClocks times `polls` clocks (0: without a poll) or another one of the CTA has given up (a flag in shared memory): the
+// kernel then tears down without its result and says so in the library's status word (tc_gave_up). By the clock, since a poll may sleep, for how long is up to the hardware: counted, 2^24 of
+// them need not be over within minutes. The clock is read after every 16 polls that found nothing.
+constexpr long long kPollClocks = 512;
 __device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile int* gave_up, unsigned polls) {
-    for (unsigned i = 0; i < polls; ++i) {
+    long long since = 0;
+    for (unsigned i = 1; polls; ++i) {
         uint32_t done;
         asm volatile(
             "{\n.reg .pred p;\n"
@@ -171,7 +174,10 @@ __device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile
             "selp.u32 %0, 1, 0, p;\n}\n"
             : "=r"(done) : "r"(s_addr(bar)), "r"(parity) : "memory");
         if (done) return true;
-        if ((i & 1023) == 1023 && *gave_up) return false;
+        if (i & 15) continue;
+        const long long now = clock64();
+        if (!since) since = now;
+        if (*gave_up || now - since > kPollClocks * (long long)polls) break;
     }
     *gave_up = 1;
     return false;
