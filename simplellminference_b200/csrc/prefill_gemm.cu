@@ -356,9 +356,13 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
         *gave_up = p.wait_clocks == 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    // The forms of tcgen05.alloc and tcgen05.dealloc for a pair act on both CTAs' tensor memory: whoever issues one has to make sure that the peer runs already and is still there. Hence the barrier
+    // of the pair in front of the first and the one behind the last (see the end). No third one is needed for the peer's allocation: the leader's first product waits for the peer's bytes, which
+    // the peer asks for when it has its columns.
+    if (PAIR) cluster_sync_all();   // and the peer's barriers are initialised before anything signals them
     if (warp == 1) { if (PAIR) tc_alloc_pair(tmem_slot, kPfTmemCols); else tc_alloc(tmem_slot, kPfTmemCols); }
     tc_fence_before();
-    if (PAIR) cluster_sync_all(); else __syncthreads();   // pair: the peer's barriers are initialised before anything signals them
+    __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     // programmatic dependent launch: everything above overlapped the previous kernel's tail; its results (A, the residual
@@ -490,11 +494,14 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
     }
     tc_fence_before();
     if (PAIR) cluster_sync_all(); else __syncthreads();   // pair: nobody leaves while the peer may still signal its barriers / read its operands
-    if (__syncthreads_or(*gave_up)) tc_gave_up(p.status);
+    if (*gave_up) tc_gave_up(p.status);                   // set, if at all, in front of the barrier
     if (warp == 1) {
         tc_fence_after();
         if (PAIR) tc_dealloc_pair(tmem_base, kPfTmemCols); else tc_dealloc(tmem_base, kPfTmemCols);
     }
+    // pair: nobody leaves before both have given up the tensor memory. An SM whose CTA had left could hold another kernel's CTA, with columns of its own, when the peer's dealloc for the pair came
+    // through; the wait for columns is the one in this kernel that nothing bounds.
+    if (PAIR) cluster_sync_all();
 }
 
 // -------------------------------------------------------------------------------------------- host ----
