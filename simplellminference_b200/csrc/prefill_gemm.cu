@@ -419,6 +419,15 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
                     if (++stage == ST) { stage = 0; phase ^= 1; }
                 }
             }
+            // The last arrivals on `empty`, which no load waits for, come from the leader's SM: this CTA stays until they are in, its shared memory is another's afterwards. (A stage never
+            // used is empty from the start.) They are in before the last accumulator is, so nothing waits longer for it.
+            if (PAIR) {
+#pragma unroll 1
+                for (int s = 0; ok && s < ST; ++s) {
+                    ok = pf_wait<PAIR>(empty + stage, phase ^ 1, gave_up, p.wait_clocks);
+                    if (++stage == ST) { stage = 0; phase ^= 1; }
+                }
+            }
         }
         __syncwarp();
     } else if (warp == 1) {
