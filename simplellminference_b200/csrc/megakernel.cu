@@ -1,8 +1,8 @@
 // csrc/megakernel.cu — the whole decode step as ONE persistent cooperative kernel (sm_100a).
 //
 // Why: with one kernel per fused op (decode_fused.cuh) every launch boundary drains the HBM pipe — measured
-// on B200: 2-5 us of ramp + tail per GEMV kernel x 128 kernels, and a 12 us latency chain per attention launch
-// (profiles/r01_launches_fused_path.md). Here the step is one launch of `SM count` CTAs (1 per SM, 16 warps) that walks
+// on B200: 2-5 us of ramp + tail per GEMV kernel x 128 kernels, and a 12 us latency chain per attention launch.
+// Here the step is one launch of `SM count` CTAs (1 per SM, 16 warps) that walks
 // the phases  A qkv | B attention | C wo | D gate_up | E down  of every layer and finally F classifier+argmax,
 // separated by grid barriers, and the WEIGHT STREAM NEVER STOPS:
 //
